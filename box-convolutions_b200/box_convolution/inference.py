@@ -12,8 +12,7 @@ the Python and launch overhead out of single-frame latency (the scenario of the 
 """
 import torch
 
-from ._cabi import check, lib
-from .ext import _require_cuda_float, _stream, _workspace
+from . import _torch_binding as _native
 
 
 def fold_batchnorm(bn):
@@ -37,43 +36,10 @@ def fused_box_block(module, input, *, input_relu=False, scale=None, shift=None, 
     residual  tensor of the output's shape or None;
     out       where to write (may be ``residual`` for an in-place skip connection); allocated if None.
     """
-    _require_cuda_float(input, "input", torch.float32)
-    if input.dim() != 4 or input.size(1) != module.in_planes:
-        raise RuntimeError("fused_box_block: input must be (N, %d, h, w)" % module.in_planes)
-    input = input.detach().contiguous()
-    N, C, h, w = input.shape
-    F = module.num_filters
-    dev = input.device
-
-    def per_channel(t, name):
-        if t is None:
-            return None
-        _require_cuda_float(t, name, torch.float32)
-        if t.numel() != C * F or t.device != dev:
-            raise RuntimeError("fused_box_block: %s must hold %d values on the input's device" % (name, C * F))
-        return t.detach().contiguous()
-
-    scale, shift = per_channel(scale, "scale"), per_channel(shift, "shift")
-    if out is None:
-        out = torch.empty((N, C * F, h, w), dtype=torch.float32, device=dev)
-    for t, name in ((residual, "residual"), (out, "out")):
-        if t is None:
-            continue
-        _require_cuda_float(t, name, torch.float32)
-        if tuple(t.shape) != (N, C * F, h, w) or not t.is_contiguous() or t.device != dev:
-            raise RuntimeError("fused_box_block: %s must be a contiguous (N, %d, h, w) tensor on the input's device" % (name, C * F))
-    params = [p.detach().contiguous() for p in (module.x_min, module.x_max, module.y_min, module.y_max)]
-    with torch.cuda.device(dev):
-        ws = _workspace(lib.bc_boxconv2d_forward_workspace(N, C, F, h, w), dev)
-        check(lib.bc_boxconv2d_forward_fused(
-            input.data_ptr(), *[p.data_ptr() for p in params],
-            float(module.reparametrization_h), float(module.reparametrization_w), out.data_ptr(),
-            N, C, F, h, w, int(bool(module.normalize)), int(bool(module.exact)),
-            int(bool(input_relu)), scale.data_ptr() if scale is not None else None,
-            shift.data_ptr() if shift is not None else None,
-            residual.detach().data_ptr() if residual is not None else None, int(bool(output_relu)),
-            ws.data_ptr(), ws.numel(), _stream()), "bc_boxconv2d_forward_fused")
-    return out
+    return _native.fused_block(
+        input, module.x_min, module.x_max, module.y_min, module.y_max,
+        module.reparametrization_h, module.reparametrization_w, module.normalize, module.exact,
+        input_relu, scale, shift, residual, output_relu, out, module.in_planes)
 
 
 class GraphedForward:

@@ -50,6 +50,10 @@ int check_launch(const char *what);
 // cudaErrorNotReady, for one, is not sticky) and returns BC_ERR_CUDA.
 int cuda_failed(cudaError_t e, const char *what);
 
+// Allows `kernel` up to `bytes` of dynamic shared memory on the current device (done once per thread,
+// kernel and device).
+int raise_smem_limit(const void *kernel, int bytes);
+
 // Kernel ids reported by the profiling aid (bc_profile_get / bc_kernel_name).
 enum KernelId {
     KID_INTEGRAL = 1, KID_FORWARD_GLOBAL, KID_BACKWARD_GLOBAL, KID_FINISH_PARAM_GRADS, KID_CLIP,
@@ -114,14 +118,20 @@ int launch_backward_global(const T *x, const T *x_integ, const T *go_integ, cons
                            bool exact, int need_mask, T *grad_input, T *grad_params, T *partials,
                            cudaStream_t s);
 
-template <typename T>
-int launch_clip(T *x_min, T *x_max, T *y_min, T *y_max, int count, double rep_h, double rep_w,
-                double max_h, double max_w, bool exact, cudaStream_t s, T *packed = nullptr);
+template <typename S, typename T>
+int launch_clip(S *x_min, S *x_max, S *y_min, S *y_max, int count, double rep_h, double rep_w,
+                double max_h, double max_w, bool exact, cudaStream_t s, T *packed);
+// 16-bit parameters (io_kind: BC_IO_F16 / BC_IO_BF16), float copy
+int launch_clip_narrow(void *x_min, void *x_max, void *y_min, void *y_max, int io_kind, int count, double rep_h, double rep_w,
+                       double max_h, double max_w, bool exact, cudaStream_t s, float *packed);
+int launch_pack(const void *x_min, const void *x_max, const void *y_min, const void *y_max, int io_kind, int count, float *packed,
+                cudaStream_t s);
 
+// grad_params is stored as io_kind says when T is float (BC_IO_*), as T otherwise
 template <typename T>
 int launch_finish_param_grads(const T *partials, const BoxParamsT<T> &bp, int count, int per_box,
                               bool normalize, bool exact, T rep_h, T rep_w, int need_mask,
-                              T *grad_params, cudaStream_t s);
+                              void *grad_params, cudaStream_t s, int io_kind = BC_IO_F32);
 
 // float integral image with an optional ReLU on the values read
 // lpad/rpad > 0 write rows as [lpad zeros | I[a][0..w] | rpad copies of I[a][w]] (pitch lpad + w + 1 + rpad)
@@ -153,7 +163,8 @@ int launch_forward_plane_narrow(const void *x, int io_kind, const BoxParams &bp,
                                 int w, bool normalize, bool exact, cudaStream_t s);
 int launch_backward_plane_narrow(const void *x, const void *grad_output, int io_kind, const BoxParams &bp, float rep_h,
                                  float rep_w, int N, int C, int F, int h, int w, bool normalize, bool exact,
-                                 int need_mask, void *grad_input, float *grad_params, float *partials, cudaStream_t s);
+                                 int need_mask, void *grad_input, void *grad_params, int grad_params_kind, float *partials,
+                                 cudaStream_t s);
 
 // Column-band kernels for planes that do not fit in shared memory whole (box_band_smem.cu): they
 // gather from integral images in global memory in the padded row layout

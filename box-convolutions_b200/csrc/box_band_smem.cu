@@ -292,9 +292,7 @@ template <class K>
 int band_opt_in(K kernel, size_t bytes)
 {
     if (bytes <= 40 * 1024) return BC_OK;
-    if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes))
-        return cuda_failed(e, "shared memory opt-in");
-    return BC_OK;
+    return raise_smem_limit(reinterpret_cast<const void *>(kernel), (int)kBandMaxSmem);
 }
 
 }  // namespace

@@ -8,6 +8,9 @@
 // (plane, tile); the block loops over the filters so that grad-input is accumulated in
 // registers and written once, and leaves five partial sums per filter that the finishing kernel
 // turns into the parameter gradients (no atomics: a fixed summation order, bit-reproducible).
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
 #include "bc_common.cuh"
 #include "bc_walk.cuh"
 
@@ -266,7 +269,7 @@ backward_global_kernel(const T *__restrict__ x, const T *__restrict__ x_integ,
 template <typename T>
 __global__ void finish_param_grads_kernel(const T *__restrict__ partials, BoxParamsT<T> bp, int count,
                                           int per_box, bool normalize, bool exact, T rep_h, T rep_w,
-                                          int need_mask, T *__restrict__ grad_params)
+                                          int need_mask, void *__restrict__ grad_params, int io_kind)
 {
     grid_dependency_wait();
     const int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -287,14 +290,19 @@ __global__ void finish_param_grads_kernel(const T *__restrict__ partials, BoxPar
         finish_param_grads(s, box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact, rep_h, rep_w, g);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (need_mask & (BC_NEED_X_MIN << j)) grad_params[(int64_t)j * count + k] = g[j];
+            if (need_mask & (BC_NEED_X_MIN << j)) {
+                const int64_t at = (int64_t)j * count + k;
+                if (io_kind == BC_IO_F16) static_cast<__half *>(grad_params)[at] = __float2half_rn((float)g[j]);
+                else if (io_kind == BC_IO_BF16) static_cast<__nv_bfloat16 *>(grad_params)[at] = __float2bfloat16_rn((float)g[j]);
+                else static_cast<T *>(grad_params)[at] = g[j];
+            }
     }
 }
 
 template <typename T>
 int launch_finish_param_grads(const T *partials, const BoxParamsT<T> &bp, int count, int per_box,
                               bool normalize, bool exact, T rep_h, T rep_w, int need_mask,
-                              T *grad_params, cudaStream_t s)
+                              void *grad_params, cudaStream_t s, int io_kind)
 {
     const int warps_per_block = 4;
     const int blocks = (count + warps_per_block - 1) / warps_per_block;
@@ -302,7 +310,7 @@ int launch_finish_param_grads(const T *partials, const BoxParamsT<T> &bp, int co
         LaunchScope scope(KID_FINISH_PARAM_GRADS, s);
         if (cudaError_t e = launch_overlapped(finish_param_grads_kernel<T>, (unsigned)blocks, warps_per_block * 32, 0, s,
                                               partials, bp, count, per_box, normalize, exact, rep_h, rep_w, need_mask,
-                                              grad_params))
+                                              grad_params, io_kind))
             return cuda_failed(e, "finish_param_grads");
     }
     return check_launch("finish_param_grads");
@@ -378,8 +386,8 @@ int launch_backward_global(const T *x, const T *x_integ, const T *go_integ, cons
 }
 
 // the two instantiations of the general path
-template int launch_finish_param_grads<float>(const float *, const BoxParamsT<float> &, int, int, bool, bool, float, float, int, float *, cudaStream_t);
-template int launch_finish_param_grads<double>(const double *, const BoxParamsT<double> &, int, int, bool, bool, double, double, int, double *, cudaStream_t);
+template int launch_finish_param_grads<float>(const float *, const BoxParamsT<float> &, int, int, bool, bool, float, float, int, void *, cudaStream_t, int);
+template int launch_finish_param_grads<double>(const double *, const BoxParamsT<double> &, int, int, bool, bool, double, double, int, void *, cudaStream_t, int);
 template int launch_forward_global<float>(const float *, const BoxParamsT<float> &, float *, int, int, int, int, int, bool, bool, cudaStream_t);
 template int launch_forward_global<double>(const double *, const BoxParamsT<double> &, double *, int, int, int, int, int, bool, bool, cudaStream_t);
 template int launch_backward_global<float>(const float *, const float *, const float *, const BoxParamsT<float> &, float, float, int, int, int, int, int, bool, bool, int, float *, float *, float *, cudaStream_t);

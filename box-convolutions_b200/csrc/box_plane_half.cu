@@ -20,17 +20,18 @@ int launch_forward_plane_narrow(const void *x, int io_kind, const BoxParams &bp,
 
 int launch_backward_plane_narrow(const void *x, const void *grad_output, int io_kind, const BoxParams &bp, float rep_h,
                                  float rep_w, int N, int C, int F, int h, int w, bool normalize, bool exact,
-                                 int need_mask, void *grad_input, float *grad_params, float *partials, cudaStream_t s)
+                                 int need_mask, void *grad_input, void *grad_params, int grad_params_kind, float *partials,
+                                 cudaStream_t s)
 {
     if (io_kind == BC_IO_F16)
         return launch_backward_plane_t<__half>(static_cast<const __half *>(x), static_cast<const __half *>(grad_output), bp,
                                                rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask,
-                                               static_cast<__half *>(grad_input), grad_params, partials, s);
+                                               static_cast<__half *>(grad_input), grad_params, grad_params_kind, partials, s);
     if (io_kind == BC_IO_BF16)
         return launch_backward_plane_t<__nv_bfloat16>(static_cast<const __nv_bfloat16 *>(x),
                                                       static_cast<const __nv_bfloat16 *>(grad_output), bp, rep_h, rep_w, N,
                                                       C, F, h, w, normalize, exact, need_mask,
-                                                      static_cast<__nv_bfloat16 *>(grad_input), grad_params, partials, s);
+                                                      static_cast<__nv_bfloat16 *>(grad_input), grad_params, grad_params_kind, partials, s);
     return BC_ERR_UNSUPPORTED;
 }
 

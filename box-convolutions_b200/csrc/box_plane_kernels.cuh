@@ -739,13 +739,14 @@ backward_plane_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_outp
     }
 }
 
+// The limit is raised to its maximum once per kernel and device (it is a ceiling, not a reservation: what a
+// launch occupies is what it asks for), so that threads launching different sizes do not lower it for
+// one another and a launch does not pay for the call.
 template <class K>
 int opt_in_smem(K kernel, size_t bytes)
 {
     if (bytes <= 34 * 1024) return BC_OK;     // static scratch included, this stays under the 48 KB default
-    if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes))
-        return cuda_failed(e, "shared memory opt-in");
-    return BC_OK;
+    return raise_smem_limit(reinterpret_cast<const void *>(kernel), kMaxSmem);
 }
 
 inline bool aligned_to(const void *p, int bytes) { return (reinterpret_cast<uintptr_t>(p) & (uintptr_t)(bytes - 1)) == 0; }
@@ -817,7 +818,7 @@ int launch_forward_plane_t(const IO *x, const BoxParams &bp, const Fusion *fu, I
 template <typename IO>
 int launch_backward_plane_t(const IO *x, const IO *grad_output, const BoxParams &bp, float rep_h, float rep_w, int N,
                             int C, int F, int h, int w, bool normalize, bool exact, int need_mask, IO *grad_input,
-                            float *grad_params, float *partials, cudaStream_t s)
+                            void *grad_params, int grad_params_kind, float *partials, cudaStream_t s)
 {
     const int64_t planes = (int64_t)N * C;
     if (planes > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
@@ -864,7 +865,7 @@ int launch_backward_plane_t(const IO *x, const IO *grad_output, const BoxParams 
     st = check_launch("backward_plane");
     if (st != BC_OK || !need_params) return st;
     return launch_finish_param_grads<float>(partials, bp, C * F, N, normalize, exact, rep_h, rep_w, need_mask,
-                                            grad_params, s);
+                                            grad_params, s, grad_params_kind);
 }
 
 // Bounded waits that expired in the kernels of this translation unit (synchronises).

@@ -25,7 +25,7 @@ int launch_backward_plane(const float *x, const float *grad_output, const BoxPar
                           cudaStream_t s)
 {
     return launch_backward_plane_t<float>(x, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask,
-                                          grad_input, grad_params, partials, s);
+                                          grad_input, grad_params, BC_IO_F32, partials, s);
 }
 
 // Number of bounded waits that expired on the current device since the library was loaded

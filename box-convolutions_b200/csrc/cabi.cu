@@ -27,6 +27,20 @@ int cuda_failed(cudaError_t e, const char *what)
     return BC_ERR_CUDA;
 }
 
+int raise_smem_limit(const void *kernel, int bytes)
+{
+    struct Done { const void *kernel; int device; };
+    static thread_local std::vector<Done> done;
+    int device = -1;
+    if (cudaError_t e = cudaGetDevice(&device)) return cuda_failed(e, "cudaGetDevice");
+    for (const Done &d : done)
+        if (d.kernel == kernel && d.device == device) return BC_OK;
+    if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes))
+        return cuda_failed(e, "shared memory opt-in");
+    done.push_back({kernel, device});
+    return BC_OK;
+}
+
 // ---- launch counter and per-kernel event timing
 static std::atomic<uint64_t> g_launches{0};
 static std::mutex g_prof_mutex;
@@ -162,7 +176,7 @@ static int clip_entry(T *x_min, T *x_max, T *y_min, T *y_max, int count, double 
     if (count == 0) return BC_OK;
     if (!x_min || !x_max || !y_min || !y_max) return BC_ERR_NULL_POINTER;
     if (reparametrization_h == 0.0 || reparametrization_w == 0.0) return BC_ERR_BAD_SHAPE;
-    return launch_clip<T>(x_min, x_max, y_min, y_max, count, reparametrization_h, reparametrization_w,
+    return launch_clip<T, T>(x_min, x_max, y_min, y_max, count, reparametrization_h, reparametrization_w,
                           max_input_h, max_input_w, exact != 0, stream, packed);
 }
 
@@ -281,6 +295,27 @@ int bc_clip_parameters_f64(double *x_min, double *x_max, double *y_min, double *
 {
     return clip_entry<double>(x_min, x_max, y_min, y_max, count, reparametrization_h, reparametrization_w,
                               max_input_h, max_input_w, exact, stream);
+}
+
+int bc_clip_parameters_narrow(void *x_min, void *x_max, void *y_min, void *y_max, int io_kind, int count,
+                              double reparametrization_h, double reparametrization_w, double max_input_h,
+                              double max_input_w, int exact, float *packed_out, bc_stream_t stream)
+{
+    if (count < 0) return BC_ERR_BAD_SHAPE;
+    if (count == 0) return BC_OK;
+    if (!x_min || !x_max || !y_min || !y_max) return BC_ERR_NULL_POINTER;
+    if (reparametrization_h == 0.0 || reparametrization_w == 0.0) return BC_ERR_BAD_SHAPE;
+    return launch_clip_narrow(x_min, x_max, y_min, y_max, io_kind, count, reparametrization_h, reparametrization_w,
+                              max_input_h, max_input_w, exact != 0, stream, packed_out);
+}
+
+int bc_pack_parameters(const void *x_min, const void *x_max, const void *y_min, const void *y_max, int io_kind, int count,
+                       float *packed_out, bc_stream_t stream)
+{
+    if (count < 0) return BC_ERR_BAD_SHAPE;
+    if (count == 0) return BC_OK;
+    if (!x_min || !x_max || !y_min || !y_max || !packed_out) return BC_ERR_NULL_POINTER;
+    return launch_pack(x_min, x_max, y_min, y_max, io_kind, count, packed_out, stream);
 }
 
 size_t bc_boxconv2d_forward_workspace(int N, int C, int F, int h, int w)
@@ -431,12 +466,13 @@ int bc_boxconv2d_forward_narrow(const void *input, int io_kind, const float *x_m
     return launch_forward_plane_narrow(input, io_kind, bp, output, N, C, F, h, w, normalize != 0, exact != 0, stream);
 }
 
-int bc_boxconv2d_backward_narrow(const void *input, int io_kind, const float *x_min, const float *x_max,
-                                 const float *y_min, const float *y_max, const void *grad_output,
-                                 float reparametrization_h, float reparametrization_w, int N, int C,
-                                 int F, int h, int w, int normalize, int exact, int need_mask,
-                                 void *grad_input, float *grad_params, void *workspace,
-                                 size_t workspace_bytes, bc_stream_t stream)
+// grad_params_kind: how the parameter gradients are stored (BC_IO_*)
+static int backward_narrow(const void *input, int io_kind, const float *x_min, const float *x_max,
+                           const float *y_min, const float *y_max, const void *grad_output,
+                           float reparametrization_h, float reparametrization_w, int N, int C,
+                           int F, int h, int w, int normalize, int exact, int need_mask,
+                           void *grad_input, void *grad_params, int grad_params_kind, void *workspace,
+                           size_t workspace_bytes, bc_stream_t stream)
 {
     if (!sizes_ok(N, C, F, h, w)) return BC_ERR_BAD_SHAPE;
     if (io_kind != BC_IO_F16 && io_kind != BC_IO_BF16) return BC_ERR_UNSUPPORTED;
@@ -447,9 +483,11 @@ int bc_boxconv2d_backward_narrow(const void *input, int io_kind, const float *x_
         if (need_params && C > 0 && F > 0) {
             if (!grad_params) return BC_ERR_NULL_POINTER;
             for (int j = 0; j < 4; ++j)
-                if (need_mask & (BC_NEED_X_MIN << j))
-                    if (cudaError_t e = cudaMemsetAsync(grad_params + (size_t)j * C * F, 0, sizeof(float) * C * F, stream))
+                if (need_mask & (BC_NEED_X_MIN << j)) {
+                    const size_t bytes = (grad_params_kind == BC_IO_F32 ? 4 : 2) * (size_t)C * F;
+                    if (cudaError_t e = cudaMemsetAsync(static_cast<char *>(grad_params) + j * bytes, 0, bytes, stream))
                         return cuda_failed(e, "memset");
+                }
         }
         return BC_OK;
     }
@@ -463,7 +501,31 @@ int bc_boxconv2d_backward_narrow(const void *input, int io_kind, const float *x_
     const BoxParams bp{x_min, x_max, y_min, y_max, reparametrization_h, reparametrization_w};
     return launch_backward_plane_narrow(input, grad_output, io_kind, bp, reparametrization_h, reparametrization_w, N, C,
                                         F, h, w, normalize != 0, exact != 0, need_mask, grad_input, grad_params,
-                                        static_cast<float *>(workspace), stream);
+                                        grad_params_kind, static_cast<float *>(workspace), stream);
+}
+
+int bc_boxconv2d_backward_narrow(const void *input, int io_kind, const float *x_min, const float *x_max,
+                                 const float *y_min, const float *y_max, const void *grad_output,
+                                 float reparametrization_h, float reparametrization_w, int N, int C,
+                                 int F, int h, int w, int normalize, int exact, int need_mask,
+                                 void *grad_input, float *grad_params, void *workspace,
+                                 size_t workspace_bytes, bc_stream_t stream)
+{
+    return backward_narrow(input, io_kind, x_min, x_max, y_min, y_max, grad_output, reparametrization_h, reparametrization_w,
+                           N, C, F, h, w, normalize, exact, need_mask, grad_input, grad_params, BC_IO_F32, workspace,
+                           workspace_bytes, stream);
+}
+
+int bc_boxconv2d_backward_narrow_all(const void *input, int io_kind, const float *x_min, const float *x_max,
+                                     const float *y_min, const float *y_max, const void *grad_output,
+                                     float reparametrization_h, float reparametrization_w, int N, int C,
+                                     int F, int h, int w, int normalize, int exact, int need_mask,
+                                     void *grad_input, void *grad_params, void *workspace,
+                                     size_t workspace_bytes, bc_stream_t stream)
+{
+    return backward_narrow(input, io_kind, x_min, x_max, y_min, y_max, grad_output, reparametrization_h, reparametrization_w,
+                           N, C, F, h, w, normalize, exact, need_mask, grad_input, grad_params, io_kind, workspace,
+                           workspace_bytes, stream);
 }
 
 // ---- backward pass on the library's own scratch array (see the header for who needs this)

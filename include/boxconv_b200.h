@@ -202,7 +202,7 @@ int bc_boxconv2d_host_step(const float *x_host, const float *grad_output_host, f
  * Served for planes that the shared-memory kernels hold: bc_boxconv2d_narrow_supported() tells;
  * other shapes return BC_ERR_UNSUPPORTED and the caller converts to float.  Scratch size as for the
  * float functions. */
-enum { BC_IO_F16 = 1, BC_IO_BF16 = 2 };
+enum { BC_IO_F32 = 0, BC_IO_F16 = 1, BC_IO_BF16 = 2 };
 int bc_boxconv2d_narrow_supported(int F, int h, int w);
 int bc_boxconv2d_forward_narrow(const void *input, int io_kind, const float *x_min, const float *x_max,
                                 const float *y_min, const float *y_max, float reparametrization_h,
@@ -214,6 +214,21 @@ int bc_boxconv2d_backward_narrow(const void *input, int io_kind, const float *x_
                                  int F, int h, int w, int normalize, int exact, int need_mask,
                                  void *grad_input, float *grad_params, void *workspace,
                                  size_t workspace_bytes, bc_stream_t stream);
+/* The same with the parameter gradients stored in the 16-bit type too (rounded once, from the float sums). */
+int bc_boxconv2d_backward_narrow_all(const void *input, int io_kind, const float *x_min, const float *x_max,
+                                     const float *y_min, const float *y_max, const void *grad_output,
+                                     float reparametrization_h, float reparametrization_w, int N, int C,
+                                     int F, int h, int w, int normalize, int exact, int need_mask,
+                                     void *grad_input, void *grad_params, void *workspace,
+                                     size_t workspace_bytes, bc_stream_t stream);
+/* bc_clip_parameters() on 16-bit parameters (clipped as float, rounded when stored); packed_out, which may be
+ * NULL, receives a (4, count) float copy of the stored values. */
+int bc_clip_parameters_narrow(void *x_min, void *x_max, void *y_min, void *y_max, int io_kind, int count,
+                              double reparametrization_h, double reparametrization_w, double max_input_h,
+                              double max_input_w, int exact, float *packed_out, bc_stream_t stream);
+/* A (4, count) float copy of four parameter arrays of type io_kind (BC_IO_*), in one launch. */
+int bc_pack_parameters(const void *x_min, const void *x_max, const void *y_min, const void *y_max, int io_kind, int count,
+                       float *packed_out, bc_stream_t stream);
 
 /* ---- backward pass without caller-supplied scratch memory --------------------------------
  * This entry point has no counterpart in the reference (which allocates its temporaries with
