@@ -87,8 +87,13 @@ class BoxConv2d(torch.nn.Module):
 
     def forward(self, input):
         # in training the parameters are clipped first, as in the reference (box_convolution_module.py:183-222)
+        own = self._parameters
+        try:
+            x_min, x_max, y_min, y_max = own["x_min"], own["x_max"], own["y_min"], own["y_max"]
+        except KeyError:        # parametrised or replaced by plain tensors
+            x_min, x_max, y_min, y_max = self._parameters4()
         return _native.module_forward(
-            input, self.x_min, self.x_max, self.y_min, self.y_max,
+            input, x_min, x_max, y_min, y_max,
             self.reparametrization_h, self.reparametrization_w, self.normalize, self.exact,
             self.training, self.max_input_h, self.max_input_w)
 

@@ -57,7 +57,8 @@ int raise_smem_limit(const void *kernel, int bytes);
 // Kernel ids reported by the profiling aid (bc_profile_get / bc_kernel_name).
 enum KernelId {
     KID_INTEGRAL = 1, KID_FORWARD_GLOBAL, KID_BACKWARD_GLOBAL, KID_FINISH_PARAM_GRADS, KID_CLIP,
-    KID_FORWARD_PLANE, KID_BACKWARD_PLANE, KID_SUM_CHUNKS, KID_BACKWARD_BAND, KID_INTEGRAL_BANDS, KID_FORWARD_BAND, KID_COUNT
+    KID_FORWARD_PLANE, KID_BACKWARD_PLANE, KID_SUM_CHUNKS, KID_BACKWARD_BAND, KID_INTEGRAL_BANDS, KID_FORWARD_BAND,
+    KID_FORWARD_SLAB, KID_BACKWARD_SLAB, KID_COUNT
 };
 
 // Put around a kernel launch: counts it and, while profiling is enabled, records a CUDA event on
@@ -80,21 +81,32 @@ struct LaunchScope {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// In clusters of `cluster` CTAs.
 template <class... KArgs, class... Args>
-inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
-                                     cudaStream_t stream, Args... args)
+inline cudaError_t launch_overlapped_cluster(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, unsigned cluster,
+                                             cudaStream_t stream, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
+template <class... KArgs, class... Args>
+inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
+                                     cudaStream_t stream, Args... args)
+{
+    return launch_overlapped_cluster(kernel, grid, block, smem, 1, stream, args...);
 }
 #endif
 
@@ -166,7 +178,7 @@ int launch_backward_plane_narrow(const void *x, const void *grad_output, int io_
                                  int need_mask, void *grad_input, void *grad_params, int grad_params_kind, float *partials,
                                  cudaStream_t s);
 
-// Column-band kernels for planes that do not fit in shared memory whole (box_band_smem.cu): they
+// Column-band kernels for planes that are too wide for slabs (box_band_smem.cu): they
 // gather from integral images in global memory in the padded row layout
 // (launch_integral_image_f32 with band_lpad() / band_rpad(w)), staged band by band.
 int band_lpad();
@@ -181,5 +193,19 @@ int launch_forward_band(const float *integ_padded, const BoxParams &bp, const Fu
 int launch_backward_band(const float *x, const float *go_integ_padded, const BoxParams &bp, float rep_h, float rep_w,
                          int N, int C, int F, int h, int w, bool normalize, bool exact, int need_mask,
                          float *grad_input, float *grad_params, float *partials, cudaStream_t s);
+
+// Slab kernels for planes that do not fit in shared memory whole (box_slab.cu): they gather from integral
+// images in a workspace, written by launch_integral_quad in the quad layout (bc_quad.cuh).
+bool slab_path_fits(int F, int h, int w);
+size_t slab_integral_floats(int64_t planes, int h, int w);
+size_t slab_partials_bytes(int N, int C, int F, int h, int w);
+int launch_integral_quad(const void *in, int io_kind, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s);
+// null `fu` = plain forward (16-bit outputs: always)
+int launch_forward_slab(const float *integ, const BoxParams &bp, const Fusion *fu, void *out, int io_kind, int N, int C, int F,
+                        int h, int w, bool normalize, bool exact, cudaStream_t s);
+int launch_backward_slab(const void *x, int io_kind, const float *go_integ, const BoxParams &bp, float rep_h, float rep_w, int N,
+                         int C, int F, int h, int w, bool normalize, bool exact, int need_mask, void *grad_input, void *grad_params,
+                         int grad_params_kind, float *partials, cudaStream_t s);
+int read_wait_timeouts_slab(int *count);
 
 }  // namespace bc

@@ -36,11 +36,9 @@
 // output value takes about five 4-byte words from the integral image in shared memory, against
 // four bytes of HBM traffic.
 #pragma once
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
-
 #include "bc_common.cuh"
 #include "bc_smem_walk.cuh"
+#include "bc_tile_io.cuh"
 
 namespace bc {
 
@@ -107,121 +105,6 @@ __device__ __forceinline__ void init_integral_padding(float *sI, const Geometry 
         sI[a * pitch + (a >> 3) + c] = 0.0f;
     }
 }
-
-// ---- asynchronous bulk copies (TMA, no tensor map) global -> shared, completion on an mbarrier.
-// Every wait is bounded: when the limit expires the kernel counts the event in g_wait_timeouts
-// and carries on, so a lost copy shows up as a reported error instead of a hung GPU.
-static __device__ int g_wait_timeouts = 0;      // one counter per translation unit that includes this file
-constexpr long long kWaitLimitCycles = 2000000000LL;      // about a second
-
-__device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t mbar)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
-    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(mbar) : "memory");
-}
-// Hint that `bytes` (a multiple of 16) at `src` (16-byte aligned) will be copied soon: brings them into L2.
-__device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes)
-{
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity)
-{
-    const long long t0 = clock64();
-    for (;;) {
-        uint32_t done;
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-                     " selp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(done) : "r"(mbar), "r"(parity), "r"(2000u) : "memory");
-        if (done) return true;
-        if (clock64() - t0 > kWaitLimitCycles) return false;
-    }
-}
-
-// ---- storage types of the big tensors --------------------------------------------------------
-// The kernels are instantiated for float, __half and __nv_bfloat16 input / grad_output / output /
-// grad_input tensors.  Narrow types are converted as they are loaded and rounded to nearest as they
-// are stored; the integral images, every accumulator and the parameter gradients stay float.
-// load4 / store4 move the 4 values of one strip row with one instruction (16 or 8 bytes).
-template <typename IO>
-struct Io;
-
-template <>
-struct Io<float> {
-    static constexpr int kVecBytes = 16;
-    static __device__ __forceinline__ float4 load4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
-    static __device__ __forceinline__ float load1(const float *p) { return __ldg(p); }
-    static __device__ __forceinline__ void store4(float *p, float a, float b, float c, float d)
-    {
-        *reinterpret_cast<float4 *>(p) = make_float4(a, b, c, d);
-    }
-    static __device__ __forceinline__ void store1(float *p, float v) { *p = v; }
-    static __device__ __forceinline__ float4 lds4(uint32_t a) { return lds128(a); }
-};
-
-__device__ __forceinline__ uint2 lds64(uint32_t a)
-{
-    uint2 v;
-    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
-    return v;
-}
-
-template <>
-struct Io<__half> {
-    static constexpr int kVecBytes = 8;
-    static __device__ __forceinline__ float4 widen(uint2 r)
-    {
-        const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&r.x));
-        const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&r.y));
-        return make_float4(a.x, a.y, b.x, b.y);
-    }
-    static __device__ __forceinline__ float4 load4(const __half *p) { return widen(__ldg(reinterpret_cast<const uint2 *>(p))); }
-    static __device__ __forceinline__ float load1(const __half *p) { return __half2float(__ldg(p)); }
-    static __device__ __forceinline__ void store4(__half *p, float a, float b, float c, float d)
-    {
-        const __half2 lo = __floats2half2_rn(a, b), hi = __floats2half2_rn(c, d);
-        uint2 r;
-        r.x = *reinterpret_cast<const uint32_t *>(&lo);
-        r.y = *reinterpret_cast<const uint32_t *>(&hi);
-        *reinterpret_cast<uint2 *>(p) = r;
-    }
-    static __device__ __forceinline__ void store1(__half *p, float v) { *p = __float2half_rn(v); }
-    static __device__ __forceinline__ float4 lds4(uint32_t a) { return widen(lds64(a)); }
-};
-
-template <>
-struct Io<__nv_bfloat16> {
-    static constexpr int kVecBytes = 8;
-    static __device__ __forceinline__ float4 widen(uint2 r)
-    {
-        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&r.x));
-        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&r.y));
-        return make_float4(a.x, a.y, b.x, b.y);
-    }
-    static __device__ __forceinline__ float4 load4(const __nv_bfloat16 *p) { return widen(__ldg(reinterpret_cast<const uint2 *>(p))); }
-    static __device__ __forceinline__ float load1(const __nv_bfloat16 *p) { return __bfloat162float(__ldg(p)); }
-    static __device__ __forceinline__ void store4(__nv_bfloat16 *p, float a, float b, float c, float d)
-    {
-        const __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
-        uint2 r;
-        r.x = *reinterpret_cast<const uint32_t *>(&lo);
-        r.y = *reinterpret_cast<const uint32_t *>(&hi);
-        *reinterpret_cast<uint2 *>(p) = r;
-    }
-    static __device__ __forceinline__ void store1(__nv_bfloat16 *p, float v) { *p = __float2bfloat16_rn(v); }
-    static __device__ __forceinline__ float4 lds4(uint32_t a) { return widen(lds64(a)); }
-};
-
-template <typename IO>
-struct IsFloat { static constexpr bool value = false; };
-template <>
-struct IsFloat<float> { static constexpr bool value = true; };
 
 // Register block of a strip while the integral image is being built.
 template <int T>
@@ -749,8 +632,6 @@ int opt_in_smem(K kernel, size_t bytes)
     return raise_smem_limit(reinterpret_cast<const void *>(kernel), kMaxSmem);
 }
 
-inline bool aligned_to(const void *p, int bytes) { return (reinterpret_cast<uintptr_t>(p) & (uintptr_t)(bytes - 1)) == 0; }
-
 inline size_t plane_forward_smem_bytes(int h, int w)
 {
     return ((size_t)layout_floats(h, w) + 2 * (size_t)warp_tiles(h, w) * kTile) * sizeof(float);
@@ -866,13 +747,6 @@ int launch_backward_plane_t(const IO *x, const IO *grad_output, const BoxParams 
     if (st != BC_OK || !need_params) return st;
     return launch_finish_param_grads<float>(partials, bp, C * F, N, normalize, exact, rep_h, rep_w, need_mask,
                                             grad_params, s, grad_params_kind);
-}
-
-// Bounded waits that expired in the kernels of this translation unit (synchronises).
-inline int read_wait_timeouts_here(int *count)
-{
-    if (cudaError_t e = cudaMemcpyFromSymbol(count, g_wait_timeouts, sizeof(int))) return cuda_failed(e, "read_wait_timeouts");
-    return BC_OK;
 }
 
 }  // namespace

@@ -32,12 +32,14 @@ int launch_backward_plane(const float *x, const float *grad_output, const BoxPar
 // (synchronises).  Nonzero means an asynchronous copy never signalled completion.
 int read_wait_timeouts(int *count)
 {
-    int here = 0, narrow = 0;
+    int here = 0, narrow = 0, slab = 0;
     int st = read_wait_timeouts_here(&here);
     if (st != BC_OK) return st;
     st = read_wait_timeouts_narrow(&narrow);
     if (st != BC_OK) return st;
-    *count = here + narrow;
+    st = read_wait_timeouts_slab(&slab);
+    if (st != BC_OK) return st;
+    *count = here + narrow + slab;
     return BC_OK;
 }
 

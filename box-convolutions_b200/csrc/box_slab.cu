@@ -1,0 +1,588 @@
+// Forward and backward for planes too large to keep in shared memory whole.
+//
+// Two kernels a pass.  integral_quad_kernel writes the integral images of a batch of planes to a workspace,
+// rows in the quad layout (bc_quad.cuh).  The gather kernels then work on slabs: R rows of one plane, full
+// width.  What a slab of a box filter reads of the integral image is two runs of R + 1 adjacent rows, one on
+// either side of the box, each a contiguous piece of memory: two bulk copies per filter bring them to shared
+// memory, double-buffered, so the copies of the next filter run while the current one is gathered.
+//
+// Against gathering from column bands (32 columns, full height) a slab costs 2 (R+1)/R words of L2 traffic an
+// output instead of 2.5, two copy instructions instead of thousands of 16-byte ones, and reads shared
+// memory with 5 (R+1)/R words an output instead of 8.
+#include "bc_common.cuh"
+#include "bc_quad.cuh"
+#include "bc_tile_io.cuh"
+
+namespace bc {
+
+namespace {
+
+constexpr int kSlabMaxWarps = 16;
+constexpr size_t kSlabMaxSmem = 200 * 1024;
+constexpr int kStripRows = 8;              // rows per warp
+constexpr int kScanRows = 8;               // rows a warp of the integral kernel keeps in registers
+
+// ---- integral images ----------------------------------------------------------------------------
+// A CTA (one warp per 128 columns) walks down its rows: each lane keeps running column sums of its four
+// columns, scans eight rows at a time along the row (in the lane, across the warp by shuffles, across the
+// warps through shared memory, one barrier per eight rows) and stores them straight from registers; the next
+// eight rows are being loaded meanwhile.  No tile in shared memory, one pass over HBM.
+// With few planes a cluster of CTAs shares one: each first sums the columns of its rows, takes from the CTAs
+// above what they add to its columns (distributed shared memory), and then walks.
+template <typename IO, bool VEC>
+__device__ __forceinline__ float4 load_quad(const IO *row, int c, int w, bool row_ok)
+{
+    if (!row_ok || c >= w) return make_float4(0.f, 0.f, 0.f, 0.f);
+    if (VEC) return Io<IO>::load4(row + c);
+    float4 v = make_float4(Io<IO>::load1(row + c), 0.f, 0.f, 0.f);
+    if (c + 1 < w) v.y = Io<IO>::load1(row + c + 1);
+    if (c + 2 < w) v.z = Io<IO>::load1(row + c + 2);
+    if (c + 3 < w) v.w = Io<IO>::load1(row + c + 3);
+    return v;
+}
+
+__device__ __forceinline__ float4 relu4(float4 v)
+{
+    return make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+}
+
+// Inclusive sum over the warp; the shuffle's own predicate tells which lanes have somebody to add.
+__device__ __forceinline__ float warp_scan(float v)
+{
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1)
+        asm volatile("{\n .reg .f32 u;\n .reg .pred p;\n shfl.sync.up.b32 u|p, %0, %1, 0, 0xffffffff;\n @p add.f32 %0, %0, u;\n}"
+                     : "+f"(v) : "r"(d));
+    return v;
+}
+
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank)
+{
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float4 cluster_load4(uint32_t addr)
+{
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename IO, bool VEC, bool RELU, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 5 : 1)
+integral_quad_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, int w, int rows_per_cta, int cluster)
+{
+    __shared__ __align__(16) float sTot[2][kSlabMaxWarps][kScanRows];
+    extern __shared__ float4 sCol[];           // column sums of this CTA's rows (clusters only)
+    grid_dependency_release();
+    const int lane = threadIdx.x & 31, warp = uniform(threadIdx.x >> 5), nwarps = blockDim.x >> 5;
+    const int64_t plane = blockIdx.x / cluster;
+    const int rank = blockIdx.x % cluster;
+    const int L = threadIdx.x, c = L * 4;
+    const int cells = quad_cells(w), pitch = 4 * cells;
+    const int r0 = min(rank * rows_per_cta, h), r1 = min(r0 + rows_per_cta, h);
+    const IO *src = in + plane * (int64_t)h * w;
+    float *dst = out + plane * (int64_t)(h + 1) * pitch;
+
+    grid_dependency_wait();
+    float4 nxt[kScanRows];
+#pragma unroll
+    for (int i = 0; i < kScanRows; ++i) nxt[i] = load_quad<IO, VEC>(src + (int64_t)(r0 + i) * w, c, w, r0 + i < r1);
+
+    float run[4] = {0.f, 0.f, 0.f, 0.f};
+    if (cluster > 1) {
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 v[kScanRows];
+#pragma unroll
+        for (int i = 0; i < kScanRows; ++i) v[i] = nxt[i];
+        for (int r = r0; r < r1; r += kScanRows) {
+            float4 ahead[kScanRows];
+#pragma unroll
+            for (int i = 0; i < kScanRows; ++i) {
+                const int rn = r + kScanRows + i;
+                ahead[i] = load_quad<IO, VEC>(src + (int64_t)rn * w, c, w, rn < r1);
+            }
+#pragma unroll
+            for (int i = 0; i < kScanRows; ++i) {
+                if (RELU) v[i] = relu4(v[i]);
+                sum.x += v[i].x; sum.y += v[i].y; sum.z += v[i].z; sum.w += v[i].w;
+                v[i] = ahead[i];
+            }
+        }
+        sCol[L] = sum;
+        cluster_sync();
+        const uint32_t own = smem_u32(sCol) + L * 16;
+        for (int k = 0; k < rank; ++k) {
+            const float4 u = cluster_load4(cluster_map(own, k));
+            run[0] += u.x; run[1] += u.y; run[2] += u.z; run[3] += u.w;
+        }
+        cluster_sync();      // no CTA leaves while another still reads its sums
+    }
+
+    if (rank == 0)
+        for (int i = threadIdx.x; i < pitch; i += blockDim.x) dst[i] = 0.0f;      // the zero row on top
+    // Where this lane's columns c+1 .. c+4 go in a row.  Some lanes of the first and last warps also write one
+    // word of the constant zeros at the left, or of the copies of the last value behind the last warp's columns.
+    const int p123 = L + 1;
+    const bool in123 = p123 < cells, in0 = p123 + 1 < cells;
+    float *row = dst + (int64_t)(r0 + 1) * pitch;
+    float *d1 = row + cells + p123, *d2 = d1 + cells, *d3 = d2 + cells, *d0 = row + p123 + 1;
+    int extra_at = -1;
+    if (warp == 0 && lane < 5) extra_at = lane < 4 ? lane * cells : 1;
+    const bool zero = extra_at >= 0;
+    if (warp == nwarps - 1 && lane >= 8 && lane < 20) {
+        const int cell = 32 * nwarps + 1 + ((lane - 8) >> 2), sub = lane & 3;
+        if (cell < cells && (sub || cell > 32 * nwarps + 1)) extra_at = sub * cells + cell;
+    }
+    float *extra = row + extra_at;
+    const bool edge_warp = warp == 0 || warp == nwarps - 1;
+
+    int buf = 0;
+    for (int r = r0; r < r1; r += kScanRows) {
+        float4 v[kScanRows];
+        float carry[kScanRows];
+#pragma unroll
+        for (int i = 0; i < kScanRows; ++i) {
+            v[i] = RELU ? relu4(nxt[i]) : nxt[i];
+            const int rn = r + kScanRows + i;
+            nxt[i] = load_quad<IO, VEC>(src + (int64_t)rn * w, c, w, rn < r1);
+        }
+#pragma unroll
+        for (int i = 0; i < kScanRows; ++i) {
+            run[0] += v[i].x; run[1] += v[i].y; run[2] += v[i].z; run[3] += v[i].w;
+            v[i].x = run[0];
+            v[i].y = run[1] + v[i].x;
+            v[i].z = run[2] + v[i].y;
+            v[i].w = run[3] + v[i].z;
+            const float incl = warp_scan(v[i].w);
+            carry[i] = incl - v[i].w;
+            if (lane == 31) sTot[buf][warp][i] = incl;
+        }
+        if (nwarps > 1) {
+            __syncthreads();
+            for (int k = 0; k < warp; ++k) {
+#pragma unroll
+                for (int i = 0; i < kScanRows; i += 4) {
+                    const float4 a = *reinterpret_cast<const float4 *>(&sTot[buf][k][i]);
+                    carry[i] += a.x; carry[i + 1] += a.y; carry[i + 2] += a.z; carry[i + 3] += a.w;
+                }
+            }
+            buf ^= 1;
+        }
+#pragma unroll
+        for (int i = 0; i < kScanRows; ++i) {
+            if (r + i < r1) {
+                const float x4 = v[i].w + carry[i];
+                if (in123) {
+                    *d1 = v[i].x + carry[i];
+                    *d2 = v[i].y + carry[i];
+                    *d3 = v[i].z + carry[i];
+                }
+                if (in0) *d0 = x4;
+                if (edge_warp) {
+                    const float last = __shfl_sync(0xffffffffu, x4, 31);
+                    if (extra_at >= 0) *extra = zero ? 0.0f : last;
+                    extra += pitch;
+                }
+                d0 += pitch; d1 += pitch; d2 += pitch; d3 += pitch;
+            }
+        }
+    }
+}
+
+// ---- gathers --------------------------------------------------------------------------------------
+// The two runs of integral rows a slab needs for one filter, clamped to the plane.
+struct SlabRows {
+    int lo_first, lo_count, hi_first, hi_count;
+};
+__device__ __forceinline__ SlabRows slab_rows(const BoxTaps &t, int p0, int rows, int h)
+{
+    SlabRows s;
+    s.lo_first = min(max(p0 + t.lo_r - 1, 0), h);
+    s.lo_count = min(max(p0 + rows - 1 + t.lo_r, 0), h) - s.lo_first + 1;
+    s.hi_first = min(max(p0 + t.hi_r, 0), h);
+    s.hi_count = min(max(p0 + rows + t.hi_r, 0), h) - s.hi_first + 1;
+    return s;
+}
+
+struct SlabShape {
+    int R, slabs, col_tiles, stage_bytes;      // rows per slab, slabs per plane, 128-column tiles, bytes of one side's stage
+};
+
+__device__ __forceinline__ void slab_issue(const float *plane, int pitch, const BoxTaps &t, int p0, int rows, int h, uint32_t lo32,
+                                           uint32_t hi32, uint32_t mbar)
+{
+    const SlabRows s = slab_rows(t, p0, rows, h);
+    const uint32_t row_bytes = (uint32_t)pitch * 4u;
+    bulk_load(lo32, plane + (int64_t)s.lo_first * pitch, (uint32_t)s.lo_count * row_bytes, mbar);
+    bulk_load(hi32, plane + (int64_t)s.hi_first * pitch, (uint32_t)s.hi_count * row_bytes, mbar);
+}
+
+// FUSED: the inference steps of `Fusion` (the output may then alias the residual).
+template <typename IO, bool VEC, bool FUSED, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 6 : 1)
+forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int C, int F, int h, int w, SlabShape sh, int fsplit,
+                    bool normalize, bool exact, Fusion fu)
+{
+    extern __shared__ __align__(128) unsigned char slab_stage[];
+    __shared__ __align__(8) unsigned long long mbar;
+    grid_dependency_release();
+    const int lane = threadIdx.x & 31, warp = uniform(threadIdx.x >> 5);
+    // (32-bit: a 64-bit division would take what follows out of the uniform registers)
+    const int part = blockIdx.x % fsplit, b = blockIdx.x / fsplit;
+    const int slab = b % sh.slabs, plane_at = b / sh.slabs, c = plane_at % C;
+    const int64_t nc = plane_at;
+    const int f_begin = (F * part) / fsplit, f_end = (F * (part + 1)) / fsplit, nf = f_end - f_begin;
+    const int cells = quad_cells(w), pitch = 4 * cells, row_bytes = pitch * 4;
+    const int p_slab = slab * sh.R, rows = min(sh.R, h - p_slab);
+    const uint32_t stage32 = smem_u32(slab_stage), mbar32 = smem_u32(&mbar);
+    float *sTaps = reinterpret_cast<float *>(slab_stage + 2 * sh.stage_bytes);      // behind the stages: the boxes
+    const float *plane = integ + nc * (int64_t)(h + 1) * pitch;
+
+    if (threadIdx.x == 0) {
+        mbar_init(mbar32, 2);
+        fence_mbar_init();
+    }
+    grid_dependency_wait();
+    if ((int)threadIdx.x < nf) {
+        const Box box = load_box(bp, c * F + f_begin + threadIdx.x);
+        store_taps(sTaps + threadIdx.x * kTapWords, taps_forward(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        fence_proxy_async();
+        slab_issue(plane, pitch, load_taps(sTaps), p_slab, rows, h, stage32, stage32 + sh.stage_bytes, mbar32);
+    }
+
+    const int rg = warp / sh.col_tiles, ct = warp - rg * sh.col_tiles;
+    const int q0 = ct * 128 + lane * kStrip, p0 = p_slab + rg * kStripRows;
+    const int mine = min(kStripRows, p_slab + rows - p0);      // rows of this warp (may be <= 0)
+    const bool in_plane = q0 < w;      // (lanes past the plane gather too, from clamped columns, and store nothing)
+    bool timed_out = false;
+    for (int k = 0; k < nf; ++k) {
+        const int f = f_begin + k;
+        timed_out |= !mbar_wait(mbar32, k & 1);
+        const BoxTaps t = load_taps_uniform(sTaps + k * kTapWords);
+        if (mine > 0) {
+            const SlabRows s = slab_rows(t, p_slab, rows, h);
+            const uint32_t lo32 = stage32 - s.lo_first * row_bytes;
+            const uint32_t hi32 = stage32 + sh.stage_bytes - s.hi_first * row_bytes;
+            const QuadCols cols = quad_cols(t, q0 >> 2, cells);
+            const ColW2 cw = col_weights(t);
+            const float sfl = t.scale * t.f_lo_r, sfh = t.scale * t.f_hi_r;
+            const QuadRows<kStripRows> q = quad_rows<kStripRows>(t, p0, h, lo32, hi32, row_bytes, lane);
+            float mul = 1.0f, add = 0.0f;
+            if (FUSED) {
+                if (fu.scale) mul = __ldg(fu.scale + c * F + f);
+                if (fu.shift) add = __ldg(fu.shift + c * F + f);
+            }
+            int64_t off = (nc * F + f) * (int64_t)h * w + (int64_t)p0 * w + q0;
+            f2_t prev[kStrip];
+            quad_pair(cols, q.lo[0], q.hi[0], cw, prev);
+#pragma unroll
+            for (int i = 0; i < kStripRows; ++i) {
+                if (i < mine) {
+                    f2_t cur[kStrip];
+                    quad_pair(cols, q.lo[i + 1], q.hi[i + 1], cw, cur);
+                    float v[kStrip];
+                    quad_forward_row(prev, cur, t.scale, sfl, sfh, v);
+#pragma unroll
+                    for (int m = 0; m < kStrip; ++m) prev[m] = cur[m];
+                    if (FUSED) {
+#pragma unroll
+                        for (int m = 0; m < kStrip; ++m) {
+                            v[m] = v[m] * mul + add;
+                            if (fu.residual && q0 + m < w) v[m] += fu.residual[off + m];      // plain loads: may alias `out`
+                            if (fu.output_relu) v[m] = fmaxf(v[m], 0.0f);
+                        }
+                    }
+                    if (VEC) {
+                        if (in_plane) Io<IO>::store4(out + off, v[0], v[1], v[2], v[3]);
+                    } else {
+#pragma unroll
+                        for (int m = 0; m < kStrip; ++m)
+                            if (q0 + m < w) Io<IO>::store1(out + off + m, v[m]);
+                    }
+                    off += w;
+                }
+            }
+        }
+        __syncthreads();      // the stage has been read
+        if (threadIdx.x == 0 && k + 1 < nf) {
+            fence_proxy_async();
+            slab_issue(plane, pitch, load_taps(sTaps + (k + 1) * kTapWords), p_slab, rows, h, stage32, stage32 + sh.stage_bytes, mbar32);
+        }
+    }
+    if (timed_out && lane == 0) atomicAdd(&g_wait_timeouts, 1);
+}
+
+// Per slab: the four input values and the grad-input accumulators of a lane's rows stay in registers over the
+// filters; the five sums are reduced per warp and filter, and per CTA at the end.
+template <typename IO, bool VEC, bool NEED_PARAMS, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1)
+backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ go_integ, BoxParams bp, IO *__restrict__ grad_input,
+                     float *__restrict__ partials, int N, int C, int F, int h, int w, SlabShape sh, bool normalize, bool exact,
+                     bool write_gin)
+{
+    extern __shared__ __align__(128) unsigned char slab_stage[];
+    __shared__ __align__(8) unsigned long long mbar;
+    grid_dependency_release();
+    const int lane = threadIdx.x & 31, warp = uniform(threadIdx.x >> 5), nwarps = blockDim.x >> 5;
+    const int slab = blockIdx.x % sh.slabs;
+    const int64_t nc = blockIdx.x / sh.slabs;
+    const int c = (int)(nc % C), n = (int)(nc / C);
+    const int cells = quad_cells(w), pitch = 4 * cells, row_bytes = pitch * 4;
+    const int p_slab = slab * sh.R, rows = min(sh.R, h - p_slab);
+    const uint32_t stage32 = smem_u32(slab_stage), mbar32 = smem_u32(&mbar);
+    float *sTaps = reinterpret_cast<float *>(slab_stage + 2 * sh.stage_bytes);      // behind the stages: the boxes, then
+    float *red = sTaps + F * kTapWords;                                             // [F][warps][5] sums
+    const int64_t ipl = (int64_t)(h + 1) * pitch;
+    const float *planes = go_integ + nc * F * ipl;
+
+    if (threadIdx.x == 0) {
+        mbar_init(mbar32, 2);
+        fence_mbar_init();
+    }
+    grid_dependency_wait();
+    if ((int)threadIdx.x < F) {
+        const Box box = load_box(bp, c * F + threadIdx.x);
+        store_taps(sTaps + threadIdx.x * kTapWords, taps_mirrored(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        fence_proxy_async();
+        slab_issue(planes, pitch, load_taps(sTaps), p_slab, rows, h, stage32, stage32 + sh.stage_bytes, mbar32);
+    }
+
+    const int rg = warp / sh.col_tiles, ct = warp - rg * sh.col_tiles;
+    const int q0 = ct * 128 + lane * kStrip, p0 = p_slab + rg * kStripRows;
+    const int mine = min(kStripRows, p_slab + rows - p0);
+    const bool active = q0 < w && mine > 0;      // (lanes past the plane gather too, from clamped columns, with x = 0)
+    const int64_t pix = nc * (int64_t)h * w + (int64_t)p0 * w + q0;
+    float xv[kStripRows][kStrip], gin[kStripRows][kStrip];
+#pragma unroll
+    for (int i = 0; i < kStripRows; ++i) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (NEED_PARAMS) v = load_quad<IO, VEC>(x + pix - q0 + (int64_t)i * w, q0, w, i < mine);
+        xv[i][0] = v.x; xv[i][1] = v.y; xv[i][2] = v.z; xv[i][3] = v.w;
+#pragma unroll
+        for (int m = 0; m < kStrip; ++m) gin[i][m] = 0.0f;
+    }
+    bool timed_out = false;
+    for (int f = 0; f < F; ++f) {
+        timed_out |= !mbar_wait(mbar32, f & 1);
+        float sums[kNumSums] = {0.f, 0.f, 0.f, 0.f, 0.f};
+        const BoxTaps t = load_taps_uniform(sTaps + f * kTapWords);
+        if (mine > 0) {
+            const SlabRows s = slab_rows(t, p_slab, rows, h);
+            const uint32_t lo32 = stage32 - s.lo_first * row_bytes;
+            const uint32_t hi32 = stage32 + sh.stage_bytes - s.hi_first * row_bytes;
+            quad_backward_strip<kStripRows, NEED_PARAMS>(
+                t, quad_cols(t, q0 >> 2, cells), quad_rows<kStripRows>(t, p0, h, lo32, hi32, row_bytes, lane), col_weights(t), xv, gin,
+                sums, mine);
+        }
+        if (NEED_PARAMS) {
+            const float s = warp_sum5(sums, lane);
+            const int slot = sum5_slot(lane);
+            if (slot >= 0) red[(f * nwarps + warp) * kNumSums + slot] = s;
+        }
+        __syncthreads();      // the stage has been read
+        if (threadIdx.x == 0 && f + 1 < F) {
+            fence_proxy_async();
+            slab_issue(planes + (f + 1) * ipl, pitch, load_taps(sTaps + (f + 1) * kTapWords), p_slab, rows, h, stage32,
+                       stage32 + sh.stage_bytes, mbar32);
+        }
+    }
+    if (timed_out && lane == 0) atomicAdd(&g_wait_timeouts, 1);
+
+    if (NEED_PARAMS) {
+        for (int i = threadIdx.x; i < F * kNumSums; i += blockDim.x) {
+            const int f = i / kNumSums, j = i - f * kNumSums;
+            float s = 0.0f;
+            for (int k = 0; k < nwarps; ++k) s += red[(f * nwarps + k) * kNumSums + j];
+            partials[(((int64_t)(c * F + f) * N + n) * sh.slabs + slab) * kNumSums + j] = s;
+        }
+    }
+    if (write_gin && active) {
+        IO *dst = grad_input + pix;
+#pragma unroll
+        for (int i = 0; i < kStripRows; ++i) {
+            if (i < mine) {
+                if (VEC) {
+                    Io<IO>::store4(dst, gin[i][0], gin[i][1], gin[i][2], gin[i][3]);
+                } else {
+#pragma unroll
+                    for (int m = 0; m < kStrip; ++m)
+                        if (q0 + m < w) Io<IO>::store1(dst + m, gin[i][m]);
+                }
+                dst += w;
+            }
+        }
+    }
+}
+
+inline SlabShape slab_shape(int h, int w)
+{
+    SlabShape s;
+    s.col_tiles = (w + 127) / 128;
+    const int groups = 4 / s.col_tiles > 1 ? 4 / s.col_tiles : 1;      // about four warps a CTA
+    s.R = groups * kStripRows;
+    s.slabs = (h + s.R - 1) / s.R;
+    s.stage_bytes = ((s.R + 1) * quad_pitch(w) * 4 + 127) & ~127;
+    return s;
+}
+inline int slab_threads(const SlabShape &s) { return 32 * s.col_tiles * (s.R / kStripRows); }
+// (the table of boxes and the per-warp sums of up to 32 filters sit behind the stage)
+inline size_t slab_smem(const SlabShape &s, int F, bool sums)
+{
+    return 2 * (size_t)s.stage_bytes + (size_t)F * kTapWords * sizeof(float) +
+           (sums ? (size_t)F * (slab_threads(s) / 32) * kNumSums * sizeof(float) : 0);
+}
+
+template <typename IO>
+int integral_quad_t(const IO *in, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s)
+{
+    const int warps = (w + 127) / 128;
+    // few planes: clusters of up to 8 CTAs share one, as long as each keeps 16 rows
+    int cluster = 1;
+    while (cluster < 8 && planes * cluster < 2 * 148 && h >= 32 * cluster) cluster *= 2;
+    const int rows = ((h + cluster - 1) / cluster + kScanRows - 1) / kScanRows * kScanRows;
+    const bool vec = w % 4 == 0 && aligned_to(in, Io<IO>::kVecBytes);
+    if (planes * cluster > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
+    void (*kern)(const IO *, float *, int, int, int, int);
+    constexpr int S = 128, L = 32 * kSlabMaxWarps;
+    if (warps * 32 <= S) {
+        if (relu) kern = vec ? integral_quad_kernel<IO, true, true, S> : integral_quad_kernel<IO, false, true, S>;
+        else kern = vec ? integral_quad_kernel<IO, true, false, S> : integral_quad_kernel<IO, false, false, S>;
+    } else {
+        if (relu) kern = vec ? integral_quad_kernel<IO, true, true, L> : integral_quad_kernel<IO, false, true, L>;
+        else kern = vec ? integral_quad_kernel<IO, true, false, L> : integral_quad_kernel<IO, false, false, L>;
+    }
+    {
+        LaunchScope scope(KID_INTEGRAL, s);
+        if (cudaError_t e = launch_overlapped_cluster(kern, (unsigned)(planes * cluster), warps * 32,
+                                                      cluster > 1 ? warps * 32 * sizeof(float4) : 0, cluster, s, in, out, h, w, rows,
+                                                      cluster))
+            return cuda_failed(e, "integral_quad");
+    }
+    return check_launch("integral_quad");
+}
+
+template <typename IO>
+int forward_slab_t(const float *integ, const BoxParams &bp, const Fusion *fu, IO *out, int N, int C, int F, int h, int w,
+                   bool normalize, bool exact, cudaStream_t s)
+{
+    const SlabShape sh = slab_shape(h, w);
+    const int64_t base = (int64_t)N * C * sh.slabs;
+    // one CTA a slab takes all its filters in turn; fewer each when there are not enough CTAs for two on every SM
+    int fsplit = 1;
+    while (fsplit < F && base * fsplit < 2 * 148) fsplit = fsplit * 2 < F ? fsplit * 2 : F;
+    if (base * fsplit > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
+    const bool vec = w % 4 == 0 && aligned_to(out, Io<IO>::kVecBytes);
+    void (*kern)(const float *, BoxParams, IO *, int, int, int, int, SlabShape, int, bool, bool, Fusion);
+    constexpr bool FU = IsFloat<IO>::value;
+    constexpr int S = 128, L = 32 * kSlabMaxWarps;
+    if (slab_threads(sh) <= S) {
+        if (fu) kern = vec ? forward_slab_kernel<IO, true, FU, S> : forward_slab_kernel<IO, false, FU, S>;
+        else kern = vec ? forward_slab_kernel<IO, true, false, S> : forward_slab_kernel<IO, false, false, S>;
+    } else {
+        if (fu) kern = vec ? forward_slab_kernel<IO, true, FU, L> : forward_slab_kernel<IO, false, FU, L>;
+        else kern = vec ? forward_slab_kernel<IO, true, false, L> : forward_slab_kernel<IO, false, false, L>;
+    }
+    int st = raise_smem_limit(reinterpret_cast<const void *>(kern), (int)kSlabMaxSmem);
+    if (st != BC_OK) return st;
+    const Fusion none{0, nullptr, nullptr, nullptr, 0};
+    {
+        LaunchScope scope(KID_FORWARD_SLAB, s);
+        if (cudaError_t e = launch_overlapped(kern, (unsigned)(base * fsplit), slab_threads(sh), slab_smem(sh, (F + fsplit - 1) / fsplit, false), s, integ, bp, out, C,
+                                              F, h, w, sh, fsplit, normalize, exact, fu ? *fu : none))
+            return cuda_failed(e, "forward_slab");
+    }
+    return check_launch("forward_slab");
+}
+
+template <typename IO>
+int backward_slab_t(const IO *x, const float *go_integ, const BoxParams &bp, float rep_h, float rep_w, int N, int C, int F, int h,
+                    int w, bool normalize, bool exact, int need_mask, IO *grad_input, void *grad_params, int grad_params_kind,
+                    float *partials, cudaStream_t s)
+{
+    const SlabShape sh = slab_shape(h, w);
+    const int64_t blocks = (int64_t)N * C * sh.slabs;
+    if (blocks > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
+    const bool need_params = (need_mask & (BC_NEED_ALL & ~BC_NEED_INPUT)) != 0;
+    const bool write_gin = (need_mask & BC_NEED_INPUT) != 0;
+    const bool vec = w % 4 == 0 && aligned_to(x, Io<IO>::kVecBytes) && (!write_gin || aligned_to(grad_input, Io<IO>::kVecBytes));
+    void (*kern)(const IO *, const float *, BoxParams, IO *, float *, int, int, int, int, int, SlabShape, bool, bool, bool);
+    constexpr int S = 128, L = 32 * kSlabMaxWarps;
+    if (slab_threads(sh) <= S) {
+        if (need_params) kern = vec ? backward_slab_kernel<IO, true, true, S> : backward_slab_kernel<IO, false, true, S>;
+        else kern = vec ? backward_slab_kernel<IO, true, false, S> : backward_slab_kernel<IO, false, false, S>;
+    } else {
+        if (need_params) kern = vec ? backward_slab_kernel<IO, true, true, L> : backward_slab_kernel<IO, false, true, L>;
+        else kern = vec ? backward_slab_kernel<IO, true, false, L> : backward_slab_kernel<IO, false, false, L>;
+    }
+    int st = raise_smem_limit(reinterpret_cast<const void *>(kern), (int)kSlabMaxSmem);
+    if (st != BC_OK) return st;
+    {
+        LaunchScope scope(KID_BACKWARD_SLAB, s);
+        if (cudaError_t e = launch_overlapped(kern, (unsigned)blocks, slab_threads(sh), slab_smem(sh, F, need_params), s, x, go_integ, bp, grad_input,
+                                              partials, N, C, F, h, w, sh, normalize, exact, write_gin))
+            return cuda_failed(e, "backward_slab");
+    }
+    st = check_launch("backward_slab");
+    if (st != BC_OK || !need_params) return st;
+    return launch_finish_param_grads<float>(partials, bp, C * F, N * sh.slabs, normalize, exact, rep_h, rep_w, need_mask,
+                                            grad_params, s, grad_params_kind);
+}
+
+}  // namespace
+
+bool slab_path_fits(int F, int h, int w)
+{
+    return h >= 1 && w >= 1 && F <= kMaxFilters && (w + 127) / 128 <= kSlabMaxWarps && slab_smem(slab_shape(h, w), F, true) <= kSlabMaxSmem;
+}
+size_t slab_integral_floats(int64_t planes, int h, int w) { return (size_t)planes * (size_t)(h + 1) * (size_t)quad_pitch(w); }
+size_t slab_partials_bytes(int N, int C, int F, int h, int w)
+{
+    return (size_t)C * F * N * slab_shape(h, w).slabs * kNumSums * sizeof(float);
+}
+
+int launch_integral_quad(const void *in, int io_kind, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s)
+{
+    if (planes == 0) return BC_OK;
+    if (io_kind == BC_IO_F16) return integral_quad_t(static_cast<const __half *>(in), out, planes, h, w, relu, s);
+    if (io_kind == BC_IO_BF16) return integral_quad_t(static_cast<const __nv_bfloat16 *>(in), out, planes, h, w, relu, s);
+    return integral_quad_t(static_cast<const float *>(in), out, planes, h, w, relu, s);
+}
+
+int launch_forward_slab(const float *integ, const BoxParams &bp, const Fusion *fu, void *out, int io_kind, int N, int C, int F,
+                        int h, int w, bool normalize, bool exact, cudaStream_t s)
+{
+    if (io_kind == BC_IO_F16) return forward_slab_t(integ, bp, nullptr, static_cast<__half *>(out), N, C, F, h, w, normalize, exact, s);
+    if (io_kind == BC_IO_BF16)
+        return forward_slab_t(integ, bp, nullptr, static_cast<__nv_bfloat16 *>(out), N, C, F, h, w, normalize, exact, s);
+    return forward_slab_t(integ, bp, fu, static_cast<float *>(out), N, C, F, h, w, normalize, exact, s);
+}
+
+int launch_backward_slab(const void *x, int io_kind, const float *go_integ, const BoxParams &bp, float rep_h, float rep_w, int N,
+                         int C, int F, int h, int w, bool normalize, bool exact, int need_mask, void *grad_input, void *grad_params,
+                         int grad_params_kind, float *partials, cudaStream_t s)
+{
+    if (io_kind == BC_IO_F16)
+        return backward_slab_t(static_cast<const __half *>(x), go_integ, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask,
+                               static_cast<__half *>(grad_input), grad_params, grad_params_kind, partials, s);
+    if (io_kind == BC_IO_BF16)
+        return backward_slab_t(static_cast<const __nv_bfloat16 *>(x), go_integ, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact,
+                               need_mask, static_cast<__nv_bfloat16 *>(grad_input), grad_params, grad_params_kind, partials, s);
+    return backward_slab_t(static_cast<const float *>(x), go_integ, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask,
+                           static_cast<float *>(grad_input), grad_params, grad_params_kind, partials, s);
+}
+
+int read_wait_timeouts_slab(int *count) { return read_wait_timeouts_here(count); }
+
+}  // namespace bc

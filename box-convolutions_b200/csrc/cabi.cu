@@ -322,17 +322,24 @@ size_t bc_boxconv2d_forward_workspace(int N, int C, int F, int h, int w)
 {
     if (!sizes_ok(N, C, F, h, w) || any_empty(N, C, F, h, w)) return 0;
     if (plane_path_fits_forward(F, h, w)) return 0;
+    if (slab_path_fits(F, h, w)) return align_up(slab_integral_floats((int64_t)N * C, h, w) * sizeof(float), 256);
     if (band_path_fits_forward(h, w)) return align_up(band_integral_floats((int64_t)N * C, h, w) * sizeof(float), 256);
     return integral_bytes((int64_t)N * C, h, w);
 }
 
-// Forward of planes that do not fit in shared memory: integral images to the workspace (padded rows
-// for the column-band kernel where a band fits, plain rows for the general kernel otherwise).
+// Forward of planes that do not fit in shared memory: integral images to the workspace, in the row layout
+// of the kernel that gathers from them: slabs up to 2048 columns (32 filters), column bands for wider planes of
+// few rows, the general kernel for the rest.
 static int forward_from_workspace(const float *input, const BoxParams &bp, const Fusion *fu, float *output, int N,
                                   int C, int F, int h, int w, bool normalize, bool exact, float *integ,
                                   cudaStream_t stream)
 {
     const bool relu_in = fu && fu->input_relu;
+    if (slab_path_fits(F, h, w)) {
+        int st = launch_integral_quad(input, BC_IO_F32, integ, (int64_t)N * C, h, w, relu_in, stream);
+        if (st != BC_OK) return st;
+        return launch_forward_slab(integ, bp, fu, output, BC_IO_F32, N, C, F, h, w, normalize, exact, stream);
+    }
     if (band_path_fits_forward(h, w)) {
         int st = launch_integral_image_f32(input, integ, (int64_t)N * C, h, w, relu_in, stream, band_lpad(), band_rpad(w));
         if (st != BC_OK) return st;
@@ -389,10 +396,27 @@ size_t bc_boxconv2d_backward_workspace(int N, int C, int F, int h, int w, int ne
     if (!sizes_ok(N, C, F, h, w) || any_empty(N, C, F, h, w) || !(need_mask & BC_NEED_ALL)) return 0;
     if (plane_path_fits_backward(F, h, w))
         return align_up((size_t)C * F * N * kNumSums * sizeof(float), 256);
+    if (slab_path_fits(F, h, w))
+        return align_up(slab_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256) +
+               align_up(slab_partials_bytes(N, C, F, h, w), 256);
     if (band_path_fits_backward(F, h, w))
         return align_up(band_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256) +
                align_up(band_partials_bytes(N, C, F, w), 256);
     return integral_bytes((int64_t)N * C * F, h, w) + align_up(backward_partials_bytes(N, C, F, h, w), 256);
+}
+
+// Backward of planes that do not fit in shared memory, by slabs (workspace already checked).
+static int backward_slabs(const void *input, int io_kind, const void *grad_output, const BoxParams &bp, float rep_h, float rep_w,
+                          int N, int C, int F, int h, int w, bool normalize, bool exact, int need_mask, void *grad_input,
+                          void *grad_params, int grad_params_kind, void *workspace, cudaStream_t stream)
+{
+    float *go_integ = static_cast<float *>(workspace);
+    float *partials = reinterpret_cast<float *>(static_cast<char *>(workspace) +
+                                                align_up(slab_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256));
+    int st = launch_integral_quad(grad_output, io_kind, go_integ, (int64_t)N * C * F, h, w, false, stream);
+    if (st != BC_OK) return st;
+    return launch_backward_slab(input, io_kind, go_integ, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
+                                grad_params, grad_params_kind, partials, stream);
 }
 
 int bc_boxconv2d_backward(const float *input, const float *x_min, const float *x_max,
@@ -430,6 +454,9 @@ int bc_boxconv2d_backward(const float *input, const float *x_min, const float *x
         return launch_backward_plane(input, grad_output, bp, reparametrization_h, reparametrization_w, N, C,
                                      F, h, w, normalize != 0, exact != 0, need_mask, grad_input,
                                      grad_params, static_cast<float *>(workspace), stream);
+    if (slab_path_fits(F, h, w))
+        return backward_slabs(input, BC_IO_F32, grad_output, bp, reparametrization_h, reparametrization_w, N, C, F, h, w,
+                              normalize != 0, exact != 0, need_mask, grad_input, grad_params, BC_IO_F32, workspace, stream);
     float *go_integ = static_cast<float *>(workspace);
     float *partials = reinterpret_cast<float *>(static_cast<char *>(workspace) + ib);
     if (band) {
@@ -466,6 +493,46 @@ int bc_boxconv2d_forward_narrow(const void *input, int io_kind, const float *x_m
     return launch_forward_plane_narrow(input, io_kind, bp, output, N, C, F, h, w, normalize != 0, exact != 0, stream);
 }
 
+int bc_boxconv2d_narrow_all_supported(int F, int h, int w)
+{
+    return (F > 0 && h > 0 && w > 0 && (bc_boxconv2d_narrow_supported(F, h, w) || slab_path_fits(F, h, w))) ? 1 : 0;
+}
+
+// Planes that one of the two plane kernels does not hold go through slabs in both directions.
+size_t bc_boxconv2d_narrow_workspace(int N, int C, int F, int h, int w, int need_mask)
+{
+    if (!sizes_ok(N, C, F, h, w) || any_empty(N, C, F, h, w)) return 0;
+    const bool plane = bc_boxconv2d_narrow_supported(F, h, w) != 0;
+    if (!(need_mask & BC_NEED_ALL))
+        return plane ? 0 : align_up(slab_integral_floats((int64_t)N * C, h, w) * sizeof(float), 256);
+    if (plane) return bc_boxconv2d_backward_workspace(N, C, F, h, w, need_mask);
+    return align_up(slab_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256) +
+           align_up(slab_partials_bytes(N, C, F, h, w), 256);
+}
+
+int bc_boxconv2d_forward_narrow_all(const void *input, int io_kind, const float *x_min, const float *x_max,
+                                    const float *y_min, const float *y_max, float reparametrization_h,
+                                    float reparametrization_w, void *output, int N, int C, int F, int h,
+                                    int w, int normalize, int exact, void *workspace, size_t workspace_bytes,
+                                    bc_stream_t stream)
+{
+    if (!sizes_ok(N, C, F, h, w)) return BC_ERR_BAD_SHAPE;
+    if (any_empty(N, C, F, h, w) || bc_boxconv2d_narrow_supported(F, h, w))
+        return bc_boxconv2d_forward_narrow(input, io_kind, x_min, x_max, y_min, y_max, reparametrization_h,
+                                           reparametrization_w, output, N, C, F, h, w, normalize, exact, stream);
+    if (io_kind != BC_IO_F16 && io_kind != BC_IO_BF16) return BC_ERR_UNSUPPORTED;
+    if (!input || !x_min || !x_max || !y_min || !y_max || !output) return BC_ERR_NULL_POINTER;
+    if (!slab_path_fits(F, h, w)) return BC_ERR_UNSUPPORTED;
+    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) ||
+        workspace_bytes < bc_boxconv2d_narrow_workspace(N, C, F, h, w, 0))
+        return BC_ERR_WORKSPACE;
+    const BoxParams bp{x_min, x_max, y_min, y_max, reparametrization_h, reparametrization_w};
+    float *integ = static_cast<float *>(workspace);
+    int st = launch_integral_quad(input, io_kind, integ, (int64_t)N * C, h, w, false, stream);
+    if (st != BC_OK) return st;
+    return launch_forward_slab(integ, bp, nullptr, output, io_kind, N, C, F, h, w, normalize != 0, exact != 0, stream);
+}
+
 // grad_params_kind: how the parameter gradients are stored (BC_IO_*)
 static int backward_narrow(const void *input, int io_kind, const float *x_min, const float *x_max,
                            const float *y_min, const float *y_max, const void *grad_output,
@@ -494,11 +561,15 @@ static int backward_narrow(const void *input, int io_kind, const float *x_min, c
     if (!input || !x_min || !x_max || !y_min || !y_max || !grad_output) return BC_ERR_NULL_POINTER;
     if ((need_mask & BC_NEED_INPUT) && !grad_input) return BC_ERR_NULL_POINTER;
     if (need_params && !grad_params) return BC_ERR_NULL_POINTER;
-    if (!plane_path_fits_backward(F, h, w)) return BC_ERR_UNSUPPORTED;
+    const bool plane = bc_boxconv2d_narrow_supported(F, h, w) != 0;
+    if (!plane && !slab_path_fits(F, h, w)) return BC_ERR_UNSUPPORTED;
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) ||
-        workspace_bytes < bc_boxconv2d_backward_workspace(N, C, F, h, w, need_mask))
+        workspace_bytes < bc_boxconv2d_narrow_workspace(N, C, F, h, w, need_mask))
         return BC_ERR_WORKSPACE;
     const BoxParams bp{x_min, x_max, y_min, y_max, reparametrization_h, reparametrization_w};
+    if (!plane)
+        return backward_slabs(input, io_kind, grad_output, bp, reparametrization_h, reparametrization_w, N, C, F, h, w,
+                              normalize != 0, exact != 0, need_mask, grad_input, grad_params, grad_params_kind, workspace, stream);
     return launch_backward_plane_narrow(input, grad_output, io_kind, bp, reparametrization_h, reparametrization_w, N, C,
                                         F, h, w, normalize != 0, exact != 0, need_mask, grad_input, grad_params,
                                         grad_params_kind, static_cast<float *>(workspace), stream);
@@ -644,6 +715,8 @@ const char *bc_kernel_name(int kernel_id)
         case KID_BACKWARD_BAND: return "backward_band_kernel";
         case KID_INTEGRAL_BANDS: return "integral_band_fixup_kernels";
         case KID_FORWARD_BAND: return "forward_band_kernel";
+        case KID_FORWARD_SLAB: return "forward_slab_kernel";
+        case KID_BACKWARD_SLAB: return "backward_slab_kernel";
         default: return "unknown";
     }
 }

@@ -70,6 +70,18 @@ Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType dtype, const Tensor &lik
     return Tensor(at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt));
 }
 
+// Slice `i` of a dense tensor's first dimension as a tensor over the same storage, without the dispatcher and
+// view bookkeeping of select() (a microsecond each, four times a backward pass).
+Tensor slice_of(const Tensor &packed, int64_t i)
+{
+    Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(packed.storage()), packed.key_set(), packed.dtype());
+    c10::TensorImpl *impl = t.unsafeGetTensorImpl();
+    const auto sizes = packed.sizes().slice(1);
+    impl->set_storage_offset(packed.storage_offset() + i * c10::multiply_integers(sizes));
+    impl->set_sizes_contiguous(sizes);
+    return t;
+}
+
 // (the caching allocator hands out blocks aligned to 512 bytes)
 Tensor new_workspace(size_t bytes, const Tensor &like)
 {
@@ -142,16 +154,18 @@ ParamPtrs of_packed(const Tensor &packed)
 Tensor run_forward(const Tensor &x, const ParamPtrs &q, const Sizes &s, const Options &o, bc_stream_t stream)
 {
     Tensor out = new_tensor({s.N, (int64_t)s.C * s.F, s.h, s.w}, x.scalar_type(), x);
-    if (is_narrow(x.scalar_type())) {
-        check_status(bc_boxconv2d_forward_narrow(x.const_data_ptr(), io_kind(x.scalar_type()), q.p[0], q.p[1], q.p[2], q.p[3],
-                                                 (float)o.rep_h, (float)o.rep_w, out.data_ptr(), s.N, s.C, s.F, s.h, s.w,
-                                                 o.normalize, o.exact, stream),
+    const bool narrow = is_narrow(x.scalar_type());
+    Tensor ws;
+    const size_t bytes = narrow ? bc_boxconv2d_narrow_workspace(s.N, s.C, s.F, s.h, s.w, 0)
+                                : bc_boxconv2d_forward_workspace(s.N, s.C, s.F, s.h, s.w);
+    if (bytes) ws = new_workspace(bytes, x);
+    if (narrow) {
+        check_status(bc_boxconv2d_forward_narrow_all(x.const_data_ptr(), io_kind(x.scalar_type()), q.p[0], q.p[1], q.p[2], q.p[3],
+                                                     (float)o.rep_h, (float)o.rep_w, out.data_ptr(), s.N, s.C, s.F, s.h, s.w,
+                                                     o.normalize, o.exact, bytes ? ws.data_ptr() : nullptr, bytes, stream),
                      "BoxConv2d forward");
         return out;
     }
-    Tensor ws;
-    const size_t bytes = bc_boxconv2d_forward_workspace(s.N, s.C, s.F, s.h, s.w);
-    if (bytes) ws = new_workspace(bytes, x);
     check_status(bc_boxconv2d_forward(x.const_data_ptr<float>(), q.p[0], q.p[1], q.p[2], q.p[3], (float)o.rep_h, (float)o.rep_w,
                                       out.data_ptr<float>(), s.N, s.C, s.F, s.h, s.w, o.normalize, o.exact,
                                       bytes ? ws.data_ptr() : nullptr, bytes, stream),
@@ -291,7 +305,7 @@ Gradients box_backward(const Tensor &integrated, Four p, const Tensor &grad_outp
                      : backward_call<float>(I, p, g, rep_h, rep_w, s, normalize, exact, mask, gin, gp, ws.data_ptr(), bytes, stream),
                  "box_convolution_backward");
     for (int i = 0; i < 4; ++i)
-        if (mask & (BC_NEED_X_MIN << i)) out[1 + i] = gparams.select(0, i);
+        if (mask & (BC_NEED_X_MIN << i)) out[1 + i] = slice_of(gparams, i);
     return out;
 }
 
@@ -356,8 +370,8 @@ Tensor clip(const Four &p, double rep_h, double rep_w, double max_h, double max_
 // integral image or the output: the fused entry points work from the input itself, so only the input and
 // one packed copy of the parameters live until backward.  The copy matters because the module changes its
 // parameters in place (clipping) between a forward and the backward that belongs to it.
-// float64 (gradient checks) chains the four functions, as the reference does.  16-bit tensors of planes
-// that the shared-memory kernels do not hold go through float32 copies.
+// float64 (gradient checks) chains the four functions, as the reference does.  16-bit tensors
+// outside what the 16-bit entry points serve (very wide planes, many filters) go through float32 copies.
 
 struct Saved : torch::CustomClassHolder {
     double rep_h, rep_w;
@@ -386,7 +400,7 @@ Tensor forward_any(const Tensor &input, const Four &p, const Options &o, Kept *k
                            o.normalize, o.exact);
     }
     const bool narrow = is_narrow(dtype);
-    if (narrow && !bc_boxconv2d_narrow_supported(s.F, s.h, s.w)) x = x.to(at::kFloat);
+    if (narrow && s.h && s.w && s.F && !bc_boxconv2d_narrow_all_supported(s.F, s.h, s.w)) x = x.to(at::kFloat);
     const bc_stream_t stream = current_stream(x);
     Tensor packed = o.snapshot;
     if (packed.defined() && !(packed.scalar_type() == at::kFloat && packed.device() == x.device() && packed.is_contiguous() &&
@@ -427,7 +441,8 @@ Gradients backward_any(const Tensor &x, const Tensor &params, Tensor grad_output
     Tensor gparams;
     if (mask & BC_NEED_INPUT) out[0] = new_tensor(x.sizes(), dtype, x);
     if (mask & ~BC_NEED_INPUT) gparams = new_tensor({4, s.C, s.F}, dtype, x);
-    const size_t bytes = bc_boxconv2d_backward_workspace(s.N, s.C, s.F, s.h, s.w, mask);
+    const size_t bytes = is_narrow(dtype) ? bc_boxconv2d_narrow_workspace(s.N, s.C, s.F, s.h, s.w, mask)
+                                          : bc_boxconv2d_backward_workspace(s.N, s.C, s.F, s.h, s.w, mask);
     Tensor ws = new_workspace(bytes, x);
     const ParamPtrs q = of_packed(params);
     void *gin = out[0].defined() ? out[0].data_ptr() : nullptr, *gp = gparams.defined() ? gparams.data_ptr() : nullptr;
@@ -447,7 +462,7 @@ Gradients backward_any(const Tensor &x, const Tensor &params, Tensor grad_output
         if (gparams.defined()) gparams = gparams.to(a.dtype);
     }
     for (int i = 0; i < 4; ++i)
-        if (mask & (BC_NEED_X_MIN << i)) out[1 + i] = gparams.select(0, i);
+        if (mask & (BC_NEED_X_MIN << i)) out[1 + i] = slice_of(gparams, i);
     return out;
 }
 
@@ -474,7 +489,11 @@ struct BoxConvolution : torch::autograd::Function<BoxConvolution> {
         for (int i = 0; i < 5; ++i)
             if (ctx->needs_input_grad(i)) mask |= 1 << i;
         Gradients g = backward_any(saved[0], saved[1], grads[0], *static_cast<const Saved *>(target.get()), mask);
-        return {g[0], g[1], g[2], g[3], g[4], Tensor()};
+        torch::autograd::variable_list list;
+        list.reserve(6);
+        for (Tensor &t : g) list.push_back(std::move(t));      // sole owner: a first accumulation takes the tensor itself
+        list.emplace_back();
+        return list;
     }
 };
 

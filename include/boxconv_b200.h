@@ -214,7 +214,16 @@ int bc_boxconv2d_backward_narrow(const void *input, int io_kind, const float *x_
                                  int F, int h, int w, int normalize, int exact, int need_mask,
                                  void *grad_input, float *grad_params, void *workspace,
                                  size_t workspace_bytes, bc_stream_t stream);
-/* The same with the parameter gradients stored in the 16-bit type too (rounded once, from the float sums). */
+/* The same for larger planes as well (bc_boxconv2d_narrow_all_supported() tells; up to 2048 columns and 32
+ * filters), through float integral images in a workspace of bc_boxconv2d_narrow_workspace() bytes (need_mask 0 for
+ * the forward), and with the parameter gradients stored in the 16-bit type too, rounded once from the float sums. */
+int bc_boxconv2d_narrow_all_supported(int F, int h, int w);
+size_t bc_boxconv2d_narrow_workspace(int N, int C, int F, int h, int w, int need_mask);
+int bc_boxconv2d_forward_narrow_all(const void *input, int io_kind, const float *x_min, const float *x_max,
+                                    const float *y_min, const float *y_max, float reparametrization_h,
+                                    float reparametrization_w, void *output, int N, int C, int F, int h,
+                                    int w, int normalize, int exact, void *workspace, size_t workspace_bytes,
+                                    bc_stream_t stream);
 int bc_boxconv2d_backward_narrow_all(const void *input, int io_kind, const float *x_min, const float *x_max,
                                      const float *y_min, const float *y_max, const void *grad_output,
                                      float reparametrization_h, float reparametrization_w, int N, int C,
