@@ -58,7 +58,7 @@ int raise_smem_limit(const void *kernel, int bytes);
 enum KernelId {
     KID_INTEGRAL = 1, KID_FORWARD_GLOBAL, KID_BACKWARD_GLOBAL, KID_FINISH_PARAM_GRADS, KID_CLIP,
     KID_FORWARD_PLANE, KID_BACKWARD_PLANE, KID_SUM_CHUNKS, KID_BACKWARD_BAND, KID_INTEGRAL_BANDS, KID_FORWARD_BAND,
-    KID_FORWARD_SLAB, KID_BACKWARD_SLAB, KID_COUNT
+    KID_FORWARD_SLAB, KID_BACKWARD_SLAB, KID_FORWARD_QUAD, KID_BACKWARD_QUAD, KID_COUNT
 };
 
 // Put around a kernel launch: counts it and, while profiling is enabled, records a CUDA event on

@@ -29,26 +29,37 @@ __device__ __forceinline__ BoxTaps load_taps_uniform(const float *tab)
     return t;
 }
 
+// Inclusive sum over the warp; the shuffle's own predicate tells which lanes have somebody to add.
+__device__ __forceinline__ float warp_scan(float v)
+{
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1)
+        asm volatile("{\n .reg .f32 u;\n .reg .pred p;\n shfl.sync.up.b32 u|p, %0, %1, 0, 0xffffffff;\n @p add.f32 %0, %0, u;\n}"
+                     : "+f"(v) : "r"(d));
+    return v;
+}
+
 // Byte offsets within a row of the five taps on either side of the box, for the strip of columns 4*j .. 4*j+3.
 // `shift` (the tap's column less the strip's) is the same for the whole warp.
 struct QuadCols {
     uint32_t lo[kStrip + 1], hi[kStrip + 1];
 };
-__device__ __forceinline__ void quad_window(uint32_t (&off)[kStrip + 1], int j, int shift, int cells)
+// `cells`: of the plane's own columns (quad_cells(w)); `stride`: of a sub-row, which may be longer.
+__device__ __forceinline__ void quad_window(uint32_t (&off)[kStrip + 1], int j, int shift, int cells, int stride)
 {
     const int r = shift & 3, j0 = j + (shift >> 2);
     const uint32_t a = (uint32_t)(min(max(j0, -1), cells - 2) + 1) * 4u, b = (uint32_t)(min(max(j0 + 1, -1), cells - 2) + 1) * 4u;
 #pragma unroll
     for (int m = 0; m <= kStrip; ++m) {
         const int s = r + m;
-        off[m] = (uint32_t)((s & 3) * cells * 4) + (s < 4 ? a : b);
+        off[m] = (uint32_t)((s & 3) * stride * 4) + (s < 4 ? a : b);
     }
 }
-__device__ __forceinline__ QuadCols quad_cols(const BoxTaps &t, int j, int cells)
+__device__ __forceinline__ QuadCols quad_cols(const BoxTaps &t, int j, int cells, int stride)
 {
     QuadCols c;
-    quad_window(c.lo, j, t.lo_c - 1, cells);
-    quad_window(c.hi, j, t.hi_c, cells);
+    quad_window(c.lo, j, t.lo_c - 1, cells, stride);
+    quad_window(c.hi, j, t.hi_c, cells, stride);
     return c;
 }
 
@@ -141,49 +152,58 @@ __device__ __forceinline__ float warp_sum5(const float (&v)[kNumSums], int lane)
 }
 
 // One filter's contribution of a strip of R rows to grad-input and to the five sums.  `x(i)` gives the four
-// input values of row i; rows at or past `rows` do not exist.
+// input values of row i; FULL: the strip has all its rows, else those at or past `rows` do not exist (x is zero there).
 // The column strips enter the sums weighted by u(j), what the rows of the box make of the input values next to
 // tap row j: sum_i x_i (row combination of e) = sum_j e(j) (w_a x_(j+1) + w_b x_j).
-template <int R, bool NEED_PARAMS>
+template <int R, bool NEED_PARAMS, bool FULL, class XRow>
 __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const QuadCols &cols, const QuadRows<R> &q, const ColW2 &cw,
-                                                    const float (&x)[R][kStrip], float (&gin)[R][kStrip], float (&sums)[kNumSums],
-                                                    int rows)
+                                                    XRow &&x, float (&gin)[R][kStrip], float (&sums)[kNumSums], int rows)
 {
+    f2_t pd[kStrip];
     if (NEED_PARAMS) {
         const f2_t wa = pack2(-t.f_lo_r, 1.0f - t.f_hi_r), wb = pack2(t.f_lo_r - 1.0f, t.f_hi_r);
         f2_t topbot = pack2(0.f, 0.f), left = topbot, right = topbot;
         float s_out = 0.f;
-        f2_t pd[kStrip], el[kStrip], eh[kStrip];
+        f2_t el[kStrip], eh[kStrip], xx[kStrip];
         quad_pair_e(cols, q.lo[0], q.hi[0], cw, pd, el, eh);
+        {
+            const float4 e = x(0);
+            xx[0] = pack2(e.x, e.x); xx[1] = pack2(e.y, e.y); xx[2] = pack2(e.z, e.z); xx[3] = pack2(e.w, e.w);
+        }
 #pragma unroll
         for (int m = 0; m < kStrip; ++m) {
-            const f2_t u = mul2(wa, pack2(x[0][m], x[0][m]));
+            const f2_t u = mul2(wa, xx[m]);
             left = fma2(u, el[m], left);
             right = fma2(u, eh[m], right);
         }
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            if (i < rows) {
-                f2_t cd[kStrip];
+            if (FULL || i < rows) {
+                f2_t cd[kStrip], xn[kStrip];
                 quad_pair_e(cols, q.lo[i + 1], q.hi[i + 1], cw, cd, el, eh);
+                if (i + 1 < R) {
+                    const float4 e = x(i + 1);
+                    xn[0] = pack2(e.x, e.x); xn[1] = pack2(e.y, e.y); xn[2] = pack2(e.z, e.z); xn[3] = pack2(e.w, e.w);
+                }
 #pragma unroll
                 for (int m = 0; m < kStrip; ++m) {
-                    const f2_t xx = pack2(x[i][m], x[i][m]);
-                    f2_t u = mul2(wb, xx);
-                    if (i + 1 < R) u = fma2(wa, pack2(x[i + 1][m], x[i + 1][m]), u);      // (zero past the last row)
+                    f2_t u = mul2(wb, xx[m]);
+                    if (i + 1 < R) u = fma2(wa, xn[m], u);
                     left = fma2(u, el[m], left);
                     right = fma2(u, eh[m], right);
                     const f2_t dd = sub2(cd[m], pd[m]);
-                    float lo_new, hi_new, lo_old, hi_old, top, bot;
+                    float lo_new, hi_new, lo_old, hi_old, top, bot, xv, xv2;
                     unpack2(cd[m], lo_new, hi_new);
                     unpack2(pd[m], lo_old, hi_old);
                     unpack2(dd, top, bot);
+                    unpack2(xx[m], xv, xv2);
                     const float g = (hi_old - lo_new) + t.f_hi_r * bot + t.f_lo_r * top;
-                    (void)hi_new; (void)lo_old;
-                    topbot = fma2(xx, dd, topbot);
-                    s_out += x[i][m] * g;
+                    (void)hi_new; (void)lo_old; (void)xv2;
+                    topbot = fma2(xx[m], dd, topbot);
+                    s_out += xv * g;
                     gin[i][m] += g * t.scale;
                     pd[m] = cd[m];
+                    if (i + 1 < R) xx[m] = xn[m];
                 }
             }
         }
@@ -193,11 +213,10 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
         unpack2(left, a, b); sums[3] = a + b;
         unpack2(right, a, b); sums[4] = a + b;
     } else {
-        f2_t pd[kStrip];
         quad_pair(cols, q.lo[0], q.hi[0], cw, pd);
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            if (i < rows) {
+            if (FULL || i < rows) {
                 f2_t cd[kStrip];
                 quad_pair(cols, q.lo[i + 1], q.hi[i + 1], cw, cd);
 #pragma unroll

@@ -126,6 +126,77 @@ struct IsFloat { static constexpr bool value = false; };
 template <>
 struct IsFloat<float> { static constexpr bool value = true; };
 
+// ---- rows of four columns a lane, whatever their alignment -------------------------------------
+// A warp works on 128 adjacent columns, lane L on columns c .. c+3 with c = c0 + 4 L.  Rows whose length is no
+// multiple of four start anywhere relative to a 4-element boundary; k, the same for the whole warp, is by how
+// many elements.  The memory access is then done on the aligned group that begins k elements earlier, one
+// vector access a lane, and the elements move k places between neighbouring lanes by shuffles.
+// All 32 lanes take part.  ALIGNED: k is zero for every row and w a multiple of four.
+template <typename IO>
+__device__ __forceinline__ int row_shift(const IO *row)
+{
+    return (int)(reinterpret_cast<uintptr_t>(row) / sizeof(IO)) & 3;
+}
+
+// Columns c .. c+3 of the row; zero from column w on, or when the row does not exist.
+template <typename IO, bool ALIGNED>
+__device__ __forceinline__ float4 load_row4(const IO *row, int c, int w, bool row_ok, int lane)
+{
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (ALIGNED) return row_ok && c < w ? Io<IO>::load4(row + c) : zero;
+    const int k = row_shift(row);
+    float4 a = row_ok && c - k < w ? Io<IO>::load4(row + (c - k)) : zero;
+    if (k) {
+        float4 n;      // the group that follows: the next lane's
+        n.x = __shfl_down_sync(0xffffffffu, a.x, 1);
+        n.y = k > 1 ? __shfl_down_sync(0xffffffffu, a.y, 1) : 0.f;
+        n.z = k > 2 ? __shfl_down_sync(0xffffffffu, a.z, 1) : 0.f;
+        if (lane == 31) n = row_ok && c + 4 - k < w ? Io<IO>::load4(row + (c + 4 - k)) : zero;
+        if (k == 1) a = make_float4(a.y, a.z, a.w, n.x);
+        else if (k == 2) a = make_float4(a.z, a.w, n.x, n.y);
+        else a = make_float4(a.w, n.x, n.y, n.z);
+    }
+    if (c >= w) a.x = 0.f;
+    if (c + 1 >= w) a.y = 0.f;
+    if (c + 2 >= w) a.z = 0.f;
+    if (c + 3 >= w) a.w = 0.f;
+    return a;
+}
+
+template <typename IO, bool ALIGNED>
+__device__ __forceinline__ void store_row4(IO *row, int c, int w, const float (&v)[4], int lane)
+{
+    if (ALIGNED) {
+        if (c < w) Io<IO>::store4(row + c, v[0], v[1], v[2], v[3]);
+        return;
+    }
+    const int k = row_shift(row);
+    float o[4] = {v[0], v[1], v[2], v[3]};
+    if (k) {
+        const float p3 = __shfl_up_sync(0xffffffffu, v[3], 1);
+        const float p2 = k > 1 ? __shfl_up_sync(0xffffffffu, v[2], 1) : 0.f;
+        const float p1 = k > 2 ? __shfl_up_sync(0xffffffffu, v[1], 1) : 0.f;
+        if (k == 1) { o[3] = v[2]; o[2] = v[1]; o[1] = v[0]; o[0] = p3; }
+        else if (k == 2) { o[3] = v[1]; o[2] = v[0]; o[1] = p3; o[0] = p2; }
+        else { o[3] = v[0]; o[2] = p3; o[1] = p2; o[0] = p1; }
+        if (lane == 31) {      // its last k columns have no lane after them
+#pragma unroll
+            for (int m = 1; m < 4; ++m)
+                if (m >= 4 - k && c + m < w) Io<IO>::store1(row + c + m, v[m]);
+        }
+    }
+    const int first = lane == 0 ? c : c - k;      // lane 0 has no lane before it
+    if (first == c - k && c - k + 4 <= w) {
+        Io<IO>::store4(row + (c - k), o[0], o[1], o[2], o[3]);
+    } else {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const int at = c - k + m;
+            if (at >= first && at < w) Io<IO>::store1(row + at, o[m]);
+        }
+    }
+}
+
 inline bool aligned_to(const void *p, int bytes) { return (reinterpret_cast<uintptr_t>(p) & (uintptr_t)(bytes - 1)) == 0; }
 
 // Bounded waits that expired in the kernels of this translation unit (synchronises).

@@ -39,6 +39,7 @@
 #include "bc_common.cuh"
 #include "bc_smem_walk.cuh"
 #include "bc_tile_io.cuh"
+#include "box_quad_plane.cuh"
 
 namespace bc {
 
@@ -659,6 +660,7 @@ template <typename IO>
 int launch_forward_plane_t(const IO *x, const BoxParams &bp, const Fusion *fu, IO *out, int N, int C, int F, int h,
                            int w, bool normalize, bool exact, cudaStream_t s)
 {
+    if (quad_fits_forward(F, h, w)) return launch_forward_quad_t<IO>(x, bp, fu, out, N, C, F, h, w, normalize, exact, s);
     const int64_t planes = (int64_t)N * C;
     // Split the filters of a plane over two CTAs when there are too few planes to balance 148 SMs
     // (each part rebuilds the integral image; the second read of the plane comes from L2).
@@ -701,6 +703,9 @@ int launch_backward_plane_t(const IO *x, const IO *grad_output, const BoxParams 
                             int C, int F, int h, int w, bool normalize, bool exact, int need_mask, IO *grad_input,
                             void *grad_params, int grad_params_kind, float *partials, cudaStream_t s)
 {
+    if (quad_fits_backward(F, h, w))
+        return launch_backward_quad_t<IO>(x, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
+                                          grad_params, grad_params_kind, partials, s);
     const int64_t planes = (int64_t)N * C;
     if (planes > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
     const bool need_params = (need_mask & (BC_NEED_ALL & ~BC_NEED_INPUT)) != 0;

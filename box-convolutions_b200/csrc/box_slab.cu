@@ -29,31 +29,9 @@ constexpr int kScanRows = 8;               // rows a warp of the integral kernel
 // eight rows are being loaded meanwhile.  No tile in shared memory, one pass over HBM.
 // With few planes a cluster of CTAs shares one: each first sums the columns of its rows, takes from the CTAs
 // above what they add to its columns (distributed shared memory), and then walks.
-template <typename IO, bool VEC>
-__device__ __forceinline__ float4 load_quad(const IO *row, int c, int w, bool row_ok)
-{
-    if (!row_ok || c >= w) return make_float4(0.f, 0.f, 0.f, 0.f);
-    if (VEC) return Io<IO>::load4(row + c);
-    float4 v = make_float4(Io<IO>::load1(row + c), 0.f, 0.f, 0.f);
-    if (c + 1 < w) v.y = Io<IO>::load1(row + c + 1);
-    if (c + 2 < w) v.z = Io<IO>::load1(row + c + 2);
-    if (c + 3 < w) v.w = Io<IO>::load1(row + c + 3);
-    return v;
-}
-
 __device__ __forceinline__ float4 relu4(float4 v)
 {
     return make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
-}
-
-// Inclusive sum over the warp; the shuffle's own predicate tells which lanes have somebody to add.
-__device__ __forceinline__ float warp_scan(float v)
-{
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1)
-        asm volatile("{\n .reg .f32 u;\n .reg .pred p;\n shfl.sync.up.b32 u|p, %0, %1, 0, 0xffffffff;\n @p add.f32 %0, %0, u;\n}"
-                     : "+f"(v) : "r"(d));
-    return v;
 }
 
 __device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank)
@@ -92,7 +70,7 @@ integral_quad_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, 
     grid_dependency_wait();
     float4 nxt[kScanRows];
 #pragma unroll
-    for (int i = 0; i < kScanRows; ++i) nxt[i] = load_quad<IO, VEC>(src + (int64_t)(r0 + i) * w, c, w, r0 + i < r1);
+    for (int i = 0; i < kScanRows; ++i) nxt[i] = load_row4<IO, VEC>(src + (int64_t)(r0 + i) * w, c, w, r0 + i < r1, lane);
 
     float run[4] = {0.f, 0.f, 0.f, 0.f};
     if (cluster > 1) {
@@ -105,7 +83,7 @@ integral_quad_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, 
 #pragma unroll
             for (int i = 0; i < kScanRows; ++i) {
                 const int rn = r + kScanRows + i;
-                ahead[i] = load_quad<IO, VEC>(src + (int64_t)rn * w, c, w, rn < r1);
+                ahead[i] = load_row4<IO, VEC>(src + (int64_t)rn * w, c, w, rn < r1, lane);
             }
 #pragma unroll
             for (int i = 0; i < kScanRows; ++i) {
@@ -150,7 +128,7 @@ integral_quad_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, 
         for (int i = 0; i < kScanRows; ++i) {
             v[i] = RELU ? relu4(nxt[i]) : nxt[i];
             const int rn = r + kScanRows + i;
-            nxt[i] = load_quad<IO, VEC>(src + (int64_t)rn * w, c, w, rn < r1);
+            nxt[i] = load_row4<IO, VEC>(src + (int64_t)rn * w, c, w, rn < r1, lane);
         }
 #pragma unroll
         for (int i = 0; i < kScanRows; ++i) {
@@ -262,7 +240,7 @@ forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int 
     const int rg = warp / sh.col_tiles, ct = warp - rg * sh.col_tiles;
     const int q0 = ct * 128 + lane * kStrip, p0 = p_slab + rg * kStripRows;
     const int mine = min(kStripRows, p_slab + rows - p0);      // rows of this warp (may be <= 0)
-    const bool in_plane = q0 < w;      // (lanes past the plane gather too, from clamped columns, and store nothing)
+    // (lanes past the plane gather too, from clamped columns, and store nothing)
     bool timed_out = false;
     for (int k = 0; k < nf; ++k) {
         const int f = f_begin + k;
@@ -272,7 +250,7 @@ forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int 
             const SlabRows s = slab_rows(t, p_slab, rows, h);
             const uint32_t lo32 = stage32 - s.lo_first * row_bytes;
             const uint32_t hi32 = stage32 + sh.stage_bytes - s.hi_first * row_bytes;
-            const QuadCols cols = quad_cols(t, q0 >> 2, cells);
+            const QuadCols cols = quad_cols(t, q0 >> 2, cells, cells);
             const ColW2 cw = col_weights(t);
             const float sfl = t.scale * t.f_lo_r, sfh = t.scale * t.f_hi_r;
             const QuadRows<kStripRows> q = quad_rows<kStripRows>(t, p0, h, lo32, hi32, row_bytes, lane);
@@ -301,13 +279,7 @@ forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int 
                             if (fu.output_relu) v[m] = fmaxf(v[m], 0.0f);
                         }
                     }
-                    if (VEC) {
-                        if (in_plane) Io<IO>::store4(out + off, v[0], v[1], v[2], v[3]);
-                    } else {
-#pragma unroll
-                        for (int m = 0; m < kStrip; ++m)
-                            if (q0 + m < w) Io<IO>::store1(out + off + m, v[m]);
-                    }
+                    store_row4<IO, VEC>(out + off - q0, q0, w, v, lane);
                     off += w;
                 }
             }
@@ -362,13 +334,13 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ go_inte
     const int rg = warp / sh.col_tiles, ct = warp - rg * sh.col_tiles;
     const int q0 = ct * 128 + lane * kStrip, p0 = p_slab + rg * kStripRows;
     const int mine = min(kStripRows, p_slab + rows - p0);
-    const bool active = q0 < w && mine > 0;      // (lanes past the plane gather too, from clamped columns, with x = 0)
+    // (lanes past the plane gather too, from clamped columns, with x = 0)
     const int64_t pix = nc * (int64_t)h * w + (int64_t)p0 * w + q0;
     float xv[kStripRows][kStrip], gin[kStripRows][kStrip];
 #pragma unroll
     for (int i = 0; i < kStripRows; ++i) {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (NEED_PARAMS) v = load_quad<IO, VEC>(x + pix - q0 + (int64_t)i * w, q0, w, i < mine);
+        if (NEED_PARAMS) v = load_row4<IO, VEC>(x + pix - q0 + (int64_t)i * w, q0, w, i < mine, lane);
         xv[i][0] = v.x; xv[i][1] = v.y; xv[i][2] = v.z; xv[i][3] = v.w;
 #pragma unroll
         for (int m = 0; m < kStrip; ++m) gin[i][m] = 0.0f;
@@ -382,9 +354,13 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ go_inte
             const SlabRows s = slab_rows(t, p_slab, rows, h);
             const uint32_t lo32 = stage32 - s.lo_first * row_bytes;
             const uint32_t hi32 = stage32 + sh.stage_bytes - s.hi_first * row_bytes;
-            quad_backward_strip<kStripRows, NEED_PARAMS>(
-                t, quad_cols(t, q0 >> 2, cells), quad_rows<kStripRows>(t, p0, h, lo32, hi32, row_bytes, lane), col_weights(t), xv, gin,
-                sums, mine);
+            const QuadCols cols = quad_cols(t, q0 >> 2, cells, cells);
+            const QuadRows<kStripRows> q = quad_rows<kStripRows>(t, p0, h, lo32, hi32, row_bytes, lane);
+            auto xrow = [&](int i) { return make_float4(xv[i][0], xv[i][1], xv[i][2], xv[i][3]); };
+            if (mine == kStripRows)
+                quad_backward_strip<kStripRows, NEED_PARAMS, true>(t, cols, q, col_weights(t), xrow, gin, sums, mine);
+            else
+                quad_backward_strip<kStripRows, NEED_PARAMS, false>(t, cols, q, col_weights(t), xrow, gin, sums, mine);
         }
         if (NEED_PARAMS) {
             const float s = warp_sum5(sums, lane);
@@ -408,21 +384,11 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ go_inte
             partials[(((int64_t)(c * F + f) * N + n) * sh.slabs + slab) * kNumSums + j] = s;
         }
     }
-    if (write_gin && active) {
-        IO *dst = grad_input + pix;
+    if (write_gin && mine > 0) {
+        IO *row = grad_input + pix - q0;
 #pragma unroll
-        for (int i = 0; i < kStripRows; ++i) {
-            if (i < mine) {
-                if (VEC) {
-                    Io<IO>::store4(dst, gin[i][0], gin[i][1], gin[i][2], gin[i][3]);
-                } else {
-#pragma unroll
-                    for (int m = 0; m < kStrip; ++m)
-                        if (q0 + m < w) Io<IO>::store1(dst + m, gin[i][m]);
-                }
-                dst += w;
-            }
-        }
+        for (int i = 0; i < kStripRows; ++i, row += w)
+            if (i < mine) store_row4<IO, VEC>(row, q0, w, gin[i], lane);
     }
 }
 

@@ -717,6 +717,8 @@ const char *bc_kernel_name(int kernel_id)
         case KID_FORWARD_BAND: return "forward_band_kernel";
         case KID_FORWARD_SLAB: return "forward_slab_kernel";
         case KID_BACKWARD_SLAB: return "backward_slab_kernel";
+        case KID_FORWARD_QUAD: return "forward_quad_kernel";
+        case KID_BACKWARD_QUAD: return "backward_quad_kernel";
         default: return "unknown";
     }
 }
