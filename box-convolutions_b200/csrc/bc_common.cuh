@@ -166,6 +166,14 @@ int launch_backward_plane(const float *x, const float *grad_output, const BoxPar
                           int need_mask, float *grad_input, float *grad_params, float *partials,
                           cudaStream_t s);
 
+// From the input's integral image (plain rows) instead of the input.
+bool plane_path_fits_backward_integ(int F, int h, int w);
+int launch_forward_plane_integ(const float *integ, const BoxParams &bp, float *out, int N, int C, int F, int h, int w,
+                               bool normalize, bool exact, cudaStream_t s);
+int launch_backward_plane_integ(const float *x_integ, const float *grad_output, const BoxParams &bp, float rep_h, float rep_w,
+                                int N, int C, int F, int h, int w, bool normalize, bool exact, int need_mask, float *grad_input,
+                                float *grad_params, float *partials, cudaStream_t s);
+
 int read_wait_timeouts(int *count);
 int read_wait_timeouts_narrow(int *count);
 
@@ -200,10 +208,13 @@ bool slab_path_fits(int F, int h, int w);
 size_t slab_integral_floats(int64_t planes, int h, int w);
 size_t slab_partials_bytes(int N, int C, int F, int h, int w);
 int launch_integral_quad(const void *in, int io_kind, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s);
+// The same kernel writing plain (h+1) x (w+1) rows; w up to 2048, h and w at least 1.
+int launch_integral_scan(const float *in, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s);
 // null `fu` = plain forward (16-bit outputs: always)
 int launch_forward_slab(const float *integ, const BoxParams &bp, const Fusion *fu, void *out, int io_kind, int N, int C, int F,
                         int h, int w, bool normalize, bool exact, cudaStream_t s);
-int launch_backward_slab(const void *x, int io_kind, const float *go_integ, const BoxParams &bp, float rep_h, float rep_w, int N,
+// x_integ (float only): the input's integral image in plain rows, used when x is null
+int launch_backward_slab(const void *x, const float *x_integ, int io_kind, const float *go_integ, const BoxParams &bp, float rep_h, float rep_w, int N,
                          int C, int F, int h, int w, bool normalize, bool exact, int need_mask, void *grad_input, void *grad_params,
                          int grad_params_kind, float *partials, cudaStream_t s);
 int read_wait_timeouts_slab(int *count);

@@ -31,6 +31,11 @@ __device__ __forceinline__ float4 lds128(uint32_t a)
     asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
     return v;
 }
+__device__ __forceinline__ void sts128(uint32_t a, float4 v)
+{
+    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
 // Two floats in one 64-bit register for the packed fp32 pipe of sm_100 (add/sub/mul/fma.f32x2):
 // one issue slot does the arithmetic of two lanes.  .x is the low half.
 typedef unsigned long long f2_t;
@@ -60,6 +65,13 @@ __device__ __forceinline__ f2_t sub2(f2_t a, f2_t b)
 {
     f2_t r;
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+__device__ __forceinline__ f2_t add2(f2_t a, f2_t b)
+{
+    f2_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
 

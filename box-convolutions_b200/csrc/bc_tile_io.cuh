@@ -126,6 +126,12 @@ struct IsFloat { static constexpr bool value = false; };
 template <>
 struct IsFloat<float> { static constexpr bool value = true; };
 
+// Pixel at the upper left of the four integral-image values around `I` (rows of `pitch`).
+__device__ __forceinline__ float pixel_of_integral(const float *I, int pitch)
+{
+    return __ldg(I + pitch + 1) - __ldg(I + 1) - __ldg(I + pitch) + __ldg(I);
+}
+
 // ---- rows of four columns a lane, whatever their alignment -------------------------------------
 // A warp works on 128 adjacent columns, lane L on columns c .. c+3 with c = c0 + 4 L.  Rows whose length is no
 // multiple of four start anywhere relative to a 4-element boundary; k, the same for the whole warp, is by how

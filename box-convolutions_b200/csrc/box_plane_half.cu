@@ -10,10 +10,10 @@ int launch_forward_plane_narrow(const void *x, int io_kind, const BoxParams &bp,
                                 int w, bool normalize, bool exact, cudaStream_t s)
 {
     if (io_kind == BC_IO_F16)
-        return launch_forward_plane_t<__half>(static_cast<const __half *>(x), bp, nullptr, static_cast<__half *>(out), N, C,
+        return launch_forward_plane_t<__half>(static_cast<const __half *>(x), nullptr, bp, nullptr, static_cast<__half *>(out), N, C,
                                               F, h, w, normalize, exact, s);
     if (io_kind == BC_IO_BF16)
-        return launch_forward_plane_t<__nv_bfloat16>(static_cast<const __nv_bfloat16 *>(x), bp, nullptr,
+        return launch_forward_plane_t<__nv_bfloat16>(static_cast<const __nv_bfloat16 *>(x), nullptr, bp, nullptr,
                                                      static_cast<__nv_bfloat16 *>(out), N, C, F, h, w, normalize, exact, s);
     return BC_ERR_UNSUPPORTED;
 }
@@ -24,11 +24,11 @@ int launch_backward_plane_narrow(const void *x, const void *grad_output, int io_
                                  cudaStream_t s)
 {
     if (io_kind == BC_IO_F16)
-        return launch_backward_plane_t<__half>(static_cast<const __half *>(x), static_cast<const __half *>(grad_output), bp,
+        return launch_backward_plane_t<__half>(static_cast<const __half *>(x), nullptr, static_cast<const __half *>(grad_output), bp,
                                                rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask,
                                                static_cast<__half *>(grad_input), grad_params, grad_params_kind, partials, s);
     if (io_kind == BC_IO_BF16)
-        return launch_backward_plane_t<__nv_bfloat16>(static_cast<const __nv_bfloat16 *>(x),
+        return launch_backward_plane_t<__nv_bfloat16>(static_cast<const __nv_bfloat16 *>(x), nullptr,
                                                       static_cast<const __nv_bfloat16 *>(grad_output), bp, rep_h, rep_w, N,
                                                       C, F, h, w, normalize, exact, need_mask,
                                                       static_cast<__nv_bfloat16 *>(grad_input), grad_params, grad_params_kind, partials, s);

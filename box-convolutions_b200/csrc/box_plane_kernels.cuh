@@ -268,7 +268,7 @@ __device__ __forceinline__ Walk make_walk(uint32_t sI32, const BoxTaps &t, int q
 // so it is not declared restrict).
 template <typename IO, int T, bool FAST, bool FUSED = false>
 __global__ void __launch_bounds__(T == 1 ? 256 : 512, T == 1 ? 4 : 1)
-forward_plane_kernel(const IO *__restrict__ x, BoxParams bp, IO *out, int C, int F,
+forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, BoxParams bp, IO *out, int C, int F,
                      int h, int w, int fsplit, bool normalize, bool exact, Fusion fu)
 {
     extern __shared__ float4 smem4[];
@@ -288,7 +288,7 @@ forward_plane_kernel(const IO *__restrict__ x, BoxParams bp, IO *out, int C, int
     const int cg = lane & 7, rg = lane >> 3;
 
     // a hint only: the plane on its way to L2 while this CTA still waits for the kernel in front
-    if (FAST && IsFloat<IO>::value && threadIdx.x == 0 && part == 0)
+    if (FAST && x && IsFloat<IO>::value && threadIdx.x == 0 && part == 0)
         bulk_prefetch_l2(x + nc * (int64_t)h * w, (uint32_t)(h * w) * 4u);
     Strip st[T];
 #pragma unroll
@@ -303,7 +303,15 @@ forward_plane_kernel(const IO *__restrict__ x, BoxParams bp, IO *out, int C, int
         store_taps(sTaps + threadIdx.x * kTapWords,
                    taps_forward(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
     }
-    {
+    if (!x) {      // the caller has the integral image itself: it is only copied
+        const float *I = integ + nc * (int64_t)(h + 1) * (w + 1);
+        const int pitch = g.pitch4 >> 2;
+        __syncthreads();      // (the zero padding has been written)
+        for (int a = warp; a <= h; a += nwarps)
+            for (int col = lane; col < w + 1 + kPad; col += 32)
+                sI[a * pitch + (a >> 3) + kPad + col] = __ldg(I + (int64_t)a * (w + 1) + min(col, w));
+        __syncthreads();
+    } else {
         Blocks<T> blk;
         build_rows<IO, T, FAST, false, FUSED>(blk, st, x + nc * (int64_t)h * w, 0u, sRow, g, cg, rg, FUSED && fu.input_relu);
         build_columns<T, FAST>(blk, st, sRow, sCol, g, cg, rg);
@@ -389,7 +397,7 @@ forward_plane_kernel(const IO *__restrict__ x, BoxParams bp, IO *out, int C, int
 // STAGED, narrow ones are converted by the threads as they are copied in.
 template <typename IO, int T, bool FAST, bool STAGED, bool NEED_PARAMS, bool XSMEM = true>
 __global__ void __launch_bounds__(512)
-backward_plane_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_output, BoxParams bp,
+backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const IO *__restrict__ grad_output, BoxParams bp,
                       IO *__restrict__ grad_input, float *__restrict__ partials, int N, int C, int F,
                       int h, int w, bool normalize, bool exact, bool write_gin)
 {
@@ -433,10 +441,10 @@ backward_plane_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_outp
         // While this CTA waits for the kernel in front of it, its first planes can already travel to L2
         // (a hint: if that kernel is still writing them, L2 receives its writes as well).
         bulk_prefetch_l2(gbase, plane_bytes);
-        if (NEED_PARAMS && X_BY_COPY) bulk_prefetch_l2(x + nc * (int64_t)npix, plane_bytes);
+        if (NEED_PARAMS && X_BY_COPY && !x_integ) bulk_prefetch_l2(x + nc * (int64_t)npix, plane_bytes);
         grid_dependency_wait();      // grad_output and the input may come from the kernel in front
         bulk_load(sG32, gbase, plane_bytes, mbarG);
-        if (NEED_PARAMS && X_BY_COPY) bulk_load(sX32, x + nc * (int64_t)npix, plane_bytes, mbarX);
+        if (NEED_PARAMS && X_BY_COPY && !x_integ) bulk_load(sX32, x + nc * (int64_t)npix, plane_bytes, mbarX);
         if (F > 1) bulk_prefetch_l2(gbase + (int64_t)npix, plane_bytes);
     }
     init_integral_padding(sI, g);
@@ -449,7 +457,12 @@ backward_plane_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_outp
         store_taps(sTaps + tid * kTapWords, taps_mirrored(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
     }
     if (STAGED) __syncthreads();                           // barriers initialised before anyone waits
-    if (!X_BY_COPY && NEED_PARAMS && XSMEM) {
+    if (NEED_PARAMS && XSMEM && x_integ) {
+        // (read by the first gather, which follows the barriers of the first build)
+        const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1);
+        for (int p = warp; p < h; p += nwarps)
+            for (int q = lane; q < w; q += 32) sX[p * w + q] = pixel_of_integral(I + p * (w + 1) + q, w + 1);
+    } else if (!X_BY_COPY && NEED_PARAMS && XSMEM) {
         // (read by the first gather, which follows the barriers of the first build)
         const IO *xp = x + nc * (int64_t)npix;
         if (FAST) {
@@ -492,7 +505,7 @@ backward_plane_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_outp
                     if (st[k].active && st[k].p0 + i < h)
                         asm volatile("prefetch.global.L2 [%0];" ::"l"(gbase + (f + 1) * (int64_t)npix + st[k].pix + i * w));
         }
-        if (X_BY_COPY && NEED_PARAMS && f == 0) timed_out |= !mbar_wait(mbarX, 0);
+        if (X_BY_COPY && NEED_PARAMS && !x_integ && f == 0) timed_out |= !mbar_wait(mbarX, 0);
 
         const BoxTaps t = load_taps(sTaps + f * kTapWords);
         const ColW2 cw = col_weights(t);
@@ -650,6 +663,13 @@ inline bool plane_fits_forward(int F, int h, int w)
     return F <= kMaxFilters && warp_tiles(h, w) <= kMaxTiles && plane_forward_smem_bytes(h, w) <= kMaxSmem;
 }
 
+// Backward from the input's integral image: the kernels that keep the input plane in shared memory.
+inline bool plane_fits_backward_integ(int F, int h, int w)
+{
+    return F <= kMaxFilters && warp_tiles(h, w) <= kMaxTiles &&
+           (quad_fits_backward(F, h, w) || plane_backward_smem_bytes(h, w, true, false, 4) <= kMaxSmem);
+}
+
 inline bool plane_fits_backward(int F, int h, int w)
 {
     return F <= kMaxFilters && warp_tiles(h, w) <= kMaxTiles && plane_backward_smem_bytes(h, w, false, false, 4) <= kMaxSmem;
@@ -657,10 +677,10 @@ inline bool plane_fits_backward(int F, int h, int w)
 
 // `fu` (inference steps around the gather) exists for float tensors only.
 template <typename IO>
-int launch_forward_plane_t(const IO *x, const BoxParams &bp, const Fusion *fu, IO *out, int N, int C, int F, int h,
+int launch_forward_plane_t(const IO *x, const float *integ, const BoxParams &bp, const Fusion *fu, IO *out, int N, int C, int F, int h,
                            int w, bool normalize, bool exact, cudaStream_t s)
 {
-    if (quad_fits_forward(F, h, w)) return launch_forward_quad_t<IO>(x, bp, fu, out, N, C, F, h, w, normalize, exact, s);
+    if (quad_fits_forward(F, h, w)) return launch_forward_quad_t<IO>(x, integ, bp, fu, out, N, C, F, h, w, normalize, exact, s);
     const int64_t planes = (int64_t)N * C;
     // Split the filters of a plane over two CTAs when there are too few planes to balance 148 SMs
     // (each part rebuilds the integral image; the second read of the plane comes from L2).
@@ -676,7 +696,7 @@ int launch_forward_plane_t(const IO *x, const BoxParams &bp, const Fusion *fu, I
     const int vec = Io<IO>::kVecBytes;
     const bool fast = (h % kR == 0) && (w % kStrip == 0) && aligned_to(x, vec) && aligned_to(out, vec) &&
                       (!fu || !fu->residual || aligned_to(fu->residual, 16));
-    void (*kern)(const IO *, BoxParams, IO *, int, int, int, int, int, bool, bool, Fusion);
+    void (*kern)(const IO *, const float *, BoxParams, IO *, int, int, int, int, int, bool, bool, Fusion);
     if (fu && IsFloat<IO>::value) {
         if (fast) kern = T == 1 ? forward_plane_kernel<IO, 1, true, IsFloat<IO>::value> : forward_plane_kernel<IO, 2, true, IsFloat<IO>::value>;
         else kern = T == 1 ? forward_plane_kernel<IO, 1, false, IsFloat<IO>::value> : forward_plane_kernel<IO, 2, false, IsFloat<IO>::value>;
@@ -691,7 +711,7 @@ int launch_forward_plane_t(const IO *x, const BoxParams &bp, const Fusion *fu, I
     const Fusion none{0, nullptr, nullptr, nullptr, 0};
     {
         LaunchScope scope(KID_FORWARD_PLANE, s);
-        if (cudaError_t e = launch_overlapped(kern, (unsigned)(planes * fsplit), warps * 32, smem, s, x, bp, out, C, F, h, w,
+        if (cudaError_t e = launch_overlapped(kern, (unsigned)(planes * fsplit), warps * 32, smem, s, x, integ, bp, out, C, F, h, w,
                                               fsplit, normalize, exact, fu ? *fu : none))
             return cuda_failed(e, "forward_plane");
     }
@@ -699,12 +719,12 @@ int launch_forward_plane_t(const IO *x, const BoxParams &bp, const Fusion *fu, I
 }
 
 template <typename IO>
-int launch_backward_plane_t(const IO *x, const IO *grad_output, const BoxParams &bp, float rep_h, float rep_w, int N,
+int launch_backward_plane_t(const IO *x, const float *x_integ, const IO *grad_output, const BoxParams &bp, float rep_h, float rep_w, int N,
                             int C, int F, int h, int w, bool normalize, bool exact, int need_mask, IO *grad_input,
                             void *grad_params, int grad_params_kind, float *partials, cudaStream_t s)
 {
     if (quad_fits_backward(F, h, w))
-        return launch_backward_quad_t<IO>(x, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
+        return launch_backward_quad_t<IO>(x, x_integ, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
                                           grad_params, grad_params_kind, partials, s);
     const int64_t planes = (int64_t)N * C;
     if (planes > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
@@ -727,7 +747,7 @@ int launch_backward_plane_t(const IO *x, const IO *grad_output, const BoxParams 
                         aligned_to(x, 16) && ((size_t)h * w * io) % 16 == 0 &&
                         (with_staging <= two_ctas || plane_backward_smem_bytes(h, w, need_params, false, io) > two_ctas);
     const size_t smem = plane_backward_smem_bytes(h, w, need_params && xsmem, staged, io);
-    void (*kern)(const IO *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, bool, bool, bool);
+    void (*kern)(const IO *, const float *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, bool, bool, bool);
     if (!xsmem) {
         if (fast) kern = T == 1 ? backward_plane_kernel<IO, 1, true, false, true, false> : backward_plane_kernel<IO, 2, true, false, true, false>;
         else kern = T == 1 ? backward_plane_kernel<IO, 1, false, false, true, false> : backward_plane_kernel<IO, 2, false, false, true, false>;
@@ -744,7 +764,7 @@ int launch_backward_plane_t(const IO *x, const IO *grad_output, const BoxParams 
     if (st != BC_OK) return st;
     {
         LaunchScope scope(KID_BACKWARD_PLANE, s);
-        if (cudaError_t e = launch_overlapped(kern, (unsigned)planes, warps * 32, smem, s, x, grad_output, bp, grad_input,
+        if (cudaError_t e = launch_overlapped(kern, (unsigned)planes, warps * 32, smem, s, x, x_integ, grad_output, bp, grad_input,
                                               partials, N, C, F, h, w, normalize, exact, write_gin))
             return cuda_failed(e, "backward_plane");
     }

@@ -6,17 +6,18 @@ namespace bc {
 
 bool plane_path_fits_forward(int F, int h, int w) { return plane_fits_forward(F, h, w); }
 bool plane_path_fits_backward(int F, int h, int w) { return plane_fits_backward(F, h, w); }
+bool plane_path_fits_backward_integ(int F, int h, int w) { return plane_fits_backward_integ(F, h, w); }
 
 int launch_forward_plane(const float *x, const BoxParams &bp, float *out, int N, int C, int F, int h,
                          int w, bool normalize, bool exact, cudaStream_t s)
 {
-    return launch_forward_plane_t<float>(x, bp, nullptr, out, N, C, F, h, w, normalize, exact, s);
+    return launch_forward_plane_t<float>(x, nullptr, bp, nullptr, out, N, C, F, h, w, normalize, exact, s);
 }
 
 int launch_forward_plane_fused(const float *x, const BoxParams &bp, const Fusion &fu, float *out, int N, int C,
                                int F, int h, int w, bool normalize, bool exact, cudaStream_t s)
 {
-    return launch_forward_plane_t<float>(x, bp, &fu, out, N, C, F, h, w, normalize, exact, s);
+    return launch_forward_plane_t<float>(x, nullptr, bp, &fu, out, N, C, F, h, w, normalize, exact, s);
 }
 
 int launch_backward_plane(const float *x, const float *grad_output, const BoxParams &bp, float rep_h,
@@ -24,7 +25,21 @@ int launch_backward_plane(const float *x, const float *grad_output, const BoxPar
                           int need_mask, float *grad_input, float *grad_params, float *partials,
                           cudaStream_t s)
 {
-    return launch_backward_plane_t<float>(x, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask,
+    return launch_backward_plane_t<float>(x, nullptr, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask,
+                                          grad_input, grad_params, BC_IO_F32, partials, s);
+}
+
+int launch_forward_plane_integ(const float *integ, const BoxParams &bp, float *out, int N, int C, int F, int h, int w,
+                               bool normalize, bool exact, cudaStream_t s)
+{
+    return launch_forward_plane_t<float>(nullptr, integ, bp, nullptr, out, N, C, F, h, w, normalize, exact, s);
+}
+
+int launch_backward_plane_integ(const float *x_integ, const float *grad_output, const BoxParams &bp, float rep_h, float rep_w,
+                                int N, int C, int F, int h, int w, bool normalize, bool exact, int need_mask, float *grad_input,
+                                float *grad_params, float *partials, cudaStream_t s)
+{
+    return launch_backward_plane_t<float>(nullptr, x_integ, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask,
                                           grad_input, grad_params, BC_IO_F32, partials, s);
 }
 

@@ -33,24 +33,21 @@ struct QuadImage {
 };
 __host__ __device__ inline int quad_image_bytes(int h, int ct) { return (h + 1) * (32 * ct + 3) * 16; }
 
-// Shared memory behind the image: column sums (512 bytes a tile), row sums (32 bytes a tile), then the boxes.
+// Shared memory behind the image: last rows (512 bytes a tile), row sums (32 bytes a tile), a scan corner per warp
+// (kScanBytes), then the boxes.
 struct QuadSmem {
-    uint32_t image, col, row, taps;
+    uint32_t image, col, row, scan, taps;
 };
-__device__ __forceinline__ QuadSmem quad_smem(const void *base, int h, int ct, int ntiles)
+__device__ __forceinline__ QuadSmem quad_smem(const void *base, int h, int ct, int ntiles, int nwarps)
 {
     QuadSmem s;
     s.image = smem_u32(base);
     asm volatile("" : "+r"(s.image));      // opaque: the compiler would rather work the window's base out again at every use
     s.col = s.image + quad_image_bytes(h, ct);
     s.row = s.col + ntiles * 512;
-    s.taps = s.row + ntiles * 32;
+    s.scan = s.row + ntiles * 32;
+    s.taps = s.scan + nwarps * (kTileRows * 36 * 4);
     return s;
-}
-
-__device__ __forceinline__ void sts128(uint32_t a, float4 v)
-{
-    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
 // A warp's tile: 8 rows x 128 columns, 4 columns a lane.
@@ -82,36 +79,78 @@ __device__ __forceinline__ void quad_zero_padding(uint32_t image, int h)
     }
 }
 
+// A lane's 8 x 4 values, each row as two packed pairs (columns c, c+1 and c+2, c+3).
+struct QuadBlock {
+    f2_t a[kTileRows], b[kTileRows];
+};
+
 // FULL: the tile has all its rows.
 template <typename IO, bool VEC, bool FULL>
-__device__ __forceinline__ void quad_load_tile(float4 (&v)[kTileRows], const QuadTile &t, const IO *plane, int w, int lane)
+__device__ __forceinline__ void quad_load_tile(QuadBlock &v, const QuadTile &t, const IO *plane, int w, int lane)
 {
     const IO *row = plane + t.p0 * w;
 #pragma unroll
-    for (int i = 0; i < kTileRows; ++i) v[i] = load_row4<IO, VEC>(row + i * w, t.c, w, FULL || i < t.rows, lane);
+    for (int i = 0; i < kTileRows; ++i) {
+        const float4 e = load_row4<IO, VEC>(row + i * w, t.c, w, FULL || i < t.rows, lane);
+        v.a[i] = pack2(e.x, e.y);
+        v.b[i] = pack2(e.z, e.w);
+    }
 }
 
 // Build, first part: the tile's own 2-D prefix sums; with several column tiles only down its columns and along
-// its rows within the tile, the rows' totals being published (followed by a barrier, then quad_join_rows()).
+// its rows within the tile, the rows' totals being published (followed by a barrier).
+// The sums of a row's 32 lanes are scanned eight rows at once through a corner of shared memory: four lanes a
+// row, each with eight of its values, then two shuffle steps.  Shuffling every row by itself takes five
+// shuffles and five additions a row, twice the instructions.
+constexpr int kScanPitch = 36;      // words per row: eight lanes' 16-byte accesses fall into distinct banks
+constexpr int kScanBytes = kTileRows * kScanPitch * 4;
 template <int CT>
-__device__ __forceinline__ void quad_scan(float4 (&v)[kTileRows], float (&carry)[kTileRows], const QuadTile &t, const QuadSmem &s, int lane)
+__device__ __forceinline__ void quad_scan(QuadBlock &v, float (&carry)[kTileRows], const QuadTile &t, const QuadSmem &s, int warp, int lane)
 {
-#pragma unroll
-    for (int i = 1; i < kTileRows; ++i) { v[i].x += v[i - 1].x; v[i].y += v[i - 1].y; v[i].z += v[i - 1].z; v[i].w += v[i - 1].w; }
+    const uint32_t scan = s.scan + warp * kScanBytes;
 #pragma unroll
     for (int i = 0; i < kTileRows; ++i) {
-        v[i].y += v[i].x;
-        v[i].z += v[i].y;
-        v[i].w += v[i].z;
-        const float incl = warp_scan(v[i].w);
-        carry[i] = incl - v[i].w;
-        if (CT > 1 && lane == 31) sts<0>(s.row + (t.rt * CT + t.ct) * 32 + i * 4, incl);
+        if (i) { v.a[i] = add2(v.a[i], v.a[i - 1]); v.b[i] = add2(v.b[i], v.b[i - 1]); }
     }
+    __syncwarp();
+    auto row_of = [&](auto I) {
+        constexpr int i = decltype(I)::value;
+        float x, y, z, u;
+        unpack2(v.a[i], x, y);
+        unpack2(v.b[i], z, u);
+        y += x; z += y; u += z;
+        v.a[i] = pack2(x, y);
+        v.b[i] = pack2(z, u);
+        sts<i * kScanPitch * 4>(scan + lane * 4, u);
+    };
+    row_of(Index<0>{}); row_of(Index<1>{}); row_of(Index<2>{}); row_of(Index<3>{});
+    row_of(Index<4>{}); row_of(Index<5>{}); row_of(Index<6>{}); row_of(Index<7>{});
+    __syncwarp();
+    const int k = lane & 3;
+    const uint32_t mine = scan + (lane >> 2) * (kScanPitch * 4) + k * 32;
+    float4 p = lds128(mine), q = lds128(mine + 16);
+    p.y += p.x; p.z += p.y; p.w += p.z;
+    q.x += p.w; q.y += q.x; q.z += q.y; q.w += q.z;
+    float before = q.w;
+    {
+        const float u1 = __shfl_up_sync(0xffffffffu, before, 1);
+        if (k >= 1) before += u1;
+        const float u2 = __shfl_up_sync(0xffffffffu, before, 2);
+        if (k >= 2) before += u2;
+    }
+    if (CT > 1 && k == 3) sts<0>(s.row + (t.rt * CT + t.ct) * 32 + (lane >> 2) * 4, before);
+    before -= q.w;
+    sts128(mine, make_float4(before, before + p.x, before + p.y, before + p.z));
+    sts128(mine + 16, make_float4(before + p.w, before + q.x, before + q.y, before + q.z));
+    __syncwarp();
+    auto carry_of = [&](auto I) { constexpr int i = decltype(I)::value; carry[i] = lds<i * kScanPitch * 4>(scan + lane * 4); };
+    carry_of(Index<0>{}); carry_of(Index<1>{}); carry_of(Index<2>{}); carry_of(Index<3>{});
+    carry_of(Index<4>{}); carry_of(Index<5>{}); carry_of(Index<6>{}); carry_of(Index<7>{});
 }
 // Second part: carries joined, the tile's last row published as what it adds to the tiles below.  Followed by a
 // barrier.
 template <int CT>
-__device__ __forceinline__ void quad_publish(float4 (&v)[kTileRows], float (&carry)[kTileRows], const QuadTile &t, const QuadSmem &s, int lane)
+__device__ __forceinline__ void quad_publish(QuadBlock &v, float (&carry)[kTileRows], const QuadTile &t, const QuadSmem &s, int lane)
 {
     if (CT > 1) {
         for (int k = 0; k < t.ct; ++k) {
@@ -121,29 +160,42 @@ __device__ __forceinline__ void quad_publish(float4 (&v)[kTileRows], float (&car
         }
     }
 #pragma unroll
-    for (int i = 0; i < kTileRows; ++i) { v[i].x += carry[i]; v[i].y += carry[i]; v[i].z += carry[i]; v[i].w += carry[i]; }
-    sts128(s.col + (t.rt * CT + t.ct) * 512 + lane * 16, v[kTileRows - 1]);
+    for (int i = 0; i < kTileRows; ++i) {
+        const f2_t c = pack2(carry[i], carry[i]);
+        v.a[i] = add2(v.a[i], c);
+        v.b[i] = add2(v.b[i], c);
+    }
+    float4 e;
+    unpack2(v.a[kTileRows - 1], e.x, e.y);
+    unpack2(v.b[kTileRows - 1], e.z, e.w);
+    sts128(s.col + (t.rt * CT + t.ct) * 512 + lane * 16, e);
 }
 // Third part: what the tiles above add, and the stores.  Followed by a barrier.
 template <int CT, bool FULL>
-__device__ __forceinline__ void quad_store(const float4 (&v)[kTileRows], const QuadTile &t, const QuadSmem &s, int w, int lane)
+__device__ __forceinline__ void quad_store(QuadBlock &v, const QuadTile &t, const QuadSmem &s, int w, int lane)
 {
     using Q = QuadImage<CT>;
-    float4 up = make_float4(0.f, 0.f, 0.f, 0.f);
+    f2_t up_a = pack2(0.f, 0.f), up_b = up_a;
     uint32_t above = s.col + t.ct * 512 + lane * 16;
     for (int r = 0; r < t.rt; ++r, above += CT * 512) {
         const float4 u = lds128(above);
-        up.x += u.x; up.y += u.y; up.z += u.z; up.w += u.w;
+        up_a = add2(up_a, pack2(u.x, u.y));
+        up_b = add2(up_b, pack2(u.z, u.w));
     }
+#pragma unroll
+    for (int i = 0; i < kTileRows; ++i) { v.a[i] = add2(v.a[i], up_a); v.b[i] = add2(v.b[i], up_b); }
     // column c+1 of integral row p0+1: sub-row 1, cell c/4 + 1
     const uint32_t at = s.image + (t.p0 + 1) * Q::kRow + ((t.c >> 2) + 1) * 4;
     auto put = [&](auto I) {
         constexpr int kI = decltype(I)::value;
         if (FULL || kI < t.rows) {
-            sts<kI * Q::kRow + Q::kSub>(at, v[kI].x + up.x);
-            sts<kI * Q::kRow + 2 * Q::kSub>(at, v[kI].y + up.y);
-            sts<kI * Q::kRow + 3 * Q::kSub>(at, v[kI].z + up.z);
-            sts<kI * Q::kRow + 4>(at, v[kI].w + up.w);
+            float x, y, z, u;
+            unpack2(v.a[kI], x, y);
+            unpack2(v.b[kI], z, u);
+            sts<kI * Q::kRow + Q::kSub>(at, x);
+            sts<kI * Q::kRow + 2 * Q::kSub>(at, y);
+            sts<kI * Q::kRow + 3 * Q::kSub>(at, z);
+            sts<kI * Q::kRow + 4>(at, u);
         }
     };
     put(Index<0>{}); put(Index<1>{}); put(Index<2>{}); put(Index<3>{});
@@ -155,7 +207,9 @@ __device__ __forceinline__ void quad_store(const float4 (&v)[kTileRows], const Q
         const uint32_t extra = s.image + (t.p0 + 1) * Q::kRow + sub * Q::kSub + cell * 4;
         auto copy = [&](auto I) {
             constexpr int i = decltype(I)::value;
-            const float last = __shfl_sync(0xffffffffu, v[i].w + up.w, 31);
+            float z, u;
+            unpack2(v.b[i], z, u);
+            const float last = __shfl_sync(0xffffffffu, u, 31);
             if (lane < 7 && (FULL || i < t.rows)) sts<i * Q::kRow>(extra, last);
         };
         copy(Index<0>{}); copy(Index<1>{}); copy(Index<2>{}); copy(Index<3>{});
@@ -167,9 +221,10 @@ __device__ __forceinline__ void quad_store(const float4 (&v)[kTileRows], const Q
 // into tasks of one filter, one column tile and `chunk` row tiles, walked top to bottom so that a tap-row pair
 // is loaded once per row and once more per task.
 // FAST: rows and tensors aligned for vector accesses, heights a multiple of 8.
+// A null `x`: `integ` holds the plane's integral image, plain rows of w + 1 floats, which is only copied.
 template <typename IO, int CT, int T, bool FAST, bool FUSED, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 3 : 1)
-forward_quad_kernel(const IO *__restrict__ x, BoxParams bp, IO *out, int C, int F, int h, int w, int row_tiles, int fsplit, int chunk,
+forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, BoxParams bp, IO *out, int C, int F, int h, int w, int row_tiles, int fsplit, int chunk,
                     bool normalize, bool exact, Fusion fu)
 {
     using Q = QuadImage<CT>;
@@ -180,15 +235,28 @@ forward_quad_kernel(const IO *__restrict__ x, BoxParams bp, IO *out, int C, int 
     const int f_begin = (F * part) / fsplit, nf = (F * (part + 1)) / fsplit - f_begin;
     const int64_t npix = (int64_t)h * w, nc = plane_at;
     const int cells = quad_cells(w), ntiles = row_tiles * CT;
-    const QuadSmem s = quad_smem(smem4, h, CT, ntiles);
+    const QuadSmem s = quad_smem(smem4, h, CT, ntiles, nwarps);
     float *sTaps = reinterpret_cast<float *>(reinterpret_cast<char *>(smem4) + (s.taps - s.image));
 
     quad_zero_padding<CT>(s.image, h);
     // registers and shared memory only up to here; now what the kernel in front of this one may have written
     grid_dependency_wait();
-    {
+    if (!x) {
+        if ((int)threadIdx.x < nf) {
+            const Box box = load_box(bp, c * F + f_begin + threadIdx.x);
+            store_taps(sTaps + threadIdx.x * kTapWords, taps_forward(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
+        }
+        const float *I = integ + nc * (int64_t)(h + 1) * (w + 1);
+        __syncthreads();      // (the zero padding has been written)
+        for (int a = warp; a <= h; a += nwarps) {
+            for (int col = lane; col < 4 * (cells - 1); col += 32) {
+                const float e = __ldg(I + (int64_t)a * (w + 1) + min(col, w));
+                sts<0>(s.image + a * Q::kRow + (col & 3) * Q::kSub + ((col >> 2) + 1) * 4, e);
+            }
+        }
+    } else {
         QuadTile tile[T];
-        float4 v[T][kTileRows];
+        QuadBlock v[T];
         float carry[T][kTileRows];
 #pragma unroll
         for (int k = 0; k < T; ++k) {
@@ -204,10 +272,15 @@ forward_quad_kernel(const IO *__restrict__ x, BoxParams bp, IO *out, int C, int 
             if (!tile[k].rows) continue;
             if (FUSED && fu.input_relu) {
 #pragma unroll
-                for (int i = 0; i < kTileRows; ++i)
-                    v[k][i] = make_float4(fmaxf(v[k][i].x, 0.f), fmaxf(v[k][i].y, 0.f), fmaxf(v[k][i].z, 0.f), fmaxf(v[k][i].w, 0.f));
+                for (int i = 0; i < kTileRows; ++i) {
+                    float e0, e1;
+                    unpack2(v[k].a[i], e0, e1);
+                    v[k].a[i] = pack2(fmaxf(e0, 0.f), fmaxf(e1, 0.f));
+                    unpack2(v[k].b[i], e0, e1);
+                    v[k].b[i] = pack2(fmaxf(e0, 0.f), fmaxf(e1, 0.f));
+                }
             }
-            quad_scan<CT>(v[k], carry[k], tile[k], s, lane);
+            quad_scan<CT>(v[k], carry[k], tile[k], s, warp, lane);
         }
         if (CT > 1) __syncthreads();
 #pragma unroll
@@ -284,7 +357,7 @@ forward_quad_kernel(const IO *__restrict__ x, BoxParams bp, IO *out, int C, int 
 // grad_output plane is requested into L2 while the current one is gathered.
 template <typename IO, int CT, bool FAST, bool NEED_PARAMS, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 2 : 1)
-backward_quad_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_output, BoxParams bp, IO *__restrict__ grad_input,
+backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const IO *__restrict__ grad_output, BoxParams bp, IO *__restrict__ grad_input,
                      float *__restrict__ partials, int N, int C, int F, int h, int w, int row_tiles, bool normalize, bool exact,
                      bool write_gin)
 {
@@ -295,7 +368,7 @@ backward_quad_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_outpu
     const int64_t nc = blockIdx.x;
     const int c = blockIdx.x % C, n = blockIdx.x / C;
     const int npix = h * w, cells = quad_cells(w), ntiles = row_tiles * CT;
-    const QuadSmem s = quad_smem(smem4, h, CT, ntiles);
+    const QuadSmem s = quad_smem(smem4, h, CT, ntiles, nwarps);
     float *sTaps = reinterpret_cast<float *>(reinterpret_cast<char *>(smem4) + (s.taps - s.image));
     float *red = sTaps + F * kTapWords;                                                        // [F][warps][5]
     const uint32_t sx = s.taps + ((F * (kTapWords + ntiles * kNumSums) * 4 + 15) & ~15) + warp * (kTileRows * 512) + lane * 16;
@@ -306,10 +379,22 @@ backward_quad_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_outpu
     quad_zero_padding<CT>(s.image, h);
     grid_dependency_wait();
     if (NEED_PARAMS) {
-        float4 v[kTileRows];
-        quad_load_tile<IO, FAST, FAST>(v, tile, x + nc * npix, w, lane);
+        if (x_integ) {
+            // the caller has only the input's integral image: its pixels are second differences
+            const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1) + (int64_t)tile.p0 * (w + 1);
+#pragma unroll 1
+            for (int i = 0; i < kTileRows; ++i, I += w + 1) {
+                float e[4];
 #pragma unroll
-        for (int i = 0; i < kTileRows; ++i) sts128(sx + i * 512, v[i]);
+                for (int m = 0; m < 4; ++m) e[m] = i < tile.rows && tile.c + m < w ? pixel_of_integral(I + tile.c + m, w + 1) : 0.0f;
+                sts128(sx + i * 512, make_float4(e[0], e[1], e[2], e[3]));
+            }
+        } else {
+            const IO *row = x + nc * npix + tile.p0 * w;
+#pragma unroll
+            for (int i = 0; i < kTileRows; ++i)
+                sts128(sx + i * 512, load_row4<IO, FAST>(row + i * w, tile.c, w, FAST || i < tile.rows, lane));
+        }
     }
     if ((int)threadIdx.x < F) {
         const Box box = load_box(bp, c * F + threadIdx.x);
@@ -322,12 +407,12 @@ backward_quad_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_outpu
         for (int m = 0; m < kStrip; ++m) gin[i][m] = 0.0f;
     for (int f = 0; f < F; ++f) {
         {
-            float4 v[kTileRows];
+            QuadBlock v;
             float carry[kTileRows];
             quad_load_tile<IO, FAST, FAST>(v, tile, gbase + f * (int64_t)npix, w, lane);
             if (FAST && threadIdx.x == 0 && f + 1 < F)
                 bulk_prefetch_l2(gbase + (f + 1) * (int64_t)npix, (uint32_t)npix * (uint32_t)sizeof(IO));
-            quad_scan<CT>(v, carry, tile, s, lane);
+            quad_scan<CT>(v, carry, tile, s, warp, lane);
             if (CT > 1) __syncthreads();
             quad_publish<CT>(v, carry, tile, s, lane);
             __syncthreads();      // (also: every gather of the previous filter is done)
@@ -368,7 +453,7 @@ inline int quad_col_tiles(int w) { return (w + 127) / 128; }
 inline size_t quad_forward_smem(int F, int h, int w)
 {
     const int ct = quad_col_tiles(w), tiles = quad_row_tiles(h) * ct;
-    return (size_t)quad_image_bytes(h, ct) + tiles * 544 + F * kTapWords * 4;
+    return (size_t)quad_image_bytes(h, ct) + tiles * (544 + kScanBytes) + F * kTapWords * 4;
 }
 inline size_t quad_backward_smem(int F, int h, int w)
 {
@@ -390,7 +475,7 @@ inline bool quad_fits_backward(int F, int h, int w)
 }
 
 template <typename IO>
-int launch_forward_quad_t(const IO *x, const BoxParams &bp, const Fusion *fu, IO *out, int N, int C, int F, int h, int w,
+int launch_forward_quad_t(const IO *x, const float *integ, const BoxParams &bp, const Fusion *fu, IO *out, int N, int C, int F, int h, int w,
                           bool normalize, bool exact, cudaStream_t s)
 {
     const int row_tiles = quad_row_tiles(h), col_tiles = quad_col_tiles(w), tiles = row_tiles * col_tiles;
@@ -411,7 +496,7 @@ int launch_forward_quad_t(const IO *x, const BoxParams &bp, const Fusion *fu, IO
     }
     const bool fast = w % 4 == 0 && h % kTileRows == 0 && aligned_to(x, Io<IO>::kVecBytes) && aligned_to(out, Io<IO>::kVecBytes) &&
                      (!fu || !fu->residual || aligned_to(fu->residual, 16));
-    void (*kern)(const IO *, BoxParams, IO *, int, int, int, int, int, int, int, bool, bool, Fusion);
+    void (*kern)(const IO *, const float *, BoxParams, IO *, int, int, int, int, int, int, int, bool, bool, Fusion);
     auto pick = [&](auto ct) {
         constexpr int CT = decltype(ct)::value, S = 256, L = 512;
         constexpr bool FU = IsFloat<IO>::value;
@@ -430,7 +515,7 @@ int launch_forward_quad_t(const IO *x, const BoxParams &bp, const Fusion *fu, IO
     const Fusion none{0, nullptr, nullptr, nullptr, 0};
     {
         LaunchScope scope(KID_FORWARD_QUAD, s);
-        if (cudaError_t e = launch_overlapped(kern, (unsigned)(planes * fsplit), warps * 32, quad_forward_smem(nf, h, w), s, x, bp, out,
+        if (cudaError_t e = launch_overlapped(kern, (unsigned)(planes * fsplit), warps * 32, quad_forward_smem(nf, h, w), s, x, integ, bp, out,
                                               C, F, h, w, row_tiles, fsplit, chunk, normalize, exact, fu ? *fu : none))
             return cuda_failed(e, "forward_quad");
     }
@@ -438,7 +523,7 @@ int launch_forward_quad_t(const IO *x, const BoxParams &bp, const Fusion *fu, IO
 }
 
 template <typename IO>
-int launch_backward_quad_t(const IO *x, const IO *grad_output, const BoxParams &bp, float rep_h, float rep_w, int N, int C, int F,
+int launch_backward_quad_t(const IO *x, const float *x_integ, const IO *grad_output, const BoxParams &bp, float rep_h, float rep_w, int N, int C, int F,
                            int h, int w, bool normalize, bool exact, int need_mask, IO *grad_input, void *grad_params,
                            int grad_params_kind, float *partials, cudaStream_t s)
 {
@@ -449,7 +534,7 @@ int launch_backward_quad_t(const IO *x, const IO *grad_output, const BoxParams &
     const bool write_gin = (need_mask & BC_NEED_INPUT) != 0;
     const bool fast = w % 4 == 0 && h % kTileRows == 0 && ((size_t)h * w * sizeof(IO)) % 16 == 0 && aligned_to(x, Io<IO>::kVecBytes) &&
                      aligned_to(grad_output, 16) && (!write_gin || aligned_to(grad_input, Io<IO>::kVecBytes));
-    void (*kern)(const IO *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, int, bool, bool, bool);
+    void (*kern)(const IO *, const float *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, int, bool, bool, bool);
     auto pick = [&](auto ct) {
         constexpr int CT = decltype(ct)::value, S = 256, L = 512;
         if (tiles <= 8) {
@@ -466,7 +551,7 @@ int launch_backward_quad_t(const IO *x, const IO *grad_output, const BoxParams &
     if (st != BC_OK) return st;
     {
         LaunchScope scope(KID_BACKWARD_QUAD, s);
-        if (cudaError_t e = launch_overlapped(kern, (unsigned)planes, tiles * 32, quad_backward_smem(F, h, w), s, x, grad_output, bp,
+        if (cudaError_t e = launch_overlapped(kern, (unsigned)planes, tiles * 32, quad_backward_smem(F, h, w), s, x, x_integ, grad_output, bp,
                                               grad_input, partials, N, C, F, h, w, row_tiles, normalize, exact, write_gin))
             return cuda_failed(e, "backward_quad");
     }

@@ -1,6 +1,6 @@
 // Forward and backward for planes too large to keep in shared memory whole.
 //
-// Two kernels a pass.  integral_quad_kernel writes the integral images of a batch of planes to a workspace,
+// Two kernels a pass.  integral_scan_kernel writes the integral images of a batch of planes to a workspace,
 // rows in the quad layout (bc_quad.cuh).  The gather kernels then work on slabs: R rows of one plane, full
 // width.  What a slab of a box filter reads of the integral image is two runs of R + 1 adjacent rows, one on
 // either side of the box, each a contiguous piece of memory: two bulk copies per filter bring them to shared
@@ -51,9 +51,10 @@ __device__ __forceinline__ void cluster_sync()
     asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <typename IO, bool VEC, bool RELU, int MAXT>
+// QUAD: rows in the quad layout; else plain rows of w + 1 floats, the public integral image.
+template <typename IO, bool VEC, bool RELU, bool QUAD, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 5 : 1)
-integral_quad_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, int w, int rows_per_cta, int cluster)
+integral_scan_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, int w, int rows_per_cta, int cluster)
 {
     __shared__ __align__(16) float sTot[2][kSlabMaxWarps][kScanRows];
     extern __shared__ float4 sCol[];           // column sums of this CTA's rows (clusters only)
@@ -62,7 +63,7 @@ integral_quad_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, 
     const int64_t plane = blockIdx.x / cluster;
     const int rank = blockIdx.x % cluster;
     const int L = threadIdx.x, c = L * 4;
-    const int cells = quad_cells(w), pitch = 4 * cells;
+    const int cells = quad_cells(w), pitch = QUAD ? 4 * cells : w + 1;
     const int r0 = min(rank * rows_per_cta, h), r1 = min(r0 + rows_per_cta, h);
     const IO *src = in + plane * (int64_t)h * w;
     float *dst = out + plane * (int64_t)(h + 1) * pitch;
@@ -154,7 +155,14 @@ integral_quad_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, 
         }
 #pragma unroll
         for (int i = 0; i < kScanRows; ++i) {
-            if (r + i < r1) {
+            if (!QUAD) {
+                if (r + i < r1) {
+                    const float o[4] = {v[i].x + carry[i], v[i].y + carry[i], v[i].z + carry[i], v[i].w + carry[i]};
+                    store_row4<float, false>(row + 1, c, w, o, lane);
+                    if (threadIdx.x == 0) *row = 0.0f;
+                    row += pitch;
+                }
+            } else if (r + i < r1) {
                 const float x4 = v[i].w + carry[i];
                 if (in123) {
                     *d1 = v[i].x + carry[i];
@@ -297,7 +305,7 @@ forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int 
 // filters; the five sums are reduced per warp and filter, and per CTA at the end.
 template <typename IO, bool VEC, bool NEED_PARAMS, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1)
-backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ go_integ, BoxParams bp, IO *__restrict__ grad_input,
+backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const float *__restrict__ go_integ, BoxParams bp, IO *__restrict__ grad_input,
                      float *__restrict__ partials, int N, int C, int F, int h, int w, SlabShape sh, bool normalize, bool exact,
                      bool write_gin)
 {
@@ -336,15 +344,29 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ go_inte
     const int mine = min(kStripRows, p_slab + rows - p0);
     // (lanes past the plane gather too, from clamped columns, with x = 0)
     const int64_t pix = nc * (int64_t)h * w + (int64_t)p0 * w + q0;
-    float xv[kStripRows][kStrip], gin[kStripRows][kStrip];
+    // the lane's input values wait in shared memory, where only their own warp touches them
+    const uint32_t sx = smem_u32(red) + ((F * nwarps * kNumSums * 4 + 15) & ~15) + warp * (kStripRows * 512) + lane * 16;
+    if (NEED_PARAMS) {
+        if (x) {
+            const IO *row = x + pix - q0;
 #pragma unroll
-    for (int i = 0; i < kStripRows; ++i) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (NEED_PARAMS) v = load_row4<IO, VEC>(x + pix - q0 + (int64_t)i * w, q0, w, i < mine, lane);
-        xv[i][0] = v.x; xv[i][1] = v.y; xv[i][2] = v.z; xv[i][3] = v.w;
+            for (int i = 0; i < kStripRows; ++i) sts128(sx + i * 512, load_row4<IO, VEC>(row + (int64_t)i * w, q0, w, i < mine, lane));
+        } else {      // the caller has only the input's integral image: its pixels are second differences
+            const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1) + (int64_t)p0 * (w + 1) + q0;
+#pragma unroll 1
+            for (int i = 0; i < kStripRows; ++i, I += w + 1) {
+                float e[4];
+#pragma unroll
+                for (int m = 0; m < kStrip; ++m) e[m] = i < mine && q0 + m < w ? pixel_of_integral(I + m, w + 1) : 0.0f;
+                sts128(sx + i * 512, make_float4(e[0], e[1], e[2], e[3]));
+            }
+        }
+    }
+    float gin[kStripRows][kStrip];
+#pragma unroll
+    for (int i = 0; i < kStripRows; ++i)
 #pragma unroll
         for (int m = 0; m < kStrip; ++m) gin[i][m] = 0.0f;
-    }
     bool timed_out = false;
     for (int f = 0; f < F; ++f) {
         timed_out |= !mbar_wait(mbar32, f & 1);
@@ -356,7 +378,7 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ go_inte
             const uint32_t hi32 = stage32 + sh.stage_bytes - s.hi_first * row_bytes;
             const QuadCols cols = quad_cols(t, q0 >> 2, cells, cells);
             const QuadRows<kStripRows> q = quad_rows<kStripRows>(t, p0, h, lo32, hi32, row_bytes, lane);
-            auto xrow = [&](int i) { return make_float4(xv[i][0], xv[i][1], xv[i][2], xv[i][3]); };
+            auto xrow = [&](int i) { return lds128(sx + i * 512); };
             if (mine == kStripRows)
                 quad_backward_strip<kStripRows, NEED_PARAMS, true>(t, cols, q, col_weights(t), xrow, gin, sums, mine);
             else
@@ -403,15 +425,15 @@ inline SlabShape slab_shape(int h, int w)
     return s;
 }
 inline int slab_threads(const SlabShape &s) { return 32 * s.col_tiles * (s.R / kStripRows); }
-// (the table of boxes and the per-warp sums of up to 32 filters sit behind the stage)
+// (the table of boxes and the per-warp sums of up to 32 filters, then the slab's input values, sit behind the stage)
 inline size_t slab_smem(const SlabShape &s, int F, bool sums)
 {
     return 2 * (size_t)s.stage_bytes + (size_t)F * kTapWords * sizeof(float) +
-           (sums ? (size_t)F * (slab_threads(s) / 32) * kNumSums * sizeof(float) : 0);
+           (sums ? (size_t)F * (slab_threads(s) / 32) * kNumSums * sizeof(float) + 16 + (size_t)slab_threads(s) * kStripRows * 16 : 0);
 }
 
-template <typename IO>
-int integral_quad_t(const IO *in, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s)
+template <typename IO, bool QUAD>
+int integral_scan_t(const IO *in, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s)
 {
     const int warps = (w + 127) / 128;
     // few planes: clusters of up to 8 CTAs share one, as long as each keeps 16 rows
@@ -423,20 +445,20 @@ int integral_quad_t(const IO *in, float *out, int64_t planes, int h, int w, bool
     void (*kern)(const IO *, float *, int, int, int, int);
     constexpr int S = 128, L = 32 * kSlabMaxWarps;
     if (warps * 32 <= S) {
-        if (relu) kern = vec ? integral_quad_kernel<IO, true, true, S> : integral_quad_kernel<IO, false, true, S>;
-        else kern = vec ? integral_quad_kernel<IO, true, false, S> : integral_quad_kernel<IO, false, false, S>;
+        if (relu) kern = vec ? integral_scan_kernel<IO, true, true, QUAD, S> : integral_scan_kernel<IO, false, true, QUAD, S>;
+        else kern = vec ? integral_scan_kernel<IO, true, false, QUAD, S> : integral_scan_kernel<IO, false, false, QUAD, S>;
     } else {
-        if (relu) kern = vec ? integral_quad_kernel<IO, true, true, L> : integral_quad_kernel<IO, false, true, L>;
-        else kern = vec ? integral_quad_kernel<IO, true, false, L> : integral_quad_kernel<IO, false, false, L>;
+        if (relu) kern = vec ? integral_scan_kernel<IO, true, true, QUAD, L> : integral_scan_kernel<IO, false, true, QUAD, L>;
+        else kern = vec ? integral_scan_kernel<IO, true, false, QUAD, L> : integral_scan_kernel<IO, false, false, QUAD, L>;
     }
     {
         LaunchScope scope(KID_INTEGRAL, s);
         if (cudaError_t e = launch_overlapped_cluster(kern, (unsigned)(planes * cluster), warps * 32,
                                                       cluster > 1 ? warps * 32 * sizeof(float4) : 0, cluster, s, in, out, h, w, rows,
                                                       cluster))
-            return cuda_failed(e, "integral_quad");
+            return cuda_failed(e, "integral_scan");
     }
-    return check_launch("integral_quad");
+    return check_launch("integral_scan");
 }
 
 template <typename IO>
@@ -473,7 +495,7 @@ int forward_slab_t(const float *integ, const BoxParams &bp, const Fusion *fu, IO
 }
 
 template <typename IO>
-int backward_slab_t(const IO *x, const float *go_integ, const BoxParams &bp, float rep_h, float rep_w, int N, int C, int F, int h,
+int backward_slab_t(const IO *x, const float *x_integ, const float *go_integ, const BoxParams &bp, float rep_h, float rep_w, int N, int C, int F, int h,
                     int w, bool normalize, bool exact, int need_mask, IO *grad_input, void *grad_params, int grad_params_kind,
                     float *partials, cudaStream_t s)
 {
@@ -483,7 +505,7 @@ int backward_slab_t(const IO *x, const float *go_integ, const BoxParams &bp, flo
     const bool need_params = (need_mask & (BC_NEED_ALL & ~BC_NEED_INPUT)) != 0;
     const bool write_gin = (need_mask & BC_NEED_INPUT) != 0;
     const bool vec = w % 4 == 0 && aligned_to(x, Io<IO>::kVecBytes) && (!write_gin || aligned_to(grad_input, Io<IO>::kVecBytes));
-    void (*kern)(const IO *, const float *, BoxParams, IO *, float *, int, int, int, int, int, SlabShape, bool, bool, bool);
+    void (*kern)(const IO *, const float *, const float *, BoxParams, IO *, float *, int, int, int, int, int, SlabShape, bool, bool, bool);
     constexpr int S = 128, L = 32 * kSlabMaxWarps;
     if (slab_threads(sh) <= S) {
         if (need_params) kern = vec ? backward_slab_kernel<IO, true, true, S> : backward_slab_kernel<IO, false, true, S>;
@@ -496,7 +518,7 @@ int backward_slab_t(const IO *x, const float *go_integ, const BoxParams &bp, flo
     if (st != BC_OK) return st;
     {
         LaunchScope scope(KID_BACKWARD_SLAB, s);
-        if (cudaError_t e = launch_overlapped(kern, (unsigned)blocks, slab_threads(sh), slab_smem(sh, F, need_params), s, x, go_integ, bp, grad_input,
+        if (cudaError_t e = launch_overlapped(kern, (unsigned)blocks, slab_threads(sh), slab_smem(sh, F, need_params), s, x, x_integ, go_integ, bp, grad_input,
                                               partials, N, C, F, h, w, sh, normalize, exact, write_gin))
             return cuda_failed(e, "backward_slab");
     }
@@ -521,9 +543,14 @@ size_t slab_partials_bytes(int N, int C, int F, int h, int w)
 int launch_integral_quad(const void *in, int io_kind, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s)
 {
     if (planes == 0) return BC_OK;
-    if (io_kind == BC_IO_F16) return integral_quad_t(static_cast<const __half *>(in), out, planes, h, w, relu, s);
-    if (io_kind == BC_IO_BF16) return integral_quad_t(static_cast<const __nv_bfloat16 *>(in), out, planes, h, w, relu, s);
-    return integral_quad_t(static_cast<const float *>(in), out, planes, h, w, relu, s);
+    if (io_kind == BC_IO_F16) return integral_scan_t<__half, true>(static_cast<const __half *>(in), out, planes, h, w, relu, s);
+    if (io_kind == BC_IO_BF16) return integral_scan_t<__nv_bfloat16, true>(static_cast<const __nv_bfloat16 *>(in), out, planes, h, w, relu, s);
+    return integral_scan_t<float, true>(static_cast<const float *>(in), out, planes, h, w, relu, s);
+}
+
+int launch_integral_scan(const float *in, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s)
+{
+    return integral_scan_t<float, false>(in, out, planes, h, w, relu, s);
 }
 
 int launch_forward_slab(const float *integ, const BoxParams &bp, const Fusion *fu, void *out, int io_kind, int N, int C, int F,
@@ -535,17 +562,17 @@ int launch_forward_slab(const float *integ, const BoxParams &bp, const Fusion *f
     return forward_slab_t(integ, bp, fu, static_cast<float *>(out), N, C, F, h, w, normalize, exact, s);
 }
 
-int launch_backward_slab(const void *x, int io_kind, const float *go_integ, const BoxParams &bp, float rep_h, float rep_w, int N,
+int launch_backward_slab(const void *x, const float *x_integ, int io_kind, const float *go_integ, const BoxParams &bp, float rep_h, float rep_w, int N,
                          int C, int F, int h, int w, bool normalize, bool exact, int need_mask, void *grad_input, void *grad_params,
                          int grad_params_kind, float *partials, cudaStream_t s)
 {
     if (io_kind == BC_IO_F16)
-        return backward_slab_t(static_cast<const __half *>(x), go_integ, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask,
+        return backward_slab_t(static_cast<const __half *>(x), nullptr, go_integ, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask,
                                static_cast<__half *>(grad_input), grad_params, grad_params_kind, partials, s);
     if (io_kind == BC_IO_BF16)
-        return backward_slab_t(static_cast<const __nv_bfloat16 *>(x), go_integ, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact,
+        return backward_slab_t(static_cast<const __nv_bfloat16 *>(x), nullptr, go_integ, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact,
                                need_mask, static_cast<__nv_bfloat16 *>(grad_input), grad_params, grad_params_kind, partials, s);
-    return backward_slab_t(static_cast<const float *>(x), go_integ, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask,
+    return backward_slab_t(static_cast<const float *>(x), x_integ, go_integ, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask,
                            static_cast<float *>(grad_input), grad_params, grad_params_kind, partials, s);
 }
 

@@ -3,6 +3,7 @@
 #include <stdio.h>
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 #include <string.h>
 
@@ -91,6 +92,20 @@ static inline size_t integral_bytes(int64_t planes, int h, int w)
 
 
 
+// Backward of planes that do not fit in shared memory, by slabs (workspace already checked).
+static int backward_slabs(const void *input, const float *x_integ, int io_kind, const void *grad_output, const BoxParams &bp, float rep_h, float rep_w,
+                          int N, int C, int F, int h, int w, bool normalize, bool exact, int need_mask, void *grad_input,
+                          void *grad_params, int grad_params_kind, void *workspace, cudaStream_t stream)
+{
+    float *go_integ = static_cast<float *>(workspace);
+    float *partials = reinterpret_cast<float *>(static_cast<char *>(workspace) +
+                                                align_up(slab_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256));
+    int st = launch_integral_quad(grad_output, io_kind, go_integ, (int64_t)N * C * F, h, w, false, stream);
+    if (st != BC_OK) return st;
+    return launch_backward_slab(input, x_integ, io_kind, go_integ, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
+                                grad_params, grad_params_kind, partials, stream);
+}
+
 // ---- the four extension functions, for float and double ------------------------------------
 template <typename T>
 static size_t integral_bytes_t(int64_t planes, int h, int w)
@@ -116,6 +131,11 @@ static int forward_entry(const T *input_integrated, const T *x_min, const T *x_m
     if (any_empty(N, C, F, h, w)) return BC_OK;
     if (!input_integrated || !x_min || !x_max || !y_min || !y_max || !output) return BC_ERR_NULL_POINTER;
     const BoxParamsT<T> bp{x_min, x_max, y_min, y_max, T(1), T(1)};
+    if constexpr (std::is_same<T, float>::value) {
+        // a plane whose integral image fits in shared memory is gathered from there
+        if (plane_path_fits_forward(F, h, w))
+            return launch_forward_plane_integ(input_integrated, bp, output, N, C, F, h, w, normalize != 0, exact != 0, stream);
+    }
     return launch_forward_global<T>(input_integrated, bp, output, N, C, F, h, w, normalize != 0, exact != 0, stream);
 }
 
@@ -123,6 +143,12 @@ template <typename T>
 static size_t backward_workspace_entry(int N, int C, int F, int h, int w, int need_mask)
 {
     if (!sizes_ok(N, C, F, h, w) || any_empty(N, C, F, h, w) || !(need_mask & BC_NEED_ALL)) return 0;
+    if (std::is_same<T, float>::value) {
+        if (plane_path_fits_backward_integ(F, h, w)) return align_up((size_t)C * F * N * kNumSums * sizeof(float), 256);
+        if (slab_path_fits(F, h, w))
+            return align_up(slab_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256) +
+                   align_up(slab_partials_bytes(N, C, F, h, w), 256);
+    }
     return integral_bytes_t<T>((int64_t)N * C * F, h, w) +
            align_up(backward_partials_bytes(N, C, F, h, w, sizeof(T)), 256);
 }
@@ -156,12 +182,21 @@ static int backward_entry(const T *input_integrated, const T *x_min, const T *x_
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) ||
         workspace_bytes < backward_workspace_entry<T>(N, C, F, h, w, need_mask))
         return BC_ERR_WORKSPACE;
+    const BoxParamsT<T> bp{x_min, x_max, y_min, y_max, T(1), T(1)};
+    if constexpr (std::is_same<T, float>::value) {
+        if (plane_path_fits_backward_integ(F, h, w))
+            return launch_backward_plane_integ(input_integrated, grad_output, bp, reparametrization_h, reparametrization_w, N, C, F, h,
+                                               w, normalize != 0, exact != 0, need_mask, grad_input, grad_params,
+                                               static_cast<float *>(workspace), stream);
+        if (slab_path_fits(F, h, w))
+            return backward_slabs(nullptr, input_integrated, BC_IO_F32, grad_output, bp, reparametrization_h, reparametrization_w, N, C,
+                                  F, h, w, normalize != 0, exact != 0, need_mask, grad_input, grad_params, BC_IO_F32, workspace, stream);
+    }
     T *go_integ = static_cast<T *>(workspace);
     T *partials = reinterpret_cast<T *>(static_cast<char *>(workspace) + ib);
 
     int st = launch_integral_image<T>(grad_output, go_integ, (int64_t)N * C * F, h, w, stream);
     if (st != BC_OK) return st;
-    const BoxParamsT<T> bp{x_min, x_max, y_min, y_max, T(1), T(1)};
     return launch_backward_global<T>(nullptr, input_integrated, go_integ, bp, reparametrization_h,
                                      reparametrization_w, N, C, F, h, w, normalize != 0, exact != 0,
                                      need_mask, grad_input, grad_params, partials, stream);
@@ -405,20 +440,6 @@ size_t bc_boxconv2d_backward_workspace(int N, int C, int F, int h, int w, int ne
     return integral_bytes((int64_t)N * C * F, h, w) + align_up(backward_partials_bytes(N, C, F, h, w), 256);
 }
 
-// Backward of planes that do not fit in shared memory, by slabs (workspace already checked).
-static int backward_slabs(const void *input, int io_kind, const void *grad_output, const BoxParams &bp, float rep_h, float rep_w,
-                          int N, int C, int F, int h, int w, bool normalize, bool exact, int need_mask, void *grad_input,
-                          void *grad_params, int grad_params_kind, void *workspace, cudaStream_t stream)
-{
-    float *go_integ = static_cast<float *>(workspace);
-    float *partials = reinterpret_cast<float *>(static_cast<char *>(workspace) +
-                                                align_up(slab_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256));
-    int st = launch_integral_quad(grad_output, io_kind, go_integ, (int64_t)N * C * F, h, w, false, stream);
-    if (st != BC_OK) return st;
-    return launch_backward_slab(input, io_kind, go_integ, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
-                                grad_params, grad_params_kind, partials, stream);
-}
-
 int bc_boxconv2d_backward(const float *input, const float *x_min, const float *x_max,
                           const float *y_min, const float *y_max, const float *grad_output,
                           float reparametrization_h, float reparametrization_w, int N, int C,
@@ -455,7 +476,7 @@ int bc_boxconv2d_backward(const float *input, const float *x_min, const float *x
                                      F, h, w, normalize != 0, exact != 0, need_mask, grad_input,
                                      grad_params, static_cast<float *>(workspace), stream);
     if (slab_path_fits(F, h, w))
-        return backward_slabs(input, BC_IO_F32, grad_output, bp, reparametrization_h, reparametrization_w, N, C, F, h, w,
+        return backward_slabs(input, nullptr, BC_IO_F32, grad_output, bp, reparametrization_h, reparametrization_w, N, C, F, h, w,
                               normalize != 0, exact != 0, need_mask, grad_input, grad_params, BC_IO_F32, workspace, stream);
     float *go_integ = static_cast<float *>(workspace);
     float *partials = reinterpret_cast<float *>(static_cast<char *>(workspace) + ib);
@@ -568,7 +589,7 @@ static int backward_narrow(const void *input, int io_kind, const float *x_min, c
         return BC_ERR_WORKSPACE;
     const BoxParams bp{x_min, x_max, y_min, y_max, reparametrization_h, reparametrization_w};
     if (!plane)
-        return backward_slabs(input, io_kind, grad_output, bp, reparametrization_h, reparametrization_w, N, C, F, h, w,
+        return backward_slabs(input, nullptr, io_kind, grad_output, bp, reparametrization_h, reparametrization_w, N, C, F, h, w,
                               normalize != 0, exact != 0, need_mask, grad_input, grad_params, grad_params_kind, workspace, stream);
     return launch_backward_plane_narrow(input, grad_output, io_kind, bp, reparametrization_h, reparametrization_w, N, C,
                                         F, h, w, normalize != 0, exact != 0, need_mask, grad_input, grad_params,
