@@ -144,23 +144,58 @@ __device__ __forceinline__ int row_shift(const IO *row)
     return (int)(reinterpret_cast<uintptr_t>(row) / sizeof(IO)) & 3;
 }
 
-// Columns c .. c+3 of the row; zero from column w on, or when the row does not exist.
+// Eight rows are loaded at a time: first all loads (rows8_load), then, where the values are used, the moves
+// between lanes (rows8_get), so that the loads of all rows are in flight together.  The group that follows
+// lane 31's is loaded for row i by lane i.
+struct Rows8 {
+    float4 a[8], next;
+};
+// Rows row0, row0 + w, ...; those at or past `rows` do not exist and read as zero.
 template <typename IO, bool ALIGNED>
-__device__ __forceinline__ float4 load_row4(const IO *row, int c, int w, bool row_ok, int lane)
+__device__ __forceinline__ void rows8_load(Rows8 &g, const IO *row0, int w, int c, int rows, int lane)
 {
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (ALIGNED) return row_ok && c < w ? Io<IO>::load4(row + c) : zero;
-    const int k = row_shift(row);
-    float4 a = row_ok && c - k < w ? Io<IO>::load4(row + (c - k)) : zero;
+    if (ALIGNED) {
+        const IO *p = row0 + c;
+#pragma unroll
+        for (int i = 0; i < 8; ++i, p += w) g.a[i] = i < rows && c < w ? Io<IO>::load4(p) : zero;
+        return;
+    }
+    const int k0 = row_shift(row0);
+    const IO *p = row0 + c;
+#pragma unroll
+    for (int i = 0; i < 8; ++i, p += w) {
+        const int k = (k0 + i * w) & 3;
+        g.a[i] = i < rows && c - k < w ? Io<IO>::load4(p - k) : zero;
+    }
+    const int k = (k0 + lane * w) & 3, at = c - lane * 4 + 128 - k;
+    g.next = lane < rows && lane < 8 && k && at < w ? Io<IO>::load4(row0 + lane * w + at) : zero;
+}
+// Columns c .. c+3 of row i; zero from column w on.
+template <typename IO, bool ALIGNED>
+__device__ __forceinline__ float4 rows8_get(const Rows8 &g, const IO *row0, int w, int c, int lane, int i)
+{
+    float4 a = g.a[i];
+    if (ALIGNED) return a;
+    const int k = (row_shift(row0) + i * w) & 3;
     if (k) {
-        float4 n;      // the group that follows: the next lane's
-        n.x = __shfl_down_sync(0xffffffffu, a.x, 1);
-        n.y = k > 1 ? __shfl_down_sync(0xffffffffu, a.y, 1) : 0.f;
-        n.z = k > 2 ? __shfl_down_sync(0xffffffffu, a.z, 1) : 0.f;
-        if (lane == 31) n = row_ok && c + 4 - k < w ? Io<IO>::load4(row + (c + 4 - k)) : zero;
-        if (k == 1) a = make_float4(a.y, a.z, a.w, n.x);
-        else if (k == 2) a = make_float4(a.z, a.w, n.x, n.y);
-        else a = make_float4(a.w, n.x, n.y, n.z);
+        const unsigned full = 0xffffffffu;
+        float n0 = __shfl_down_sync(full, a.x, 1), n1 = 0.f, n2 = 0.f;
+        const float e0 = __shfl_sync(full, g.next.x, i);
+        if (lane == 31) n0 = e0;
+        if (k > 1) {
+            n1 = __shfl_down_sync(full, a.y, 1);
+            const float e1 = __shfl_sync(full, g.next.y, i);
+            if (lane == 31) n1 = e1;
+        }
+        if (k > 2) {
+            n2 = __shfl_down_sync(full, a.z, 1);
+            const float e2 = __shfl_sync(full, g.next.z, i);
+            if (lane == 31) n2 = e2;
+        }
+        if (k == 1) a = make_float4(a.y, a.z, a.w, n0);
+        else if (k == 2) a = make_float4(a.z, a.w, n0, n1);
+        else a = make_float4(a.w, n0, n1, n2);
     }
     if (c >= w) a.x = 0.f;
     if (c + 1 >= w) a.y = 0.f;

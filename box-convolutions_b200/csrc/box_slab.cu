@@ -20,7 +20,7 @@ namespace {
 constexpr int kSlabMaxWarps = 16;
 constexpr size_t kSlabMaxSmem = 200 * 1024;
 constexpr int kStripRows = 8;              // rows per warp
-constexpr int kScanRows = 8;               // rows a warp of the integral kernel keeps in registers
+constexpr int kScanRows = 8;               // rows a warp of the integral kernel works on at a time
 
 // ---- integral images ----------------------------------------------------------------------------
 // A CTA (one warp per 128 columns) walks down its rows: each lane keeps running column sums of its four
@@ -53,7 +53,7 @@ __device__ __forceinline__ void cluster_sync()
 
 // QUAD: rows in the quad layout; else plain rows of w + 1 floats, the public integral image.
 template <typename IO, bool VEC, bool RELU, bool QUAD, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 5 : 1)
+__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? (VEC ? 5 : 4) : 1)
 integral_scan_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, int w, int rows_per_cta, int cluster)
 {
     __shared__ __align__(16) float sTot[2][kSlabMaxWarps][kScanRows];
@@ -69,29 +69,26 @@ integral_scan_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, 
     float *dst = out + plane * (int64_t)(h + 1) * pitch;
 
     grid_dependency_wait();
-    float4 nxt[kScanRows];
-#pragma unroll
-    for (int i = 0; i < kScanRows; ++i) nxt[i] = load_row4<IO, VEC>(src + (int64_t)(r0 + i) * w, c, w, r0 + i < r1, lane);
+    Rows8 nxt;
+    const IO *from = src + (int64_t)r0 * w;
+    rows8_load<IO, VEC>(nxt, from, w, c, r1 - r0, lane);
 
     float run[4] = {0.f, 0.f, 0.f, 0.f};
     if (cluster > 1) {
         float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 v[kScanRows];
-#pragma unroll
-        for (int i = 0; i < kScanRows; ++i) v[i] = nxt[i];
+        Rows8 g = nxt;
+        const IO *at = from;
         for (int r = r0; r < r1; r += kScanRows) {
-            float4 ahead[kScanRows];
+            Rows8 ahead;
+            rows8_load<IO, VEC>(ahead, at + (int64_t)kScanRows * w, w, c, r1 - r - kScanRows, lane);
 #pragma unroll
             for (int i = 0; i < kScanRows; ++i) {
-                const int rn = r + kScanRows + i;
-                ahead[i] = load_row4<IO, VEC>(src + (int64_t)rn * w, c, w, rn < r1, lane);
+                float4 v = rows8_get<IO, VEC>(g, at, w, c, lane, i);
+                if (RELU) v = relu4(v);
+                sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
             }
-#pragma unroll
-            for (int i = 0; i < kScanRows; ++i) {
-                if (RELU) v[i] = relu4(v[i]);
-                sum.x += v[i].x; sum.y += v[i].y; sum.z += v[i].z; sum.w += v[i].w;
-                v[i] = ahead[i];
-            }
+            g = ahead;
+            at += (int64_t)kScanRows * w;
         }
         sCol[L] = sum;
         cluster_sync();
@@ -127,10 +124,11 @@ integral_scan_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, 
         float carry[kScanRows];
 #pragma unroll
         for (int i = 0; i < kScanRows; ++i) {
-            v[i] = RELU ? relu4(nxt[i]) : nxt[i];
-            const int rn = r + kScanRows + i;
-            nxt[i] = load_row4<IO, VEC>(src + (int64_t)rn * w, c, w, rn < r1, lane);
+            v[i] = rows8_get<IO, VEC>(nxt, from, w, c, lane, i);
+            if (RELU) v[i] = relu4(v[i]);
         }
+        from += (int64_t)kScanRows * w;
+        rows8_load<IO, VEC>(nxt, from, w, c, r1 - r - kScanRows, lane);
 #pragma unroll
         for (int i = 0; i < kScanRows; ++i) {
             run[0] += v[i].x; run[1] += v[i].y; run[2] += v[i].z; run[3] += v[i].w;
@@ -349,8 +347,10 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
     if (NEED_PARAMS) {
         if (x) {
             const IO *row = x + pix - q0;
+            Rows8 g;
+            rows8_load<IO, VEC>(g, row, w, q0, mine, lane);
 #pragma unroll
-            for (int i = 0; i < kStripRows; ++i) sts128(sx + i * 512, load_row4<IO, VEC>(row + (int64_t)i * w, q0, w, i < mine, lane));
+            for (int i = 0; i < kStripRows; ++i) sts128(sx + i * 512, rows8_get<IO, VEC>(g, row, w, q0, lane, i));
         } else {      // the caller has only the input's integral image: its pixels are second differences
             const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1) + (int64_t)p0 * (w + 1) + q0;
 #pragma unroll 1

@@ -11,11 +11,15 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
-#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
 
 #include <array>
+#include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 
@@ -373,12 +377,6 @@ Tensor clip(const Four &p, double rep_h, double rep_w, double max_h, double max_
 // float64 (gradient checks) chains the four functions, as the reference does.  16-bit tensors
 // outside what the 16-bit entry points serve (very wide planes, many filters) go through float32 copies.
 
-struct Saved : torch::CustomClassHolder {
-    double rep_h, rep_w;
-    bool normalize, exact;
-    at::ScalarType dtype;        // of the input as the caller passed it
-};
-
 // The forward of one call.  `keep` receives what backward needs, or is null when nothing will be
 // differentiated (then the parameters are read where they are, where the kernels can).
 struct Kept {
@@ -422,17 +420,17 @@ Tensor forward_any(const Tensor &input, const Four &p, const Options &o, Kept *k
     return out.scalar_type() == dtype ? out : out.to(dtype);
 }
 
-Gradients backward_any(const Tensor &x, const Tensor &params, Tensor grad_output, const Saved &a, int mask)
+Gradients backward_any(const Tensor &x, const Tensor &params, Tensor grad_output, const Options &a, at::ScalarType caller, int mask)
 {
     Gradients out;
     if (!mask) return out;
-    if (a.dtype == at::kDouble)
+    if (caller == at::kDouble)
         return box_backward(x, {params.select(0, 0), params.select(0, 1), params.select(0, 2), params.select(0, 3)}, grad_output,
                             a.rep_h, a.rep_w, a.normalize, a.exact, mask);
     const c10::cuda::CUDAGuard guard(x.device());
     const Sizes s{(int)x.size(0), (int)x.size(1), (int)params.size(2), (int)x.size(2), (int)x.size(3)};
     const at::ScalarType dtype = x.scalar_type();
-    if (is_narrow(a.dtype)) {
+    if (is_narrow(caller)) {
         if (grad_output.scalar_type() != dtype) grad_output = grad_output.to(dtype);
     } else {
         require_cuda_float(grad_output, "grad_output", at::kFloat);
@@ -457,44 +455,51 @@ Gradients backward_any(const Tensor &x, const Tensor &params, Tensor grad_output
                                        (float)a.rep_h, (float)a.rep_w, s.N, s.C, s.F, s.h, s.w, a.normalize, a.exact, mask,
                                        static_cast<float *>(gin), static_cast<float *>(gp), ws.data_ptr(), bytes, stream);
     check_status(status, "BoxConv2d backward");
-    if (dtype != a.dtype) {
-        if (out[0].defined()) out[0] = out[0].to(a.dtype);
-        if (gparams.defined()) gparams = gparams.to(a.dtype);
+    if (dtype != caller) {
+        if (out[0].defined()) out[0] = out[0].to(caller);
+        if (gparams.defined()) gparams = gparams.to(caller);
     }
     for (int i = 0; i < 4; ++i)
         if (mask & (BC_NEED_X_MIN << i)) out[1 + i] = slice_of(gparams, i);
     return out;
 }
 
-struct BoxConvolution : torch::autograd::Function<BoxConvolution> {
-    static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &input, const Tensor &x_min, const Tensor &x_max,
-                          const Tensor &y_min, const Tensor &y_max, const Options *o)
-    {
-        Kept keep;
-        Tensor out = forward_any(input, {x_min, x_max, y_min, y_max}, *o, &keep);
-        auto a = c10::make_intrusive<Saved>();
-        a->rep_h = o->rep_h; a->rep_w = o->rep_w;
-        a->normalize = o->normalize; a->exact = o->exact;
-        a->dtype = input.scalar_type();
-        ctx->saved_data["a"] = c10::IValue::make_capsule(std::move(a));
-        ctx->save_for_backward({keep.x, keep.params});
-        return out;
-    }
+// A plain autograd node: what torch::autograd::Function adds (a dictionary for the saved values, wrapping of the
+// outputs) takes longer than launching the kernels.
+struct BoxConvolutionBackward : torch::autograd::Node {
+    torch::autograd::SavedVariable x;
+    Tensor params;
+    Options options;
+    at::ScalarType caller;       // dtype of the input as the caller passed it
+    std::mutex mutex;
 
-    static torch::autograd::variable_list backward(torch::autograd::AutogradContext *ctx, torch::autograd::variable_list grads)
+    torch::autograd::variable_list apply(torch::autograd::variable_list &&grads) override
     {
-        const auto saved = ctx->get_saved_variables();
-        const auto target = ctx->saved_data["a"].toCapsule();
         int mask = 0;
         for (int i = 0; i < 5; ++i)
-            if (ctx->needs_input_grad(i)) mask |= 1 << i;
-        Gradients g = backward_any(saved[0], saved[1], grads[0], *static_cast<const Saved *>(target.get()), mask);
-        torch::autograd::variable_list list;
-        list.reserve(6);
-        for (Tensor &t : g) list.push_back(std::move(t));      // sole owner: a first accumulation takes the tensor itself
-        list.emplace_back();
+            if (task_should_compute_output(i)) mask |= 1 << i;
+        torch::autograd::variable_list list(5);
+        if (!grads[0].defined() || !mask) return list;
+        Tensor in, packed;
+        {
+            std::lock_guard<std::mutex> lock(mutex);
+            in = x.unpack();      // (checks that the input has not been changed in place and that the graph is still alive)
+            packed = params;
+        }
+        const at::NoGradGuard no_grad;
+        Gradients g = backward_any(in, packed, grads[0], options, caller, mask);
+        for (int i = 0; i < 5; ++i) list[i] = std::move(g[i]);      // sole owner: a first accumulation takes the tensor itself
         return list;
     }
+
+    void release_variables() override
+    {
+        std::lock_guard<std::mutex> lock(mutex);
+        x.reset_data();
+        params.reset();
+    }
+
+    std::string name() const override { return "BoxConvolutionBackward"; }
 };
 
 Tensor apply(const Tensor &input, const Four &p, const Options &o)
@@ -502,7 +507,21 @@ Tensor apply(const Tensor &input, const Four &p, const Options &o)
     const bool wanted = input.requires_grad() || p[0].requires_grad() || p[1].requires_grad() || p[2].requires_grad() ||
                         p[3].requires_grad();
     if (!wanted || !at::GradMode::is_enabled()) return forward_any(input, p, o, nullptr);
-    return BoxConvolution::apply(input, p[0], p[1], p[2], p[3], &o);
+    Kept keep;
+    Tensor out;
+    {
+        const at::NoGradGuard no_grad;
+        out = forward_any(input, p, o, &keep);
+    }
+    auto node = std::shared_ptr<BoxConvolutionBackward>(new BoxConvolutionBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(input, p[0], p[1], p[2], p[3]));
+    node->x = torch::autograd::SavedVariable(keep.x, false);
+    node->params = keep.params;
+    node->options = o;
+    node->options.snapshot = Tensor();
+    node->caller = input.scalar_type();
+    torch::autograd::set_history(out, node);
+    return out;
 }
 
 // ---- inference tail of one box block (inference.py documents the arguments)
