@@ -186,6 +186,21 @@ __device__ __forceinline__ void quad_store(QuadBlock &v, const QuadTile &t, cons
     }
 #pragma unroll
     for (int i = 0; i < kTileRows; ++i) { v.a[i] = add2(v.a[i], up_a); v.b[i] = add2(v.b[i], up_b); }
+    // Columns past w have to hold exactly what column w holds (a box border out there contributes nothing), but a
+    // lane's scan adds the row up in an order of its own: lanes past the plane take the value from the plane's last.
+    const bool edge = t.ct == CT - 1;
+    float last[kTileRows];
+    if (edge) {
+        const int from = ((w - 1) >> 2) & 31;
+        const bool past = t.c >= w;
+#pragma unroll
+        for (int i = 0; i < kTileRows; ++i) {
+            float z, u;
+            unpack2(v.b[i], z, u);
+            last[i] = __shfl_sync(0xffffffffu, u, from);
+            if (past) v.a[i] = v.b[i] = pack2(last[i], last[i]);
+        }
+    }
     // column c+1 of integral row p0+1: sub-row 1, cell c/4 + 1
     const uint32_t at = s.image + (t.p0 + 1) * Q::kRow + ((t.c >> 2) + 1) * 4;
     auto put = [&](auto I) {
@@ -204,15 +219,12 @@ __device__ __forceinline__ void quad_store(QuadBlock &v, const QuadTile &t, cons
     put(Index<4>{}); put(Index<5>{}); put(Index<6>{}); put(Index<7>{});
     // Cells of columns past the last lane's (planes whose width comes within eight columns of the tiles'): seven
     // words a row, one lane each.
-    if (t.ct == CT - 1 && (w >> 2) + 2 > 32 * CT) {
+    if (edge && (w >> 2) + 2 > 32 * CT) {
         const int sub = lane < 3 ? lane + 1 : lane - 3, cell = lane < 3 ? 32 * CT + 1 : 32 * CT + 2;
         const uint32_t extra = s.image + (t.p0 + 1) * Q::kRow + sub * Q::kSub + cell * 4;
         auto copy = [&](auto I) {
             constexpr int i = decltype(I)::value;
-            float z, u;
-            unpack2(v.b[i], z, u);
-            const float last = __shfl_sync(0xffffffffu, u, 31);
-            if (lane < 7 && (FULL || i < t.rows)) sts<i * Q::kRow>(extra, last);
+            if (lane < 7 && (FULL || i < t.rows)) sts<i * Q::kRow>(extra, last[i]);
         };
         copy(Index<0>{}); copy(Index<1>{}); copy(Index<2>{}); copy(Index<3>{});
         copy(Index<4>{}); copy(Index<5>{}); copy(Index<6>{}); copy(Index<7>{});

@@ -116,7 +116,7 @@ integral_scan_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, 
         if (cell < cells && (sub || cell > 32 * nwarps + 1)) extra_at = sub * cells + cell;
     }
     float *extra = row + extra_at;
-    const bool edge_warp = warp == 0 || warp == nwarps - 1;
+    const bool last_warp = warp == nwarps - 1, edge_warp = warp == 0 || last_warp;
 
     int buf = 0;
     for (int r = r0; r < r1; r += kScanRows) {
@@ -161,15 +161,20 @@ integral_scan_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, 
                     row += pitch;
                 }
             } else if (r + i < r1) {
-                const float x4 = v[i].w + carry[i];
+                float x4 = v[i].w + carry[i], add = carry[i];
+                float last = 0.0f;
+                if (last_warp) {
+                    // columns past w: exactly the value at w, which this lane's scan adds up in another order
+                    last = __shfl_sync(0xffffffffu, x4, ((w - 1) >> 2) & 31);
+                    if (c >= w) x4 = add = last;      // (v is zero there)
+                }
                 if (in123) {
-                    *d1 = v[i].x + carry[i];
-                    *d2 = v[i].y + carry[i];
-                    *d3 = v[i].z + carry[i];
+                    *d1 = v[i].x + add;
+                    *d2 = v[i].y + add;
+                    *d3 = v[i].z + add;
                 }
                 if (in0) *d0 = x4;
                 if (edge_warp) {
-                    const float last = __shfl_sync(0xffffffffu, x4, 31);
                     if (extra_at >= 0) *extra = zero ? 0.0f : last;
                     extra += pitch;
                 }
