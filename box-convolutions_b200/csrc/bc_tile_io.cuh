@@ -34,6 +34,13 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes
 {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
+// The same hint for memory of any alignment, spread over the CTA's threads.
+__device__ __forceinline__ void prefetch_l2(const void *p, size_t bytes)
+{
+    const char *c = static_cast<const char *>(p);
+    for (size_t at = (size_t)threadIdx.x * 128; at < bytes; at += (size_t)blockDim.x * 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(c + at));
+}
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity)
 {
     const long long t0 = clock64();
@@ -60,6 +67,8 @@ struct Io<float> {
     static constexpr int kVecBytes = 16;
     static __device__ __forceinline__ float4 load4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
     static __device__ __forceinline__ float load1(const float *p) { return __ldg(p); }
+    // for memory that this kernel may also write
+    static __device__ __forceinline__ float4 load4_plain(const float *p) { return *reinterpret_cast<const float4 *>(p); }
     static __device__ __forceinline__ void store4(float *p, float a, float b, float c, float d)
     {
         *reinterpret_cast<float4 *>(p) = make_float4(a, b, c, d);
@@ -150,15 +159,20 @@ __device__ __forceinline__ int row_shift(const IO *row)
 struct Rows8 {
     float4 a[8], next;
 };
-// Rows row0, row0 + w, ...; those at or past `rows` do not exist and read as zero.
-template <typename IO, bool ALIGNED>
+// Rows row0, row0 + w, ...; those at or past `rows` do not exist and read as zero.  PLAIN: the kernel may
+// write the rows later.
+template <typename IO, bool ALIGNED, bool PLAIN = false>
 __device__ __forceinline__ void rows8_load(Rows8 &g, const IO *row0, int w, int c, int rows, int lane)
 {
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto load = [](const IO *at) {
+        if constexpr (PLAIN) return Io<IO>::load4_plain(at);
+        else return Io<IO>::load4(at);
+    };
     if (ALIGNED) {
         const IO *p = row0 + c;
 #pragma unroll
-        for (int i = 0; i < 8; ++i, p += w) g.a[i] = i < rows && c < w ? Io<IO>::load4(p) : zero;
+        for (int i = 0; i < 8; ++i, p += w) g.a[i] = i < rows && c < w ? load(p) : zero;
         return;
     }
     const int k0 = row_shift(row0);
@@ -166,10 +180,10 @@ __device__ __forceinline__ void rows8_load(Rows8 &g, const IO *row0, int w, int 
 #pragma unroll
     for (int i = 0; i < 8; ++i, p += w) {
         const int k = (k0 + i * w) & 3;
-        g.a[i] = i < rows && c - k < w ? Io<IO>::load4(p - k) : zero;
+        g.a[i] = i < rows && c - k < w ? load(p - k) : zero;
     }
     const int k = (k0 + lane * w) & 3, at = c - lane * 4 + 128 - k;
-    g.next = lane < rows && lane < 8 && k && at < w ? Io<IO>::load4(row0 + lane * w + at) : zero;
+    g.next = lane < rows && lane < 8 && k && at < w ? load(row0 + lane * w + at) : zero;
 }
 // Columns c .. c+3 of row i; zero from column w on.
 template <typename IO, bool ALIGNED>

@@ -267,7 +267,7 @@ __device__ __forceinline__ Walk make_walk(uint32_t sI32, const BoxTaps &t, int q
 // FUSED: the inference steps of `Fusion` around the gather (the output may then alias the residual,
 // so it is not declared restrict).
 template <typename IO, int T, bool FAST, bool FUSED = false>
-__global__ void __launch_bounds__(T == 1 ? 256 : 512, T == 1 ? 4 : 1)
+__global__ void __launch_bounds__(T == 1 ? 256 : 512, T == 1 ? (FUSED ? 2 : 4) : 1)
 forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, BoxParams bp, IO *out, int C, int F,
                      int h, int w, int fsplit, bool normalize, bool exact, Fusion fu)
 {
@@ -288,6 +288,7 @@ forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, 
     const int cg = lane & 7, rg = lane >> 3;
 
     // a hint only: the plane on its way to L2 while this CTA still waits for the kernel in front
+    if (FUSED && fu.residual) prefetch_l2(fu.residual + (nc * F + f_begin) * (int64_t)h * w, (size_t)(f_end - f_begin) * h * w * sizeof(float));
     if (FAST && x && IsFloat<IO>::value && threadIdx.x == 0 && part == 0)
         bulk_prefetch_l2(x + nc * (int64_t)h * w, (uint32_t)(h * w) * 4u);
     Strip st[T];
@@ -335,6 +336,20 @@ forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, 
             load_pair(wk, st[k].p0 + t.lo_r - 1, st[k].p0 + t.hi_r, cw, prev);
             IO *dst = o + st[k].pix;
             const float *res = (FUSED && fu.residual) ? fu.residual + (nc * F + f) * (int64_t)h * w + st[k].pix : nullptr;
+            float4 skip[FUSED ? kR : 1];       // all residual rows in flight before the gather
+            if (FUSED && res) {
+#pragma unroll
+                for (int i = 0; i < kR; ++i, res += w) {
+                    if (FAST) {
+                        skip[FUSED ? i : 0] = *reinterpret_cast<const float4 *>(res);
+                    } else {
+                        const bool in = st[k].p0 + i < h;
+                        const int q = st[k].q0;
+                        skip[FUSED ? i : 0] = make_float4(in ? res[0] : 0.f, in && q + 1 < w ? res[1] : 0.f, in && q + 2 < w ? res[2] : 0.f,
+                                                          in && q + 3 < w ? res[3] : 0.f);
+                    }
+                }
+            }
 #pragma unroll
             for (int i = 0; i < kR; ++i) {
                 const int p = st[k].p0 + i;
@@ -357,15 +372,8 @@ forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, 
 #pragma unroll
                         for (int m = 0; m < kStrip; ++m) v[m] = v[m] * mul + add;
                         if (res) {
-                            if (FAST) {
-                                const float4 r = *reinterpret_cast<const float4 *>(res);
-                                v[0] += r.x; v[1] += r.y; v[2] += r.z; v[3] += r.w;
-                            } else {
-#pragma unroll
-                                for (int m = 0; m < kStrip; ++m)
-                                    if (st[k].q0 + m < w) v[m] += res[m];
-                            }
-                            res += w;
+                            const float4 r = skip[FUSED ? i : 0];
+                            v[0] += r.x; v[1] += r.y; v[2] += r.z; v[3] += r.w;
                         }
                         if (fu.output_relu) {
 #pragma unroll

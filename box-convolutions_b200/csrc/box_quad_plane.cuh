@@ -236,8 +236,11 @@ __device__ __forceinline__ void quad_store(QuadBlock &v, const QuadTile &t, cons
 // is loaded once per row and once more per task.
 // FAST: rows and tensors aligned for vector accesses, heights a multiple of 8.
 // A null `x`: `integ` holds the plane's integral image, plain rows of w + 1 floats, which is only copied.
+// FUSED: the inference steps of `Fusion` (the output may then alias the residual).  Such calls are single frames, a
+// few CTAs an SM at most: registers are there to have all residual rows of a task in flight before its gather,
+// and the planes travel to L2 while the CTA still waits for the kernel in front.
 template <typename IO, int CT, int T, bool FAST, bool FUSED, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 3 : 1)
+__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (FUSED ? 2 : 3) : 1)
 forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, BoxParams bp, IO *out, int C, int F, int h, int w, int row_tiles, int fsplit, int chunk,
                     bool normalize, bool exact, Fusion fu)
 {
@@ -252,6 +255,10 @@ forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
     const QuadSmem s = quad_smem(smem4, h, CT, ntiles, nwarps);
     float *sTaps = reinterpret_cast<float *>(reinterpret_cast<char *>(smem4) + (s.taps - s.image));
 
+    if (FUSED) {      // hints only
+        prefetch_l2(x + nc * npix, npix * sizeof(IO));
+        if (fu.residual) prefetch_l2(fu.residual + (nc * F + f_begin) * npix, (size_t)nf * npix * sizeof(float));
+    }
     quad_zero_padding<CT>(s.image, h);
     // registers and shared memory only up to here; now what the kernel in front of this one may have written
     grid_dependency_wait();
@@ -324,9 +331,11 @@ forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
         const int p_begin = g * chunk * kTileRows, p_end = min(p_begin + chunk * kTileRows, h);
         const int64_t first = (nc * F + f) * npix + (int64_t)p_begin * w;
         IO *row = out + first;
-        const float *res = FUSED && fu.residual ? fu.residual + first + q0 : nullptr;
+        const float *res = FUSED && fu.residual ? fu.residual + first : nullptr;
         f2_t prev[kStrip];
         for (int p0 = p_begin; p0 < p_end; p0 += kTileRows) {
+            Rows8 skip;
+            if (FUSED && res) rows8_load<float, FAST, true>(skip, res, w, q0, FAST ? kTileRows : p_end - p0, lane);
             const QuadRows<kTileRows> r = quad_rows<kTileRows>(t, p0, h, s.image, s.image, Q::kRow, lane);
             if (p0 == p_begin) quad_pair(cols, r.lo[0], r.hi[0], cw, prev);
 #pragma unroll
@@ -341,16 +350,9 @@ forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
                     if (FUSED) {
 #pragma unroll
                         for (int m = 0; m < kStrip; ++m) v[m] = v[m] * mul + add;
-                        if (res) {      // plain loads: the residual may be the output
-                            if (FAST) {
-                                const float4 e = q0 < w ? *reinterpret_cast<const float4 *>(res) : make_float4(0.f, 0.f, 0.f, 0.f);
-                                v[0] += e.x; v[1] += e.y; v[2] += e.z; v[3] += e.w;
-                            } else {
-#pragma unroll
-                                for (int m = 0; m < kStrip; ++m)
-                                    if (q0 + m < w) v[m] += res[m];
-                            }
-                            res += w;
+                        if (res) {
+                            const float4 e = rows8_get<float, FAST>(skip, res, w, q0, lane, i);
+                            v[0] += e.x; v[1] += e.y; v[2] += e.z; v[3] += e.w;
                         }
                         if (fu.output_relu) {
 #pragma unroll
@@ -361,6 +363,7 @@ forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
                     row += w;
                 }
             }
+            if (FUSED && res) res += kTileRows * w;
         }
     }
 }

@@ -214,7 +214,7 @@ __device__ __forceinline__ void slab_issue(const float *plane, int pitch, const 
 
 // FUSED: the inference steps of `Fusion` (the output may then alias the residual).
 template <typename IO, bool VEC, bool FUSED, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 6 : 1)
+__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? (FUSED ? 4 : 6) : 1)
 forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int C, int F, int h, int w, SlabShape sh, int fsplit,
                     bool normalize, bool exact, Fusion fu)
 {
@@ -236,6 +236,11 @@ forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int 
     if (threadIdx.x == 0) {
         mbar_init(mbar32, 2);
         fence_mbar_init();
+    }
+    if (FUSED && fu.residual) {      // hints only, while the integral images are still being written
+        const int64_t npix = (int64_t)h * w;
+        for (int f = f_begin; f < f_end; ++f)
+            prefetch_l2(fu.residual + (nc * F + f) * npix + (int64_t)p_slab * w, (size_t)rows * w * sizeof(float));
     }
     grid_dependency_wait();
     if ((int)threadIdx.x < nf) {
@@ -271,6 +276,9 @@ forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int 
                 if (fu.shift) add = __ldg(fu.shift + c * F + f);
             }
             int64_t off = (nc * F + f) * (int64_t)h * w + (int64_t)p0 * w + q0;
+            Rows8 skip;      // all residual rows in flight before the gather
+            const float *res = FUSED && fu.residual ? fu.residual + off - q0 : nullptr;
+            if (FUSED && res) rows8_load<float, VEC, true>(skip, res, w, q0, mine, lane);
             f2_t prev[kStrip];
             quad_pair(cols, q.lo[0], q.hi[0], cw, prev);
 #pragma unroll
@@ -284,10 +292,14 @@ forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int 
                     for (int m = 0; m < kStrip; ++m) prev[m] = cur[m];
                     if (FUSED) {
 #pragma unroll
-                        for (int m = 0; m < kStrip; ++m) {
-                            v[m] = v[m] * mul + add;
-                            if (fu.residual && q0 + m < w) v[m] += fu.residual[off + m];      // plain loads: may alias `out`
-                            if (fu.output_relu) v[m] = fmaxf(v[m], 0.0f);
+                        for (int m = 0; m < kStrip; ++m) v[m] = v[m] * mul + add;
+                        if (res) {
+                            const float4 e = rows8_get<float, VEC>(skip, res, w, q0, lane, i);
+                            v[0] += e.x; v[1] += e.y; v[2] += e.z; v[3] += e.w;
+                        }
+                        if (fu.output_relu) {
+#pragma unroll
+                            for (int m = 0; m < kStrip; ++m) v[m] = fmaxf(v[m], 0.0f);
                         }
                     }
                     store_row4<IO, VEC>(out + off - q0, q0, w, v, lane);
@@ -476,7 +488,7 @@ int forward_slab_t(const float *integ, const BoxParams &bp, const Fusion *fu, IO
     int fsplit = 1;
     while (fsplit < F && base * fsplit < 2 * 148) fsplit = fsplit * 2 < F ? fsplit * 2 : F;
     if (base * fsplit > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
-    const bool vec = w % 4 == 0 && aligned_to(out, Io<IO>::kVecBytes);
+    const bool vec = w % 4 == 0 && aligned_to(out, Io<IO>::kVecBytes) && (!fu || !fu->residual || aligned_to(fu->residual, 16));
     void (*kern)(const float *, BoxParams, IO *, int, int, int, int, SlabShape, int, bool, bool, Fusion);
     constexpr bool FU = IsFloat<IO>::value;
     constexpr int S = 128, L = 32 * kSlabMaxWarps;
