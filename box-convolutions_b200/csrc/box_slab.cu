@@ -20,169 +20,6 @@ namespace {
 constexpr int kSlabMaxWarps = 16;
 constexpr size_t kSlabMaxSmem = 200 * 1024;
 constexpr int kStripRows = 8;              // rows per warp
-constexpr int kScanRows = 8;               // rows a warp of the integral kernel works on at a time
-
-// ---- integral images ----------------------------------------------------------------------------
-// A CTA (one warp per 128 columns) walks down its rows: each lane keeps running column sums of its four
-// columns, scans eight rows at a time along the row (in the lane, across the warp by shuffles, across the
-// warps through shared memory, one barrier per eight rows) and stores them straight from registers; the next
-// eight rows are being loaded meanwhile.  No tile in shared memory, one pass over HBM.
-// With few planes a cluster of CTAs shares one: each first sums the columns of its rows, takes from the CTAs
-// above what they add to its columns (distributed shared memory), and then walks.
-__device__ __forceinline__ float4 relu4(float4 v)
-{
-    return make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
-}
-
-__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank)
-{
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ float4 cluster_load4(uint32_t addr)
-{
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-__device__ __forceinline__ void cluster_sync()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// QUAD: rows in the quad layout; else plain rows of w + 1 floats, the public integral image.
-template <typename IO, bool VEC, bool RELU, bool QUAD, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? (VEC ? 5 : 4) : 1)
-integral_scan_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, int w, int rows_per_cta, int cluster)
-{
-    __shared__ __align__(16) float sTot[2][kSlabMaxWarps][kScanRows];
-    extern __shared__ float4 sCol[];           // column sums of this CTA's rows (clusters only)
-    grid_dependency_release();
-    const int lane = threadIdx.x & 31, warp = uniform(threadIdx.x >> 5), nwarps = blockDim.x >> 5;
-    const int64_t plane = blockIdx.x / cluster;
-    const int rank = blockIdx.x % cluster;
-    const int L = threadIdx.x, c = L * 4;
-    const int cells = quad_cells(w), pitch = QUAD ? 4 * cells : w + 1;
-    const int r0 = min(rank * rows_per_cta, h), r1 = min(r0 + rows_per_cta, h);
-    const IO *src = in + plane * (int64_t)h * w;
-    float *dst = out + plane * (int64_t)(h + 1) * pitch;
-
-    grid_dependency_wait();
-    Rows8 nxt;
-    const IO *from = src + (int64_t)r0 * w;
-    rows8_load<IO, VEC>(nxt, from, w, c, r1 - r0, lane);
-
-    float run[4] = {0.f, 0.f, 0.f, 0.f};
-    if (cluster > 1) {
-        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-        Rows8 g = nxt;
-        const IO *at = from;
-        for (int r = r0; r < r1; r += kScanRows) {
-            Rows8 ahead;
-            rows8_load<IO, VEC>(ahead, at + (int64_t)kScanRows * w, w, c, r1 - r - kScanRows, lane);
-#pragma unroll
-            for (int i = 0; i < kScanRows; ++i) {
-                float4 v = rows8_get<IO, VEC>(g, at, w, c, lane, i);
-                if (RELU) v = relu4(v);
-                sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
-            }
-            g = ahead;
-            at += (int64_t)kScanRows * w;
-        }
-        sCol[L] = sum;
-        cluster_sync();
-        const uint32_t own = smem_u32(sCol) + L * 16;
-        for (int k = 0; k < rank; ++k) {
-            const float4 u = cluster_load4(cluster_map(own, k));
-            run[0] += u.x; run[1] += u.y; run[2] += u.z; run[3] += u.w;
-        }
-        cluster_sync();      // no CTA leaves while another still reads its sums
-    }
-
-    if (rank == 0)
-        for (int i = threadIdx.x; i < pitch; i += blockDim.x) dst[i] = 0.0f;      // the zero row on top
-    // Where this lane's columns c+1 .. c+4 go in a row.  Some lanes of the first and last warps also write one
-    // word of the constant zeros at the left, or of the copies of the last value behind the last warp's columns.
-    const int p123 = L + 1;
-    const bool in123 = p123 < cells, in0 = p123 + 1 < cells;
-    float *row = dst + (int64_t)(r0 + 1) * pitch;
-    float *d1 = row + cells + p123, *d2 = d1 + cells, *d3 = d2 + cells, *d0 = row + p123 + 1;
-    int extra_at = -1;
-    if (warp == 0 && lane < 5) extra_at = lane < 4 ? lane * cells : 1;
-    const bool zero = extra_at >= 0;
-    if (warp == nwarps - 1 && lane >= 8 && lane < 20) {
-        const int cell = 32 * nwarps + 1 + ((lane - 8) >> 2), sub = lane & 3;
-        if (cell < cells && (sub || cell > 32 * nwarps + 1)) extra_at = sub * cells + cell;
-    }
-    float *extra = row + extra_at;
-    const bool last_warp = warp == nwarps - 1, edge_warp = warp == 0 || last_warp;
-
-    int buf = 0;
-    for (int r = r0; r < r1; r += kScanRows) {
-        float4 v[kScanRows];
-        float carry[kScanRows];
-#pragma unroll
-        for (int i = 0; i < kScanRows; ++i) {
-            v[i] = rows8_get<IO, VEC>(nxt, from, w, c, lane, i);
-            if (RELU) v[i] = relu4(v[i]);
-        }
-        from += (int64_t)kScanRows * w;
-        rows8_load<IO, VEC>(nxt, from, w, c, r1 - r - kScanRows, lane);
-#pragma unroll
-        for (int i = 0; i < kScanRows; ++i) {
-            run[0] += v[i].x; run[1] += v[i].y; run[2] += v[i].z; run[3] += v[i].w;
-            v[i].x = run[0];
-            v[i].y = run[1] + v[i].x;
-            v[i].z = run[2] + v[i].y;
-            v[i].w = run[3] + v[i].z;
-            const float incl = warp_scan(v[i].w);
-            carry[i] = incl - v[i].w;
-            if (lane == 31) sTot[buf][warp][i] = incl;
-        }
-        if (nwarps > 1) {
-            __syncthreads();
-            for (int k = 0; k < warp; ++k) {
-#pragma unroll
-                for (int i = 0; i < kScanRows; i += 4) {
-                    const float4 a = *reinterpret_cast<const float4 *>(&sTot[buf][k][i]);
-                    carry[i] += a.x; carry[i + 1] += a.y; carry[i + 2] += a.z; carry[i + 3] += a.w;
-                }
-            }
-            buf ^= 1;
-        }
-#pragma unroll
-        for (int i = 0; i < kScanRows; ++i) {
-            if (!QUAD) {
-                if (r + i < r1) {
-                    const float o[4] = {v[i].x + carry[i], v[i].y + carry[i], v[i].z + carry[i], v[i].w + carry[i]};
-                    store_row4<float, false>(row + 1, c, w, o, lane);
-                    if (threadIdx.x == 0) *row = 0.0f;
-                    row += pitch;
-                }
-            } else if (r + i < r1) {
-                float x4 = v[i].w + carry[i], add = carry[i];
-                float last = 0.0f;
-                if (last_warp) {
-                    // columns past w: exactly the value at w, which this lane's scan adds up in another order
-                    last = __shfl_sync(0xffffffffu, x4, ((w - 1) >> 2) & 31);
-                    if (c >= w) x4 = add = last;      // (v is zero there)
-                }
-                if (in123) {
-                    *d1 = v[i].x + add;
-                    *d2 = v[i].y + add;
-                    *d3 = v[i].z + add;
-                }
-                if (in0) *d0 = x4;
-                if (edge_warp) {
-                    if (extra_at >= 0) *extra = zero ? 0.0f : last;
-                    extra += pitch;
-                }
-                d0 += pitch; d1 += pitch; d2 += pitch; d3 += pitch;
-            }
-        }
-    }
-}
 
 // ---- gathers --------------------------------------------------------------------------------------
 // The two runs of integral rows a slab needs for one filter, clamped to the plane.
@@ -449,35 +286,6 @@ inline size_t slab_smem(const SlabShape &s, int F, bool sums)
            (sums ? (size_t)F * (slab_threads(s) / 32) * kNumSums * sizeof(float) + 16 + (size_t)slab_threads(s) * kStripRows * 16 : 0);
 }
 
-template <typename IO, bool QUAD>
-int integral_scan_t(const IO *in, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s)
-{
-    const int warps = (w + 127) / 128;
-    // few planes: clusters of up to 8 CTAs share one, as long as each keeps 16 rows
-    int cluster = 1;
-    while (cluster < 8 && planes * cluster < 2 * 148 && h >= 32 * cluster) cluster *= 2;
-    const int rows = ((h + cluster - 1) / cluster + kScanRows - 1) / kScanRows * kScanRows;
-    const bool vec = w % 4 == 0 && aligned_to(in, Io<IO>::kVecBytes);
-    if (planes * cluster > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
-    void (*kern)(const IO *, float *, int, int, int, int);
-    constexpr int S = 128, L = 32 * kSlabMaxWarps;
-    if (warps * 32 <= S) {
-        if (relu) kern = vec ? integral_scan_kernel<IO, true, true, QUAD, S> : integral_scan_kernel<IO, false, true, QUAD, S>;
-        else kern = vec ? integral_scan_kernel<IO, true, false, QUAD, S> : integral_scan_kernel<IO, false, false, QUAD, S>;
-    } else {
-        if (relu) kern = vec ? integral_scan_kernel<IO, true, true, QUAD, L> : integral_scan_kernel<IO, false, true, QUAD, L>;
-        else kern = vec ? integral_scan_kernel<IO, true, false, QUAD, L> : integral_scan_kernel<IO, false, false, QUAD, L>;
-    }
-    {
-        LaunchScope scope(KID_INTEGRAL, s);
-        if (cudaError_t e = launch_overlapped_cluster(kern, (unsigned)(planes * cluster), warps * 32,
-                                                      cluster > 1 ? warps * 32 * sizeof(float4) : 0, cluster, s, in, out, h, w, rows,
-                                                      cluster))
-            return cuda_failed(e, "integral_scan");
-    }
-    return check_launch("integral_scan");
-}
-
 template <typename IO>
 int forward_slab_t(const float *integ, const BoxParams &bp, const Fusion *fu, IO *out, int N, int C, int F, int h, int w,
                    bool normalize, bool exact, cudaStream_t s)
@@ -555,19 +363,6 @@ size_t slab_integral_floats(int64_t planes, int h, int w) { return (size_t)plane
 size_t slab_partials_bytes(int N, int C, int F, int h, int w)
 {
     return (size_t)C * F * N * slab_shape(h, w).slabs * kNumSums * sizeof(float);
-}
-
-int launch_integral_quad(const void *in, int io_kind, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s)
-{
-    if (planes == 0) return BC_OK;
-    if (io_kind == BC_IO_F16) return integral_scan_t<__half, true>(static_cast<const __half *>(in), out, planes, h, w, relu, s);
-    if (io_kind == BC_IO_BF16) return integral_scan_t<__nv_bfloat16, true>(static_cast<const __nv_bfloat16 *>(in), out, planes, h, w, relu, s);
-    return integral_scan_t<float, true>(static_cast<const float *>(in), out, planes, h, w, relu, s);
-}
-
-int launch_integral_scan(const float *in, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s)
-{
-    return integral_scan_t<float, false>(in, out, planes, h, w, relu, s);
 }
 
 int launch_forward_slab(const float *integ, const BoxParams &bp, const Fusion *fu, void *out, int io_kind, int N, int C, int F,
