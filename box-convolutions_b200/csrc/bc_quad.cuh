@@ -29,13 +29,15 @@ __device__ __forceinline__ BoxTaps load_taps_uniform(const float *tab)
     return t;
 }
 
-// Inclusive sum over the warp; the shuffle's own predicate tells which lanes have somebody to add.
+// Inclusive sum over the warp, or over each group of LN lanes; the shuffle's own predicate tells which lanes have
+// somebody to add.
+template <int LN = 32>
 __device__ __forceinline__ float warp_scan(float v)
 {
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1)
-        asm volatile("{\n .reg .f32 u;\n .reg .pred p;\n shfl.sync.up.b32 u|p, %0, %1, 0, 0xffffffff;\n @p add.f32 %0, %0, u;\n}"
-                     : "+f"(v) : "r"(d));
+    for (int d = 1; d < LN; d <<= 1)
+        asm volatile("{\n .reg .f32 u;\n .reg .pred p;\n shfl.sync.up.b32 u|p, %0, %1, %2, 0xffffffff;\n @p add.f32 %0, %0, u;\n}"
+                     : "+f"(v) : "r"(d), "n"((32 - LN) << 8));
     return v;
 }
 

@@ -146,7 +146,8 @@ __device__ __forceinline__ float pixel_of_integral(const float *I, int pitch)
 // multiple of four start anywhere relative to a 4-element boundary; k, the same for the whole warp, is by how
 // many elements.  The memory access is then done on the aligned group that begins k elements earlier, one
 // vector access a lane, and the elements move k places between neighbouring lanes by shuffles.
-// All 32 lanes take part.  ALIGNED: k is zero for every row and w a multiple of four.
+// All 32 lanes take part.  LN < 32: the warp is cut into groups of LN lanes, each on rows of its own (8 rows, or a
+// multiple, apart), and c0 is 0; `lane` is then the lane within its group.  ALIGNED: k is zero for every row and w a multiple of four.
 template <typename IO>
 __device__ __forceinline__ int row_shift(const IO *row)
 {
@@ -161,7 +162,7 @@ struct Rows8 {
 };
 // Rows row0, row0 + w, ...; those at or past `rows` do not exist and read as zero.  PLAIN: the kernel may
 // write the rows later.
-template <typename IO, bool ALIGNED, bool PLAIN = false>
+template <typename IO, bool ALIGNED, bool PLAIN = false, int LN = 32>
 __device__ __forceinline__ void rows8_load(Rows8 &g, const IO *row0, int w, int c, int rows, int lane)
 {
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -182,11 +183,11 @@ __device__ __forceinline__ void rows8_load(Rows8 &g, const IO *row0, int w, int 
         const int k = (k0 + i * w) & 3;
         g.a[i] = i < rows && c - k < w ? load(p - k) : zero;
     }
-    const int k = (k0 + lane * w) & 3, at = c - lane * 4 + 128 - k;
+    const int k = (k0 + lane * w) & 3, at = c - lane * 4 + 4 * LN - k;
     g.next = lane < rows && lane < 8 && k && at < w ? load(row0 + lane * w + at) : zero;
 }
 // Columns c .. c+3 of row i; zero from column w on.
-template <typename IO, bool ALIGNED>
+template <typename IO, bool ALIGNED, int LN = 32>
 __device__ __forceinline__ float4 rows8_get(const Rows8 &g, const IO *row0, int w, int c, int lane, int i)
 {
     float4 a = g.a[i];
@@ -195,17 +196,17 @@ __device__ __forceinline__ float4 rows8_get(const Rows8 &g, const IO *row0, int 
     if (k) {
         const unsigned full = 0xffffffffu;
         float n0 = __shfl_down_sync(full, a.x, 1), n1 = 0.f, n2 = 0.f;
-        const float e0 = __shfl_sync(full, g.next.x, i);
-        if (lane == 31) n0 = e0;
+        const float e0 = __shfl_sync(full, g.next.x, i, LN);
+        if (lane == LN - 1) n0 = e0;
         if (k > 1) {
-            n1 = __shfl_down_sync(full, a.y, 1);
-            const float e1 = __shfl_sync(full, g.next.y, i);
-            if (lane == 31) n1 = e1;
+            n1 = __shfl_down_sync(full, a.y, 1, LN);
+            const float e1 = __shfl_sync(full, g.next.y, i, LN);
+            if (lane == LN - 1) n1 = e1;
         }
         if (k > 2) {
-            n2 = __shfl_down_sync(full, a.z, 1);
-            const float e2 = __shfl_sync(full, g.next.z, i);
-            if (lane == 31) n2 = e2;
+            n2 = __shfl_down_sync(full, a.z, 1, LN);
+            const float e2 = __shfl_sync(full, g.next.z, i, LN);
+            if (lane == LN - 1) n2 = e2;
         }
         if (k == 1) a = make_float4(a.y, a.z, a.w, n0);
         else if (k == 2) a = make_float4(a.z, a.w, n0, n1);
@@ -218,28 +219,30 @@ __device__ __forceinline__ float4 rows8_get(const Rows8 &g, const IO *row0, int 
     return a;
 }
 
-template <typename IO, bool ALIGNED>
-__device__ __forceinline__ void store_row4(IO *row, int c, int w, const float (&v)[4], int lane)
+// `ok`: the row exists.
+template <typename IO, bool ALIGNED, int LN = 32>
+__device__ __forceinline__ void store_row4(IO *row, int c, int w, const float (&v)[4], int lane, bool ok = true)
 {
     if (ALIGNED) {
-        if (c < w) Io<IO>::store4(row + c, v[0], v[1], v[2], v[3]);
+        if (ok && c < w) Io<IO>::store4(row + c, v[0], v[1], v[2], v[3]);
         return;
     }
     const int k = row_shift(row);
     float o[4] = {v[0], v[1], v[2], v[3]};
     if (k) {
-        const float p3 = __shfl_up_sync(0xffffffffu, v[3], 1);
-        const float p2 = k > 1 ? __shfl_up_sync(0xffffffffu, v[2], 1) : 0.f;
-        const float p1 = k > 2 ? __shfl_up_sync(0xffffffffu, v[1], 1) : 0.f;
+        const float p3 = __shfl_up_sync(0xffffffffu, v[3], 1, LN);
+        const float p2 = k > 1 ? __shfl_up_sync(0xffffffffu, v[2], 1, LN) : 0.f;
+        const float p1 = k > 2 ? __shfl_up_sync(0xffffffffu, v[1], 1, LN) : 0.f;
         if (k == 1) { o[3] = v[2]; o[2] = v[1]; o[1] = v[0]; o[0] = p3; }
         else if (k == 2) { o[3] = v[1]; o[2] = v[0]; o[1] = p3; o[0] = p2; }
         else { o[3] = v[0]; o[2] = p3; o[1] = p2; o[0] = p1; }
-        if (lane == 31) {      // its last k columns have no lane after them
+        if (ok && lane == LN - 1) {      // its last k columns have no lane after them
 #pragma unroll
             for (int m = 1; m < 4; ++m)
                 if (m >= 4 - k && c + m < w) Io<IO>::store1(row + c + m, v[m]);
         }
     }
+    if (!ok) return;
     const int first = lane == 0 ? c : c - k;      // lane 0 has no lane before it
     if (first == c - k && c - k + 4 <= w) {
         Io<IO>::store4(row + (c - k), o[0], o[1], o[2], o[3]);

@@ -678,9 +678,8 @@ inline bool plane_fits_backward_integ(int F, int h, int w)
            (quad_fits_backward(F, h, w) || plane_backward_smem_bytes(h, w, true, false, 4) <= kMaxSmem);
 }
 
-// Planes of more than 8 tiles of 32 x 32 occupy an SM alone in the backward kernel of this file, whose phases
-// then overlap with nothing.  Where they are wide enough for slabs, integral images in L2 and slabs are faster
-// ((16,16,4,96,160): 87 us against 97; (2,8,4,128,256): 29 against 67).
+// From the input's integral image, planes of more than 8 tiles of 32 x 32, which occupy an SM alone in the backward
+// kernel of this file, are better off as slabs where they are wide enough ((4,16,4,96,160): 36 us against 48).
 inline bool plane_prefers_slabs_backward(int F, int h, int w)
 {
     return w > 96 && warp_tiles(h, w) > 8 && !quad_fits_backward(F, h, w);

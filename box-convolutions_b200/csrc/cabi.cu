@@ -94,11 +94,8 @@ static inline size_t integral_bytes(int64_t planes, int h, int w)
 
 static size_t plane_partials_bytes(int N, int C, int F) { return align_up((size_t)C * F * N * kNumSums * sizeof(float), 256); }
 
-// Backward on the whole-plane kernels?  (They may hold the plane and slabs be faster all the same.)
-static bool plane_backward(int F, int h, int w)
-{
-    return plane_path_fits_backward(F, h, w) && !(plane_path_prefers_slabs_backward(F, h, w) && slab_path_fits(F, h, w));
-}
+// Backward from the input's integral image on the whole-plane kernels?  (They may hold the plane and slabs be
+// faster all the same.)
 static bool plane_backward_integ(int F, int h, int w)
 {
     return plane_path_fits_backward_integ(F, h, w) && !(plane_path_prefers_slabs_backward(F, h, w) && slab_path_fits(F, h, w));
@@ -112,7 +109,7 @@ static int backward_slabs(const void *input, const float *x_integ, int io_kind, 
     float *go_integ = static_cast<float *>(workspace);
     float *partials = reinterpret_cast<float *>(static_cast<char *>(workspace) +
                                                 align_up(slab_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256));
-    int st = launch_integral_quad(grad_output, io_kind, go_integ, (int64_t)N * C * F, h, w, false, stream);
+    int st = launch_integral_quad_ordered(grad_output, io_kind, go_integ, (int64_t)N * C * F, h, w, stream);
     if (st != BC_OK) return st;
     return launch_backward_slab(input, x_integ, io_kind, go_integ, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
                                 grad_params, grad_params_kind, partials, stream);
@@ -441,7 +438,7 @@ int bc_boxconv2d_forward_fused(const float *input, const float *x_min, const flo
 size_t bc_boxconv2d_backward_workspace(int N, int C, int F, int h, int w, int need_mask)
 {
     if (!sizes_ok(N, C, F, h, w) || any_empty(N, C, F, h, w) || !(need_mask & BC_NEED_ALL)) return 0;
-    if (plane_backward(F, h, w))
+    if (plane_path_fits_backward(F, h, w))
         return plane_partials_bytes(N, C, F);
     if (slab_path_fits(F, h, w))
         return align_up(slab_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256) +
@@ -452,13 +449,12 @@ size_t bc_boxconv2d_backward_workspace(int N, int C, int F, int h, int w, int ne
     return integral_bytes((int64_t)N * C * F, h, w) + align_up(backward_partials_bytes(N, C, F, h, w), 256);
 }
 
-// `plane`: on the whole-plane kernels (decided by the caller; the workspace must match)
-static int backward_float(const float *input, const float *x_min, const float *x_max,
+int bc_boxconv2d_backward(const float *input, const float *x_min, const float *x_max,
                           const float *y_min, const float *y_max, const float *grad_output,
                           float reparametrization_h, float reparametrization_w, int N, int C,
                           int F, int h, int w, int normalize, int exact, int need_mask,
                           float *grad_input, float *grad_params, void *workspace,
-                          size_t workspace_bytes, bool plane, bc_stream_t stream)
+                          size_t workspace_bytes, bc_stream_t stream)
 {
     if (!sizes_ok(N, C, F, h, w)) return BC_ERR_BAD_SHAPE;
     need_mask &= BC_NEED_ALL;
@@ -482,9 +478,9 @@ static int backward_float(const float *input, const float *x_min, const float *x
     const size_t ib = band ? align_up(band_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256)
                            : integral_bytes((int64_t)N * C * F, h, w);
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) ||
-        workspace_bytes < (plane ? plane_partials_bytes(N, C, F) : bc_boxconv2d_backward_workspace(N, C, F, h, w, need_mask)))
+        workspace_bytes < bc_boxconv2d_backward_workspace(N, C, F, h, w, need_mask))
         return BC_ERR_WORKSPACE;
-    if (plane)
+    if (plane_path_fits_backward(F, h, w))
         return launch_backward_plane(input, grad_output, bp, reparametrization_h, reparametrization_w, N, C,
                                      F, h, w, normalize != 0, exact != 0, need_mask, grad_input,
                                      grad_params, static_cast<float *>(workspace), stream);
@@ -505,19 +501,6 @@ static int backward_float(const float *input, const float *x_min, const float *x
     return launch_backward_global<float>(input, nullptr, go_integ, bp, reparametrization_h,
                                   reparametrization_w, N, C, F, h, w, normalize != 0, exact != 0,
                                   need_mask, grad_input, grad_params, partials, stream);
-}
-
-int bc_boxconv2d_backward(const float *input, const float *x_min, const float *x_max,
-                          const float *y_min, const float *y_max, const float *grad_output,
-                          float reparametrization_h, float reparametrization_w, int N, int C,
-                          int F, int h, int w, int normalize, int exact, int need_mask,
-                          float *grad_input, float *grad_params, void *workspace,
-                          size_t workspace_bytes, bc_stream_t stream)
-{
-    if (!sizes_ok(N, C, F, h, w)) return BC_ERR_BAD_SHAPE;
-    return backward_float(input, x_min, x_max, y_min, y_max, grad_output, reparametrization_h, reparametrization_w, N, C, F, h, w,
-                          normalize, exact, need_mask, grad_input, grad_params, workspace, workspace_bytes, plane_backward(F, h, w),
-                          stream);
 }
 
 // ---- float16 / bfloat16 tensors on the shared-memory kernels
@@ -542,7 +525,7 @@ int bc_boxconv2d_forward_narrow(const void *input, int io_kind, const float *x_m
 
 int bc_boxconv2d_narrow_all_supported(int F, int h, int w)
 {
-    return (F > 0 && h > 0 && w > 0 && ((plane_path_fits_forward(F, h, w) && plane_backward(F, h, w)) || slab_path_fits(F, h, w))) ? 1 : 0;
+    return (F > 0 && h > 0 && w > 0 && ((plane_path_fits_forward(F, h, w) && plane_path_fits_backward(F, h, w)) || slab_path_fits(F, h, w))) ? 1 : 0;
 }
 
 size_t bc_boxconv2d_narrow_workspace(int N, int C, int F, int h, int w, int need_mask)
@@ -550,7 +533,7 @@ size_t bc_boxconv2d_narrow_workspace(int N, int C, int F, int h, int w, int need
     if (!sizes_ok(N, C, F, h, w) || any_empty(N, C, F, h, w)) return 0;
     if (!(need_mask & BC_NEED_ALL))
         return plane_path_fits_forward(F, h, w) ? 0 : align_up(slab_integral_floats((int64_t)N * C, h, w) * sizeof(float), 256);
-    if (plane_backward(F, h, w)) return plane_partials_bytes(N, C, F);
+    if (plane_path_fits_backward(F, h, w)) return plane_partials_bytes(N, C, F);
     return align_up(slab_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256) +
            align_up(slab_partials_bytes(N, C, F, h, w), 256);
 }
@@ -606,7 +589,7 @@ static int backward_narrow(const void *input, int io_kind, const float *x_min, c
     if (!input || !x_min || !x_max || !y_min || !y_max || !grad_output) return BC_ERR_NULL_POINTER;
     if ((need_mask & BC_NEED_INPUT) && !grad_input) return BC_ERR_NULL_POINTER;
     if (need_params && !grad_params) return BC_ERR_NULL_POINTER;
-    const bool plane = plane_backward(F, h, w);
+    const bool plane = plane_path_fits_backward(F, h, w);
     if (!plane && !slab_path_fits(F, h, w)) return BC_ERR_UNSUPPORTED;
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) ||
         workspace_bytes < bc_boxconv2d_narrow_workspace(N, C, F, h, w, need_mask))
@@ -683,10 +666,7 @@ int bc_boxconv2d_backward_static(const float *input, const float *x_min, const f
                                  float *grad_input, float *grad_params, bc_stream_t stream)
 {
     if (!sizes_ok(N, C, F, h, w)) return BC_ERR_BAD_SHAPE;
-    // whole-plane kernels wherever they hold the plane: slabs, faster for some of those, need room for integral images
-    const bool plane = plane_path_fits_backward(F, h, w);
-    const bool nothing = any_empty(N, C, F, h, w) || !(need_mask & BC_NEED_ALL);
-    const size_t need = nothing ? 0 : plane ? plane_partials_bytes(N, C, F) : bc_boxconv2d_backward_workspace(N, C, F, h, w, need_mask);
+    const size_t need = bc_boxconv2d_backward_workspace(N, C, F, h, w, need_mask);
     if (need > BC_STATIC_SCRATCH_BYTES) {
         snprintf(g_last_error, sizeof(g_last_error),
                  "bc_boxconv2d_backward_static: this problem needs %zu bytes of scratch, the built-in array has %u",
@@ -696,8 +676,9 @@ int bc_boxconv2d_backward_static(const float *input, const float *x_min, const f
     int status = BC_OK;
     void *scratch = static_scratch_address(&status);
     if (!scratch) return status;
-    return backward_float(input, x_min, x_max, y_min, y_max, grad_output, reparametrization_h, reparametrization_w, N, C, F, h, w,
-                          normalize, exact, need_mask, grad_input, grad_params, scratch, BC_STATIC_SCRATCH_BYTES, plane, stream);
+    return bc_boxconv2d_backward(input, x_min, x_max, y_min, y_max, grad_output, reparametrization_h,
+                                 reparametrization_w, N, C, F, h, w, normalize, exact, need_mask,
+                                 grad_input, grad_params, scratch, BC_STATIC_SCRATCH_BYTES, stream);
 }
 
 uint64_t bc_launch_count(void) { return g_launches.load(); }

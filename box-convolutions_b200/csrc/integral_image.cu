@@ -15,9 +15,6 @@
 //                    128-bit stores apart from at most 3 scalar elements at either end.
 #include "bc_common.cuh"
 
-#ifndef SCAN_RULE
-#define SCAN_RULE (!lpad && h >= 1 && w >= 1 && w <= 2048)
-#endif
 namespace bc {
 
 namespace {
@@ -411,7 +408,7 @@ int launch_integral_image_f32(const float *in, float *out, int64_t planes, int h
 {
     if (planes == 0) return BC_OK;
     if (planes > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
-    if (SCAN_RULE) return launch_integral_scan(in, out, planes, h, w, relu_in, s);
+    if (!lpad && h >= 1 && w >= 1 && w <= 2048) return launch_integral_scan(in, out, planes, h, w, relu_in, s);
     const int pw = lpad + w + 1 + rpad;
     const bool vec4 = (w % 4 == 0) && ((reinterpret_cast<uintptr_t>(in) & 15) == 0);
     // A few tall planes (at most 64) cannot fill the GPU with one CTA each (a CTA walks down its plane tile by
