@@ -155,23 +155,31 @@ __device__ __forceinline__ float warp_sum5(const float (&v)[kNumSums], int lane)
 
 // One filter's contribution of a strip of R rows to grad-input and to the five sums.  `x(i)` gives the four
 // input values of row i; FULL: the strip has all its rows, else those at or past `rows` do not exist (x is zero there).
+// gin: (columns 0, 1) and (2, 3) of each row.
 // The column strips enter the sums weighted by u(j), what the rows of the box make of the input values next to
 // tap row j: sum_i x_i (row combination of e) = sum_j e(j) (w_a x_(j+1) + w_b x_j).
 template <int R, bool NEED_PARAMS, bool FULL, class XRow>
 __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const QuadCols &cols, const QuadRows<R> &q, const ColW2 &cw,
-                                                    XRow &&x, float (&gin)[R][kStrip], float (&sums)[kNumSums], int rows)
+                                                    XRow &&x, f2_t (&gin)[R][2], float (&sums)[kNumSums], int rows)
 {
     f2_t pd[kStrip];
+    const f2_t scale = pack2(t.scale, t.scale);
+    // gather value of one column from its two tap-row pairs and their difference
+    auto gather = [&](f2_t cur, f2_t prev, f2_t diff) {
+        float lo_new, hi_new, lo_old, hi_old, top, bot;
+        unpack2(cur, lo_new, hi_new);
+        unpack2(prev, lo_old, hi_old);
+        unpack2(diff, top, bot);
+        (void)hi_new; (void)lo_old;
+        return (hi_old - lo_new) + t.f_hi_r * bot + t.f_lo_r * top;
+    };
     if (NEED_PARAMS) {
         const f2_t wa = pack2(-t.f_lo_r, 1.0f - t.f_hi_r), wb = pack2(t.f_lo_r - 1.0f, t.f_hi_r);
-        f2_t topbot = pack2(0.f, 0.f), left = topbot, right = topbot;
-        float s_out = 0.f;
+        f2_t topbot = pack2(0.f, 0.f), left = topbot, right = topbot, out2 = topbot;
         f2_t el[kStrip], eh[kStrip], xx[kStrip];
         quad_pair_e(cols, q.lo[0], q.hi[0], cw, pd, el, eh);
-        {
-            const float4 e = x(0);
-            xx[0] = pack2(e.x, e.x); xx[1] = pack2(e.y, e.y); xx[2] = pack2(e.z, e.z); xx[3] = pack2(e.w, e.w);
-        }
+        float4 e = x(0);
+        xx[0] = pack2(e.x, e.x); xx[1] = pack2(e.y, e.y); xx[2] = pack2(e.z, e.z); xx[3] = pack2(e.w, e.w);
 #pragma unroll
         for (int m = 0; m < kStrip; ++m) {
             const f2_t u = mul2(wa, xx[m]);
@@ -181,10 +189,11 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
 #pragma unroll
         for (int i = 0; i < R; ++i) {
             if (FULL || i < rows) {
-                f2_t cd[kStrip], xn[kStrip];
+                f2_t cd[kStrip], xn[kStrip], dd[kStrip];
+                const f2_t x01 = pack2(e.x, e.y), x23 = pack2(e.z, e.w);
                 quad_pair_e(cols, q.lo[i + 1], q.hi[i + 1], cw, cd, el, eh);
                 if (i + 1 < R) {
-                    const float4 e = x(i + 1);
+                    e = x(i + 1);
                     xn[0] = pack2(e.x, e.x); xn[1] = pack2(e.y, e.y); xn[2] = pack2(e.z, e.z); xn[3] = pack2(e.w, e.w);
                 }
 #pragma unroll
@@ -193,24 +202,23 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
                     if (i + 1 < R) u = fma2(wa, xn[m], u);
                     left = fma2(u, el[m], left);
                     right = fma2(u, eh[m], right);
-                    const f2_t dd = sub2(cd[m], pd[m]);
-                    float lo_new, hi_new, lo_old, hi_old, top, bot, xv, xv2;
-                    unpack2(cd[m], lo_new, hi_new);
-                    unpack2(pd[m], lo_old, hi_old);
-                    unpack2(dd, top, bot);
-                    unpack2(xx[m], xv, xv2);
-                    const float g = (hi_old - lo_new) + t.f_hi_r * bot + t.f_lo_r * top;
-                    (void)hi_new; (void)lo_old; (void)xv2;
-                    topbot = fma2(xx[m], dd, topbot);
-                    s_out += xv * g;
-                    gin[i][m] += g * t.scale;
+                    dd[m] = sub2(cd[m], pd[m]);
+                    topbot = fma2(xx[m], dd[m], topbot);
+                }
+                const f2_t g01 = pack2(gather(cd[0], pd[0], dd[0]), gather(cd[1], pd[1], dd[1]));
+                const f2_t g23 = pack2(gather(cd[2], pd[2], dd[2]), gather(cd[3], pd[3], dd[3]));
+                out2 = fma2(x01, g01, fma2(x23, g23, out2));
+                gin[i][0] = fma2(g01, scale, gin[i][0]);
+                gin[i][1] = fma2(g23, scale, gin[i][1]);
+#pragma unroll
+                for (int m = 0; m < kStrip; ++m) {
                     pd[m] = cd[m];
                     if (i + 1 < R) xx[m] = xn[m];
                 }
             }
         }
         float a, b;
-        sums[0] = s_out;
+        unpack2(out2, a, b); sums[0] = a + b;
         unpack2(topbot, sums[1], sums[2]);
         unpack2(left, a, b); sums[3] = a + b;
         unpack2(right, a, b); sums[4] = a + b;
@@ -220,17 +228,15 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
         for (int i = 0; i < R; ++i) {
             if (FULL || i < rows) {
                 f2_t cd[kStrip];
+                float g[kStrip];
                 quad_pair(cols, q.lo[i + 1], q.hi[i + 1], cw, cd);
 #pragma unroll
                 for (int m = 0; m < kStrip; ++m) {
-                    float lo_new, hi_new, lo_old, hi_old, top, bot;
-                    unpack2(cd[m], lo_new, hi_new);
-                    unpack2(pd[m], lo_old, hi_old);
-                    unpack2(sub2(cd[m], pd[m]), top, bot);
-                    (void)hi_new; (void)lo_old;
-                    gin[i][m] += ((hi_old - lo_new) + t.f_hi_r * bot + t.f_lo_r * top) * t.scale;
+                    g[m] = gather(cd[m], pd[m], sub2(cd[m], pd[m]));
                     pd[m] = cd[m];
                 }
+                gin[i][0] = fma2(pack2(g[0], g[1]), scale, gin[i][0]);
+                gin[i][1] = fma2(pack2(g[2], g[3]), scale, gin[i][1]);
             }
         }
     }

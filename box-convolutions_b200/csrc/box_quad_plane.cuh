@@ -418,11 +418,9 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
         const Box box = load_box(bp, c * F + threadIdx.x);
         store_taps(sTaps + threadIdx.x * kTapWords, taps_mirrored(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
     }
-    float gin[kTileRows][kStrip];
+    f2_t gin[kTileRows][2];
 #pragma unroll
-    for (int i = 0; i < kTileRows; ++i)
-#pragma unroll
-        for (int m = 0; m < kStrip; ++m) gin[i][m] = 0.0f;
+    for (int i = 0; i < kTileRows; ++i) gin[i][0] = gin[i][1] = pack2(0.f, 0.f);
     for (int f = 0; f < F; ++f) {
         {
             QuadBlock v;
@@ -462,7 +460,12 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
         IO *row = grad_input + nc * npix + tile.p0 * w;
 #pragma unroll
         for (int i = 0; i < kTileRows; ++i, row += w)
-            if (FAST || i < tile.rows) store_row4<IO, FAST>(row, tile.c, w, gin[i], lane);
+            if (FAST || i < tile.rows) {
+                float v[kStrip];
+                unpack2(gin[i][0], v[0], v[1]);
+                unpack2(gin[i][1], v[2], v[3]);
+                store_row4<IO, FAST>(row, tile.c, w, v, lane);
+            }
     }
 }
 

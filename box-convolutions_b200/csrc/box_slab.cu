@@ -216,11 +216,9 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
             }
         }
     }
-    float gin[kStripRows][kStrip];
+    f2_t gin[kStripRows][2];
 #pragma unroll
-    for (int i = 0; i < kStripRows; ++i)
-#pragma unroll
-        for (int m = 0; m < kStrip; ++m) gin[i][m] = 0.0f;
+    for (int i = 0; i < kStripRows; ++i) gin[i][0] = gin[i][1] = pack2(0.f, 0.f);
     bool timed_out = false;
     for (int f = 0; f < F; ++f) {
         timed_out |= !mbar_wait(mbar32, f & 1);
@@ -264,7 +262,12 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
         IO *row = grad_input + pix - q0;
 #pragma unroll
         for (int i = 0; i < kStripRows; ++i, row += w)
-            if (i < mine) store_row4<IO, VEC>(row, q0, w, gin[i], lane);
+            if (i < mine) {
+                float v[kStrip];
+                unpack2(gin[i][0], v[0], v[1]);
+                unpack2(gin[i][1], v[2], v[3]);
+                store_row4<IO, VEC>(row, q0, w, v, lane);
+            }
     }
 }
 
