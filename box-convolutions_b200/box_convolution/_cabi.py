@@ -43,12 +43,12 @@ SIGNATURES = {
     "bc_boxconv2d_narrow_supported": (_i, [_i] * 3),
     "bc_boxconv2d_forward_narrow": (_i, [_vp, _i] + [_vp] * 4 + [_f, _f, _vp] + [_i] * 7 + [_vp]),
     "bc_boxconv2d_backward_narrow": (_i, [_vp, _i] + [_vp] * 5 + [_f, _f] + [_i] * 8 + [_vp, _vp, _vp, _sz, _vp]),
-    "bc_boxconv2d_backward_narrow_all": (_i, [_vp, _i] + [_vp] * 5 + [_f, _f] + [_i] * 8 + [_vp, _vp, _vp, _sz, _vp]),
+    "bc_boxconv2d_backward_any": (_i, [_vp, _i] + [_vp] * 5 + [_f, _f] + [_i] * 8 + [_vp, _vp, _vp, _sz, _vp, _vp]),
     "bc_boxconv2d_narrow_all_supported": (_i, [_i] * 3),
     "bc_boxconv2d_narrow_workspace": (_sz, [_i] * 6),
     "bc_boxconv2d_forward_narrow_all": (_i, [_vp, _i] + [_vp] * 4 + [_f, _f, _vp] + [_i] * 7 + [_vp, _sz, _vp]),
-    "bc_clip_parameters_narrow": (_i, [_vp] * 4 + [_i, _i, _d, _d, _d, _d, _i, _vp, _vp]),
-    "bc_pack_parameters": (_i, [_vp] * 4 + [_i, _i, _vp, _vp]),
+    "bc_clip_parameters_any": (_i, [_vp] * 4 + [_i, _i, _d, _d, _d, _d, _i, _vp, _vp, _i, _vp]),
+    "bc_pack_parameters": (_i, [_vp] * 4 + [_i, _i, _vp, _vp, _i, _vp]),
     "bc_boxconv2d_host_step_workspace": (_sz, [_i] * 6),
     "bc_boxconv2d_host_step": (_i, [_vp] * 9 + [_f, _f, _d, _d] + [_i] * 9 + [_vp, _sz, _vp, _vp, _vp]),
     "bc_launch_count": (ctypes.c_uint64, []),

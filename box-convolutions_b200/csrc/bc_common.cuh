@@ -15,6 +15,8 @@ template <typename T>
 struct BoxParamsT {
     const T *x_min, *x_max, *y_min, *y_max;
     T mul_h, mul_w;
+    // one per channel, zero between launches, or null: lets backward kernels finish the parameter gradients themselves
+    unsigned *counters = nullptr;
 };
 using BoxParams = BoxParamsT<float>;
 
@@ -132,12 +134,12 @@ int launch_backward_global(const T *x, const T *x_integ, const T *go_integ, cons
 
 template <typename S, typename T>
 int launch_clip(S *x_min, S *x_max, S *y_min, S *y_max, int count, double rep_h, double rep_w,
-                double max_h, double max_w, bool exact, cudaStream_t s, T *packed);
-// 16-bit parameters (io_kind: BC_IO_F16 / BC_IO_BF16), float copy
-int launch_clip_narrow(void *x_min, void *x_max, void *y_min, void *y_max, int io_kind, int count, double rep_h, double rep_w,
-                       double max_h, double max_w, bool exact, cudaStream_t s, float *packed);
+                double max_h, double max_w, bool exact, cudaStream_t s, T *packed, unsigned *zeroed = nullptr, int zeroed_count = 0);
+// parameters of type io_kind (BC_IO_*), float copy; `zeroed` (may be null) receives zeroed_count zeros
+int launch_clip_any(void *x_min, void *x_max, void *y_min, void *y_max, int io_kind, int count, double rep_h, double rep_w,
+                    double max_h, double max_w, bool exact, cudaStream_t s, float *packed, unsigned *zeroed, int zeroed_count);
 int launch_pack(const void *x_min, const void *x_max, const void *y_min, const void *y_max, int io_kind, int count, float *packed,
-                cudaStream_t s);
+                unsigned *zeroed, int zeroed_count, cudaStream_t s);
 
 // grad_params is stored as io_kind says when T is float (BC_IO_*), as T otherwise
 template <typename T>

@@ -8,10 +8,8 @@
 // (plane, tile); the block loops over the filters so that grad-input is accumulated in
 // registers and written once, and leaves five partial sums per filter that the finishing kernel
 // turns into the parameter gradients (no atomics: a fixed summation order, bit-reproducible).
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
-
 #include "bc_common.cuh"
+#include "bc_finish.cuh"
 #include "bc_walk.cuh"
 
 namespace bc {
@@ -275,28 +273,7 @@ __global__ void finish_param_grads_kernel(const T *__restrict__ partials, BoxPar
     const int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (k >= count) return;
-    const T *src = partials + (int64_t)k * per_box * kNumSums;
-    T acc[kNumSums] = {T(0), T(0), T(0), T(0), T(0)};
-    for (int i = lane; i < per_box; i += 32) {
-#pragma unroll
-        for (int j = 0; j < kNumSums; ++j) acc[j] += src[(int64_t)i * kNumSums + j];
-    }
-#pragma unroll
-    for (int j = 0; j < kNumSums; ++j) acc[j] = warp_sum(acc[j]);
-    if (lane == 0) {
-        const BoxT<T> box = load_box(bp, k);
-        const ParamSumsT<T> s = {acc[0], acc[1], acc[2], acc[3], acc[4]};
-        T g[4];
-        finish_param_grads(s, box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact, rep_h, rep_w, g);
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (need_mask & (BC_NEED_X_MIN << j)) {
-                const int64_t at = (int64_t)j * count + k;
-                if (io_kind == BC_IO_F16) static_cast<__half *>(grad_params)[at] = __float2half_rn((float)g[j]);
-                else if (io_kind == BC_IO_BF16) static_cast<__nv_bfloat16 *>(grad_params)[at] = __float2bfloat16_rn((float)g[j]);
-                else static_cast<T *>(grad_params)[at] = g[j];
-            }
-    }
+    finish_box<T>(partials, bp, k, count, per_box, normalize, exact, rep_h, rep_w, need_mask, grad_params, io_kind, lane);
 }
 
 template <typename T>

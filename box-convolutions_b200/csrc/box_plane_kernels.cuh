@@ -37,6 +37,7 @@
 // four bytes of HBM traffic.
 #pragma once
 #include "bc_common.cuh"
+#include "bc_finish.cuh"
 #include "bc_smem_walk.cuh"
 #include "bc_tile_io.cuh"
 #include "box_quad_plane.cuh"
@@ -407,7 +408,7 @@ template <typename IO, int T, bool FAST, bool STAGED, bool NEED_PARAMS, bool XSM
 __global__ void __launch_bounds__(512)
 backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const IO *__restrict__ grad_output, BoxParams bp,
                       IO *__restrict__ grad_input, float *__restrict__ partials, int N, int C, int F,
-                      int h, int w, bool normalize, bool exact, bool write_gin)
+                      int h, int w, bool normalize, bool exact, bool write_gin, Finish fin)
 {
     extern __shared__ float4 smem4[];
     const Geometry g = geometry(h, w);
@@ -642,6 +643,7 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
             }
         }
     }
+    if (NEED_PARAMS) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
 }
 
 // The limit is raised to its maximum once per kernel and device (it is a ceiling, not a reservation: what a
@@ -762,7 +764,7 @@ int launch_backward_plane_t(const IO *x, const float *x_integ, const IO *grad_ou
                         aligned_to(x, 16) && ((size_t)h * w * io) % 16 == 0 &&
                         (with_staging <= two_ctas || plane_backward_smem_bytes(h, w, need_params, false, io) > two_ctas);
     const size_t smem = plane_backward_smem_bytes(h, w, need_params && xsmem, staged, io);
-    void (*kern)(const IO *, const float *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, bool, bool, bool);
+    void (*kern)(const IO *, const float *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, bool, bool, bool, Finish);
     if (!xsmem) {
         if (fast) kern = T == 1 ? backward_plane_kernel<IO, 1, true, false, true, false> : backward_plane_kernel<IO, 2, true, false, true, false>;
         else kern = T == 1 ? backward_plane_kernel<IO, 1, false, false, true, false> : backward_plane_kernel<IO, 2, false, false, true, false>;
@@ -775,16 +777,17 @@ int launch_backward_plane_t(const IO *x, const float *x_integ, const IO *grad_ou
         kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, false, false, true> : backward_plane_kernel<IO, 1, false, false, false>)
                       : (need_params ? backward_plane_kernel<IO, 2, false, false, true> : backward_plane_kernel<IO, 2, false, false, false>);
     }
+    const Finish fin = finish_here(bp, need_params, planes, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w);
     int st = opt_in_smem(kern, smem);
     if (st != BC_OK) return st;
     {
         LaunchScope scope(KID_BACKWARD_PLANE, s);
         if (cudaError_t e = launch_overlapped(kern, (unsigned)planes, warps * 32, smem, s, x, x_integ, grad_output, bp, grad_input,
-                                              partials, N, C, F, h, w, normalize, exact, write_gin))
+                                              partials, N, C, F, h, w, normalize, exact, write_gin, fin))
             return cuda_failed(e, "backward_plane");
     }
     st = check_launch("backward_plane");
-    if (st != BC_OK || !need_params) return st;
+    if (st != BC_OK || !need_params || fin.total) return st;
     return launch_finish_param_grads<float>(partials, bp, C * F, N, normalize, exact, rep_h, rep_w, need_mask,
                                             grad_params, s, grad_params_kind);
 }

@@ -10,6 +10,7 @@
 // The gather is that of the slab kernels: five words of shared memory an output and side, no bank conflicts.
 #pragma once
 #include "bc_common.cuh"
+#include "bc_finish.cuh"
 #include "bc_quad.cuh"
 #include "bc_tile_io.cuh"
 
@@ -376,7 +377,7 @@ template <typename IO, int CT, bool FAST, bool NEED_PARAMS, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 2 : 1)
 backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const IO *__restrict__ grad_output, BoxParams bp, IO *__restrict__ grad_input,
                      float *__restrict__ partials, int N, int C, int F, int h, int w, int row_tiles, bool normalize, bool exact,
-                     bool write_gin)
+                     bool write_gin, Finish fin)
 {
     using Q = QuadImage<CT>;
     extern __shared__ float4 smem4[];
@@ -467,6 +468,7 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
                 store_row4<IO, FAST>(row, tile.c, w, v, lane);
             }
     }
+    if (NEED_PARAMS) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
 }
 
 inline int quad_row_tiles(int h) { return (h + kTileRows - 1) / kTileRows; }
@@ -557,7 +559,7 @@ int launch_backward_quad_t(const IO *x, const float *x_integ, const IO *grad_out
     const bool write_gin = (need_mask & BC_NEED_INPUT) != 0;
     const bool fast = w % 4 == 0 && h % kTileRows == 0 && ((size_t)h * w * sizeof(IO)) % 16 == 0 && aligned_to(x, Io<IO>::kVecBytes) &&
                      aligned_to(grad_output, 16) && (!write_gin || aligned_to(grad_input, Io<IO>::kVecBytes));
-    void (*kern)(const IO *, const float *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, int, bool, bool, bool);
+    void (*kern)(const IO *, const float *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, int, bool, bool, bool, Finish);
     auto pick = [&](auto ct) {
         constexpr int CT = decltype(ct)::value, S = 256, L = 512;
         if (tiles <= 8) {
@@ -570,16 +572,17 @@ int launch_backward_quad_t(const IO *x, const float *x_integ, const IO *grad_out
     };
     if (col_tiles == 1) pick(Index<1>{});
     else pick(Index<2>{});
+    const Finish fin = finish_here(bp, need_params, planes, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w);
     int st = raise_smem_limit(reinterpret_cast<const void *>(kern), (int)kQuadMaxSmem);
     if (st != BC_OK) return st;
     {
         LaunchScope scope(KID_BACKWARD_QUAD, s);
         if (cudaError_t e = launch_overlapped(kern, (unsigned)planes, tiles * 32, quad_backward_smem(F, h, w), s, x, x_integ, grad_output, bp,
-                                              grad_input, partials, N, C, F, h, w, row_tiles, normalize, exact, write_gin))
+                                              grad_input, partials, N, C, F, h, w, row_tiles, normalize, exact, write_gin, fin))
             return cuda_failed(e, "backward_quad");
     }
     st = check_launch("backward_quad");
-    if (st != BC_OK || !need_params) return st;
+    if (st != BC_OK || !need_params || fin.total) return st;
     return launch_finish_param_grads<float>(partials, bp, C * F, N, normalize, exact, rep_h, rep_w, need_mask, grad_params, s,
                                             grad_params_kind);
 }

@@ -10,6 +10,7 @@
 // output instead of 2.5, two copy instructions instead of thousands of 16-byte ones, and reads shared
 // memory with 5 (R+1)/R words an output instead of 8.
 #include "bc_common.cuh"
+#include "bc_finish.cuh"
 #include "bc_quad.cuh"
 #include "bc_tile_io.cuh"
 
@@ -159,7 +160,7 @@ template <typename IO, bool VEC, bool NEED_PARAMS, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1)
 backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const float *__restrict__ go_integ, BoxParams bp, IO *__restrict__ grad_input,
                      float *__restrict__ partials, int N, int C, int F, int h, int w, SlabShape sh, bool normalize, bool exact,
-                     bool write_gin)
+                     bool write_gin, Finish fin)
 {
     extern __shared__ __align__(128) unsigned char slab_stage[];
     __shared__ __align__(8) unsigned long long mbar;
@@ -269,6 +270,7 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
                 store_row4<IO, VEC>(row, q0, w, v, lane);
             }
     }
+    if (NEED_PARAMS) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
 }
 
 inline SlabShape slab_shape(int h, int w)
@@ -333,7 +335,7 @@ int backward_slab_t(const IO *x, const float *x_integ, const float *go_integ, co
     const bool need_params = (need_mask & (BC_NEED_ALL & ~BC_NEED_INPUT)) != 0;
     const bool write_gin = (need_mask & BC_NEED_INPUT) != 0;
     const bool vec = w % 4 == 0 && aligned_to(x, Io<IO>::kVecBytes) && (!write_gin || aligned_to(grad_input, Io<IO>::kVecBytes));
-    void (*kern)(const IO *, const float *, const float *, BoxParams, IO *, float *, int, int, int, int, int, SlabShape, bool, bool, bool);
+    void (*kern)(const IO *, const float *, const float *, BoxParams, IO *, float *, int, int, int, int, int, SlabShape, bool, bool, bool, Finish);
     constexpr int S = 128, L = 32 * kSlabMaxWarps;
     if (slab_threads(sh) <= S) {
         if (need_params) kern = vec ? backward_slab_kernel<IO, true, true, S> : backward_slab_kernel<IO, false, true, S>;
@@ -342,16 +344,17 @@ int backward_slab_t(const IO *x, const float *x_integ, const float *go_integ, co
         if (need_params) kern = vec ? backward_slab_kernel<IO, true, true, L> : backward_slab_kernel<IO, false, true, L>;
         else kern = vec ? backward_slab_kernel<IO, true, false, L> : backward_slab_kernel<IO, false, false, L>;
     }
+    const Finish fin = finish_here(bp, need_params, blocks, C, grad_params, grad_params_kind, need_mask, N * sh.slabs, rep_h, rep_w);
     int st = raise_smem_limit(reinterpret_cast<const void *>(kern), (int)kSlabMaxSmem);
     if (st != BC_OK) return st;
     {
         LaunchScope scope(KID_BACKWARD_SLAB, s);
         if (cudaError_t e = launch_overlapped(kern, (unsigned)blocks, slab_threads(sh), slab_smem(sh, F, need_params), s, x, x_integ, go_integ, bp, grad_input,
-                                              partials, N, C, F, h, w, sh, normalize, exact, write_gin))
+                                              partials, N, C, F, h, w, sh, normalize, exact, write_gin, fin))
             return cuda_failed(e, "backward_slab");
     }
     st = check_launch("backward_slab");
-    if (st != BC_OK || !need_params) return st;
+    if (st != BC_OK || !need_params || fin.total) return st;
     return launch_finish_param_grads<float>(partials, bp, C * F, N * sh.slabs, normalize, exact, rep_h, rep_w, need_mask,
                                             grad_params, s, grad_params_kind);
 }

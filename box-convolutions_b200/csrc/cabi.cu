@@ -341,25 +341,26 @@ int bc_clip_parameters_f64(double *x_min, double *x_max, double *y_min, double *
                               max_input_h, max_input_w, exact, stream);
 }
 
-int bc_clip_parameters_narrow(void *x_min, void *x_max, void *y_min, void *y_max, int io_kind, int count,
-                              double reparametrization_h, double reparametrization_w, double max_input_h,
-                              double max_input_w, int exact, float *packed_out, bc_stream_t stream)
+int bc_clip_parameters_any(void *x_min, void *x_max, void *y_min, void *y_max, int io_kind, int count,
+                           double reparametrization_h, double reparametrization_w, double max_input_h,
+                           double max_input_w, int exact, float *packed_out, unsigned *zeroed, int zeroed_count,
+                           bc_stream_t stream)
 {
-    if (count < 0) return BC_ERR_BAD_SHAPE;
+    if (count < 0 || zeroed_count < 0 || zeroed_count > count) return BC_ERR_BAD_SHAPE;
     if (count == 0) return BC_OK;
     if (!x_min || !x_max || !y_min || !y_max) return BC_ERR_NULL_POINTER;
     if (reparametrization_h == 0.0 || reparametrization_w == 0.0) return BC_ERR_BAD_SHAPE;
-    return launch_clip_narrow(x_min, x_max, y_min, y_max, io_kind, count, reparametrization_h, reparametrization_w,
-                              max_input_h, max_input_w, exact != 0, stream, packed_out);
+    return launch_clip_any(x_min, x_max, y_min, y_max, io_kind, count, reparametrization_h, reparametrization_w,
+                           max_input_h, max_input_w, exact != 0, stream, packed_out, zeroed, zeroed_count);
 }
 
 int bc_pack_parameters(const void *x_min, const void *x_max, const void *y_min, const void *y_max, int io_kind, int count,
-                       float *packed_out, bc_stream_t stream)
+                       float *packed_out, unsigned *zeroed, int zeroed_count, bc_stream_t stream)
 {
-    if (count < 0) return BC_ERR_BAD_SHAPE;
+    if (count < 0 || zeroed_count < 0 || zeroed_count > count) return BC_ERR_BAD_SHAPE;
     if (count == 0) return BC_OK;
     if (!x_min || !x_max || !y_min || !y_max || !packed_out) return BC_ERR_NULL_POINTER;
-    return launch_pack(x_min, x_max, y_min, y_max, io_kind, count, packed_out, stream);
+    return launch_pack(x_min, x_max, y_min, y_max, io_kind, count, packed_out, zeroed, zeroed_count, stream);
 }
 
 size_t bc_boxconv2d_forward_workspace(int N, int C, int F, int h, int w)
@@ -449,12 +450,12 @@ size_t bc_boxconv2d_backward_workspace(int N, int C, int F, int h, int w, int ne
     return integral_bytes((int64_t)N * C * F, h, w) + align_up(backward_partials_bytes(N, C, F, h, w), 256);
 }
 
-int bc_boxconv2d_backward(const float *input, const float *x_min, const float *x_max,
+static int backward_float(const float *input, const float *x_min, const float *x_max,
                           const float *y_min, const float *y_max, const float *grad_output,
                           float reparametrization_h, float reparametrization_w, int N, int C,
                           int F, int h, int w, int normalize, int exact, int need_mask,
                           float *grad_input, float *grad_params, void *workspace,
-                          size_t workspace_bytes, bc_stream_t stream)
+                          size_t workspace_bytes, unsigned *counters, bc_stream_t stream)
 {
     if (!sizes_ok(N, C, F, h, w)) return BC_ERR_BAD_SHAPE;
     need_mask &= BC_NEED_ALL;
@@ -473,7 +474,7 @@ int bc_boxconv2d_backward(const float *input, const float *x_min, const float *x
     if (!input || !x_min || !x_max || !y_min || !y_max || !grad_output) return BC_ERR_NULL_POINTER;
     if ((need_mask & BC_NEED_INPUT) && !grad_input) return BC_ERR_NULL_POINTER;
     if (need_params && !grad_params) return BC_ERR_NULL_POINTER;
-    const BoxParams bp{x_min, x_max, y_min, y_max, reparametrization_h, reparametrization_w};
+    const BoxParams bp{x_min, x_max, y_min, y_max, reparametrization_h, reparametrization_w, counters};
     const bool band = band_path_fits_backward(F, h, w);
     const size_t ib = band ? align_up(band_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256)
                            : integral_bytes((int64_t)N * C * F, h, w);
@@ -501,6 +502,17 @@ int bc_boxconv2d_backward(const float *input, const float *x_min, const float *x
     return launch_backward_global<float>(input, nullptr, go_integ, bp, reparametrization_h,
                                   reparametrization_w, N, C, F, h, w, normalize != 0, exact != 0,
                                   need_mask, grad_input, grad_params, partials, stream);
+}
+
+int bc_boxconv2d_backward(const float *input, const float *x_min, const float *x_max,
+                          const float *y_min, const float *y_max, const float *grad_output,
+                          float reparametrization_h, float reparametrization_w, int N, int C,
+                          int F, int h, int w, int normalize, int exact, int need_mask,
+                          float *grad_input, float *grad_params, void *workspace,
+                          size_t workspace_bytes, bc_stream_t stream)
+{
+    return backward_float(input, x_min, x_max, y_min, y_max, grad_output, reparametrization_h, reparametrization_w, N, C, F, h, w,
+                          normalize, exact, need_mask, grad_input, grad_params, workspace, workspace_bytes, nullptr, stream);
 }
 
 // ---- float16 / bfloat16 tensors on the shared-memory kernels
@@ -567,7 +579,7 @@ static int backward_narrow(const void *input, int io_kind, const float *x_min, c
                            float reparametrization_h, float reparametrization_w, int N, int C,
                            int F, int h, int w, int normalize, int exact, int need_mask,
                            void *grad_input, void *grad_params, int grad_params_kind, void *workspace,
-                           size_t workspace_bytes, bc_stream_t stream)
+                           size_t workspace_bytes, unsigned *counters, bc_stream_t stream)
 {
     if (!sizes_ok(N, C, F, h, w)) return BC_ERR_BAD_SHAPE;
     if (io_kind != BC_IO_F16 && io_kind != BC_IO_BF16) return BC_ERR_UNSUPPORTED;
@@ -594,7 +606,7 @@ static int backward_narrow(const void *input, int io_kind, const float *x_min, c
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) ||
         workspace_bytes < bc_boxconv2d_narrow_workspace(N, C, F, h, w, need_mask))
         return BC_ERR_WORKSPACE;
-    const BoxParams bp{x_min, x_max, y_min, y_max, reparametrization_h, reparametrization_w};
+    const BoxParams bp{x_min, x_max, y_min, y_max, reparametrization_h, reparametrization_w, counters};
     if (!plane)
         return backward_slabs(input, nullptr, io_kind, grad_output, bp, reparametrization_h, reparametrization_w, N, C, F, h, w,
                               normalize != 0, exact != 0, need_mask, grad_input, grad_params, grad_params_kind, workspace, stream);
@@ -612,19 +624,24 @@ int bc_boxconv2d_backward_narrow(const void *input, int io_kind, const float *x_
 {
     return backward_narrow(input, io_kind, x_min, x_max, y_min, y_max, grad_output, reparametrization_h, reparametrization_w,
                            N, C, F, h, w, normalize, exact, need_mask, grad_input, grad_params, BC_IO_F32, workspace,
-                           workspace_bytes, stream);
+                           workspace_bytes, nullptr, stream);
 }
 
-int bc_boxconv2d_backward_narrow_all(const void *input, int io_kind, const float *x_min, const float *x_max,
-                                     const float *y_min, const float *y_max, const void *grad_output,
-                                     float reparametrization_h, float reparametrization_w, int N, int C,
-                                     int F, int h, int w, int normalize, int exact, int need_mask,
-                                     void *grad_input, void *grad_params, void *workspace,
-                                     size_t workspace_bytes, bc_stream_t stream)
+int bc_boxconv2d_backward_any(const void *input, int io_kind, const float *x_min, const float *x_max,
+                              const float *y_min, const float *y_max, const void *grad_output,
+                              float reparametrization_h, float reparametrization_w, int N, int C,
+                              int F, int h, int w, int normalize, int exact, int need_mask,
+                              void *grad_input, void *grad_params, void *workspace,
+                              size_t workspace_bytes, unsigned *counters, bc_stream_t stream)
 {
+    if (io_kind == BC_IO_F32)
+        return backward_float(static_cast<const float *>(input), x_min, x_max, y_min, y_max, static_cast<const float *>(grad_output),
+                              reparametrization_h, reparametrization_w, N, C, F, h, w, normalize, exact, need_mask,
+                              static_cast<float *>(grad_input), static_cast<float *>(grad_params), workspace, workspace_bytes,
+                              counters, stream);
     return backward_narrow(input, io_kind, x_min, x_max, y_min, y_max, grad_output, reparametrization_h, reparametrization_w,
                            N, C, F, h, w, normalize, exact, need_mask, grad_input, grad_params, io_kind, workspace,
-                           workspace_bytes, stream);
+                           workspace_bytes, counters, stream);
 }
 
 // ---- backward pass on the library's own scratch array (see the header for who needs this)

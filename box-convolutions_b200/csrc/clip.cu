@@ -40,14 +40,15 @@ __device__ __forceinline__ void clip_pair(S *pmin, S *pmax, double inv_rep, doub
 
 // `packed` (may be null): a (4, count) copy of the clipped values in the order x_min, x_max, y_min,
 // y_max, written by the same threads: the snapshot of the parameters that a forward pass keeps for
-// its backward pass, without a launch of its own.
+// its backward pass, without a launch of its own.  `zeroed` (may be null): counters that the backward pass needs.
 template <typename S, typename T>
 __global__ void clip_kernel(S *x_min, S *x_max, S *y_min, S *y_max, int count,
                             double inv_rep_h, double inv_rep_w, double min_size, double max_h, double max_w,
-                            T *packed)
+                            T *packed, unsigned *zeroed, int zeroed_count)
 {
     grid_dependency_release();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (zeroed && i < zeroed_count) zeroed[i] = 0u;      // (zeroed_count is at most 2 * count)
     if (i < count) {
         clip_pair<S, T>(x_min + i, x_max + i, inv_rep_h, min_size, max_h);
         if (packed) { packed[i] = widen(x_min[i]); packed[count + i] = widen(x_max[i]); }
@@ -60,11 +61,13 @@ __global__ void clip_kernel(S *x_min, S *x_max, S *y_min, S *y_max, int count,
 
 // The copy alone, for calls that clip nothing.
 template <typename S>
-__global__ void pack_kernel(const S *x_min, const S *x_max, const S *y_min, const S *y_max, int count, float *packed)
+__global__ void pack_kernel(const S *x_min, const S *x_max, const S *y_min, const S *y_max, int count, float *packed,
+                            unsigned *zeroed, int zeroed_count)
 {
     grid_dependency_release();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
+    if (zeroed && i < zeroed_count) zeroed[i] = 0u;      // (at most count)
     packed[i] = widen(x_min[i]);
     packed[count + i] = widen(x_max[i]);
     packed[2 * count + i] = widen(y_min[i]);
@@ -75,7 +78,7 @@ __global__ void pack_kernel(const S *x_min, const S *x_max, const S *y_min, cons
 
 template <typename S, typename T>
 int launch_clip(S *x_min, S *x_max, S *y_min, S *y_max, int count, double rep_h,
-                double rep_w, double max_h, double max_w, bool exact, cudaStream_t s, T *packed)
+                double rep_w, double max_h, double max_w, bool exact, cudaStream_t s, T *packed, unsigned *zeroed, int zeroed_count)
 {
     if (count == 0) return BC_OK;
     // minimum sizes are single-precision constants in the reference (interface.cpp:405-406)
@@ -85,46 +88,50 @@ int launch_clip(S *x_min, S *x_max, S *y_min, S *y_max, int count, double rep_h,
     {
         LaunchScope scope(KID_CLIP, s);
         clip_kernel<S, T><<<blocks, threads, 0, s>>>(x_min, x_max, y_min, y_max, count, 1.0 / rep_h, 1.0 / rep_w,
-                                                     min_size, max_h, max_w, packed);
+                                                     min_size, max_h, max_w, packed, zeroed, zeroed_count);
     }
     return check_launch("clip_parameters");
 }
 
 template int launch_clip<float, float>(float *, float *, float *, float *, int, double, double, double, double, bool, cudaStream_t,
-                                       float *);
+                                       float *, unsigned *, int);
 template int launch_clip<double, double>(double *, double *, double *, double *, int, double, double, double, double, bool,
-                                         cudaStream_t, double *);
+                                         cudaStream_t, double *, unsigned *, int);
 
-int launch_clip_narrow(void *x_min, void *x_max, void *y_min, void *y_max, int io_kind, int count, double rep_h, double rep_w,
-                       double max_h, double max_w, bool exact, cudaStream_t s, float *packed)
+template <typename S>
+static int clip_as(void *x_min, void *x_max, void *y_min, void *y_max, int count, double rep_h, double rep_w, double max_h, double max_w,
+                   bool exact, cudaStream_t s, float *packed, unsigned *zeroed, int zeroed_count)
 {
-    if (io_kind == BC_IO_F16)
-        return launch_clip<__half, float>(static_cast<__half *>(x_min), static_cast<__half *>(x_max), static_cast<__half *>(y_min),
-                                          static_cast<__half *>(y_max), count, rep_h, rep_w, max_h, max_w, exact, s, packed);
-    if (io_kind == BC_IO_BF16)
-        return launch_clip<__nv_bfloat16, float>(static_cast<__nv_bfloat16 *>(x_min), static_cast<__nv_bfloat16 *>(x_max),
-                                                 static_cast<__nv_bfloat16 *>(y_min), static_cast<__nv_bfloat16 *>(y_max), count,
-                                                 rep_h, rep_w, max_h, max_w, exact, s, packed);
-    return BC_ERR_UNSUPPORTED;
+    return launch_clip<S, float>(static_cast<S *>(x_min), static_cast<S *>(x_max), static_cast<S *>(y_min), static_cast<S *>(y_max), count,
+                                 rep_h, rep_w, max_h, max_w, exact, s, packed, zeroed, zeroed_count);
+}
+
+int launch_clip_any(void *x_min, void *x_max, void *y_min, void *y_max, int io_kind, int count, double rep_h, double rep_w,
+                    double max_h, double max_w, bool exact, cudaStream_t s, float *packed, unsigned *zeroed, int zeroed_count)
+{
+    auto fn = io_kind == BC_IO_F32 ? clip_as<float> : io_kind == BC_IO_F16 ? clip_as<__half> : io_kind == BC_IO_BF16 ? clip_as<__nv_bfloat16> : nullptr;
+    if (!fn) return BC_ERR_UNSUPPORTED;
+    return fn(x_min, x_max, y_min, y_max, count, rep_h, rep_w, max_h, max_w, exact, s, packed, zeroed, zeroed_count);
 }
 
 template <typename S>
 static void pack_as(const void *x_min, const void *x_max, const void *y_min, const void *y_max, int count, float *packed,
-                    cudaStream_t s)
+                    unsigned *zeroed, int zeroed_count, cudaStream_t s)
 {
     pack_kernel<S><<<(count + 127) / 128, 128, 0, s>>>(static_cast<const S *>(x_min), static_cast<const S *>(x_max),
-                                                       static_cast<const S *>(y_min), static_cast<const S *>(y_max), count, packed);
+                                                       static_cast<const S *>(y_min), static_cast<const S *>(y_max), count, packed, zeroed,
+                                                       zeroed_count);
 }
 
 int launch_pack(const void *x_min, const void *x_max, const void *y_min, const void *y_max, int io_kind, int count, float *packed,
-                cudaStream_t s)
+                unsigned *zeroed, int zeroed_count, cudaStream_t s)
 {
     if (count == 0) return BC_OK;
     {
         LaunchScope scope(KID_CLIP, s);
-        if (io_kind == BC_IO_F32) pack_as<float>(x_min, x_max, y_min, y_max, count, packed, s);
-        else if (io_kind == BC_IO_F16) pack_as<__half>(x_min, x_max, y_min, y_max, count, packed, s);
-        else if (io_kind == BC_IO_BF16) pack_as<__nv_bfloat16>(x_min, x_max, y_min, y_max, count, packed, s);
+        if (io_kind == BC_IO_F32) pack_as<float>(x_min, x_max, y_min, y_max, count, packed, zeroed, zeroed_count, s);
+        else if (io_kind == BC_IO_F16) pack_as<__half>(x_min, x_max, y_min, y_max, count, packed, zeroed, zeroed_count, s);
+        else if (io_kind == BC_IO_BF16) pack_as<__nv_bfloat16>(x_min, x_max, y_min, y_max, count, packed, zeroed, zeroed_count, s);
         else return BC_ERR_UNSUPPORTED;
     }
     return check_launch("pack_parameters");

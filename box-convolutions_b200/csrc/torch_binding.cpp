@@ -108,6 +108,7 @@ struct Options {
     double rep_h, rep_w;
     bool normalize, exact;
     Tensor snapshot;         // packed (4, C, F) float32 copy of the parameters, or undefined
+    unsigned *counters = nullptr;      // that go with it, or null
 };
 
 // Checks of the module's forward; the parameters must have the input's dtype.
@@ -132,16 +133,35 @@ Sizes check_forward(const Tensor &input, const Four &p)
     return {to_int(input.size(0)), to_int(input.size(1)), to_int(p[0].size(1)), to_int(input.size(2)), to_int(input.size(3))};
 }
 
+// A packed float32 copy of the parameters, (4, C, F), with C counters behind it that are zero whenever no kernel
+// of its backward pass is running.
+struct Snapshot {
+    Tensor packed;
+    unsigned *counters = nullptr;      // in packed's storage
+};
+Snapshot new_snapshot(at::IntArrayRef sizes, const Tensor &like)
+{
+    const int64_t n = c10::multiply_integers(sizes), rows = sizes.empty() ? 0 : sizes[0];
+    Snapshot s;
+    s.packed = new_tensor({4 * n + rows}, at::kFloat, like);
+    s.counters = reinterpret_cast<unsigned *>(s.packed.data_ptr<float>() + 4 * n);
+    std::vector<int64_t> shape{4};
+    shape.insert(shape.end(), sizes.begin(), sizes.end());
+    s.packed.unsafeGetTensorImpl()->set_sizes_contiguous(shape);
+    return s;
+}
+
 // Packed float32 copy of the parameters as they are now, in one launch.
-Tensor pack_parameters(const Four &p, const Sizes &s, bc_stream_t stream)
+Snapshot pack_parameters(const Four &p, const Sizes &s, bc_stream_t stream)
 {
     Four q;
     for (int i = 0; i < 4; ++i) q[i] = p[i].contiguous();
-    Tensor packed = new_tensor({4, s.C, s.F}, at::kFloat, p[0]);
+    Snapshot snap = new_snapshot({s.C, s.F}, p[0]);
     check_status(bc_pack_parameters(q[0].const_data_ptr(), q[1].const_data_ptr(), q[2].const_data_ptr(), q[3].const_data_ptr(),
-                                    io_kind(p[0].scalar_type()), s.C * s.F, packed.data_ptr<float>(), stream),
+                                    io_kind(p[0].scalar_type()), s.C * s.F, snap.packed.data_ptr<float>(), snap.counters,
+                                    snap.counters ? s.C : 0, stream),
                  "BoxConv2d forward");
-    return packed;
+    return snap;
 }
 
 // The kernels' view of the four parameter arrays: slices of a packed copy, or four tensors.
@@ -314,7 +334,7 @@ Gradients box_backward(const Tensor &integrated, Four p, const Tensor &grad_outp
 }
 
 // In place; `packed` (float32 and narrower): also returns a packed float32 copy of the clipped values.
-Tensor clip(const Four &p, double rep_h, double rep_w, double max_h, double max_w, bool exact, bool packed)
+Snapshot clip(const Four &p, double rep_h, double rep_w, double max_h, double max_w, bool exact, bool packed)
 {
     const at::ScalarType dtype = p[0].scalar_type();
     for (int i = 0; i < 4; ++i) {
@@ -331,7 +351,7 @@ Tensor clip(const Four &p, double rep_h, double rep_w, double max_h, double max_
         clip(dense, rep_h, rep_w, max_h, max_w, exact, false);
         at::NoGradGuard no_grad;
         for (int i = 0; i < 4; ++i) p[i].copy_(dense[i]);
-        return Tensor();
+        return {};
     }
     for (int i = 0; i < 4; ++i)
         if (!p[i].is_contiguous()) fail(std::string(kParamNames[i]) + " must be contiguous");
@@ -343,26 +363,15 @@ Tensor clip(const Four &p, double rep_h, double rep_w, double max_h, double max_
     void *q[4];
     for (int i = 0; i < 4; ++i) q[i] = p[i].data_ptr();
     int status;
-    Tensor out;
+    Snapshot out;
     if (dtype == at::kDouble) {
         status = bc_clip_parameters_f64((double *)q[0], (double *)q[1], (double *)q[2], (double *)q[3], count, rep_h, rep_w, max_h,
                                         max_w, exact, stream);
     } else {
-        if (packed) {
-            auto sizes = p[0].sizes().vec();
-            sizes.insert(sizes.begin(), 4);
-            out = new_tensor(sizes, at::kFloat, p[0]);
-        }
-        float *dst = packed ? out.data_ptr<float>() : nullptr;
-        if (is_narrow(dtype))
-            status = bc_clip_parameters_narrow(q[0], q[1], q[2], q[3], io_kind(dtype), count, rep_h, rep_w, max_h, max_w, exact, dst,
-                                               stream);
-        else if (packed)
-            status = bc_clip_parameters_packed((float *)q[0], (float *)q[1], (float *)q[2], (float *)q[3], count, rep_h, rep_w,
-                                               max_h, max_w, exact, dst, stream);
-        else
-            status = bc_clip_parameters((float *)q[0], (float *)q[1], (float *)q[2], (float *)q[3], count, rep_h, rep_w, max_h,
-                                        max_w, exact, stream);
+        if (packed) out = new_snapshot(p[0].sizes(), p[0]);
+        status = bc_clip_parameters_any(q[0], q[1], q[2], q[3], io_kind(dtype), count, rep_h, rep_w, max_h, max_w, exact,
+                                        packed ? out.packed.data_ptr<float>() : nullptr, out.counters,
+                                        packed && count ? to_int(p[0].size(0)) : 0, stream);
     }
     check_status(status, "clip_parameters");
     return out;
@@ -382,6 +391,7 @@ Tensor clip(const Four &p, double rep_h, double rep_w, double max_h, double max_
 struct Kept {
     Tensor x;                    // the input; its integral image for float64
     Tensor params;               // packed (4, C, F): stored units, float32; pixels for float64
+    unsigned *counters = nullptr;
 };
 
 Tensor forward_any(const Tensor &input, const Four &p, const Options &o, Kept *keep)
@@ -393,7 +403,7 @@ Tensor forward_any(const Tensor &input, const Four &p, const Options &o, Kept *k
     if (dtype == at::kDouble) {
         Tensor pixels = at::stack({p[0].detach() * o.rep_h, p[1].detach() * o.rep_h, p[2].detach() * o.rep_w, p[3].detach() * o.rep_w});
         const Tensor integrated = integral_image(x);
-        if (keep) *keep = {integrated, pixels};
+        if (keep) *keep = {integrated, pixels, nullptr};
         return box_forward(integrated, {pixels.select(0, 0), pixels.select(0, 1), pixels.select(0, 2), pixels.select(0, 3)},
                            o.normalize, o.exact);
     }
@@ -401,12 +411,17 @@ Tensor forward_any(const Tensor &input, const Four &p, const Options &o, Kept *k
     if (narrow && s.h && s.w && s.F && !bc_boxconv2d_narrow_all_supported(s.F, s.h, s.w)) x = x.to(at::kFloat);
     const bc_stream_t stream = current_stream(x);
     Tensor packed = o.snapshot;
+    unsigned *counters = o.counters;
     if (packed.defined() && !(packed.scalar_type() == at::kFloat && packed.device() == x.device() && packed.is_contiguous() &&
                               packed.sizes() == at::IntArrayRef({4, s.C, s.F})))
         packed = Tensor();
     ParamPtrs q;
     Four dense;                  // (keeps contiguous copies alive across the launch)
-    if (!packed.defined() && (keep || narrow)) packed = pack_parameters(p, s, stream);
+    if (!packed.defined() && (keep || narrow)) {
+        const Snapshot snap = pack_parameters(p, s, stream);
+        packed = snap.packed;
+        counters = snap.counters;
+    }
     if (packed.defined()) {
         q = of_packed(packed);
     } else {
@@ -416,7 +431,7 @@ Tensor forward_any(const Tensor &input, const Four &p, const Options &o, Kept *k
         }
     }
     Tensor out = run_forward(x, q, s, o, stream);
-    if (keep) *keep = {x, packed};
+    if (keep) *keep = {x, packed, counters};
     return out.scalar_type() == dtype ? out : out.to(dtype);
 }
 
@@ -436,25 +451,31 @@ Gradients backward_any(const Tensor &x, const Tensor &params, Tensor grad_output
         require_cuda_float(grad_output, "grad_output", at::kFloat);
     }
     const Tensor g = grad_output.contiguous();
-    Tensor gparams;
     if (mask & BC_NEED_INPUT) out[0] = new_tensor(x.sizes(), dtype, x);
-    if (mask & ~BC_NEED_INPUT) gparams = new_tensor({4, s.C, s.F}, dtype, x);
     const size_t bytes = is_narrow(dtype) ? bc_boxconv2d_narrow_workspace(s.N, s.C, s.F, s.h, s.w, mask)
                                           : bc_boxconv2d_backward_workspace(s.N, s.C, s.F, s.h, s.w, mask);
-    Tensor ws = new_workspace(bytes, x);
+    // One allocation for the parameter gradients and, where it is small, the workspace behind them.
+    constexpr size_t kSmall = 64 * 1024;
+    Tensor gparams, scratch;
+    void *ws = nullptr;
+    if (mask & ~BC_NEED_INPUT) {
+        const size_t elem = c10::elementSize(dtype), gap = ((size_t)4 * s.C * s.F * elem + 255) / 256 * 256;
+        const bool together = bytes <= kSmall;
+        gparams = new_tensor({(int64_t)(together ? (gap + bytes + elem - 1) / elem : (size_t)4 * s.C * s.F)}, dtype, x);
+        if (together) ws = static_cast<char *>(gparams.data_ptr()) + gap;
+        gparams.unsafeGetTensorImpl()->set_sizes_contiguous({4, s.C, s.F});
+    }
+    if (!ws) {
+        scratch = new_workspace(bytes, x);
+        ws = scratch.data_ptr();
+    }
     const ParamPtrs q = of_packed(params);
     void *gin = out[0].defined() ? out[0].data_ptr() : nullptr, *gp = gparams.defined() ? gparams.data_ptr() : nullptr;
     const bc_stream_t stream = current_stream(x);
-    int status;
-    if (is_narrow(dtype))
-        status = bc_boxconv2d_backward_narrow_all(x.const_data_ptr(), io_kind(dtype), q.p[0], q.p[1], q.p[2], q.p[3], g.const_data_ptr(),
-                                                  (float)a.rep_h, (float)a.rep_w, s.N, s.C, s.F, s.h, s.w, a.normalize, a.exact, mask,
-                                                  gin, gp, ws.data_ptr(), bytes, stream);
-    else
-        status = bc_boxconv2d_backward(x.const_data_ptr<float>(), q.p[0], q.p[1], q.p[2], q.p[3], g.const_data_ptr<float>(),
-                                       (float)a.rep_h, (float)a.rep_w, s.N, s.C, s.F, s.h, s.w, a.normalize, a.exact, mask,
-                                       static_cast<float *>(gin), static_cast<float *>(gp), ws.data_ptr(), bytes, stream);
-    check_status(status, "BoxConv2d backward");
+    check_status(bc_boxconv2d_backward_any(x.const_data_ptr(), io_kind(dtype), q.p[0], q.p[1], q.p[2], q.p[3], g.const_data_ptr(),
+                                           (float)a.rep_h, (float)a.rep_w, s.N, s.C, s.F, s.h, s.w, a.normalize, a.exact, mask, gin, gp,
+                                           ws, bytes, a.counters, stream),
+                 "BoxConv2d backward");
     if (dtype != caller) {
         if (out[0].defined()) out[0] = out[0].to(caller);
         if (gparams.defined()) gparams = gparams.to(caller);
@@ -518,7 +539,8 @@ Tensor apply(const Tensor &input, const Four &p, const Options &o)
     node->x = torch::autograd::SavedVariable(keep.x, false);
     node->params = keep.params;
     node->options = o;
-    node->options.snapshot = Tensor();
+    node->options.snapshot = Tensor();      // (node->params holds it)
+    node->options.counters = keep.counters;
     node->caller = input.scalar_type();
     torch::autograd::set_history(out, node);
     return out;
@@ -641,7 +663,11 @@ PyObject *py_module_forward(PyObject *, PyObject *const *v, Py_ssize_t n)
     {
         py::gil_scoped_release release;
         // the launch that clips also leaves the copy of the parameters that backward will use
-        if (clipping) o.snapshot = clip(p, o.rep_h, o.rep_w, max_h, max_w, o.exact, p[0].scalar_type() != at::kDouble);
+        if (clipping) {
+            const Snapshot snap = clip(p, o.rep_h, o.rep_w, max_h, max_w, o.exact, p[0].scalar_type() != at::kDouble);
+            o.snapshot = snap.packed;
+            o.counters = snap.counters;
+        }
         out = apply(input, p, o);
     }
     return wrap(out);
@@ -737,7 +763,7 @@ PyObject *py_clip(PyObject *, PyObject *const *v, Py_ssize_t n)
     Tensor out;
     {
         py::gil_scoped_release release;
-        out = clip(p, rep_h, rep_w, max_h, max_w, exact, packed);
+        out = clip(p, rep_h, rep_w, max_h, max_w, exact, packed).packed;
     }
     return wrap(out);
     END_HANDLE_TH_ERRORS

@@ -216,7 +216,7 @@ int bc_boxconv2d_backward_narrow(const void *input, int io_kind, const float *x_
                                  size_t workspace_bytes, bc_stream_t stream);
 /* The same for larger planes as well (bc_boxconv2d_narrow_all_supported() tells; up to 2048 columns and 32
  * filters), through float integral images in a workspace of bc_boxconv2d_narrow_workspace() bytes (need_mask 0 for
- * the forward), and with the parameter gradients stored in the 16-bit type too, rounded once from the float sums. */
+ * the forward). */
 int bc_boxconv2d_narrow_all_supported(int F, int h, int w);
 size_t bc_boxconv2d_narrow_workspace(int N, int C, int F, int h, int w, int need_mask);
 int bc_boxconv2d_forward_narrow_all(const void *input, int io_kind, const float *x_min, const float *x_max,
@@ -224,20 +224,30 @@ int bc_boxconv2d_forward_narrow_all(const void *input, int io_kind, const float 
                                     float reparametrization_w, void *output, int N, int C, int F, int h,
                                     int w, int normalize, int exact, void *workspace, size_t workspace_bytes,
                                     bc_stream_t stream);
-int bc_boxconv2d_backward_narrow_all(const void *input, int io_kind, const float *x_min, const float *x_max,
-                                     const float *y_min, const float *y_max, const void *grad_output,
-                                     float reparametrization_h, float reparametrization_w, int N, int C,
-                                     int F, int h, int w, int normalize, int exact, int need_mask,
-                                     void *grad_input, void *grad_params, void *workspace,
-                                     size_t workspace_bytes, bc_stream_t stream);
-/* bc_clip_parameters() on 16-bit parameters (clipped as float, rounded when stored); packed_out, which may be
- * NULL, receives a (4, count) float copy of the stored values. */
-int bc_clip_parameters_narrow(void *x_min, void *x_max, void *y_min, void *y_max, int io_kind, int count,
-                              double reparametrization_h, double reparametrization_w, double max_input_h,
-                              double max_input_w, int exact, float *packed_out, bc_stream_t stream);
-/* A (4, count) float copy of four parameter arrays of type io_kind (BC_IO_*), in one launch. */
+
+/* ---- what a host binding needs for one launch per step of the pass -------------------------
+ * Backward pass of tensors of type io_kind (BC_IO_*); 16-bit tensors as above, with the parameter gradients stored
+ * in the 16-bit type too, rounded once from the float sums.  Workspace: bc_boxconv2d_backward_workspace() or
+ * bc_boxconv2d_narrow_workspace() bytes.  counters: C unsigned integers on the device that are zero before
+ * the call, and again after it, or NULL.  With them small problems finish their parameter gradients inside the
+ * backward kernel instead of in a launch of its own.  Calls that are not ordered by a stream need counters of
+ * their own. */
+int bc_boxconv2d_backward_any(const void *input, int io_kind, const float *x_min, const float *x_max,
+                              const float *y_min, const float *y_max, const void *grad_output,
+                              float reparametrization_h, float reparametrization_w, int N, int C,
+                              int F, int h, int w, int normalize, int exact, int need_mask,
+                              void *grad_input, void *grad_params, void *workspace,
+                              size_t workspace_bytes, unsigned *counters, bc_stream_t stream);
+/* bc_clip_parameters() on parameters of type io_kind (16-bit ones are clipped as float and rounded when stored);
+ * packed_out, which may be NULL, receives a (4, count) float copy of the stored values, and zeroed, which may be
+ * NULL, zeroed_count (at most count) zeros: the counters of the backward pass. */
+int bc_clip_parameters_any(void *x_min, void *x_max, void *y_min, void *y_max, int io_kind, int count,
+                           double reparametrization_h, double reparametrization_w, double max_input_h,
+                           double max_input_w, int exact, float *packed_out, unsigned *zeroed, int zeroed_count,
+                           bc_stream_t stream);
+/* A (4, count) float copy of four parameter arrays of type io_kind (BC_IO_*), in one launch; zeroed as above. */
 int bc_pack_parameters(const void *x_min, const void *x_max, const void *y_min, const void *y_max, int io_kind, int count,
-                       float *packed_out, bc_stream_t stream);
+                       float *packed_out, unsigned *zeroed, int zeroed_count, bc_stream_t stream);
 
 /* ---- backward pass without caller-supplied scratch memory --------------------------------
  * This entry point has no counterpart in the reference (which allocates its temporaries with
