@@ -186,32 +186,26 @@ __device__ __forceinline__ void rows8_load(Rows8 &g, const IO *row0, int w, int 
     const int k = (k0 + lane * w) & 3, at = c - lane * 4 + 4 * LN - k;
     g.next = lane < rows && lane < 8 && k && at < w ? load(row0 + lane * w + at) : zero;
 }
-// Columns c .. c+3 of row i; zero from column w on.
+// Columns c .. c+3 of row i; zero from column w on.  The shift by k is done in two steps, by one and by two places,
+// each with or without effect: four ways through the code would cost more instruction fetches than that saves.
 template <typename IO, bool ALIGNED, int LN = 32>
 __device__ __forceinline__ float4 rows8_get(const Rows8 &g, const IO *row0, int w, int c, int lane, int i)
 {
     float4 a = g.a[i];
     if (ALIGNED) return a;
     const int k = (row_shift(row0) + i * w) & 3;
-    if (k) {
-        const unsigned full = 0xffffffffu;
-        float n0 = __shfl_down_sync(full, a.x, 1), n1 = 0.f, n2 = 0.f;
-        const float e0 = __shfl_sync(full, g.next.x, i, LN);
-        if (lane == LN - 1) n0 = e0;
-        if (k > 1) {
-            n1 = __shfl_down_sync(full, a.y, 1, LN);
-            const float e1 = __shfl_sync(full, g.next.y, i, LN);
-            if (lane == LN - 1) n1 = e1;
-        }
-        if (k > 2) {
-            n2 = __shfl_down_sync(full, a.z, 1, LN);
-            const float e2 = __shfl_sync(full, g.next.z, i, LN);
-            if (lane == LN - 1) n2 = e2;
-        }
-        if (k == 1) a = make_float4(a.y, a.z, a.w, n0);
-        else if (k == 2) a = make_float4(a.z, a.w, n0, n1);
-        else a = make_float4(a.w, n0, n1, n2);
+    const bool one = k & 1, two = k & 2, end = lane == LN - 1;
+    const unsigned full = 0xffffffffu;
+    const float e0 = __shfl_sync(full, g.next.x, i, LN), e1 = __shfl_sync(full, g.next.y, i, LN), e2 = __shfl_sync(full, g.next.z, i, LN);
+    float n0 = __shfl_down_sync(full, a.x, 1, LN);
+    if (end) n0 = e0;
+    if (one) a = make_float4(a.y, a.z, a.w, n0);
+    float m0 = __shfl_down_sync(full, a.x, 1, LN), m1 = __shfl_down_sync(full, a.y, 1, LN);
+    if (end) {
+        m0 = one ? e1 : e0;
+        m1 = one ? e2 : e1;
     }
+    if (two) a = make_float4(a.z, a.w, m0, m1);
     if (c >= w) a.x = 0.f;
     if (c + 1 >= w) a.y = 0.f;
     if (c + 2 >= w) a.z = 0.f;
@@ -219,9 +213,40 @@ __device__ __forceinline__ float4 rows8_get(const Rows8 &g, const IO *row0, int 
     return a;
 }
 
-// `ok`: the row exists.
+// `ok`: the row exists.  Unaligned rows: one vector store a lane for the aligned groups that lie inside the row and
+// belong to this warp whole, and single elements for the rest: the 4 - k elements in front of the first group (the
+// first lane's), the k behind the last one (the last lane's), and what the row's end cuts off a group.
 template <typename IO, bool ALIGNED, int LN = 32>
 __device__ __forceinline__ void store_row4(IO *row, int c, int w, const float (&v)[4], int lane, bool ok = true)
+{
+    if (ALIGNED) {
+        if (ok && c < w) Io<IO>::store4(row + c, v[0], v[1], v[2], v[3]);
+        return;
+    }
+    const int k = row_shift(row);
+    const unsigned full = 0xffffffffu;
+    float o[4] = {v[0], v[1], v[2], v[3]};
+    const float p3 = __shfl_up_sync(full, o[3], 1, LN);
+    if (k & 1) { o[3] = o[2]; o[2] = o[1]; o[1] = o[0]; o[0] = p3; }
+    const float q2 = __shfl_up_sync(full, o[2], 1, LN), q3 = __shfl_up_sync(full, o[3], 1, LN);
+    if (k & 2) { o[3] = o[1]; o[2] = o[0]; o[1] = q3; o[0] = q2; }
+    const int at = c - k;                                     // first column of the lane's group
+    const bool whole = at + 4 <= w && (lane > 0 || k == 0);
+    if (ok && whole) Io<IO>::store4(row + at, o[0], o[1], o[2], o[3]);
+    const bool cut = (lane > 0 || k == 0) && at + 4 > w;                  // the row ends inside the group (or before it)
+    IO *single = row + (cut ? at : c);
+    const int room = w - (cut ? at : c);
+    const int from = cut ? 0 : lane == LN - 1 ? 4 - k : lane == 0 ? 0 : 4, to = cut ? 4 : lane == 0 && k ? 4 - k : lane == LN - 1 ? 4 : 0;
+    // (a group of one lane would be first and last at once; LN is at least 8)
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+        if (ok && m >= from && m < to && m < room) Io<IO>::store1(single + m, cut ? o[m] : v[m]);
+}
+
+// The same as branches on the shift k: twice the code, which kernels that store all the time can afford, and fewer
+// instructions (integral images of 512 planes of 256 x 512: 105 us against 115; forward of (8,16,4,149,201): 48 against 52).
+template <typename IO, bool ALIGNED, int LN = 32>
+__device__ __forceinline__ void store_row4_wide(IO *row, int c, int w, const float (&v)[4], int lane, bool ok = true)
 {
     if (ALIGNED) {
         if (ok && c < w) Io<IO>::store4(row + c, v[0], v[1], v[2], v[3]);

@@ -240,17 +240,20 @@ __device__ __forceinline__ void quad_store(QuadBlock &v, const QuadTile &t, cons
 // FUSED: the inference steps of `Fusion` (the output may then alias the residual).  Such calls are single frames, a
 // few CTAs an SM at most: registers are there to have all residual rows of a task in flight before its gather,
 // and the planes travel to L2 while the CTA still waits for the kernel in front.
+// Row parts (rsplit): few large planes, a CTA gathers only some of the rows for its filters.
 template <typename IO, int CT, int T, bool FAST, bool FUSED, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (FUSED ? 2 : 3) : 1)
-forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, BoxParams bp, IO *out, int C, int F, int h, int w, int row_tiles, int fsplit, int chunk,
-                    bool normalize, bool exact, Fusion fu)
+forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, BoxParams bp, IO *out, int C, int F, int h, int w, int row_tiles, int fsplit,
+                    int rsplit, int chunk, bool normalize, bool exact, Fusion fu)
 {
     using Q = QuadImage<CT>;
     extern __shared__ float4 smem4[];
     grid_dependency_release();
     const int lane = threadIdx.x & 31, warp = uniform(threadIdx.x >> 5), nwarps = blockDim.x >> 5;
-    const int part = blockIdx.x % fsplit, plane_at = blockIdx.x / fsplit, c = plane_at % C;
+    const int row_part = blockIdx.x % rsplit, b = blockIdx.x / rsplit;
+    const int part = b % fsplit, plane_at = b / fsplit, c = plane_at % C;
     const int f_begin = (F * part) / fsplit, nf = (F * (part + 1)) / fsplit - f_begin;
+    const int first_tile = (row_tiles * row_part) / rsplit, end_tile = (row_tiles * (row_part + 1)) / rsplit;
     const int64_t npix = (int64_t)h * w, nc = plane_at;
     const int cells = quad_cells(w), ntiles = row_tiles * CT;
     const QuadSmem s = quad_smem(smem4, h, CT, ntiles, nwarps);
@@ -258,7 +261,12 @@ forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
 
     if (FUSED) {      // hints only
         prefetch_l2(x + nc * npix, npix * sizeof(IO));
-        if (fu.residual) prefetch_l2(fu.residual + (nc * F + f_begin) * npix, (size_t)nf * npix * sizeof(float));
+        if (fu.residual) {
+            const int64_t p0 = first_tile * kTileRows * w, p1 = min(end_tile * kTileRows, h) * w;
+            if (rsplit == 1) prefetch_l2(fu.residual + (nc * F + f_begin) * npix, (size_t)nf * npix * sizeof(float));
+            else
+                for (int k = 0; k < nf; ++k) prefetch_l2(fu.residual + (nc * F + f_begin + k) * npix + p0, (size_t)(p1 - p0) * sizeof(float));
+        }
     }
     quad_zero_padding<CT>(s.image, h);
     // registers and shared memory only up to here; now what the kernel in front of this one may have written
@@ -315,7 +323,7 @@ forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
     }
     __syncthreads();
 
-    const int groups = (row_tiles + chunk - 1) / chunk, ntasks = nf * groups * CT;
+    const int groups = (end_tile - first_tile + chunk - 1) / chunk, ntasks = nf * groups * CT;
     for (int task = warp; task < ntasks; task += nwarps) {
         const int rest = task / nf, k = task - rest * nf, f = f_begin + k;
         const int g = rest / CT, ct = rest - g * CT;
@@ -329,7 +337,7 @@ forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
             if (fu.scale) mul = __ldg(fu.scale + c * F + f);
             if (fu.shift) add = __ldg(fu.shift + c * F + f);
         }
-        const int p_begin = g * chunk * kTileRows, p_end = min(p_begin + chunk * kTileRows, h);
+        const int p_begin = (first_tile + g * chunk) * kTileRows, p_end = min(min(first_tile + (g + 1) * chunk, end_tile) * kTileRows, h);
         const int64_t first = (nc * F + f) * npix + (int64_t)p_begin * w;
         IO *row = out + first;
         const float *res = FUSED && fu.residual ? fu.residual + first : nullptr;
@@ -360,7 +368,7 @@ forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
                             for (int m = 0; m < kStrip; ++m) v[m] = fmaxf(v[m], 0.0f);
                         }
                     }
-                    store_row4<IO, FAST>(row, q0, w, v, lane);
+                    store_row4_wide<IO, FAST>(row, q0, w, v, lane);
                     row += w;
                 }
             }
@@ -485,13 +493,15 @@ inline size_t quad_backward_smem(int F, int h, int w)
 }
 // Narrower planes leave more than half of a warp's lanes idle and are better off in 32 x 32 tiles.
 constexpr int kQuadMinWidth = 65;
-inline bool quad_fits_forward(int F, int h, int w)
+// few: the launch leaves SMs idle anyway.
+inline bool quad_fits_forward(int F, int h, int w, bool few = false)
 {
     const int tiles = quad_row_tiles(h) * quad_col_tiles(w);
     if (w < kQuadMinWidth || w > 256 || F > kMaxFilters || tiles > 2 * kQuadMaxWarps || quad_forward_smem(F, h, w) > kQuadMaxSmem) return false;
     // More than eight tiles means two a warp and a CTA that has its SM to itself: only where three quarters of the
-    // tiles' pixels exist (96 x 160, 63 %: 47 us against 33 in 32 x 32 tiles; 128 x 256: 35 against 37).
-    return tiles <= 8 || 4 * (int64_t)h * w >= 3 * (int64_t)tiles * 1024;
+    // tiles' pixels exist (96 x 160, 63 %: 47 us against 33 in 32 x 32 tiles; 128 x 256: 35 against 37), or where it
+    // has an SM to itself in any case (one 96 x 160 frame: 7.4 us against 8.2).
+    return tiles <= 8 || 4 * (int64_t)h * w >= 3 * (int64_t)tiles * 1024 || few;
 }
 inline bool quad_fits_backward(int F, int h, int w)
 {
@@ -509,19 +519,24 @@ int launch_forward_quad_t(const IO *x, const float *integ, const BoxParams &bp, 
     if (F % 2 == 0 && planes < 148 * 6) fsplit = 2;
     while (fsplit < F && F % (fsplit * 2) == 0 && planes * fsplit * 2 <= 148 * 2) fsplit *= 2;
     if (planes * fsplit > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
+    const bool fast = w % 4 == 0 && h % kTileRows == 0 && aligned_to(x, Io<IO>::kVecBytes) && aligned_to(out, Io<IO>::kVecBytes) &&
+                      (!fu || !fu->residual || aligned_to(fu->residual, 16));
     const int T = tiles > 8 ? 2 : 1;
+    // Planes of more than 16 tiles that leave SMs idle: CTAs that each gather a part of the rows, from integral images of
+    // their own ((1,16,4,128,256), 64 -> 128 CTAs: 12.0 -> 9.8 us a block tail).
+    int rsplit = 1;
+    while (tiles > 16 && planes * fsplit * rsplit * 2 <= 148 && rsplit < 4) rsplit *= 2;
     const int warps = (tiles + T - 1) / T, nf = (F + fsplit - 1) / fsplit;
     // rows per task: few long tasks read fewer tap rows twice, but every warp should get the same share
     int chunk = 1;
     double best = 1e30;
-    for (int k = 1; k <= row_tiles; ++k) {
-        const int tasks = nf * ((row_tiles + k - 1) / k) * col_tiles;
+    const int part_tiles = (row_tiles + rsplit - 1) / rsplit;
+    for (int k = 1; k <= part_tiles; ++k) {
+        const int tasks = nf * ((part_tiles + k - 1) / k) * col_tiles;
         const double cost = ((tasks + warps - 1) / warps) * (k * kTileRows + 2.0);
         if (cost < best) { best = cost; chunk = k; }
     }
-    const bool fast = w % 4 == 0 && h % kTileRows == 0 && aligned_to(x, Io<IO>::kVecBytes) && aligned_to(out, Io<IO>::kVecBytes) &&
-                     (!fu || !fu->residual || aligned_to(fu->residual, 16));
-    void (*kern)(const IO *, const float *, BoxParams, IO *, int, int, int, int, int, int, int, bool, bool, Fusion);
+    void (*kern)(const IO *, const float *, BoxParams, IO *, int, int, int, int, int, int, int, int, bool, bool, Fusion);
     auto pick = [&](auto ct) {
         constexpr int CT = decltype(ct)::value, S = 256, L = 512;
         constexpr bool FU = IsFloat<IO>::value;
@@ -540,8 +555,8 @@ int launch_forward_quad_t(const IO *x, const float *integ, const BoxParams &bp, 
     const Fusion none{0, nullptr, nullptr, nullptr, 0};
     {
         LaunchScope scope(KID_FORWARD_QUAD, s);
-        if (cudaError_t e = launch_overlapped(kern, (unsigned)(planes * fsplit), warps * 32, quad_forward_smem(nf, h, w), s, x, integ, bp, out,
-                                              C, F, h, w, row_tiles, fsplit, chunk, normalize, exact, fu ? *fu : none))
+        if (cudaError_t e = launch_overlapped(kern, (unsigned)(planes * fsplit * rsplit), warps * 32, quad_forward_smem(nf, h, w), s, x, integ, bp, out,
+                                              C, F, h, w, row_tiles, fsplit, rsplit, chunk, normalize, exact, fu ? *fu : none))
             return cuda_failed(e, "forward_quad");
     }
     return check_launch("forward_quad");

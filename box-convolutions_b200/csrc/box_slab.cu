@@ -140,7 +140,7 @@ forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int 
                             for (int m = 0; m < kStrip; ++m) v[m] = fmaxf(v[m], 0.0f);
                         }
                     }
-                    store_row4<IO, VEC>(out + off - q0, q0, w, v, lane);
+                    store_row4_wide<IO, VEC>(out + off - q0, q0, w, v, lane);
                     off += w;
                 }
             }

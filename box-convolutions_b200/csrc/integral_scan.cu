@@ -96,7 +96,7 @@ struct RowSink {
     {
         if (!QUAD) {
             const float o[4] = {v.x + carry, v.y + carry, v.z + carry, v.w + carry};
-            store_row4<float, false, LN>(row + 1, c, w, o, lane, ok);
+            store_row4_wide<float, false, LN>(row + 1, c, w, o, lane, ok);
             if (ok && first) *row = 0.0f;
             row += pitch;
             return;
