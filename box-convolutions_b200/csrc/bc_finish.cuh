@@ -45,28 +45,30 @@ __device__ __forceinline__ void finish_box(const T *partials, const BoxParamsT<T
 }
 
 // The finishing step inside a backward kernel: the last of the `total` CTAs that work on channel c to get here does it
-// for the channel's F boxes, in the same order of additions as the kernel of its own.  It saves a launch, which is
-// worth it where a step is bound by launches (3 us of host time); on larger grids the fence that every CTA pays
-// for costs more than the launch ((32,32,4,64,128) bfloat16, 1024 CTAs: 78.3 + 2.5 us in two launches, 84.5 in one),
-// so launchers leave total at 0 there.
+// for the channel's F boxes, in the same order of additions as the kernel of its own.  It saves a launch, 3 us of
+// host time, which is worth it where a step is bound by the host.  Where it is bound by the GPU, the fence that
+// every CTA pays for and the registers cost more than the launch ((8,16,4,128,256): 80 + 2.5 us in two launches, 88 in
+// one), so kernels have it as a template parameter and launchers ask for it up to kFinishMaxOutputs outputs.
+template <bool B>
+struct Flag { static constexpr bool value = B; };      // (picks a kernel's instantiation)
+
 struct Finish {
     void *grad_params;
     int io_kind, need_mask, per_box;
     float rep_h, rep_w;
     unsigned total;
 };
-constexpr int64_t kFinishMaxCtas = 4 * 148;
+constexpr int64_t kFinishMaxCtas = 4 * 148, kFinishMaxOutputs = 8 << 20;      // (a GPU time of about 45 us a step)
 
-inline Finish finish_here(const BoxParams &bp, bool need_params, int64_t ctas, int C, void *grad_params, int io_kind, int need_mask,
-                          int per_box, float rep_h, float rep_w)
+inline Finish finish_here(const BoxParams &bp, bool need_params, int64_t ctas, int64_t outputs, int C, void *grad_params, int io_kind,
+                          int need_mask, int per_box, float rep_h, float rep_w)
 {
-    const bool here = need_params && bp.counters && ctas <= kFinishMaxCtas;
+    const bool here = need_params && bp.counters && ctas <= kFinishMaxCtas && outputs <= kFinishMaxOutputs;
     return Finish{grad_params, io_kind, need_mask, per_box, rep_h, rep_w, here ? (unsigned)(ctas / C) : 0u};
 }
 
-// Called by all threads of a CTA after it has written its partial sums.  Not inlined: it runs once, and inlined it
-// costs the gather loops above it registers.
-static __device__ __noinline__ void finish_if_last_call(const Finish &fin, const float *partials, const BoxParams &bp, int c, int C, int F,
+// Called by all threads of a CTA after it has written its partial sums.
+__device__ __forceinline__ void finish_if_last(const Finish &fin, const float *partials, const BoxParams &bp, int c, int C, int F,
                                                bool normalize, bool exact)
 {
     __shared__ unsigned last;
@@ -80,12 +82,6 @@ static __device__ __noinline__ void finish_if_last_call(const Finish &fin, const
     for (int f = threadIdx.x >> 5; f < F; f += blockDim.x >> 5)
         finish_box<float>(partials, bp, c * F + f, C * F, fin.per_box, normalize, exact, fin.rep_h, fin.rep_w, fin.need_mask,
                           fin.grad_params, fin.io_kind, threadIdx.x & 31);
-}
-
-__device__ __forceinline__ void finish_if_last(const Finish &fin, const float *partials, const BoxParams &bp, int c, int C, int F,
-                                               bool normalize, bool exact)
-{
-    if (fin.total) finish_if_last_call(fin, partials, bp, c, C, F, normalize, exact);
 }
 
 }  // namespace bc

@@ -404,7 +404,7 @@ forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, 
 // as they are needed, which lets planes of up to ~48 000 pixels use this kernel).
 // The input plane in shared memory is float whatever IO is: float planes arrive by a bulk copy when
 // STAGED, narrow ones are converted by the threads as they are copied in.
-template <typename IO, int T, bool FAST, bool STAGED, bool NEED_PARAMS, bool XSMEM = true>
+template <typename IO, int T, bool FAST, bool STAGED, bool NEED_PARAMS, bool XSMEM = true, bool COUNTED = false>
 __global__ void __launch_bounds__(512)
 backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const IO *__restrict__ grad_output, BoxParams bp,
                       IO *__restrict__ grad_input, float *__restrict__ partials, int N, int C, int F,
@@ -643,7 +643,7 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
             }
         }
     }
-    if (NEED_PARAMS) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
+    if (COUNTED) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
 }
 
 // The limit is raised to its maximum once per kernel and device (it is a ceiling, not a reservation: what a
@@ -765,19 +765,24 @@ int launch_backward_plane_t(const IO *x, const float *x_integ, const IO *grad_ou
                         (with_staging <= two_ctas || plane_backward_smem_bytes(h, w, need_params, false, io) > two_ctas);
     const size_t smem = plane_backward_smem_bytes(h, w, need_params && xsmem, staged, io);
     void (*kern)(const IO *, const float *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, bool, bool, bool, Finish);
-    if (!xsmem) {
-        if (fast) kern = T == 1 ? backward_plane_kernel<IO, 1, true, false, true, false> : backward_plane_kernel<IO, 2, true, false, true, false>;
-        else kern = T == 1 ? backward_plane_kernel<IO, 1, false, false, true, false> : backward_plane_kernel<IO, 2, false, false, true, false>;
-    } else if (staged) {
-        kern = need_params ? backward_plane_kernel<IO, 1, true, true, true> : backward_plane_kernel<IO, 1, true, true, false>;
-    } else if (fast) {
-        kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, true, false, true> : backward_plane_kernel<IO, 1, true, false, false>)
-                      : (need_params ? backward_plane_kernel<IO, 2, true, false, true> : backward_plane_kernel<IO, 2, true, false, false>);
-    } else {
-        kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, false, false, true> : backward_plane_kernel<IO, 1, false, false, false>)
-                      : (need_params ? backward_plane_kernel<IO, 2, false, false, true> : backward_plane_kernel<IO, 2, false, false, false>);
-    }
-    const Finish fin = finish_here(bp, need_params, planes, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w);
+    const Finish fin = finish_here(bp, need_params, planes, planes * F * h * w, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w);
+    auto pick = [&](auto counted) {
+        constexpr bool K = decltype(counted)::value;
+        if (!xsmem) {
+            if (fast) kern = T == 1 ? backward_plane_kernel<IO, 1, true, false, true, false, K> : backward_plane_kernel<IO, 2, true, false, true, false, K>;
+            else kern = T == 1 ? backward_plane_kernel<IO, 1, false, false, true, false, K> : backward_plane_kernel<IO, 2, false, false, true, false, K>;
+        } else if (staged) {
+            kern = need_params ? backward_plane_kernel<IO, 1, true, true, true, true, K> : backward_plane_kernel<IO, 1, true, true, false>;
+        } else if (fast) {
+            kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, true, false, true, true, K> : backward_plane_kernel<IO, 1, true, false, false>)
+                          : (need_params ? backward_plane_kernel<IO, 2, true, false, true, true, K> : backward_plane_kernel<IO, 2, true, false, false>);
+        } else {
+            kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, false, false, true, true, K> : backward_plane_kernel<IO, 1, false, false, false>)
+                          : (need_params ? backward_plane_kernel<IO, 2, false, false, true, true, K> : backward_plane_kernel<IO, 2, false, false, false>);
+        }
+    };
+    if (fin.total) pick(Flag<true>{});
+    else pick(Flag<false>{});
     int st = opt_in_smem(kern, smem);
     if (st != BC_OK) return st;
     {

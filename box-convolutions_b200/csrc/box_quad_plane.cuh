@@ -381,7 +381,7 @@ forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
 // memory and gathered with the mirrored box.  The grad-input accumulators of a lane's 8 x 4 pixels stay in
 // registers; its input values wait in shared memory, where only their own warp touches them.  The next
 // grad_output plane is requested into L2 while the current one is gathered.
-template <typename IO, int CT, bool FAST, bool NEED_PARAMS, int MAXT>
+template <typename IO, int CT, bool FAST, bool NEED_PARAMS, bool COUNTED, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 2 : 1)
 backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const IO *__restrict__ grad_output, BoxParams bp, IO *__restrict__ grad_input,
                      float *__restrict__ partials, int N, int C, int F, int h, int w, int row_tiles, bool normalize, bool exact,
@@ -476,7 +476,7 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
                 store_row4<IO, FAST>(row, tile.c, w, v, lane);
             }
     }
-    if (NEED_PARAMS) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
+    if (COUNTED) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
 }
 
 inline int quad_row_tiles(int h) { return (h + kTileRows - 1) / kTileRows; }
@@ -575,19 +575,20 @@ int launch_backward_quad_t(const IO *x, const float *x_integ, const IO *grad_out
     const bool fast = w % 4 == 0 && h % kTileRows == 0 && ((size_t)h * w * sizeof(IO)) % 16 == 0 && aligned_to(x, Io<IO>::kVecBytes) &&
                      aligned_to(grad_output, 16) && (!write_gin || aligned_to(grad_input, Io<IO>::kVecBytes));
     void (*kern)(const IO *, const float *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, int, bool, bool, bool, Finish);
-    auto pick = [&](auto ct) {
+    const Finish fin = finish_here(bp, need_params, planes, planes * F * h * w, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w);
+    auto pick = [&](auto ct, auto counted) {
         constexpr int CT = decltype(ct)::value, S = 256, L = 512;
+        constexpr bool K = decltype(counted)::value;
         if (tiles <= 8) {
-            if (need_params) kern = fast ? backward_quad_kernel<IO, CT, true, true, S> : backward_quad_kernel<IO, CT, false, true, S>;
-            else kern = fast ? backward_quad_kernel<IO, CT, true, false, S> : backward_quad_kernel<IO, CT, false, false, S>;
+            if (need_params) kern = fast ? backward_quad_kernel<IO, CT, true, true, K, S> : backward_quad_kernel<IO, CT, false, true, K, S>;
+            else kern = fast ? backward_quad_kernel<IO, CT, true, false, false, S> : backward_quad_kernel<IO, CT, false, false, false, S>;
         } else {
-            if (need_params) kern = fast ? backward_quad_kernel<IO, CT, true, true, L> : backward_quad_kernel<IO, CT, false, true, L>;
-            else kern = fast ? backward_quad_kernel<IO, CT, true, false, L> : backward_quad_kernel<IO, CT, false, false, L>;
+            if (need_params) kern = fast ? backward_quad_kernel<IO, CT, true, true, K, L> : backward_quad_kernel<IO, CT, false, true, K, L>;
+            else kern = fast ? backward_quad_kernel<IO, CT, true, false, false, L> : backward_quad_kernel<IO, CT, false, false, false, L>;
         }
     };
-    if (col_tiles == 1) pick(Index<1>{});
-    else pick(Index<2>{});
-    const Finish fin = finish_here(bp, need_params, planes, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w);
+    if (fin.total) col_tiles == 1 ? pick(Index<1>{}, Flag<true>{}) : pick(Index<2>{}, Flag<true>{});
+    else col_tiles == 1 ? pick(Index<1>{}, Flag<false>{}) : pick(Index<2>{}, Flag<false>{});
     int st = raise_smem_limit(reinterpret_cast<const void *>(kern), (int)kQuadMaxSmem);
     if (st != BC_OK) return st;
     {

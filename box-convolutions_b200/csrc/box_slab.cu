@@ -156,7 +156,7 @@ forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int 
 
 // Per slab: the four input values and the grad-input accumulators of a lane's rows stay in registers over the
 // filters; the five sums are reduced per warp and filter, and per CTA at the end.
-template <typename IO, bool VEC, bool NEED_PARAMS, int MAXT>
+template <typename IO, bool VEC, bool NEED_PARAMS, bool COUNTED, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1)
 backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const float *__restrict__ go_integ, BoxParams bp, IO *__restrict__ grad_input,
                      float *__restrict__ partials, int N, int C, int F, int h, int w, SlabShape sh, bool normalize, bool exact,
@@ -270,7 +270,7 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
                 store_row4<IO, VEC>(row, q0, w, v, lane);
             }
     }
-    if (NEED_PARAMS) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
+    if (COUNTED) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
 }
 
 inline SlabShape slab_shape(int h, int w)
@@ -336,15 +336,20 @@ int backward_slab_t(const IO *x, const float *x_integ, const float *go_integ, co
     const bool write_gin = (need_mask & BC_NEED_INPUT) != 0;
     const bool vec = w % 4 == 0 && aligned_to(x, Io<IO>::kVecBytes) && (!write_gin || aligned_to(grad_input, Io<IO>::kVecBytes));
     void (*kern)(const IO *, const float *, const float *, BoxParams, IO *, float *, int, int, int, int, int, SlabShape, bool, bool, bool, Finish);
-    constexpr int S = 128, L = 32 * kSlabMaxWarps;
-    if (slab_threads(sh) <= S) {
-        if (need_params) kern = vec ? backward_slab_kernel<IO, true, true, S> : backward_slab_kernel<IO, false, true, S>;
-        else kern = vec ? backward_slab_kernel<IO, true, false, S> : backward_slab_kernel<IO, false, false, S>;
-    } else {
-        if (need_params) kern = vec ? backward_slab_kernel<IO, true, true, L> : backward_slab_kernel<IO, false, true, L>;
-        else kern = vec ? backward_slab_kernel<IO, true, false, L> : backward_slab_kernel<IO, false, false, L>;
-    }
-    const Finish fin = finish_here(bp, need_params, blocks, C, grad_params, grad_params_kind, need_mask, N * sh.slabs, rep_h, rep_w);
+    const Finish fin = finish_here(bp, need_params, blocks, (int64_t)N * C * F * h * w, C, grad_params, grad_params_kind, need_mask, N * sh.slabs, rep_h, rep_w);
+    auto pick = [&](auto counted) {
+        constexpr int S = 128, L = 32 * kSlabMaxWarps;
+        constexpr bool K = decltype(counted)::value;
+        if (slab_threads(sh) <= S) {
+            if (need_params) kern = vec ? backward_slab_kernel<IO, true, true, K, S> : backward_slab_kernel<IO, false, true, K, S>;
+            else kern = vec ? backward_slab_kernel<IO, true, false, false, S> : backward_slab_kernel<IO, false, false, false, S>;
+        } else {
+            if (need_params) kern = vec ? backward_slab_kernel<IO, true, true, K, L> : backward_slab_kernel<IO, false, true, K, L>;
+            else kern = vec ? backward_slab_kernel<IO, true, false, false, L> : backward_slab_kernel<IO, false, false, false, L>;
+        }
+    };
+    if (fin.total) pick(Flag<true>{});
+    else pick(Flag<false>{});
     int st = raise_smem_limit(reinterpret_cast<const void *>(kern), (int)kSlabMaxSmem);
     if (st != BC_OK) return st;
     {
