@@ -1,0 +1,128 @@
+"""Sizes at which the kernels' tiles, clusters and dispatch rules begin and end: the float32 kernels against
+the float64 ones (general kernels, checked against the oracle in test_gpu_f64.py), integral images against a
+float64 cumulative sum.
+
+Tolerances: outputs and grad-input 1e-4, parameter gradients 1e-3 of the largest magnitude, the bars of the
+parity tests (see _compare for what the largest is taken over).  Integral images of values in [0, 1): every entry is a sum of positive terms, so its relative
+error is at most (number of additions on its path) x 2^-24; the longest path here is some 2100 rows and
+columns one after the other, 1.3e-4, and 1e-5 is what the tree-shaped sums have to stay below.
+"""
+import numpy as np
+import pytest
+import torch
+
+from conftest import max_rel
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def bc():
+    import box_convolution
+    assert torch.cuda.is_available()
+    return box_convolution
+
+
+# lane groups of 8 and 16 (w <= 32, <= 64), one and several warps a row; 8-row tiles; one CTA, clusters, clusters
+# that read their plane twice, one CTA walking down; the widest row and one beyond (the older kernel)
+@pytest.mark.parametrize("planes,h,w", [
+    (1, 1, 1), (3, 7, 31), (5, 8, 32), (2, 9, 33), (3, 129, 64), (2, 513, 30), (4, 33, 65), (2, 128, 128), (3, 136, 129),
+    (1, 1100, 40), (2, 300, 511), (1, 70, 2048), (1, 9, 2049), (150, 140, 130), (149, 17, 257), (110, 140, 1200), (1, 2100, 8),
+])
+def test_integral_image_edges(bc, planes, h, w):
+    x = torch.rand(planes, h, w, device="cuda", generator=torch.Generator("cuda").manual_seed(h + w))
+    got = bc.integral_image(x)
+    assert (got[:, 0] == 0).all() and (got[:, :, 0] == 0).all()
+    want = x.double().cumsum(-1).cumsum(-2)
+    assert ((got[:, 1:, 1:].double() - want).abs() <= 1e-5 * want).all()
+    flat = torch.empty(x.numel() + 1, device="cuda")[1:].view_as(x).copy_(x)          # rows that no vector access fits
+    assert ((bc.integral_image(flat)[:, 1:, 1:].double() - want).abs() <= 1e-5 * want).all()
+
+
+def _boxes(rng, C, F, h, w, exact):
+    lo = 0.3 if exact else 1.2
+    cx = rng.uniform(-h / 2, h / 2, (C, F)); ex = rng.uniform(lo, h / 3 + lo, (C, F))
+    cy = rng.uniform(-w / 2, w / 2, (C, F)); ey = rng.uniform(lo, w / 3 + lo, (C, F))
+    return [a.astype(np.float32) for a in (cx - ex, cx + ex, cy - ey, cy + ey)]
+
+
+def _compare(got, want):
+    """[output, grad_input, four parameter gradients] against float64.  A parameter gradient is a sum of N h w products
+    of either sign that is divided by nothing: with a filter or two one of them can come out near zero by
+    accident while its rounding error, about 2^-24 sqrt(N h w) times a product, does not.  So the errors of
+    the four are measured against the largest of them."""
+    for a, b in zip(got[:2], want[:2]):
+        assert max_rel(a.cpu().numpy(), b.cpu().numpy()) < 1e-4
+    a, b = (torch.stack([t.double() for t in run[2:]]).cpu().numpy() for run in (got, want))
+    assert max_rel(a, b) < 1e-3
+
+
+# whole planes in 8 x 128 tiles (one and two column tiles, up to and above eight tiles, full and cut rows), slabs
+# (several column tiles, the last slab cut, wide rows), the grad_output integral in clusters, in bands, with two tiles
+# a thread, walked down; unaligned rows everywhere; a small grid that finishes in the backward kernel and one above it
+SHAPES = [(1, 2, 2, 8, 65), (2, 2, 3, 64, 128), (1, 3, 2, 65, 127), (1, 2, 1, 63, 129), (1, 2, 2, 64, 256), (1, 1, 2, 72, 250),
+          (1, 2, 2, 128, 126), (1, 1, 3, 121, 93), (2, 1, 2, 128, 252), (1, 1, 2, 256, 256), (1, 2, 2, 201, 257), (1, 2, 3, 30, 1030),
+          (1, 1, 2, 72, 2000), (1, 1, 2, 150, 2000), (2, 35, 1, 150, 1992), (3, 25, 2, 240, 220), (2, 3, 2, 1100, 48), (1, 1, 1, 230, 2047),
+          (20, 30, 2, 8, 68), (4, 5, 32, 9, 90)]
+
+
+@pytest.mark.parametrize("normalize,exact", [(True, True), (False, False)])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_training_edges_against_float64(bc, shape, normalize, exact):
+    N, C, F, h, w = shape
+    rng = np.random.default_rng(h * 3000 + w)
+    gen = torch.Generator("cuda").manual_seed(h + w)
+    x = torch.randn(N, C, h, w, device="cuda", generator=gen)
+    go = torch.randn(N, C * F, h, w, device="cuda", generator=gen)
+    pix = [torch.from_numpy(p).cuda() for p in _boxes(rng, C, F, h, w, exact)]
+    pix[2][0, 0], pix[3][0, 0] = w + 1.25, w + 7.5            # a box wholly beyond the right border: no gradient at all
+    runs = []
+    for dtype in (torch.float32, torch.float64):
+        args = [t.detach().to(dtype).requires_grad_() for t in [x] + pix]
+        out = bc.BoxConvolutionFunction.apply(*args, 1.0, 1.0, normalize, exact)
+        first = torch.autograd.grad(out, args, go.to(dtype), retain_graph=True)
+        again = torch.autograd.grad(out, args, go.to(dtype))
+        assert all(torch.equal(a, b) for a, b in zip(first, again))
+        runs.append([out.detach()] + list(first))
+    _compare(*runs)
+    assert all(g[0, 0] == 0 for g in runs[0][2:])
+
+
+# the same through the four functions, which gather from the caller's integral image
+@pytest.mark.parametrize("shape", [(1, 2, 2, 64, 128), (2, 2, 3, 33, 70), (1, 2, 2, 96, 160), (1, 1, 2, 121, 250), (1, 2, 2, 201, 257)])
+def test_four_functions_edges_against_float64(bc, shape):
+    N, C, F, h, w = shape
+    rng = np.random.default_rng(h * 7 + w)
+    x, go = torch.randn(N, C, h, w, device="cuda"), torch.randn(N, C * F, h, w, device="cuda")
+    pix = [torch.from_numpy(p).cuda() for p in _boxes(rng, C, F, h, w, True)]
+    runs = []
+    for dtype in (torch.float32, torch.float64):
+        integ, ps = bc.integral_image(x.to(dtype)), [p.to(dtype) for p in pix]
+        out = bc.box_convolution_forward(integ, *ps, True, True)
+        runs.append([out] + bc.box_convolution_backward(integ, *ps, go.to(dtype), out, 8.0, 8.0, True, True, True, True, True, True, True))
+    _compare(*runs)
+
+
+# residual rows of any alignment, in place; a frame whose planes are split over CTAs by rows
+@pytest.mark.parametrize("shape", [(1, 3, 2, 64, 128), (1, 2, 2, 128, 256), (1, 2, 4, 120, 201), (1, 2, 2, 30, 61), (1, 1, 2, 201, 301)])
+def test_fused_tail_edges(bc, shape):
+    N, C, F, h, w = shape
+    m = bc.BoxConv2d(C, F, h, w).cuda().eval()
+    x, skip = torch.randn(N, C, h, w, device="cuda"), torch.randn(N, C * F, h, w, device="cuda")
+    scale, shift = torch.rand(C * F, device="cuda") + 0.5, torch.rand(C * F, device="cuda") - 0.5
+    with torch.no_grad():
+        want = torch.relu(m(torch.relu(x)) * scale.view(1, -1, 1, 1) + shift.view(1, -1, 1, 1) + skip)
+    for offset in (0, 1):                                       # aligned and unaligned buffers
+        buf = torch.empty(skip.numel() + offset, device="cuda")[offset:].view_as(skip).copy_(skip)
+        got = bc.fused_box_block(m, x, input_relu=True, scale=scale, shift=shift, residual=buf, output_relu=True, out=buf)
+        assert (got - want).abs().max() <= 2e-5 * max(1.0, want.abs().max().item())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_narrow_parameters_are_clipped_as_floats(bc, dtype):
+    """One launch clips 16-bit parameters: float arithmetic on their values, rounded when stored."""
+    p = [torch.randn(5, 3, device="cuda").to(dtype) for _ in range(4)]
+    wide = [t.float() for t in p]
+    bc.clip_parameters(*p, 8.0, 16.0, 8.0, 16.0, True)
+    bc.clip_parameters(*wide, 8.0, 16.0, 8.0, 16.0, True)
+    assert all(torch.equal(a, b.to(dtype)) for a, b in zip(p, wide))
