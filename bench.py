@@ -84,6 +84,9 @@ NCU_TRAFFIC = {
     # profiles/plane_kernels_cfg5_dram_bytes.md (batch 256: 67 108 864 input elements)
     "backward_plane_kernel": [(88.25e6, 4194304), (1591.1e6, 67108864)],
     "forward_plane_kernel": [(29.05e6, 4194304), (1281.5e6, 67108864)],
+    # profiles/quad_slab_kernels_ncu.md
+    "backward_quad_kernel": [(84.23e6, 4194304), (1589.4e6, 67108864)],
+    "forward_quad_kernel": [(24.16e6, 4194304), (1278.5e6, 67108864)],
 }
 
 
@@ -469,6 +472,10 @@ def kernel_algorithmic_bytes(kernel, N, C, F, h, w):
         "backward_global_kernel": 4 * (F * Ei + 2 * E),
         "forward_band_kernel": 4 * (Ei + F * E),
         "backward_band_kernel": 4 * (F * Ei + 2 * E),
+        "forward_slab_kernel": 4 * (Ei + F * E),
+        "backward_slab_kernel": 4 * (F * Ei + 2 * E),
+        "forward_quad_kernel": 4 * E * (1 + F),
+        "backward_quad_kernel": 4 * E * (F + 2),
         "forward_plane_kernel": 4 * E * (1 + F),
         "backward_plane_kernel": 4 * E * (F + 2),
     }.get(kernel)
