@@ -153,14 +153,16 @@ __device__ __forceinline__ float warp_sum5(const float (&v)[kNumSums], int lane)
     return s;
 }
 
-// One filter's contribution of a strip of R rows to grad-input and to the five sums.  `x(i)` gives the four
-// input values of row i; FULL: the strip has all its rows, else those at or past `rows` do not exist (x is zero there).
-// gin: (columns 0, 1) and (2, 3) of each row.
+// One filter's contribution of a strip of R rows to grad-input and to the five sums.  FULL: the strip has all its rows,
+// else those at or past `rows` do not exist (their input values are zero there).
+// at: the strip's input values and grad-input accumulators.  `first()` returns the input values of row 0, `fetch(i)`
+// starts fetching row i's accumulators and the input values of row i + 1, which `next()` returns, `add(i, ...)` adds
+// to the accumulators.
 // The column strips enter the sums weighted by u(j), what the rows of the box make of the input values next to
 // tap row j: sum_i x_i (row combination of e) = sum_j e(j) (w_a x_(j+1) + w_b x_j).
-template <int R, bool NEED_PARAMS, bool FULL, class XRow>
+template <int R, bool NEED_PARAMS, bool FULL, class Cells>
 __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const QuadCols &cols, const QuadRows<R> &q, const ColW2 &cw,
-                                                    XRow &&x, f2_t (&gin)[R][2], float (&sums)[kNumSums], int rows)
+                                                    Cells &&at, float (&sums)[kNumSums], int rows)
 {
     f2_t pd[kStrip];
     const f2_t scale = pack2(t.scale, t.scale);
@@ -178,7 +180,7 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
         f2_t topbot = pack2(0.f, 0.f), left = topbot, right = topbot, out2 = topbot;
         f2_t el[kStrip], eh[kStrip], xx[kStrip];
         quad_pair_e(cols, q.lo[0], q.hi[0], cw, pd, el, eh);
-        float4 e = x(0);
+        float4 e = at.first();
         xx[0] = pack2(e.x, e.x); xx[1] = pack2(e.y, e.y); xx[2] = pack2(e.z, e.z); xx[3] = pack2(e.w, e.w);
 #pragma unroll
         for (int m = 0; m < kStrip; ++m) {
@@ -191,9 +193,11 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
             if (FULL || i < rows) {
                 f2_t cd[kStrip], xn[kStrip], dd[kStrip];
                 const f2_t x01 = pack2(e.x, e.y), x23 = pack2(e.z, e.w);
+                at.fetch(i);
                 quad_pair_e(cols, q.lo[i + 1], q.hi[i + 1], cw, cd, el, eh);
+                const float4 below = at.next();
                 if (i + 1 < R) {
-                    e = x(i + 1);
+                    e = below;
                     xn[0] = pack2(e.x, e.x); xn[1] = pack2(e.y, e.y); xn[2] = pack2(e.z, e.z); xn[3] = pack2(e.w, e.w);
                 }
 #pragma unroll
@@ -208,8 +212,7 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
                 const f2_t g01 = pack2(gather(cd[0], pd[0], dd[0]), gather(cd[1], pd[1], dd[1]));
                 const f2_t g23 = pack2(gather(cd[2], pd[2], dd[2]), gather(cd[3], pd[3], dd[3]));
                 out2 = fma2(x01, g01, fma2(x23, g23, out2));
-                gin[i][0] = fma2(g01, scale, gin[i][0]);
-                gin[i][1] = fma2(g23, scale, gin[i][1]);
+                at.add(i, g01, g23, scale);
 #pragma unroll
                 for (int m = 0; m < kStrip; ++m) {
                     pd[m] = cd[m];
@@ -229,14 +232,15 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
             if (FULL || i < rows) {
                 f2_t cd[kStrip];
                 float g[kStrip];
+                at.fetch(i);
                 quad_pair(cols, q.lo[i + 1], q.hi[i + 1], cw, cd);
+                at.next();
 #pragma unroll
                 for (int m = 0; m < kStrip; ++m) {
                     g[m] = gather(cd[m], pd[m], sub2(cd[m], pd[m]));
                     pd[m] = cd[m];
                 }
-                gin[i][0] = fma2(pack2(g[0], g[1]), scale, gin[i][0]);
-                gin[i][1] = fma2(pack2(g[2], g[3]), scale, gin[i][1]);
+                at.add(i, pack2(g[0], g[1]), pack2(g[2], g[3]), scale);
             }
         }
     }

@@ -1,5 +1,5 @@
-// Shared-memory-resident kernels for planes small enough to keep on chip (the 1/8-frame ENet
-// shape, 64 x 128, is the design point).  HBM traffic is the compulsory minimum: the forward
+// Shared-memory-resident kernels for planes small enough to keep on chip and too narrow (64 columns) or too large
+// for the quad layout's tiles of 8 x 128 (box_quad_plane.cuh).  HBM traffic is the compulsory minimum: the forward
 // reads the input once and writes the output once; the backward reads the input and grad_output
 // once and writes grad_input once.  No integral image ever goes to global memory.
 //

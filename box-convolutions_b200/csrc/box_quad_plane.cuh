@@ -13,6 +13,7 @@
 #include "bc_finish.cuh"
 #include "bc_quad.cuh"
 #include "bc_tile_io.cuh"
+#include "bc_tmem.cuh"
 
 namespace bc {
 
@@ -378,11 +379,13 @@ forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
 }
 
 // Backward: one CTA per plane, one tile per warp.  Per filter the grad_output plane is integrated in shared
-// memory and gathered with the mirrored box.  The grad-input accumulators of a lane's 8 x 4 pixels stay in
-// registers; its input values wait in shared memory, where only their own warp touches them.  The next
-// grad_output plane is requested into L2 while the current one is gathered.
+// memory and gathered with the mirrored box.  The grad-input accumulators of a lane's 8 x 4 pixels and its input
+// values wait in tensor memory (bc_tmem.cuh).  The next grad_output plane is requested into L2 while the
+// current one is gathered.
+// Bound by the latencies of its phases, which other CTAs of the SM have to cover: (256,32,4,64,128) with accumulators in
+// registers and input values in shared memory, two CTAs an SM: 564 us; like this, three: 512 us.
 template <typename IO, int CT, bool FAST, bool NEED_PARAMS, bool COUNTED, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 2 : 1)
+__global__ void __launch_bounds__(MAXT, MAXT > 256 ? 1 : FAST || NEED_PARAMS ? 3 : 2)
 backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const IO *__restrict__ grad_output, BoxParams bp, IO *__restrict__ grad_input,
                      float *__restrict__ partials, int N, int C, int F, int h, int w, int row_tiles, bool normalize, bool exact,
                      bool write_gin, Finish fin)
@@ -397,39 +400,45 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
     const QuadSmem s = quad_smem(smem4, h, CT, ntiles, nwarps);
     float *sTaps = reinterpret_cast<float *>(reinterpret_cast<char *>(smem4) + (s.taps - s.image));
     float *red = sTaps + F * kTapWords;                                                        // [F][warps][5]
-    const uint32_t sx = s.taps + ((F * (kTapWords + ntiles * kNumSums) * 4 + 15) & ~15) + warp * (kTileRows * 512) + lane * 16;
+    __shared__ uint32_t tmem_base;
     const IO *gbase = grad_output + nc * F * (int64_t)npix;
     const QuadTile tile = quad_tile<CT>(warp, lane, h);
 
     if (FAST && threadIdx.x == 0) bulk_prefetch_l2(gbase, (uint32_t)npix * (uint32_t)sizeof(IO));
     quad_zero_padding<CT>(s.image, h);
     grid_dependency_wait();
-    if (NEED_PARAMS) {
-        if (x_integ) {
-            // the caller has only the input's integral image: its pixels are second differences
-            const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1) + (int64_t)tile.p0 * (w + 1);
-#pragma unroll 1
-            for (int i = 0; i < kTileRows; ++i, I += w + 1) {
-                float e[4];
-#pragma unroll
-                for (int m = 0; m < 4; ++m) e[m] = i < tile.rows && tile.c + m < w ? pixel_of_integral(I + tile.c + m, w + 1) : 0.0f;
-                sts128(sx + i * 512, make_float4(e[0], e[1], e[2], e[3]));
-            }
-        } else {
-            const IO *row = x + nc * npix + tile.p0 * w;
-            Rows8 g;
-            rows8_load<IO, FAST>(g, row, w, tile.c, FAST ? kTileRows : tile.rows, lane);
-#pragma unroll
-            for (int i = 0; i < kTileRows; ++i) sts128(sx + i * 512, rows8_get<IO, FAST>(g, row, w, tile.c, lane, i));
-        }
-    }
+    const IO *xrow = x + nc * npix + tile.p0 * w;
+    Rows8 g;
+    if (NEED_PARAMS && x) rows8_load<IO, FAST>(g, xrow, w, tile.c, FAST ? kTileRows : tile.rows, lane);      // in flight meanwhile
+    __syncwarp();
+    if (warp == nwarps - 1) tmem_alloc(&tmem_base, tmem_columns(nwarps));
     if ((int)threadIdx.x < F) {
         const Box box = load_box(bp, c * F + threadIdx.x);
         store_taps(sTaps + threadIdx.x * kTapWords, taps_mirrored(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
     }
-    f2_t gin[kTileRows][2];
+    __syncthreads();
+    tmem_acquire();
+    TmemRows kept(tmem_base, warp);
+    if (NEED_PARAMS) {
+        if (!x) {
+            // the caller has only the input's integral image: its pixels are second differences
+            const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1) + (int64_t)tile.p0 * (w + 1);
+#pragma unroll 4
+            for (int i = 0; i < kTileRows; ++i, I += w + 1) {
+                float e[4];
 #pragma unroll
-    for (int i = 0; i < kTileRows; ++i) gin[i][0] = gin[i][1] = pack2(0.f, 0.f);
+                for (int m = 0; m < 4; ++m) e[m] = i < tile.rows && tile.c + m < w ? pixel_of_integral(I + tile.c + m, w + 1) : 0.0f;
+                kept.init(i, make_float4(e[0], e[1], e[2], e[3]));
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < kTileRows; ++i) kept.init(i, rows8_get<IO, FAST>(g, xrow, w, tile.c, lane, i));
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < kTileRows; ++i) kept.init(i, make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+    kept.sync();
     for (int f = 0; f < F; ++f) {
         {
             QuadBlock v;
@@ -448,8 +457,8 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
         const BoxTaps t = load_taps_uniform(sTaps + f * kTapWords);
         quad_backward_strip<kTileRows, NEED_PARAMS, FAST>(t, quad_cols(t, tile.c >> 2, cells, Q::kCells),
                                                           quad_rows<kTileRows>(t, tile.p0, h, s.image, s.image, Q::kRow, lane),
-                                                          col_weights(t), [&](int i) { return lds128(sx + i * 512); }, gin, sums,
-                                                          tile.rows);
+                                                          col_weights(t), kept, sums, tile.rows);
+        kept.sync();
         if (NEED_PARAMS) {
             const float sum = warp_sum5(sums, lane);
             const int slot = sum5_slot(lane);
@@ -470,12 +479,14 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
 #pragma unroll
         for (int i = 0; i < kTileRows; ++i, row += w)
             if (FAST || i < tile.rows) {
-                float v[kStrip];
-                unpack2(gin[i][0], v[0], v[1]);
-                unpack2(gin[i][1], v[2], v[3]);
+                const float4 g = kept.grad_input(i);
+                float v[kStrip] = {g.x, g.y, g.z, g.w};
                 store_row4<IO, FAST>(row, tile.c, w, v, lane);
             }
     }
+    tmem_release();
+    __syncthreads();
+    if (warp == 0) tmem_free(tmem_base, tmem_columns(nwarps));
     if (COUNTED) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
 }
 
@@ -489,7 +500,7 @@ inline size_t quad_forward_smem(int F, int h, int w)
 inline size_t quad_backward_smem(int F, int h, int w)
 {
     const size_t tiles = (size_t)quad_row_tiles(h) * quad_col_tiles(w);
-    return quad_forward_smem(F, h, w) + F * tiles * kNumSums * 4 + 16 + tiles * kTileRows * 512;
+    return quad_forward_smem(F, h, w) + F * tiles * kNumSums * 4;
 }
 // Narrower planes leave more than half of a warp's lanes idle and are better off in 32 x 32 tiles.
 constexpr int kQuadMinWidth = 65;

@@ -1,18 +1,24 @@
 // Forward and backward for planes too large to keep in shared memory whole.
 //
-// Two kernels a pass.  integral_scan_kernel writes the integral images of a batch of planes to a workspace,
+// Two kernels a pass.  integral_scan.cu writes the integral images of a batch of planes to a workspace,
 // rows in the quad layout (bc_quad.cuh).  The gather kernels then work on slabs: R rows of one plane, full
 // width.  What a slab of a box filter reads of the integral image is two runs of R + 1 adjacent rows, one on
 // either side of the box, each a contiguous piece of memory: two bulk copies per filter bring them to shared
-// memory, double-buffered, so the copies of the next filter run while the current one is gathered.
+// memory.  A CTA has one stage and up to four warps wherever the plane's width allows; six of them on an SM
+// (five in the backward) cover one another's copies.
 //
 // Against gathering from column bands (32 columns, full height) a slab costs 2 (R+1)/R words of L2 traffic an
 // output instead of 2.5, two copy instructions instead of thousands of 16-byte ones, and reads shared
 // memory with 5 (R+1)/R words an output instead of 8.
+//
+// Bound by the shared-memory pipe (77 % in the forward) and the issue slots (68 % / 61 %); the data comes from L2.
+// (8,16,4,256,512): forward 164 -> 86 us, backward 211 -> 121 us against column bands.  A training step of
+// (8,16,4,128,256) planes on whole-plane kernels takes the same time, so those stay there.
 #include "bc_common.cuh"
 #include "bc_finish.cuh"
 #include "bc_quad.cuh"
 #include "bc_tile_io.cuh"
+#include "bc_tmem.cuh"
 
 namespace bc {
 
@@ -154,16 +160,17 @@ forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int 
     if (timed_out && lane == 0) atomicAdd(&g_wait_timeouts, 1);
 }
 
-// Per slab: the four input values and the grad-input accumulators of a lane's rows stay in registers over the
-// filters; the five sums are reduced per warp and filter, and per CTA at the end.
+// The input values and the grad-input accumulators of a lane's rows wait in tensor memory (bc_tmem.cuh); the five sums
+// are reduced per warp and filter, and per CTA at the end.
 template <typename IO, bool VEC, bool NEED_PARAMS, bool COUNTED, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1)
+__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 5 : 1)
 backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const float *__restrict__ go_integ, BoxParams bp, IO *__restrict__ grad_input,
                      float *__restrict__ partials, int N, int C, int F, int h, int w, SlabShape sh, bool normalize, bool exact,
                      bool write_gin, Finish fin)
 {
     extern __shared__ __align__(128) unsigned char slab_stage[];
     __shared__ __align__(8) unsigned long long mbar;
+    __shared__ uint32_t tmem_base;
     grid_dependency_release();
     const int lane = threadIdx.x & 31, warp = uniform(threadIdx.x >> 5), nwarps = blockDim.x >> 5;
     const int slab = blockIdx.x % sh.slabs;
@@ -177,6 +184,13 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
     const int64_t ipl = (int64_t)(h + 1) * pitch;
     const float *planes = go_integ + nc * F * ipl;
 
+    const int rg = warp / sh.col_tiles, ct = warp - rg * sh.col_tiles;
+    const int q0 = ct * 128 + lane * kStrip, p0 = p_slab + rg * kStripRows;
+    const int mine = min(kStripRows, p_slab + rows - p0);
+    // (lanes past the plane gather too, from clamped columns, with x = 0)
+    const int64_t pix = nc * (int64_t)h * w + (int64_t)p0 * w + q0;
+    const IO *xrow = x + pix - q0;
+    Rows8 g;
     if (threadIdx.x == 0) {
         mbar_init(mbar32, 2);
         fence_mbar_init();
@@ -186,40 +200,36 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
         const Box box = load_box(bp, c * F + threadIdx.x);
         store_taps(sTaps + threadIdx.x * kTapWords, taps_mirrored(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
     }
+    if (NEED_PARAMS && x) rows8_load<IO, VEC>(g, xrow, w, q0, mine, lane);      // in flight meanwhile
+    __syncwarp();
+    if (warp == nwarps - 1) tmem_alloc(&tmem_base, tmem_columns(nwarps));
     __syncthreads();
+    tmem_acquire();
+    TmemRows kept(tmem_base, warp);
     if (threadIdx.x == 0) {
         fence_proxy_async();
         slab_issue(planes, pitch, load_taps(sTaps), p_slab, rows, h, stage32, stage32 + sh.stage_bytes, mbar32);
     }
 
-    const int rg = warp / sh.col_tiles, ct = warp - rg * sh.col_tiles;
-    const int q0 = ct * 128 + lane * kStrip, p0 = p_slab + rg * kStripRows;
-    const int mine = min(kStripRows, p_slab + rows - p0);
-    // (lanes past the plane gather too, from clamped columns, with x = 0)
-    const int64_t pix = nc * (int64_t)h * w + (int64_t)p0 * w + q0;
-    // the lane's input values wait in shared memory, where only their own warp touches them
-    const uint32_t sx = smem_u32(red) + ((F * nwarps * kNumSums * 4 + 15) & ~15) + warp * (kStripRows * 512) + lane * 16;
     if (NEED_PARAMS) {
         if (x) {
-            const IO *row = x + pix - q0;
-            Rows8 g;
-            rows8_load<IO, VEC>(g, row, w, q0, mine, lane);
 #pragma unroll
-            for (int i = 0; i < kStripRows; ++i) sts128(sx + i * 512, rows8_get<IO, VEC>(g, row, w, q0, lane, i));
+            for (int i = 0; i < kStripRows; ++i) kept.init(i, rows8_get<IO, VEC>(g, xrow, w, q0, lane, i));
         } else {      // the caller has only the input's integral image: its pixels are second differences
             const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1) + (int64_t)p0 * (w + 1) + q0;
-#pragma unroll 1
+#pragma unroll 4
             for (int i = 0; i < kStripRows; ++i, I += w + 1) {
                 float e[4];
 #pragma unroll
                 for (int m = 0; m < kStrip; ++m) e[m] = i < mine && q0 + m < w ? pixel_of_integral(I + m, w + 1) : 0.0f;
-                sts128(sx + i * 512, make_float4(e[0], e[1], e[2], e[3]));
+                kept.init(i, make_float4(e[0], e[1], e[2], e[3]));
             }
         }
-    }
-    f2_t gin[kStripRows][2];
+    } else {
 #pragma unroll
-    for (int i = 0; i < kStripRows; ++i) gin[i][0] = gin[i][1] = pack2(0.f, 0.f);
+        for (int i = 0; i < kStripRows; ++i) kept.init(i, make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+    kept.sync();
     bool timed_out = false;
     for (int f = 0; f < F; ++f) {
         timed_out |= !mbar_wait(mbar32, f & 1);
@@ -231,11 +241,11 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
             const uint32_t hi32 = stage32 + sh.stage_bytes - s.hi_first * row_bytes;
             const QuadCols cols = quad_cols(t, q0 >> 2, cells, cells);
             const QuadRows<kStripRows> q = quad_rows<kStripRows>(t, p0, h, lo32, hi32, row_bytes, lane);
-            auto xrow = [&](int i) { return lds128(sx + i * 512); };
             if (mine == kStripRows)
-                quad_backward_strip<kStripRows, NEED_PARAMS, true>(t, cols, q, col_weights(t), xrow, gin, sums, mine);
+                quad_backward_strip<kStripRows, NEED_PARAMS, true>(t, cols, q, col_weights(t), kept, sums, mine);
             else
-                quad_backward_strip<kStripRows, NEED_PARAMS, false>(t, cols, q, col_weights(t), xrow, gin, sums, mine);
+                quad_backward_strip<kStripRows, NEED_PARAMS, false>(t, cols, q, col_weights(t), kept, sums, mine);
+            kept.sync();
         }
         if (NEED_PARAMS) {
             const float s = warp_sum5(sums, lane);
@@ -264,12 +274,14 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
 #pragma unroll
         for (int i = 0; i < kStripRows; ++i, row += w)
             if (i < mine) {
-                float v[kStrip];
-                unpack2(gin[i][0], v[0], v[1]);
-                unpack2(gin[i][1], v[2], v[3]);
+                const float4 g = kept.grad_input(i);
+                float v[kStrip] = {g.x, g.y, g.z, g.w};
                 store_row4<IO, VEC>(row, q0, w, v, lane);
             }
     }
+    tmem_release();
+    __syncthreads();
+    if (warp == 0) tmem_free(tmem_base, tmem_columns(nwarps));
     if (COUNTED) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
 }
 
@@ -284,11 +296,11 @@ inline SlabShape slab_shape(int h, int w)
     return s;
 }
 inline int slab_threads(const SlabShape &s) { return 32 * s.col_tiles * (s.R / kStripRows); }
-// (the table of boxes and the per-warp sums of up to 32 filters, then the slab's input values, sit behind the stage)
+// (the table of boxes and the per-warp sums of up to 32 filters sit behind the stage)
 inline size_t slab_smem(const SlabShape &s, int F, bool sums)
 {
     return 2 * (size_t)s.stage_bytes + (size_t)F * kTapWords * sizeof(float) +
-           (sums ? (size_t)F * (slab_threads(s) / 32) * kNumSums * sizeof(float) + 16 + (size_t)slab_threads(s) * kStripRows * 16 : 0);
+           (sums ? (size_t)F * (slab_threads(s) / 32) * kNumSums * sizeof(float) : 0);
 }
 
 template <typename IO>
