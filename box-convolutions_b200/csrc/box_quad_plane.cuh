@@ -385,7 +385,7 @@ forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
 // Bound by the latencies of its phases, which other CTAs of the SM have to cover: (256,32,4,64,128) with accumulators in
 // registers and input values in shared memory, two CTAs an SM: 564 us; like this, three: 512 us.
 template <typename IO, int CT, bool FAST, bool NEED_PARAMS, bool COUNTED, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT > 256 ? 1 : FAST || NEED_PARAMS ? 3 : 2)
+__global__ void __launch_bounds__(MAXT, MAXT > 384 ? 1 : MAXT > 256 ? 2 : FAST || NEED_PARAMS ? 3 : 2)
 backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const IO *__restrict__ grad_output, BoxParams bp, IO *__restrict__ grad_input,
                      float *__restrict__ partials, int N, int C, int F, int h, int w, int row_tiles, bool normalize, bool exact,
                      bool write_gin, Finish fin)
@@ -588,15 +588,16 @@ int launch_backward_quad_t(const IO *x, const float *x_integ, const IO *grad_out
     void (*kern)(const IO *, const float *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, int, bool, bool, bool, Finish);
     const Finish fin = finish_here(bp, need_params, planes, planes * F * h * w, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w);
     auto pick = [&](auto ct, auto counted) {
-        constexpr int CT = decltype(ct)::value, S = 256, L = 512;
+        constexpr int CT = decltype(ct)::value;
         constexpr bool K = decltype(counted)::value;
-        if (tiles <= 8) {
-            if (need_params) kern = fast ? backward_quad_kernel<IO, CT, true, true, K, S> : backward_quad_kernel<IO, CT, false, true, K, S>;
-            else kern = fast ? backward_quad_kernel<IO, CT, true, false, false, S> : backward_quad_kernel<IO, CT, false, false, false, S>;
-        } else {
-            if (need_params) kern = fast ? backward_quad_kernel<IO, CT, true, true, K, L> : backward_quad_kernel<IO, CT, false, true, K, L>;
-            else kern = fast ? backward_quad_kernel<IO, CT, true, false, false, L> : backward_quad_kernel<IO, CT, false, false, false, L>;
-        }
+        auto sized = [&](auto threads) {
+            constexpr int T = decltype(threads)::value;
+            if (need_params) kern = fast ? backward_quad_kernel<IO, CT, true, true, K, T> : backward_quad_kernel<IO, CT, false, true, K, T>;
+            else kern = fast ? backward_quad_kernel<IO, CT, true, false, false, T> : backward_quad_kernel<IO, CT, false, false, false, T>;
+        };
+        if (tiles <= 8) sized(Index<256>{});
+        else if (tiles <= 12) sized(Index<384>{});      // registers for two CTAs an SM
+        else sized(Index<512>{});
     };
     if (fin.total) col_tiles == 1 ? pick(Index<1>{}, Flag<true>{}) : pick(Index<2>{}, Flag<true>{});
     else col_tiles == 1 ? pick(Index<1>{}, Flag<false>{}) : pick(Index<2>{}, Flag<false>{});

@@ -126,3 +126,33 @@ def test_narrow_parameters_are_clipped_as_floats(bc, dtype):
     bc.clip_parameters(*p, 8.0, 16.0, 8.0, 16.0, True)
     bc.clip_parameters(*wide, 8.0, 16.0, 8.0, 16.0, True)
     assert all(torch.equal(a, b.to(dtype)) for a, b in zip(p, wide))
+
+
+# one, several, 8, 9 (up to 12), 13 and 16 warps a CTA, with and without cut rows, and slabs of 4 and 5 warps: more CTAs
+# than an SM has tensor memory for, from two streams at a time
+@pytest.mark.parametrize("shape", [(8, 150, 2, 8, 96), (4, 150, 2, 33, 100), (4, 80, 2, 64, 128), (4, 80, 2, 66, 128), (4, 80, 1, 96, 70),
+                                   (2, 80, 1, 100, 128), (2, 80, 2, 64, 256), (2, 40, 2, 180, 300), (2, 30, 2, 180, 600)])
+def test_backward_from_two_streams(bc, shape):
+    """Every accumulator and input value comes back from where its own warp left it: bit for bit what a launch alone
+    returns, and that against float64."""
+    N, C, F, h, w = shape
+    rng = np.random.default_rng(h * 11 + w)
+    pix = [torch.from_numpy(p).cuda() for p in _boxes(rng, C, F, h, w, True)]
+    xs = [torch.randn(N, C, h, w, device="cuda") for _ in range(2)]
+    gos = [torch.randn(N, C * F, h, w, device="cuda") for _ in range(2)]
+
+    def run(k, dtype=torch.float32):
+        args = [t.to(dtype).requires_grad_() for t in [xs[k].detach()] + [p.detach().clone() for p in pix]]
+        out = bc.BoxConvolutionFunction.apply(*args, 1.0, 1.0, True, True)
+        return [out.detach()] + list(torch.autograd.grad(out, args, gos[k].to(dtype)))
+    alone = [run(0), run(1)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for _ in range(3):
+        got = []
+        for k in range(2):
+            with torch.cuda.stream(streams[k]):
+                got.append(run(k))
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for k in range(2) for a, b in zip(got[k], alone[k]))
+    _compare(alone[1], run(1, torch.float64))
