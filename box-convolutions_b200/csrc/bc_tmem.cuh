@@ -13,8 +13,9 @@ namespace bc {
 
 constexpr int kTmemColumns = 64;      // per warp
 
-// Columns of a CTA: warps w and w + 4 share lanes.  A power of two, at most 256 (16 warps).
-__device__ __forceinline__ uint32_t tmem_columns(int nwarps) { return nwarps > 8 ? 256u : nwarps > 4 ? 128u : 64u; }
+// Columns of a CTA of at most 16 warps with T tiles each: warps w and w + 4 share lanes.  A power of two.
+template <int T = 1>
+__device__ __forceinline__ uint32_t tmem_columns(int nwarps) { return (nwarps > 8 ? 256u : nwarps > 4 ? 128u : 64u) * T; }
 
 // One whole warp allocates and frees.  An allocation waits for columns that other CTAs of the SM hold, so a CTA
 // allocates only behind grid_dependency_wait(): one that still waits for the kernel in front must not hold what
@@ -63,21 +64,25 @@ __device__ __forceinline__ void tmem_wait_load(float4 &a)
 }
 __device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// A lane's 8 rows.  Row i's eight words: its grad-input accumulators, then the input values of row i + 1 (behind row
-// 7: those of row 0), which the gather of row i needs too, so that it fetches both at once.  All accesses are the
-// whole warp's, in converged code.
+// A lane's 8 rows of tile k of its warp's T.  Row i's eight words: its grad-input accumulators, then the input values
+// of row i + AHEAD (modulo 8) that the gather of row i needs too, so that it fetches both at once.  All accesses are
+// the whole warp's, in converged code.
+template <int AHEAD, int T = 1>
 struct TmemRows {
     uint32_t base;
     float4 g, e;
-    __device__ __forceinline__ TmemRows(uint32_t cta_base, int warp) : base(cta_base + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * kTmemColumns) {}
+    __device__ __forceinline__ TmemRows(uint32_t cta_base, int warp, int k = 0)
+        : base(cta_base + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * T + k) * kTmemColumns)
+    {
+    }
     // before the first filter: row i's input values; accumulators that are zero
     __device__ __forceinline__ void init(int i, const float4 &x)
     {
         __syncwarp();
-        tmem_store8(base + 8 * ((i + 7) & 7), make_float4(0.f, 0.f, 0.f, 0.f), x);
+        tmem_store8(base + 8 * ((i + 8 - AHEAD) & 7), make_float4(0.f, 0.f, 0.f, 0.f), x);
     }
     __device__ __forceinline__ void sync() { tmem_wait_store(); }      // between filters, and behind init()
-    __device__ __forceinline__ float4 first()
+    __device__ __forceinline__ float4 first()      // AHEAD 1: row 0's input values
     {
         float4 v;
         __syncwarp();

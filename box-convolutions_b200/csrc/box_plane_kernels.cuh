@@ -40,6 +40,7 @@
 #include "bc_finish.cuh"
 #include "bc_smem_walk.cuh"
 #include "bc_tile_io.cuh"
+#include "bc_tmem.cuh"
 #include "box_quad_plane.cuh"
 
 namespace bc {
@@ -395,16 +396,18 @@ forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, 
     }
 }
 
-// T = warp tiles per warp: grad-input accumulators are registers, so the number of strips a
-// thread owns is a compile-time constant.
+// T = warp tiles per warp: grad-input accumulators are registers, so the number of strips a thread owns is a
+// compile-time constant.
+// X_AT: where the input plane waits.  In shared memory; or nowhere, its values being read from global memory as they
+// are needed, which lets planes of up to ~48 000 pixels use this kernel; or, with the accumulators, in tensor memory
+// (bc_tmem.cuh, T = 2), where that makes room for a second CTA on the SM.
+enum XAt { X_SHARED, X_GLOBAL, X_TENSOR };
 // STAGED: the input plane and each grad_output plane arrive in shared memory by asynchronous bulk
 // copies (one instruction per plane, issued by one thread); the copy of the next grad_output
 // plane runs while the current one is gathered.
-// XSMEM: the input plane is kept in shared memory (else its values are read from global memory
-// as they are needed, which lets planes of up to ~48 000 pixels use this kernel).
 // The input plane in shared memory is float whatever IO is: float planes arrive by a bulk copy when
 // STAGED, narrow ones are converted by the threads as they are copied in.
-template <typename IO, int T, bool FAST, bool STAGED, bool NEED_PARAMS, bool XSMEM = true, bool COUNTED = false>
+template <typename IO, int T, bool FAST, bool STAGED, bool NEED_PARAMS, XAt X_AT = X_SHARED, bool COUNTED = false>
 __global__ void __launch_bounds__(512)
 backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const IO *__restrict__ grad_output, BoxParams bp,
                       IO *__restrict__ grad_input, float *__restrict__ partials, int N, int C, int F,
@@ -416,9 +419,10 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
     float *sI = reinterpret_cast<float *>(smem4);          // integral(grad_output plane)
     float *sRow = sI + layout_floats(h, w);
     float *sCol = sRow + g.ntiles * kTile;
-    float *sX = sCol + g.ntiles * kTile;                   // the input plane, pitch w (NEED_PARAMS)
-    float *sG = sX + (NEED_PARAMS && XSMEM ? npix : 0);    // staged grad_output plane, as stored (STAGED)
-    constexpr bool X_BY_COPY = STAGED && IsFloat<IO>::value;
+    float *sX = sCol + g.ntiles * kTile;                   // the input plane, pitch w (XSMEM)
+    constexpr bool X_BY_COPY = STAGED && IsFloat<IO>::value, TMEM = X_AT == X_TENSOR, XSMEM = NEED_PARAMS && X_AT == X_SHARED;
+    float *sG = sX + (XSMEM ? npix : 0);                   // staged grad_output plane, as stored (STAGED)
+    __shared__ uint32_t tmem_base;
     __shared__ __align__(16) float sTaps[kMaxFilters * kTapWords];
     __shared__ float red[16][kNumSums];
     __shared__ __align__(8) unsigned long long mbar[2];
@@ -465,13 +469,48 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
         const Box box = load_box(bp, c * F + tid);
         store_taps(sTaps + tid * kTapWords, taps_mirrored(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
     }
-    if (STAGED) __syncthreads();                           // barriers initialised before anyone waits
-    if (NEED_PARAMS && XSMEM && x_integ) {
+    __syncwarp();
+    if (TMEM && warp == nwarps - 1) tmem_alloc(&tmem_base, tmem_columns<T>(nwarps));
+    if (STAGED || TMEM) __syncthreads();                   // barriers initialised before anyone waits
+    if (TMEM) {
+        tmem_acquire();
+        const IO *xp = x + nc * (int64_t)npix;
+        const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1);
+#pragma unroll
+        for (int k = 0; k < T; ++k) {
+            if (!st[k].tile) continue;
+            TmemRows<0, T> kept(tmem_base, warp, k);
+#pragma unroll
+            for (int i = 0; i < kR; ++i) {
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (st[k].active && (FAST || st[k].p0 + i < h)) {
+                    if (x_integ) {      // the caller has only the input's integral image: its pixels are second differences
+                        const float *Ip = I + (int64_t)(st[k].p0 + i) * (w + 1) + st[k].q0;
+                        v.x = pixel_of_integral(Ip, w + 1);
+                        if (st[k].q0 + 1 < w) v.y = pixel_of_integral(Ip + 1, w + 1);
+                        if (st[k].q0 + 2 < w) v.z = pixel_of_integral(Ip + 2, w + 1);
+                        if (st[k].q0 + 3 < w) v.w = pixel_of_integral(Ip + 3, w + 1);
+                    } else if (FAST) {
+                        v = Io<IO>::load4(xp + st[k].pix + i * w);
+                    } else {
+                        const IO *row = xp + st[k].pix + i * w;
+                        v.x = Io<IO>::load1(row);
+                        if (st[k].q0 + 1 < w) v.y = Io<IO>::load1(row + 1);
+                        if (st[k].q0 + 2 < w) v.z = Io<IO>::load1(row + 2);
+                        if (st[k].q0 + 3 < w) v.w = Io<IO>::load1(row + 3);
+                    }
+                }
+                kept.init(i, v);
+            }
+        }
+        tmem_wait_store();
+    }
+    if (XSMEM && x_integ) {
         // (read by the first gather, which follows the barriers of the first build)
         const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1);
         for (int p = warp; p < h; p += nwarps)
             for (int q = lane; q < w; q += 32) sX[p * w + q] = pixel_of_integral(I + p * (w + 1) + q, w + 1);
-    } else if (!X_BY_COPY && NEED_PARAMS && XSMEM) {
+    } else if (!X_BY_COPY && XSMEM) {
         // (read by the first gather, which follows the barriers of the first build)
         const IO *xp = x + nc * (int64_t)npix;
         if (FAST) {
@@ -527,27 +566,38 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
         f2_t leftP = pack2(0.f, 0.f), leftQ = pack2(0.f, 0.f), rightP = pack2(0.f, 0.f), rightQ = pack2(0.f, 0.f);
 #pragma unroll
         for (int k = 0; k < T; ++k) {
-            if (st[k].active) {
+            if (TMEM ? st[k].tile : st[k].active) {
                 const Walk wk = make_walk(sI32, t, st[k].q0, g);
                 if (NEED_PARAMS) {
+                    TmemRows<0, T> kept(TMEM ? tmem_base : 0u, warp, k);
                     f2_t pd[kStrip], pel[kStrip], peh[kStrip];
-                    load_pair_e(wk, st[k].p0 + t.lo_r - 1, st[k].p0 + t.hi_r, cw, pd, pel, peh);
+                    if (!TMEM || st[k].active) load_pair_e(wk, st[k].p0 + t.lo_r - 1, st[k].p0 + t.hi_r, cw, pd, pel, peh);
                     uint32_t xa = sX32 + st[k].pix * 4;
-                    const IO *xg = x + nc * (int64_t)npix + st[k].pix;         // used when !XSMEM
+                    const IO *xg = x + nc * (int64_t)npix + st[k].pix;         // X_GLOBAL
 #pragma unroll
                     for (int i = 0; i < kR; ++i) {
                         const int p = st[k].p0 + i;
-                        if (FAST || p < h) {
-                            f2_t cd[kStrip], cel[kStrip], ceh[kStrip];
-                            load_pair_e(wk, p + t.lo_r, p + t.hi_r + 1, cw, cd, cel, ceh);
-                            float xv[kStrip];
-                            if (FAST) {
+                        const bool there = (!TMEM || st[k].active) && (FAST || p < h);
+                        f2_t cd[kStrip], cel[kStrip], ceh[kStrip];
+                        float xv[kStrip], gg[kStrip];
+                        if (TMEM) {
+                            __syncwarp();
+                            kept.fetch(i);
+                        }
+                        if (there) load_pair_e(wk, p + t.lo_r, p + t.hi_r + 1, cw, cd, cel, ceh);
+                        if (TMEM) {
+                            __syncwarp();
+                            const float4 v = kept.next();
+                            xv[0] = v.x; xv[1] = v.y; xv[2] = v.z; xv[3] = v.w;
+                        }
+                        if (there) {
+                            if (TMEM) {
+                            } else if (FAST) {
                                 const float4 v = XSMEM ? lds128(xa) : Io<IO>::load4(xg);
                                 xv[0] = v.x; xv[1] = v.y; xv[2] = v.z; xv[3] = v.w;
                             } else {
 #pragma unroll
-                                for (int m = 0; m < kStrip; ++m)
-                                    xv[m] = st[k].q0 + m < w ? (XSMEM ? sX[p * w + st[k].q0 + m] : Io<IO>::load1(xg + m)) : 0.0f;
+                                for (int m = 0; m < kStrip; ++m) xv[m] = st[k].q0 + m < w ? (XSMEM ? sX[p * w + st[k].q0 + m] : Io<IO>::load1(xg + m)) : 0.0f;
                             }
                             xa += w * 4;
                             xg += w;
@@ -560,10 +610,10 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
                                 unpack2(cd[m], lo_new, hi_new);
                                 unpack2(pd[m], lo_old, hi_old);
                                 unpack2(dd, top, bot);
-                                const float gg = (hi_old - lo_new) + t.f_hi_r * bot + t.f_lo_r * top;
+                                gg[m] = (hi_old - lo_new) + t.f_hi_r * bot + t.f_lo_r * top;
                                 topbot2 = fma2(xx, dd, topbot2);
-                                s_out += xv[m] * gg;
-                                gin[k][i][m] += gg * t.scale;
+                                s_out += xv[m] * gg[m];
+                                if (!TMEM) gin[k][i][m] += gg[m] * t.scale;
                                 // e_lo / e_hi: the two column strips
                                 leftP = fma2(xx, pel[m], leftP);
                                 leftQ = fma2(xx, cel[m], leftQ);
@@ -571,6 +621,14 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
                                 rightQ = fma2(xx, ceh[m], rightQ);
                                 pd[m] = cd[m]; pel[m] = cel[m]; peh[m] = ceh[m];
                             }
+                        }
+                        if (TMEM) {
+                            if (there) {
+                                kept.g.x += gg[0] * t.scale; kept.g.y += gg[1] * t.scale;
+                                kept.g.z += gg[2] * t.scale; kept.g.w += gg[3] * t.scale;
+                            }
+                            __syncwarp();
+                            tmem_store4(kept.base + 8 * i, kept.g);
                         }
                     }
                 } else {
@@ -597,6 +655,7 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
                 }
             }
         }
+        if (TMEM) tmem_wait_store();
         if (NEED_PARAMS) {
             float tb_top, tb_bot, la, lc, lb, ld, ra, rc, rb, rd;
             unpack2(topbot2, tb_top, tb_bot);
@@ -628,6 +687,14 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
         IO *gi = grad_input + nc * (int64_t)npix;
 #pragma unroll
         for (int k = 0; k < T; ++k) {
+            if (TMEM && st[k].tile) {
+                TmemRows<0, T> kept(tmem_base, warp, k);
+#pragma unroll
+                for (int i = 0; i < kR; ++i) {
+                    const float4 v = kept.grad_input(i);
+                    gin[k][i][0] = v.x; gin[k][i][1] = v.y; gin[k][i][2] = v.z; gin[k][i][3] = v.w;
+                }
+            }
             if (st[k].active) {
                 IO *dst = gi + st[k].pix;
 #pragma unroll
@@ -642,6 +709,11 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
                 }
             }
         }
+    }
+    if (TMEM) {
+        tmem_release();
+        __syncthreads();
+        if (warp == 0) tmem_free(tmem_base, tmem_columns<T>(nwarps));
     }
     if (COUNTED) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
 }
@@ -756,29 +828,38 @@ int launch_backward_plane_t(const IO *x, const float *x_integ, const IO *grad_ou
                       (!write_gin || aligned_to(grad_input, vec));
     // bulk copies need 16-byte aligned planes of a multiple of 16 bytes and room for the staging buffer;
     // staging must not cost a resident CTA (two fit below ~112 KB each)
-    // the input plane joins the integral image in shared memory when both fit
-    const bool xsmem = !need_params || plane_backward_smem_bytes(h, w, true, false, io) <= kMaxSmem;
-    const size_t with_staging = plane_backward_smem_bytes(h, w, need_params, true, io);
+    // More than eight tiles.  Rows that no vector access fits: the input plane goes to tensor memory, read once with scalar
+    // loads instead of once a filter from wherever it is ((16,32,4,100,200) backward 373 -> 314 us, (8,32,4,300,60) 189 -> 150).
+    // Else it joins the integral image in shared memory, unless the two then leave no room for a second CTA that there
+    // would be planes for: (24,32,4,96,160) 275 -> 220 us; both reasons: (16,32,4,93,157) 310 -> 173 us.  Where two CTAs fit
+    // anyway, or only one by its registers, tensor memory is slower: (8,16,4,128,256) 80 -> 90 us, a wait and
+    // two warp barriers a row.
     const size_t two_ctas = 112 * 1024;
-    const bool staged = fast && T == 1 && xsmem && with_staging <= kMaxSmem && aligned_to(grad_output, 16) &&
+    const bool tensor = need_params && T > 1 &&
+                        (!fast || (warps <= 8 && planes > 148 && plane_backward_smem_bytes(h, w, true, false, io) > two_ctas &&
+                                   plane_backward_smem_bytes(h, w, false, false, io) <= two_ctas));
+    const bool xsmem = need_params && !tensor && plane_backward_smem_bytes(h, w, true, false, io) <= kMaxSmem;
+    const size_t with_staging = plane_backward_smem_bytes(h, w, xsmem, true, io);
+    const bool staged = fast && T == 1 && (xsmem || !need_params) && with_staging <= kMaxSmem && aligned_to(grad_output, 16) &&
                         aligned_to(x, 16) && ((size_t)h * w * io) % 16 == 0 &&
-                        (with_staging <= two_ctas || plane_backward_smem_bytes(h, w, need_params, false, io) > two_ctas);
-    const size_t smem = plane_backward_smem_bytes(h, w, need_params && xsmem, staged, io);
+                        (with_staging <= two_ctas || plane_backward_smem_bytes(h, w, xsmem, false, io) > two_ctas);
+    const size_t smem = plane_backward_smem_bytes(h, w, xsmem, staged, io);
     void (*kern)(const IO *, const float *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, bool, bool, bool, Finish);
     const Finish fin = finish_here(bp, need_params, planes, planes * F * h * w, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w);
     auto pick = [&](auto counted) {
         constexpr bool K = decltype(counted)::value;
-        if (!xsmem) {
-            if (fast) kern = T == 1 ? backward_plane_kernel<IO, 1, true, false, true, false, K> : backward_plane_kernel<IO, 2, true, false, true, false, K>;
-            else kern = T == 1 ? backward_plane_kernel<IO, 1, false, false, true, false, K> : backward_plane_kernel<IO, 2, false, false, true, false, K>;
+        if (tensor) {
+            kern = fast ? backward_plane_kernel<IO, 2, true, false, true, X_TENSOR, K> : backward_plane_kernel<IO, 2, false, false, true, X_TENSOR, K>;
+        } else if (need_params && !xsmem) {
+            kern = backward_plane_kernel<IO, 2, true, false, true, X_GLOBAL, K>;      // (planes of up to eight tiles always fit)
         } else if (staged) {
-            kern = need_params ? backward_plane_kernel<IO, 1, true, true, true, true, K> : backward_plane_kernel<IO, 1, true, true, false>;
+            kern = need_params ? backward_plane_kernel<IO, 1, true, true, true, X_SHARED, K> : backward_plane_kernel<IO, 1, true, true, false>;
         } else if (fast) {
-            kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, true, false, true, true, K> : backward_plane_kernel<IO, 1, true, false, false>)
-                          : (need_params ? backward_plane_kernel<IO, 2, true, false, true, true, K> : backward_plane_kernel<IO, 2, true, false, false>);
+            kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, true, false, true, X_SHARED, K> : backward_plane_kernel<IO, 1, true, false, false>)
+                          : (need_params ? backward_plane_kernel<IO, 2, true, false, true, X_SHARED, K> : backward_plane_kernel<IO, 2, true, false, false>);
         } else {
-            kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, false, false, true, true, K> : backward_plane_kernel<IO, 1, false, false, false>)
-                          : (need_params ? backward_plane_kernel<IO, 2, false, false, true, true, K> : backward_plane_kernel<IO, 2, false, false, false>);
+            kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, false, false, true, X_SHARED, K> : backward_plane_kernel<IO, 1, false, false, false>)
+                          : backward_plane_kernel<IO, 2, false, false, false>;
         }
     };
     if (fin.total) pick(Flag<true>{});

@@ -418,7 +418,7 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
     }
     __syncthreads();
     tmem_acquire();
-    TmemRows kept(tmem_base, warp);
+    TmemRows<1> kept(tmem_base, warp);
     if (NEED_PARAMS) {
         if (!x) {
             // the caller has only the input's integral image: its pixels are second differences

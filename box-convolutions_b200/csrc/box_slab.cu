@@ -205,7 +205,7 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
     if (warp == nwarps - 1) tmem_alloc(&tmem_base, tmem_columns(nwarps));
     __syncthreads();
     tmem_acquire();
-    TmemRows kept(tmem_base, warp);
+    TmemRows<1> kept(tmem_base, warp);
     if (threadIdx.x == 0) {
         fence_proxy_async();
         slab_issue(planes, pitch, load_taps(sTaps), p_slab, rows, h, stage32, stage32 + sh.stage_bytes, mbar32);
