@@ -11,8 +11,8 @@
 // output instead of 2.5, two copy instructions instead of thousands of 16-byte ones, and reads shared
 // memory with 5 (R+1)/R words an output instead of 8.
 //
-// Bound by the shared-memory pipe (77 % in the forward) and the issue slots (68 % / 61 %); the data comes from L2.
-// (8,16,4,256,512): forward 164 -> 86 us, backward 211 -> 121 us against column bands.  A training step of
+// Bound by the shared-memory pipe (77 % in the forward) and the issue slots (67 %); the data comes from L2.
+// (8,16,4,256,512): forward 164 -> 86 us, backward 211 -> 121 us against column bands, 113 us with tensor memory.  A training step of
 // (8,16,4,128,256) planes on whole-plane kernels takes the same time, so those stay there.
 #include "bc_common.cuh"
 #include "bc_finish.cuh"
