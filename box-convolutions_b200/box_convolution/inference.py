@@ -34,7 +34,8 @@ def fused_box_block(module, input, *, input_relu=False, scale=None, shift=None, 
               first so that they have been clipped once, as the reference does);
     scale, shift  tensors of ``in_planes * num_filters`` values or None;
     residual  tensor of the output's shape or None;
-    out       where to write (may be ``residual`` for an in-place skip connection); allocated if None.
+    out       where to write (may be ``residual`` for an in-place skip connection, and with one filter also
+              ``input``); allocated if None.
     """
     return _native.fused_block(
         input, module.x_min, module.x_max, module.y_min, module.y_max,

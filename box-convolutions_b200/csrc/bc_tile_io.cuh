@@ -282,6 +282,12 @@ __device__ __forceinline__ void store_row4_wide(IO *row, int c, int w, const flo
 
 inline bool aligned_to(const void *p, int bytes) { return (reinterpret_cast<uintptr_t>(p) & (uintptr_t)(bytes - 1)) == 0; }
 
+inline bool ranges_overlap(const void *a, size_t a_bytes, const void *b, size_t b_bytes)
+{
+    const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
+    return p < q + b_bytes && q < p + a_bytes;
+}
+
 // Bounded waits that expired in the kernels of this translation unit (synchronises).
 inline int read_wait_timeouts_here(int *count)
 {

@@ -534,9 +534,11 @@ int launch_forward_quad_t(const IO *x, const float *integ, const BoxParams &bp, 
                       (!fu || !fu->residual || aligned_to(fu->residual, 16));
     const int T = tiles > 8 ? 2 : 1;
     // Planes of more than 16 tiles that leave SMs idle: CTAs that each gather a part of the rows, from integral images of
-    // their own ((1,16,4,128,256), 64 -> 128 CTAs: 12.0 -> 9.8 us a block tail).
+    // their own ((1,16,4,128,256), 64 -> 128 CTAs: 12.0 -> 9.8 us a block tail).  Not where the output lies over the input
+    // (one filter, in place): a CTA that starts late would integrate rows that another has already replaced.
     int rsplit = 1;
-    while (tiles > 16 && planes * fsplit * rsplit * 2 <= 148 && rsplit < 4) rsplit *= 2;
+    const bool in_place = x && ranges_overlap(x, (size_t)planes * h * w * sizeof(IO), out, (size_t)planes * F * h * w * sizeof(IO));
+    while (!in_place && tiles > 16 && planes * fsplit * rsplit * 2 <= 148 && rsplit < 4) rsplit *= 2;
     const int warps = (tiles + T - 1) / T, nf = (F + fsplit - 1) / fsplit;
     // rows per task: few long tasks read fewer tap rows twice, but every warp should get the same share
     int chunk = 1;

@@ -118,6 +118,22 @@ def test_fused_tail_edges(bc, shape):
         assert (got - want).abs().max() <= 2e-5 * max(1.0, want.abs().max().item())
 
 
+# one filter: input, residual and output may be the same tensor; whole planes of one and of more than sixteen tiles, which
+# would be split by rows, 32 x 32 tiles, and slabs
+@pytest.mark.parametrize("shape", [(1, 3, 64, 128), (1, 16, 128, 256), (1, 4, 121, 250), (1, 5, 40, 50), (1, 2, 201, 300)])
+def test_fused_tail_over_its_own_input(bc, shape):
+    N, C, h, w = shape
+    m = bc.BoxConv2d(C, 1, h, w).cuda().eval()
+    x = torch.randn(N, C, h, w, device="cuda")
+    want = bc.fused_box_block(m, x, input_relu=True, residual=x, output_relu=True)
+    with torch.no_grad():
+        assert (want - torch.relu(m(torch.relu(x)) + x)).abs().max() <= 2e-5 * max(1.0, want.abs().max().item())
+    for _ in range(20):
+        got = x.clone()
+        assert bc.fused_box_block(m, got, input_relu=True, residual=got, output_relu=True, out=got) is got
+        assert (got - want).abs().max() <= 2e-5 * max(1.0, want.abs().max().item())
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_narrow_parameters_are_clipped_as_floats(bc, dtype):
     """One launch clips 16-bit parameters: float arithmetic on their values, rounded when stored."""
