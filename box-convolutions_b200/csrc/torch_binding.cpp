@@ -333,6 +333,11 @@ Gradients box_backward(const Tensor &integrated, Four p, const Tensor &grad_outp
     return out;
 }
 
+bool all_contiguous(const Four &p)
+{
+    return p[0].is_contiguous() && p[1].is_contiguous() && p[2].is_contiguous() && p[3].is_contiguous();
+}
+
 // In place; `packed` (float32 and narrower): also returns a packed float32 copy of the clipped values.
 Snapshot clip(const Four &p, double rep_h, double rep_w, double max_h, double max_w, bool exact, bool packed)
 {
@@ -344,8 +349,7 @@ Snapshot clip(const Four &p, double rep_h, double rep_w, double max_h, double ma
         require_cuda_float(p[i], kParamNames[i], dtype, true);
     }
     if (packed && dtype == at::kDouble) fail("box_convolution: a packed copy is made of float32 or narrower parameters only");
-    if (is_narrow(dtype) && !packed &&
-        !(p[0].is_contiguous() && p[1].is_contiguous() && p[2].is_contiguous() && p[3].is_contiguous())) {
+    if (is_narrow(dtype) && !packed && !all_contiguous(p)) {
         Four dense;
         for (int i = 0; i < 4; ++i) dense[i] = p[i].contiguous();
         clip(dense, rep_h, rep_w, max_h, max_w, exact, false);
@@ -664,9 +668,16 @@ PyObject *py_module_forward(PyObject *, PyObject *const *v, Py_ssize_t n)
         py::gil_scoped_release release;
         // the launch that clips also leaves the copy of the parameters that backward will use
         if (clipping) {
-            const Snapshot snap = clip(p, o.rep_h, o.rep_w, max_h, max_w, o.exact, p[0].scalar_type() != at::kDouble);
-            o.snapshot = snap.packed;
-            o.counters = snap.counters;
+            const at::ScalarType dtype = p[0].scalar_type();
+            if (is_narrow(dtype) && !all_contiguous(p)) {
+                // (clipped in copies and written back, without counting as a change to the parameters in place)
+                clip({p[0].variable_data(), p[1].variable_data(), p[2].variable_data(), p[3].variable_data()}, o.rep_h, o.rep_w,
+                     max_h, max_w, o.exact, false);
+            } else {
+                const Snapshot snap = clip(p, o.rep_h, o.rep_w, max_h, max_w, o.exact, dtype != at::kDouble);
+                o.snapshot = snap.packed;
+                o.counters = snap.counters;
+            }
         }
         out = apply(input, p, o);
     }

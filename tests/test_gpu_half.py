@@ -99,3 +99,23 @@ def test_half_module_and_need_mask(bc, dtype):
     with torch.no_grad():
         again = m(x)
     assert torch.equal(again, out.detach())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_half_module_trains_with_parameters_that_are_not_contiguous(bc, dtype):
+    """Clipped in copies and written back: the step of the module whose parameters are the same values in a row."""
+    torch.manual_seed(7)
+    m = bc.BoxConv2d(3, 4, 64, 128).cuda().to(dtype)
+    with torch.no_grad():
+        m.x_min[0, 0] = 0.9; m.y_max[2, 1] = m.y_min[2, 1]         # one border to pull back, one box to re-open
+    t = bc.BoxConv2d(3, 4, 64, 128).cuda().to(dtype)
+    for name in ("x_min", "x_max", "y_min", "y_max"):
+        setattr(t, name, torch.nn.Parameter(getattr(m, name).detach().t().contiguous().t()))
+    x, go = torch.randn(2, 3, 64, 128, device="cuda").to(dtype), torch.randn(2, 12, 64, 128, device="cuda").to(dtype)
+    outs = []
+    for net in (m, t):
+        y = net(x)
+        y.backward(go)
+        outs.append([y] + [p for p in net.parameters()] + [p.grad for p in net.parameters()])
+    assert not t.x_min.is_contiguous()
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
