@@ -29,8 +29,22 @@ __device__ __forceinline__ BoxTaps load_taps_uniform(const float *tab)
     return t;
 }
 
-// Inclusive sum over the warp, or over each group of LN lanes; the shuffle's own predicate tells which lanes have
-// somebody to add.
+// Inclusive sum over the warp, or over each group of LN lanes, and in `before` the sum of the lanes in front, which is
+// added up by itself: taking a lane's own value off again would leave its infinity or its rounding in the columns to
+// its left.  The shuffle's own predicate tells which lanes have somebody to add.
+template <int LN = 32>
+__device__ __forceinline__ float warp_prefix(float v, float &before)
+{
+    before = 0.0f;
+#pragma unroll
+    for (int d = 1; d < LN; d <<= 1)
+        asm volatile("{\n .reg .f32 u;\n .reg .pred p;\n shfl.sync.up.b32 u|p, %0, %2, %3, 0xffffffff;\n @p add.f32 %1, %1, u;\n"
+                     " @p add.f32 %0, %0, u;\n}"
+                     : "+f"(v), "+f"(before) : "r"(d), "n"((32 - LN) << 8));
+    return v;
+}
+
+// The inclusive sum alone.
 template <int LN = 32>
 __device__ __forceinline__ float warp_scan(float v)
 {

@@ -240,8 +240,7 @@ integral_tile_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, 
             v[i].y += up.y + v[i].x;
             v[i].z += up.z + v[i].y;
             v[i].w += up.w + v[i].z;
-            const float incl = warp_scan<LN>(v[i].w);
-            carry[i] = incl - v[i].w;
+            const float incl = warp_prefix<LN>(v[i].w, carry[i]);
             if (LN == 32 && W > 1 && lane == 31) sTot[warp][i] = incl;
         }
         __syncthreads();

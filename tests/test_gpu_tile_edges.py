@@ -39,6 +39,23 @@ def test_integral_image_edges(bc, planes, h, w):
     assert ((bc.integral_image(flat)[:, 1:, 1:].double() - want).abs() <= 1e-5 * want).all()
 
 
+# a value that is infinite, not a number or just large stays where it belongs: below and to the right of its pixel
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 1e30])
+@pytest.mark.parametrize("planes,h,w", [(2, 50, 50), (3, 33, 31), (1, 63, 129), (2, 20, 250), (2, 40, 256), (1, 16, 24), (150, 140, 130)])
+def test_integral_image_does_not_spread_values_to_the_left(bc, planes, h, w, value):
+    x = torch.rand(planes, h, w, device="cuda", generator=torch.Generator("cuda").manual_seed(h * w))
+    for r, c in ((0, 0), (7, 3), (h // 2, w // 2), (h - 1, w - 1), (h - 3, 5)):
+        x[0, r, c] = 0
+        want = bc.integral_image(x)
+        x[0, r, c] = value
+        got = bc.integral_image(x)
+        x[0, r, c] = 0.5
+        touched = torch.zeros_like(got, dtype=torch.bool)
+        touched[0, r + 1:, c + 1:] = True
+        assert torch.equal(got[~touched], want[~touched]), (r, c)
+        assert not torch.isfinite(got[touched]).any() if value != 1e30 else ((got[touched] / value - 1).abs() < 1e-6).all()
+
+
 def _boxes(rng, C, F, h, w, exact):
     lo = 0.3 if exact else 1.2
     cx = rng.uniform(-h / 2, h / 2, (C, F)); ex = rng.uniform(lo, h / 3 + lo, (C, F))
