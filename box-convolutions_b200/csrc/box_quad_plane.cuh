@@ -135,15 +135,13 @@ __device__ __forceinline__ void quad_scan(QuadBlock &v, float (&carry)[kTileRows
     float4 p = lds128(mine), q = lds128(mine + 16);
     p.y += p.x; p.z += p.y; p.w += p.z;
     q.x += p.w; q.y += q.x; q.z += q.y; q.w += q.z;
-    float before = q.w;
-    {
-        const float u1 = __shfl_up_sync(0xffffffffu, before, 1);
-        if (k >= 1) before += u1;
-        const float u2 = __shfl_up_sync(0xffffffffu, before, 2);
-        if (k >= 2) before += u2;
-    }
-    if (CT > 1 && k == 3) sts<0>(s.row + (t.rt * CT + t.ct) * 32 + (lane >> 2) * 4, before);
-    before -= q.w;
+    // What the row has in front of the four lanes' shares, added up by itself: taking a lane's own share off an inclusive
+    // sum again would leave its infinity or its rounding in the 32 columns to its left.
+    const float one = __shfl_up_sync(0xffffffffu, q.w, 1);
+    float before = k >= 1 ? one : 0.0f;
+    const float two = __shfl_up_sync(0xffffffffu, q.w + before, 2);
+    if (k >= 2) before += two;
+    if (CT > 1 && k == 3) sts<0>(s.row + (t.rt * CT + t.ct) * 32 + (lane >> 2) * 4, before + q.w);
     sts128(mine, make_float4(before, before + p.x, before + p.y, before + p.z));
     sts128(mine + 16, make_float4(before + p.w, before + q.x, before + q.y, before + q.z));
     __syncwarp();

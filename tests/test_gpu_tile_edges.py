@@ -105,6 +105,27 @@ def test_training_edges_against_float64(bc, shape, normalize, exact):
     assert all(g[0, 0] == 0 for g in runs[0][2:])
 
 
+# whole planes in 8 x 128 tiles, one and two a row, and slabs: a column of large or infinite values has no effect on
+# boxes that end to the left of it
+@pytest.mark.parametrize("value", [1e8, float("inf"), float("nan")])
+@pytest.mark.parametrize("shape", [(1, 2, 2, 64, 128), (1, 2, 2, 56, 240), (1, 2, 2, 128, 256), (1, 2, 2, 60, 116), (1, 1, 2, 201, 300)])
+def test_large_values_stay_on_their_side(bc, shape, value):
+    N, C, F, h, w = shape
+    gen = torch.Generator("cuda").manual_seed(w)
+    x = torch.randn(N, C, h, w, device="cuda", generator=gen)
+    go = torch.randn(N, C * F, h, w, device="cuda", generator=gen)
+    pix = [torch.full((C, F), v, device="cuda") for v in (-2.3, 1.6, -3.4, 2.7)]
+    runs = []
+    for last in (0.0, value):
+        x[..., -1] = last
+        go[..., -1] = last
+        a = x.clone().requires_grad_()
+        out = bc.BoxConvolutionFunction.apply(a, *pix, 1.0, 1.0, True, True)
+        runs.append([out.detach(), torch.autograd.grad(out, a, go)[0]])
+    for clean, got in zip(*runs):
+        assert torch.equal(got[..., :w - 8], clean[..., :w - 8])      # (the boxes reach less than five columns)
+
+
 # the same through the four functions, which gather from the caller's integral image
 @pytest.mark.parametrize("shape", [(1, 2, 2, 64, 128), (2, 2, 3, 33, 70), (1, 2, 2, 96, 160), (1, 1, 2, 121, 250), (1, 2, 2, 201, 257)])
 def test_four_functions_edges_against_float64(bc, shape):
