@@ -8,7 +8,7 @@ import torch
 
 from . import _torch_binding as _native
 from . import ext
-from .function import reparametrize
+from .function import BoxConvolutionFunction, reparametrize
 
 
 class BoxConv2d(torch.nn.Module):
@@ -92,10 +92,18 @@ class BoxConv2d(torch.nn.Module):
             x_min, x_max, y_min, y_max = own["x_min"], own["x_max"], own["y_min"], own["y_max"]
         except KeyError:        # parametrised or replaced by plain tensors
             x_min, x_max, y_min, y_max = self._parameters4()
-        return _native.module_forward(
+        output = _native.module_forward(
             input, x_min, x_max, y_min, y_max,
             self.reparametrization_h, self.reparametrization_w, self.normalize, self.exact,
             self.training, self.max_input_h, self.max_input_w)
+        if output is not NotImplemented:
+            return output
+        # inside a trace, a function transform or forward-mode differentiation
+        if self.training:
+            self._clip_parameters()
+        return BoxConvolutionFunction.apply(
+            input, x_min, x_max, y_min, y_max,
+            self.reparametrization_h, self.reparametrization_w, self.normalize, self.exact)
 
     def draw_boxes(self, channels=None, resolution=(600, 600), weights=None):
         """Rasterises the boxes into an ``(H, W, 3)`` uint8 numpy image for debugging: the frame

@@ -7,6 +7,7 @@
 // a step where the kernels of a (1, 8, 4, 32, 32) block take 15.  Here the checks, the allocations and the
 // autograd node are C++, and the functions are plain CPython fast calls, because converting a dozen
 // arguments through a generic binding layer costs as much as launching a kernel.
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -524,8 +525,21 @@ struct BoxConvolutionBackward : torch::autograd::Node {
         params.reset();
     }
 
-    std::string name() const override { return "BoxConvolutionBackward"; }
+    std::string name() const override { return "BoxConvolutionFunctionBackward"; }
 };
+
+// Calls that the node cannot serve and that go through the Python class, a torch.autograd.Function: a trace records it
+// as an operation (this call would leave its result in the trace as a constant), and it refuses tangents of
+// forward-mode differentiation and function transforms (which would pass by unseen).
+bool needs_python_function(const Tensor &input, const Four &p)
+{
+    using c10::impl::tls_is_dispatch_key_included;
+    if (tls_is_dispatch_key_included(at::DispatchKey::Tracer) ||
+        tls_is_dispatch_key_included(at::DispatchKey::FuncTorchDynamicLayerFrontMode))
+        return true;
+    auto has_tangent = [](const Tensor &t) { return t._fw_grad(/*level=*/0).defined(); };
+    return has_tangent(input) || has_tangent(p[0]) || has_tangent(p[1]) || has_tangent(p[2]) || has_tangent(p[3]);
+}
 
 Tensor apply(const Tensor &input, const Four &p, const Options &o)
 {
@@ -654,6 +668,7 @@ PyObject *wrap(const Tensor &t)
 }
 
 // module_forward(input, x_min, x_max, y_min, y_max, rep_h, rep_w, normalize, exact, clip, max_h, max_w)
+//   -> NotImplemented, with nothing done, where the Python class has to be called
 PyObject *py_module_forward(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
     HANDLE_TH_ERRORS
@@ -663,6 +678,7 @@ PyObject *py_module_forward(PyObject *, PyObject *const *v, Py_ssize_t n)
     Options o{a.number(), a.number(), a.flag(), a.flag(), Tensor()};
     const bool clipping = a.flag();
     const double max_h = a.number(), max_w = a.number();
+    if (needs_python_function(input, p)) Py_RETURN_NOTIMPLEMENTED;
     Tensor out;
     {
         py::gil_scoped_release release;
@@ -685,7 +701,7 @@ PyObject *py_module_forward(PyObject *, PyObject *const *v, Py_ssize_t n)
     END_HANDLE_TH_ERRORS
 }
 
-// apply(input, x_min, x_max, y_min, y_max, rep_h, rep_w, normalize, exact, snapshot or None)
+// apply(input, x_min, x_max, y_min, y_max, rep_h, rep_w, normalize, exact, snapshot or None) -> output or NotImplemented
 PyObject *py_apply(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
     HANDLE_TH_ERRORS
@@ -694,12 +710,67 @@ PyObject *py_apply(PyObject *, PyObject *const *v, Py_ssize_t n)
     const Four p = a.params();
     Options o{a.number(), a.number(), a.flag(), a.flag(), Tensor()};
     o.snapshot = a.optional_tensor("snapshot");
+    if (needs_python_function(input, p)) Py_RETURN_NOTIMPLEMENTED;
     Tensor out;
     {
         py::gil_scoped_release release;
         out = apply(input, p, o);
     }
     return wrap(out);
+    END_HANDLE_TH_ERRORS
+}
+
+// The two halves of the Python class.
+// forward_saved(arguments of apply) -> (output, and the two tensors that backward_saved needs)
+PyObject *py_forward_saved(PyObject *, PyObject *const *v, Py_ssize_t n)
+{
+    HANDLE_TH_ERRORS
+    Args a(v, n, 10);
+    const Tensor input = a.tensor("input");
+    const Four p = a.params();
+    Options o{a.number(), a.number(), a.flag(), a.flag(), Tensor()};
+    o.snapshot = a.optional_tensor("snapshot");
+    Tensor out;
+    Kept keep;
+    {
+        py::gil_scoped_release release;
+        at::NoGradGuard no_grad;
+        at::tracer::impl::NoTracerDispatchMode no_tracer;      // (a trace records the function as a whole)
+        out = forward_any(input, p, o, &keep);
+    }
+    if (c10::impl::tls_is_dispatch_key_included(at::DispatchKey::Tracer)) {      // an output whose allocation the trace has seen
+        const Tensor seen = at::empty(out.sizes(), out.options());
+        at::tracer::impl::NoTracerDispatchMode no_tracer;
+        seen.copy_(out);
+        out = seen;
+    }
+    THPObjectPtr list(PyTuple_New(3));
+    if (!list) throw python_error();
+    PyTuple_SET_ITEM(list.get(), 0, wrap(out));
+    PyTuple_SET_ITEM(list.get(), 1, wrap(keep.x));
+    PyTuple_SET_ITEM(list.get(), 2, wrap(keep.params));
+    return list.release();
+    END_HANDLE_TH_ERRORS
+}
+
+// backward_saved(the two tensors, grad_output, rep_h, rep_w, normalize, exact, need_mask) -> five gradients or None
+PyObject *py_backward_saved(PyObject *, PyObject *const *v, Py_ssize_t n)
+{
+    HANDLE_TH_ERRORS
+    Args a(v, n, 8);
+    const Tensor x = a.tensor("input"), params = a.tensor("parameters"), g = a.tensor("grad_output");
+    const Options o{a.number(), a.number(), a.flag(), a.flag(), Tensor()};
+    const int mask = (int)a.integer();
+    Gradients out;
+    {
+        py::gil_scoped_release release;
+        at::NoGradGuard no_grad;
+        out = backward_any(x, params, g, o, g.scalar_type(), mask);      // (the engine hands over the output's type)
+    }
+    THPObjectPtr list(PyList_New(5));
+    if (!list) throw python_error();
+    for (int i = 0; i < 5; ++i) PyList_SET_ITEM(list.get(), i, wrap(out[i]));
+    return list.release();
     END_HANDLE_TH_ERRORS
 }
 
@@ -805,7 +876,7 @@ PyObject *py_fused_block(PyObject *, PyObject *const *v, Py_ssize_t n)
 }
 
 #define BC_FAST(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {BC_FAST(module_forward), BC_FAST(apply), BC_FAST(integral_image), BC_FAST(box_forward),
+PyMethodDef methods[] = {BC_FAST(module_forward), BC_FAST(apply), BC_FAST(forward_saved), BC_FAST(backward_saved), BC_FAST(integral_image), BC_FAST(box_forward),
                          BC_FAST(box_backward), BC_FAST(clip), BC_FAST(fused_block), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_torch_binding", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

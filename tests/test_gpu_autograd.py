@@ -1,0 +1,74 @@
+"""What PyTorch asks of an autograd function besides a gradient: traces, saved-tensor hooks, forward-mode
+differentiation, function transforms, gradients that are not there."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def bc():
+    import box_convolution
+    assert torch.cuda.is_available()
+    return box_convolution
+
+
+def _module(bc, dtype=torch.float32, shape=(2, 3, 4, 40, 72)):
+    N, C, F, h, w = shape
+    torch.manual_seed(3)
+    m = bc.BoxConv2d(C, F, h, w).cuda().to(dtype)
+    return m, torch.randn(N, C, h, w, device="cuda").to(dtype)
+
+
+def test_the_function_is_an_autograd_function(bc):
+    assert issubclass(bc.BoxConvolutionFunction, torch.autograd.Function)
+    m, x = _module(bc)
+    assert m(x).grad_fn.name() == "BoxConvolutionFunctionBackward"
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.bfloat16])
+def test_forward_and_backward_of_the_class(bc, dtype):
+    """The Python halves against the node that ordinary calls get, bit for bit."""
+    class Sub(bc.BoxConvolutionFunction):
+        pass
+
+    m, x = _module(bc, dtype)
+    m.eval()
+    runs = []
+    for f in (bc.BoxConvolutionFunction, Sub):
+        args = [t.detach().clone().requires_grad_() for t in (x, m.x_min, m.x_max, m.y_min, m.y_max)]
+        out = f.apply(*args, m.reparametrization_h, m.reparametrization_w, True, True)
+        runs.append([out] + list(torch.autograd.grad(out, args, torch.ones_like(out))))
+        args[1].requires_grad_(False)
+        out = f.apply(*args, m.reparametrization_h, m.reparametrization_w, True, True)
+        runs[-1] += torch.autograd.grad(out, [args[0], args[4]], torch.ones_like(out))
+    assert all(a.dtype == b.dtype and torch.equal(a, b) for a, b in zip(*runs))
+
+
+def test_trace_computes_on_new_inputs(bc):
+    m, x = _module(bc)
+    m.eval()
+    traced = torch.jit.trace(m, x, check_trace=False)
+    for other in (x, torch.randn_like(x)):
+        assert torch.equal(traced(other), m(other))
+
+
+def test_forward_mode_is_refused(bc):
+    import torch.autograd.forward_ad as fwad
+    for training in (True, False):
+        m, x = _module(bc)
+        m.train(training)
+        with fwad.dual_level():
+            with pytest.raises((NotImplementedError, RuntimeError), match="forward|jvp"):
+                m(fwad.make_dual(x, torch.ones_like(x)))
+
+
+def test_function_transforms_are_refused(bc):
+    m, x = _module(bc)
+    m.eval()
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(m)(torch.stack([x, x]))
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda t: m(t).sum())(x)
+    with pytest.raises(RuntimeError):      # nothing of the transform reaches the call
+        torch.func.vmap(lambda k: m(x).sum() * k)(torch.ones(2, device="cuda"))
