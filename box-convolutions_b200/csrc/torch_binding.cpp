@@ -109,7 +109,7 @@ struct Options {
     double rep_h, rep_w;
     bool normalize, exact;
     Tensor snapshot;         // packed (4, C, F) float32 copy of the parameters, or undefined
-    unsigned *counters = nullptr;      // that go with it, or null
+    Tensor counters;         // what counters_of() finds the counters in that go with it, or undefined
 };
 
 // Checks of the module's forward; the parameters must have the input's dtype.
@@ -134,35 +134,33 @@ Sizes check_forward(const Tensor &input, const Four &p)
     return {to_int(input.size(0)), to_int(input.size(1)), to_int(p[0].size(1)), to_int(input.size(2)), to_int(input.size(3))};
 }
 
-// A packed float32 copy of the parameters, (4, C, F), with C counters behind it that are zero whenever no kernel
-// of its backward pass is running.
-struct Snapshot {
-    Tensor packed;
-    unsigned *counters = nullptr;      // in packed's storage
-};
-Snapshot new_snapshot(at::IntArrayRef sizes, const Tensor &like)
+// A packed float32 copy of the parameters, (4, C, F), with C counters behind it in its storage that are zero whenever
+// no kernel of its backward pass is running.
+Tensor new_snapshot(at::IntArrayRef sizes, const Tensor &like)
 {
     const int64_t n = c10::multiply_integers(sizes), rows = sizes.empty() ? 0 : sizes[0];
-    Snapshot s;
-    s.packed = new_tensor({4 * n + rows}, at::kFloat, like);
-    s.counters = reinterpret_cast<unsigned *>(s.packed.data_ptr<float>() + 4 * n);
+    Tensor packed = new_tensor({4 * n + rows}, at::kFloat, like);
     std::vector<int64_t> shape{4};
     shape.insert(shape.end(), sizes.begin(), sizes.end());
-    s.packed.unsafeGetTensorImpl()->set_sizes_contiguous(shape);
-    return s;
+    packed.unsafeGetTensorImpl()->set_sizes_contiguous(shape);
+    return packed;
+}
+// The counters behind a tensor that new_snapshot() has made (and nobody else), null for an undefined one.
+unsigned *counters_of(const Tensor &packed)
+{
+    return packed.defined() ? reinterpret_cast<unsigned *>(packed.data_ptr<float>() + packed.numel()) : nullptr;
 }
 
 // Packed float32 copy of the parameters as they are now, in one launch.
-Snapshot pack_parameters(const Four &p, const Sizes &s, bc_stream_t stream)
+Tensor pack_parameters(const Four &p, const Sizes &s, bc_stream_t stream)
 {
     Four q;
     for (int i = 0; i < 4; ++i) q[i] = p[i].contiguous();
-    Snapshot snap = new_snapshot({s.C, s.F}, p[0]);
+    Tensor packed = new_snapshot({s.C, s.F}, p[0]);
     check_status(bc_pack_parameters(q[0].const_data_ptr(), q[1].const_data_ptr(), q[2].const_data_ptr(), q[3].const_data_ptr(),
-                                    io_kind(p[0].scalar_type()), s.C * s.F, snap.packed.data_ptr<float>(), snap.counters,
-                                    snap.counters ? s.C : 0, stream),
+                                    io_kind(p[0].scalar_type()), s.C * s.F, packed.data_ptr<float>(), counters_of(packed), s.C, stream),
                  "BoxConv2d forward");
-    return snap;
+    return packed;
 }
 
 // The kernels' view of the four parameter arrays: slices of a packed copy, or four tensors.
@@ -339,8 +337,8 @@ bool all_contiguous(const Four &p)
     return p[0].is_contiguous() && p[1].is_contiguous() && p[2].is_contiguous() && p[3].is_contiguous();
 }
 
-// In place; `packed` (float32 and narrower): also returns a packed float32 copy of the clipped values.
-Snapshot clip(const Four &p, double rep_h, double rep_w, double max_h, double max_w, bool exact, bool packed)
+// In place; `packed` (float32 and narrower): also returns a packed float32 copy of the clipped values (new_snapshot()).
+Tensor clip(const Four &p, double rep_h, double rep_w, double max_h, double max_w, bool exact, bool packed)
 {
     const at::ScalarType dtype = p[0].scalar_type();
     for (int i = 0; i < 4; ++i) {
@@ -368,14 +366,14 @@ Snapshot clip(const Four &p, double rep_h, double rep_w, double max_h, double ma
     void *q[4];
     for (int i = 0; i < 4; ++i) q[i] = p[i].data_ptr();
     int status;
-    Snapshot out;
+    Tensor out;
     if (dtype == at::kDouble) {
         status = bc_clip_parameters_f64((double *)q[0], (double *)q[1], (double *)q[2], (double *)q[3], count, rep_h, rep_w, max_h,
                                         max_w, exact, stream);
     } else {
         if (packed) out = new_snapshot(p[0].sizes(), p[0]);
         status = bc_clip_parameters_any(q[0], q[1], q[2], q[3], io_kind(dtype), count, rep_h, rep_w, max_h, max_w, exact,
-                                        packed ? out.packed.data_ptr<float>() : nullptr, out.counters,
+                                        packed ? out.data_ptr<float>() : nullptr, counters_of(out),
                                         packed && count ? to_int(p[0].size(0)) : 0, stream);
     }
     check_status(status, "clip_parameters");
@@ -396,7 +394,7 @@ Snapshot clip(const Four &p, double rep_h, double rep_w, double max_h, double ma
 struct Kept {
     Tensor x;                    // the input; its integral image for float64
     Tensor params;               // packed (4, C, F): stored units, float32; pixels for float64
-    unsigned *counters = nullptr;
+    Tensor counters;             // as in Options
 };
 
 Tensor forward_any(const Tensor &input, const Four &p, const Options &o, Kept *keep)
@@ -408,25 +406,20 @@ Tensor forward_any(const Tensor &input, const Four &p, const Options &o, Kept *k
     if (dtype == at::kDouble) {
         Tensor pixels = at::stack({p[0].detach() * o.rep_h, p[1].detach() * o.rep_h, p[2].detach() * o.rep_w, p[3].detach() * o.rep_w});
         const Tensor integrated = integral_image(x);
-        if (keep) *keep = {integrated, pixels, nullptr};
+        if (keep) *keep = {integrated, pixels, Tensor()};
         return box_forward(integrated, {pixels.select(0, 0), pixels.select(0, 1), pixels.select(0, 2), pixels.select(0, 3)},
                            o.normalize, o.exact);
     }
     const bool narrow = is_narrow(dtype);
     if (narrow && s.h && s.w && s.F && !bc_boxconv2d_narrow_all_supported(s.F, s.h, s.w)) x = x.to(at::kFloat);
     const bc_stream_t stream = current_stream(x);
-    Tensor packed = o.snapshot;
-    unsigned *counters = o.counters;
+    Tensor packed = o.snapshot, counters = o.counters;
     if (packed.defined() && !(packed.scalar_type() == at::kFloat && packed.device() == x.device() && packed.is_contiguous() &&
                               packed.sizes() == at::IntArrayRef({4, s.C, s.F})))
         packed = Tensor();
     ParamPtrs q;
     Four dense;                  // (keeps contiguous copies alive across the launch)
-    if (!packed.defined() && (keep || narrow)) {
-        const Snapshot snap = pack_parameters(p, s, stream);
-        packed = snap.packed;
-        counters = snap.counters;
-    }
+    if (!packed.defined() && (keep || narrow)) packed = counters = pack_parameters(p, s, stream);
     if (packed.defined()) {
         q = of_packed(packed);
     } else {
@@ -479,7 +472,7 @@ Gradients backward_any(const Tensor &x, const Tensor &params, Tensor grad_output
     const bc_stream_t stream = current_stream(x);
     check_status(bc_boxconv2d_backward_any(x.const_data_ptr(), io_kind(dtype), q.p[0], q.p[1], q.p[2], q.p[3], g.const_data_ptr(),
                                            (float)a.rep_h, (float)a.rep_w, s.N, s.C, s.F, s.h, s.w, a.normalize, a.exact, mask, gin, gp,
-                                           ws, bytes, a.counters, stream),
+                                           ws, bytes, counters_of(a.counters), stream),
                  "BoxConv2d backward");
     if (dtype != caller) {
         if (out[0].defined()) out[0] = out[0].to(caller);
@@ -493,8 +486,8 @@ Gradients backward_any(const Tensor &x, const Tensor &params, Tensor grad_output
 // A plain autograd node: what torch::autograd::Function adds (a dictionary for the saved values, wrapping of the
 // outputs) takes longer than launching the kernels.
 struct BoxConvolutionBackward : torch::autograd::Node {
-    torch::autograd::SavedVariable x;
-    Tensor params;
+    // (hooks on saved tensors see both; the counters stay where they are and so belong to `options`)
+    torch::autograd::SavedVariable x, params;
     Options options;
     at::ScalarType caller;       // dtype of the input as the caller passed it
     std::mutex mutex;
@@ -510,7 +503,7 @@ struct BoxConvolutionBackward : torch::autograd::Node {
         {
             std::lock_guard<std::mutex> lock(mutex);
             in = x.unpack();      // (checks that the input has not been changed in place and that the graph is still alive)
-            packed = params;
+            packed = params.unpack();
         }
         const at::NoGradGuard no_grad;
         Gradients g = backward_any(in, packed, grads[0], options, caller, mask);
@@ -522,7 +515,8 @@ struct BoxConvolutionBackward : torch::autograd::Node {
     {
         std::lock_guard<std::mutex> lock(mutex);
         x.reset_data();
-        params.reset();
+        params.reset_data();
+        options.counters.reset();
     }
 
     std::string name() const override { return "BoxConvolutionFunctionBackward"; }
@@ -555,7 +549,7 @@ Tensor apply(const Tensor &input, const Four &p, const Options &o)
     auto node = std::shared_ptr<BoxConvolutionBackward>(new BoxConvolutionBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(input, p[0], p[1], p[2], p[3]));
     node->x = torch::autograd::SavedVariable(keep.x, false);
-    node->params = keep.params;
+    node->params = torch::autograd::SavedVariable(keep.params, false);
     node->options = o;
     node->options.snapshot = Tensor();      // (node->params holds it)
     node->options.counters = keep.counters;
@@ -690,9 +684,7 @@ PyObject *py_module_forward(PyObject *, PyObject *const *v, Py_ssize_t n)
                 clip({p[0].variable_data(), p[1].variable_data(), p[2].variable_data(), p[3].variable_data()}, o.rep_h, o.rep_w,
                      max_h, max_w, o.exact, false);
             } else {
-                const Snapshot snap = clip(p, o.rep_h, o.rep_w, max_h, max_w, o.exact, dtype != at::kDouble);
-                o.snapshot = snap.packed;
-                o.counters = snap.counters;
+                o.snapshot = o.counters = clip(p, o.rep_h, o.rep_w, max_h, max_w, o.exact, dtype != at::kDouble);
             }
         }
         out = apply(input, p, o);
@@ -845,7 +837,7 @@ PyObject *py_clip(PyObject *, PyObject *const *v, Py_ssize_t n)
     Tensor out;
     {
         py::gil_scoped_release release;
-        out = clip(p, rep_h, rep_w, max_h, max_w, exact, packed).packed;
+        out = clip(p, rep_h, rep_w, max_h, max_w, exact, packed);
     }
     return wrap(out);
     END_HANDLE_TH_ERRORS

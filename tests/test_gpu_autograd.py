@@ -72,3 +72,42 @@ def test_function_transforms_are_refused(bc):
         torch.func.grad(lambda t: m(t).sum())(x)
     with pytest.raises(RuntimeError):      # nothing of the transform reaches the call
         torch.func.vmap(lambda k: m(x).sum() * k)(torch.ones(2, device="cuda"))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.float16])
+def test_saved_tensor_hooks_see_input_and_parameters(bc, dtype):
+    """What they hand back is what the backward pass works on, wherever it has been meanwhile."""
+    m, x = _module(bc, dtype)
+    x.requires_grad_()
+    m(x).sum().backward()
+    want = [x.grad] + [p.grad for p in m.parameters()]
+    x.grad = None
+    m.zero_grad(set_to_none=True)
+    sizes = []
+
+    def pack(t):
+        sizes.append(tuple(t.shape))
+        return t.detach().cpu().clone()
+
+    def unpack(t):      # with other memory behind it
+        return torch.cat([t.cuda().reshape(-1), torch.full((64,), 7, device="cuda", dtype=t.dtype)])[:t.numel()].view(t.shape)
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+        y = m(x)
+    y.sum().backward()
+    assert (4, 3, 4) in sizes and len(sizes) == 2
+    assert all(torch.equal(a, b) for a, b in zip([x.grad] + [p.grad for p in m.parameters()], want))
+    with torch.autograd.graph.save_on_cpu():
+        y = m(x)
+    x.grad = None
+    y.sum().backward()
+    assert torch.equal(x.grad, want[0])
+
+
+def test_a_snapshot_changed_before_backward_is_noticed(bc):
+    m, x = _module(bc)
+    snapshot = torch.stack([p.detach() for p in m._parameters4()])
+    y = bc.BoxConvolutionFunction.apply(x, *m._parameters4(), m.reparametrization_h, m.reparametrization_w, True, True, snapshot)
+    snapshot.zero_()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.sum().backward()
