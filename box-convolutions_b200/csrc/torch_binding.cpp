@@ -498,15 +498,17 @@ struct BoxConvolutionBackward : torch::autograd::Node {
         for (int i = 0; i < 5; ++i)
             if (task_should_compute_output(i)) mask |= 1 << i;
         torch::autograd::variable_list list(5);
-        if (!grads[0].defined() || !mask) return list;
+        if (!mask) return list;
+        const at::NoGradGuard no_grad;
+        // (a function behind this one that returned nothing: zeros, as torch.autograd.Function has it)
+        const Tensor grad = grads[0].defined() ? grads[0] : input_metadata(0).zeros_like();
         Tensor in, packed;
         {
             std::lock_guard<std::mutex> lock(mutex);
             in = x.unpack();      // (checks that the input has not been changed in place and that the graph is still alive)
             packed = params.unpack();
         }
-        const at::NoGradGuard no_grad;
-        Gradients g = backward_any(in, packed, grads[0], options, caller, mask);
+        Gradients g = backward_any(in, packed, grad, options, caller, mask);
         for (int i = 0; i < 5; ++i) list[i] = std::move(g[i]);      // sole owner: a first accumulation takes the tensor itself
         return list;
     }

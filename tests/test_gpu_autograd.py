@@ -111,3 +111,19 @@ def test_a_snapshot_changed_before_backward_is_noticed(bc):
     snapshot.zero_()
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         y.sum().backward()
+
+
+def test_a_missing_gradient_counts_as_zeros(bc):
+    class Nothing(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, t):
+            return t.clone()
+
+        @staticmethod
+        def backward(ctx, g):
+            return None
+
+    m, x = _module(bc)
+    x.requires_grad_()
+    grads = torch.autograd.grad(Nothing.apply(m(x)).sum(), [x] + list(m.parameters()))
+    assert all((g == 0).all() for g in grads)
