@@ -452,27 +452,15 @@ Gradients backward_any(const Tensor &x, const Tensor &params, Tensor grad_output
     if (mask & BC_NEED_INPUT) out[0] = new_tensor(x.sizes(), dtype, x);
     const size_t bytes = is_narrow(dtype) ? bc_boxconv2d_narrow_workspace(s.N, s.C, s.F, s.h, s.w, mask)
                                           : bc_boxconv2d_backward_workspace(s.N, s.C, s.F, s.h, s.w, mask);
-    // One allocation for the parameter gradients and, where it is small, the workspace behind them.
-    constexpr size_t kSmall = 64 * 1024;
-    Tensor gparams, scratch;
-    void *ws = nullptr;
-    if (mask & ~BC_NEED_INPUT) {
-        const size_t elem = c10::elementSize(dtype), gap = ((size_t)4 * s.C * s.F * elem + 255) / 256 * 256;
-        const bool together = bytes <= kSmall;
-        gparams = new_tensor({(int64_t)(together ? (gap + bytes + elem - 1) / elem : (size_t)4 * s.C * s.F)}, dtype, x);
-        if (together) ws = static_cast<char *>(gparams.data_ptr()) + gap;
-        gparams.unsafeGetTensorImpl()->set_sizes_contiguous({4, s.C, s.F});
-    }
-    if (!ws) {
-        scratch = new_workspace(bytes, x);
-        ws = scratch.data_ptr();
-    }
+    // (an allocation of its own for the scratch: the gradients' storage lives, and is saved and sent, as long as they are)
+    Tensor gparams, scratch = new_workspace(bytes, x);
+    if (mask & ~BC_NEED_INPUT) gparams = new_tensor({4, s.C, s.F}, dtype, x);
     const ParamPtrs q = of_packed(params);
     void *gin = out[0].defined() ? out[0].data_ptr() : nullptr, *gp = gparams.defined() ? gparams.data_ptr() : nullptr;
     const bc_stream_t stream = current_stream(x);
     check_status(bc_boxconv2d_backward_any(x.const_data_ptr(), io_kind(dtype), q.p[0], q.p[1], q.p[2], q.p[3], g.const_data_ptr(),
                                            (float)a.rep_h, (float)a.rep_w, s.N, s.C, s.F, s.h, s.w, a.normalize, a.exact, mask, gin, gp,
-                                           ws, bytes, counters_of(a.counters), stream),
+                                           scratch.data_ptr(), bytes, counters_of(a.counters), stream),
                  "BoxConv2d backward");
     if (dtype != caller) {
         if (out[0].defined()) out[0] = out[0].to(caller);

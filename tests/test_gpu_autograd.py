@@ -127,3 +127,13 @@ def test_a_missing_gradient_counts_as_zeros(bc):
     x.requires_grad_()
     grads = torch.autograd.grad(Nothing.apply(m(x)).sum(), [x] + list(m.parameters()))
     assert all((g == 0).all() for g in grads)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gradients_bring_no_scratch_with_them(bc, dtype):
+    """The four parameter gradients share one buffer (which is reduced in one piece over ranks), and nothing else does."""
+    m, x = _module(bc, dtype)
+    m(x).sum().backward()
+    assert {p.grad.untyped_storage().nbytes() for p in m.parameters()} == {4 * m.x_min.numel() * m.x_min.element_size()}
+    packed, copied = bc.packed_box_gradient(m)
+    assert not copied and torch.equal(packed, torch.stack([p.grad for p in m._parameters4()]))
