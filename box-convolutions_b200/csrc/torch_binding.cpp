@@ -380,6 +380,12 @@ Tensor clip(const Four &p, double rep_h, double rep_w, double max_h, double max_
     return out;
 }
 
+// What was written behind autograd's back counts as a change in place.
+void mark_changed(const Tensor &t)
+{
+    if (!t.is_inference()) t.unsafeGetTensorImpl()->bump_version();
+}
+
 // ---- the module's forward and its autograd node ------------------------------------------------
 //
 // Unlike the reference (box_convolution/box_convolution_function.py:30-65) the node does not keep the
@@ -828,6 +834,9 @@ PyObject *py_clip(PyObject *, PyObject *const *v, Py_ssize_t n)
     {
         py::gil_scoped_release release;
         out = clip(p, rep_h, rep_w, max_h, max_w, exact, packed);
+        // 16-bit parameters were once copied back by PyTorch, which checks that no saved value has changed; it still can
+        if (!packed && is_narrow(p[0].scalar_type()) && all_contiguous(p))
+            for (const Tensor &t : p) mark_changed(t);
     }
     return wrap(out);
     END_HANDLE_TH_ERRORS

@@ -119,3 +119,13 @@ def test_half_module_trains_with_parameters_that_are_not_contiguous(bc, dtype):
         outs.append([y] + [p for p in net.parameters()] + [p.grad for p in net.parameters()])
     assert not t.x_min.is_contiguous()
     assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_clipping_half_parameters_is_a_change_in_place(bc, dtype):
+    """A backward pass that saved the values from before the clip says so instead of using the new ones."""
+    p = [torch.randn(3, 2, device="cuda").to(dtype).requires_grad_() for _ in range(4)]
+    loss = sum((t * t).sum() for t in p)
+    bc.clip_parameters(*p, 8.0, 16.0, 8.0, 16.0, True)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        loss.backward()
