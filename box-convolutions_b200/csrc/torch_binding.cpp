@@ -374,7 +374,7 @@ Tensor clip(const Four &p, double rep_h, double rep_w, double max_h, double max_
         if (packed) out = new_snapshot(p[0].sizes(), p[0]);
         status = bc_clip_parameters_any(q[0], q[1], q[2], q[3], io_kind(dtype), count, rep_h, rep_w, max_h, max_w, exact,
                                         packed ? out.data_ptr<float>() : nullptr, counters_of(out),
-                                        packed && count ? to_int(p[0].size(0)) : 0, stream);
+                                        packed && count && p[0].dim() ? to_int(p[0].size(0)) : 0, stream);
     }
     check_status(status, "clip_parameters");
     return out;

@@ -137,3 +137,13 @@ def test_gradients_bring_no_scratch_with_them(bc, dtype):
     assert {p.grad.untyped_storage().nbytes() for p in m.parameters()} == {4 * m.x_min.numel() * m.x_min.element_size()}
     packed, copied = bc.packed_box_gradient(m)
     assert not copied and torch.equal(packed, torch.stack([p.grad for p in m._parameters4()]))
+
+
+def test_packed_clip_of_single_numbers(bc):
+    """Parameters without dimensions are four numbers."""
+    from box_convolution import ext
+    p = [torch.tensor(v, device="cuda") for v in (-0.9, 0.9, 0.1, 0.1)]
+    q = [t.clone().view(1, 1) for t in p]
+    packed = ext.clip_parameters_packed(*p, 8.0, 16.0, 8.0, 16.0, True)
+    want = ext.clip_parameters_packed(*q, 8.0, 16.0, 8.0, 16.0, True)
+    assert packed.shape == (4,) and torch.equal(packed, want.view(4)) and torch.equal(packed, torch.stack(p))
