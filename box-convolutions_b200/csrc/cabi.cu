@@ -3,6 +3,7 @@
 #include <stdio.h>
 #include <atomic>
 #include <mutex>
+#include <new>
 #include <type_traits>
 #include <vector>
 #include <string.h>
@@ -38,7 +39,10 @@ int raise_smem_limit(const void *kernel, int bytes)
         if (d.kernel == kernel && d.device == device) return BC_OK;
     if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes))
         return cuda_failed(e, "shared memory opt-in");
-    done.push_back({kernel, device});
+    try {
+        done.push_back({kernel, device});
+    } catch (const std::bad_alloc &) {      // (nothing is thrown through a C entry point; the call is made again next time)
+    }
     return BC_OK;
 }
 
