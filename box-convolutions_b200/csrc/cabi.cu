@@ -440,26 +440,43 @@ int bc_boxconv2d_forward_fused(const float *input, const float *x_min, const flo
     return forward_from_workspace(input, bp, &fu, output, N, C, F, h, w, normalize != 0, exact != 0, integ, stream);
 }
 
-size_t bc_boxconv2d_backward_workspace(int N, int C, int F, int h, int w, int need_mask)
+static size_t backward_slabs_bytes(int N, int C, int F, int h, int w)
+{
+    return align_up(slab_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256) +
+           align_up(slab_partials_bytes(N, C, F, h, w), 256);
+}
+
+// Scratch of the float backward pass in at most `limit` bytes, where it has the choice: slabs pad the rows of their
+// integral images more than the older kernels for large planes do (one column: 12 floats against 2), which serve
+// what then exceeds the limit.
+static bool backward_on_slabs(int N, int C, int F, int h, int w, size_t limit)
+{
+    return slab_path_fits(F, h, w) && backward_slabs_bytes(N, C, F, h, w) <= limit;
+}
+static size_t backward_workspace_within(int N, int C, int F, int h, int w, int need_mask, size_t limit)
 {
     if (!sizes_ok(N, C, F, h, w) || any_empty(N, C, F, h, w) || !(need_mask & BC_NEED_ALL)) return 0;
     if (plane_path_fits_backward(F, h, w))
         return plane_partials_bytes(N, C, F);
-    if (slab_path_fits(F, h, w))
-        return align_up(slab_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256) +
-               align_up(slab_partials_bytes(N, C, F, h, w), 256);
+    if (backward_on_slabs(N, C, F, h, w, limit)) return backward_slabs_bytes(N, C, F, h, w);
     if (band_path_fits_backward(F, h, w))
         return align_up(band_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256) +
                align_up(band_partials_bytes(N, C, F, w), 256);
     return integral_bytes((int64_t)N * C * F, h, w) + align_up(backward_partials_bytes(N, C, F, h, w), 256);
 }
 
+size_t bc_boxconv2d_backward_workspace(int N, int C, int F, int h, int w, int need_mask)
+{
+    return backward_workspace_within(N, C, F, h, w, need_mask, SIZE_MAX);
+}
+
+// limit: as in backward_workspace_within()
 static int backward_float(const float *input, const float *x_min, const float *x_max,
                           const float *y_min, const float *y_max, const float *grad_output,
                           float reparametrization_h, float reparametrization_w, int N, int C,
                           int F, int h, int w, int normalize, int exact, int need_mask,
                           float *grad_input, float *grad_params, void *workspace,
-                          size_t workspace_bytes, unsigned *counters, bc_stream_t stream)
+                          size_t workspace_bytes, unsigned *counters, bc_stream_t stream, size_t limit = SIZE_MAX)
 {
     if (!sizes_ok(N, C, F, h, w)) return BC_ERR_BAD_SHAPE;
     need_mask &= BC_NEED_ALL;
@@ -483,13 +500,13 @@ static int backward_float(const float *input, const float *x_min, const float *x
     const size_t ib = band ? align_up(band_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256)
                            : integral_bytes((int64_t)N * C * F, h, w);
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) ||
-        workspace_bytes < bc_boxconv2d_backward_workspace(N, C, F, h, w, need_mask))
+        workspace_bytes < backward_workspace_within(N, C, F, h, w, need_mask, limit))
         return BC_ERR_WORKSPACE;
     if (plane_path_fits_backward(F, h, w))
         return launch_backward_plane(input, grad_output, bp, reparametrization_h, reparametrization_w, N, C,
                                      F, h, w, normalize != 0, exact != 0, need_mask, grad_input,
                                      grad_params, static_cast<float *>(workspace), stream);
-    if (slab_path_fits(F, h, w))
+    if (backward_on_slabs(N, C, F, h, w, limit))
         return backward_slabs(input, nullptr, BC_IO_F32, grad_output, bp, reparametrization_h, reparametrization_w, N, C, F, h, w,
                               normalize != 0, exact != 0, need_mask, grad_input, grad_params, BC_IO_F32, workspace, stream);
     float *go_integ = static_cast<float *>(workspace);
@@ -687,7 +704,7 @@ int bc_boxconv2d_backward_static(const float *input, const float *x_min, const f
                                  float *grad_input, float *grad_params, bc_stream_t stream)
 {
     if (!sizes_ok(N, C, F, h, w)) return BC_ERR_BAD_SHAPE;
-    const size_t need = bc_boxconv2d_backward_workspace(N, C, F, h, w, need_mask);
+    const size_t need = backward_workspace_within(N, C, F, h, w, need_mask, BC_STATIC_SCRATCH_BYTES);
     if (need > BC_STATIC_SCRATCH_BYTES) {
         snprintf(g_last_error, sizeof(g_last_error),
                  "bc_boxconv2d_backward_static: this problem needs %zu bytes of scratch, the built-in array has %u",
@@ -697,9 +714,9 @@ int bc_boxconv2d_backward_static(const float *input, const float *x_min, const f
     int status = BC_OK;
     void *scratch = static_scratch_address(&status);
     if (!scratch) return status;
-    return bc_boxconv2d_backward(input, x_min, x_max, y_min, y_max, grad_output, reparametrization_h,
-                                 reparametrization_w, N, C, F, h, w, normalize, exact, need_mask,
-                                 grad_input, grad_params, scratch, BC_STATIC_SCRATCH_BYTES, stream);
+    return backward_float(input, x_min, x_max, y_min, y_max, grad_output, reparametrization_h, reparametrization_w, N, C, F, h, w,
+                          normalize, exact, need_mask, grad_input, grad_params, scratch, BC_STATIC_SCRATCH_BYTES, nullptr, stream,
+                          BC_STATIC_SCRATCH_BYTES);
 }
 
 uint64_t bc_launch_count(void) { return g_launches.load(); }

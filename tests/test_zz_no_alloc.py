@@ -113,6 +113,23 @@ def test_static_scratch_backward_empty_call_is_the_cheap_first_call():
     assert st == 0
 
 
+# tall narrow planes and one just too large for the whole-plane kernels: the slabs' padded rows would exceed the array
+@pytest.mark.parametrize("shape", [(1, 3, 8, 3667, 1), (2, 2, 8, 2381, 5), (4, 2, 4, 1201, 19), (1, 4, 1, 666, 385)])
+def test_static_scratch_backward_takes_the_route_that_fits(shape):
+    from box_convolution._cabi import lib
+    N, C, F, h, w = shape
+    assert lib.bc_boxconv2d_backward_workspace(N, C, F, h, w, 31) > 4 << 20
+    rng = np.random.default_rng(h)
+    x = torch.from_numpy(rng.standard_normal((N, C, h, w)).astype(np.float32)).cuda()
+    go = torch.from_numpy(rng.standard_normal((N, C * F, h, w)).astype(np.float32)).cuda()
+    lo, hi = rng.uniform(-h / 3, 0, (2, C, F)), rng.uniform(1.2, h / 3, (2, C, F))
+    pix = [torch.from_numpy(a.astype(np.float32)).cuda() for a in (lo[0], hi[0], lo[1] * w / h, hi[1] * w / h + 1.2)]
+    want = _backward(lib, False, x, go, pix, 1.0, 1.0)
+    got = _backward(lib, True, x, go, pix, 1.0, 1.0)
+    assert want[0] == 0 and got[0] == 0
+    assert max_rel(got[1], want[1]) < 1e-4 and max_rel(got[2], want[2]) < 1e-3
+
+
 def test_static_scratch_backward_refuses_what_does_not_fit():
     from box_convolution import _cabi
     lib = _cabi.lib
