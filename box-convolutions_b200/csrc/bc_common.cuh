@@ -56,6 +56,9 @@ int cuda_failed(cudaError_t e, const char *what);
 // kernel and device).
 int raise_smem_limit(const void *kernel, int bytes);
 
+// Is the stream being captured into a graph?
+bool is_capturing(cudaStream_t s);
+
 // Kernel ids reported by the profiling aid (bc_profile_get / bc_kernel_name).
 enum KernelId {
     KID_INTEGRAL = 1, KID_FORWARD_GLOBAL, KID_BACKWARD_GLOBAL, KID_FINISH_PARAM_GRADS, KID_CLIP,

@@ -48,7 +48,8 @@ __device__ __forceinline__ void finish_box(const T *partials, const BoxParamsT<T
 // for the channel's F boxes, in the same order of additions as the kernel of its own.  It saves a launch, 3 us of
 // host time, which is worth it where a step is bound by the host.  Where it is bound by the GPU, the fence that
 // every CTA pays for and the registers cost more than the launch ((8,16,4,128,256): 80 + 2.5 us in two launches, 88 in
-// one), so kernels have it as a template parameter and launchers ask for it up to kFinishMaxOutputs outputs.
+// one), so kernels have it as a template parameter and launchers ask for it up to kFinishMaxOutputs outputs, and not
+// while the stream is captured into a graph: a replay has no host time to save.
 template <bool B>
 struct Flag { static constexpr bool value = B; };      // (picks a kernel's instantiation)
 
@@ -61,9 +62,9 @@ struct Finish {
 constexpr int64_t kFinishMaxCtas = 4 * 148, kFinishMaxOutputs = 8 << 20;      // (a GPU time of about 45 us a step)
 
 inline Finish finish_here(const BoxParams &bp, bool need_params, int64_t ctas, int64_t outputs, int C, void *grad_params, int io_kind,
-                          int need_mask, int per_box, float rep_h, float rep_w)
+                          int need_mask, int per_box, float rep_h, float rep_w, cudaStream_t stream)
 {
-    const bool here = need_params && bp.counters && ctas <= kFinishMaxCtas && outputs <= kFinishMaxOutputs;
+    const bool here = need_params && bp.counters && ctas <= kFinishMaxCtas && outputs <= kFinishMaxOutputs && !is_capturing(stream);
     return Finish{grad_params, io_kind, need_mask, per_box, rep_h, rep_w, here ? (unsigned)(ctas / C) : 0u};
 }
 

@@ -845,7 +845,12 @@ int launch_backward_plane_t(const IO *x, const float *x_integ, const IO *grad_ou
                         (with_staging <= two_ctas || plane_backward_smem_bytes(h, w, xsmem, false, io) > two_ctas);
     const size_t smem = plane_backward_smem_bytes(h, w, xsmem, staged, io);
     void (*kern)(const IO *, const float *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, bool, bool, bool, Finish);
-    const Finish fin = finish_here(bp, need_params, planes, planes * F * h * w, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w);
+    // With the input plane in shared memory, finishing here costs more than the launch it saves, from all but the
+    // smallest problems on ((18,14,8,40,56): 41 us against 32 with the launch; (9,12,4,248,48): 67 against 53; (1,8,4,32,32): 17 against 14.5
+    // and 3 us of the host); in tensor memory it costs nothing.
+    const int64_t outputs = planes * F * h * w;
+    const bool may_finish = need_params && (tensor || (planes <= 148 && outputs <= 256 * 1024));
+    const Finish fin = finish_here(bp, may_finish, planes, outputs, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w, s);
     auto pick = [&](auto counted) {
         constexpr bool K = decltype(counted)::value;
         if (tensor) {

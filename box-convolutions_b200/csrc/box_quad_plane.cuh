@@ -586,7 +586,7 @@ int launch_backward_quad_t(const IO *x, const float *x_integ, const IO *grad_out
     const bool fast = w % 4 == 0 && h % kTileRows == 0 && ((size_t)h * w * sizeof(IO)) % 16 == 0 && aligned_to(x, Io<IO>::kVecBytes) &&
                      aligned_to(grad_output, 16) && (!write_gin || aligned_to(grad_input, Io<IO>::kVecBytes));
     void (*kern)(const IO *, const float *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, int, bool, bool, bool, Finish);
-    const Finish fin = finish_here(bp, need_params, planes, planes * F * h * w, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w);
+    const Finish fin = finish_here(bp, need_params, planes, planes * F * h * w, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w, s);
     auto pick = [&](auto ct, auto counted) {
         constexpr int CT = decltype(ct)::value;
         constexpr bool K = decltype(counted)::value;

@@ -348,7 +348,7 @@ int backward_slab_t(const IO *x, const float *x_integ, const float *go_integ, co
     const bool write_gin = (need_mask & BC_NEED_INPUT) != 0;
     const bool vec = w % 4 == 0 && aligned_to(x, Io<IO>::kVecBytes) && (!write_gin || aligned_to(grad_input, Io<IO>::kVecBytes));
     void (*kern)(const IO *, const float *, const float *, BoxParams, IO *, float *, int, int, int, int, int, SlabShape, bool, bool, bool, Finish);
-    const Finish fin = finish_here(bp, need_params, blocks, (int64_t)N * C * F * h * w, C, grad_params, grad_params_kind, need_mask, N * sh.slabs, rep_h, rep_w);
+    const Finish fin = finish_here(bp, need_params, blocks, (int64_t)N * C * F * h * w, C, grad_params, grad_params_kind, need_mask, N * sh.slabs, rep_h, rep_w, s);
     auto pick = [&](auto counted) {
         constexpr int S = 128, L = 32 * kSlabMaxWarps;
         constexpr bool K = decltype(counted)::value;

@@ -46,6 +46,16 @@ int raise_smem_limit(const void *kernel, int bytes)
     return BC_OK;
 }
 
+bool is_capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {
+        (void)cudaGetLastError();      // (the legacy stream while another one is captured)
+        return false;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
 // ---- launch counter and per-kernel event timing
 static std::atomic<uint64_t> g_launches{0};
 static std::mutex g_prof_mutex;

@@ -147,3 +147,38 @@ def test_packed_clip_of_single_numbers(bc):
     packed = ext.clip_parameters_packed(*p, 8.0, 16.0, 8.0, 16.0, True)
     want = ext.clip_parameters_packed(*q, 8.0, 16.0, 8.0, 16.0, True)
     assert packed.shape == (4,) and torch.equal(packed, want.view(4)) and torch.equal(packed, torch.stack(p))
+
+
+# 32 x 32 tiles, whole planes in 8 x 128 tiles, slabs
+@pytest.mark.parametrize("shape", [(2, 3, 4, 32, 32), (2, 3, 4, 40, 72), (1, 2, 2, 201, 260)])
+def test_captured_step_finishes_in_a_launch_of_its_own(bc, shape):
+    """Outside a graph small steps finish their parameter gradients in the backward kernel; a replay has the kernel that
+    only does this, and the same bits."""
+    from box_convolution import _cabi
+    m, x = _module(bc, shape=shape)
+    go = torch.randn(shape[0], shape[1] * shape[2], *shape[3:], device="cuda")
+
+    def step():
+        m.zero_grad(set_to_none=True)
+        m(x).backward(go)
+        return [p.grad for p in m.parameters()]
+
+    want = [g.clone() for g in step()]
+    before = _cabi.lib.bc_launch_count()
+    step()
+    eager = _cabi.lib.bc_launch_count() - before
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    before = _cabi.lib.bc_launch_count()
+    with torch.cuda.graph(graph):
+        got = step()
+    assert _cabi.lib.bc_launch_count() - before == eager + 1
+    for _ in range(2):
+        for g in got:
+            g.fill_(7)
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
