@@ -753,10 +753,11 @@ inline bool plane_fits_backward_integ(int F, int h, int w)
 }
 
 // From the input's integral image, planes of more than 8 tiles of 32 x 32, which occupy an SM alone in the backward
-// kernel of this file, are better off as slabs where they are wide enough ((4,16,4,96,160): 36 us against 48).
-inline bool plane_prefers_slabs_backward(int F, int h, int w)
+// kernel of this file, are better off as slabs where they are wide enough ((4,16,4,96,160): 36 us against 48) or leave
+// half of the SMs idle ((1,17,8,143,44): 32 us against 82, (5,4,4,216,56): 28 against 58; (22,15,2,136,40): 54 against 48).
+inline bool plane_prefers_slabs_backward(int64_t planes, int F, int h, int w)
 {
-    return w > 96 && warp_tiles(h, w) > 8 && !quad_fits_backward(F, h, w);
+    return (w > 96 || planes <= 74) && warp_tiles(h, w) > 8 && !quad_fits_backward(F, h, w);
 }
 
 inline bool plane_fits_backward(int F, int h, int w)

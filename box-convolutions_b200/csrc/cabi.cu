@@ -110,9 +110,9 @@ static size_t plane_partials_bytes(int N, int C, int F) { return align_up((size_
 
 // Backward from the input's integral image on the whole-plane kernels?  (They may hold the plane and slabs be
 // faster all the same.)
-static bool plane_backward_integ(int F, int h, int w)
+static bool plane_backward_integ(int64_t planes, int F, int h, int w)
 {
-    return plane_path_fits_backward_integ(F, h, w) && !(plane_path_prefers_slabs_backward(F, h, w) && slab_path_fits(F, h, w));
+    return plane_path_fits_backward_integ(F, h, w) && !(plane_path_prefers_slabs_backward(planes, F, h, w) && slab_path_fits(F, h, w));
 }
 
 // Backward of planes that do not fit in shared memory, by slabs (workspace already checked).
@@ -167,7 +167,7 @@ static size_t backward_workspace_entry(int N, int C, int F, int h, int w, int ne
 {
     if (!sizes_ok(N, C, F, h, w) || any_empty(N, C, F, h, w) || !(need_mask & BC_NEED_ALL)) return 0;
     if (std::is_same<T, float>::value) {
-        if (plane_backward_integ(F, h, w)) return plane_partials_bytes(N, C, F);
+        if (plane_backward_integ((int64_t)N * C, F, h, w)) return plane_partials_bytes(N, C, F);
         if (slab_path_fits(F, h, w))
             return align_up(slab_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256) +
                    align_up(slab_partials_bytes(N, C, F, h, w), 256);
@@ -207,7 +207,7 @@ static int backward_entry(const T *input_integrated, const T *x_min, const T *x_
         return BC_ERR_WORKSPACE;
     const BoxParamsT<T> bp{x_min, x_max, y_min, y_max, T(1), T(1)};
     if constexpr (std::is_same<T, float>::value) {
-        if (plane_backward_integ(F, h, w))
+        if (plane_backward_integ((int64_t)N * C, F, h, w))
             return launch_backward_plane_integ(input_integrated, grad_output, bp, reparametrization_h, reparametrization_w, N, C, F, h,
                                                w, normalize != 0, exact != 0, need_mask, grad_input, grad_params,
                                                static_cast<float *>(workspace), stream);

@@ -126,8 +126,10 @@ def test_large_values_stay_on_their_side(bc, shape, value):
         assert torch.equal(got[..., :w - 8], clean[..., :w - 8])      # (the boxes reach less than five columns)
 
 
-# the same through the four functions, which gather from the caller's integral image
-@pytest.mark.parametrize("shape", [(1, 2, 2, 64, 128), (2, 2, 3, 33, 70), (1, 2, 2, 96, 160), (1, 1, 2, 121, 250), (1, 2, 2, 201, 257)])
+# the same through the four functions, which gather from the caller's integral image: copied to shared memory or read where
+# it is; the input rebuilt from it into shared memory, tensor memory (rows of either alignment) and slabs
+@pytest.mark.parametrize("shape", [(1, 2, 2, 64, 128), (2, 2, 3, 33, 70), (1, 2, 2, 96, 160), (1, 1, 2, 121, 250), (1, 2, 2, 201, 257),
+                                   (1, 2, 2, 300, 60), (3, 30, 1, 300, 60), (5, 30, 1, 256, 56), (2, 3, 1, 140, 150), (9, 40, 3, 20, 30)])
 def test_four_functions_edges_against_float64(bc, shape):
     N, C, F, h, w = shape
     rng = np.random.default_rng(h * 7 + w)
