@@ -770,7 +770,7 @@ template <typename IO>
 int launch_forward_plane_t(const IO *x, const float *integ, const BoxParams &bp, const Fusion *fu, IO *out, int N, int C, int F, int h,
                            int w, bool normalize, bool exact, cudaStream_t s)
 {
-    if (quad_fits_forward(F, h, w, (int64_t)N * C * F <= 148)) return launch_forward_quad_t<IO>(x, integ, bp, fu, out, N, C, F, h, w, normalize, exact, s);
+    if (quad_fits_forward(F, h, w) && quad_prefers_forward((int64_t)N * C, F, h, w)) return launch_forward_quad_t<IO>(x, integ, bp, fu, out, N, C, F, h, w, normalize, exact, s);
     const int64_t planes = (int64_t)N * C;
     // Split the filters of a plane over two CTAs when there are too few planes to balance 148 SMs
     // (each part rebuilds the integral image; the second read of the plane comes from L2).

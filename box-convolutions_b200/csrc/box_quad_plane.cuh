@@ -502,15 +502,42 @@ inline size_t quad_backward_smem(int F, int h, int w)
 }
 // Narrower planes leave more than half of a warp's lanes idle and are better off in 32 x 32 tiles.
 constexpr int kQuadMinWidth = 65;
-// few: the launch leaves SMs idle anyway.
-inline bool quad_fits_forward(int F, int h, int w, bool few = false)
+// How many CTAs share a plane's filters, and its rows: planes of more than 16 tiles that leave SMs idle, CTAs that each
+// gather a part of the rows from integral images of their own ((1,16,4,128,256), 64 -> 128 CTAs: 12.0 -> 9.8 us a block tail).
+struct QuadSplit {
+    int filters, rows;
+};
+inline QuadSplit quad_forward_split(int64_t planes, int F, int tiles)
+{
+    QuadSplit s{1, 1};
+    if (F % 2 == 0 && planes < 148 * 6) s.filters = 2;
+    while (s.filters < F && F % (s.filters * 2) == 0 && planes * s.filters * 2 <= 148 * 2) s.filters *= 2;
+    while (tiles > 16 && planes * s.filters * s.rows * 2 <= 148 && s.rows < 4) s.rows *= 2;
+    return s;
+}
+
+// Forward in tiles of 8 x 128 or of 32 x 32, where both fit?  A tile of either kind is 1024 pixels and a warp's work.
+// Rows that vector accesses fit, and all rows of the tiles: as many tiles or fewer, which compares what is wasted past
+// the plane ((8,16,4,128,256), 32 to 32: 31 us against 34; 448 planes of 48 x 120, F = 4, 6 to 8: 18 against 23; (4,16,4,96,160), 24 to
+// 15: 16 against 11; 1032 planes of 64 x 80, F = 4, 8 to 6: 37 against 34), and launches that leave SMs idle, for the shorter
+// chain of the 8 x 128 build.  Rows that no vector access fits are loaded and stored through shuffles, and cut rows at
+// the bottom take guarded code: work that a single and nearly full column tile repays ((7,63,4,244,125), float16: 135 us
+// against 170, (3,56,2,78,99): 13.5 against 17.5, (56,9,4,35,104): 21 against 23) and others do not ((27,26,4,31,162): 46 against 35;
+// (5,7,3,37,69): 11 against 7.4; (37,5,4,34,68): 10.7 against 9.4), unless the CTA has its SM to itself either way, the rows are
+// aligned and three quarters of the tiles' pixels exist ((3,38,6,63,216): 24 against 25; (117,5,8,68,92): 78 against 67).  A
+// split by rows, which 32 x 32 tiles do not have, pays whatever the rows ((3,5,3,116,186): 12 against 21).
+inline bool quad_prefers_forward(int64_t planes, int F, int h, int w)
+{
+    const int tiles = quad_row_tiles(h) * quad_col_tiles(w), square = ((h + 31) / 32) * ((w + 31) / 32);
+    if (quad_forward_split(planes, F, tiles).rows > 1) return true;
+    const bool few = planes * F <= 148, full = 4 * (int64_t)h * w >= 3 * (int64_t)tiles * 1024;
+    if (w % 4 == 0 && h % kTileRows == 0) return tiles <= square || few;
+    return (w > 96 && w <= 128 && (tiles <= 8 || full)) || (w % 4 == 0 && tiles > 8 && (full || few));
+}
+inline bool quad_fits_forward(int F, int h, int w)
 {
     const int tiles = quad_row_tiles(h) * quad_col_tiles(w);
-    if (w < kQuadMinWidth || w > 256 || F > kMaxFilters || tiles > 2 * kQuadMaxWarps || quad_forward_smem(F, h, w) > kQuadMaxSmem) return false;
-    // More than eight tiles means two a warp and a CTA that has its SM to itself: only where three quarters of the
-    // tiles' pixels exist (96 x 160, 63 %: 47 us against 33 in 32 x 32 tiles; 128 x 256: 35 against 37), or where it
-    // has an SM to itself in any case (one 96 x 160 frame: 7.4 us against 8.2).
-    return tiles <= 8 || 4 * (int64_t)h * w >= 3 * (int64_t)tiles * 1024 || few;
+    return w >= kQuadMinWidth && w <= 256 && F <= kMaxFilters && tiles <= 2 * kQuadMaxWarps && quad_forward_smem(F, h, w) <= kQuadMaxSmem;
 }
 inline bool quad_fits_backward(int F, int h, int w)
 {
@@ -524,19 +551,16 @@ int launch_forward_quad_t(const IO *x, const float *integ, const BoxParams &bp, 
 {
     const int row_tiles = quad_row_tiles(h), col_tiles = quad_col_tiles(w), tiles = row_tiles * col_tiles;
     const int64_t planes = (int64_t)N * C;
-    int fsplit = 1;
-    if (F % 2 == 0 && planes < 148 * 6) fsplit = 2;
-    while (fsplit < F && F % (fsplit * 2) == 0 && planes * fsplit * 2 <= 148 * 2) fsplit *= 2;
+    const QuadSplit split = quad_forward_split(planes, F, tiles);
+    const int fsplit = split.filters;
     if (planes * fsplit > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
     const bool fast = w % 4 == 0 && h % kTileRows == 0 && aligned_to(x, Io<IO>::kVecBytes) && aligned_to(out, Io<IO>::kVecBytes) &&
                       (!fu || !fu->residual || aligned_to(fu->residual, 16));
     const int T = tiles > 8 ? 2 : 1;
-    // Planes of more than 16 tiles that leave SMs idle: CTAs that each gather a part of the rows, from integral images of
-    // their own ((1,16,4,128,256), 64 -> 128 CTAs: 12.0 -> 9.8 us a block tail).  Not where the output lies over the input
-    // (one filter, in place): a CTA that starts late would integrate rows that another has already replaced.
-    int rsplit = 1;
+    // No row parts where the output lies over the input (one filter, in place): a CTA that starts late would integrate rows
+    // that another has already replaced.
     const bool in_place = x && ranges_overlap(x, (size_t)planes * h * w * sizeof(IO), out, (size_t)planes * F * h * w * sizeof(IO));
-    while (!in_place && tiles > 16 && planes * fsplit * rsplit * 2 <= 148 && rsplit < 4) rsplit *= 2;
+    const int rsplit = in_place ? 1 : split.rows;
     const int warps = (tiles + T - 1) / T, nf = (F + fsplit - 1) / fsplit;
     // rows per task: few long tasks read fewer tap rows twice, but every warp should get the same share
     int chunk = 1;
