@@ -216,7 +216,10 @@ size_t slab_partials_bytes(int N, int C, int F, int h, int w);
 int launch_integral_quad(const void *in, int io_kind, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s);
 // Of grad_output, in the order of additions that its integral images have always had (integral_scan.cu).
 int launch_integral_quad_ordered(const void *in, int io_kind, float *out, int64_t planes, int h, int w, cudaStream_t s);
-// The same kernel writing plain (h+1) x (w+1) rows; w up to 2048, h and w at least 1.
+// Would that kernel leave the GPU mostly idle?  Slabs are then not worth their integral images.
+bool integral_scan_starves(int64_t planes, int h, int w);
+// The same kernel writing plain (h+1) x (w+1) rows; w up to 2048, h and w at least 1; `suits`: faster than the older one.
+bool integral_scan_suits(const float *in, int64_t planes, int h, int w);
 int launch_integral_scan(const float *in, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s);
 // null `fu` = plain forward (16-bit outputs: always)
 int launch_forward_slab(const float *integ, const BoxParams &bp, const Fusion *fu, void *out, int io_kind, int N, int C, int F,

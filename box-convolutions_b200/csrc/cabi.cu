@@ -108,11 +108,15 @@ static inline size_t integral_bytes(int64_t planes, int h, int w)
 
 static size_t plane_partials_bytes(int N, int C, int F) { return align_up((size_t)C * F * N * kNumSums * sizeof(float), 256); }
 
+// Slabs, for float tensors whose `planes` integral images of a pass are not too few and too large for the kernel that
+// makes them?  (16-bit tensors have no other way.)
+static bool slabs_suit(int64_t planes, int F, int h, int w) { return slab_path_fits(F, h, w) && !integral_scan_starves(planes, h, w); }
+
 // Backward from the input's integral image on the whole-plane kernels?  (They may hold the plane and slabs be
 // faster all the same.)
 static bool plane_backward_integ(int64_t planes, int F, int h, int w)
 {
-    return plane_path_fits_backward_integ(F, h, w) && !(plane_path_prefers_slabs_backward(planes, F, h, w) && slab_path_fits(F, h, w));
+    return plane_path_fits_backward_integ(F, h, w) && !(plane_path_prefers_slabs_backward(planes, F, h, w) && slabs_suit(planes * F, F, h, w));
 }
 
 // Backward of planes that do not fit in shared memory, by slabs (workspace already checked).
@@ -168,7 +172,7 @@ static size_t backward_workspace_entry(int N, int C, int F, int h, int w, int ne
     if (!sizes_ok(N, C, F, h, w) || any_empty(N, C, F, h, w) || !(need_mask & BC_NEED_ALL)) return 0;
     if (std::is_same<T, float>::value) {
         if (plane_backward_integ((int64_t)N * C, F, h, w)) return plane_partials_bytes(N, C, F);
-        if (slab_path_fits(F, h, w))
+        if (slabs_suit((int64_t)N * C * F, F, h, w))
             return align_up(slab_integral_floats((int64_t)N * C * F, h, w) * sizeof(float), 256) +
                    align_up(slab_partials_bytes(N, C, F, h, w), 256);
     }
@@ -211,7 +215,7 @@ static int backward_entry(const T *input_integrated, const T *x_min, const T *x_
             return launch_backward_plane_integ(input_integrated, grad_output, bp, reparametrization_h, reparametrization_w, N, C, F, h,
                                                w, normalize != 0, exact != 0, need_mask, grad_input, grad_params,
                                                static_cast<float *>(workspace), stream);
-        if (slab_path_fits(F, h, w))
+        if (slabs_suit((int64_t)N * C * F, F, h, w))
             return backward_slabs(nullptr, input_integrated, BC_IO_F32, grad_output, bp, reparametrization_h, reparametrization_w, N, C,
                                   F, h, w, normalize != 0, exact != 0, need_mask, grad_input, grad_params, BC_IO_F32, workspace, stream);
     }
@@ -381,7 +385,7 @@ size_t bc_boxconv2d_forward_workspace(int N, int C, int F, int h, int w)
 {
     if (!sizes_ok(N, C, F, h, w) || any_empty(N, C, F, h, w)) return 0;
     if (plane_path_fits_forward(F, h, w)) return 0;
-    if (slab_path_fits(F, h, w)) return align_up(slab_integral_floats((int64_t)N * C, h, w) * sizeof(float), 256);
+    if (slabs_suit((int64_t)N * C, F, h, w)) return align_up(slab_integral_floats((int64_t)N * C, h, w) * sizeof(float), 256);
     if (band_path_fits_forward(h, w)) return align_up(band_integral_floats((int64_t)N * C, h, w) * sizeof(float), 256);
     return integral_bytes((int64_t)N * C, h, w);
 }
@@ -394,7 +398,7 @@ static int forward_from_workspace(const float *input, const BoxParams &bp, const
                                   cudaStream_t stream)
 {
     const bool relu_in = fu && fu->input_relu;
-    if (slab_path_fits(F, h, w)) {
+    if (slabs_suit((int64_t)N * C, F, h, w)) {
         int st = launch_integral_quad(input, BC_IO_F32, integ, (int64_t)N * C, h, w, relu_in, stream);
         if (st != BC_OK) return st;
         return launch_forward_slab(integ, bp, fu, output, BC_IO_F32, N, C, F, h, w, normalize, exact, stream);
@@ -461,7 +465,7 @@ static size_t backward_slabs_bytes(int N, int C, int F, int h, int w)
 // what then exceeds the limit.
 static bool backward_on_slabs(int N, int C, int F, int h, int w, size_t limit)
 {
-    return slab_path_fits(F, h, w) && backward_slabs_bytes(N, C, F, h, w) <= limit;
+    return slabs_suit((int64_t)N * C * F, F, h, w) && backward_slabs_bytes(N, C, F, h, w) <= limit;
 }
 static size_t backward_workspace_within(int N, int C, int F, int h, int w, int need_mask, size_t limit)
 {

@@ -411,7 +411,7 @@ int launch_integral_image_f32(const float *in, float *out, int64_t planes, int h
 {
     if (planes == 0) return BC_OK;
     if (planes > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
-    if (!lpad && h >= 1 && w >= 1 && w <= 2048) return launch_integral_scan(in, out, planes, h, w, relu_in, s);
+    if (!lpad && h >= 1 && w >= 1 && integral_scan_suits(in, planes, h, w)) return launch_integral_scan(in, out, planes, h, w, relu_in, s);
     const int pw = lpad + w + 1 + rpad;
     const bool vec4 = (w % 4 == 0) && ((reinterpret_cast<uintptr_t>(in) & 15) == 0);
     // A few tall planes (at most 64) cannot fill the GPU with one CTA each (a CTA walks down its plane tile by

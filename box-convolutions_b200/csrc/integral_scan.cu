@@ -405,20 +405,21 @@ integral_ordered_kernel(const IO *__restrict__ in, float *__restrict__ out, int 
 
 // How a plane of `tiles` warps' rows and `warps` warps a row is dealt out.  Few planes: to a cluster of at most 8 CTAs of
 // up to 16 warps, which hold it whole if they can (steps = 1; else they read it twice).  Many: to one CTA of 8 warps,
-// which walks down it ((512,256,512): 105 us against 154 as clusters; CTAs of 16 warps 116), or of 16 where there are
-// fewer planes than SMs ((128,280,560): 64 us, clusters 72).
+// which walks down it ((512,256,512): 102 us against 148 as clusters; CTAs of 16 warps 109), or of 16 where there are
+// fewer planes than SMs and a cluster would read them twice in two steps ((130,161,715): 64 us, clusters 78; in three
+// steps, (108,260,860): 92, 81).  `many16`: planes up to which the CTAs that walk have 16 warps.
 struct ScanShape {
     int G, ctas, steps;
 };
-inline ScanShape scan_shape(int64_t planes, int tiles, int warps)
+inline ScanShape scan_shape(int64_t planes, int tiles, int warps, int many16 = 148)
 {
     ScanShape s;
     const int most = kScanWarps / warps;
     s.ctas = (tiles + most - 1) / most;
     s.steps = 1;
-    if (s.ctas > 1 && (planes >= 148 || (planes >= 100 && s.ctas > 8))) {
+    if (s.ctas > 1 && (planes >= 148 || (planes >= 100 && s.ctas > 8 && s.ctas <= 16))) {
         s.ctas = 1;
-        const int fit = planes < 148 ? most : (8 / warps > 1 ? 8 / warps : 1);
+        const int fit = planes < many16 ? most : (8 / warps > 1 ? 8 / warps : 1);
         s.steps = (tiles + fit - 1) / fit;
     } else if (s.ctas > 8) {
         s.steps = (s.ctas + 7) / 8;
@@ -434,7 +435,9 @@ int integral_tile_t(const IO *in, float *out, int64_t planes, int h, int w, bool
 {
     const int warps = LN < 32 ? 1 : (w + 127) / 128, warp_rows = kScanRows * (32 / LN);
     const bool vec = w % 4 == 0 && aligned_to(in, Io<IO>::kVecBytes);
-    const ScanShape sh = scan_shape(planes, (h + warp_rows - 1) / warp_rows, warps);
+    // two CTAs of 16 warps an SM: up to one and a half rounds of them ((256,280,560): 80 us, 149 with 8 warps; (404,60,341):
+    // 21, 33; (424,568,105): 67, 77); not in the quad layout (368 planes of 110 x 450: 6 us more)
+    const ScanShape sh = scan_shape(planes, (h + warp_rows - 1) / warp_rows, warps, QUAD ? 148 : 3 * 148);
     if (planes * sh.ctas > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
     void (*kern)(const IO *, float *, int, int, int, int, int, int, bool);
     if (sh.G * warps <= 8) kern = vec ? integral_tile_kernel<IO, true, QUAD, LN, 256> : integral_tile_kernel<IO, false, QUAD, LN, 256>;
@@ -516,6 +519,32 @@ int launch_integral_quad_ordered(const void *in, int io_kind, float *out, int64_
     if (io_kind == BC_IO_F16) return integral_ordered_t(static_cast<const __half *>(in), out, planes, h, w, s);
     if (io_kind == BC_IO_BF16) return integral_ordered_t(static_cast<const __nv_bfloat16 *>(in), out, planes, h, w, s);
     return integral_ordered_t(static_cast<const float *>(in), out, planes, h, w, s);
+}
+
+static int scan_steps(int64_t planes, int h, int w, int lanes)
+{
+    const int rows = kScanRows * (32 / lanes);
+    return scan_shape(planes, (h + rows - 1) / rows, lanes < 32 ? 1 : (w + 127) / 128).steps;      // (of up to 147 planes)
+}
+
+// A plane or two, down which a cluster would walk many steps while the rest of the GPU has nothing to do: the kernels of
+// integral_image.cu cut them into bands that all SMs share (forward of (1,1,1,4000,900): 68 us against 125,
+// (1,1,4,2048,2048): 121 against 164, (1,2,2,20000,1): 62 against 129; of (1,2,2,2000,600), eleven steps: 50 against 52).
+bool integral_scan_starves(int64_t planes, int h, int w)
+{
+    return w <= 128 * kScanWarps && planes <= 2 && scan_steps(planes, h, w, 32) > 12;
+}
+
+// Plain rows.  The older kernel is faster on few planes of many steps as long as what its bands read again is in L2
+// ((1,2048,2048): 51 us against 128, (15,583,1121): 69 against 79; (11,2190,879): 328 against 166), and on nearly as many planes as
+// there are SMs, which clusters read twice, if their rows fit vector accesses ((128,280,560): 60 us against 69,
+// (108,260,860): 72 against 81; with other row lengths it is two to four times slower).
+bool integral_scan_suits(const float *in, int64_t planes, int h, int w)
+{
+    if (w > 128 * kScanWarps) return false;
+    const int steps = scan_steps(planes, h, w, w <= 32 ? 8 : w <= 64 ? 16 : 32);
+    if (planes <= 64 && steps > 8 && planes * h * w * 8 <= 96 << 20) return false;
+    return !(w % 4 == 0 && aligned_to(in, 16) && planes >= 100 && planes < 148 && steps > 1);
 }
 
 int launch_integral_scan(const float *in, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s)

@@ -27,7 +27,7 @@ def bc():
 # that read their plane twice, one CTA walking down; the widest row and one beyond (the older kernel)
 @pytest.mark.parametrize("planes,h,w", [
     (1, 1, 1), (3, 7, 31), (5, 8, 32), (2, 9, 33), (3, 129, 64), (2, 513, 30), (4, 33, 65), (2, 128, 128), (3, 136, 129),
-    (1, 1100, 40), (2, 300, 511), (1, 70, 2048), (1, 9, 2049), (150, 140, 130), (149, 17, 257), (110, 140, 1200), (1, 2100, 8),
+    (1, 1100, 40), (2, 300, 511), (1, 70, 2048), (1, 9, 2049), (150, 140, 130), (149, 17, 257), (110, 140, 1200), (1, 2100, 8), (1, 1100, 2000), (110, 141, 1201), (200, 150, 301),
 ])
 def test_integral_image_edges(bc, planes, h, w):
     x = torch.rand(planes, h, w, device="cuda", generator=torch.Generator("cuda").manual_seed(h + w))
@@ -80,7 +80,7 @@ def _compare(got, want):
 SHAPES = [(1, 2, 2, 8, 65), (2, 2, 3, 64, 128), (1, 3, 2, 65, 127), (1, 2, 1, 63, 129), (1, 2, 2, 64, 256), (1, 1, 2, 72, 250),
           (1, 2, 2, 128, 126), (1, 1, 3, 121, 93), (2, 1, 2, 128, 252), (1, 1, 2, 256, 256), (1, 2, 2, 201, 257), (1, 2, 3, 30, 1030),
           (1, 1, 2, 72, 2000), (1, 1, 2, 150, 2000), (2, 35, 1, 150, 1992), (3, 25, 2, 240, 220), (2, 3, 2, 1100, 48), (1, 1, 1, 230, 2047),
-          (20, 30, 2, 8, 68), (4, 5, 32, 9, 90)]
+          (20, 30, 2, 8, 68), (4, 5, 32, 9, 90), (1, 1, 2, 13000, 5)]
 
 
 @pytest.mark.parametrize("normalize,exact", [(True, True), (False, False)])
