@@ -266,9 +266,32 @@ __device__ __forceinline__ Walk make_walk(uint32_t sI32, const BoxTaps &t, int q
     return o;
 }
 
+// Rows 0 .. h of an integral image (plain rows of w + 1 floats) into shared memory by a CTA's warps: `put(a, col, value)`
+// for the columns 0 .. cols-1, of which those past w repeat the value at w.  A warp has nine rows in flight; with one,
+// whose load the store waits for, a CTA spent most of its time here ((1,8,4,32,32): 18 us, now 6.5).
+template <class Put>
+__device__ __forceinline__ void copy_integral_rows(const float *I, int h, int w, int cols, int warp, int nwarps, int lane, Put &&put)
+{
+    constexpr int kRowsInFlight = 9;      // (eight, and row 0, where a warp's share is a tile of eight rows)
+    const int stride = nwarps * (w + 1);
+    for (int a0 = warp; a0 <= h; a0 += kRowsInFlight * nwarps) {
+        for (int col = lane; col < cols; col += 32) {
+            const float *at = I + a0 * (w + 1) + min(col, w);
+            float e[kRowsInFlight];
+#pragma unroll
+            for (int i = 0; i < kRowsInFlight; ++i) e[i] = a0 + i * nwarps <= h ? __ldg(at + i * stride) : 0.0f;
+#pragma unroll
+            for (int i = 0; i < kRowsInFlight; ++i)
+                if (a0 + i * nwarps <= h) put(a0 + i * nwarps, col, e[i]);
+        }
+    }
+}
+
 // FUSED: the inference steps of `Fusion` around the gather (the output may then alias the residual,
 // so it is not declared restrict).
-template <typename IO, int T, bool FAST, bool FUSED = false>
+// INTEG: `integ` holds the plane's integral image, plain rows of w + 1 floats, which is only copied (instantiations of
+// their own: as a run-time branch it cost the others 3 to 5 %).
+template <typename IO, int T, bool FAST, bool FUSED = false, bool INTEG = false>
 __global__ void __launch_bounds__(T == 1 ? 256 : 512, T == 1 ? (FUSED ? 2 : 4) : 1)
 forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, BoxParams bp, IO *out, int C, int F,
                      int h, int w, int fsplit, bool normalize, bool exact, Fusion fu)
@@ -291,7 +314,7 @@ forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, 
 
     // a hint only: the plane on its way to L2 while this CTA still waits for the kernel in front
     if (FUSED && fu.residual) prefetch_l2(fu.residual + (nc * F + f_begin) * (int64_t)h * w, (size_t)(f_end - f_begin) * h * w * sizeof(float));
-    if (FAST && x && IsFloat<IO>::value && threadIdx.x == 0 && part == 0)
+    if (FAST && !INTEG && IsFloat<IO>::value && threadIdx.x == 0 && part == 0)
         bulk_prefetch_l2(x + nc * (int64_t)h * w, (uint32_t)(h * w) * 4u);
     Strip st[T];
 #pragma unroll
@@ -306,13 +329,12 @@ forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, 
         store_taps(sTaps + threadIdx.x * kTapWords,
                    taps_forward(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
     }
-    if (!x) {      // the caller has the integral image itself: it is only copied
+    if (INTEG) {
         const float *I = integ + nc * (int64_t)(h + 1) * (w + 1);
         const int pitch = g.pitch4 >> 2;
         __syncthreads();      // (the zero padding has been written)
-        for (int a = warp; a <= h; a += nwarps)
-            for (int col = lane; col < w + 1 + kPad; col += 32)
-                sI[a * pitch + (a >> 3) + kPad + col] = __ldg(I + (int64_t)a * (w + 1) + min(col, w));
+        copy_integral_rows(I, h, w, w + 1 + kPad, warp, nwarps, lane,
+                           [&](int a, int col, float e) { sI[a * pitch + (a >> 3) + kPad + col] = e; });
         __syncthreads();
     } else {
         Blocks<T> blk;
@@ -407,7 +429,8 @@ enum XAt { X_SHARED, X_GLOBAL, X_TENSOR };
 // plane runs while the current one is gathered.
 // The input plane in shared memory is float whatever IO is: float planes arrive by a bulk copy when
 // STAGED, narrow ones are converted by the threads as they are copied in.
-template <typename IO, int T, bool FAST, bool STAGED, bool NEED_PARAMS, XAt X_AT = X_SHARED, bool COUNTED = false>
+// INTEG: the input is given as its integral image (instantiations of their own: as a run-time branch it cost the others 5 %).
+template <typename IO, int T, bool FAST, bool STAGED, bool NEED_PARAMS, XAt X_AT = X_SHARED, bool COUNTED = false, bool INTEG = false>
 __global__ void __launch_bounds__(512)
 backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const IO *__restrict__ grad_output, BoxParams bp,
                       IO *__restrict__ grad_input, float *__restrict__ partials, int N, int C, int F,
@@ -454,10 +477,10 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
         // While this CTA waits for the kernel in front of it, its first planes can already travel to L2
         // (a hint: if that kernel is still writing them, L2 receives its writes as well).
         bulk_prefetch_l2(gbase, plane_bytes);
-        if (NEED_PARAMS && X_BY_COPY && !x_integ) bulk_prefetch_l2(x + nc * (int64_t)npix, plane_bytes);
+        if (NEED_PARAMS && X_BY_COPY && !INTEG) bulk_prefetch_l2(x + nc * (int64_t)npix, plane_bytes);
         grid_dependency_wait();      // grad_output and the input may come from the kernel in front
         bulk_load(sG32, gbase, plane_bytes, mbarG);
-        if (NEED_PARAMS && X_BY_COPY && !x_integ) bulk_load(sX32, x + nc * (int64_t)npix, plane_bytes, mbarX);
+        if (NEED_PARAMS && X_BY_COPY && !INTEG) bulk_load(sX32, x + nc * (int64_t)npix, plane_bytes, mbarX);
         if (F > 1) bulk_prefetch_l2(gbase + (int64_t)npix, plane_bytes);
     }
     init_integral_padding(sI, g);
@@ -484,7 +507,7 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
             for (int i = 0; i < kR; ++i) {
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (st[k].active && (FAST || st[k].p0 + i < h)) {
-                    if (x_integ) {      // the caller has only the input's integral image: its pixels are second differences
+                    if (INTEG) {      // the caller has only the input's integral image: its pixels are second differences
                         const float *Ip = I + (int64_t)(st[k].p0 + i) * (w + 1) + st[k].q0;
                         v.x = pixel_of_integral(Ip, w + 1);
                         if (st[k].q0 + 1 < w) v.y = pixel_of_integral(Ip + 1, w + 1);
@@ -505,7 +528,7 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
         }
         tmem_wait_store();
     }
-    if (XSMEM && x_integ) {
+    if (XSMEM && INTEG) {
         // (read by the first gather, which follows the barriers of the first build)
         const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1);
         for (int p = warp; p < h; p += nwarps)
@@ -553,7 +576,7 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
                     if (st[k].active && st[k].p0 + i < h)
                         asm volatile("prefetch.global.L2 [%0];" ::"l"(gbase + (f + 1) * (int64_t)npix + st[k].pix + i * w));
         }
-        if (X_BY_COPY && NEED_PARAMS && !x_integ && f == 0) timed_out |= !mbar_wait(mbarX, 0);
+        if (X_BY_COPY && NEED_PARAMS && !INTEG && f == 0) timed_out |= !mbar_wait(mbarX, 0);
 
         const BoxTaps t = load_taps(sTaps + f * kTapWords);
         const ColW2 cw = col_weights(t);
@@ -770,7 +793,8 @@ template <typename IO>
 int launch_forward_plane_t(const IO *x, const float *integ, const BoxParams &bp, const Fusion *fu, IO *out, int N, int C, int F, int h,
                            int w, bool normalize, bool exact, cudaStream_t s)
 {
-    if (quad_fits_forward(F, h, w) && quad_prefers_forward((int64_t)N * C, F, h, w)) return launch_forward_quad_t<IO>(x, integ, bp, fu, out, N, C, F, h, w, normalize, exact, s);
+    if (quad_fits_forward(F, h, w) && (x ? quad_prefers_forward((int64_t)N * C, F, h, w) : quad_prefers_forward_integ((int64_t)N * C, F, h, w)))
+        return launch_forward_quad_t<IO>(x, integ, bp, fu, out, N, C, F, h, w, normalize, exact, s);
     const int64_t planes = (int64_t)N * C;
     // Split the filters of a plane over two CTAs when there are too few planes to balance 148 SMs
     // (each part rebuilds the integral image; the second read of the plane comes from L2).
@@ -787,7 +811,11 @@ int launch_forward_plane_t(const IO *x, const float *integ, const BoxParams &bp,
     const bool fast = (h % kR == 0) && (w % kStrip == 0) && aligned_to(x, vec) && aligned_to(out, vec) &&
                       (!fu || !fu->residual || aligned_to(fu->residual, 16));
     void (*kern)(const IO *, const float *, BoxParams, IO *, int, int, int, int, int, bool, bool, Fusion);
-    if (fu && IsFloat<IO>::value) {
+    constexpr bool FL = IsFloat<IO>::value;      // (integral images are float)
+    if (!x) {
+        if (fast) kern = T == 1 ? forward_plane_kernel<IO, 1, true, false, FL> : forward_plane_kernel<IO, 2, true, false, FL>;
+        else kern = T == 1 ? forward_plane_kernel<IO, 1, false, false, FL> : forward_plane_kernel<IO, 2, false, false, FL>;
+    } else if (fu && IsFloat<IO>::value) {
         if (fast) kern = T == 1 ? forward_plane_kernel<IO, 1, true, IsFloat<IO>::value> : forward_plane_kernel<IO, 2, true, IsFloat<IO>::value>;
         else kern = T == 1 ? forward_plane_kernel<IO, 1, false, IsFloat<IO>::value> : forward_plane_kernel<IO, 2, false, IsFloat<IO>::value>;
     } else if (fu) {
@@ -852,24 +880,25 @@ int launch_backward_plane_t(const IO *x, const float *x_integ, const IO *grad_ou
     const int64_t outputs = planes * F * h * w;
     const bool may_finish = need_params && (tensor || (planes <= 148 && outputs <= 256 * 1024));
     const Finish fin = finish_here(bp, may_finish, planes, outputs, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w, s);
-    auto pick = [&](auto counted) {
-        constexpr bool K = decltype(counted)::value;
+    auto pick = [&](auto counted, auto integ) {
+        constexpr bool K = decltype(counted)::value, I = decltype(integ)::value;
         if (tensor) {
-            kern = fast ? backward_plane_kernel<IO, 2, true, false, true, X_TENSOR, K> : backward_plane_kernel<IO, 2, false, false, true, X_TENSOR, K>;
+            kern = fast ? backward_plane_kernel<IO, 2, true, false, true, X_TENSOR, K, I> : backward_plane_kernel<IO, 2, false, false, true, X_TENSOR, K, I>;
         } else if (need_params && !xsmem) {
-            kern = backward_plane_kernel<IO, 2, true, false, true, X_GLOBAL, K>;      // (planes of up to eight tiles always fit)
+            kern = backward_plane_kernel<IO, 2, true, false, true, X_GLOBAL, K>;      // (planes of up to eight tiles always fit; never from an integral image)
         } else if (staged) {
-            kern = need_params ? backward_plane_kernel<IO, 1, true, true, true, X_SHARED, K> : backward_plane_kernel<IO, 1, true, true, false>;
+            kern = need_params ? backward_plane_kernel<IO, 1, true, true, true, X_SHARED, K, I> : backward_plane_kernel<IO, 1, true, true, false>;
         } else if (fast) {
-            kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, true, false, true, X_SHARED, K> : backward_plane_kernel<IO, 1, true, false, false>)
-                          : (need_params ? backward_plane_kernel<IO, 2, true, false, true, X_SHARED, K> : backward_plane_kernel<IO, 2, true, false, false>);
+            kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, true, false, true, X_SHARED, K, I> : backward_plane_kernel<IO, 1, true, false, false>)
+                          : (need_params ? backward_plane_kernel<IO, 2, true, false, true, X_SHARED, K, I> : backward_plane_kernel<IO, 2, true, false, false>);
         } else {
-            kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, false, false, true, X_SHARED, K> : backward_plane_kernel<IO, 1, false, false, false>)
+            kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, false, false, true, X_SHARED, K, I> : backward_plane_kernel<IO, 1, false, false, false>)
                           : backward_plane_kernel<IO, 2, false, false, false>;
         }
     };
-    if (fin.total) pick(Flag<true>{});
-    else pick(Flag<false>{});
+    if (x_integ) pick(Flag<false>{}, Flag<IsFloat<IO>::value>{});      // (the four functions have no counters)
+    else if (fin.total) pick(Flag<true>{}, Flag<false>{});
+    else pick(Flag<false>{}, Flag<false>{});
     int st = opt_in_smem(kern, smem);
     if (st != BC_OK) return st;
     {

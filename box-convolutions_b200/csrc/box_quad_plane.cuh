@@ -534,6 +534,16 @@ inline bool quad_prefers_forward(int64_t planes, int F, int h, int w)
     if (w % 4 == 0 && h % kTileRows == 0) return tiles <= square || few;
     return (w > 96 && w <= 128 && (tiles <= 8 || full)) || (w % 4 == 0 && tiles > 8 && (full || few));
 }
+// The same from the plane's integral image, which both kernels copy, this one a row a warp at a time: large planes of two
+// column tiles, and small ones of full rows (684 planes of 80 x 248, F = 3: 92 us against 110; 448 of 48 x 120, F = 4: 21
+// against 25; (97,9,4,112,104): 177 against 107; 1024 planes of 64 x 128, F = 4: 62 against 55).
+inline bool quad_prefers_forward_integ(int64_t planes, int F, int h, int w)
+{
+    if (!quad_prefers_forward(planes, F, h, w)) return false;
+    const int tiles = quad_row_tiles(h) * quad_col_tiles(w), square = ((h + 31) / 32) * ((w + 31) / 32);
+    if (quad_col_tiles(w) == 2) return tiles <= 8 || tiles > 16;
+    return tiles <= 8 && tiles < square && w % 4 == 0 && h % kTileRows == 0;
+}
 inline bool quad_fits_forward(int F, int h, int w)
 {
     const int tiles = quad_row_tiles(h) * quad_col_tiles(w);
