@@ -163,6 +163,7 @@ int launch_forward_plane_fused(const float *x, const BoxParams &bp, const Fusion
 // Shared-memory-resident path for small planes (box_plane_smem.cu).
 bool plane_path_fits_forward(int F, int h, int w);
 bool plane_path_fits_backward(int F, int h, int w);
+bool plane_path_prefers_global_forward_integ(int64_t planes, int F, int h, int w);
 bool plane_path_prefers_slabs_backward(int64_t planes, int F, int h, int w);
 int launch_forward_plane(const float *x, const BoxParams &bp, float *out, int N, int C, int F, int h,
                          int w, bool normalize, bool exact, cudaStream_t s);

@@ -775,6 +775,17 @@ inline bool plane_fits_backward_integ(int F, int h, int w)
            (quad_fits_backward(F, h, w) || plane_backward_smem_bytes(h, w, true, false, 4) <= kMaxSmem);
 }
 
+// Forward from the input's integral image: copying it to shared memory pays where several filters, or several CTAs an
+// SM, share the copy's latency ((4,16,4,96,160): 13 us, straight from global memory 23; 3060 planes of 120 x 56, F = 3: 96, 316).
+// Not for one or two filters of large planes, which have an SM to themselves ((83,20,1,97,199): 180 against 115;
+// (65,11,2,224,120): 163 against 106), nor where few such planes leave most SMs idle, which the tiles of the global kernel do
+// not ((1,11,6,166,135): 23 against 15; (2,5,6,176,40): 12 against 8.5).
+inline bool plane_prefers_global_forward_integ(int64_t planes, int F, int h, int w)
+{
+    const int tiles = warp_tiles(h, w);
+    return (F <= 2 && tiles >= 16) || (planes * 8 <= 148 && tiles >= 12);
+}
+
 // From the input's integral image, planes of more than 8 tiles of 32 x 32, which occupy an SM alone in the backward
 // kernel of this file, are better off as slabs where they are wide enough ((4,16,4,96,160): 36 us against 48) or leave
 // half of the SMs idle ((1,17,8,143,44): 32 us against 82, (5,4,4,216,56): 28 against 58; (22,15,2,136,40): 54 against 48).

@@ -6,6 +6,7 @@ namespace bc {
 
 bool plane_path_fits_forward(int F, int h, int w) { return plane_fits_forward(F, h, w); }
 bool plane_path_fits_backward(int F, int h, int w) { return plane_fits_backward(F, h, w); }
+bool plane_path_prefers_global_forward_integ(int64_t planes, int F, int h, int w) { return plane_prefers_global_forward_integ(planes, F, h, w); }
 bool plane_path_prefers_slabs_backward(int64_t planes, int F, int h, int w) { return plane_prefers_slabs_backward(planes, F, h, w); }
 bool plane_path_fits_backward_integ(int F, int h, int w) { return plane_fits_backward_integ(F, h, w); }
 

@@ -159,8 +159,8 @@ static int forward_entry(const T *input_integrated, const T *x_min, const T *x_m
     if (!input_integrated || !x_min || !x_max || !y_min || !y_max || !output) return BC_ERR_NULL_POINTER;
     const BoxParamsT<T> bp{x_min, x_max, y_min, y_max, T(1), T(1)};
     if constexpr (std::is_same<T, float>::value) {
-        // a plane whose integral image fits in shared memory is gathered from there
-        if (plane_path_fits_forward(F, h, w))
+        // a plane whose integral image fits in shared memory is gathered from there, if that is faster
+        if (plane_path_fits_forward(F, h, w) && !plane_path_prefers_global_forward_integ((int64_t)N * C, F, h, w))
             return launch_forward_plane_integ(input_integrated, bp, output, N, C, F, h, w, normalize != 0, exact != 0, stream);
     }
     return launch_forward_global<T>(input_integrated, bp, output, N, C, F, h, w, normalize != 0, exact != 0, stream);
