@@ -44,7 +44,11 @@ def rounded(a, dtype):
     ((2, 3, 4, 64, 128), True),      # the 1/8-frame block: unguarded kernels, staged planes
     ((1, 2, 3, 40, 131), True),      # odd sizes: guarded kernels
     ((1, 2, 2, 128, 256), True),     # two tiles per warp, input plane read from global memory
-    ((1, 1, 2, 300, 300), False),    # too large for the shared-memory kernels: float copies
+    ((1, 1, 2, 300, 300), False),    # too large for the whole-plane kernels: slabs, whose integral images are float
+    ((1, 2, 2, 201, 257), False),    # slabs of rows that no vector access fits
+    ((1, 2, 2, 72, 250), True),      # such rows in 32 x 32 tiles, the input plane in tensor memory
+    ((2, 80, 1, 96, 160), True),     # the same with aligned rows
+    ((1, 1, 33, 40, 44), False),     # more filters than the kernels' tables hold: float copies
 ])
 @pytest.mark.parametrize("normalize,exact", [(True, True), (False, False)])
 def test_half_tensors_against_the_float_oracle(bc, dtype, shape, narrow, normalize, exact):

@@ -184,10 +184,12 @@ def test_narrow_parameters_are_clipped_as_floats(bc, dtype):
     assert all(torch.equal(a, b.to(dtype)) for a, b in zip(p, wide))
 
 
-# one, several, 8, 9 (up to 12), 13 and 16 warps a CTA, with and without cut rows, and slabs of 4 and 5 warps: more CTAs
-# than an SM has tensor memory for, from two streams at a time
+# one, several, 8, 9 (up to 12), 13 and 16 warps a CTA, with and without cut rows, slabs of 4 and 5 warps, and 32 x 32 tiles
+# two a warp, eight warps with aligned rows (two CTAs an SM ask for all its tensor memory) and twelve with others (one does):
+# more CTAs than an SM has tensor memory for, from two streams at a time
 @pytest.mark.parametrize("shape", [(8, 150, 2, 8, 96), (4, 150, 2, 33, 100), (4, 80, 2, 64, 128), (4, 80, 2, 66, 128), (4, 80, 1, 96, 70),
-                                   (2, 80, 1, 100, 128), (2, 80, 2, 64, 256), (2, 40, 2, 180, 300), (2, 30, 2, 180, 600)])
+                                   (2, 80, 1, 100, 128), (2, 80, 2, 64, 256), (2, 40, 2, 180, 300), (2, 30, 2, 180, 600),
+                                   (4, 40, 2, 96, 160), (2, 80, 2, 72, 250)])
 def test_backward_from_two_streams(bc, shape):
     """Every accumulator and input value comes back from where its own warp left it: bit for bit what a launch alone
     returns, and that against float64."""
