@@ -29,22 +29,8 @@ __device__ __forceinline__ BoxTaps load_taps_uniform(const float *tab)
     return t;
 }
 
-// Inclusive sum over the warp, or over each group of LN lanes, and in `before` the sum of the lanes in front, which is
-// added up by itself: taking a lane's own value off again would leave its infinity or its rounding in the columns to
-// its left.  The shuffle's own predicate tells which lanes have somebody to add.
-template <int LN = 32>
-__device__ __forceinline__ float warp_prefix(float v, float &before)
-{
-    before = 0.0f;
-#pragma unroll
-    for (int d = 1; d < LN; d <<= 1)
-        asm volatile("{\n .reg .f32 u;\n .reg .pred p;\n shfl.sync.up.b32 u|p, %0, %2, %3, 0xffffffff;\n @p add.f32 %1, %1, u;\n"
-                     " @p add.f32 %0, %0, u;\n}"
-                     : "+f"(v), "+f"(before) : "r"(d), "n"((32 - LN) << 8));
-    return v;
-}
-
-// The inclusive sum alone.
+// Inclusive sum over the warp, or over each group of LN lanes; the shuffle's own predicate tells which lanes have
+// somebody to add.
 template <int LN = 32>
 __device__ __forceinline__ float warp_scan(float v)
 {
@@ -53,6 +39,17 @@ __device__ __forceinline__ float warp_scan(float v)
         asm volatile("{\n .reg .f32 u;\n .reg .pred p;\n shfl.sync.up.b32 u|p, %0, %1, %2, 0xffffffff;\n @p add.f32 %0, %0, u;\n}"
                      : "+f"(v) : "r"(d), "n"((32 - LN) << 8));
     return v;
+}
+
+// The same, and in `before` the inclusive sum of the lane in front (zero for the first): taking a lane's own value off
+// its inclusive sum again would leave its infinity or its rounding in the columns to its left.
+template <int LN = 32>
+__device__ __forceinline__ float warp_prefix(float v, float &before)
+{
+    const float incl = warp_scan<LN>(v);
+    asm volatile("{\n .reg .f32 u;\n .reg .pred p;\n shfl.sync.up.b32 u|p, %1, 1, %2, 0xffffffff;\n selp.f32 %0, u, 0f00000000, p;\n}"
+                 : "=f"(before) : "f"(incl), "n"((32 - LN) << 8));
+    return incl;
 }
 
 // Byte offsets within a row of the five taps on either side of the box, for the strip of columns 4*j .. 4*j+3.
