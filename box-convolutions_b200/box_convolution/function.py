@@ -9,9 +9,9 @@ there) and the term the reference takes from the saved output is recomputed, so 
 packed copy of the parameters are kept alive between forward and backward.
 
 float64 tensors (gradient checks) take the general kernels, chained as the reference chains them.
-float16 / bfloat16 tensors: planes that the shared-memory kernels hold are read and written in their
-16-bit type by those kernels (float arithmetic on chip, float parameter gradients rounded at the end);
-larger planes go through float copies, and results and gradients are rounded back.
+float16 / bfloat16 tensors of up to 2048 columns and 32 filters are read and written in their 16-bit type
+(float arithmetic and integral images, parameter gradients rounded once at the end); wider planes and
+more filters go through float copies, and results and gradients are rounded back.
 """
 import torch
 

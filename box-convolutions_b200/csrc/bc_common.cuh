@@ -215,7 +215,7 @@ bool slab_path_fits(int F, int h, int w);
 size_t slab_integral_floats(int64_t planes, int h, int w);
 size_t slab_partials_bytes(int N, int C, int F, int h, int w);
 int launch_integral_quad(const void *in, int io_kind, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s);
-// Of grad_output, in the order of additions that its integral images have always had (integral_scan.cu).
+// Of grad_output, in integral_image_kernel's order of additions where integral_ordered_kernel serves it (integral_scan.cu).
 int launch_integral_quad_ordered(const void *in, int io_kind, float *out, int64_t planes, int h, int w, cudaStream_t s);
 // Would that kernel leave the GPU mostly idle?  Slabs are then not worth their integral images.
 bool integral_scan_starves(int64_t planes, int h, int w);

@@ -1,15 +1,17 @@
-// Shared-memory-resident kernels for planes small enough to keep on chip and too narrow (64 columns) or too large
-// for the quad layout's tiles of 8 x 128 (box_quad_plane.cuh).  HBM traffic is the compulsory minimum: the forward
+// Shared-memory-resident kernels in tiles of 32 x 32, for planes small enough to keep on chip that are too narrow (64
+// columns) or too large for the quad layout's tiles of 8 x 128, or waste less in these (quad_prefers_forward() in
+// box_quad_plane.cuh).  HBM traffic is the compulsory minimum: the forward
 // reads the input once and writes the output once; the backward reads the input and grad_output
 // once and writes grad_input once.  No integral image ever goes to global memory.
 //
 // Forward : one CTA per (plane, group of filters).  The plane's integral image is built in shared
 //           memory, then every thread walks its 4-column x 8-row strip (bc_walk.cuh scheme) for
 //           each filter of the group and writes 128-bit rows of the output.
-// Backward: one CTA per plane.  The input plane stays in shared memory; for each filter the
-//           grad_output plane is integrated in shared memory and gathered with the mirrored box.
-//           Grad-input accumulates in registers over the filters; the five sums that finish the
-//           parameter gradients are reduced per CTA and left for finish_param_grads_kernel.
+// Backward: one CTA per plane.  For each filter the grad_output plane is integrated in shared memory and
+//           gathered with the mirrored box.  The input plane waits in shared memory, in tensor memory or nowhere
+//           (enum XAt), grad-input accumulates over the filters in registers or beside it in tensor memory.  The
+//           five sums that finish the parameter gradients are reduced per CTA and left for
+//           finish_param_grads_kernel or the channel's last CTA (bc_finish.cuh).
 //
 // Thread layout (same for building the integral image and for gathering): a warp owns a tile of
 // 32 x 32 pixels; lane = 8 column groups (cg, 4 columns each) x 4 row groups (rg, 8 rows each).

@@ -277,9 +277,13 @@ __device__ __forceinline__ float row_prefix(float4 &v, float &total)
 
 // The same, in a fixed order of additions: along the rows first, then down the columns one row after the other from
 // the top of the plane, or of the plane's band when there are `bands` of `band_tiles` tiles each (what the bands
-// above add up to is added last).  This is the order in which integral images of grad_output have always been
-// added up.  Parameter gradients of large planes hang on its rounding (differences of sums of 1e5 values: relative
-// errors of 1e-5), so a change of order shows in the fifth digit of results that users compare between versions.
+// above add up to is added last).  This is the order in which integral_image_kernel adds up planes whose rows a vector
+// access fits, and in which integral images of grad_output have been added up since before this kernel; it includes
+// that kernel's way of taking a lane's own sum off the warp's.  Parameter gradients of large planes hang on its
+// rounding (differences of sums of 1e5 values: relative errors of 1e-5), so a change of order shows in the fifth digit of
+// results that users compare between versions.  Not every plane has it: rows of other lengths, tensors that begin
+// off a vector's alignment and some tall planes go to the other kernel (integral_ordered_t), which rounds otherwise, so
+// that the same values at another address can give gradients that differ in that digit.
 // What is serial are only the additions: tile after tile through shared memory, about 130 cycles each, CTA after
 // CTA through distributed shared memory.
 // T: 8-row tiles a thread holds (2 where one would need more than 8 CTAs a plane).

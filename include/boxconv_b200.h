@@ -152,7 +152,8 @@ int bc_boxconv2d_forward(const float *input, const float *x_min, const float *x_
  *   k = c*F + f.
  *   input_relu   nonzero: ReLU on the input as it is read;
  *   out_scale, out_shift  (C*F) each, the folded BatchNorm of the output channels; NULL = 1 / 0;
- *   residual     (N, C*F, h, w) or NULL; may be the output buffer itself (in-place skip connection);
+ *   residual     (N, C*F, h, w) or NULL; may be the output buffer itself (in-place skip connection), and with
+ *                F = 1 both may be the input;
  *   output_relu  nonzero: ReLU on the result.
  * No gradients.  Workspace as bc_boxconv2d_forward_workspace(). */
 int bc_boxconv2d_forward_fused(const float *input, const float *x_min, const float *x_max,
