@@ -44,6 +44,7 @@
 #include "bc_tile_io.cuh"
 #include "bc_tmem.cuh"
 #include "box_quad_plane.cuh"
+#include "box_tmem_plane.cuh"
 
 namespace bc {
 
@@ -806,6 +807,8 @@ template <typename IO>
 int launch_forward_plane_t(const IO *x, const float *integ, const BoxParams &bp, const Fusion *fu, IO *out, int N, int C, int F, int h,
                            int w, bool normalize, bool exact, cudaStream_t s)
 {
+    if (x && !fu && tmem_suits_forward((int64_t)N * C, F, h, w) && aligned_to(x, Io<IO>::kVecBytes) && aligned_to(out, Io<IO>::kVecBytes))
+        return launch_forward_tmem_t<IO>(x, bp, out, N, C, F, h, w, normalize, exact, s);
     if (quad_fits_forward(F, h, w) && (x ? quad_prefers_forward((int64_t)N * C, F, h, w) : quad_prefers_forward_integ((int64_t)N * C, F, h, w)))
         return launch_forward_quad_t<IO>(x, integ, bp, fu, out, N, C, F, h, w, normalize, exact, s);
     const int64_t planes = (int64_t)N * C;
