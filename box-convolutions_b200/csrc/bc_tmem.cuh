@@ -61,12 +61,6 @@ __device__ __forceinline__ void tmem_load16(uint32_t at, float4 (&v)[4])
                    "=f"(v[2].x), "=f"(v[2].y), "=f"(v[2].z), "=f"(v[2].w), "=f"(v[3].x), "=f"(v[3].y), "=f"(v[3].z), "=f"(v[3].w)
                  : "r"(at) : "memory");
 }
-__device__ __forceinline__ void tmem_store16(uint32_t at, const float4 (&v)[4])
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                 ::"r"(at), "f"(v[0].x), "f"(v[0].y), "f"(v[0].z), "f"(v[0].w), "f"(v[1].x), "f"(v[1].y), "f"(v[1].z), "f"(v[1].w),
-                 "f"(v[2].x), "f"(v[2].y), "f"(v[2].z), "f"(v[2].w), "f"(v[3].x), "f"(v[3].y), "f"(v[3].z), "f"(v[3].w) : "memory");
-}
 // (the loaded registers are operands, so that nothing uses them before)
 __device__ __forceinline__ void tmem_wait_load(float4 &a, float4 &b)
 {

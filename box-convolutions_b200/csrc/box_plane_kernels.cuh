@@ -44,7 +44,6 @@
 #include "bc_tile_io.cuh"
 #include "bc_tmem.cuh"
 #include "box_quad_plane.cuh"
-#include "box_tmem_backward.cuh"
 #include "box_tmem_plane.cuh"
 
 namespace bc {
@@ -858,13 +857,6 @@ int launch_backward_plane_t(const IO *x, const float *x_integ, const IO *grad_ou
                             int C, int F, int h, int w, bool normalize, bool exact, int need_mask, IO *grad_input,
                             void *grad_params, int grad_params_kind, float *partials, cudaStream_t s)
 {
-    constexpr int kAll = BC_NEED_ALL & ~BC_NEED_INPUT;
-    if (x && (need_mask & kAll) && (need_mask & BC_NEED_INPUT) && tmem_suits_backward((int64_t)N * C, F, h, w) && aligned_to(x, 16) &&
-        aligned_to(grad_output, 16) && aligned_to(grad_input, Io<IO>::kVecBytes)) {
-        const int st = launch_backward_tmem_t<IO>(x, grad_output, bp, N, C, F, h, w, normalize, exact, grad_input, partials, s);
-        return st != BC_OK ? st : launch_finish_param_grads<float>(partials, bp, C * F, N, normalize, exact, rep_h, rep_w, need_mask, grad_params, s,
-                                                                   grad_params_kind);
-    }
     if (quad_fits_backward(F, h, w))
         return launch_backward_quad_t<IO>(x, x_integ, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
                                           grad_params, grad_params_kind, partials, s);

@@ -101,18 +101,34 @@ __device__ __forceinline__ void quad_load_tile(QuadBlock &v, const QuadTile &t, 
     }
 }
 
-// What a row has in front of each lane, for eight rows at once: `u`, the lanes' sums, become the sums of the lanes in front.
-// The sums of a row's 32 lanes are scanned through a corner of shared memory: four lanes a row, each with eight of its
-// values, then two shuffle steps.  Shuffling every row by itself takes five shuffles and five additions a row, twice
-// the instructions.  Returns, in the lanes 3, 7, 11 ..., the sum of row lane / 4.
+// Build, first part: the tile's own 2-D prefix sums; with several column tiles only down its columns and along
+// its rows within the tile, the rows' totals being published (followed by a barrier).
+// The sums of a row's 32 lanes are scanned eight rows at once through a corner of shared memory: four lanes a
+// row, each with eight of its values, then two shuffle steps.  Shuffling every row by itself takes five
+// shuffles and five additions a row, twice the instructions.
 constexpr int kScanPitch = 36;      // words per row: eight lanes' 16-byte accesses fall into distinct banks
 constexpr int kScanBytes = kTileRows * kScanPitch * 4;
-__device__ __forceinline__ float rows8_before(uint32_t scan, float (&u)[kTileRows], int lane)
+template <int CT>
+__device__ __forceinline__ void quad_scan(QuadBlock &v, float (&carry)[kTileRows], const QuadTile &t, const QuadSmem &s, int warp, int lane)
 {
+    const uint32_t scan = s.scan + warp * kScanBytes;
+#pragma unroll
+    for (int i = 0; i < kTileRows; ++i) {
+        if (i) { v.a[i] = add2(v.a[i], v.a[i - 1]); v.b[i] = add2(v.b[i], v.b[i - 1]); }
+    }
     __syncwarp();
-    auto put = [&](auto I) { constexpr int i = decltype(I)::value; sts<i * kScanPitch * 4>(scan + lane * 4, u[i]); };
-    put(Index<0>{}); put(Index<1>{}); put(Index<2>{}); put(Index<3>{});
-    put(Index<4>{}); put(Index<5>{}); put(Index<6>{}); put(Index<7>{});
+    auto row_of = [&](auto I) {
+        constexpr int i = decltype(I)::value;
+        float x, y, z, u;
+        unpack2(v.a[i], x, y);
+        unpack2(v.b[i], z, u);
+        y += x; z += y; u += z;
+        v.a[i] = pack2(x, y);
+        v.b[i] = pack2(z, u);
+        sts<i * kScanPitch * 4>(scan + lane * 4, u);
+    };
+    row_of(Index<0>{}); row_of(Index<1>{}); row_of(Index<2>{}); row_of(Index<3>{});
+    row_of(Index<4>{}); row_of(Index<5>{}); row_of(Index<6>{}); row_of(Index<7>{});
     __syncwarp();
     const int k = lane & 3;
     const uint32_t mine = scan + (lane >> 2) * (kScanPitch * 4) + k * 32;
@@ -125,36 +141,13 @@ __device__ __forceinline__ float rows8_before(uint32_t scan, float (&u)[kTileRow
     float before = k >= 1 ? one : 0.0f;
     const float two = __shfl_up_sync(0xffffffffu, q.w + before, 2);
     if (k >= 2) before += two;
+    if (CT > 1 && k == 3) sts<0>(s.row + (t.rt * CT + t.ct) * 32 + (lane >> 2) * 4, before + q.w);
     sts128(mine, make_float4(before, before + p.x, before + p.y, before + p.z));
     sts128(mine + 16, make_float4(before + p.w, before + q.x, before + q.y, before + q.z));
     __syncwarp();
-    auto get = [&](auto I) { constexpr int i = decltype(I)::value; u[i] = lds<i * kScanPitch * 4>(scan + lane * 4); };
-    get(Index<0>{}); get(Index<1>{}); get(Index<2>{}); get(Index<3>{});
-    get(Index<4>{}); get(Index<5>{}); get(Index<6>{}); get(Index<7>{});
-    return before + q.w;
-}
-
-// Build, first part: the tile's own 2-D prefix sums; with several column tiles only down its columns and along
-// its rows within the tile, the rows' totals being published (followed by a barrier).
-template <int CT>
-__device__ __forceinline__ void quad_scan(QuadBlock &v, float (&carry)[kTileRows], const QuadTile &t, const QuadSmem &s, int warp, int lane)
-{
-#pragma unroll
-    for (int i = 0; i < kTileRows; ++i) {
-        if (i) { v.a[i] = add2(v.a[i], v.a[i - 1]); v.b[i] = add2(v.b[i], v.b[i - 1]); }
-    }
-#pragma unroll
-    for (int i = 0; i < kTileRows; ++i) {
-        float x, y, z, u;
-        unpack2(v.a[i], x, y);
-        unpack2(v.b[i], z, u);
-        y += x; z += y; u += z;
-        v.a[i] = pack2(x, y);
-        v.b[i] = pack2(z, u);
-        carry[i] = u;
-    }
-    const float total = rows8_before(s.scan + warp * kScanBytes, carry, lane);
-    if (CT > 1 && (lane & 3) == 3) sts<0>(s.row + (t.rt * CT + t.ct) * 32 + (lane >> 2) * 4, total);
+    auto carry_of = [&](auto I) { constexpr int i = decltype(I)::value; carry[i] = lds<i * kScanPitch * 4>(scan + lane * 4); };
+    carry_of(Index<0>{}); carry_of(Index<1>{}); carry_of(Index<2>{}); carry_of(Index<3>{});
+    carry_of(Index<4>{}); carry_of(Index<5>{}); carry_of(Index<6>{}); carry_of(Index<7>{});
 }
 // Second part: carries joined, the tile's last row published as what it adds to the tiles below.  Followed by a
 // barrier.

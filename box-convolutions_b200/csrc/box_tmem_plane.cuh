@@ -77,13 +77,12 @@ __device__ __forceinline__ void tmem_make_rows(const TmemUnit &n, const BoxTaps 
     tmem_wait_store();
 }
 
-// The warp's rows of box sums from the unit's rows of D, four at a time: sink(p, g) takes rows p .. p+3, two pairs of
-// columns each, times the box's scale unless RAW.
-template <bool RAW, class Sink>
-__device__ __forceinline__ void tmem_box_rows(const TmemUnit &n, const BoxTaps &t, Sink &&sink)
+// The warp's output rows from the unit's rows of D; `row`: the first of them.
+template <typename IO>
+__device__ __forceinline__ void tmem_use_rows(const TmemUnit &n, const BoxTaps &t, IO *row, int q0, int w)
 {
-    const float whole = RAW ? 1.0f : t.scale, high = whole * t.f_hi_r, low = whole * t.f_lo_r;
-    const f2_t whole2 = pack2(whole, whole), high2 = pack2(high, high), low2 = pack2(low, low);
+    const float sfl = t.scale * t.f_lo_r, sfh = t.scale * t.f_hi_r;
+    const f2_t scale2 = pack2(t.scale, t.scale), sfl2 = pack2(sfl, sfl), sfh2 = pack2(sfh, sfh);
     // The integral rows a .. a+3 combined (row 0 is zero, rows past the plane repeat its last).
     auto fetch = [&](float4 (&v)[4], int a) {
         __syncwarp();
@@ -115,35 +114,21 @@ __device__ __forceinline__ void tmem_box_rows(const TmemUnit &n, const BoxTaps &
         float4 L[4], H[4];      // those at lo and hi+1
         fetch(L, p + t.lo_r);
         fetch(H, p + t.hi_r + 1);
-        f2_t g[4][2];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            auto pair = [&](f2_t a, f2_t b, f2_t lo, f2_t hi) {
-                const f2_t mid = RAW ? sub2(b, lo) : mul2(sub2(b, lo), whole2);
-                return fma2(low2, sub2(lo, a), fma2(high2, sub2(hi, b), mid));
+            float v[kStrip];
+            auto pair = [&](f2_t a, f2_t b, f2_t lo, f2_t hi, float &v0, float &v1) {
+                const f2_t mid = mul2(sub2(b, lo), scale2);
+                unpack2(fma2(sfl2, sub2(lo, a), fma2(sfh2, sub2(hi, b), mid)), v0, v1);
             };
-            g[i][0] = pair(pack2(A.x, A.y), pack2(B.x, B.y), pack2(L[i].x, L[i].y), pack2(H[i].x, H[i].y));
-            g[i][1] = pair(pack2(A.z, A.w), pack2(B.z, B.w), pack2(L[i].z, L[i].w), pack2(H[i].z, H[i].w));
+            pair(pack2(A.x, A.y), pack2(B.x, B.y), pack2(L[i].x, L[i].y), pack2(H[i].x, H[i].y), v[0], v[1]);
+            pair(pack2(A.z, A.w), pack2(B.z, B.w), pack2(L[i].z, L[i].w), pack2(H[i].z, H[i].w), v[2], v[3]);
+            if (q0 < w) Io<IO>::store4(row + q0, v[0], v[1], v[2], v[3]);
+            row += w;
             A = L[i];
             B = H[i];
         }
-        sink(p, g);
     }
-}
-
-// The warp's output rows; `row`: the first of them.
-template <typename IO>
-__device__ __forceinline__ void tmem_use_rows(const TmemUnit &n, const BoxTaps &t, IO *row, int q0, int w)
-{
-    tmem_box_rows<false>(n, t, [&](int, f2_t (&g)[4][2]) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i, row += w) {
-            float v[kStrip];
-            unpack2(g[i][0], v[0], v[1]);
-            unpack2(g[i][1], v[2], v[3]);
-            if (q0 < w) Io<IO>::store4(row + q0, v[0], v[1], v[2], v[3]);
-        }
-    });
 }
 
 __device__ __forceinline__ TmemUnit tmem_unit(uint32_t tmem_base, int lanes, int part, int parts, int row_tiles, int h)
