@@ -91,20 +91,35 @@ __device__ __forceinline__ float lds_row(uint32_t row, uint32_t off)
 // costs one shuffle an address instead of the same clamps and multiplications in every lane.
 template <int R>
 struct QuadRows {
-    uint32_t lo[R + 1], hi[R + 1];
+    uint32_t lo_at[R + 1], hi_at[R + 1];
+    __device__ __forceinline__ uint32_t lo(int j) const { return lo_at[j]; }
+    __device__ __forceinline__ uint32_t hi(int j) const { return hi_at[j]; }
+};
+// The same, handed out where they are used: 2 R + 1 registers fewer.
+template <int R>
+struct QuadRowsLater {
+    uint32_t mine;
+    __device__ __forceinline__ uint32_t lo(int j) const { return __shfl_sync(0xffffffffu, mine, j); }
+    __device__ __forceinline__ uint32_t hi(int j) const { return __shfl_sync(0xffffffffu, mine, R + 1 + j); }
 };
 template <int R>
-__device__ __forceinline__ QuadRows<R> quad_rows(const BoxTaps &t, int p0, int h, uint32_t lo32, uint32_t hi32, int row_bytes, int lane)
+__device__ __forceinline__ QuadRowsLater<R> quad_rows_later(const BoxTaps &t, int p0, int h, uint32_t lo32, uint32_t hi32, int row_bytes, int lane)
 {
     static_assert(2 * (R + 1) <= 32, "one lane per address");
     const bool hi = lane > R;
     const int a = p0 - 1 + (hi ? lane - R - 1 + t.hi_r + 1 : lane + t.lo_r);
     const uint32_t mine = (hi ? hi32 : lo32) + (uint32_t)(min(max(a, 0), h) * row_bytes);
+    return QuadRowsLater<R>{mine};
+}
+template <int R>
+__device__ __forceinline__ QuadRows<R> quad_rows(const BoxTaps &t, int p0, int h, uint32_t lo32, uint32_t hi32, int row_bytes, int lane)
+{
+    const QuadRowsLater<R> later = quad_rows_later<R>(t, p0, h, lo32, hi32, row_bytes, lane);
     QuadRows<R> q;
 #pragma unroll
     for (int j = 0; j <= R; ++j) {
-        q.lo[j] = __shfl_sync(0xffffffffu, mine, j);
-        q.hi[j] = __shfl_sync(0xffffffffu, mine, R + 1 + j);
+        q.lo_at[j] = later.lo(j);
+        q.hi_at[j] = later.hi(j);
     }
     return q;
 }
@@ -171,8 +186,8 @@ __device__ __forceinline__ float warp_sum5(const float (&v)[kNumSums], int lane)
 // to the accumulators.
 // The column strips enter the sums weighted by u(j), what the rows of the box make of the input values next to
 // tap row j: sum_i x_i (row combination of e) = sum_j e(j) (w_a x_(j+1) + w_b x_j).
-template <int R, bool NEED_PARAMS, bool FULL, class Cells>
-__device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const QuadCols &cols, const QuadRows<R> &q, const ColW2 &cw,
+template <int R, bool NEED_PARAMS, bool FULL, class Rows, class Cells>
+__device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const QuadCols &cols, const Rows &q, const ColW2 &cw,
                                                     Cells &&at, float (&sums)[kNumSums], int rows)
 {
     f2_t pd[kStrip];
@@ -190,7 +205,7 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
         const f2_t wa = pack2(-t.f_lo_r, 1.0f - t.f_hi_r), wb = pack2(t.f_lo_r - 1.0f, t.f_hi_r);
         f2_t topbot = pack2(0.f, 0.f), left = topbot, right = topbot, out2 = topbot;
         f2_t el[kStrip], eh[kStrip], xx[kStrip];
-        quad_pair_e(cols, q.lo[0], q.hi[0], cw, pd, el, eh);
+        quad_pair_e(cols, q.lo(0), q.hi(0), cw, pd, el, eh);
         float4 e = at.first();
         xx[0] = pack2(e.x, e.x); xx[1] = pack2(e.y, e.y); xx[2] = pack2(e.z, e.z); xx[3] = pack2(e.w, e.w);
 #pragma unroll
@@ -205,7 +220,7 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
                 f2_t cd[kStrip], xn[kStrip], dd[kStrip];
                 const f2_t x01 = pack2(e.x, e.y), x23 = pack2(e.z, e.w);
                 at.fetch(i);
-                quad_pair_e(cols, q.lo[i + 1], q.hi[i + 1], cw, cd, el, eh);
+                quad_pair_e(cols, q.lo(i + 1), q.hi(i + 1), cw, cd, el, eh);
                 const float4 below = at.next();
                 if (i + 1 < R) {
                     e = below;
@@ -237,14 +252,14 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
         unpack2(left, a, b); sums[3] = a + b;
         unpack2(right, a, b); sums[4] = a + b;
     } else {
-        quad_pair(cols, q.lo[0], q.hi[0], cw, pd);
+        quad_pair(cols, q.lo(0), q.hi(0), cw, pd);
 #pragma unroll
         for (int i = 0; i < R; ++i) {
             if (FULL || i < rows) {
                 f2_t cd[kStrip];
                 float g[kStrip];
                 at.fetch(i);
-                quad_pair(cols, q.lo[i + 1], q.hi[i + 1], cw, cd);
+                quad_pair(cols, q.lo(i + 1), q.hi(i + 1), cw, cd);
                 at.next();
 #pragma unroll
                 for (int m = 0; m < kStrip; ++m) {

@@ -345,12 +345,12 @@ forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
             Rows8 skip;
             if (FUSED && res) rows8_load<float, FAST, true>(skip, res, w, q0, FAST ? kTileRows : p_end - p0, lane);
             const QuadRows<kTileRows> r = quad_rows<kTileRows>(t, p0, h, s.image, s.image, Q::kRow, lane);
-            if (p0 == p_begin) quad_pair(cols, r.lo[0], r.hi[0], cw, prev);
+            if (p0 == p_begin) quad_pair(cols, r.lo(0), r.hi(0), cw, prev);
 #pragma unroll
             for (int i = 0; i < kTileRows; ++i) {
                 if (FAST || p0 + i < p_end) {
                     f2_t cur[kStrip];
-                    quad_pair(cols, r.lo[i + 1], r.hi[i + 1], cw, cur);
+                    quad_pair(cols, r.lo(i + 1), r.hi(i + 1), cw, cur);
                     float v[kStrip];
                     quad_forward_row(prev, cur, t.scale, sfl, sfh, v);
 #pragma unroll
@@ -488,6 +488,128 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
     if (COUNTED) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
 }
 
+// Backward of planes of 17 to 32 tiles, two column tiles wide: two tiles a warp, their input values and grad-input accumulators in
+// the whole of tensor memory; a CTA has its SM to itself.  Aligned planes (FAST in the kernel above).  The 32 x 32-tile kernel,
+// which had these planes before, keeps accumulators in registers and reads the input plane again from L2 for every
+// filter, and its tap loads conflict where rows are clamped at the plane's border.
+// (8,16,4,128,256): 79 -> 52 us, bfloat16 (10,16,4,80,240): 115 -> 65.  Every warp has two whole tiles; asked whether it has, the compiler
+// ran out of registers (456 bytes of spills, 64 us).
+template <typename IO, bool NEED_PARAMS, bool COUNTED>
+__global__ void __launch_bounds__(512)
+backward_quad_pair_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_output, BoxParams bp, IO *__restrict__ grad_input,
+                          float *__restrict__ partials, int N, int C, int F, int h, int w, int row_tiles, bool normalize, bool exact, bool write_gin, Finish fin)
+{
+    constexpr int CT = 2, T = 2;
+    using Q = QuadImage<CT>;
+    extern __shared__ float4 smem4[];
+    grid_dependency_release();
+    const int lane = threadIdx.x & 31, warp = uniform(threadIdx.x >> 5), nwarps = blockDim.x >> 5;
+    const int64_t nc = blockIdx.x;
+    const int c = blockIdx.x % C, n = blockIdx.x / C;
+    const int npix = h * w, cells = quad_cells(w), ntiles = row_tiles * CT;
+    const QuadSmem s = quad_smem(smem4, h, CT, ntiles, nwarps);
+    float *sTaps = reinterpret_cast<float *>(reinterpret_cast<char *>(smem4) + (s.taps - s.image));
+    float *red = sTaps + F * kTapWords;                                                        // [F][warps][5]
+    __shared__ uint32_t tmem_base;
+    const IO *gbase = grad_output + nc * F * (int64_t)npix;
+    auto tile_of = [&](int k) { return quad_tile<CT>(warp + k * nwarps, lane, h); };      // (all of them exist, with all their rows)
+
+    if (threadIdx.x == 0) bulk_prefetch_l2(gbase, (uint32_t)npix * (uint32_t)sizeof(IO));
+    quad_zero_padding<CT>(s.image, h);
+    grid_dependency_wait();
+    __syncwarp();
+    if (warp == nwarps - 1) tmem_alloc(&tmem_base, tmem_columns<T>(nwarps));
+    if ((int)threadIdx.x < F) {
+        const Box box = load_box(bp, c * F + threadIdx.x);
+        store_taps(sTaps + threadIdx.x * kTapWords, taps_mirrored(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
+    }
+    __syncthreads();
+    tmem_acquire();
+#pragma unroll 1
+    for (int k = 0; k < T; ++k) {
+        const QuadTile t = tile_of(k);
+        TmemRows<1, T> kept(tmem_base, warp, k);
+        const IO *xrow = x + nc * npix + t.p0 * w;
+        Rows8 g;
+        if (NEED_PARAMS) rows8_load<IO, true>(g, xrow, w, t.c, kTileRows, lane);
+#pragma unroll
+        for (int i = 0; i < kTileRows; ++i)
+            kept.init(i, NEED_PARAMS ? rows8_get<IO, true>(g, xrow, w, t.c, lane, i) : make_float4(0.f, 0.f, 0.f, 0.f));
+        kept.sync();
+    }
+#pragma unroll 1
+    for (int f = 0; f < F; ++f) {
+        {
+            QuadTile tile[T];
+            QuadBlock v[T];
+            float carry[T][kTileRows];
+#pragma unroll
+            for (int k = 0; k < T; ++k) {
+                tile[k] = tile_of(k);
+                quad_load_tile<IO, true, true>(v[k], tile[k], gbase + f * (int64_t)npix, w, lane);
+            }
+            if (threadIdx.x == 0 && f + 1 < F) bulk_prefetch_l2(gbase + (f + 1) * (int64_t)npix, (uint32_t)npix * (uint32_t)sizeof(IO));
+#pragma unroll
+            for (int k = 0; k < T; ++k)
+                quad_scan<CT>(v[k], carry[k], tile[k], s, warp, lane);
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < T; ++k)
+                quad_publish<CT>(v[k], carry[k], tile[k], s, lane);
+            __syncthreads();      // (also: every gather of the previous filter is done)
+#pragma unroll
+            for (int k = 0; k < T; ++k)
+                quad_store<CT, true>(v[k], tile[k], s, w, lane);
+        }
+        __syncthreads();
+        const BoxTaps t = load_taps_uniform(sTaps + f * kTapWords);
+        float all[kNumSums] = {0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+        for (int k = 0; k < T; ++k) {
+            const QuadTile tile = tile_of(k);
+            TmemRows<1, T> kept(tmem_base, warp, k);
+            float sums[kNumSums] = {0.f, 0.f, 0.f, 0.f, 0.f};
+            quad_backward_strip<kTileRows, NEED_PARAMS, true>(t, quad_cols(t, tile.c >> 2, cells, Q::kCells),
+                                                              quad_rows_later<kTileRows>(t, tile.p0, h, s.image, s.image, Q::kRow, lane), col_weights(t), kept,
+                                                              sums, kTileRows);
+            kept.sync();
+#pragma unroll
+            for (int j = 0; j < kNumSums; ++j) all[j] += sums[j];
+        }
+        if (NEED_PARAMS) {
+            const float sum = warp_sum5(all, lane);
+            const int slot = sum5_slot(lane);
+            if (slot >= 0) red[(f * nwarps + warp) * kNumSums + slot] = sum;
+        }
+    }
+    if (NEED_PARAMS) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < F * kNumSums; i += blockDim.x) {
+            const int f = i / kNumSums, j = i - f * kNumSums;
+            float sum = 0.0f;
+            for (int k = 0; k < nwarps; ++k) sum += red[(f * nwarps + k) * kNumSums + j];
+            partials[((int64_t)(c * F + f) * N + n) * kNumSums + j] = sum;
+        }
+    }
+    if (write_gin) {
+#pragma unroll 1
+        for (int k = 0; k < T; ++k) {
+            const QuadTile tile = tile_of(k);
+            TmemRows<1, T> kept(tmem_base, warp, k);
+            IO *row = grad_input + nc * npix + tile.p0 * w;
+#pragma unroll
+            for (int i = 0; i < kTileRows; ++i, row += w) {
+                const float4 g = kept.grad_input(i);
+                if (tile.c < w) Io<IO>::store4(row + tile.c, g.x, g.y, g.z, g.w);
+            }
+        }
+    }
+    tmem_release();
+    __syncthreads();
+    if (warp == 0) tmem_free(tmem_base, tmem_columns<T>(nwarps));
+    if (COUNTED) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
+}
+
 inline int quad_row_tiles(int h) { return (h + kTileRows - 1) / kTileRows; }
 inline int quad_col_tiles(int w) { return (w + 127) / 128; }
 inline size_t quad_forward_smem(int F, int h, int w)
@@ -553,6 +675,17 @@ inline bool quad_fits_backward(int F, int h, int w)
 {
     return w >= kQuadMinWidth && w <= 256 && F <= kMaxFilters && quad_row_tiles(h) * quad_col_tiles(w) <= kQuadMaxWarps &&
            quad_backward_smem(F, h, w) <= kQuadMaxSmem;
+}
+
+// Planes of 17 to 32 tiles with two of them a warp: aligned ones two column tiles wide.  In 16 bits, whose 32 x 32-tile kernel
+// leaves room for a second CTA, where these tiles waste little more than those ((10,16,4,96,160), 24 tiles for 15: 67 us
+// against 58; (10,16,4,80,240), 20 for 24: 65 against 115).  Float: (24,16,4,96,160): 122, 123; (55,16,4,128,156): 278, 370;
+// (30,16,2,88,188): 92, 129; (40,16,4,104,224): 232, 345.
+inline bool quad_pair_suits_backward(int F, int h, int w, bool wide)
+{
+    const int tiles = quad_row_tiles(h) * quad_col_tiles(w), square = ((h + 31) / 32) * ((w + 31) / 32);
+    return w > 128 && w <= 256 && w % 4 == 0 && h % kTileRows == 0 && F <= kMaxFilters && tiles > kQuadMaxWarps && tiles <= 2 * kQuadMaxWarps &&
+           (wide || 2 * tiles <= 3 * square) && quad_backward_smem(F, h, w) <= kQuadMaxSmem;
 }
 
 template <typename IO>
@@ -647,6 +780,34 @@ int launch_backward_quad_t(const IO *x, const float *x_integ, const IO *grad_out
     if (st != BC_OK || !need_params || fin.total) return st;
     return launch_finish_param_grads<float>(partials, bp, C * F, N, normalize, exact, rep_h, rep_w, need_mask, grad_params, s,
                                             grad_params_kind);
+}
+
+template <typename IO>
+int launch_backward_quad_pair_t(const IO *x, const IO *grad_output, const BoxParams &bp, float rep_h, float rep_w, int N, int C, int F, int h, int w,
+                                bool normalize, bool exact, int need_mask, IO *grad_input, void *grad_params, int grad_params_kind, float *partials,
+                                cudaStream_t s)
+{
+    const int row_tiles = quad_row_tiles(h);
+    const int64_t planes = (int64_t)N * C;
+    if (planes > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
+    const bool need_params = (need_mask & (BC_NEED_ALL & ~BC_NEED_INPUT)) != 0, write_gin = (need_mask & BC_NEED_INPUT) != 0;
+    const Finish fin = finish_here(bp, need_params, planes, planes * F * h * w, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w, s);
+    void (*kern)(const IO *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, int, bool, bool, bool, Finish) =
+        !need_params ? backward_quad_pair_kernel<IO, false, false>
+        : fin.total  ? backward_quad_pair_kernel<IO, true, true>
+                     : backward_quad_pair_kernel<IO, true, false>;
+    int st = raise_smem_limit(reinterpret_cast<const void *>(kern), (int)kQuadMaxSmem);
+    if (st != BC_OK) return st;
+    {
+        LaunchScope scope(KID_BACKWARD_QUAD, s);
+        // (row_tiles warps: two column tiles, two tiles a warp)
+        if (cudaError_t e = launch_overlapped(kern, (unsigned)planes, row_tiles * 32, quad_backward_smem(F, h, w), s, x, grad_output, bp, grad_input, partials,
+                                              N, C, F, h, w, row_tiles, normalize, exact, write_gin, fin))
+            return cuda_failed(e, "backward_quad_pair");
+    }
+    st = check_launch("backward_quad_pair");
+    if (st != BC_OK || !need_params || fin.total) return st;
+    return launch_finish_param_grads<float>(partials, bp, C * F, N, normalize, exact, rep_h, rep_w, need_mask, grad_params, s, grad_params_kind);
 }
 
 }  // namespace

@@ -124,12 +124,12 @@ forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int 
             const float *res = FUSED && fu.residual ? fu.residual + off - q0 : nullptr;
             if (FUSED && res) rows8_load<float, VEC, true>(skip, res, w, q0, mine, lane);
             f2_t prev[kStrip];
-            quad_pair(cols, q.lo[0], q.hi[0], cw, prev);
+            quad_pair(cols, q.lo(0), q.hi(0), cw, prev);
 #pragma unroll
             for (int i = 0; i < kStripRows; ++i) {
                 if (i < mine) {
                     f2_t cur[kStrip];
-                    quad_pair(cols, q.lo[i + 1], q.hi[i + 1], cw, cur);
+                    quad_pair(cols, q.lo(i + 1), q.hi(i + 1), cw, cur);
                     float v[kStrip];
                     quad_forward_row(prev, cur, t.scale, sfl, sfh, v);
 #pragma unroll
