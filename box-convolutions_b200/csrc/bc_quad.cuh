@@ -202,53 +202,56 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
         return (hi_old - lo_new) + t.f_hi_r * bot + t.f_lo_r * top;
     };
     if (NEED_PARAMS) {
-        const f2_t wa = pack2(-t.f_lo_r, 1.0f - t.f_hi_r), wb = pack2(t.f_lo_r - 1.0f, t.f_hi_r);
-        f2_t topbot = pack2(0.f, 0.f), left = topbot, right = topbot, out2 = topbot;
-        f2_t el[kStrip], eh[kStrip], xx[kStrip];
+        f2_t left = pack2(0.f, 0.f), right = left, out2 = left;
+        float s_top = 0.f, s_bot = 0.f;
+        f2_t el[kStrip], eh[kStrip];
         quad_pair_e(cols, q.lo(0), q.hi(0), cw, pd, el, eh);
         float4 e = at.first();
-        xx[0] = pack2(e.x, e.x); xx[1] = pack2(e.y, e.y); xx[2] = pack2(e.z, e.z); xx[3] = pack2(e.w, e.w);
+        auto weigh = [&](float x, float next) {      // what the rows of the box make of the input values next to a pair of tap rows
+            const float dx = next - x;
+            return pack2(fmaf(-t.f_lo_r, dx, -x), fmaf(-t.f_hi_r, dx, next));
+        };
+        {
+            const float x0[kStrip] = {e.x, e.y, e.z, e.w};
 #pragma unroll
-        for (int m = 0; m < kStrip; ++m) {
-            const f2_t u = mul2(wa, xx[m]);
-            left = fma2(u, el[m], left);
-            right = fma2(u, eh[m], right);
+            for (int m = 0; m < kStrip; ++m) {
+                const f2_t u = weigh(0.f, x0[m]);
+                left = fma2(u, el[m], left);
+                right = fma2(u, eh[m], right);
+            }
         }
 #pragma unroll
         for (int i = 0; i < R; ++i) {
             if (FULL || i < rows) {
-                f2_t cd[kStrip], xn[kStrip], dd[kStrip];
-                const f2_t x01 = pack2(e.x, e.y), x23 = pack2(e.z, e.w);
+                f2_t cd[kStrip], dd[kStrip];
                 at.fetch(i);
                 quad_pair_e(cols, q.lo(i + 1), q.hi(i + 1), cw, cd, el, eh);
                 const float4 below = at.next();
-                if (i + 1 < R) {
-                    e = below;
-                    xn[0] = pack2(e.x, e.x); xn[1] = pack2(e.y, e.y); xn[2] = pack2(e.z, e.z); xn[3] = pack2(e.w, e.w);
-                }
+                const float x0[kStrip] = {e.x, e.y, e.z, e.w};
+                const float x1[kStrip] = {i + 1 < R ? below.x : 0.f, i + 1 < R ? below.y : 0.f, i + 1 < R ? below.z : 0.f, i + 1 < R ? below.w : 0.f};
 #pragma unroll
                 for (int m = 0; m < kStrip; ++m) {
-                    f2_t u = mul2(wb, xx[m]);
-                    if (i + 1 < R) u = fma2(wa, xn[m], u);
+                    const f2_t u = weigh(x0[m], x1[m]);
                     left = fma2(u, el[m], left);
                     right = fma2(u, eh[m], right);
                     dd[m] = sub2(cd[m], pd[m]);
-                    topbot = fma2(xx[m], dd[m], topbot);
+                    float top, bot;
+                    unpack2(dd[m], top, bot);
+                    s_top = fmaf(x0[m], top, s_top);
+                    s_bot = fmaf(x0[m], bot, s_bot);
                 }
                 const f2_t g01 = pack2(gather(cd[0], pd[0], dd[0]), gather(cd[1], pd[1], dd[1]));
                 const f2_t g23 = pack2(gather(cd[2], pd[2], dd[2]), gather(cd[3], pd[3], dd[3]));
-                out2 = fma2(x01, g01, fma2(x23, g23, out2));
+                out2 = fma2(pack2(e.x, e.y), g01, fma2(pack2(e.z, e.w), g23, out2));
                 at.add(i, g01, g23, scale);
 #pragma unroll
-                for (int m = 0; m < kStrip; ++m) {
-                    pd[m] = cd[m];
-                    if (i + 1 < R) xx[m] = xn[m];
-                }
+                for (int m = 0; m < kStrip; ++m) pd[m] = cd[m];
+                if (i + 1 < R) e = below;
             }
         }
         float a, b;
         unpack2(out2, a, b); sums[0] = a + b;
-        unpack2(topbot, sums[1], sums[2]);
+        sums[1] = s_top; sums[2] = s_bot;
         unpack2(left, a, b); sums[3] = a + b;
         unpack2(right, a, b); sums[4] = a + b;
     } else {
