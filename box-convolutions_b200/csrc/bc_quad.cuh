@@ -86,7 +86,7 @@ __device__ __forceinline__ float lds_row(uint32_t row, uint32_t off)
     return v;
 }
 
-// Shared addresses of the tap rows of a strip of R rows: lo[j+1], hi[j+1] for the rows p0+j+lo_r and p0+j+hi_r+1,
+// Shared addresses of the tap rows of a strip of R rows: lo(j+1), hi(j+1) for the rows p0+j+lo_r and p0+j+hi_r+1,
 // j = -1 .. R-1, clamped to the plane.  Lane k works out the k-th address and hands it to the warp, which
 // costs one shuffle an address instead of the same clamps and multiplications in every lane.
 template <int R>

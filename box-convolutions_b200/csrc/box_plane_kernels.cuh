@@ -1,6 +1,6 @@
 // Shared-memory-resident kernels in tiles of 32 x 32, for planes small enough to keep on chip that are too narrow (64
-// columns) or too large for the quad layout's tiles of 8 x 128, or waste less in these (quad_prefers_forward() in
-// box_quad_plane.cuh).  HBM traffic is the compulsory minimum: the forward
+// columns) or too large for the quad layout's tiles of 8 x 128, or waste less in these (quad_prefers_forward() and
+// quad_pair_suits_backward() in box_quad_plane.cuh).  HBM traffic is the compulsory minimum: the forward
 // reads the input once and writes the output once; the backward reads the input and grad_output
 // once and writes grad_input once.  No integral image ever goes to global memory.
 //
