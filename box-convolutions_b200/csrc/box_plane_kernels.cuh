@@ -857,13 +857,13 @@ int launch_backward_plane_t(const IO *x, const float *x_integ, const IO *grad_ou
                             int C, int F, int h, int w, bool normalize, bool exact, int need_mask, IO *grad_input,
                             void *grad_params, int grad_params_kind, float *partials, cudaStream_t s)
 {
-    if (quad_fits_backward(F, h, w))
-        return launch_backward_quad_t<IO>(x, x_integ, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
-                                          grad_params, grad_params_kind, partials, s);
-    if (x && quad_pair_suits_backward(F, h, w, IsFloat<IO>::value) && aligned_to(x, Io<IO>::kVecBytes) && aligned_to(grad_output, 16) &&
+    if (x && quad_pair_suits_backward((int64_t)N * C, F, h, w, IsFloat<IO>::value) && aligned_to(x, Io<IO>::kVecBytes) && aligned_to(grad_output, 16) &&
         (!(need_mask & BC_NEED_INPUT) || aligned_to(grad_input, Io<IO>::kVecBytes)))
         return launch_backward_quad_pair_t<IO>(x, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input, grad_params,
                                                grad_params_kind, partials, s);
+    if (quad_fits_backward(F, h, w))
+        return launch_backward_quad_t<IO>(x, x_integ, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
+                                          grad_params, grad_params_kind, partials, s);
     const int64_t planes = (int64_t)N * C;
     if (planes > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
     const bool need_params = (need_mask & (BC_NEED_ALL & ~BC_NEED_INPUT)) != 0;

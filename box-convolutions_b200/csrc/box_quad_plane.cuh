@@ -488,18 +488,18 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
     if (COUNTED) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
 }
 
-// Backward of planes of 17 to 32 tiles, two column tiles wide: two tiles a warp, their input values and grad-input accumulators in
-// the whole of tensor memory; a CTA has its SM to itself.  Aligned planes (FAST in the kernel above).  The 32 x 32-tile kernel,
-// which had these planes before, keeps accumulators in registers and reads the input plane again from L2 for every
+// Backward of larger aligned planes (FAST in the kernel above), two tiles a warp: 17 to 32 tiles, two column tiles wide, take the
+// whole of tensor memory for their input values and grad-input accumulators, and the SM; 13 to 16 tiles half of either.
+// The 32 x 32-tile kernel, which had the former before, keeps accumulators in registers and reads the input plane again from L2 for every
 // filter, and its tap loads conflict where rows are clamped at the plane's border.
 // (8,16,4,128,256): 79 -> 52 us, bfloat16 (10,16,4,80,240): 115 -> 65.  Every warp has two whole tiles; asked whether it has, the compiler
 // ran out of registers (456 bytes of spills, 64 us).
-template <typename IO, bool NEED_PARAMS, bool COUNTED>
-__global__ void __launch_bounds__(512)
+template <typename IO, int CT, bool NEED_PARAMS, bool COUNTED, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 2 : 1)
 backward_quad_pair_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_output, BoxParams bp, IO *__restrict__ grad_input,
                           float *__restrict__ partials, int N, int C, int F, int h, int w, int row_tiles, bool normalize, bool exact, bool write_gin, Finish fin)
 {
-    constexpr int CT = 2, T = 2;
+    constexpr int T = 2;
     using Q = QuadImage<CT>;
     extern __shared__ float4 smem4[];
     grid_dependency_release();
@@ -552,7 +552,7 @@ backward_quad_pair_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_
 #pragma unroll
             for (int k = 0; k < T; ++k)
                 quad_scan<CT>(v[k], carry[k], tile[k], s, warp, lane);
-            __syncthreads();
+            if (CT > 1) __syncthreads();
 #pragma unroll
             for (int k = 0; k < T; ++k)
                 quad_publish<CT>(v[k], carry[k], tile[k], s, lane);
@@ -677,15 +677,19 @@ inline bool quad_fits_backward(int F, int h, int w)
            quad_backward_smem(F, h, w) <= kQuadMaxSmem;
 }
 
-// Planes of 17 to 32 tiles with two of them a warp: aligned ones two column tiles wide.  In 16 bits, whose 32 x 32-tile kernel
-// leaves room for a second CTA, where these tiles waste little more than those ((10,16,4,96,160), 24 tiles for 15: 67 us
-// against 58; (10,16,4,80,240), 20 for 24: 65 against 115).  Float: (24,16,4,96,160): 122, 123; (55,16,4,128,156): 278, 370;
-// (30,16,2,88,188): 92, 129; (40,16,4,104,224): 232, 345.
-inline bool quad_pair_suits_backward(int F, int h, int w, bool wide)
+// Aligned planes with two tiles a warp.  17 to 32 tiles, two column tiles wide: in 16 bits, whose 32 x 32-tile kernel leaves
+// room for a second CTA, where these tiles waste little more than those ((10,16,4,96,160), 24 tiles for 15: 67 us against
+// 58; (10,16,4,80,240), 20 for 24: 65 against 115); float always ((24,16,4,96,160): 122, 123; (55,16,4,128,156): 278, 370;
+// (30,16,2,88,188): 92, 129; (40,16,4,104,224): 232, 345).  13 to 16 tiles, which as one tile a warp have an SM to themselves:
+// two CTAs of half the warps, if there are planes for two ((16,32,4,128,128): 96, 117; (16,32,4,64,256): 99, 115;
+// (64,32,4,112,96): 265, 334; 144 planes of 128 x 120: 28.7, 26.6).  Not of 9 to 12 tiles, two CTAs an SM either way
+// ((16,32,4,96,128): 73, 69; (16,32,4,40,248): 71, 64).
+inline bool quad_pair_suits_backward(int64_t planes, int F, int h, int w, bool wide)
 {
     const int tiles = quad_row_tiles(h) * quad_col_tiles(w), square = ((h + 31) / 32) * ((w + 31) / 32);
-    return w > 128 && w <= 256 && w % 4 == 0 && h % kTileRows == 0 && F <= kMaxFilters && tiles > kQuadMaxWarps && tiles <= 2 * kQuadMaxWarps &&
-           (wide || 2 * tiles <= 3 * square) && quad_backward_smem(F, h, w) <= kQuadMaxSmem;
+    if (w < kQuadMinWidth || w > 256 || w % 4 || h % kTileRows || F > kMaxFilters || tiles % 2 || quad_backward_smem(F, h, w) > kQuadMaxSmem) return false;
+    if (tiles <= kQuadMaxWarps) return tiles > 12 && planes > 148;
+    return tiles <= 2 * kQuadMaxWarps && (wide || 2 * tiles <= 3 * square);
 }
 
 template <typename IO>
@@ -792,16 +796,22 @@ int launch_backward_quad_pair_t(const IO *x, const IO *grad_output, const BoxPar
     if (planes > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
     const bool need_params = (need_mask & (BC_NEED_ALL & ~BC_NEED_INPUT)) != 0, write_gin = (need_mask & BC_NEED_INPUT) != 0;
     const Finish fin = finish_here(bp, need_params, planes, planes * F * h * w, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w, s);
-    void (*kern)(const IO *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, int, bool, bool, bool, Finish) =
-        !need_params ? backward_quad_pair_kernel<IO, false, false>
-        : fin.total  ? backward_quad_pair_kernel<IO, true, true>
-                     : backward_quad_pair_kernel<IO, true, false>;
+    void (*kern)(const IO *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, int, bool, bool, bool, Finish);
+    auto pick = [&](auto ct, auto threads) {
+        constexpr int CT = decltype(ct)::value, T = decltype(threads)::value;
+        kern = !need_params ? backward_quad_pair_kernel<IO, CT, false, false, T>
+               : fin.total  ? backward_quad_pair_kernel<IO, CT, true, true, T>
+                            : backward_quad_pair_kernel<IO, CT, true, false, T>;
+    };
+    const int warps = row_tiles * quad_col_tiles(w) / 2;
+    if (quad_col_tiles(w) == 1) pick(Index<1>{}, Index<256>{});
+    else if (warps <= 8) pick(Index<2>{}, Index<256>{});
+    else pick(Index<2>{}, Index<512>{});
     int st = raise_smem_limit(reinterpret_cast<const void *>(kern), (int)kQuadMaxSmem);
     if (st != BC_OK) return st;
     {
         LaunchScope scope(KID_BACKWARD_QUAD, s);
-        // (row_tiles warps: two column tiles, two tiles a warp)
-        if (cudaError_t e = launch_overlapped(kern, (unsigned)planes, row_tiles * 32, quad_backward_smem(F, h, w), s, x, grad_output, bp, grad_input, partials,
+        if (cudaError_t e = launch_overlapped(kern, (unsigned)planes, warps * 32, quad_backward_smem(F, h, w), s, x, grad_output, bp, grad_input, partials,
                                               N, C, F, h, w, row_tiles, normalize, exact, write_gin, fin))
             return cuda_failed(e, "backward_quad_pair");
     }
