@@ -15,7 +15,7 @@ constexpr int kTmemColumns = 64;      // per warp
 
 // Columns of a CTA of at most 16 warps with T tiles each: warps w and w + 4 share lanes.  A power of two.
 template <int T = 1>
-__device__ __forceinline__ uint32_t tmem_columns(int nwarps) { return (nwarps > 8 ? 256u : nwarps > 4 ? 128u : 64u) * T; }
+__host__ __device__ __forceinline__ uint32_t tmem_columns(int nwarps) { return (nwarps > 8 ? 256u : nwarps > 4 ? 128u : 64u) * T; }
 
 // One whole warp allocates and frees.  An allocation waits for columns that other CTAs of the SM hold, so a CTA
 // allocates only behind grid_dependency_wait(): one that still waits for the kernel in front must not hold what

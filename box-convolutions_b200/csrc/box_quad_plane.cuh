@@ -488,8 +488,8 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
     if (COUNTED) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
 }
 
-// Backward of larger aligned planes (FAST in the kernel above), two tiles a warp: 17 to 32 tiles, two column tiles wide, take the
-// whole of tensor memory for their input values and grad-input accumulators, and the SM; 13 to 16 tiles half of either.
+// Backward of larger aligned planes (FAST in the kernel above), two tiles a warp: 18 to 32 tiles, two column tiles wide, take the
+// whole of tensor memory for their input values and grad-input accumulators, and the SM; 14 and 16 tiles half of either.
 // The 32 x 32-tile kernel, which had the former before, keeps accumulators in registers and reads the input plane again from L2 for every
 // filter, and its tap loads conflict where rows are clamped at the plane's border.
 // (8,16,4,128,256): 79 -> 52 us, bfloat16 (10,16,4,80,240): 115 -> 65.  Every warp has two whole tiles; asked whether it has, the compiler
@@ -677,19 +677,27 @@ inline bool quad_fits_backward(int F, int h, int w)
            quad_backward_smem(F, h, w) <= kQuadMaxSmem;
 }
 
-// Aligned planes with two tiles a warp.  17 to 32 tiles, two column tiles wide: in 16 bits, whose 32 x 32-tile kernel leaves
+// Threads at most of the pair kernel that is launched for a CTA of `warps` warps; 0: there is none.
+inline int quad_pair_max_threads(int col_tiles, int warps)
+{
+    if (warps <= 8) return 256;
+    return col_tiles == 2 && warps <= kQuadMaxWarps ? 512 : 0;
+}
+
+// Aligned planes with two tiles a warp, so with an even number of tiles.  18 to 32 tiles in two columns (one column of them has
+// no kernel of more than eight warps: 32 x 32 tiles): in 16 bits, whose 32 x 32-tile kernel leaves
 // room for a second CTA, where these tiles waste little more than those ((10,16,4,96,160), 24 tiles for 15: 67 us against
 // 58; (10,16,4,80,240), 20 for 24: 65 against 115); float always ((24,16,4,96,160): 122, 123; (55,16,4,128,156): 278, 370;
-// (30,16,2,88,188): 92, 129; (40,16,4,104,224): 232, 345).  13 to 16 tiles, which as one tile a warp have an SM to themselves:
+// (30,16,2,88,188): 92, 129; (40,16,4,104,224): 232, 345).  14 and 16 tiles, which as one tile a warp have an SM to themselves:
 // two CTAs of half the warps, if there are planes for two ((16,32,4,128,128): 96, 117; (16,32,4,64,256): 99, 115;
-// (64,32,4,112,96): 265, 334; 144 planes of 128 x 120: 28.7, 26.6).  Not of 9 to 12 tiles, two CTAs an SM either way
+// (64,32,4,112,96): 265, 334; 144 planes of 128 x 120: 28.7, 26.6).  Not of 10 and 12 tiles, two CTAs an SM either way
 // ((16,32,4,96,128): 73, 69; (16,32,4,40,248): 71, 64).
 inline bool quad_pair_suits_backward(int64_t planes, int F, int h, int w, bool wide)
 {
-    const int tiles = quad_row_tiles(h) * quad_col_tiles(w), square = ((h + 31) / 32) * ((w + 31) / 32);
+    const int col_tiles = quad_col_tiles(w), tiles = quad_row_tiles(h) * col_tiles, square = ((h + 31) / 32) * ((w + 31) / 32);
     if (w < kQuadMinWidth || w > 256 || w % 4 || h % kTileRows || F > kMaxFilters || tiles % 2 || quad_backward_smem(F, h, w) > kQuadMaxSmem) return false;
     if (tiles <= kQuadMaxWarps) return tiles > 12 && planes > 148;
-    return tiles <= 2 * kQuadMaxWarps && (wide || 2 * tiles <= 3 * square);
+    return col_tiles == 2 && tiles <= 2 * kQuadMaxWarps && (wide || 2 * tiles <= 3 * square);
 }
 
 template <typename IO>
@@ -803,10 +811,11 @@ int launch_backward_quad_pair_t(const IO *x, const IO *grad_output, const BoxPar
                : fin.total  ? backward_quad_pair_kernel<IO, CT, true, true, T>
                             : backward_quad_pair_kernel<IO, CT, true, false, T>;
     };
-    const int warps = row_tiles * quad_col_tiles(w) / 2;
-    if (quad_col_tiles(w) == 1) pick(Index<1>{}, Index<256>{});
-    else if (warps <= 8) pick(Index<2>{}, Index<256>{});
-    else pick(Index<2>{}, Index<512>{});
+    const int col_tiles = quad_col_tiles(w), warps = row_tiles * col_tiles / 2, bound = quad_pair_max_threads(col_tiles, warps);
+    if (!bound) return BC_ERR_UNSUPPORTED;
+    if (bound == 512) pick(Index<2>{}, Index<512>{});
+    else if (col_tiles == 2) pick(Index<2>{}, Index<256>{});
+    else pick(Index<1>{}, Index<256>{});
     int st = raise_smem_limit(reinterpret_cast<const void *>(kern), (int)kQuadMaxSmem);
     if (st != BC_OK) return st;
     {

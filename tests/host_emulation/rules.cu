@@ -1,0 +1,18 @@
+// The dispatch rules of the whole-plane kernels and the launches they lead to, for the unit tests: host code only, compiled by
+// tests/test_dispatch_rules_host.py.
+#include "box_plane_kernels.cuh"
+
+namespace bc {
+
+// Threads of the pair backward's launch, the bound of the kernel that is launched and the tensor-memory columns of a CTA;
+// 0 where the rule sends the plane elsewhere.
+extern "C" int rule_pair_backward(int64_t planes, int F, int h, int w, int wide, int *bound, int *columns)
+{
+    if (!quad_pair_suits_backward(planes, F, h, w, wide != 0)) return 0;
+    const int warps = quad_row_tiles(h) * quad_col_tiles(w) / 2;
+    *bound = quad_pair_max_threads(quad_col_tiles(w), warps);
+    *columns = (int)tmem_columns<2>(warps);
+    return warps * 32;
+}
+
+}  // namespace bc

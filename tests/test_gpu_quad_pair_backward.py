@@ -1,6 +1,7 @@
-"""Backward of aligned planes of 13 to 32 tiles of 8 x 128 with two tiles a warp: the smallest and largest of them, numbers of planes
-at which those of up to 16 tiles begin, widths that leave the second column tile nearly empty or fill it, every subset of gradients, 16-bit tensors, and an address that no
-vector access fits, which another kernel serves; against the float64 kernels.
+"""Backward of aligned planes of 14 to 32 tiles of 8 x 128 with two tiles a warp: the smallest and largest of them, numbers of planes
+at which those of up to 16 tiles begin, widths that leave the second column tile nearly empty or fill it, every subset of gradients,
+16-bit tensors, and the planes beside them that other kernels serve: odd numbers of tiles, more than 16 of one column, and an
+address that no vector access fits; against the float64 kernels.
 
 Tolerances as in the parity tests: grad-input 1e-4 and parameter gradients 1e-3 of the largest magnitude (the four together: one
 of them can come out near zero by accident); 16-bit results are rounded once more, by at most 2^-8 (bfloat16) or 2^-11
@@ -44,7 +45,10 @@ def _grads(m, x, g):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("exact,normalize", [(True, True), (False, True), (True, False)])
 @pytest.mark.parametrize("shape", [(1, 2, 2, 72, 132), (2, 3, 1, 72, 256), (3, 2, 3, 80, 200), (1, 2, 4, 128, 256), (2, 1, 2, 128, 228), (1, 150, 2, 72, 160), (1, 148, 2, 112, 68), (1, 149, 2, 112, 68),
-                                   (2, 75, 3, 128, 128), (1, 150, 2, 56, 160), (5, 30, 1, 64, 256)])
+                                   (2, 75, 3, 128, 128), (1, 150, 2, 56, 160), (5, 30, 1, 64, 256),
+                                   # one column of 13, 15, 17 and of 18 to 32 tiles
+                                   (1, 150, 2, 104, 128), (2, 75, 1, 120, 96), (2, 3, 2, 136, 128),
+                                   (1, 2, 2, 144, 68), (2, 3, 4, 160, 128), (1, 160, 1, 192, 96), (2, 2, 3, 240, 100), (1, 2, 4, 256, 128)])
 def test_gradients_against_float64(shape, exact, normalize, dtype):
     if dtype == torch.float16 and not normalize:
         pytest.skip("sums that are divided by nothing exceed 65504")
