@@ -46,6 +46,16 @@ using BoxTaps = BoxTapsT<float>;
 
 BC_HD int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
+// A border's whole part as a tap offset.  At 2^30 pixels a border is outside of every plane (sides are below 2^24) and stays
+// there: kernels add pixels and a few rows to offsets before they clamp them to the plane, or ask whether a run of rows lies
+// inside it, and such a sum must not wrap around.
+template <typename T>
+BC_HD int tap_offset(T v)
+{
+    const T far = T(1 << 30);
+    return (int)(v < -far ? -far : (v > far ? far : v));
+}
+
 // Reciprocal of the box area (or of one side), src/box_convolution.cpp:765-793.  In rounded
 // mode the box is first shrunk to whole pixels.
 template <typename T>
@@ -65,10 +75,10 @@ BC_HD BoxTapsT<T> taps_forward(T xmin, T xmax, T ymin, T ymax, bool normalize, b
 {
     BoxTapsT<T> t;
     T v;
-    v = bc_ceil(xmin);  t.lo_r = (int)v;      t.f_lo_r = v - xmin;
-    v = bc_ceil(ymin);  t.lo_c = (int)v;      t.f_lo_c = v - ymin;
-    v = bc_floor(xmax); t.hi_r = (int)v + 1;  t.f_hi_r = xmax - v;
-    v = bc_floor(ymax); t.hi_c = (int)v + 1;  t.f_hi_c = ymax - v;
+    v = bc_ceil(xmin);  t.lo_r = tap_offset(v);      t.f_lo_r = v - xmin;
+    v = bc_ceil(ymin);  t.lo_c = tap_offset(v);      t.f_lo_c = v - ymin;
+    v = bc_floor(xmax); t.hi_r = tap_offset(v) + 1;  t.f_hi_r = xmax - v;
+    v = bc_floor(ymax); t.hi_c = tap_offset(v) + 1;  t.f_hi_c = ymax - v;
     if (!exact) t.f_lo_r = t.f_lo_c = t.f_hi_r = t.f_hi_c = T(0);
     t.scale = normalize ? inv_area(xmin, xmax, ymin, ymax, exact, true, true) : T(1);
     return t;
@@ -81,10 +91,10 @@ BC_HD BoxTapsT<T> taps_mirrored(T xmin, T xmax, T ymin, T ymax, bool normalize, 
 {
     BoxTapsT<T> t;
     T v;
-    v = bc_ceil(-xmax);          t.lo_r = (int)v;  t.f_lo_r = v + xmax;
-    v = bc_ceil(-ymax);          t.lo_c = (int)v;  t.f_lo_c = v + ymax;
-    v = bc_floor(-xmin) + T(1);  t.hi_r = (int)v;  t.f_hi_r = -xmin + T(1) - v;
-    v = bc_floor(-ymin) + T(1);  t.hi_c = (int)v;  t.f_hi_c = -ymin + T(1) - v;
+    v = bc_ceil(-xmax);          t.lo_r = tap_offset(v);  t.f_lo_r = v + xmax;
+    v = bc_ceil(-ymax);          t.lo_c = tap_offset(v);  t.f_lo_c = v + ymax;
+    v = bc_floor(-xmin) + T(1);  t.hi_r = tap_offset(v);  t.f_hi_r = -xmin + T(1) - v;
+    v = bc_floor(-ymin) + T(1);  t.hi_c = tap_offset(v);  t.f_hi_c = -ymin + T(1) - v;
     if (!exact) t.f_lo_r = t.f_lo_c = t.f_hi_r = t.f_hi_c = T(0);
     t.scale = normalize ? inv_area(xmin, xmax, ymin, ymax, exact, true, true) : T(1);
     return t;

@@ -8,6 +8,14 @@
 
 using namespace bc;
 
+// lo_r, hi_r, lo_c, hi_c of a box, and of its mirror image
+extern "C" void emu_taps(float xmin, float xmax, float ymin, float ymax, int exact, int *forward, int *mirrored)
+{
+    const BoxTaps f = taps_forward(xmin, xmax, ymin, ymax, false, exact != 0), m = taps_mirrored(xmin, xmax, ymin, ymax, false, exact != 0);
+    forward[0] = f.lo_r; forward[1] = f.hi_r; forward[2] = f.lo_c; forward[3] = f.hi_c;
+    mirrored[0] = m.lo_r; mirrored[1] = m.hi_r; mirrored[2] = m.lo_c; mirrored[3] = m.hi_c;
+}
+
 extern "C" void emu_forward(const float *integ, const float *xmin, const float *xmax,
                             const float *ymin, const float *ymax, float *out, int N, int C, int F,
                             int h, int w, int normalize, int exact, int rows_per_thread)

@@ -214,3 +214,29 @@ def test_backward_from_two_streams(bc, shape):
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for k in range(2) for a, b in zip(got[k], alone[k]))
     _compare(alone[1], run(1, torch.float64))
+
+
+# Borders that no int holds, the largest finite ones, and (where fractions are dropped) infinite ones give what borders just
+# outside of the plane give, to the last bit: every tap is clamped to the same row or column.  One shape a family of kernels: rows
+# in tensor memory and one tile a warp, two tiles a warp, 8 x 128 tiles, 32 x 32 tiles, slabs, bands, rows too wide for both; float64.
+@pytest.mark.parametrize("far,exact", [(2.0 ** 31, True), (3e38, True), (3e9, False), (float("inf"), False)])
+@pytest.mark.parametrize("shape,dtype", [((1, 80, 4, 64, 128), torch.float32), ((1, 150, 4, 128, 128), torch.bfloat16), ((1, 2, 4, 128, 256), torch.float32),
+                                         ((2, 2, 3, 60, 120), torch.float32), ((1, 3, 2, 40, 50), torch.float32), ((1, 2, 4, 150, 300), torch.float32),
+                                         ((1, 1, 4, 24, 2100), torch.float32), ((1, 1, 40, 30, 40), torch.float32), ((1, 2, 4, 30, 40), torch.float64)])
+def test_far_borders_are_borders_just_outside(bc, shape, dtype, far, exact):
+    N, C, F, h, w = shape
+    gen = torch.Generator("cuda").manual_seed(h + w)
+    x = torch.randn(N, C, h, w, device="cuda", generator=gen, dtype=torch.float32).to(dtype)
+    g = torch.randn(N, C * F, h, w, device="cuda", generator=gen, dtype=torch.float32).to(dtype)
+    lo = torch.tensor([-1, -1, -3.5, -1, 1, -2.25]).repeat(C * F // 6 + 1)[:C * F].view(C, F)      # 1: far away; else pixels
+    hi = torch.tensor([1, 6.75, 1, -1, 1, 4.5]).repeat(C * F // 6 + 1)[:C * F].view(C, F)
+
+    def run(at):
+        side = [torch.where(v.abs() == 1, v * at, v).to(dtype).cuda() for v in (lo, hi)]
+        params = [v.clone().requires_grad_() for v in (side[0], side[1], side[0].flip(1), side[1].flip(1))]
+        xin = x.clone().requires_grad_()
+        out = bc.BoxConvolutionFunction.apply(xin, *params, 1.0, 1.0, False, exact)
+        out.backward(g)
+        return [out.detach(), xin.grad] + [p.grad for p in params]
+    for a, b in zip(run(far), run(2.0 * max(h, w))):
+        assert torch.equal(a, b)

@@ -91,3 +91,37 @@ def test_walk_matches_oracle_random(emu, normalize, exact):
         assert max_rel(gin, ref[0]) < 5e-6, trial
         for k in range(4):
             assert max_rel(gp[k], ref[1 + k]) < 5e-5, (trial, k)
+
+
+# borders that no int holds, the largest finite ones, and (where the fractions are dropped) infinite ones
+FAR = (2.0 ** 31, 3e9, 3e38)
+
+
+@pytest.mark.parametrize("far", FAR + (np.inf,))
+def test_tap_offsets_leave_room_for_a_pixel_on_either_side(emu, far):
+    forward, mirrored = (ctypes.c_int * 4)(), (ctypes.c_int * 4)()
+    sides = 1 << 24      # planes have fewer rows and columns than that
+    for xmin, xmax in ((-far, -far), (-far, far), (far, far), (-3.5, far), (-far, 2.25)):
+        emu.emu_taps(*[ctypes.c_float(v) for v in (xmin, xmax, xmin, xmax)], 0, forward, mirrored)
+        for taps, lo, hi in ((forward, xmin, xmax), (mirrored, -xmax, -xmin)):
+            for got, border in ((taps[0], lo), (taps[1], hi), (taps[2], lo), (taps[3], hi)):
+                assert abs(got) <= 2 ** 31 - 1 - 2 * sides      # (pixel + offset + a few rows stays an int)
+                if abs(border) == far:
+                    assert abs(got) > sides and (got > 0) == (border > 0)
+
+
+@pytest.mark.parametrize("far", FAR)
+def test_far_borders_are_borders_just_outside(emu, far):
+    rng = np.random.default_rng(3)
+    h, w = 21, 34
+    x = rng.standard_normal((1, 1, h, w)).astype(np.float32)
+    go = rng.standard_normal((1, 6, h, w)).astype(np.float32)
+    lo, hi = [-1.0, -1.0, -3.5, -1.0, 1.0, -2.25], [1.0, 6.75, 1.0, -1.0, 1.0, 4.5]      # 1: far away, else pixels
+
+    def params(at):
+        v = [np.array([at * e if abs(e) == 1.0 else e for e in side], np.float32).reshape(1, 6) for side in (lo, hi)]
+        return [v[0], v[1], v[0][:, ::-1], v[1][:, ::-1]]
+    integ = oracle.integral_image(x)
+    assert np.array_equal(emu_forward(emu, integ, params(far), False, True), emu_forward(emu, integ, params(2.0 * w), False, True))
+    for a, b in zip(emu_backward(emu, x, go, params(far), 1.0, 1.0, False, True), emu_backward(emu, x, go, params(2.0 * w), 1.0, 1.0, False, True)):
+        assert np.array_equal(a, b)
