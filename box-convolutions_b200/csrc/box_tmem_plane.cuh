@@ -24,9 +24,18 @@ namespace {
 
 constexpr int kTmemMaxRows = 128;
 
-// Barrier among `threads` threads of the CTA; those that only arrive do not wait.
-__device__ __forceinline__ void unit_barrier(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
-__device__ __forceinline__ void unit_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+// Barrier among `threads` threads of the CTA; those that only arrive do not wait.  The instructions count whole warps and ask for
+// converged ones, and some lanes come from a store that others, past the plane, did not make.
+__device__ __forceinline__ void unit_barrier(int id, int threads)
+{
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void unit_arrive(int id, int threads)
+{
+    __syncwarp();
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
 
 // What the warps of a unit share: integral row a (1 .. h) of the unit is at the columns 4 (a - 1) .. of `rows32`.
 struct TmemUnit {
@@ -259,7 +268,6 @@ forward_tmem_stream_kernel(const IO *__restrict__ x, BoxParams bp, IO *__restric
                 const Box box = load_box(bp, (int)(nc % C) * F + f);
                 store_taps(sTaps[b] + f * kTapWords, taps_forward(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
             }
-            __syncwarp();
             unit_arrive(6 + b, 64 * W);
         }
     } else {
