@@ -207,10 +207,10 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
         f2_t el[kStrip], eh[kStrip];
         quad_pair_e(cols, q.lo(0), q.hi(0), cw, pd, el, eh);
         float4 e = at.first();
-        auto weigh = [&](float x, float next) {      // what the rows of the box make of the input values next to a pair of tap rows
-            const float dx = next - x;
-            return pack2(fmaf(-t.f_lo_r, dx, -x), fmaf(-t.f_hi_r, dx, next));
-        };
+        // What the rows of the box make of the input values next to a pair of tap rows.  (Two products: the values' difference,
+        // an operation less, is infinite for large ones of opposite sign.)
+        const float wb_top = t.f_lo_r - 1.0f, wa_bot = 1.0f - t.f_hi_r;
+        auto weigh = [&](float x, float next) { return pack2(fmaf(-t.f_lo_r, next, wb_top * x), fmaf(wa_bot, next, t.f_hi_r * x)); };
         {
             const float x0[kStrip] = {e.x, e.y, e.z, e.w};
 #pragma unroll

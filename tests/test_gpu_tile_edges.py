@@ -105,6 +105,29 @@ def test_training_edges_against_float64(bc, shape, normalize, exact):
     assert all(g[0, 0] == 0 for g in runs[0][2:])
 
 
+# large values of opposite sign below one another, whose difference no float holds: the gradients of the parameters are finite.  Within
+# a warp's rows, across them, at the plane's top and bottom; 8 x 128 tiles, two of them a warp, slabs, 32 x 32 tiles
+@pytest.mark.parametrize("shape", [(1, 4, 2, 64, 128), (1, 4, 3, 61, 120), (1, 4, 2, 128, 256), (1, 4, 2, 152, 300), (1, 4, 2, 40, 50)])
+def test_large_neighbours_of_opposite_sign(bc, shape):
+    N, C, F, h, w = shape
+    rng = np.random.default_rng(h)
+    gen = torch.Generator("cuda").manual_seed(w)
+    x = torch.randn(N, C, h, w, device="cuda", generator=gen)
+    for c, r in enumerate((0, 3, 7, h - 2)):
+        x[:, c, r, w // 3], x[:, c, r + 1, w // 3] = 2e38, -2e38
+    go = 1e-30 * torch.randn(N, C * F, h, w, device="cuda", generator=gen)
+    boxes = [torch.from_numpy(b).cuda() for b in _boxes(rng, C, F, h, w, True)]
+
+    def grads(dtype):
+        params = [b.clone().to(dtype).detach().requires_grad_() for b in boxes]
+        bc.BoxConvolutionFunction.apply(x.to(dtype), *params, 1.0, 1.0, True, True).backward(go.to(dtype))
+        return torch.stack([p.grad.double() for p in params]).cpu().numpy()
+    # (of the largest of all planes: where a box does not reach the two values, rounding errors of zero are multiplied by them)
+    got, want = grads(torch.float32), grads(torch.float64)
+    assert np.isfinite(got).all()
+    assert max_rel(got, want) < 1e-3
+
+
 # whole planes in 8 x 128 tiles, one and two a row, and slabs: a column of large or infinite values has no effect on
 # boxes that end to the left of it
 @pytest.mark.parametrize("value", [1e8, float("inf"), float("nan")])
