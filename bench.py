@@ -476,6 +476,9 @@ def kernel_algorithmic_bytes(kernel, N, C, F, h, w):
         "backward_slab_kernel": 4 * (F * Ei + 2 * E),
         "forward_quad_kernel": 4 * E * (1 + F),
         "backward_quad_kernel": 4 * E * (F + 2),
+        "forward_tmem_kernel": 4 * E * (1 + F),
+        "forward_tmem_stream_kernel": 4 * E * (1 + F),
+        "backward_quad_pair_kernel": 4 * E * (F + 2),
         "forward_plane_kernel": 4 * E * (1 + F),
         "backward_plane_kernel": 4 * E * (F + 2),
     }.get(kernel)

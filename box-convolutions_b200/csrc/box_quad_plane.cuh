@@ -819,7 +819,7 @@ int launch_backward_quad_pair_t(const IO *x, const IO *grad_output, const BoxPar
     int st = raise_smem_limit(reinterpret_cast<const void *>(kern), (int)kQuadMaxSmem);
     if (st != BC_OK) return st;
     {
-        LaunchScope scope(KID_BACKWARD_QUAD, s);
+        LaunchScope scope(KID_BACKWARD_QUAD_PAIR, s);
         if (cudaError_t e = launch_overlapped(kern, (unsigned)planes, warps * 32, quad_backward_smem(F, h, w), s, x, grad_output, bp, grad_input, partials,
                                               N, C, F, h, w, row_tiles, normalize, exact, write_gin, fin))
             return cuda_failed(e, "backward_quad_pair");

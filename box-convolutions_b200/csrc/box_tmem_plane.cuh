@@ -352,7 +352,7 @@ int launch_forward_tmem_t(const IO *x, const BoxParams &bp, IO *out, int N, int 
     int st = raise_smem_limit(flow ? reinterpret_cast<const void *>(flow) : reinterpret_cast<const void *>(kern), (int)kQuadMaxSmem);
     if (st != BC_OK) return st;
     {
-        LaunchScope scope(KID_FORWARD_QUAD, s);
+        LaunchScope scope(flow ? KID_FORWARD_TMEM_STREAM : KID_FORWARD_TMEM, s);
         const int64_t ctas = std::min<int64_t>(planes, warps == 8 ? 2 * 148 : 148);
         const cudaError_t e = flow ? launch_overlapped(flow, (unsigned)ctas, 2 * warps * 32, tmem_stream_smem(h, w), s, x, bp, out, (int)planes, C, F, h, w,
                                                        row_tiles, columns, normalize, exact)

@@ -799,6 +799,9 @@ const char *bc_kernel_name(int kernel_id)
         case KID_BACKWARD_SLAB: return "backward_slab_kernel";
         case KID_FORWARD_QUAD: return "forward_quad_kernel";
         case KID_BACKWARD_QUAD: return "backward_quad_kernel";
+        case KID_FORWARD_TMEM: return "forward_tmem_kernel";
+        case KID_FORWARD_TMEM_STREAM: return "forward_tmem_stream_kernel";
+        case KID_BACKWARD_QUAD_PAIR: return "backward_quad_pair_kernel";
         default: return "unknown";
     }
 }

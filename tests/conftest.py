@@ -32,3 +32,23 @@ def max_rel(a, b):
     if denom == 0:
         return np.abs(a - b).max()
     return np.abs(a - b).max() / denom
+
+
+def kernels_run(call):
+    """Names of the library's kernels that `call()` launches on the current device, in order."""
+    import ctypes
+
+    import torch
+    from box_convolution import _cabi
+    lib, kernel, ms = _cabi.lib, ctypes.c_int(), ctypes.c_float()
+    _cabi.check(lib.bc_profile_start(64), "bc_profile_start")
+    try:
+        call()
+        torch.cuda.synchronize()
+    finally:
+        lib.bc_profile_stop()
+    names = []
+    for i in range(lib.bc_profile_count()):
+        _cabi.check(lib.bc_profile_get(i, ctypes.byref(kernel), ctypes.byref(ms)), "bc_profile_get")
+        names.append(lib.bc_kernel_name(kernel.value).decode())
+    return names

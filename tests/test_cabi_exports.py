@@ -45,6 +45,16 @@ def test_status_strings_and_argument_checks_without_a_gpu():
     assert lib.bc_boxconv2d_backward_workspace(2, 3, 4, 8, 8, 0) == 0
 
 
+def test_every_kernel_has_a_name_of_its_own():
+    from box_convolution import _cabi
+    ids = re.search(r"enum KernelId \{(.*?)KID_COUNT", open(os.path.join(PKG_DIR, "csrc", "bc_common.cuh")).read(), re.S).group(1)
+    count = ids.count("KID_")
+    names = [_cabi.lib.bc_kernel_name(i) for i in range(1, count + 1)]
+    assert len(set(names)) == count and b"unknown" not in names
+    assert _cabi.lib.bc_kernel_name(0) == _cabi.lib.bc_kernel_name(count + 1) == b"unknown"
+    assert {b"forward_tmem_kernel", b"forward_tmem_stream_kernel", b"backward_quad_pair_kernel"} <= set(names)
+
+
 def test_header_compiles_as_plain_c_and_links(tmp_path):
     """The boundary is a C ABI: a C99 translation unit that includes the header and takes the
     address of entry points must compile with gcc and link against the library."""

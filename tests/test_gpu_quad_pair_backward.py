@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 import torch
 
-from conftest import max_rel
+from conftest import kernels_run, max_rel
 
 pytestmark = pytest.mark.gpu
 
@@ -81,3 +81,17 @@ def test_same_values_at_another_address():
     gin_off, gp_off = _grads(m, x, off)
     assert max_rel(gin_off.cpu().numpy(), gin.cpu().numpy()) < 1e-5      # (other kernels, another order of additions)
     assert max_rel(gp_off.cpu().numpy(), gp.cpu().numpy()) < 1e-4
+
+
+# both sides of the rule's lines: one and two columns of 16 and 18 tiles, even and odd numbers, planes for two CTAs an SM, types
+@pytest.mark.parametrize("shape,dtype,kernel", [
+    ((1, 149, 2, 128, 128), torch.float32, "backward_quad_pair_kernel"), ((1, 149, 2, 112, 68), torch.bfloat16, "backward_quad_pair_kernel"),
+    ((1, 148, 2, 128, 128), torch.float32, "backward_quad_kernel"), ((1, 149, 2, 120, 128), torch.float32, "backward_quad_kernel"),
+    ((1, 149, 2, 104, 128), torch.float16, "backward_quad_kernel"), ((1, 149, 2, 96, 128), torch.float32, "backward_quad_kernel"),
+    ((1, 3, 2, 144, 128), torch.float32, "backward_plane_kernel"), ((1, 3, 2, 136, 128), torch.float32, "backward_plane_kernel"),
+    ((1, 3, 2, 256, 68), torch.bfloat16, "backward_plane_kernel"), ((1, 3, 2, 72, 132), torch.float32, "backward_quad_pair_kernel"),
+    ((1, 3, 2, 128, 256), torch.float16, "backward_quad_pair_kernel"), ((1, 3, 2, 96, 160), torch.bfloat16, "backward_plane_kernel"),
+    ((1, 3, 2, 73, 256), torch.float32, "backward_plane_kernel"), ((1, 3, 2, 72, 254), torch.float32, "backward_plane_kernel")])
+def test_kernel_that_serves_a_plane(shape, dtype, kernel):
+    m, x, g = _case(shape, True, True, dtype)
+    assert kernel in kernels_run(lambda: _grads(m, x, g))

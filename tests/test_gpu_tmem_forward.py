@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 import torch
 
-from conftest import max_rel
+from conftest import kernels_run, max_rel
 
 pytestmark = pytest.mark.gpu
 
@@ -73,3 +73,18 @@ def test_boxes_beyond_the_plane():
         out = BoxConvolutionFunction.apply(x, m.x_min, m.x_max, m.y_min, m.y_max, m.reparametrization_h, m.reparametrization_w, False, True)
     # what is left is the rounding of 16 terms, sums of up to h w values in [0, 1) each, that cancel
     assert out.abs().max() < 16 * 2.0 ** -24 * h * w
+
+
+# both sides of the rule's lines: planes, tiles for either kernel, filters that leave quarters of tensor memory idle, alignment, heights
+@pytest.mark.parametrize("shape,kernel", [
+    ((2, 37, 4, 64, 128), "forward_tmem_stream_kernel"), ((1, 73, 4, 64, 128), "forward_quad_kernel"),
+    ((1, 74, 4, 128, 128), "forward_tmem_stream_kernel"), ((1, 74, 4, 128, 256), "forward_tmem_kernel"),
+    ((1, 223, 4, 128, 128), "forward_tmem_stream_kernel"), ((1, 149, 4, 128, 128), "forward_quad_kernel"),
+    ((1, 80, 5, 64, 128), "forward_quad_kernel"), ((1, 80, 4, 60, 128), "forward_quad_kernel"), ((1, 80, 4, 64, 126), "forward_quad_kernel"),
+    ((1, 80, 4, 136, 128), "forward_quad_kernel"), ((1, 80, 4, 96, 132), "forward_plane_kernel"), ((1, 80, 4, 64, 64), "forward_plane_kernel")])
+def test_kernel_that_serves_a_plane(shape, kernel):
+    import box_convolution as bc
+    N, C, F, h, w = shape
+    m, x = _module(bc, shape, True, True), torch.randn(N, C, h, w, device="cuda")
+    with torch.no_grad():
+        assert kernel in kernels_run(lambda: m(x))
