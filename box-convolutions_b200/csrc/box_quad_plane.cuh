@@ -688,7 +688,9 @@ inline int quad_pair_max_threads(int col_tiles, int warps)
 // no kernel of more than eight warps: 32 x 32 tiles): in 16 bits, whose 32 x 32-tile kernel leaves
 // room for a second CTA, where these tiles waste little more than those ((10,16,4,96,160), 24 tiles for 15: 67 us against
 // 58; (10,16,4,80,240), 20 for 24: 65 against 115); float always ((24,16,4,96,160): 122, 123; (55,16,4,128,156): 278, 370;
-// (30,16,2,88,188): 92, 129; (40,16,4,104,224): 232, 345).  14 and 16 tiles, which as one tile a warp have an SM to themselves:
+// (30,16,2,88,188): 92, 129; (40,16,4,104,224): 232, 345), but not where 32 x 32 tiles are 16 at most, two CTAs an SM, and there are
+// planes for two (planes x filters x rows x columns: 1471 x 1 x 88 x 156, bfloat16: 129, 105; 748 x 2 x 80 x 132: 116, 103; 550 x 4 x 96 x 156: 285, 258;
+// 425 x 6 x 80 x 160 the other way: 147, 160; 84 x 4 x 96 x 144: 35.9, 46.1).  14 and 16 tiles, which as one tile a warp have an SM to themselves:
 // two CTAs of half the warps, if there are planes for two ((16,32,4,128,128): 96, 117; (16,32,4,64,256): 99, 115;
 // (64,32,4,112,96): 265, 334; 144 planes of 128 x 120: 28.7, 26.6).  Not of 10 and 12 tiles, two CTAs an SM either way
 // ((16,32,4,96,128): 73, 69; (16,32,4,40,248): 71, 64).
@@ -697,7 +699,8 @@ inline bool quad_pair_suits_backward(int64_t planes, int F, int h, int w, bool w
     const int col_tiles = quad_col_tiles(w), tiles = quad_row_tiles(h) * col_tiles, square = ((h + 31) / 32) * ((w + 31) / 32);
     if (w < kQuadMinWidth || w > 256 || w % 4 || h % kTileRows || F > kMaxFilters || tiles % 2 || quad_backward_smem(F, h, w) > kQuadMaxSmem) return false;
     if (tiles <= kQuadMaxWarps) return tiles > 12 && planes > 148;
-    return col_tiles == 2 && tiles <= 2 * kQuadMaxWarps && (wide || 2 * tiles <= 3 * square);
+    if (col_tiles != 2 || tiles > 2 * kQuadMaxWarps || (square <= 16 && planes > 148)) return false;
+    return wide || 2 * tiles <= 3 * square;
 }
 
 template <typename IO>

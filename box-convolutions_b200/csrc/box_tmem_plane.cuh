@@ -316,16 +316,26 @@ inline size_t tmem_stream_smem(int h, int w)
 }
 
 // Which planes: rows and tensors aligned for vector accesses, heights a multiple of 8 (with guarded rows the quad kernel is
-// as fast: (110,16,4,41,116): 63 us here, 59 there; (129,16,4,32,104): 33 and 37).  At least three of the four quarters of
-// tensor memory at work, and a second column tile that is not mostly empty ((171,16,4,56,132): 143 us, in 32 x 32 tiles 130;
-// (19,16,4,56,208): 28, 35).  Enough planes, as their filters are not split over CTAs ((4,16,4,48,216): 10.9 us, 8.3;
-// (5,16,4,40,232): 10.4, 11.8), and where an SM runs one streaming CTA not a little more than one round of them ((13,16,4,64,228): 23.9
-// us, 22.8; (154,16,4,72,120): 93, 108).  (256,32,4,64,128): 273 -> 230 us; (8,16,4,128,256): 30.5 -> 22.
+// as fast: (110,16,4,41,116): 63 us here, 59 there; (129,16,4,32,104): 33 and 37).  Enough planes, as their filters are not
+// split over CTAs ((4,16,4,48,216): 10.9 us, 8.3; (5,16,4,40,232): 10.4, 11.8), and where an SM runs one streaming CTA not a little
+// more than one round of them ((13,16,4,64,228): 23.9 us, 22.8; (154,16,4,72,120): 93, 108).  (256,32,4,64,128): 273 -> 230 us;
+// (8,16,4,128,256): 30.5 -> 22.
+// A second column tile that is not mostly empty: up to 160 columns 32 x 32 tiles waste less (planes x filters x rows x columns,
+// here and there: 2878 x 4 x 96 x 160: 318 us, 205; 340 x 6 x 80 x 160: 56, 44; 510 x 6 x 32 x 160: 26, 23; 1321 x 8 x 104 x 160 the other way:
+// 248, 262; from 164 to 192 columns 0.90 of the time at the median of 148 sizes).
+// At least three of the four quarters of tensor memory at work.  Three of them, over more than one plane an SM, only where few
+// lanes idle as well, or the plane has but three units (1171 x 3 x 128 x 172, bfloat16: 164 us, 124; 2332 x 6 x 24 x 84: 52, 41;
+// 191 x 3 x 24 x 228: 10.8, 8.2; but 147 x 3 x 104 x 72: 9.5, 12.9).
+// One or two rows of tiles, which leave a gathering warp eight rows or none, in two columns: many filters, or the
+// quad kernel's shorter chain wins (228 x 2 x 8 x 188: 5.7 us, 4.8; 188 x 4 x 8 x 208: 7.3, 6.2; 184 x 2 x 16 x 244: 7.0, 6.1; 260 x 16 x 8 x 256: 13.9, 19.5;
+// 604 x 6 x 16 x 164: 18.9, 20.9).
 inline bool tmem_suits_forward(int64_t planes, int F, int h, int w)
 {
     const int ct = quad_col_tiles(w), tiles = quad_row_tiles(h) * ct, units = F * ct;
-    if (h % kTileRows || w % 4 || w < kQuadMinWidth || w > 256 || (ct > 1 && w < 160) || h > kTmemMaxRows || F > kMaxFilters) return false;
-    if (4 * units < 3 * ((units + 3) / 4 * 4) || planes < 74) return false;
+    if (h % kTileRows || w % 4 || w < kQuadMinWidth || w > 256 || (ct > 1 && w <= 160) || h > kTmemMaxRows || F > kMaxFilters || planes < 74) return false;
+    if (4 * units < 3 * ((units + 3) / 4 * 4)) return false;
+    if (units % 4 && planes > 148 && !(units == 3 && w > 96) && 10 * w < 9 * 128 * ct) return false;
+    if (ct > 1 && h <= 2 * kTileRows && (F < 6 || (h == kTileRows && w <= 200))) return false;
     if (tiles > 16) return tiles <= 2 * kQuadMaxWarps && tmem_forward_smem(F, h, w) <= kQuadMaxSmem;
     return tmem_stream_smem(h, w) <= kQuadMaxSmem && (tiles <= 8 || planes <= 148 || planes > 222);
 }

@@ -15,4 +15,15 @@ extern "C" int rule_pair_backward(int64_t planes, int F, int h, int w, int wide,
     return warps * 32;
 }
 
+// Does the forward through tensor memory serve the plane?  If so, the tiles of a plane, the warps that build it and the
+// tensor-memory columns of a CTA.
+extern "C" int rule_tmem_forward(int64_t planes, int F, int h, int w, int *tiles, int *warps, int *columns)
+{
+    if (!tmem_suits_forward(planes, F, h, w)) return 0;
+    *tiles = quad_row_tiles(h) * quad_col_tiles(w);
+    *warps = tmem_forward_warps(h, w);
+    *columns = h * kStrip;
+    return 1;
+}
+
 }  // namespace bc

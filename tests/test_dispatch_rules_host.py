@@ -19,6 +19,7 @@ def rules(tmp_path_factory):
                            "-I", os.path.join(PKG_DIR, "csrc"), "-o", out, src])
     lib = ctypes.CDLL(out)
     lib.rule_pair_backward.argtypes = [ctypes.c_int64] + [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)] * 2
+    lib.rule_tmem_forward.argtypes = [ctypes.c_int64] + [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_int)] * 3
     return lib
 
 
@@ -39,3 +40,37 @@ def test_pair_backward_launches_fit_their_kernels(rules):
                             assert threads <= bound.value, (planes, F, h, w, wide)
                             assert columns.value <= 512, (planes, F, h, w, wide)
     assert served == {14, 16, 18, 20, 22, 24, 26, 28, 30, 32}
+
+
+def test_tensor_memory_forward_launches_fit_their_kernels(rules):
+    tiles, warps, columns = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
+    served = set()
+    for h in range(1, 321):
+        for w in range(60, 321):
+            if (h % 8 or w % 4) and (h + w) % 17:
+                continue
+            for F in (2, 3, 4, 32):
+                for planes in (74, 148, 223, 5000):
+                    if rules.rule_tmem_forward(planes, F, h, w, ctypes.byref(tiles), ctypes.byref(warps), ctypes.byref(columns)):
+                        served.add(tiles.value)
+                        assert h % 8 == 0 and w % 4 == 0 and columns.value <= 512
+                        # one tile a building warp in the streaming kernels, two in the other, which one column of tiles does not have
+                        assert tiles.value <= 8 and warps.value == 8 or warps.value == 16 and tiles.value <= (16 if w <= 128 else 32)
+    assert {1, 2, 8, 9, 16, 18, 32} <= served
+
+
+# (planes, F, h, w, float32): sizes that the kernels served before are faster on
+FORWARD_ELSEWHERE = [(2878, 4, 96, 160), (340, 6, 80, 160), (217, 4, 120, 160), (1171, 3, 128, 172), (1799, 3, 8, 216), (191, 3, 24, 228), (2332, 6, 24, 84),
+                     (470, 3, 64, 168), (1405, 3, 64, 88), (1299, 6, 128, 80), (228, 2, 8, 188), (188, 4, 8, 208), (2114, 2, 8, 216), (184, 2, 16, 244), (1157, 4, 16, 212)]
+FORWARD_HERE = [(512, 4, 64, 128), (8192, 4, 64, 128), (128, 4, 128, 256), (101, 3, 56, 116), (147, 3, 104, 72), (500, 3, 64, 128), (123, 16, 8, 80), (967, 4, 8, 128),
+                (260, 16, 8, 256), (604, 6, 16, 164), (104, 4, 104, 164), (84, 2, 72, 172), (682, 4, 40, 184)]
+PAIR_ELSEWHERE = [(1471, 1, 88, 156, 0), (725, 4, 72, 132, 1), (748, 2, 80, 132, 1), (1992, 2, 72, 140, 0), (969, 2, 96, 148, 1), (550, 4, 96, 156, 1), (272, 4, 88, 160, 1)]
+PAIR_HERE = [(128, 4, 128, 256, 1), (128, 4, 96, 160, 1), (110, 16, 112, 132, 1), (991, 4, 128, 156, 1), (1482, 4, 112, 160, 1), (1583, 6, 104, 164, 1), (1400, 4, 72, 164, 1), (149, 4, 128, 128, 1)]
+
+
+def test_sizes_that_other_kernels_are_faster_on_go_there(rules):
+    n = [ctypes.byref(ctypes.c_int()) for _ in range(3)]
+    assert not [c for c in FORWARD_ELSEWHERE if rules.rule_tmem_forward(*c, *n)]
+    assert all(rules.rule_tmem_forward(*c, *n) for c in FORWARD_HERE)
+    assert not [c for c in PAIR_ELSEWHERE if rules.rule_pair_backward(*c, *n[:2])]
+    assert all(rules.rule_pair_backward(*c, *n[:2]) for c in PAIR_HERE)
