@@ -92,7 +92,10 @@ __device__ __forceinline__ void tmem_use_rows(const TmemUnit &n, const BoxTaps &
 {
     const float sfl = t.scale * t.f_lo_r, sfh = t.scale * t.f_hi_r;
     const f2_t scale2 = pack2(t.scale, t.scale), sfl2 = pack2(sfl, sfl), sfh2 = pack2(sfh, sfh);
-    // The integral rows a .. a+3 combined (row 0 is zero, rows past the plane repeat its last).
+    // The integral rows a .. a+3 combined (row 0 is zero, rows past the plane repeat its last).  Zero times the columns' weights:
+    // a box whose sides are no numbers gives none in the rows above the plane either.
+    const float none = 0.0f * t.f_lo_c + 0.0f * t.f_hi_c;
+    const float4 row0 = make_float4(none, none, none, none);
     auto fetch = [&](float4 (&v)[4], int a) {
         __syncwarp();
         if (a >= 1 && a + 3 <= n.h) {
@@ -104,7 +107,7 @@ __device__ __forceinline__ void tmem_use_rows(const TmemUnit &n, const BoxTaps &
             tmem_wait_load(v);
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                if (a + i < 1) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (a + i < 1) v[i] = row0;
         }
     };
     if (n.r_begin >= n.r_end) return;
@@ -115,8 +118,8 @@ __device__ __forceinline__ void tmem_use_rows(const TmemUnit &n, const BoxTaps &
         tmem_load4(n.rows32 + 4 * (min(max(a, 1), n.h) - 1), A);
         tmem_load4(n.rows32 + 4 * (min(max(b, 1), n.h) - 1), B);
         tmem_wait_load(A, B);
-        if (a < 1) A = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (b < 1) B = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (a < 1) A = row0;
+        if (b < 1) B = row0;
     }
 #pragma unroll 1
     for (int p = n.r_begin; p < n.r_end; p += 4) {

@@ -75,6 +75,25 @@ def test_boxes_beyond_the_plane():
     assert out.abs().max() < 16 * 2.0 ** -24 * h * w
 
 
+@pytest.mark.parametrize("side", range(4))
+def test_boxes_that_are_no_numbers(side):
+    """A parameter that is NaN, or infinite where fractions count, makes all outputs of its filter NaN, those above the plane too;
+    the other filters keep theirs."""
+    import box_convolution as bc
+    C, F, h, w = 80, 4, 64, 128
+    x = torch.rand(1, C, h, w, device="cuda")
+    pixels = [torch.full((C, F), v, device="cuda") for v in (-90.0, -70.0, -3.0, 3.0)]      # (above the plane for every row)
+    pixels[0][:, ::2], pixels[1][:, ::2] = -2.5, 2.25
+    clean = bc.BoxConvolutionFunction.apply(x, *pixels, 1.0, 1.0, False, True).view(C, F, h, w)
+    for value in (float("nan"), float("inf") * (-1 if side % 2 == 0 else 1)):
+        p = [v.clone() for v in pixels]
+        p[side][:, 1], p[side][:, 2] = value, value
+        assert "forward_tmem_stream_kernel" in kernels_run(lambda: bc.BoxConvolutionFunction.apply(x, *p, 1.0, 1.0, False, True))
+        out = bc.BoxConvolutionFunction.apply(x, *p, 1.0, 1.0, False, True).view(C, F, h, w)
+        assert out[:, 1:3].isnan().all()
+        assert torch.equal(out[:, ::3], clean[:, ::3])
+
+
 # both sides of the rule's lines: planes, tiles for either kernel, filters that leave quarters of tensor memory idle, alignment, heights
 @pytest.mark.parametrize("shape,kernel", [
     ((2, 37, 4, 64, 128), "forward_tmem_stream_kernel"), ((1, 73, 4, 64, 128), "forward_quad_kernel"),
