@@ -186,7 +186,11 @@ __device__ __forceinline__ float warp_sum5(const float (&v)[kNumSums], int lane)
 // to the accumulators.
 // The column strips enter the sums weighted by u(j), what the rows of the box make of the input values next to
 // tap row j: sum_i x_i (row combination of e) = sum_j e(j) (w_a x_(j+1) + w_b x_j).
-template <int R, bool NEED_PARAMS, bool FULL, class Rows, class Cells>
+// PACKED: an input value is held twice, as the factor of a pair of tap rows.  That saves operations, which pays where registers
+// leave three or two CTAs an SM and the tiles are full, of one column ((256,32,4,64,128): 504 us, scalar 522; (32,32,4,64,128) in
+// bfloat16 71 and 74; with two columns it costs 0.5 to 1 %).  Where rows are cut or unaligned, scalars ((60,16,4,40,250): 140 us in pairs, 131).
+// The same values either way.
+template <int R, bool NEED_PARAMS, bool FULL, bool PACKED = false, class Rows, class Cells>
 __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const QuadCols &cols, const Rows &q, const ColW2 &cw,
                                                     Cells &&at, float (&sums)[kNumSums], int rows)
 {
@@ -202,20 +206,27 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
         return (hi_old - lo_new) + t.f_hi_r * bot + t.f_lo_r * top;
     };
     if (NEED_PARAMS) {
-        f2_t left = pack2(0.f, 0.f), right = left, out2 = left;
+        f2_t left = pack2(0.f, 0.f), right = left, out2 = left, topbot = left;
         float s_top = 0.f, s_bot = 0.f;
-        f2_t el[kStrip], eh[kStrip];
+        f2_t el[kStrip], eh[kStrip], xx[kStrip];      // (topbot, xx: PACKED)
         quad_pair_e(cols, q.lo(0), q.hi(0), cw, pd, el, eh);
         float4 e = at.first();
         // What the rows of the box make of the input values next to a pair of tap rows.  (Two products: the values' difference,
         // an operation less, is infinite for large ones of opposite sign.)
         const float wb_top = t.f_lo_r - 1.0f, wa_bot = 1.0f - t.f_hi_r;
+        const f2_t wa = pack2(-t.f_lo_r, wa_bot), wb = pack2(wb_top, t.f_hi_r);
         auto weigh = [&](float x, float next) { return pack2(fmaf(-t.f_lo_r, next, wb_top * x), fmaf(wa_bot, next, t.f_hi_r * x)); };
         {
             const float x0[kStrip] = {e.x, e.y, e.z, e.w};
 #pragma unroll
             for (int m = 0; m < kStrip; ++m) {
-                const f2_t u = weigh(0.f, x0[m]);
+                f2_t u;
+                if constexpr (PACKED) {
+                    xx[m] = pack2(x0[m], x0[m]);
+                    u = mul2(wa, xx[m]);
+                } else {
+                    u = weigh(0.f, x0[m]);
+                }
                 left = fma2(u, el[m], left);
                 right = fma2(u, eh[m], right);
             }
@@ -231,14 +242,24 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
                 const float x1[kStrip] = {i + 1 < R ? below.x : 0.f, i + 1 < R ? below.y : 0.f, i + 1 < R ? below.z : 0.f, i + 1 < R ? below.w : 0.f};
 #pragma unroll
                 for (int m = 0; m < kStrip; ++m) {
-                    const f2_t u = weigh(x0[m], x1[m]);
+                    f2_t u;
+                    dd[m] = sub2(cd[m], pd[m]);
+                    if constexpr (PACKED) {
+                        u = mul2(wb, xx[m]);
+                        topbot = fma2(xx[m], dd[m], topbot);
+                        if (i + 1 < R) {
+                            xx[m] = pack2(x1[m], x1[m]);
+                            u = fma2(wa, xx[m], u);
+                        }
+                    } else {
+                        u = weigh(x0[m], x1[m]);
+                        float top, bot;
+                        unpack2(dd[m], top, bot);
+                        s_top = fmaf(x0[m], top, s_top);
+                        s_bot = fmaf(x0[m], bot, s_bot);
+                    }
                     left = fma2(u, el[m], left);
                     right = fma2(u, eh[m], right);
-                    dd[m] = sub2(cd[m], pd[m]);
-                    float top, bot;
-                    unpack2(dd[m], top, bot);
-                    s_top = fmaf(x0[m], top, s_top);
-                    s_bot = fmaf(x0[m], bot, s_bot);
                 }
                 const f2_t g01 = pack2(gather(cd[0], pd[0], dd[0]), gather(cd[1], pd[1], dd[1]));
                 const f2_t g23 = pack2(gather(cd[2], pd[2], dd[2]), gather(cd[3], pd[3], dd[3]));
@@ -249,6 +270,7 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
                 if (i + 1 < R) e = below;
             }
         }
+        if constexpr (PACKED) unpack2(topbot, s_top, s_bot);
         float a, b;
         unpack2(out2, a, b); sums[0] = a + b;
         sums[1] = s_top; sums[2] = s_bot;

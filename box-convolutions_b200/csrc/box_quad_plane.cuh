@@ -9,6 +9,8 @@
 // several column tiles), against three and 35 % more instructions for 32 x 32 tiles.
 // The gather is that of the slab kernels: five words of shared memory an output and side, no bank conflicts.
 #pragma once
+#include <type_traits>
+
 #include "bc_common.cuh"
 #include "bc_finish.cuh"
 #include "bc_quad.cuh"
@@ -453,9 +455,9 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
         __syncthreads();
         float sums[kNumSums] = {0.f, 0.f, 0.f, 0.f, 0.f};
         const BoxTaps t = load_taps_uniform(sTaps + f * kTapWords);
-        quad_backward_strip<kTileRows, NEED_PARAMS, FAST>(t, quad_cols(t, tile.c >> 2, cells, Q::kCells),
-                                                          quad_rows<kTileRows>(t, tile.p0, h, s.image, s.image, Q::kRow, lane),
-                                                          col_weights(t), kept, sums, tile.rows);
+        quad_backward_strip<kTileRows, NEED_PARAMS, FAST, FAST && CT == 1 && MAXT <= 384>(t, quad_cols(t, tile.c >> 2, cells, Q::kCells),
+                                                                                          quad_rows<kTileRows>(t, tile.p0, h, s.image, s.image, Q::kRow, lane),
+                                                                                          col_weights(t), kept, sums, tile.rows);
         kept.sync();
         if (NEED_PARAMS) {
             const float sum = warp_sum5(sums, lane);
@@ -500,6 +502,8 @@ backward_quad_pair_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_
                           float *__restrict__ partials, int N, int C, int F, int h, int w, int row_tiles, bool normalize, bool exact, bool write_gin, Finish fin)
 {
     constexpr int T = 2;
+    // (the scalar form spills 44 bytes here: with pairs 0.97 of the time over 5 sizes of up to 16 tiles, 0.995 over 73 larger ones; float 1.014)
+    constexpr bool kPacked = CT == 2 && std::is_same<IO, __nv_bfloat16>::value;
     using Q = QuadImage<CT>;
     extern __shared__ float4 smem4[];
     grid_dependency_release();
@@ -569,9 +573,9 @@ backward_quad_pair_kernel(const IO *__restrict__ x, const IO *__restrict__ grad_
             const QuadTile tile = tile_of(k);
             TmemRows<1, T> kept(tmem_base, warp, k);
             float sums[kNumSums] = {0.f, 0.f, 0.f, 0.f, 0.f};
-            quad_backward_strip<kTileRows, NEED_PARAMS, true>(t, quad_cols(t, tile.c >> 2, cells, Q::kCells),
-                                                              quad_rows_later<kTileRows>(t, tile.p0, h, s.image, s.image, Q::kRow, lane), col_weights(t), kept,
-                                                              sums, kTileRows);
+            quad_backward_strip<kTileRows, NEED_PARAMS, true, kPacked>(t, quad_cols(t, tile.c >> 2, cells, Q::kCells),
+                                                                       quad_rows_later<kTileRows>(t, tile.p0, h, s.image, s.image, Q::kRow, lane),
+                                                                       col_weights(t), kept, sums, kTileRows);
             kept.sync();
 #pragma unroll
             for (int j = 0; j < kNumSums; ++j) all[j] += sums[j];
