@@ -383,7 +383,7 @@ forward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
 // values wait in tensor memory (bc_tmem.cuh).  The next grad_output plane is requested into L2 while the
 // current one is gathered.
 // Bound by the latencies of its phases, which other CTAs of the SM have to cover: (256,32,4,64,128) with accumulators in
-// registers and input values in shared memory, two CTAs an SM: 564 us; like this, three: 512 us.
+// registers and input values in shared memory, two CTAs an SM: 564 us; like this, three: 504 us.
 template <typename IO, int CT, bool FAST, bool NEED_PARAMS, bool COUNTED, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT > 384 ? 1 : MAXT > 256 ? 2 : FAST || NEED_PARAMS ? 3 : 2)
 backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const IO *__restrict__ grad_output, BoxParams bp, IO *__restrict__ grad_input,
@@ -494,7 +494,7 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
 // whole of tensor memory for their input values and grad-input accumulators, and the SM; 14 and 16 tiles half of either.
 // The 32 x 32-tile kernel, which had the former before, keeps accumulators in registers and reads the input plane again from L2 for every
 // filter, and its tap loads conflict where rows are clamped at the plane's border.
-// (8,16,4,128,256): 79 -> 52 us, bfloat16 (10,16,4,80,240): 115 -> 65.  Every warp has two whole tiles; asked whether it has, the compiler
+// (8,16,4,128,256): 71 -> 51 us, bfloat16 (10,16,4,80,240): 105 -> 68.  Every warp has two whole tiles; asked whether it has, the compiler
 // ran out of registers (456 bytes of spills, 64 us).
 template <typename IO, int CT, bool NEED_PARAMS, bool COUNTED, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 2 : 1)
@@ -688,22 +688,25 @@ inline int quad_pair_max_threads(int col_tiles, int warps)
     return col_tiles == 2 && warps <= kQuadMaxWarps ? 512 : 0;
 }
 
-// Aligned planes with two tiles a warp, so with an even number of tiles.  18 to 32 tiles in two columns (one column of them has
-// no kernel of more than eight warps: 32 x 32 tiles): in 16 bits, whose 32 x 32-tile kernel leaves
-// room for a second CTA, where these tiles waste little more than those ((10,16,4,96,160), 24 tiles for 15: 67 us against
-// 58; (10,16,4,80,240), 20 for 24: 65 against 115); float always ((24,16,4,96,160): 122, 123; (55,16,4,128,156): 278, 370;
-// (30,16,2,88,188): 92, 129; (40,16,4,104,224): 232, 345), but not where 32 x 32 tiles are 16 at most, two CTAs an SM, and there are
-// planes for two (planes x filters x rows x columns: 1471 x 1 x 88 x 156, bfloat16: 129, 105; 748 x 2 x 80 x 132: 116, 103; 550 x 4 x 96 x 156: 285, 258;
-// 425 x 6 x 80 x 160 the other way: 147, 160; 84 x 4 x 96 x 144: 35.9, 46.1).  14 and 16 tiles, which as one tile a warp have an SM to themselves:
-// two CTAs of half the warps, if there are planes for two ((16,32,4,128,128): 96, 117; (16,32,4,64,256): 99, 115;
-// (64,32,4,112,96): 265, 334; 144 planes of 128 x 120: 28.7, 26.6).  Not of 10 and 12 tiles, two CTAs an SM either way
-// ((16,32,4,96,128): 73, 69; (16,32,4,40,248): 71, 64).
+// Aligned planes with two tiles a warp, so with an even number of tiles.
+// 18 to 32 tiles in two columns (one column of them has no kernel of more than eight warps: 32 x 32 tiles).  In 16 bits, whose
+// 32 x 32-tile kernel leaves room for a second CTA, where these tiles waste little more than those ((10,16,4,96,160), 24 tiles for
+// 15: 67 us against 58; (10,16,4,80,240), 20 for 24: 68 against 105); float always ((55,16,4,128,156): 274, 351; (30,16,2,88,188):
+// 83, 121; (40,16,4,104,224): 215, 330).  But of at most 16 tiles of 32 x 32 an SM runs two planes, at about half the rate: a
+// round of 148 planes here then has to save half a round there, which it does in the first and the third, and with eight filters or
+// more in any.  Planes, filters, rows, columns: (84,4,96,144) 36 us, 46; (272,4,88,160) 70, 67; (360,8,80,152) 186, 219; (425,6,80,160)
+// 147, 160; (748,2,80,132) 116, 103; (1100,4,96,156) 285, 258; (722,16,88,136) 593, 692; in bfloat16 (564,4,88,140) 136, 128;
+// (1471,1,88,156) 129, 105; (592,16,72,140) 474, 501.
+// 14 and 16 tiles, which as one tile a warp have an SM to themselves: two CTAs of half the warps, if there are planes for two
+// ((16,32,4,128,128): 94, 105; (16,32,4,64,256): 91, 108; (64,32,4,112,96): 258, 329).  Not of 10 and 12 tiles, two CTAs an SM either
+// way ((16,32,4,96,128): 73, 68; (16,32,4,40,248): 71, 65).
 inline bool quad_pair_suits_backward(int64_t planes, int F, int h, int w, bool wide)
 {
     const int col_tiles = quad_col_tiles(w), tiles = quad_row_tiles(h) * col_tiles, square = ((h + 31) / 32) * ((w + 31) / 32);
     if (w < kQuadMinWidth || w > 256 || w % 4 || h % kTileRows || F > kMaxFilters || tiles % 2 || quad_backward_smem(F, h, w) > kQuadMaxSmem) return false;
     if (tiles <= kQuadMaxWarps) return tiles > 12 && planes > 148;
-    if (col_tiles != 2 || tiles > 2 * kQuadMaxWarps || (square <= 16 && planes > 148)) return false;
+    if (col_tiles != 2 || tiles > 2 * kQuadMaxWarps) return false;
+    if (square <= 16 && F < 8 && !(planes <= 148 || (planes > 296 && planes <= 444))) return false;
     return wide || 2 * tiles <= 3 * square;
 }
 

@@ -64,8 +64,8 @@ FORWARD_ELSEWHERE = [(2878, 4, 96, 160), (340, 6, 80, 160), (217, 4, 120, 160), 
                      (470, 3, 64, 168), (1405, 3, 64, 88), (1299, 6, 128, 80), (228, 2, 8, 188), (188, 4, 8, 208), (2114, 2, 8, 216), (184, 2, 16, 244), (1157, 4, 16, 212)]
 FORWARD_HERE = [(512, 4, 64, 128), (8192, 4, 64, 128), (128, 4, 128, 256), (101, 3, 56, 116), (147, 3, 104, 72), (500, 3, 64, 128), (123, 16, 8, 80), (967, 4, 8, 128),
                 (260, 16, 8, 256), (604, 6, 16, 164), (104, 4, 104, 164), (84, 2, 72, 172), (682, 4, 40, 184)]
-PAIR_ELSEWHERE = [(1471, 1, 88, 156, 0), (725, 4, 72, 132, 1), (748, 2, 80, 132, 1), (1992, 2, 72, 140, 0), (969, 2, 96, 148, 1), (550, 4, 96, 156, 1), (272, 4, 88, 160, 1)]
-PAIR_HERE = [(128, 4, 128, 256, 1), (128, 4, 96, 160, 1), (110, 16, 112, 132, 1), (991, 4, 128, 156, 1), (1482, 4, 112, 160, 1), (1583, 6, 104, 164, 1), (1400, 4, 72, 164, 1), (149, 4, 128, 128, 1)]
+PAIR_ELSEWHERE = [(1471, 1, 88, 156, 0), (725, 4, 72, 132, 1), (748, 2, 80, 132, 1), (1992, 2, 72, 140, 0), (969, 2, 96, 148, 1), (550, 4, 96, 156, 1), (564, 4, 88, 140, 0), (272, 4, 88, 160, 1)]
+PAIR_HERE = [(722, 16, 88, 136, 1), (592, 16, 72, 140, 0), (360, 8, 80, 152, 1), (425, 6, 80, 160, 1), (383, 4, 88, 140, 0), (128, 4, 128, 256, 1), (128, 4, 96, 160, 1), (110, 16, 112, 132, 1), (991, 4, 128, 156, 1), (1482, 4, 112, 160, 1), (1583, 6, 104, 164, 1), (1400, 4, 72, 164, 1), (149, 4, 128, 128, 1)]
 
 
 def test_sizes_that_other_kernels_are_faster_on_go_there(rules):
