@@ -59,7 +59,8 @@ def test_tensor_memory_forward_launches_fit_their_kernels(rules):
     assert {1, 2, 8, 9, 16, 18, 32} <= served
 
 
-# (planes, F, h, w, float32): sizes that the kernels served before are faster on
+# Planes, filters, rows, columns (and whether float32) on both sides of the rules' lines, as measured: where other kernels are faster,
+# and where these are.
 FORWARD_ELSEWHERE = [(2878, 4, 96, 160), (340, 6, 80, 160), (217, 4, 120, 160), (1171, 3, 128, 172), (1799, 3, 8, 216), (191, 3, 24, 228), (2332, 6, 24, 84),
                      (470, 3, 64, 168), (1405, 3, 64, 88), (1299, 6, 128, 80), (228, 2, 8, 188), (188, 4, 8, 208), (2114, 2, 8, 216), (184, 2, 16, 244), (1157, 4, 16, 212)]
 FORWARD_HERE = [(512, 4, 64, 128), (8192, 4, 64, 128), (128, 4, 128, 256), (101, 3, 56, 116), (147, 3, 104, 72), (500, 3, 64, 128), (123, 16, 8, 80), (967, 4, 8, 128),

@@ -241,7 +241,8 @@ def test_backward_from_two_streams(bc, shape):
 
 # Borders that no int holds, the largest finite ones, and (where fractions are dropped) infinite ones give what borders just
 # outside of the plane give, to the last bit: every tap is clamped to the same row or column.  One shape a family of kernels: rows
-# in tensor memory and one tile a warp, two tiles a warp, 8 x 128 tiles, 32 x 32 tiles, slabs, bands, rows too wide for both; float64.
+# in tensor memory and one tile a warp, two tiles a warp, 8 x 128 tiles, 32 x 32 tiles, slabs, column bands (rows too wide, filters too
+# many for those), float64.
 @pytest.mark.parametrize("far,exact", [(2.0 ** 31, True), (3e38, True), (3e9, False), (float("inf"), False)])
 @pytest.mark.parametrize("shape,dtype", [((1, 80, 4, 64, 128), torch.float32), ((1, 150, 4, 128, 128), torch.bfloat16), ((1, 2, 4, 128, 256), torch.float32),
                                          ((2, 2, 3, 60, 120), torch.float32), ((1, 3, 2, 40, 50), torch.float32), ((1, 2, 4, 150, 300), torch.float32),
