@@ -64,7 +64,7 @@ enum KernelId {
     KID_INTEGRAL = 1, KID_FORWARD_GLOBAL, KID_BACKWARD_GLOBAL, KID_FINISH_PARAM_GRADS, KID_CLIP,
     KID_FORWARD_PLANE, KID_BACKWARD_PLANE, KID_SUM_CHUNKS, KID_BACKWARD_BAND, KID_INTEGRAL_BANDS, KID_FORWARD_BAND,
     KID_FORWARD_SLAB, KID_BACKWARD_SLAB, KID_FORWARD_QUAD, KID_BACKWARD_QUAD,
-    KID_FORWARD_TMEM, KID_FORWARD_TMEM_STREAM, KID_BACKWARD_QUAD_PAIR, KID_COUNT
+    KID_FORWARD_TMEM, KID_FORWARD_TMEM_STREAM, KID_BACKWARD_QUAD_PAIR, KID_BACKWARD_SQUARE, KID_COUNT
 };
 
 // Put around a kernel launch: counts it and, while profiling is enabled, records a CUDA event on
@@ -164,8 +164,8 @@ int launch_forward_plane_fused(const float *x, const BoxParams &bp, const Fusion
 // Shared-memory-resident path for small planes (box_plane_smem.cu).
 bool plane_path_fits_forward(int F, int h, int w);
 bool plane_path_fits_backward(int F, int h, int w);
-bool plane_path_prefers_global_forward_integ(int64_t planes, int F, int h, int w);
 bool plane_path_prefers_slabs_backward(int64_t planes, int F, int h, int w);
+bool plane_path_prefers_global_forward_integ(int64_t planes, int F, int h, int w);
 int launch_forward_plane(const float *x, const BoxParams &bp, float *out, int N, int C, int F, int h,
                          int w, bool normalize, bool exact, cudaStream_t s);
 // partials: C*F*N*5 floats
@@ -175,12 +175,17 @@ int launch_backward_plane(const float *x, const float *grad_output, const BoxPar
                           cudaStream_t s);
 
 // From the input's integral image (plain rows) instead of the input.
-bool plane_path_fits_backward_integ(int F, int h, int w);
 int launch_forward_plane_integ(const float *integ, const BoxParams &bp, float *out, int N, int C, int F, int h, int w,
                                bool normalize, bool exact, cudaStream_t s);
 int launch_backward_plane_integ(const float *x_integ, const float *grad_output, const BoxParams &bp, float rep_h, float rep_w,
                                 int N, int C, int F, int h, int w, bool normalize, bool exact, int need_mask, float *grad_input,
                                 float *grad_params, float *partials, cudaStream_t s);
+
+// Whole planes of any width (box_flat.cu); exactly one of x and x_integ (plain rows, float only) is given.
+bool flat_fits_backward(int F, int h, int w);
+int launch_backward_flat(const void *x, const float *x_integ, int io_kind, const void *grad_output, const BoxParams &bp, float rep_h, float rep_w, int N,
+                         int C, int F, int h, int w, bool normalize, bool exact, int need_mask, void *grad_input, void *grad_params,
+                         int grad_params_kind, float *partials, cudaStream_t s);
 
 int read_wait_timeouts(int *count);
 int read_wait_timeouts_narrow(int *count);

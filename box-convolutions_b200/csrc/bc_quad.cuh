@@ -135,7 +135,8 @@ __device__ __forceinline__ void quad_taps(const QuadCols &c, uint32_t row0, uint
 }
 
 // Column-combined values of a tap-row pair: d = (1-f_hi) h[m] + f_hi h[m+1] - (1-f_lo) l[m+1] - f_lo l[m].
-__device__ __forceinline__ void quad_pair(const QuadCols &c, uint32_t row0, uint32_t row1, const ColW2 &cw, f2_t (&d)[kStrip])
+template <class Cols>
+__device__ __forceinline__ void quad_pair(const Cols &c, uint32_t row0, uint32_t row1, const ColW2 &cw, f2_t (&d)[kStrip])
 {
     f2_t l[kStrip + 1], h[kStrip + 1];
     quad_taps(c, row0, row1, l, h);
@@ -144,7 +145,8 @@ __device__ __forceinline__ void quad_pair(const QuadCols &c, uint32_t row0, uint
         d[m] = fma2(cw.nfl, l[m], fma2(cw.nwl, l[m + 1], fma2(cw.fh, h[m + 1], mul2(cw.wh, h[m]))));
 }
 // The same plus the one-column strips outside the box: el = l[m+1] - l[m], eh = h[m+1] - h[m].
-__device__ __forceinline__ void quad_pair_e(const QuadCols &c, uint32_t row0, uint32_t row1, const ColW2 &cw, f2_t (&d)[kStrip],
+template <class Cols>
+__device__ __forceinline__ void quad_pair_e(const Cols &c, uint32_t row0, uint32_t row1, const ColW2 &cw, f2_t (&d)[kStrip],
                                             f2_t (&el)[kStrip], f2_t (&eh)[kStrip])
 {
     f2_t l[kStrip + 1], h[kStrip + 1];
@@ -190,8 +192,8 @@ __device__ __forceinline__ float warp_sum5(const float (&v)[kNumSums], int lane)
 // leave three or two CTAs an SM and the tiles are full, of one column ((256,32,4,64,128): 504 us, scalar 522; (32,32,4,64,128) in
 // bfloat16 71 and 74; with two columns it costs 0.5 to 1 %).  Where rows are cut or unaligned, scalars ((60,16,4,40,250): 140 us in pairs, 131).
 // The same values either way.
-template <int R, bool NEED_PARAMS, bool FULL, bool PACKED = false, class Rows, class Cells>
-__device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const QuadCols &cols, const Rows &q, const ColW2 &cw,
+template <int R, bool NEED_PARAMS, bool FULL, bool PACKED = false, bool LANES = false, class Cols, class Rows, class Cells>
+__device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Cols &cols, const Rows &q, const ColW2 &cw,
                                                     Cells &&at, float (&sums)[kNumSums], int rows)
 {
     f2_t pd[kStrip];
@@ -266,7 +268,7 @@ __device__ __forceinline__ void quad_backward_strip(const BoxTaps &t, const Quad
                 out2 = fma2(pack2(e.x, e.y), g01, fma2(pack2(e.z, e.w), g23, out2));
                 at.add(i, g01, g23, scale);
 #pragma unroll
-                for (int m = 0; m < kStrip; ++m) pd[m] = cd[m];
+                for (int m = 0; m < kStrip; ++m) pd[m] = !LANES || i + 1 < rows ? cd[m] : pack2(0.f, 0.f);
                 if (i + 1 < R) e = below;
             }
         }

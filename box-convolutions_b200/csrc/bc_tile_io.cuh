@@ -64,6 +64,7 @@ struct Io;
 
 template <>
 struct Io<float> {
+    static constexpr int kKind = BC_IO_F32;
     static constexpr int kVecBytes = 16;
     static __device__ __forceinline__ float4 load4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
     static __device__ __forceinline__ float load1(const float *p) { return __ldg(p); }
@@ -86,6 +87,7 @@ __device__ __forceinline__ uint2 lds64(uint32_t a)
 
 template <>
 struct Io<__half> {
+    static constexpr int kKind = BC_IO_F16;
     static constexpr int kVecBytes = 8;
     static __device__ __forceinline__ float4 widen(uint2 r)
     {
@@ -109,6 +111,7 @@ struct Io<__half> {
 
 template <>
 struct Io<__nv_bfloat16> {
+    static constexpr int kKind = BC_IO_BF16;
     static constexpr int kVecBytes = 8;
     static __device__ __forceinline__ float4 widen(uint2 r)
     {

@@ -1,16 +1,14 @@
-// Shared-memory-resident kernels in tiles of 32 x 32, for planes small enough to keep on chip that are too narrow (64
-// columns) or too large for the quad layout's tiles of 8 x 128, or waste less in these (quad_prefers_forward() and
-// quad_pair_suits_backward() in box_quad_plane.cuh).  HBM traffic is the compulsory minimum: the forward
-// reads the input once and writes the output once; the backward reads the input and grad_output
+// Shared-memory-resident kernels in tiles of 32 x 32, for planes small enough to keep on chip that waste less in these than in
+// tiles of 8 x 128 (quad_prefers_forward() in box_quad_plane.cuh), or by strips dealt out to lanes (bc_flat.cuh).  HBM traffic is
+// the compulsory minimum: the forward reads the input once and writes the output once; the backward reads the input and grad_output
 // once and writes grad_input once.  No integral image ever goes to global memory.
 //
 // Forward : one CTA per (plane, group of filters).  The plane's integral image is built in shared
 //           memory, then every thread walks its 4-column x 8-row strip (bc_walk.cuh scheme) for
 //           each filter of the group and writes 128-bit rows of the output.
 // Backward: one CTA per plane.  For each filter the grad_output plane is integrated in shared memory and
-//           gathered with the mirrored box.  The input plane waits in shared memory, in tensor memory or nowhere
-//           (enum XAt), grad-input accumulates over the filters in registers or beside it in tensor memory.  The
-//           five sums that finish the parameter gradients are reduced per CTA and left for
+//           gathered with the mirrored box.  The input plane waits in shared memory, grad-input accumulates over the filters in
+//           registers.  The five sums that finish the parameter gradients are reduced per CTA and left for
 //           finish_param_grads_kernel or the channel's last CTA (bc_finish.cuh).
 //
 // Thread layout (same for building the integral image and for gathering): a warp owns a tile of
@@ -28,9 +26,9 @@
 // exchange row totals through shared memory; the same again down the columns.  The block is then
 // stored with the layout above (conflict-free).
 //
-// The kernels are instantiated twice: FAST for planes whose height is a multiple of 8 and width
+// The forward is instantiated twice: FAST for planes whose height is a multiple of 8 and width
 // a multiple of 4 with aligned tensors (no per-row guards, one vector access per strip row), and
-// a guarded version for everything else.
+// a guarded version for everything else.  The backward serves the former only.
 //
 // This file holds the kernels and their launchers as templates over the storage type of the big
 // tensors (Io<> below); box_plane_smem.cu instantiates them for float, box_plane_half.cu for
@@ -421,21 +419,16 @@ forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, 
     }
 }
 
-// T = warp tiles per warp: grad-input accumulators are registers, so the number of strips a thread owns is a
-// compile-time constant.
-// X_AT: where the input plane waits.  In shared memory; or nowhere, its values being read from global memory as they
-// are needed, which lets planes of up to ~48 000 pixels use this kernel; or, with the accumulators, in tensor memory
-// (bc_tmem.cuh, T = 2), where that makes room for a second CTA on the SM.
-enum XAt { X_SHARED, X_GLOBAL, X_TENSOR };
+// Backward of aligned planes of up to eight tiles, one a warp (flat_beats_square() says which).
+// The input plane waits in shared memory, float whatever IO is: float planes arrive by a bulk copy when STAGED, narrow ones are
+// converted by the threads as they are copied in.
 // STAGED: the input plane and each grad_output plane arrive in shared memory by asynchronous bulk
 // copies (one instruction per plane, issued by one thread); the copy of the next grad_output
 // plane runs while the current one is gathered.
-// The input plane in shared memory is float whatever IO is: float planes arrive by a bulk copy when
-// STAGED, narrow ones are converted by the threads as they are copied in.
 // INTEG: the input is given as its integral image (instantiations of their own: as a run-time branch it cost the others 5 %).
-template <typename IO, int T, bool FAST, bool STAGED, bool NEED_PARAMS, XAt X_AT = X_SHARED, bool COUNTED = false, bool INTEG = false>
+template <typename IO, bool STAGED, bool NEED_PARAMS, bool COUNTED = false, bool INTEG = false>
 __global__ void __launch_bounds__(512)
-backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const IO *__restrict__ grad_output, BoxParams bp,
+backward_square_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ, const IO *__restrict__ grad_output, BoxParams bp,
                       IO *__restrict__ grad_input, float *__restrict__ partials, int N, int C, int F,
                       int h, int w, bool normalize, bool exact, bool write_gin, Finish fin)
 {
@@ -445,10 +438,9 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
     float *sI = reinterpret_cast<float *>(smem4);          // integral(grad_output plane)
     float *sRow = sI + layout_floats(h, w);
     float *sCol = sRow + g.ntiles * kTile;
-    float *sX = sCol + g.ntiles * kTile;                   // the input plane, pitch w (XSMEM)
-    constexpr bool X_BY_COPY = STAGED && IsFloat<IO>::value, TMEM = X_AT == X_TENSOR, XSMEM = NEED_PARAMS && X_AT == X_SHARED;
-    float *sG = sX + (XSMEM ? npix : 0);                   // staged grad_output plane, as stored (STAGED)
-    __shared__ uint32_t tmem_base;
+    float *sX = sCol + g.ntiles * kTile;                   // the input plane, pitch w (NEED_PARAMS)
+    constexpr bool X_BY_COPY = STAGED && IsFloat<IO>::value;
+    float *sG = sX + (NEED_PARAMS ? npix : 0);             // staged grad_output plane, as stored (STAGED)
     __shared__ __align__(16) float sTaps[kMaxFilters * kTapWords];
     __shared__ float red[16][kNumSums];
     __shared__ __align__(8) unsigned long long mbar[2];
@@ -464,9 +456,7 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
     const uint32_t plane_bytes = (uint32_t)npix * (uint32_t)sizeof(IO);
     bool timed_out = false;
 
-    Strip st[T];
-#pragma unroll
-    for (int k = 0; k < T; ++k) st[k] = make_strip(g, sI32, warp + k * nwarps, cg, rg);
+    Strip st[1] = {make_strip(g, sI32, warp, cg, rg)};
 
     // The first copies are started as early as possible, by a thread of the second warp (when there is
     // one) so that they do not queue behind the box arithmetic of the first warp's threads.  That thread
@@ -495,72 +485,30 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
         const Box box = load_box(bp, c * F + tid);
         store_taps(sTaps + tid * kTapWords, taps_mirrored(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
     }
-    __syncwarp();
-    if (TMEM && warp == nwarps - 1) tmem_alloc(&tmem_base, tmem_columns<T>(nwarps));
-    if (STAGED || TMEM) __syncthreads();                   // barriers initialised before anyone waits
-    if (TMEM) {
-        tmem_acquire();
-        const IO *xp = x + nc * (int64_t)npix;
-        const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1);
-#pragma unroll
-        for (int k = 0; k < T; ++k) {
-            if (!st[k].tile) continue;
-            TmemRows<0, T> kept(tmem_base, warp, k);
-#pragma unroll
-            for (int i = 0; i < kR; ++i) {
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (st[k].active && (FAST || st[k].p0 + i < h)) {
-                    if (INTEG) {      // the caller has only the input's integral image: its pixels are second differences
-                        const float *Ip = I + (int64_t)(st[k].p0 + i) * (w + 1) + st[k].q0;
-                        v.x = pixel_of_integral(Ip, w + 1);
-                        if (st[k].q0 + 1 < w) v.y = pixel_of_integral(Ip + 1, w + 1);
-                        if (st[k].q0 + 2 < w) v.z = pixel_of_integral(Ip + 2, w + 1);
-                        if (st[k].q0 + 3 < w) v.w = pixel_of_integral(Ip + 3, w + 1);
-                    } else if (FAST) {
-                        v = Io<IO>::load4(xp + st[k].pix + i * w);
-                    } else {
-                        const IO *row = xp + st[k].pix + i * w;
-                        v.x = Io<IO>::load1(row);
-                        if (st[k].q0 + 1 < w) v.y = Io<IO>::load1(row + 1);
-                        if (st[k].q0 + 2 < w) v.z = Io<IO>::load1(row + 2);
-                        if (st[k].q0 + 3 < w) v.w = Io<IO>::load1(row + 3);
-                    }
-                }
-                kept.init(i, v);
-            }
-        }
-        tmem_wait_store();
-    }
-    if (XSMEM && INTEG) {
+    if (STAGED) __syncthreads();                           // barriers initialised before anyone waits
+    if (NEED_PARAMS && INTEG) {
         // (read by the first gather, which follows the barriers of the first build)
         const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1);
         for (int p = warp; p < h; p += nwarps)
             for (int q = lane; q < w; q += 32) sX[p * w + q] = pixel_of_integral(I + p * (w + 1) + q, w + 1);
-    } else if (!X_BY_COPY && XSMEM) {
+    } else if (!X_BY_COPY && NEED_PARAMS) {
         // (read by the first gather, which follows the barriers of the first build)
         const IO *xp = x + nc * (int64_t)npix;
-        if (FAST) {
-            for (int i = tid; i < (npix >> 2); i += blockDim.x)
-                reinterpret_cast<float4 *>(sX)[i] = Io<IO>::load4(xp + 4 * i);
-        } else {
-            for (int i = tid; i < npix; i += blockDim.x) sX[i] = Io<IO>::load1(xp + i);
-        }
+        for (int i = tid; i < (npix >> 2); i += blockDim.x) reinterpret_cast<float4 *>(sX)[i] = Io<IO>::load4(xp + 4 * i);
     }
 
-    float gin[T][kR][kStrip];
+    float gin[kR][kStrip];
 #pragma unroll
-    for (int k = 0; k < T; ++k)
+    for (int i = 0; i < kR; ++i)
 #pragma unroll
-        for (int i = 0; i < kR; ++i)
-#pragma unroll
-            for (int m = 0; m < kStrip; ++m) gin[k][i][m] = 0.0f;
+        for (int m = 0; m < kStrip; ++m) gin[i][m] = 0.0f;
 
     for (int f = 0; f < F; ++f) {
         // (the barrier that ends the previous iteration protects sI, sRow, sCol)
         {
-            Blocks<T> blk;
+            Blocks<1> blk;
             if (STAGED) timed_out |= !mbar_wait(mbarG, f & 1);
-            build_rows<IO, T, FAST, STAGED>(blk, st, gbase + f * (int64_t)npix, sG32, sRow, g, cg, rg);
+            build_rows<IO, 1, true, STAGED>(blk, st, gbase + f * (int64_t)npix, sG32, sRow, g, cg, rg);
             if (STAGED && tid == 0 && f + 1 < F) {
                 // every thread has taken its block out of the staging buffer (barrier above)
                 fence_proxy_async();
@@ -568,16 +516,13 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
                 // the plane after that one on its way to L2 already (about 1 % on 256-sample batches)
                 if (f + 2 < F) bulk_prefetch_l2(gbase + (f + 2) * (int64_t)npix, plane_bytes);
             }
-            build_columns<T, FAST>(blk, st, sRow, sCol, g, cg, rg);
+            build_columns<1, true>(blk, st, sRow, sCol, g, cg, rg);
         }
         if (!STAGED && f + 1 < F && cg == 0) {
             // pull the next grad_output plane towards L2 while this one is gathered
 #pragma unroll
-            for (int k = 0; k < T; ++k)
-#pragma unroll
-                for (int i = 0; i < kR; ++i)
-                    if (st[k].active && st[k].p0 + i < h)
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(gbase + (f + 1) * (int64_t)npix + st[k].pix + i * w));
+            for (int i = 0; i < kR; ++i)
+                if (st[0].active) asm volatile("prefetch.global.L2 [%0];" ::"l"(gbase + (f + 1) * (int64_t)npix + st[0].pix + i * w));
         }
         if (X_BY_COPY && NEED_PARAMS && !INTEG && f == 0) timed_out |= !mbar_wait(mbarX, 0);
 
@@ -590,98 +535,61 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
         float s_out = 0.f;
         f2_t topbot2 = pack2(0.f, 0.f);
         f2_t leftP = pack2(0.f, 0.f), leftQ = pack2(0.f, 0.f), rightP = pack2(0.f, 0.f), rightQ = pack2(0.f, 0.f);
+        if (st[0].active) {
+            const int p0 = st[0].p0;
+            const Walk wk = make_walk(sI32, t, st[0].q0, g);
+            if (NEED_PARAMS) {
+                f2_t pd[kStrip], pel[kStrip], peh[kStrip];
+                load_pair_e(wk, p0 + t.lo_r - 1, p0 + t.hi_r, cw, pd, pel, peh);
+                uint32_t xa = sX32 + st[0].pix * 4;
 #pragma unroll
-        for (int k = 0; k < T; ++k) {
-            if (TMEM ? st[k].tile : st[k].active) {
-                const Walk wk = make_walk(sI32, t, st[k].q0, g);
-                if (NEED_PARAMS) {
-                    TmemRows<0, T> kept(TMEM ? tmem_base : 0u, warp, k);
-                    f2_t pd[kStrip], pel[kStrip], peh[kStrip];
-                    if (!TMEM || st[k].active) load_pair_e(wk, st[k].p0 + t.lo_r - 1, st[k].p0 + t.hi_r, cw, pd, pel, peh);
-                    uint32_t xa = sX32 + st[k].pix * 4;
-                    const IO *xg = x + nc * (int64_t)npix + st[k].pix;         // X_GLOBAL
+                for (int i = 0; i < kR; ++i) {
+                    f2_t cd[kStrip], cel[kStrip], ceh[kStrip];
+                    load_pair_e(wk, p0 + i + t.lo_r, p0 + i + t.hi_r + 1, cw, cd, cel, ceh);
+                    const float4 x4 = lds128(xa);
+                    const float xv[kStrip] = {x4.x, x4.y, x4.z, x4.w};
+                    xa += w * 4;
 #pragma unroll
-                    for (int i = 0; i < kR; ++i) {
-                        const int p = st[k].p0 + i;
-                        const bool there = (!TMEM || st[k].active) && (FAST || p < h);
-                        f2_t cd[kStrip], cel[kStrip], ceh[kStrip];
-                        float xv[kStrip], gg[kStrip];
-                        if (TMEM) {
-                            __syncwarp();
-                            kept.fetch(i);
-                        }
-                        if (there) load_pair_e(wk, p + t.lo_r, p + t.hi_r + 1, cw, cd, cel, ceh);
-                        if (TMEM) {
-                            __syncwarp();
-                            const float4 v = kept.next();
-                            xv[0] = v.x; xv[1] = v.y; xv[2] = v.z; xv[3] = v.w;
-                        }
-                        if (there) {
-                            if (TMEM) {
-                            } else if (FAST) {
-                                const float4 v = XSMEM ? lds128(xa) : Io<IO>::load4(xg);
-                                xv[0] = v.x; xv[1] = v.y; xv[2] = v.z; xv[3] = v.w;
-                            } else {
-#pragma unroll
-                                for (int m = 0; m < kStrip; ++m) xv[m] = st[k].q0 + m < w ? (XSMEM ? sX[p * w + st[k].q0 + m] : Io<IO>::load1(xg + m)) : 0.0f;
-                            }
-                            xa += w * 4;
-                            xg += w;
-#pragma unroll
-                            for (int m = 0; m < kStrip; ++m) {
-                                const f2_t xx = pack2(xv[m], xv[m]);
-                                float lo_new, hi_new, lo_old, hi_old, top, bot;
-                                // d: gather value and the two row strips
-                                const f2_t dd = sub2(cd[m], pd[m]);
-                                unpack2(cd[m], lo_new, hi_new);
-                                unpack2(pd[m], lo_old, hi_old);
-                                unpack2(dd, top, bot);
-                                gg[m] = (hi_old - lo_new) + t.f_hi_r * bot + t.f_lo_r * top;
-                                topbot2 = fma2(xx, dd, topbot2);
-                                s_out += xv[m] * gg[m];
-                                if (!TMEM) gin[k][i][m] += gg[m] * t.scale;
-                                // e_lo / e_hi: the two column strips
-                                leftP = fma2(xx, pel[m], leftP);
-                                leftQ = fma2(xx, cel[m], leftQ);
-                                rightP = fma2(xx, peh[m], rightP);
-                                rightQ = fma2(xx, ceh[m], rightQ);
-                                pd[m] = cd[m]; pel[m] = cel[m]; peh[m] = ceh[m];
-                            }
-                        }
-                        if (TMEM) {
-                            if (there) {
-                                kept.g.x += gg[0] * t.scale; kept.g.y += gg[1] * t.scale;
-                                kept.g.z += gg[2] * t.scale; kept.g.w += gg[3] * t.scale;
-                            }
-                            __syncwarp();
-                            tmem_store4(kept.base + 8 * i, kept.g);
-                        }
+                    for (int m = 0; m < kStrip; ++m) {
+                        const f2_t xx = pack2(xv[m], xv[m]);
+                        float lo_new, hi_new, lo_old, hi_old, top, bot;
+                        // d: gather value and the two row strips
+                        const f2_t dd = sub2(cd[m], pd[m]);
+                        unpack2(cd[m], lo_new, hi_new);
+                        unpack2(pd[m], lo_old, hi_old);
+                        unpack2(dd, top, bot);
+                        const float gg = (hi_old - lo_new) + t.f_hi_r * bot + t.f_lo_r * top;
+                        topbot2 = fma2(xx, dd, topbot2);
+                        s_out += xv[m] * gg;
+                        gin[i][m] += gg * t.scale;
+                        // e_lo / e_hi: the two column strips
+                        leftP = fma2(xx, pel[m], leftP);
+                        leftQ = fma2(xx, cel[m], leftQ);
+                        rightP = fma2(xx, peh[m], rightP);
+                        rightQ = fma2(xx, ceh[m], rightQ);
+                        pd[m] = cd[m]; pel[m] = cel[m]; peh[m] = ceh[m];
                     }
-                } else {
-                    f2_t prev[kStrip];
-                    load_pair(wk, st[k].p0 + t.lo_r - 1, st[k].p0 + t.hi_r, cw, prev);
+                }
+            } else {
+                f2_t prev[kStrip];
+                load_pair(wk, p0 + t.lo_r - 1, p0 + t.hi_r, cw, prev);
 #pragma unroll
-                    for (int i = 0; i < kR; ++i) {
-                        const int p = st[k].p0 + i;
-                        if (FAST || p < h) {
-                            f2_t cur[kStrip];
-                            load_pair(wk, p + t.lo_r, p + t.hi_r + 1, cw, cur);
+                for (int i = 0; i < kR; ++i) {
+                    f2_t cur[kStrip];
+                    load_pair(wk, p0 + i + t.lo_r, p0 + i + t.hi_r + 1, cw, cur);
 #pragma unroll
-                            for (int m = 0; m < kStrip; ++m) {
-                                float b, dd, a, cc, top, bot;
-                                unpack2(cur[m], b, dd);
-                                unpack2(prev[m], a, cc);
-                                unpack2(sub2(cur[m], prev[m]), top, bot);
-                                gin[k][i][m] += ((cc - b) + t.f_hi_r * bot + t.f_lo_r * top) * t.scale;
-                                (void)a; (void)dd;
-                                prev[m] = cur[m];
-                            }
-                        }
+                    for (int m = 0; m < kStrip; ++m) {
+                        float b, dd, a, cc, top, bot;
+                        unpack2(cur[m], b, dd);
+                        unpack2(prev[m], a, cc);
+                        unpack2(sub2(cur[m], prev[m]), top, bot);
+                        gin[i][m] += ((cc - b) + t.f_hi_r * bot + t.f_lo_r * top) * t.scale;
+                        (void)a; (void)dd;
+                        prev[m] = cur[m];
                     }
                 }
             }
         }
-        if (TMEM) tmem_wait_store();
         if (NEED_PARAMS) {
             float tb_top, tb_bot, la, lc, lb, ld, ra, rc, rb, rd;
             unpack2(topbot2, tb_top, tb_bot);
@@ -709,37 +617,10 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
     }
     if (STAGED && timed_out && lane == 0) atomicAdd(&g_wait_timeouts, 1);
 
-    if (write_gin) {
-        IO *gi = grad_input + nc * (int64_t)npix;
+    if (write_gin && st[0].active) {
+        IO *dst = grad_input + nc * (int64_t)npix + st[0].pix;
 #pragma unroll
-        for (int k = 0; k < T; ++k) {
-            if (TMEM && st[k].tile) {
-                TmemRows<0, T> kept(tmem_base, warp, k);
-#pragma unroll
-                for (int i = 0; i < kR; ++i) {
-                    const float4 v = kept.grad_input(i);
-                    gin[k][i][0] = v.x; gin[k][i][1] = v.y; gin[k][i][2] = v.z; gin[k][i][3] = v.w;
-                }
-            }
-            if (st[k].active) {
-                IO *dst = gi + st[k].pix;
-#pragma unroll
-                for (int i = 0; i < kR; ++i) {
-                    if (FAST) {
-                        Io<IO>::store4(dst + i * w, gin[k][i][0], gin[k][i][1], gin[k][i][2], gin[k][i][3]);
-                    } else if (st[k].p0 + i < h) {
-#pragma unroll
-                        for (int m = 0; m < kStrip; ++m)
-                            if (st[k].q0 + m < w) Io<IO>::store1(dst + i * w + m, gin[k][i][m]);
-                    }
-                }
-            }
-        }
-    }
-    if (TMEM) {
-        tmem_release();
-        __syncthreads();
-        if (warp == 0) tmem_free(tmem_base, tmem_columns<T>(nwarps));
+        for (int i = 0; i < kR; ++i, dst += w) Io<IO>::store4(dst, gin[i][0], gin[i][1], gin[i][2], gin[i][3]);
     }
     if (COUNTED) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
 }
@@ -771,13 +652,6 @@ inline bool plane_fits_forward(int F, int h, int w)
     return F <= kMaxFilters && warp_tiles(h, w) <= kMaxTiles && plane_forward_smem_bytes(h, w) <= kMaxSmem;
 }
 
-// Backward from the input's integral image: the kernels that keep the input plane in shared memory.
-inline bool plane_fits_backward_integ(int F, int h, int w)
-{
-    return F <= kMaxFilters && warp_tiles(h, w) <= kMaxTiles &&
-           (quad_fits_backward(F, h, w) || plane_backward_smem_bytes(h, w, true, false, 4) <= kMaxSmem);
-}
-
 // Forward from the input's integral image: copying it to shared memory pays where several filters, or several CTAs an
 // SM, share the copy's latency ((4,16,4,96,160): 13 us, straight from global memory 23; 3060 planes of 120 x 56, F = 3: 96, 316).
 // Not for one or two filters of large planes, which have an SM to themselves ((83,20,1,97,199): 180 against 115;
@@ -789,17 +663,42 @@ inline bool plane_prefers_global_forward_integ(int64_t planes, int F, int h, int
     return (F <= 2 && tiles >= 16) || (planes * 8 <= 148 && tiles >= 12);
 }
 
-// From the input's integral image, planes of more than 8 tiles of 32 x 32, which occupy an SM alone in the backward
-// kernel of this file, are better off as slabs where they are wide enough ((4,16,4,96,160): 36 us against 48) or leave
-// half of the SMs idle ((1,17,8,143,44): 32 us against 82, (5,4,4,216,56): 28 against 58; (22,15,2,136,40): 54 against 48).
+// (Planes of more than 32 tiles of 32 x 32 would fit the kernel that deals out strips in part; with 25 to 32 tiles of its own it is no better than slabs.)
+inline bool plane_fits_backward(int F, int h, int w) { return warp_tiles(h, w) <= kMaxTiles && flat_fits_backward(F, h, w); }
+
+// From the input's integral image, large planes are better off as slabs where they are wide enough or leave half of
+// the SMs idle ((4,16,4,96,160): 36 us against 48; (1,17,8,143,44): 32 us against 82, (5,4,4,216,56): 28 against 58).
 inline bool plane_prefers_slabs_backward(int64_t planes, int F, int h, int w)
 {
     return (w > 96 || planes <= 74) && warp_tiles(h, w) > 8 && !quad_fits_backward(F, h, w);
 }
 
-inline bool plane_fits_backward(int F, int h, int w)
+// On which planes the kernel that deals out strips (box_flat.cu) is faster than those with fixed tiles: it has fewer lanes without a
+// pixel, and a fifth more instructions a strip.  `strips`: a 32nd of its tiles.  The rules ask for sides and filters only,
+// so that a part of a batch runs on the kernel of the whole.  Samples, channels, filters, rows, columns:
+// against 8 x 128 tiles (795,2,4,40,150) 201 us -> 130; (2611,1,4,120,72) 438 -> 308; (202,3,4,48,144) 83 -> 64; but (1265,1,2,56,96), 7 tiles
+// for 5.25, 53.6 -> 56.8; (2104,1,4,80,120), 10 for 9.4, 213 -> 260; (111,8,6,86,126) 179 -> 209;
+// against pairs of them (575,1,4,128,72) 88 -> 76; (593,1,4,72,168) 166 -> 103; (653,1,8,80,240), 20 for 18.8, 318 -> 404; with one or two filters a wash;
+// against 32 x 32 tiles, more than eight: always (below); fewer, aligned: (1042,1,8,72,40) 144 -> 83; (64,40), 4 for 2.5, 61 -> 62, with fewer
+// planes 1.1 to 1.4 times as long; unaligned (2857,1,6,47,36) 233 -> 106, (2858,1,4,110,36) in bfloat16 424 -> 149.
+inline bool flat_beats_quad(int F, int h, int w)
 {
-    return F <= kMaxFilters && warp_tiles(h, w) <= kMaxTiles && plane_backward_smem_bytes(h, w, false, false, 4) <= kMaxSmem;
+    const int tiles = quad_row_tiles(h) * quad_col_tiles(w), strips = ((w + 3) / 4) * ((h + 7) / 8);
+    if (tiles <= 8) return F > 1 && tiles * 32 * 10 > strips * 16;
+    if (strips > 12 * 32) return tiles * 32 * 10 > strips * 12;
+    return tiles * 32 * 10 > strips * (w % 4 || h % 8 ? 13 : 15);
+}
+inline bool flat_beats_pair(int F, int h, int w)
+{
+    const int tiles = quad_row_tiles(h) * quad_col_tiles(w), strips = ((w + 3) / 4) * ((h + 7) / 8);
+    if (F <= 2) return false;
+    if (tiles <= kQuadMaxWarps) return tiles * 32 * 20 > strips * 27;
+    return strips <= 24 * 32 && tiles * 32 * 20 > strips * 25;
+}
+inline bool flat_beats_square(int F, int h, int w)
+{
+    const int tiles = warp_tiles(h, w), strips = ((w + 3) / 4) * ((h + 7) / 8);
+    return F > 1 && tiles > 4 && tiles * 32 * 10 > strips * 17;
 }
 
 // `fu` (inference steps around the gather) exists for float tensors only.
@@ -857,77 +756,57 @@ int launch_backward_plane_t(const IO *x, const float *x_integ, const IO *grad_ou
                             int C, int F, int h, int w, bool normalize, bool exact, int need_mask, IO *grad_input,
                             void *grad_params, int grad_params_kind, float *partials, cudaStream_t s)
 {
-    if (x && quad_pair_suits_backward((int64_t)N * C, F, h, w, IsFloat<IO>::value) && aligned_to(x, Io<IO>::kVecBytes) && aligned_to(grad_output, 16) &&
-        (!(need_mask & BC_NEED_INPUT) || aligned_to(grad_input, Io<IO>::kVecBytes)))
-        return launch_backward_quad_pair_t<IO>(x, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input, grad_params,
-                                               grad_params_kind, partials, s);
-    if (quad_fits_backward(F, h, w))
-        return launch_backward_quad_t<IO>(x, x_integ, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
-                                          grad_params, grad_params_kind, partials, s);
     const int64_t planes = (int64_t)N * C;
     if (planes > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
     const bool need_params = (need_mask & (BC_NEED_ALL & ~BC_NEED_INPUT)) != 0;
     const bool write_gin = (need_mask & BC_NEED_INPUT) != 0;
-    const int tiles = warp_tiles(h, w);
-    const int T = tiles > 8 ? 2 : 1;
-    const int warps = (tiles + T - 1) / T;
     const int vec = Io<IO>::kVecBytes;
-    const size_t io = sizeof(IO);
+    const bool pair = x && quad_pair_suits_backward(planes, F, h, w, IsFloat<IO>::value) && aligned_to(x, vec) && aligned_to(grad_output, 16) &&
+                      (!write_gin || aligned_to(grad_input, vec));
+    if (pair && !flat_beats_pair(F, h, w))
+        return launch_backward_quad_pair_t<IO>(x, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input, grad_params,
+                                               grad_params_kind, partials, s);
+    if (!pair && quad_fits_backward(F, h, w) && !flat_beats_quad(F, h, w))
+        return launch_backward_quad_t<IO>(x, x_integ, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
+                                          grad_params, grad_params_kind, partials, s);
     const bool fast = (h % kR == 0) && (w % kStrip == 0) && aligned_to(x, vec) && aligned_to(grad_output, vec) &&
                       (!write_gin || aligned_to(grad_input, vec));
+    const int tiles = warp_tiles(h, w);
+    if (!fast || w >= kQuadMinWidth || tiles > 8 || flat_beats_square(F, h, w))
+        return launch_backward_flat(x, x_integ, Io<IO>::kKind, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
+                                    grad_params, grad_params_kind, partials, s);
+    const size_t io = sizeof(IO);
     // bulk copies need 16-byte aligned planes of a multiple of 16 bytes and room for the staging buffer;
     // staging must not cost a resident CTA (two fit below ~112 KB each)
-    // More than eight tiles.  Rows that no vector access fits: the input plane goes to tensor memory, read once with scalar
-    // loads instead of once a filter from wherever it is ((16,32,4,100,200) backward 373 -> 314 us, (8,32,4,300,60) 189 -> 150).
-    // Else it joins the integral image in shared memory, unless the two then leave no room for a second CTA that there
-    // would be planes for: (24,32,4,96,160) 275 -> 220 us; both reasons: (16,32,4,93,157) 310 -> 173 us.  Where two CTAs fit
-    // anyway, or only one by its registers, tensor memory is slower: (8,16,4,128,256) 80 -> 90 us, a wait and
-    // two warp barriers a row.
     const size_t two_ctas = 112 * 1024;
-    const bool tensor = need_params && T > 1 &&
-                        (!fast || (warps <= 8 && planes > 148 && plane_backward_smem_bytes(h, w, true, false, io) > two_ctas &&
-                                   plane_backward_smem_bytes(h, w, false, false, io) <= two_ctas));
-    const bool xsmem = need_params && !tensor && plane_backward_smem_bytes(h, w, true, false, io) <= kMaxSmem;
-    const size_t with_staging = plane_backward_smem_bytes(h, w, xsmem, true, io);
-    const bool staged = fast && T == 1 && (xsmem || !need_params) && with_staging <= kMaxSmem && aligned_to(grad_output, 16) &&
-                        aligned_to(x, 16) && ((size_t)h * w * io) % 16 == 0 &&
-                        (with_staging <= two_ctas || plane_backward_smem_bytes(h, w, xsmem, false, io) > two_ctas);
-    const size_t smem = plane_backward_smem_bytes(h, w, xsmem, staged, io);
+    const size_t with_staging = plane_backward_smem_bytes(h, w, need_params, true, io);
+    const bool staged = with_staging <= kMaxSmem && aligned_to(grad_output, 16) && aligned_to(x, 16) && ((size_t)h * w * io) % 16 == 0 &&
+                        (with_staging <= two_ctas || plane_backward_smem_bytes(h, w, need_params, false, io) > two_ctas);
+    const size_t smem = plane_backward_smem_bytes(h, w, need_params, staged, io);
     void (*kern)(const IO *, const float *, const IO *, BoxParams, IO *, float *, int, int, int, int, int, bool, bool, bool, Finish);
     // With the input plane in shared memory, finishing here costs more than the launch it saves, from all but the
     // smallest problems on ((18,14,8,40,56): 41 us against 32 with the launch; (9,12,4,248,48): 67 against 53; (1,8,4,32,32): 17 against 14.5
-    // and 3 us of the host); in tensor memory it costs nothing.
+    // and 3 us of the host).
     const int64_t outputs = planes * F * h * w;
-    const bool may_finish = need_params && (tensor || (planes <= 148 && outputs <= 256 * 1024));
+    const bool may_finish = need_params && planes <= 148 && outputs <= 256 * 1024;
     const Finish fin = finish_here(bp, may_finish, planes, outputs, C, grad_params, grad_params_kind, need_mask, N, rep_h, rep_w, s);
-    auto pick = [&](auto counted, auto integ) {
-        constexpr bool K = decltype(counted)::value, I = decltype(integ)::value;
-        if (tensor) {
-            kern = fast ? backward_plane_kernel<IO, 2, true, false, true, X_TENSOR, K, I> : backward_plane_kernel<IO, 2, false, false, true, X_TENSOR, K, I>;
-        } else if (need_params && !xsmem) {
-            kern = backward_plane_kernel<IO, 2, true, false, true, X_GLOBAL, K>;      // (planes of up to eight tiles always fit; never from an integral image)
-        } else if (staged) {
-            kern = need_params ? backward_plane_kernel<IO, 1, true, true, true, X_SHARED, K, I> : backward_plane_kernel<IO, 1, true, true, false>;
-        } else if (fast) {
-            kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, true, false, true, X_SHARED, K, I> : backward_plane_kernel<IO, 1, true, false, false>)
-                          : (need_params ? backward_plane_kernel<IO, 2, true, false, true, X_SHARED, K, I> : backward_plane_kernel<IO, 2, true, false, false>);
-        } else {
-            kern = T == 1 ? (need_params ? backward_plane_kernel<IO, 1, false, false, true, X_SHARED, K, I> : backward_plane_kernel<IO, 1, false, false, false>)
-                          : backward_plane_kernel<IO, 2, false, false, false>;
-        }
+    auto pick = [&](auto copied) {
+        constexpr bool S = decltype(copied)::value;
+        if (!need_params) kern = backward_square_kernel<IO, S, false>;
+        else if (x_integ) kern = backward_square_kernel<IO, S, true, false, IsFloat<IO>::value>;      // (the four functions have no counters)
+        else kern = fin.total ? backward_square_kernel<IO, S, true, true> : backward_square_kernel<IO, S, true>;
     };
-    if (x_integ) pick(Flag<false>{}, Flag<IsFloat<IO>::value>{});      // (the four functions have no counters)
-    else if (fin.total) pick(Flag<true>{}, Flag<false>{});
-    else pick(Flag<false>{}, Flag<false>{});
+    if (staged) pick(Flag<true>{});
+    else pick(Flag<false>{});
     int st = opt_in_smem(kern, smem);
     if (st != BC_OK) return st;
     {
-        LaunchScope scope(KID_BACKWARD_PLANE, s);
-        if (cudaError_t e = launch_overlapped(kern, (unsigned)planes, warps * 32, smem, s, x, x_integ, grad_output, bp, grad_input,
+        LaunchScope scope(KID_BACKWARD_SQUARE, s);
+        if (cudaError_t e = launch_overlapped(kern, (unsigned)planes, tiles * 32, smem, s, x, x_integ, grad_output, bp, grad_input,
                                               partials, N, C, F, h, w, normalize, exact, write_gin, fin))
-            return cuda_failed(e, "backward_plane");
+            return cuda_failed(e, "backward_square");
     }
-    st = check_launch("backward_plane");
+    st = check_launch("backward_square");
     if (st != BC_OK || !need_params || fin.total) return st;
     return launch_finish_param_grads<float>(partials, bp, C * F, N, normalize, exact, rep_h, rep_w, need_mask,
                                             grad_params, s, grad_params_kind);

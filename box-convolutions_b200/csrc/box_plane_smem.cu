@@ -6,9 +6,8 @@ namespace bc {
 
 bool plane_path_fits_forward(int F, int h, int w) { return plane_fits_forward(F, h, w); }
 bool plane_path_fits_backward(int F, int h, int w) { return plane_fits_backward(F, h, w); }
-bool plane_path_prefers_global_forward_integ(int64_t planes, int F, int h, int w) { return plane_prefers_global_forward_integ(planes, F, h, w); }
 bool plane_path_prefers_slabs_backward(int64_t planes, int F, int h, int w) { return plane_prefers_slabs_backward(planes, F, h, w); }
-bool plane_path_fits_backward_integ(int F, int h, int w) { return plane_fits_backward_integ(F, h, w); }
+bool plane_path_prefers_global_forward_integ(int64_t planes, int F, int h, int w) { return plane_prefers_global_forward_integ(planes, F, h, w); }
 
 int launch_forward_plane(const float *x, const BoxParams &bp, float *out, int N, int C, int F, int h,
                          int w, bool normalize, bool exact, cudaStream_t s)

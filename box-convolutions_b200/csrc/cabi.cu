@@ -116,7 +116,7 @@ static bool slabs_suit(int64_t planes, int F, int h, int w) { return slab_path_f
 // faster all the same.)
 static bool plane_backward_integ(int64_t planes, int F, int h, int w)
 {
-    return plane_path_fits_backward_integ(F, h, w) && !(plane_path_prefers_slabs_backward(planes, F, h, w) && slabs_suit(planes * F, F, h, w));
+    return plane_path_fits_backward(F, h, w) && !(plane_path_prefers_slabs_backward(planes, F, h, w) && slabs_suit(planes * F, F, h, w));
 }
 
 // Backward of planes that do not fit in shared memory, by slabs (workspace already checked).
@@ -802,6 +802,7 @@ const char *bc_kernel_name(int kernel_id)
         case KID_FORWARD_TMEM: return "forward_tmem_kernel";
         case KID_FORWARD_TMEM_STREAM: return "forward_tmem_stream_kernel";
         case KID_BACKWARD_QUAD_PAIR: return "backward_quad_pair_kernel";
+        case KID_BACKWARD_SQUARE: return "backward_square_kernel";
         default: return "unknown";
     }
 }

@@ -9,6 +9,7 @@
 // Up to 16 such tiles are a CTA.  With few planes, up to 8 CTAs share one as a cluster, so that every element of it
 // is in flight at once; with many, a CTA walks down its plane.  What the tiles above add to a tile's columns comes
 // through shared memory and, across CTAs, through distributed shared memory.
+#include "bc_cluster.cuh"
 #include "bc_common.cuh"
 #include "bc_quad.cuh"
 #include "bc_tile_io.cuh"
@@ -26,23 +27,6 @@ __device__ __forceinline__ float4 relu4(float4 v)
 }
 
 __device__ __forceinline__ float4 add4(const float4 &a, const float4 &b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
-
-__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank)
-{
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ float4 cluster_load4(uint32_t addr)
-{
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-__device__ __forceinline__ void cluster_sync()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 // Where a lane's four columns go, row after row.  QUAD: rows in the quad layout, with the constant zeros at their
 // left and the copies of the last value behind column w, which some lanes of the first and the last warp write.

@@ -1,0 +1,78 @@
+"""Backward of whole planes by strips dealt out to lanes: sizes at which its tiles, row groups, CTAs and clusters begin and end (one strip a
+row and several a tile, rows over several tiles, eight row groups and more, samples that share a CTA and a last CTA of fewer, two tiles a
+warp, filters over several CTAs), rows that no vector access fits, 16-bit tensors, the input's integral image instead of the input, and what infinities
+reach; against the float64 kernels.
+
+Tolerances as in the parity tests: grad-input 1e-4 and parameter gradients 1e-3 of the largest magnitude; 16-bit results are
+rounded once more, by at most 2^-8 (bfloat16) or 2^-11 (float16) of their magnitude.
+"""
+import pytest
+import torch
+
+from conftest import kernels_run, max_rel
+from test_gpu_quad_pair_backward import NAMES, ROUNDING, _case, _grads
+
+pytestmark = pytest.mark.gpu
+
+# samples, channels, filters, rows, columns
+SHAPES = [(1, 1, 1, 1, 1), (3, 2, 2, 7, 3), (2, 1, 3, 9, 29), (700, 1, 2, 8, 4), (650, 2, 1, 20, 25), (331, 2, 2, 21, 31), (301, 1, 4, 33, 37), (75, 4, 2, 72, 48), (2, 3, 3, 65, 61),
+          (1, 4, 2, 64, 300), (2, 2, 5, 24, 516), (1, 3, 8, 40, 260), (150, 1, 2, 88, 124), (3, 1, 4, 100, 130), (1, 150, 1, 110, 117), (2, 2, 3, 200, 60), (1, 2, 2, 280, 26), (1, 2, 6, 1020, 30),
+          (1, 2, 3, 31, 1020), (2, 3, 4, 120, 200), (1, 2, 4, 126, 252)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_gradients_against_float64(shape, dtype):
+    m, x, g = _case(shape, shape[3] % 3 != 0, True, dtype)
+    gin, gp = _grads(m, x, g)
+    want_in, want_p = _grads(m.double(), x.double(), g.double())
+    assert max_rel(gin.double().cpu().numpy(), want_in.cpu().numpy()) < 1e-4 + ROUNDING[dtype]
+    assert max_rel(gp.cpu().numpy(), want_p.cpu().numpy()) < 1e-3 + ROUNDING[dtype]
+
+
+@pytest.mark.parametrize("shape", [s for s in SHAPES if s[0] * s[1] * s[3] * s[4] < 200000])
+def test_four_functions_and_subsets(shape):
+    import box_convolution as bc
+    m, x, g = _case(shape, True, True)
+    gin, gp = _grads(m, x, g)
+    pixels = [p.detach() for p in m.get_actual_parameters()]
+    integ = bc.integral_image(x.double()).float()
+    grads = bc.box_convolution_backward(integ, *pixels, g, g, m.reparametrization_h, m.reparametrization_w, True, True, True, True, True, True, True)
+    # (the input's pixels are differences of its rounded integral image)
+    rounding = 8 * 2.0 ** -24 * float(integ.abs().max())
+    assert max_rel(grads[0].cpu().numpy(), gin.cpu().numpy()) < 1e-4
+    assert max_rel(torch.stack([t.double() for t in grads[1:]]).cpu().numpy(), gp.cpu().numpy()) < 1e-3 + rounding
+    for n in NAMES:
+        getattr(m, n).requires_grad_(False)
+    x = x.detach().requires_grad_()
+    m(x).backward(g)
+    assert max_rel(x.grad.cpu().numpy(), gin.cpu().numpy()) < 1e-6
+
+
+@pytest.mark.parametrize("shape", [(40, 8, 6, 50, 40), (300, 1, 5, 90, 60), (160, 1, 3, 152, 96)])
+def test_a_part_of_a_batch_gives_the_bits_of_the_whole(shape):
+    """Few samples have their filters spread over a cluster of CTAs."""
+    m, x, g = _case(shape, True, True)
+    whole, _ = _grads(m, x, g)
+    assert "backward_plane_kernel" in kernels_run(lambda: _grads(m, x[:3], g[:3]))
+    for a, b in ((0, 1), (5, 8), (shape[0] - 30, shape[0])):
+        part, _ = _grads(m, x[a:b], g[a:b])
+        assert torch.equal(part, whole[a:b])
+
+
+@pytest.mark.parametrize("shape", [(2, 2, 2, 65, 61), (300, 1, 2, 21, 31), (1, 1, 2, 13, 300)])
+def test_infinities_reach_no_further_than_their_boxes(shape):
+    """An infinity in the last row of grad_output, and boxes that look away from it: grad-input of rows that do not gather from it, and
+    the parameter gradients of filters none of whose pixels do, stay as they are without it."""
+    m, x, g = _case(shape, True, True)
+    N, C, F, h, w = shape
+    with torch.no_grad():      # filter 0 of every channel gathers from rows above the pixel's own, the mirrored box below... and filter 1 from below
+        m.x_min.copy_(torch.tensor([2.5, -4.5]).expand(C, F) / m.reparametrization_h)
+        m.x_max.copy_(torch.tensor([4.25, -2.25]).expand(C, F) / m.reparametrization_h)
+    clean, clean_p = _grads(m, x, g)
+    g = g.clone().view(N, C, F, h, w)
+    g[0, 0, 0, h - 1, w // 2] = float("inf")
+    gin, gp = _grads(m, x, g.view(N, C * F, h, w))
+    # the mirrored box of filter 0 reaches from row p - 5 to p - 2: only rows that do not exist would see the last row
+    assert torch.equal(gin, clean)
+    assert torch.equal(gp, clean_p)
