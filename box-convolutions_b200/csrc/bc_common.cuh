@@ -182,6 +182,10 @@ int launch_backward_plane_integ(const float *x_integ, const float *grad_output, 
                                 float *grad_params, float *partials, cudaStream_t s);
 
 // Whole planes of any width (box_flat.cu); exactly one of x and x_integ (plain rows, float only) is given.
+bool flat_fits_forward(int F, int h, int w);
+// null `fu` = plain forward (16-bit outputs: always)
+int launch_forward_flat(const void *x, const float *integ, int io_kind, const BoxParams &bp, const Fusion *fu, void *out, int N, int C, int F, int h, int w,
+                        bool normalize, bool exact, cudaStream_t s);
 bool flat_fits_backward(int F, int h, int w);
 int launch_backward_flat(const void *x, const float *x_integ, int io_kind, const void *grad_output, const BoxParams &bp, float rep_h, float rep_w, int N,
                          int C, int F, int h, int w, bool normalize, bool exact, int need_mask, void *grad_input, void *grad_params,

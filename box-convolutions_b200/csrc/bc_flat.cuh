@@ -120,16 +120,21 @@ __device__ __forceinline__ void flat_zero_padding(uint32_t image, const FlatShap
 struct FlatBlock {
     f2_t a[kFlatRows], b[kFlatRows];      // columns c, c+1 and c+2, c+3
 };
-template <typename IO, bool VEC>
+// PLAIN: the kernel may write the rows later.
+template <typename IO, bool VEC, bool PLAIN = false>
 __device__ __forceinline__ void flat_load(FlatBlock &v, const IO *row0, int w, const FlatCell &cell, int lane, int strips)
 {
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     const int c = cell.strip * 4;
     const IO *p = row0 + c;
+    auto load = [](const IO *at) {
+        if constexpr (PLAIN) return Io<IO>::load4_plain(at);
+        else return Io<IO>::load4(at);
+    };
     if (VEC) {
         float4 e[kFlatRows];
 #pragma unroll
-        for (int i = 0; i < kFlatRows; ++i, p += w) e[i] = i < cell.rows ? Io<IO>::load4(p) : zero;
+        for (int i = 0; i < kFlatRows; ++i, p += w) e[i] = i < cell.rows ? load(p) : zero;
 #pragma unroll
         for (int i = 0; i < kFlatRows; ++i) { v.a[i] = pack2(e[i].x, e[i].y); v.b[i] = pack2(e[i].z, e[i].w); }
         return;
@@ -140,8 +145,8 @@ __device__ __forceinline__ void flat_load(FlatBlock &v, const IO *row0, int w, c
 #pragma unroll
     for (int i = 0; i < kFlatRows; ++i, p += w) {
         const int k = (k0 + i * w) & 3;
-        e[i] = i < cell.rows ? Io<IO>::load4(p - k) : zero;
-        next[i] = end && k && i < cell.rows && c + 4 - k < w ? Io<IO>::load4(p + 4 - k) : zero;
+        e[i] = i < cell.rows ? load(p - k) : zero;
+        next[i] = end && k && i < cell.rows && c + 4 - k < w ? load(p + 4 - k) : zero;
     }
 #pragma unroll
     for (int i = 0; i < kFlatRows; ++i) {
@@ -165,35 +170,30 @@ __device__ __forceinline__ void flat_load(FlatBlock &v, const IO *row0, int w, c
     }
 }
 
-// `ok`: the row exists.  Collective where rows are not aligned.
+// Columns c .. c+3 of a row, as far as they are in the plane.  Rows of any alignment: one, two or three accesses, whatever the row's first
+// element is aligned to; moving elements between lanes until groups are aligned costs more than the accesses it saves.
 template <typename IO, bool VEC>
-__device__ __forceinline__ void flat_store_row(IO *row, int c, int w, const float (&v)[kStrip], int lane, bool first, bool end, bool ok)
+__device__ __forceinline__ void flat_store_row(IO *row, int c, int w, const float (&v)[kStrip])
 {
+    IO *p = row + c;
     if (VEC) {
-        if (ok) Io<IO>::store4(row + c, v[0], v[1], v[2], v[3]);
-        return;
-    }
-    // whole aligned groups by the lane in which they end; single elements: the 4 - k in front of a row's (or the warp's) first group, the k behind
-    // the last one, and what the row's end cuts off
-    const int k = row_shift(row);
-    float o[4] = {v[0], v[1], v[2], v[3]};
-    const float p3 = __shfl_up_sync(0xffffffffu, o[3], 1);
-    if (k & 1) { o[3] = o[2]; o[2] = o[1]; o[1] = o[0]; o[0] = p3; }
-    const float q2 = __shfl_up_sync(0xffffffffu, o[2], 1), q3 = __shfl_up_sync(0xffffffffu, o[3], 1);
-    if (k & 2) { o[3] = o[1]; o[2] = o[0]; o[1] = q3; o[0] = q2; }
-    if (!ok) return;
-    const bool grouped = (!first || k == 0) && c - k + 4 <= w;
-    if (grouped) Io<IO>::store4(row + c - k, o[0], o[1], o[2], o[3]);
-    // elements c+m of this lane that no group covers; those in front of c belong to a group of this lane that the row's end cut
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        const bool mine = m < 4 - k ? !grouped : end;      // (c + m < 4 - k + c: in this lane's group, else in the next lane's)
-        if (mine && c + m < w) Io<IO>::store1(row + c + m, v[m]);
-    }
-    if (!first && !grouped) {      // the group's elements from the lane before, which that lane leaves to this one
+        Io<IO>::store4(p, v[0], v[1], v[2], v[3]);
+    } else if (c + 4 <= w) {
+        const int k = row_shift(row);
+        if (k == 0) {
+            Io<IO>::store4(p, v[0], v[1], v[2], v[3]);
+        } else if (k == 2) {
+            Io<IO>::store2(p, v[0], v[1]);
+            Io<IO>::store2(p + 2, v[2], v[3]);
+        } else {
+            Io<IO>::store1(p, v[0]);
+            Io<IO>::store2(p + 1, v[1], v[2]);
+            Io<IO>::store1(p + 3, v[3]);
+        }
+    } else {
 #pragma unroll
         for (int m = 0; m < 3; ++m)
-            if (m < k && c - k + m < w) Io<IO>::store1(row + c - k + m, o[m]);
+            if (c + m < w) Io<IO>::store1(p + m, v[m]);
     }
 }
 
@@ -409,6 +409,17 @@ inline int pow2_columns(int n)
     while (columns < n) columns *= 2;
     return columns;
 }
+// Samples that share a CTA, where a plane alone would not fill eight warps: no fewer CTAs than two an SM, and room for three on one (narrow
+// planes are half padding).
+inline int flat_samples(int N, int C, int h, int w)
+{
+    const int cells = flat_strips(w) * flat_groups(h), bytes = flat_shape(h, w, 1).plane;
+    int64_t planes = cells >= 256 ? 1 : 256 / cells;
+    const int64_t most[] = {(int64_t)N * C / 296, N, 255, 56 * 1024 / bytes};
+    for (int64_t m : most) planes = planes > m ? m : planes;
+    return planes > 1 ? (int)planes : 1;
+}
+
 struct FlatPlan {
     FlatShape sh;
     int tiles_a_warp, warps;
@@ -421,14 +432,7 @@ struct FlatPlan {
 // Filters over several CTAs: 12 planes of 120 x 133, F = 8, 119 us -> 25; (5,1,8,280,34) 96 -> 18.
 inline FlatPlan flat_backward_plan(int N, int C, int F, int h, int w, bool write_gin)
 {
-    const int cells = flat_strips(w) * flat_groups(h);
-    int planes = cells >= 256 ? 1 : 256 / cells;      // (at most 255: flat_pack())
-    const int64_t most = (int64_t)N * C / 296;      // (no fewer CTAs than two an SM)
-    if (planes > most) planes = most > 1 ? (int)most : 1;
-    if (planes > N) planes = N;
-    const int each_bytes = flat_shape(h, w, 1).plane;      // (narrow planes are half padding; three CTAs an SM should fit)
-    if (planes * each_bytes > 56 * 1024) planes = each_bytes > 28 * 1024 ? 1 : 56 * 1024 / each_bytes;
-    if (planes > 255) planes = 255;
+    const int planes = flat_samples(N, C, h, w);
     FlatPlan p;
     p.sh = flat_shape(h, w, planes);
     const int64_t ctas = (int64_t)((N + planes - 1) / planes) * C;
@@ -447,6 +451,31 @@ inline FlatPlan flat_backward_plan(int N, int C, int F, int h, int w, bool write
     const int each = p.sh.split > 1 ? (F + p.sh.split - 1) / p.sh.split : 1;
     p.sh.columns = pow2_columns(slot * each);
     if (p.sh.split > 1 && write_gin && p.smem < rows * each) p.smem = rows * each;
+    return p;
+}
+
+// ---- and a forward pass ------------------------------------------------------------------------------------
+struct FlatForwardPlan {
+    FlatShape sh;
+    int warps, fsplit, tsplit;
+    bool tight;      // no room for scan corners of their own (tall planes of up to 32 columns)
+    size_t smem;
+};
+inline FlatForwardPlan flat_forward_plan(int N, int C, int F, int h, int w)
+{
+    FlatForwardPlan p;
+    p.sh = flat_shape(h, w, flat_samples(N, C, h, w));
+    const int64_t ctas = (int64_t)((N + p.sh.planes - 1) / p.sh.planes) * C;
+    p.fsplit = F % 2 == 0 && ctas < 148 * 6 ? 2 : 1;
+    const int64_t room = p.sh.tiles <= 16 ? 148 * 2 : 148;      // (of more than 16 warps an SM takes one CTA)
+    for (int k = p.fsplit + 1; k <= F; ++k)
+        if (F % k == 0 && ctas * k <= room) p.fsplit = k;
+    p.tsplit = 1;
+    while (p.sh.tiles > 8 && ctas * p.fsplit * p.tsplit * 2 <= 148 && p.tsplit < 4) p.tsplit *= 2;
+    p.warps = p.sh.tiles;
+    p.smem = flat_smem(p.sh, 1, F);
+    p.tight = p.smem > kFlatMaxSmem && flat_image_bytes(p.sh) >= p.warps * kFlatScanBytes;
+    if (p.tight) p.smem -= p.warps * kFlatScanBytes;
     return p;
 }
 

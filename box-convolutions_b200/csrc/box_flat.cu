@@ -195,12 +195,11 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
             const FlatCell cell = flat_unpack(T == 1 || k == 0 ? packed[0] : packed[T - 1]);
             TmemRows<1, T> kept(tmem_base, warp, k);
             IO *row = grad_input + pixel_of(cell);
-            const bool first = lane == 0 || cell.strip == 0, end = lane == 31 || cell.strip == sh.strips - 1;
 #pragma unroll
             for (int i = 0; i < kFlatRows; ++i, row += w) {
                 const float4 g = kept.grad_input(i);
                 const float v[kStrip] = {g.x, g.y, g.z, g.w};
-                flat_store_row<IO, VEC>(row, cell.strip * 4, w, v, lane, first, end, i < cell.rows);
+                if (i < cell.rows) flat_store_row<IO, VEC>(row, cell.strip * 4, w, v);
                 __syncwarp();
             }
         }
@@ -216,7 +215,6 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
         for (int k = 0; k < T; ++k) {
             const FlatCell cell = flat_unpack(T == 1 || k == 0 ? packed[0] : packed[T - 1]);
             IO *row = grad_input + pixel_of(cell) + row_begin * w;
-            const bool first = lane == 0 || cell.strip == 0, end = lane == 31 || cell.strip == sh.strips - 1;
             for (int i = row_begin; i < row_end; ++i, row += w) {
                 const uint32_t at = s.image + ((i * sh.tiles + warp + k * nwarps) * 32 + lane) * 16;
                 float v[kStrip] = {0.f, 0.f, 0.f, 0.f};
@@ -227,13 +225,143 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
                         v[0] += g.x; v[1] += g.y; v[2] += g.z; v[3] += g.w;
                     }
                 }
-                flat_store_row<IO, VEC>(row, cell.strip * 4, w, v, lane, first, end, i < cell.rows);
+                if (i < cell.rows) flat_store_row<IO, VEC>(row, cell.strip * 4, w, v);
                 __syncwarp();
             }
         }
         cluster_sync();      // nobody leaves while another still reads its rows
     }
     if (COUNTED) finish_if_last(fin, partials, bp, c, C, F, normalize, exact);
+}
+
+// Forward: a CTA for `sh.planes` samples of a channel, a part of the filters and of the tiles (`fsplit`, `tsplit`).  It builds all integral images, a
+// tile a warp (64 registers: up to 32 warps, or 16 twice an SM), then its warps gather tile by tile and filter by filter.
+// A null `x`: `integ` holds the planes' integral images, plain rows of w + 1 floats, which are only copied (INTEG).
+// FUSED: the inference steps of `Fusion` (the output may then alias the residual); the planes travel to L2 while the CTA still waits for the
+// kernel in front, and all residual rows of a tile are in flight before its gather.
+template <typename IO, bool VEC, bool FUSED, bool INTEG, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1)
+forward_flat_kernel(const IO *__restrict__ x, const float *__restrict__ integ, BoxParams bp, IO *out, int N, int C, int F, int h, int w,
+                    const __grid_constant__ FlatShape sh, int fsplit, int tsplit, bool tight, bool normalize, bool exact, Fusion fu)
+{
+    extern __shared__ float4 smem4[];
+    grid_dependency_release();
+    const int lane = threadIdx.x & 31, warp = uniform(threadIdx.x >> 5), nwarps = blockDim.x >> 5;
+    const int tpart = blockIdx.x % tsplit, rest = blockIdx.x / tsplit, part = rest % fsplit, b = rest / fsplit;
+    const int c = b % C, n0 = b / C * sh.planes, planes = min(sh.planes, N - n0);
+    const int f_begin = F * part / fsplit, nf = F * (part + 1) / fsplit - f_begin;
+    const int npix = h * w;
+    FlatSmem s = flat_smem_at<1>(smem4, sh);
+    if (tight) {      // the scans' corners where the images will be, whose padding is written behind them
+        s.taps = s.scan;
+        s.scan = s.image;
+    }
+    float *sTaps = reinterpret_cast<float *>(reinterpret_cast<char *>(smem4) + (s.taps - s.image));
+    // tiles that have strips, and this CTA's share of them
+    const int have = (sh.cells * planes + 31) / 32, t_begin = have * tpart / tsplit, nt = have * (tpart + 1) / tsplit - t_begin;
+
+    if (!INTEG)      // a hint
+        for (int g = 0; g < planes; ++g) prefetch_l2(x + ((int64_t)(n0 + g) * C + c) * npix, (size_t)npix * sizeof(IO));
+    if (!tight) flat_zero_padding(s.image, sh, planes, h);
+    // registers and shared memory only up to here; now what the kernel in front of this one may have written
+    grid_dependency_wait();
+    auto boxes = [&]() {
+        if ((int)threadIdx.x < nf) {
+            const Box box = load_box(bp, c * F + f_begin + threadIdx.x);
+            store_taps(sTaps + threadIdx.x * kTapWords, taps_forward(box.xmin, box.xmax, box.ymin, box.ymax, normalize, exact));
+        }
+    };
+    if constexpr (INTEG) {
+        if (tight) flat_zero_padding(s.image, sh, planes, h);
+        boxes();
+        __syncthreads();      // (the zero padding has been written)
+        for (int g = 0; g < planes; ++g) {
+            const float *I = integ + ((int64_t)(n0 + g) * C + c) * (h + 1) * (w + 1);
+            copy_integral_rows(I, h, w, 4 * sh.strips + 8, warp, nwarps, lane, [&](int a, int col, float e) {
+                sts<8>(s.image + g * sh.plane + flat_row_at(a, sh.row, sh.skew) + (col & 3) * sh.sub + (col >> 2) * 4, e);
+            });
+        }
+    } else {
+        FlatBlock v;
+        float carry[kFlatRows];
+        const FlatCell mine = flat_cell(sh, warp * 32 + lane, planes, h);
+        flat_load<IO, VEC>(v, x + ((int64_t)(n0 + mine.plane) * C + c) * npix + mine.group * kFlatRows * w, w, mine, lane, sh.strips);
+        const uint32_t starts = __ballot_sync(0xffffffffu, mine.strip == 0);
+        boxes();
+        __syncwarp();
+        if (FUSED && fu.input_relu) {
+#pragma unroll
+            for (int i = 0; i < kFlatRows; ++i) {
+                float e0, e1;
+                unpack2(v.a[i], e0, e1);
+                v.a[i] = pack2(fmaxf(e0, 0.f), fmaxf(e1, 0.f));
+                unpack2(v.b[i], e0, e1);
+                v.b[i] = pack2(fmaxf(e0, 0.f), fmaxf(e1, 0.f));
+            }
+        }
+        flat_scan<1>(v, carry, s, warp, starts, sh.spans, warp, nwarps, lane);
+        if (sh.spans) __syncthreads();
+        flat_publish(v, carry, s, warp * 32 / sh.strips * sh.strips / 32, warp, starts, lane);
+        __syncthreads();
+        if (tight) flat_zero_padding(s.image, sh, planes, h);
+        if (sh.groups > kFlatTall) {
+            flat_sum_above(s, sh);
+            __syncthreads();
+        }
+        flat_put(v, mine, s, sh, warp, lane);
+    }
+    __syncthreads();
+
+    FlatCell cell;
+    int at = -1;
+    for (int task = warp; task < nt * nf; task += nwarps) {
+        const int k = task / nt, tile = t_begin + task - k * nt, f = f_begin + k;
+        if (tile != at) cell = flat_cell(sh, tile * 32 + lane, planes, h);
+        at = tile;
+        const BoxTaps t = load_taps_uniform(sTaps + k * kTapWords);
+        const FlatCols cols = flat_cols(t, cell, s.image, sh);
+        const FlatRows<false> q = flat_rows<false>(t, cell, h, sh);
+        const ColW2 cw = col_weights(t);
+        const float sfl = t.scale * t.f_lo_r, sfh = t.scale * t.f_hi_r;
+        float mul = 1.0f, add = 0.0f;
+        if (FUSED) {
+            if (fu.scale) mul = __ldg(fu.scale + c * F + f);
+            if (fu.shift) add = __ldg(fu.shift + c * F + f);
+        }
+        const int64_t first = (((int64_t)(n0 + cell.plane) * C + c) * F + f) * npix + cell.group * kFlatRows * w;
+        IO *row = out + first;
+        FlatBlock skip;
+        if constexpr (FUSED) {
+            if (fu.residual) flat_load<float, VEC, true>(skip, fu.residual + first, w, cell, lane, sh.strips);
+        }
+        f2_t prev[kStrip];
+        quad_pair(cols, q.lo(0), q.hi(0), cw, prev);
+#pragma unroll
+        for (int i = 0; i < kFlatRows; ++i) {
+            f2_t cur[kStrip];
+            quad_pair(cols, q.lo(i + 1), q.hi(i + 1), cw, cur);
+            float v[kStrip];
+            quad_forward_row(prev, cur, t.scale, sfl, sfh, v);
+#pragma unroll
+            for (int m = 0; m < kStrip; ++m) prev[m] = cur[m];
+            if constexpr (FUSED) {
+#pragma unroll
+                for (int m = 0; m < kStrip; ++m) v[m] = v[m] * mul + add;
+                if (fu.residual) {
+                    float e0, e1, e2, e3;
+                    unpack2(skip.a[i], e0, e1);
+                    unpack2(skip.b[i], e2, e3);
+                    v[0] += e0; v[1] += e1; v[2] += e2; v[3] += e3;
+                }
+                if (fu.output_relu) {
+#pragma unroll
+                    for (int m = 0; m < kStrip; ++m) v[m] = fmaxf(v[m], 0.0f);
+                }
+            }
+            if (i < cell.rows) flat_store_row<IO, VEC>(row, cell.strip * 4, w, v);
+            row += w;
+        }
+    }
 }
 
 template <typename IO>
@@ -274,12 +402,63 @@ int launch_backward_flat_t(const IO *x, const float *x_integ, const IO *grad_out
     return launch_finish_param_grads<float>(partials, bp, C * F, teams, normalize, exact, rep_h, rep_w, need_mask, grad_params, s, grad_params_kind);
 }
 
+template <typename IO>
+int launch_forward_flat_t(const IO *x, const float *integ, const BoxParams &bp, const Fusion *fu, IO *out, int N, int C, int F, int h, int w,
+                          bool normalize, bool exact, cudaStream_t s)
+{
+    const FlatForwardPlan plan = flat_forward_plan(N, C, F, h, w);
+    const int64_t ctas = (int64_t)((N + plan.sh.planes - 1) / plan.sh.planes) * C * plan.fsplit;
+    // No parts of a plane where the output lies over the input (one filter, in place): a CTA that starts late would integrate
+    // rows that another has already replaced.
+    const bool in_place = x && ranges_overlap(x, (size_t)N * C * h * w * sizeof(IO), out, (size_t)N * C * F * h * w * sizeof(IO));
+    const int tsplit = in_place ? 1 : plan.tsplit;
+    if (ctas * tsplit > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
+    const bool fast = w % 4 == 0 && aligned_to(x, Io<IO>::kVecBytes) && aligned_to(out, Io<IO>::kVecBytes) && (!fu || !fu->residual || aligned_to(fu->residual, 16));
+    void (*kern)(const IO *, const float *, BoxParams, IO *, int, int, int, int, int, FlatShape, int, int, bool, bool, bool, Fusion);
+    auto pick = [&](auto vecs) {
+        constexpr bool V = decltype(vecs)::value, FL = IsFloat<IO>::value;
+        // residual rows in flight want registers, unless they cost an SM its second CTA
+        if (fu) kern = plan.warps <= 10 || (plan.warps <= 20 && ctas * tsplit <= 148) ? forward_flat_kernel<IO, V, FL, false, 640> : forward_flat_kernel<IO, V, FL, false, 1024>;
+        else kern = x ? forward_flat_kernel<IO, V, false, false, 1024> : forward_flat_kernel<IO, V, false, FL, 1024>;
+    };
+    if (fast) pick(Flag<true>{});
+    else pick(Flag<false>{});
+    int st = raise_smem_limit(reinterpret_cast<const void *>(kern), (int)kFlatMaxSmem);
+    if (st != BC_OK) return st;
+    const Fusion none{0, nullptr, nullptr, nullptr, 0};
+    {
+        LaunchScope scope(KID_FORWARD_PLANE, s);
+        if (cudaError_t e = launch_overlapped(kern, (unsigned)(ctas * tsplit), plan.warps * 32, plan.smem, s, x, integ, bp, out, N, C, F, h, w, plan.sh, plan.fsplit,
+                                              tsplit, plan.tight, normalize, exact, fu ? *fu : none))
+            return cuda_failed(e, "forward_flat");
+    }
+    return check_launch("forward_flat");
+}
+
 }  // namespace
 
 bool flat_fits_backward(int F, int h, int w)
 {
     if (F > kMaxFilters || (int64_t)flat_strips(w) * flat_groups(h) > 32 * kFlatMaxTiles) return false;
     return flat_backward_plan(1, 1, F, h, w, true).smem <= kFlatMaxSmem;
+}
+
+bool flat_fits_forward(int F, int h, int w)
+{
+    if (F > kMaxFilters || (int64_t)flat_strips(w) * flat_groups(h) > 32 * kFlatMaxTiles) return false;
+    return flat_forward_plan(1, 1, F, h, w).smem <= kFlatMaxSmem;
+}
+
+int launch_forward_flat(const void *x, const float *integ, int io_kind, const BoxParams &bp, const Fusion *fu, void *out, int N, int C, int F, int h, int w,
+                        bool normalize, bool exact, cudaStream_t s)
+{
+    auto launch = [&](auto zero) {
+        using IO = decltype(zero);
+        return launch_forward_flat_t(static_cast<const IO *>(x), integ, bp, fu, static_cast<IO *>(out), N, C, F, h, w, normalize, exact, s);
+    };
+    if (io_kind == BC_IO_F32) return launch(0.0f);
+    if (fu) return BC_ERR_UNSUPPORTED;
+    return io_kind == BC_IO_F16 ? launch(__half{}) : launch(__nv_bfloat16{});
 }
 
 int launch_backward_flat(const void *x, const float *x_integ, int io_kind, const void *grad_output, const BoxParams &bp, float rep_h, float rep_w, int N,

@@ -14,6 +14,13 @@ extern "C" void flat_backward(int N, int C, int F, int h, int w, int write_gin, 
                          (flat_row_at(8, s.row, s.skew) / 4 - s.strips) % 32, (s.plane / 4 - s.cells) % 32, s.tiles, flat_image_bytes(s)};
     for (int i = 0; i < 16; ++i) out[i] = v[i];
 }
+// warps, planes, parts of the filters, parts of the tiles, shared memory, strips a row, row groups
+extern "C" void flat_forward(int N, int C, int F, int h, int w, int64_t *out)
+{
+    const FlatForwardPlan p = flat_forward_plan(N, C, F, h, w);
+    const int64_t v[] = {p.warps, p.sh.planes, p.fsplit, p.tsplit, (int64_t)p.smem, p.sh.strips, p.sh.groups, flat_image_bytes(p.sh), p.tight};
+    for (int i = 0; i < 9; ++i) out[i] = v[i];
+}
 // Offsets, as the kernels add them up, of the tap row `row` less than 16 below the start of row group `group`'s first one at `a`.
 extern "C" int flat_offset(int h, int w, int group, int a, int j)
 {

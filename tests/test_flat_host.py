@@ -54,6 +54,18 @@ def test_launches_fit(flat):
                     assert p["tiles"] * 4096 * each <= p["smem"], at
 
 
+def test_forward_launches_fit(flat):
+    for h, w in served():
+        for N, C, F in ((1, 1, 1), (1, 3, 4), (7, 1, 6), (150, 1, 32), (3000, 2, 4)):
+            v = (ctypes.c_int64 * 9)()
+            flat.flat_forward(N, C, F, h, w, v)
+            warps, planes, fsplit, tsplit, smem, strips, groups, image, tight = v
+            at = (N, C, F, h, w, list(v))
+            assert warps <= 32 and strips * groups * planes <= warps * 32 and planes <= N, at
+            assert smem <= 227 * 1024 - 64 and 1 <= fsplit <= F and F % fsplit == 0 and tsplit in (1, 2, 4), at
+            assert smem >= image + warps * 544 + 48 * F + (0 if tight else warps * 1152) and (not tight or image >= warps * 1152), at
+
+
 def test_layout(flat):
     for h, w in list(served())[::7]:
         p = plan(flat, 1, 1, 1, h, w)

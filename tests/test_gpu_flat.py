@@ -1,9 +1,11 @@
-"""Backward of whole planes by strips dealt out to lanes: sizes at which its tiles, row groups, CTAs and clusters begin and end (one strip a
+"""Whole planes by strips dealt out to lanes: sizes at which its tiles, row groups, CTAs and clusters begin and end (one strip a
 row and several a tile, rows over several tiles, eight row groups and more, samples that share a CTA and a last CTA of fewer, two tiles a
-warp, filters over several CTAs), rows that no vector access fits, 16-bit tensors, the input's integral image instead of the input, and what infinities
-reach; against the float64 kernels.
+warp, filters and tiles over several CTAs, planes that leave no
+room for scan corners), rows that no vector access fits, 16-bit tensors, the input's integral image instead of the input, and what infinities
+reach; against the float64
+kernels.
 
-Tolerances as in the parity tests: grad-input 1e-4 and parameter gradients 1e-3 of the largest magnitude; 16-bit results are
+Tolerances as in the parity tests: outputs and grad-input 1e-4 and parameter gradients 1e-3 of the largest magnitude; 16-bit results are
 rounded once more, by at most 2^-8 (bfloat16) or 2^-11 (float16) of their magnitude.
 """
 import pytest
@@ -28,6 +30,46 @@ def test_gradients_against_float64(shape, dtype):
     want_in, want_p = _grads(m.double(), x.double(), g.double())
     assert max_rel(gin.double().cpu().numpy(), want_in.cpu().numpy()) < 1e-4 + ROUNDING[dtype]
     assert max_rel(gp.cpu().numpy(), want_p.cpu().numpy()) < 1e-3 + ROUNDING[dtype]
+
+
+FORWARD = [(1, 2, 3, 72, 133), (3, 2, 4, 96, 132), (2, 75, 1, 130, 50), (40, 4, 6, 280, 26), (1, 2, 4, 1020, 30), (1, 2, 2, 1024, 32), (1, 1, 3, 31, 1020), (2, 3, 2, 93, 157), (150, 1, 2, 110, 117),
+           (1, 3, 4, 126, 252), (1, 16, 2, 192, 136), (5, 2, 1, 40, 300)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", FORWARD)
+def test_outputs_against_float64(shape, dtype):
+    m, x, _ = _case(shape, shape[3] % 3 != 0, True, dtype)
+    with torch.no_grad():
+        m.eval()
+        assert "forward_plane_kernel" in kernels_run(lambda: m(x))
+        out = m(x)
+        want = m.double()(x.double())
+    assert max_rel(out.double().cpu().numpy(), want.cpu().numpy()) < 1e-4 + ROUNDING[dtype]
+
+
+@pytest.mark.parametrize("shape", FORWARD)
+def test_fused_and_from_the_integral_image(shape):
+    import box_convolution as bc
+    N, C, F, h, w = shape
+    m, x, g = _case(shape, True, True)
+    m.eval()
+    scale, shift = torch.rand(C * F, device="cuda") + 0.5, torch.rand(C * F, device="cuda") - 0.5
+    with torch.no_grad():
+        out = bc.fused_box_block(m, x, input_relu=True, scale=scale, shift=shift, residual=g, output_relu=True, out=g.clone())
+        alias = g.clone()
+        bc.fused_box_block(m, x, input_relu=True, scale=scale, shift=shift, residual=alias, output_relu=True, out=alias)
+        integ = bc.integral_image(x.double()).float()
+        from_integ = bc.box_convolution_forward(integ, *m.get_actual_parameters(), True, True)
+        plain, m64 = m(x), m.double()
+        want = (m64(x.double().relu()) * scale.double().view(1, -1, 1, 1) + shift.double().view(1, -1, 1, 1) + g.double()).relu()
+    assert torch.equal(out, alias)
+    assert max_rel(out.double().cpu().numpy(), want.cpu().numpy()) < 1e-4
+    assert max_rel(from_integ.cpu().numpy(), plain.cpu().numpy()) < 1e-4
+    if F == 1:      # in place: output over input
+        own = x.clone()
+        bc.fused_box_block(m.float(), own, out=own)
+        assert torch.equal(own, plain)
 
 
 @pytest.mark.parametrize("shape", [s for s in SHAPES if s[0] * s[1] * s[3] * s[4] < 200000])
