@@ -79,6 +79,17 @@ class BoxConv2d(torch.nn.Module):
                             self.reparametrization_h, self.reparametrization_w,
                             self.max_input_h, self.max_input_w, self.exact)
 
+    def zero_grad(self, set_to_none=True):
+        # A training step of a small module is bound by the host, and the generators behind parameters() take
+        # a tenth of it ((1, 8, 4, 32, 32): 8.9 us of 84; here 3.6, the release of the gradients).  Anything but the four plain parameters goes the general way.
+        cls = type(self)
+        if (not set_to_none or self._modules or "_is_replica" in self.__dict__
+                or cls.parameters is not torch.nn.Module.parameters or cls.named_parameters is not torch.nn.Module.named_parameters):
+            return super().zero_grad(set_to_none)
+        for p in self._parameters.values():
+            if p is not None:
+                p.grad = None
+
     def train(self, mode=True):
         self.training = mode
         if mode is False:
