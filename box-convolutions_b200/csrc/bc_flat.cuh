@@ -170,33 +170,6 @@ __device__ __forceinline__ void flat_load(FlatBlock &v, const IO *row0, int w, c
     }
 }
 
-// Columns c .. c+3 of a row, as far as they are in the plane.  Rows of any alignment: one, two or three accesses, whatever the row's first
-// element is aligned to; moving elements between lanes until groups are aligned costs more than the accesses it saves.
-template <typename IO, bool VEC>
-__device__ __forceinline__ void flat_store_row(IO *row, int c, int w, const float (&v)[kStrip])
-{
-    IO *p = row + c;
-    if (VEC) {
-        Io<IO>::store4(p, v[0], v[1], v[2], v[3]);
-    } else if (c + 4 <= w) {
-        const int k = row_shift(row);
-        if (k == 0) {
-            Io<IO>::store4(p, v[0], v[1], v[2], v[3]);
-        } else if (k == 2) {
-            Io<IO>::store2(p, v[0], v[1]);
-            Io<IO>::store2(p + 2, v[2], v[3]);
-        } else {
-            Io<IO>::store1(p, v[0]);
-            Io<IO>::store2(p + 1, v[1], v[2]);
-            Io<IO>::store1(p + 3, v[3]);
-        }
-    } else {
-#pragma unroll
-        for (int m = 0; m < 3; ++m)
-            if (c + m < w) Io<IO>::store1(p + m, v[m]);
-    }
-}
-
 // ---- building the integral images -------------------------------------------------------------------
 // First part: a strip's own prefix sums, and `carry`: what the strips to its left add to its rows, as far as they are in the same tile.  Eight
 // rows at once through the warp's corner, four lanes a row with eight strips each; `starts`: the lanes that begin a row.

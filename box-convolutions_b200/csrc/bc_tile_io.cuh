@@ -219,38 +219,36 @@ __device__ __forceinline__ float4 rows8_get(const Rows8 &g, const IO *row0, int 
     return a;
 }
 
-// `ok`: the row exists.  Unaligned rows: one vector store a lane for the aligned groups that lie inside the row and
-// belong to this warp whole, and single elements for the rest: the 4 - k elements in front of the first group (the
-// first lane's), the k behind the last one (the last lane's), and what the row's end cuts off a group.
-template <typename IO, bool ALIGNED, int LN = 32>
-__device__ __forceinline__ void store_row4(IO *row, int c, int w, const float (&v)[4], int lane, bool ok = true)
+// Columns c .. c+3 of a row, as far as they are in the plane.  Rows of any alignment: one, two or three accesses, whatever the row's first
+// element is aligned to.  Moving elements between lanes until groups are aligned costs kernels that gather more than the accesses it saves
+// (1000 unaligned planes of up to 8 tiles, forward 1.19 of the time of single elements with, 1.05 without).
+template <typename IO, bool ALIGNED>
+__device__ __forceinline__ void store_row4(IO *row, int c, int w, const float (&v)[4])
 {
-    if (ALIGNED) {
-        if (ok && c < w) Io<IO>::store4(row + c, v[0], v[1], v[2], v[3]);
-        return;
-    }
-    const int k = row_shift(row);
-    const unsigned full = 0xffffffffu;
-    float o[4] = {v[0], v[1], v[2], v[3]};
-    const float p3 = __shfl_up_sync(full, o[3], 1, LN);
-    if (k & 1) { o[3] = o[2]; o[2] = o[1]; o[1] = o[0]; o[0] = p3; }
-    const float q2 = __shfl_up_sync(full, o[2], 1, LN), q3 = __shfl_up_sync(full, o[3], 1, LN);
-    if (k & 2) { o[3] = o[1]; o[2] = o[0]; o[1] = q3; o[0] = q2; }
-    const int at = c - k;                                     // first column of the lane's group
-    const bool whole = at + 4 <= w && (lane > 0 || k == 0);
-    if (ok && whole) Io<IO>::store4(row + at, o[0], o[1], o[2], o[3]);
-    const bool cut = (lane > 0 || k == 0) && at + 4 > w;                  // the row ends inside the group (or before it)
-    IO *single = row + (cut ? at : c);
-    const int room = w - (cut ? at : c);
-    const int from = cut ? 0 : lane == LN - 1 ? 4 - k : lane == 0 ? 0 : 4, to = cut ? 4 : lane == 0 && k ? 4 - k : lane == LN - 1 ? 4 : 0;
-    // (a group of one lane would be first and last at once; LN is at least 8)
+    IO *p = row + c;
+    if (c + 4 <= w) {
+        const int k = ALIGNED ? 0 : row_shift(row);
+        if (k == 0) {
+            Io<IO>::store4(p, v[0], v[1], v[2], v[3]);
+        } else if (k == 2) {
+            Io<IO>::store2(p, v[0], v[1]);
+            Io<IO>::store2(p + 2, v[2], v[3]);
+        } else {
+            Io<IO>::store1(p, v[0]);
+            Io<IO>::store2(p + 1, v[1], v[2]);
+            Io<IO>::store1(p + 3, v[3]);
+        }
+    } else if (!ALIGNED) {
 #pragma unroll
-    for (int m = 0; m < 4; ++m)
-        if (ok && m >= from && m < to && m < room) Io<IO>::store1(single + m, cut ? o[m] : v[m]);
+        for (int m = 0; m < 3; ++m)
+            if (c + m < w) Io<IO>::store1(p + m, v[m]);
+    }
 }
 
-// The same as branches on the shift k: twice the code, which kernels that store all the time can afford, and fewer
-// instructions (integral images of 512 planes of 256 x 512: 105 us against 115; forward of (8,16,4,149,201): 48 against 52).
+// `ok`: the row exists.  Unaligned rows: one vector store a lane for the aligned groups that lie inside the row and
+// belong to this warp whole, and single elements for the rest: the 4 - k elements in front of the first group (the
+// first lane's), the k behind the last one (the last lane's), and what the row's end cuts off a group.  For kernels that are bound by their stores:
+// branches on the shift k, twice the code and fewer instructions (integral images of 512 planes of 256 x 512: 105 us against 115).
 template <typename IO, bool ALIGNED, int LN = 32>
 __device__ __forceinline__ void store_row4_wide(IO *row, int c, int w, const float (&v)[4], int lane, bool ok = true)
 {

@@ -199,7 +199,7 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
             for (int i = 0; i < kFlatRows; ++i, row += w) {
                 const float4 g = kept.grad_input(i);
                 const float v[kStrip] = {g.x, g.y, g.z, g.w};
-                if (i < cell.rows) flat_store_row<IO, VEC>(row, cell.strip * 4, w, v);
+                if (i < cell.rows) store_row4<IO, VEC>(row, cell.strip * 4, w, v);
                 __syncwarp();
             }
         }
@@ -225,7 +225,7 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
                         v[0] += g.x; v[1] += g.y; v[2] += g.z; v[3] += g.w;
                     }
                 }
-                if (i < cell.rows) flat_store_row<IO, VEC>(row, cell.strip * 4, w, v);
+                if (i < cell.rows) store_row4<IO, VEC>(row, cell.strip * 4, w, v);
                 __syncwarp();
             }
         }
@@ -358,7 +358,7 @@ forward_flat_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
                     for (int m = 0; m < kStrip; ++m) v[m] = fmaxf(v[m], 0.0f);
                 }
             }
-            if (i < cell.rows) flat_store_row<IO, VEC>(row, cell.strip * 4, w, v);
+            if (i < cell.rows) store_row4<IO, VEC>(row, cell.strip * 4, w, v);
             row += w;
         }
     }

@@ -626,9 +626,11 @@ inline bool plane_prefers_global_forward_integ(int64_t planes, int F, int h, int
 inline bool plane_fits_backward(int F, int h, int w) { return warp_tiles(h, w) <= kMaxTiles && flat_fits_backward(F, h, w); }
 
 // From the input's integral image, large planes are better off as slabs where they are wide enough or leave half of
-// the SMs idle ((4,16,4,96,160): 36 us against 48; (1,17,8,143,44): 32 us against 82, (5,4,4,216,56): 28 against 58).
+// the SMs idle ((12,3,4,128,191): 29 us against 51; (48,1,6,64,392): 45, 85), unless twelve tiles of strips hold them and few samples spread their filters or
+// many fill the GPU ((573,1,6,29,336): 174 us as slabs, 132; (17,1,6,24,338): 24, 18; but (45,1,8,20,396): 32, 50).
 inline bool plane_prefers_slabs_backward(int64_t planes, int F, int h, int w)
 {
+    if (((w + 3) / 4) * ((h + 7) / 8) <= 12 * 32 && (planes <= 20 || planes > 148)) return false;
     return (w > 96 || planes <= 74) && warp_tiles(h, w) > 8 && !quad_fits_backward(F, h, w);
 }
 

@@ -146,7 +146,7 @@ forward_slab_kernel(const float *__restrict__ integ, BoxParams bp, IO *out, int 
                             for (int m = 0; m < kStrip; ++m) v[m] = fmaxf(v[m], 0.0f);
                         }
                     }
-                    store_row4_wide<IO, VEC>(out + off - q0, q0, w, v, lane);
+                    store_row4<IO, VEC>(out + off - q0, q0, w, v);
                     off += w;
                 }
             }
@@ -276,7 +276,7 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
             if (i < mine) {
                 const float4 g = kept.grad_input(i);
                 float v[kStrip] = {g.x, g.y, g.z, g.w};
-                store_row4<IO, VEC>(row, q0, w, v, lane);
+                store_row4<IO, VEC>(row, q0, w, v);
             }
     }
     tmem_release();
