@@ -111,60 +111,69 @@ __device__ __forceinline__ void init_integral_padding(float *sI, const Geometry 
 }
 
 // Register block of a strip while the integral image is being built.
-struct Block {
-    float v[kR][kStrip];
-    float carry[kR];
+template <int T>
+struct Blocks {
+    float v[T][kR][kStrip];
+    float carry[T][kR];
 };
 
 // Build, part 1: fetch every strip's 8 x 4 block (from the staged copy of the plane in shared
 // memory when STAGED, else from global memory), prefix it along rows inside the thread and across
 // the 8 column-group lanes, publish the tile's row totals.  Ends with a barrier, after which the
 // staged plane is no longer needed.
-template <typename IO, bool FAST, bool STAGED, bool MAYBE_RELU = false>
-__device__ __forceinline__ void build_rows(Block &b, const Strip &st, const IO *__restrict__ src,
+template <typename IO, int T, bool FAST, bool STAGED, bool MAYBE_RELU = false>
+__device__ __forceinline__ void build_rows(Blocks<T> &b, const Strip (&st)[T], const IO *__restrict__ src,
                                            uint32_t sG32, float *sRow, const Geometry &g, int cg, int rg,
                                            bool relu = false)
 {
 #pragma unroll
-    for (int i = 0; i < kR; ++i) {
-        if (STAGED) {
-            const float4 t = st.active ? Io<IO>::lds4(sG32 + (st.pix + i * g.w) * (uint32_t)sizeof(IO))
-                                          : make_float4(0.f, 0.f, 0.f, 0.f);
-            b.v[i][0] = t.x; b.v[i][1] = t.y; b.v[i][2] = t.z; b.v[i][3] = t.w;
-        } else if (FAST) {
-            const float4 t = st.active ? Io<IO>::load4(src + st.pix + i * g.w) : make_float4(0.f, 0.f, 0.f, 0.f);
-            b.v[i][0] = t.x; b.v[i][1] = t.y; b.v[i][2] = t.z; b.v[i][3] = t.w;
-        } else {
-            const bool in = st.active && st.p0 + i < g.h;
+    for (int k = 0; k < T; ++k) {
 #pragma unroll
-            for (int m = 0; m < kStrip; ++m)
-                b.v[i][m] = (in && st.q0 + m < g.w) ? Io<IO>::load1(src + st.pix + i * g.w + m) : 0.0f;
+        for (int i = 0; i < kR; ++i) {
+            if (STAGED) {
+                const float4 t = st[k].active ? Io<IO>::lds4(sG32 + (st[k].pix + i * g.w) * (uint32_t)sizeof(IO))
+                                              : make_float4(0.f, 0.f, 0.f, 0.f);
+                b.v[k][i][0] = t.x; b.v[k][i][1] = t.y; b.v[k][i][2] = t.z; b.v[k][i][3] = t.w;
+            } else if (FAST) {
+                const float4 t = st[k].active ? Io<IO>::load4(src + st[k].pix + i * g.w) : make_float4(0.f, 0.f, 0.f, 0.f);
+                b.v[k][i][0] = t.x; b.v[k][i][1] = t.y; b.v[k][i][2] = t.z; b.v[k][i][3] = t.w;
+            } else {
+                const bool in = st[k].active && st[k].p0 + i < g.h;
+#pragma unroll
+                for (int m = 0; m < kStrip; ++m)
+                    b.v[k][i][m] = (in && st[k].q0 + m < g.w) ? Io<IO>::load1(src + st[k].pix + i * g.w + m) : 0.0f;
+            }
         }
     }
     if (MAYBE_RELU && relu) {
 #pragma unroll
-        for (int i = 0; i < kR; ++i)
+        for (int k = 0; k < T; ++k)
 #pragma unroll
-            for (int m = 0; m < kStrip; ++m) b.v[i][m] = fmaxf(b.v[i][m], 0.0f);
+            for (int i = 0; i < kR; ++i)
+#pragma unroll
+                for (int m = 0; m < kStrip; ++m) b.v[k][i][m] = fmaxf(b.v[k][i][m], 0.0f);
     }
-    float tot[kR];
 #pragma unroll
-    for (int i = 0; i < kR; ++i) {
-        b.v[i][1] += b.v[i][0]; b.v[i][2] += b.v[i][1]; b.v[i][3] += b.v[i][2];
-        const float own = b.v[i][3];
-        float incl = own;
+    for (int k = 0; k < T; ++k) {
+        float tot[kR];
 #pragma unroll
-        for (int d = 1; d < 8; d <<= 1) {
-            const float u = __shfl_up_sync(0xffffffffu, incl, d, 8);
-            incl += cg >= d ? u : 0.0f;
+        for (int i = 0; i < kR; ++i) {
+            b.v[k][i][1] += b.v[k][i][0]; b.v[k][i][2] += b.v[k][i][1]; b.v[k][i][3] += b.v[k][i][2];
+            const float own = b.v[k][i][3];
+            float incl = own;
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1) {
+                const float u = __shfl_up_sync(0xffffffffu, incl, d, 8);
+                incl += cg >= d ? u : 0.0f;
+            }
+            b.carry[k][i] = incl - own;
+            tot[i] = incl;
         }
-        b.carry[i] = incl - own;
-        tot[i] = incl;
-    }
-    if (cg == 7 && st.tile) {
-        float4 *dst = reinterpret_cast<float4 *>(sRow + (st.ct * g.row_tiles + st.rt) * kTile + rg * kR);
-        dst[0] = make_float4(tot[0], tot[1], tot[2], tot[3]);
-        dst[1] = make_float4(tot[4], tot[5], tot[6], tot[7]);
+        if (cg == 7 && st[k].tile) {
+            float4 *dst = reinterpret_cast<float4 *>(sRow + (st[k].ct * g.row_tiles + st[k].rt) * kTile + rg * kR);
+            dst[0] = make_float4(tot[0], tot[1], tot[2], tot[3]);
+            dst[1] = make_float4(tot[4], tot[5], tot[6], tot[7]);
+        }
     }
     __syncthreads();
 }
@@ -172,67 +181,73 @@ __device__ __forceinline__ void build_rows(Block &b, const Strip &st, const IO *
 // Build, part 2: row totals of the tiles to the left, prefix down the columns (thread, the 4
 // row-group lanes, tiles above), store rows p0+1 .. p0+8 with the right-hand padding.  Ends with
 // a barrier: the integral image is complete.
-template <bool FAST>
-__device__ __forceinline__ void build_columns(Block &b, const Strip &st, float *sRow, float *sCol,
+template <int T, bool FAST>
+__device__ __forceinline__ void build_columns(Blocks<T> &b, const Strip (&st)[T], float *sRow, float *sCol,
                                               const Geometry &g, int cg, int rg)
 {
-    float ccarry[kStrip];
-    if (st.tile) {
-        for (int c2 = 0; c2 < st.ct; ++c2) {
-            const float4 *s = reinterpret_cast<const float4 *>(sRow + (c2 * g.row_tiles + st.rt) * kTile + rg * kR);
-            const float4 x = s[0], y = s[1];
-            b.carry[0] += x.x; b.carry[1] += x.y; b.carry[2] += x.z; b.carry[3] += x.w;
-            b.carry[4] += y.x; b.carry[5] += y.y; b.carry[6] += y.z; b.carry[7] += y.w;
+    float ccarry[T][kStrip];
+#pragma unroll
+    for (int k = 0; k < T; ++k) {
+        if (st[k].tile) {
+            for (int c2 = 0; c2 < st[k].ct; ++c2) {
+                const float4 *s = reinterpret_cast<const float4 *>(sRow + (c2 * g.row_tiles + st[k].rt) * kTile + rg * kR);
+                const float4 x = s[0], y = s[1];
+                b.carry[k][0] += x.x; b.carry[k][1] += x.y; b.carry[k][2] += x.z; b.carry[k][3] += x.w;
+                b.carry[k][4] += y.x; b.carry[k][5] += y.y; b.carry[k][6] += y.z; b.carry[k][7] += y.w;
+            }
         }
-    }
-    // apply the row carry and run the in-thread column prefix in the same sweep
+        // apply the row carry and run the in-thread column prefix in the same sweep
 #pragma unroll
-    for (int m = 0; m < kStrip; ++m) b.v[0][m] += b.carry[0];
+        for (int m = 0; m < kStrip; ++m) b.v[k][0][m] += b.carry[k][0];
 #pragma unroll
-    for (int i = 1; i < kR; ++i)
+        for (int i = 1; i < kR; ++i)
 #pragma unroll
-        for (int m = 0; m < kStrip; ++m) b.v[i][m] += b.carry[i] + b.v[i - 1][m];
+            for (int m = 0; m < kStrip; ++m) b.v[k][i][m] += b.carry[k][i] + b.v[k][i - 1][m];
 
-    float tot[kStrip];
+        float tot[kStrip];
 #pragma unroll
-    for (int m = 0; m < kStrip; ++m) {
-        const float own = b.v[kR - 1][m];
-        float incl = own;
-        float u = __shfl_up_sync(0xffffffffu, incl, 8);
-        incl += rg >= 1 ? u : 0.0f;
-        u = __shfl_up_sync(0xffffffffu, incl, 16);
-        incl += rg >= 2 ? u : 0.0f;
-        ccarry[m] = incl - own;
-        tot[m] = incl;
-    }
-    if (rg == 3 && st.tile)
-        *reinterpret_cast<float4 *>(sCol + (st.rt * g.col_tiles + st.ct) * kTile + cg * kStrip) =
-            make_float4(tot[0], tot[1], tot[2], tot[3]);
-    __syncthreads();
-    if (st.tile) {
-        for (int r2 = 0; r2 < st.rt; ++r2) {
-            const float4 x = *reinterpret_cast<const float4 *>(sCol + (r2 * g.col_tiles + st.ct) * kTile + cg * kStrip);
-            ccarry[0] += x.x; ccarry[1] += x.y; ccarry[2] += x.z; ccarry[3] += x.w;
+        for (int m = 0; m < kStrip; ++m) {
+            const float own = b.v[k][kR - 1][m];
+            float incl = own;
+            float u = __shfl_up_sync(0xffffffffu, incl, 8);
+            incl += rg >= 1 ? u : 0.0f;
+            u = __shfl_up_sync(0xffffffffu, incl, 16);
+            incl += rg >= 2 ? u : 0.0f;
+            ccarry[k][m] = incl - own;
+            tot[m] = incl;
         }
+        if (rg == 3 && st[k].tile)
+            *reinterpret_cast<float4 *>(sCol + (st[k].rt * g.col_tiles + st[k].ct) * kTile + cg * kStrip) =
+                make_float4(tot[0], tot[1], tot[2], tot[3]);
     }
-    if (st.active) {
-        const bool last = st.q0 + kStrip >= g.w;
-        const int npad = g.w - st.q0;      // padding columns still to fill (1..4) when `last`
+    __syncthreads();
 #pragma unroll
-        for (int i = 0; i < kR; ++i) {
-            if (FAST || st.p0 + i < g.h) {
-                // p0 is a multiple of 8, so only the last of the 8 rows moves to the next skew
-                const uint32_t ra = st.store + i * g.pitch4 + (i == kR - 1 ? 4 : 0);
-                const float x0 = b.v[i][0] + ccarry[0], x1 = b.v[i][1] + ccarry[1];
-                const float x2 = b.v[i][2] + ccarry[2], x3 = b.v[i][3] + ccarry[3];
-                // past the plane's last column the running value is I[a][w], which is exactly
-                // what the right-hand padding has to hold
-                sts<4>(ra, x0); sts<8>(ra, x1); sts<12>(ra, x2); sts<16>(ra, x3);
-                if (last) {
-                    sts<20>(ra, x3);
-                    if (npad > 1) sts<24>(ra, x3);
-                    if (npad > 2) sts<28>(ra, x3);
-                    if (npad > 3) sts<32>(ra, x3);
+    for (int k = 0; k < T; ++k) {
+        if (st[k].tile) {
+            for (int r2 = 0; r2 < st[k].rt; ++r2) {
+                const float4 x = *reinterpret_cast<const float4 *>(sCol + (r2 * g.col_tiles + st[k].ct) * kTile + cg * kStrip);
+                ccarry[k][0] += x.x; ccarry[k][1] += x.y; ccarry[k][2] += x.z; ccarry[k][3] += x.w;
+            }
+        }
+        if (st[k].active) {
+            const bool last = st[k].q0 + kStrip >= g.w;
+            const int npad = g.w - st[k].q0;      // padding columns still to fill (1..4) when `last`
+#pragma unroll
+            for (int i = 0; i < kR; ++i) {
+                if (FAST || st[k].p0 + i < g.h) {
+                    // p0 is a multiple of 8, so only the last of the 8 rows moves to the next skew
+                    const uint32_t ra = st[k].store + i * g.pitch4 + (i == kR - 1 ? 4 : 0);
+                    const float x0 = b.v[k][i][0] + ccarry[k][0], x1 = b.v[k][i][1] + ccarry[k][1];
+                    const float x2 = b.v[k][i][2] + ccarry[k][2], x3 = b.v[k][i][3] + ccarry[k][3];
+                    // past the plane's last column the running value is I[a][w], which is exactly
+                    // what the right-hand padding has to hold
+                    sts<4>(ra, x0); sts<8>(ra, x1); sts<12>(ra, x2); sts<16>(ra, x3);
+                    if (last) {
+                        sts<20>(ra, x3);
+                        if (npad > 1) sts<24>(ra, x3);
+                        if (npad > 2) sts<28>(ra, x3);
+                        if (npad > 3) sts<32>(ra, x3);
+                    }
                 }
             }
         }
@@ -256,8 +271,8 @@ __device__ __forceinline__ Walk make_walk(uint32_t sI32, const BoxTaps &t, int q
 // so it is not declared restrict).
 // INTEG: `integ` holds the plane's integral image, plain rows of w + 1 floats, which is only copied (instantiations of
 // their own: as a run-time branch it cost the others 3 to 5 %).
-template <typename IO, bool FAST, bool FUSED = false, bool INTEG = false>
-__global__ void __launch_bounds__(256, FUSED ? 2 : 4)
+template <typename IO, int T, bool FAST, bool FUSED = false, bool INTEG = false>
+__global__ void __launch_bounds__(T == 1 ? 256 : 512, T == 1 ? (FUSED ? 2 : 4) : 1)
 forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, BoxParams bp, IO *out, int C, int F,
                      int h, int w, int fsplit, bool normalize, bool exact, Fusion fu)
 {
@@ -281,7 +296,9 @@ forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, 
     if (FUSED && fu.residual) prefetch_l2(fu.residual + (nc * F + f_begin) * (int64_t)h * w, (size_t)(f_end - f_begin) * h * w * sizeof(float));
     if (FAST && !INTEG && IsFloat<IO>::value && threadIdx.x == 0 && part == 0)
         bulk_prefetch_l2(x + nc * (int64_t)h * w, (uint32_t)(h * w) * 4u);
-    const Strip st = make_strip(g, sI32, warp, cg, rg);
+    Strip st[T];
+#pragma unroll
+    for (int k = 0; k < T; ++k) st[k] = make_strip(g, sI32, warp + k * nwarps, cg, rg);
     init_integral_padding(sI, g);
 
     // everything above touches registers and shared memory only (and hints); from here on the parameters and
@@ -300,9 +317,9 @@ forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, 
                            [&](int a, int col, float e) { sI[a * pitch + (a >> 3) + kPad + col] = e; });
         __syncthreads();
     } else {
-        Block blk;
-        build_rows<IO, FAST, false, FUSED>(blk, st, x + nc * (int64_t)h * w, 0u, sRow, g, cg, rg, FUSED && fu.input_relu);
-        build_columns<FAST>(blk, st, sRow, sCol, g, cg, rg);
+        Blocks<T> blk;
+        build_rows<IO, T, FAST, false, FUSED>(blk, st, x + nc * (int64_t)h * w, 0u, sRow, g, cg, rg, FUSED && fu.input_relu);
+        build_columns<T, FAST>(blk, st, sRow, sCol, g, cg, rg);
     }
 
     for (int f = f_begin; f < f_end; ++f) {
@@ -315,64 +332,67 @@ forward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ integ, 
             if (fu.scale) mul = __ldg(fu.scale + c * F + f);
             if (fu.shift) add = __ldg(fu.shift + c * F + f);
         }
-        if (!st.active) continue;
-        const Walk wk = make_walk(sI32, t, st.q0, g);
-        f2_t prev[kStrip];                 // (d of row lo-1, d of row hi) of the current pixel row
-        load_pair(wk, st.p0 + t.lo_r - 1, st.p0 + t.hi_r, cw, prev);
-        IO *dst = o + st.pix;
-        const float *res = (FUSED && fu.residual) ? fu.residual + (nc * F + f) * (int64_t)h * w + st.pix : nullptr;
-        float4 skip[FUSED ? kR : 1];       // all residual rows in flight before the gather
-        if (FUSED && res) {
 #pragma unroll
-            for (int i = 0; i < kR; ++i, res += w) {
-                if (FAST) {
-                    skip[FUSED ? i : 0] = *reinterpret_cast<const float4 *>(res);
-                } else {
-                    const bool in = st.p0 + i < h;
-                    const int q = st.q0;
-                    skip[FUSED ? i : 0] = make_float4(in ? res[0] : 0.f, in && q + 1 < w ? res[1] : 0.f, in && q + 2 < w ? res[2] : 0.f,
-                                                      in && q + 3 < w ? res[3] : 0.f);
+        for (int k = 0; k < T; ++k) {
+            if (!st[k].active) continue;
+            const Walk wk = make_walk(sI32, t, st[k].q0, g);
+            f2_t prev[kStrip];                 // (d of row lo-1, d of row hi) of the current pixel row
+            load_pair(wk, st[k].p0 + t.lo_r - 1, st[k].p0 + t.hi_r, cw, prev);
+            IO *dst = o + st[k].pix;
+            const float *res = (FUSED && fu.residual) ? fu.residual + (nc * F + f) * (int64_t)h * w + st[k].pix : nullptr;
+            float4 skip[FUSED ? kR : 1];       // all residual rows in flight before the gather
+            if (FUSED && res) {
+#pragma unroll
+                for (int i = 0; i < kR; ++i, res += w) {
+                    if (FAST) {
+                        skip[FUSED ? i : 0] = *reinterpret_cast<const float4 *>(res);
+                    } else {
+                        const bool in = st[k].p0 + i < h;
+                        const int q = st[k].q0;
+                        skip[FUSED ? i : 0] = make_float4(in ? res[0] : 0.f, in && q + 1 < w ? res[1] : 0.f, in && q + 2 < w ? res[2] : 0.f,
+                                                          in && q + 3 < w ? res[3] : 0.f);
+                    }
                 }
             }
-        }
 #pragma unroll
-        for (int i = 0; i < kR; ++i) {
-            const int p = st.p0 + i;
-            if (FAST || p < h) {
-                f2_t cur[kStrip];          // (d of row lo, d of row hi+1)
-                load_pair(wk, p + t.lo_r, p + t.hi_r + 1, cw, cur);
-                float v[kStrip];
+            for (int i = 0; i < kR; ++i) {
+                const int p = st[k].p0 + i;
+                if (FAST || p < h) {
+                    f2_t cur[kStrip];          // (d of row lo, d of row hi+1)
+                    load_pair(wk, p + t.lo_r, p + t.hi_r + 1, cw, cur);
+                    float v[kStrip];
 #pragma unroll
-                for (int m = 0; m < kStrip; ++m) {
-                    // (C - B) + f_hi (D - C) + f_lo (B - A), times scale
-                    float b, dd, a, cc, top, bot;
-                    unpack2(cur[m], b, dd);
-                    unpack2(prev[m], a, cc);
-                    unpack2(sub2(cur[m], prev[m]), top, bot);
-                    v[m] = (cc - b) * t.scale + sfh * bot + sfl * top;
-                    (void)a; (void)dd;
-                    prev[m] = cur[m];
-                }
-                if (FUSED) {
-#pragma unroll
-                    for (int m = 0; m < kStrip; ++m) v[m] = v[m] * mul + add;
-                    if (res) {
-                        const float4 r = skip[FUSED ? i : 0];
-                        v[0] += r.x; v[1] += r.y; v[2] += r.z; v[3] += r.w;
+                    for (int m = 0; m < kStrip; ++m) {
+                        // (C - B) + f_hi (D - C) + f_lo (B - A), times scale
+                        float b, dd, a, cc, top, bot;
+                        unpack2(cur[m], b, dd);
+                        unpack2(prev[m], a, cc);
+                        unpack2(sub2(cur[m], prev[m]), top, bot);
+                        v[m] = (cc - b) * t.scale + sfh * bot + sfl * top;
+                        (void)a; (void)dd;
+                        prev[m] = cur[m];
                     }
-                    if (fu.output_relu) {
+                    if (FUSED) {
 #pragma unroll
-                        for (int m = 0; m < kStrip; ++m) v[m] = fmaxf(v[m], 0.0f);
+                        for (int m = 0; m < kStrip; ++m) v[m] = v[m] * mul + add;
+                        if (res) {
+                            const float4 r = skip[FUSED ? i : 0];
+                            v[0] += r.x; v[1] += r.y; v[2] += r.z; v[3] += r.w;
+                        }
+                        if (fu.output_relu) {
+#pragma unroll
+                            for (int m = 0; m < kStrip; ++m) v[m] = fmaxf(v[m], 0.0f);
+                        }
                     }
-                }
-                if (FAST) {
-                    Io<IO>::store4(dst, v[0], v[1], v[2], v[3]);
-                } else {
+                    if (FAST) {
+                        Io<IO>::store4(dst, v[0], v[1], v[2], v[3]);
+                    } else {
 #pragma unroll
-                    for (int m = 0; m < kStrip; ++m)
-                        if (st.q0 + m < w) Io<IO>::store1(dst + m, v[m]);
+                        for (int m = 0; m < kStrip; ++m)
+                            if (st[k].q0 + m < w) Io<IO>::store1(dst + m, v[m]);
+                    }
+                    dst += w;
                 }
-                dst += w;
             }
         }
     }
@@ -415,7 +435,7 @@ backward_square_kernel(const IO *__restrict__ x, const float *__restrict__ x_int
     const uint32_t plane_bytes = (uint32_t)npix * (uint32_t)sizeof(IO);
     bool timed_out = false;
 
-    const Strip st = make_strip(g, sI32, warp, cg, rg);
+    Strip st[1] = {make_strip(g, sI32, warp, cg, rg)};
 
     // The first copies are started as early as possible, by a thread of the second warp (when there is
     // one) so that they do not queue behind the box arithmetic of the first warp's threads.  That thread
@@ -465,9 +485,9 @@ backward_square_kernel(const IO *__restrict__ x, const float *__restrict__ x_int
     for (int f = 0; f < F; ++f) {
         // (the barrier that ends the previous iteration protects sI, sRow, sCol)
         {
-            Block blk;
+            Blocks<1> blk;
             if (STAGED) timed_out |= !mbar_wait(mbarG, f & 1);
-            build_rows<IO, true, STAGED>(blk, st, gbase + f * (int64_t)npix, sG32, sRow, g, cg, rg);
+            build_rows<IO, 1, true, STAGED>(blk, st, gbase + f * (int64_t)npix, sG32, sRow, g, cg, rg);
             if (STAGED && tid == 0 && f + 1 < F) {
                 // every thread has taken its block out of the staging buffer (barrier above)
                 fence_proxy_async();
@@ -475,13 +495,13 @@ backward_square_kernel(const IO *__restrict__ x, const float *__restrict__ x_int
                 // the plane after that one on its way to L2 already (about 1 % on 256-sample batches)
                 if (f + 2 < F) bulk_prefetch_l2(gbase + (f + 2) * (int64_t)npix, plane_bytes);
             }
-            build_columns<true>(blk, st, sRow, sCol, g, cg, rg);
+            build_columns<1, true>(blk, st, sRow, sCol, g, cg, rg);
         }
         if (!STAGED && f + 1 < F && cg == 0) {
             // pull the next grad_output plane towards L2 while this one is gathered
 #pragma unroll
             for (int i = 0; i < kR; ++i)
-                if (st.active) asm volatile("prefetch.global.L2 [%0];" ::"l"(gbase + (f + 1) * (int64_t)npix + st.pix + i * w));
+                if (st[0].active) asm volatile("prefetch.global.L2 [%0];" ::"l"(gbase + (f + 1) * (int64_t)npix + st[0].pix + i * w));
         }
         if (X_BY_COPY && NEED_PARAMS && !INTEG && f == 0) timed_out |= !mbar_wait(mbarX, 0);
 
@@ -494,13 +514,13 @@ backward_square_kernel(const IO *__restrict__ x, const float *__restrict__ x_int
         float s_out = 0.f;
         f2_t topbot2 = pack2(0.f, 0.f);
         f2_t leftP = pack2(0.f, 0.f), leftQ = pack2(0.f, 0.f), rightP = pack2(0.f, 0.f), rightQ = pack2(0.f, 0.f);
-        if (st.active) {
-            const int p0 = st.p0;
-            const Walk wk = make_walk(sI32, t, st.q0, g);
+        if (st[0].active) {
+            const int p0 = st[0].p0;
+            const Walk wk = make_walk(sI32, t, st[0].q0, g);
             if (NEED_PARAMS) {
                 f2_t pd[kStrip], pel[kStrip], peh[kStrip];
                 load_pair_e(wk, p0 + t.lo_r - 1, p0 + t.hi_r, cw, pd, pel, peh);
-                uint32_t xa = sX32 + st.pix * 4;
+                uint32_t xa = sX32 + st[0].pix * 4;
 #pragma unroll
                 for (int i = 0; i < kR; ++i) {
                     f2_t cd[kStrip], cel[kStrip], ceh[kStrip];
@@ -576,8 +596,8 @@ backward_square_kernel(const IO *__restrict__ x, const float *__restrict__ x_int
     }
     if (STAGED && timed_out && lane == 0) atomicAdd(&g_wait_timeouts, 1);
 
-    if (write_gin && st.active) {
-        IO *dst = grad_input + nc * (int64_t)npix + st.pix;
+    if (write_gin && st[0].active) {
+        IO *dst = grad_input + nc * (int64_t)npix + st[0].pix;
 #pragma unroll
         for (int i = 0; i < kR; ++i, dst += w) Io<IO>::store4(dst, gin[i][0], gin[i][1], gin[i][2], gin[i][3]);
     }
@@ -662,15 +682,18 @@ inline bool flat_beats_square(int F, int h, int w)
     return F > 1 && tiles > 4 && tiles * 32 * 10 > strips * 17;
 }
 
-// The same in the forward, by the fixed tiles that it has or else would have (`quad`: of 8 x 128).  More than eight of 32 x 32: always ((1050,1,8,134,33), 10 tiles for 4.8,
-// 122 us against 85; (289,2,1,168,72) 33 and 21; of 61 aligned drawn planes of few samples 0.76 of the time, of 21 with over 600 samples 0.84;
-// 139 unaligned ones 0.77).  Up to eight, with filters' CTAs to hand and several on an SM, they are as fast or faster (few samples: 0.9 of the time).
-// Against more than eight of 8 x 128: where rows are cut or unaligned, or a fifth of the lanes idle ((6,3,4,184,77) 8.9 and 6.9, (14,8,4,35,224) 16.8 and 10.1;
+// The same in the forward, by the fixed tiles that it has or else would have (`quad`: of 8 x 128).
+// More than eight of 32 x 32: where rows are cut or unaligned ((1050,1,8,134,33), 10 tiles for 4.8, 122 us against 85; 139 drawn planes 0.77 of the time), where
+// they waste more than a quarter ((693,1,1,48,280) 37.7 and 27.5; (419,1,3,272,40) 40.9 and 27.0; 40 planes 0.8; below that 1.03 to 1.15: (1239,1,1,128,96) 36 and
+// 41, (1221,1,4,88,144) 91 and 104), and of few samples ((3,1,4,280,96) 9.5 and 7.9; 25 planes 0.85).  Up to eight, with filters' CTAs to hand and several on
+// an SM, they are as fast or faster.
+// Against more than eight of 8 x 128: where rows are cut or unaligned, or two fifths of the lanes idle ((6,3,4,184,77) 8.9 and 6.9, (14,8,4,35,224) 16.8 and 10.1;
 // 41 such planes 0.81).
-inline bool flat_suits_forward(int h, int w, bool quad, bool aligned)
+inline bool flat_suits_forward(int64_t planes, int h, int w, bool quad, bool aligned)
 {
     const int tiles = quad ? quad_row_tiles(h) * quad_col_tiles(w) : warp_tiles(h, w), strips = ((w + 3) / 4) * ((h + 7) / 8);
-    return tiles > 8 && (!quad || !aligned || tiles * 32 * 10 > strips * 16);
+    if (tiles <= 8) return false;
+    return !aligned || (!quad && planes < 40) || tiles * 32 * 100 > strips * (quad ? 160 : 128);
 }
 // From the input's integral image: of few samples also smaller planes (51 aligned ones 0.87, 59 unaligned ones 0.96 of the time).
 inline bool flat_suits_forward_integ(int64_t planes, int h, int w, bool quad)
@@ -691,7 +714,7 @@ int launch_forward_plane_t(const IO *x, const float *integ, const BoxParams &bp,
     const bool fast = (h % kR == 0) && (w % kStrip == 0) && aligned_to(x, vec) && aligned_to(out, vec) &&
                       (!fu || !fu->residual || aligned_to(fu->residual, 16));
     const bool quad = quad_fits_forward(F, h, w) && (x ? quad_prefers_forward(planes, F, h, w) : quad_prefers_forward_integ(planes, F, h, w));
-    if (x ? flat_suits_forward(h, w, quad, fast) : flat_suits_forward_integ(planes, h, w, quad))
+    if (x ? flat_suits_forward(planes, h, w, quad, fast) : flat_suits_forward_integ(planes, h, w, quad))
         return launch_forward_flat(x, integ, Io<IO>::kKind, bp, fu, out, N, C, F, h, w, normalize, exact, s);
     if (quad) return launch_forward_quad_t<IO>(x, integ, bp, fu, out, N, C, F, h, w, normalize, exact, s);
     // Split the filters of a plane over two CTAs when there are too few planes to balance 148 SMs
@@ -702,19 +725,23 @@ int launch_forward_plane_t(const IO *x, const float *integ, const BoxParams &bp,
     if (planes * fsplit > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
     const size_t smem = plane_forward_smem_bytes(h, w);
     const int tiles = warp_tiles(h, w);
-    if (tiles > 8) return BC_ERR_UNSUPPORTED;      // (a tile a warp; flat_suits_forward() has taken larger planes)
+    // one tile per warp up to 8 tiles, two beyond (up to 16 warps: a CTA of a large plane has the SM to itself)
+    const int T = tiles > 8 ? 2 : 1;
+    if (T == 2 && !(fast && x)) return BC_ERR_UNSUPPORTED;      // (flat_suits_forward() has taken those)
+    const int warps = (tiles + T - 1) / T;
     void (*kern)(const IO *, const float *, BoxParams, IO *, int, int, int, int, int, bool, bool, Fusion);
     constexpr bool FL = IsFloat<IO>::value;      // (integral images are float)
     if (fu && !FL) return BC_ERR_UNSUPPORTED;
-    if (!x) kern = fast ? forward_plane_kernel<IO, true, false, FL> : forward_plane_kernel<IO, false, false, FL>;
-    else if (fu) kern = fast ? forward_plane_kernel<IO, true, FL> : forward_plane_kernel<IO, false, FL>;
-    else kern = fast ? forward_plane_kernel<IO, true> : forward_plane_kernel<IO, false>;
+    if (T == 2) kern = fu ? forward_plane_kernel<IO, 2, true, FL> : forward_plane_kernel<IO, 2, true>;
+    else if (!x) kern = fast ? forward_plane_kernel<IO, 1, true, false, FL> : forward_plane_kernel<IO, 1, false, false, FL>;
+    else if (fu) kern = fast ? forward_plane_kernel<IO, 1, true, FL> : forward_plane_kernel<IO, 1, false, FL>;
+    else kern = fast ? forward_plane_kernel<IO, 1, true> : forward_plane_kernel<IO, 1, false>;
     int st = opt_in_smem(kern, smem);
     if (st != BC_OK) return st;
     const Fusion none{0, nullptr, nullptr, nullptr, 0};
     {
         LaunchScope scope(KID_FORWARD_PLANE, s);
-        if (cudaError_t e = launch_overlapped(kern, (unsigned)(planes * fsplit), tiles * 32, smem, s, x, integ, bp, out, C, F, h, w,
+        if (cudaError_t e = launch_overlapped(kern, (unsigned)(planes * fsplit), warps * 32, smem, s, x, integ, bp, out, C, F, h, w,
                                               fsplit, normalize, exact, fu ? *fu : none))
             return cuda_failed(e, "forward_plane");
     }
