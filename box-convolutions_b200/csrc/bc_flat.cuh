@@ -325,8 +325,10 @@ struct FlatCols {
 __device__ __forceinline__ uint32_t flat_window(uint32_t (&sub)[kStrip + 1], int strip, int shift, const FlatShape &sh)
 {
     const int r = shift & 3;
+    uint32_t at = (uint32_t)(r * sh.sub);
+    sub[0] = at;
 #pragma unroll
-    for (int m = 0; m <= kStrip; ++m) sub[m] = (uint32_t)(((r + m) & 3) * sh.sub + (r + m < 4 ? 0 : 4));
+    for (int m = 1; m <= kStrip; ++m) sub[m] = at = r + m == 4 ? 4u : at + (uint32_t)sh.sub;
     return (uint32_t)(min(max(strip + (shift >> 2), -2), sh.strips) + 2) * 4u;
 }
 __device__ __forceinline__ FlatCols flat_cols(const BoxTaps &t, const FlatCell &cell, uint32_t image, const FlatShape &sh)

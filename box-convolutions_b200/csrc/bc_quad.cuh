@@ -62,11 +62,11 @@ __device__ __forceinline__ void quad_window(uint32_t (&off)[kStrip + 1], int j, 
 {
     const int r = shift & 3, j0 = j + (shift >> 2);
     const uint32_t a = (uint32_t)(min(max(j0, -1), cells - 2) + 1) * 4u, b = (uint32_t)(min(max(j0 + 1, -1), cells - 2) + 1) * 4u;
+    // tap after tap one sub-row on, from the fourth to the first of the next cell: an addition and a selection each
+    uint32_t at = (uint32_t)(r * stride * 4) + a;
+    off[0] = at;
 #pragma unroll
-    for (int m = 0; m <= kStrip; ++m) {
-        const int s = r + m;
-        off[m] = (uint32_t)((s & 3) * stride * 4) + (s < 4 ? a : b);
-    }
+    for (int m = 1; m <= kStrip; ++m) off[m] = at = r + m == 4 ? b : at + (uint32_t)(stride * 4);
 }
 __device__ __forceinline__ QuadCols quad_cols(const BoxTaps &t, int j, int cells, int stride)
 {
