@@ -322,21 +322,27 @@ __device__ __forceinline__ void flat_put(FlatBlock &v, const FlatCell &cell, con
 struct FlatCols {
     uint32_t lo, hi, lo_sub[kStrip + 1], hi_sub[kStrip + 1];
 };
+// STEPS: tap after tap, as quad_window() has it (forward 0.985 of the time over 130 drawn planes; backward 1.012, whose registers are short).
+template <bool STEPS>
 __device__ __forceinline__ uint32_t flat_window(uint32_t (&sub)[kStrip + 1], int strip, int shift, const FlatShape &sh)
 {
     const int r = shift & 3;
     uint32_t at = (uint32_t)(r * sh.sub);
-    sub[0] = at;
+    if (STEPS) sub[0] = at;
 #pragma unroll
-    for (int m = 1; m <= kStrip; ++m) sub[m] = at = r + m == 4 ? 4u : at + (uint32_t)sh.sub;
+    for (int m = STEPS ? 1 : 0; m <= kStrip; ++m) {
+        at = r + m == 4 ? 4u : at + (uint32_t)sh.sub;
+        sub[m] = STEPS ? at : (uint32_t)(((r + m) & 3) * sh.sub + (r + m < 4 ? 0 : 4));
+    }
     return (uint32_t)(min(max(strip + (shift >> 2), -2), sh.strips) + 2) * 4u;
 }
+template <bool STEPS>
 __device__ __forceinline__ FlatCols flat_cols(const BoxTaps &t, const FlatCell &cell, uint32_t image, const FlatShape &sh)
 {
     FlatCols c;
     image += cell.plane * sh.plane;
-    c.lo = image + flat_window(c.lo_sub, cell.strip, t.lo_c - 1, sh);
-    c.hi = image + flat_window(c.hi_sub, cell.strip, t.hi_c, sh);
+    c.lo = image + flat_window<STEPS>(c.lo_sub, cell.strip, t.lo_c - 1, sh);
+    c.hi = image + flat_window<STEPS>(c.hi_sub, cell.strip, t.hi_c, sh);
     return c;
 }
 __device__ __forceinline__ void quad_taps(const FlatCols &c, uint32_t row0, uint32_t row1, f2_t (&l)[kStrip + 1], f2_t (&h)[kStrip + 1])

@@ -147,6 +147,32 @@ __device__ __forceinline__ float pixel_of_integral(const float *I, int pitch)
     return __ldg(I + pitch + 1) - __ldg(I + 1) - __ldg(I + pitch) + __ldg(I);
 }
 
+// The same for eight rows of columns c .. c+3 from the integral row `I` above them on (rows of w + 1): every value is loaded once, not by all
+// four pixels around it, and all of them are in flight together.  Zero at or past `rows` and column w.
+template <class Emit>
+__device__ __forceinline__ void pixels_of_integral(const float *I, int w, int c, int rows, Emit &&emit)
+{
+    float prev[5];
+    int at[5];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+        at[m] = min(c + m, w);
+        prev[m] = rows > 0 ? __ldg(I + at[m]) : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        float cur[5], e[4];
+        I += w + 1;
+#pragma unroll
+        for (int m = 0; m < 5; ++m) cur[m] = i < rows ? __ldg(I + at[m]) : 0.0f;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) e[m] = i < rows && c + m < w ? cur[m + 1] - prev[m + 1] - cur[m] + prev[m] : 0.0f;
+        emit(i, make_float4(e[0], e[1], e[2], e[3]));
+#pragma unroll
+        for (int m = 0; m < 5; ++m) prev[m] = cur[m];
+    }
+}
+
 // ---- rows of four columns a lane, whatever their alignment -------------------------------------
 // A warp works on 128 adjacent columns, lane L on columns c .. c+3 with c = c0 + 4 L.  Rows whose length is no
 // multiple of four start anywhere relative to a 4-element boundary; k, the same for the whole warp, is by how

@@ -93,14 +93,8 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
         } else if (!x) {
             // the caller has only the input's integral image: its pixels are second differences
             const FlatCell &cell = mine;
-            const float *I = x_integ + ((int64_t)(n0 + cell.plane) * C + c) * (h + 1) * (w + 1) + cell.group * kFlatRows * (w + 1) + cell.strip * 4;
-#pragma unroll 4
-            for (int i = 0; i < kFlatRows; ++i, I += w + 1) {
-                float e[4];
-#pragma unroll
-                for (int m = 0; m < 4; ++m) e[m] = i < cell.rows && cell.strip * 4 + m < w ? pixel_of_integral(I + m, w + 1) : 0.0f;
-                kept.init(i, make_float4(e[0], e[1], e[2], e[3]));
-            }
+            const float *I = x_integ + ((int64_t)(n0 + cell.plane) * C + c) * (h + 1) * (w + 1) + cell.group * kFlatRows * (w + 1);
+            pixels_of_integral(I, w, cell.strip * 4, cell.rows, [&](int i, const float4 &e) { kept.init(i, e); });
         } else {
             FlatBlock v;
             flat_load<IO, VEC>(v, x + pixel_of(mine), w, mine, lane, sh.strips);
@@ -150,7 +144,7 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
             FlatKept<T> kept(tmem_base, warp, k, sh.split == 1 || f + 1 == f_end ? 0 : (f - f_begin + 1) * flat_slot_columns(T, nwarps),
                              lds<9 * 4>(s.taps + f * kTapWords * 4));
             float sums[kNumSums] = {0.f, 0.f, 0.f, 0.f, 0.f};
-            const FlatCols cols = flat_cols(t, cell, s.image, sh);
+            const FlatCols cols = flat_cols<false>(t, cell, s.image, sh);
             if (__all_sync(0xffffffffu, cell.rows == kFlatRows || cell.rows == 0))
                 quad_backward_strip<kFlatRows, NEED_PARAMS, true, kPacked>(t, cols, flat_rows<false>(t, cell, h, sh), cw, kept, sums, kFlatRows);
             else
@@ -319,7 +313,7 @@ forward_flat_kernel(const IO *__restrict__ x, const float *__restrict__ integ, B
         if (tile != at) cell = flat_cell(sh, tile * 32 + lane, planes, h);
         at = tile;
         const BoxTaps t = load_taps_uniform(sTaps + k * kTapWords);
-        const FlatCols cols = flat_cols(t, cell, s.image, sh);
+        const FlatCols cols = flat_cols<true>(t, cell, s.image, sh);
         const FlatRows<false> q = flat_rows<false>(t, cell, h, sh);
         const ColW2 cw = col_weights(t);
         const float sfl = t.scale * t.f_lo_r, sfh = t.scale * t.f_hi_r;

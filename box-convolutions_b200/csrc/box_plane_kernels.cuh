@@ -646,11 +646,15 @@ inline bool plane_prefers_global_forward_integ(int64_t planes, int F, int h, int
 inline bool plane_fits_backward(int F, int h, int w) { return warp_tiles(h, w) <= kMaxTiles && flat_fits_backward(F, h, w); }
 
 // From the input's integral image, large planes are better off as slabs where they are wide enough or leave half of
-// the SMs idle ((12,3,4,128,191): 29 us against 51; (48,1,6,64,392): 45, 85), unless twelve tiles of strips hold them and few samples spread their filters or
-// many fill the GPU ((573,1,6,29,336): 174 us as slabs, 132; (17,1,6,24,338): 24, 18; but (45,1,8,20,396): 32, 50).
+// the SMs idle ((8,1,1,43,326): 13.2 us against 16.8; (43,1,6,176,108), 19 tiles of strips: 38, 62), unless 16 tiles of strips hold them and the
+// filters are worth spreading over CTAs ((4,16,4,96,160): 31.6 as slabs, 27.3; (8,1,8,104,144) 31.0, 21.0; with four filters not of few rows:
+// (48,1,4,40,352) 23.6, 26.6), or 12 do and few samples spread them or many fill the GPU ((573,1,6,29,336): 174, 132; (17,1,6,24,338): 24, 18;
+// but (45,1,8,20,396): 32, 50).
 inline bool plane_prefers_slabs_backward(int64_t planes, int F, int h, int w)
 {
-    if (((w + 3) / 4) * ((h + 7) / 8) <= 12 * 32 && (planes <= 20 || planes > 148)) return false;
+    const int strips = ((w + 3) / 4) * ((h + 7) / 8);
+    if (strips <= 12 * 32 && (planes <= 20 || planes > 148)) return false;
+    if (strips > 12 * 32 && strips <= 16 * 32 && (F >= 6 || (F >= 4 && h >= 64))) return false;
     return (w > 96 || planes <= 74) && warp_tiles(h, w) > 8 && !quad_fits_backward(F, h, w);
 }
 

@@ -409,13 +409,7 @@ backward_quad_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
         if (!x) {
             // the caller has only the input's integral image: its pixels are second differences
             const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1) + (int64_t)tile.p0 * (w + 1);
-#pragma unroll 4
-            for (int i = 0; i < kTileRows; ++i, I += w + 1) {
-                float e[4];
-#pragma unroll
-                for (int m = 0; m < 4; ++m) e[m] = i < tile.rows && tile.c + m < w ? pixel_of_integral(I + tile.c + m, w + 1) : 0.0f;
-                kept.init(i, make_float4(e[0], e[1], e[2], e[3]));
-            }
+            pixels_of_integral(I, w, tile.c, tile.c < w ? tile.rows : 0, [&](int i, const float4 &e) { kept.init(i, e); });
         } else {
 #pragma unroll
             for (int i = 0; i < kTileRows; ++i) kept.init(i, rows8_get<IO, FAST>(g, xrow, w, tile.c, lane, i));

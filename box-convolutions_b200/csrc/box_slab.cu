@@ -216,14 +216,8 @@ backward_slab_kernel(const IO *__restrict__ x, const float *__restrict__ x_integ
 #pragma unroll
             for (int i = 0; i < kStripRows; ++i) kept.init(i, rows8_get<IO, VEC>(g, xrow, w, q0, lane, i));
         } else {      // the caller has only the input's integral image: its pixels are second differences
-            const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1) + (int64_t)p0 * (w + 1) + q0;
-#pragma unroll 4
-            for (int i = 0; i < kStripRows; ++i, I += w + 1) {
-                float e[4];
-#pragma unroll
-                for (int m = 0; m < kStrip; ++m) e[m] = i < mine && q0 + m < w ? pixel_of_integral(I + m, w + 1) : 0.0f;
-                kept.init(i, make_float4(e[0], e[1], e[2], e[3]));
-            }
+            const float *I = x_integ + nc * (int64_t)(h + 1) * (w + 1) + (int64_t)p0 * (w + 1);
+            pixels_of_integral(I, w, q0, q0 < w ? mine : 0, [&](int i, const float4 &e) { kept.init(i, e); });
         }
     } else {
 #pragma unroll
