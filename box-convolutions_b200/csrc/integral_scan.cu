@@ -10,6 +10,7 @@
 // is in flight at once; with many, a CTA walks down its plane.  What the tiles above add to a tile's columns comes
 // through shared memory and, across CTAs, through distributed shared memory.
 #include "bc_cluster.cuh"
+#include "scan_shape.cuh"
 #include "bc_common.cuh"
 #include "bc_quad.cuh"
 #include "bc_tile_io.cuh"
@@ -18,7 +19,6 @@ namespace bc {
 
 namespace {
 
-constexpr int kScanWarps = 16;             // warps a CTA
 constexpr int kScanRows = 8;               // rows a warp works on at a time
 
 __device__ __forceinline__ float4 relu4(float4 v)
@@ -183,12 +183,14 @@ integral_tile_kernel(const IO *__restrict__ in, float *__restrict__ out, int h, 
         for (int k = 0, r = r0; k < steps; ++k, r += stride, at += (int64_t)stride * w) {
             Rows8 t;
             rows8_load<IO, VEC, false, LN>(t, at, w, c, h - r, lane);
+            float4 pair[kScanRows / 2];      // (added up in a tree: one rounding in three of a row after the other's)
 #pragma unroll
-            for (int i = 0; i < kScanRows; ++i) {
-                float4 v = rows8_get<IO, VEC, LN>(t, at, w, c, lane, i);
-                if (relu) v = relu4(v);
-                sum = add4(sum, v);
+            for (int i = 0; i < kScanRows; i += 2) {
+                float4 u = rows8_get<IO, VEC, LN>(t, at, w, c, lane, i), v = rows8_get<IO, VEC, LN>(t, at, w, c, lane, i + 1);
+                if (relu) u = relu4(u), v = relu4(v);
+                pair[i / 2] = add4(u, v);
             }
+            sum = add4(sum, add4(add4(pair[0], pair[1]), add4(pair[2], pair[3])));
         }
         float4 total;
         over_groups(sum, total);
@@ -391,33 +393,6 @@ integral_ordered_kernel(const IO *__restrict__ in, float *__restrict__ out, int 
     }
 }
 
-// How a plane of `tiles` warps' rows and `warps` warps a row is dealt out.  Few planes: to a cluster of at most 8 CTAs of
-// up to 16 warps, which hold it whole if they can (steps = 1; else they read it twice).  Many: to one CTA of 8 warps,
-// which walks down it ((512,256,512): 102 us against 148 as clusters; CTAs of 16 warps 109), or of 16 where there are
-// fewer planes than SMs and a cluster would read them twice in two steps ((130,161,715): 64 us, clusters 78; in three
-// steps, (108,260,860): 92, 81).  `many16`: planes up to which the CTAs that walk have 16 warps.
-struct ScanShape {
-    int G, ctas, steps;
-};
-inline ScanShape scan_shape(int64_t planes, int tiles, int warps, int many16 = 148)
-{
-    ScanShape s;
-    const int most = kScanWarps / warps;
-    s.ctas = (tiles + most - 1) / most;
-    s.steps = 1;
-    if (s.ctas > 1 && (planes >= 148 || (planes >= 100 && s.ctas > 8 && s.ctas <= 16))) {
-        s.ctas = 1;
-        const int fit = planes < many16 ? most : (8 / warps > 1 ? 8 / warps : 1);
-        s.steps = (tiles + fit - 1) / fit;
-    } else if (s.ctas > 8) {
-        s.steps = (s.ctas + 7) / 8;
-        s.ctas = 8;
-    }
-    const int parts = s.ctas * s.steps;
-    s.G = (tiles + parts - 1) / parts;
-    return s;
-}
-
 template <typename IO, bool QUAD, int LN>
 int integral_tile_t(const IO *in, float *out, int64_t planes, int h, int w, bool relu, cudaStream_t s)
 {
@@ -425,7 +400,8 @@ int integral_tile_t(const IO *in, float *out, int64_t planes, int h, int w, bool
     const bool vec = w % 4 == 0 && aligned_to(in, Io<IO>::kVecBytes);
     // two CTAs of 16 warps an SM: up to one and a half rounds of them ((256,280,560): 80 us, 149 with 8 warps; (404,60,341):
     // 21, 33; (424,568,105): 67, 77); not in the quad layout (368 planes of 110 x 450: 6 us more)
-    const ScanShape sh = scan_shape(planes, (h + warp_rows - 1) / warp_rows, warps, QUAD ? 148 : 3 * 148);
+    const int tiles = (h + warp_rows - 1) / warp_rows;
+    const ScanShape sh = scan_clusters_that_fit(scan_shape(planes, tiles, warps, QUAD ? 148 : 3 * 148), planes, tiles, warps, QUAD);
     if (planes * sh.ctas > 0x7fffffffLL) return BC_ERR_BAD_SHAPE;
     void (*kern)(const IO *, float *, int, int, int, int, int, int, bool);
     if (sh.G * warps <= 8) kern = vec ? integral_tile_kernel<IO, true, QUAD, LN, 256> : integral_tile_kernel<IO, false, QUAD, LN, 256>;
