@@ -145,7 +145,10 @@ backward_plane_kernel(const IO *__restrict__ x, const float *__restrict__ x_inte
                              lds<9 * 4>(s.taps + f * kTapWords * 4));
             float sums[kNumSums] = {0.f, 0.f, 0.f, 0.f, 0.f};
             const FlatCols cols = flat_cols<false>(t, cell, s.image, sh);
-            if (__all_sync(0xffffffffu, cell.rows == kFlatRows || cell.rows == 0))
+            // Of small CTAs, of which an SM runs several, all warps take the same of the two paths: 1300 instructions each, and with both
+            // warps wait for instructions longer than for anything else (2.3 of 8.5 cycles an instruction, (300,4,4,134,33)): cut planes
+            // of up to 8 tiles, 148 or more, 0.88 of the time (35 drawn ones), fewer 1.02, of more tiles 1.00 to 1.01.
+            if (h % kFlatRows == 0 || ((sh.tiles > 8 || gridDim.x < 148) && __all_sync(0xffffffffu, cell.rows == kFlatRows || cell.rows == 0)))
                 quad_backward_strip<kFlatRows, NEED_PARAMS, true, kPacked>(t, cols, flat_rows<false>(t, cell, h, sh), cw, kept, sums, kFlatRows);
             else
                 quad_backward_strip<kFlatRows, NEED_PARAMS, true, kPacked, true>(t, cols, flat_rows<true>(t, cell, h, sh), cw, kept, sums, cell.rows);
