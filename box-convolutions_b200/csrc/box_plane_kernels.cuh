@@ -693,17 +693,21 @@ inline bool flat_beats_square(int F, int h, int w)
 // an SM, they are as fast or faster.
 // Against more than eight of 8 x 128: where rows are cut or unaligned, or two fifths of the lanes idle ((6,3,4,184,77) 8.9 and 6.9, (14,8,4,35,224) 16.8 and 10.1;
 // 41 such planes 0.81).
-inline bool flat_suits_forward(int64_t planes, int h, int w, bool quad, bool aligned)
+// Not against 8 x 128 of a few planes so large that these are split by rows ((5,1,4,112,246) fused 10.6 us, 13.5; (3,1,4,214,115) 8.9, 10.4), nor with one or
+// two filters of some ((64,1,1,91,159) 9.0, 10.9; (15,1,1,168,90) 7.6, 8.6; fused ones gain).
+inline bool flat_suits_forward(int64_t planes, int F, int h, int w, bool quad, bool aligned, bool fused)
 {
     const int tiles = quad ? quad_row_tiles(h) * quad_col_tiles(w) : warp_tiles(h, w), strips = ((w + 3) / 4) * ((h + 7) / 8);
-    if (tiles <= 8) return false;
+    if (tiles <= 8 || (quad && planes <= 6 && strips > 20 * 32)) return false;
+    if (quad && !fused && F <= 2 && planes < 100 && strips > 8 * 32) return false;
     return !aligned || (!quad && planes < 40) || tiles * 32 * 100 > strips * (quad ? 160 : 128);
 }
-// From the input's integral image: of few samples also smaller planes (51 aligned ones 0.87, 59 unaligned ones 0.96 of the time).
-inline bool flat_suits_forward_integ(int64_t planes, int h, int w, bool quad)
+// From the input's integral image: of few samples also smaller planes (51 aligned ones 0.87, 59 unaligned ones 0.96 of the time), but not of one
+// to four square tiles ((12,16,4,20,58) 8.0 us, 9.3; (1,90,8,38,41) 10.5, 13.6), nor with many filters ((1,93,8,30,75) 12.3, 14.2).
+inline bool flat_suits_forward_integ(int64_t planes, int F, int h, int w, bool quad)
 {
     const int tiles = quad ? quad_row_tiles(h) * quad_col_tiles(w) : warp_tiles(h, w);
-    return tiles > 8 || planes < 600;
+    return tiles > 8 || (planes < 600 && (quad ? planes * F < 400 : tiles > 4));
 }
 
 // `fu` (inference steps around the gather) exists for float tensors only.
@@ -718,7 +722,7 @@ int launch_forward_plane_t(const IO *x, const float *integ, const BoxParams &bp,
     const bool fast = (h % kR == 0) && (w % kStrip == 0) && aligned_to(x, vec) && aligned_to(out, vec) &&
                       (!fu || !fu->residual || aligned_to(fu->residual, 16));
     const bool quad = quad_fits_forward(F, h, w) && (x ? quad_prefers_forward(planes, F, h, w) : quad_prefers_forward_integ(planes, F, h, w));
-    if (x ? flat_suits_forward(planes, h, w, quad, fast) : flat_suits_forward_integ(planes, h, w, quad))
+    if (x ? flat_suits_forward(planes, F, h, w, quad, fast, fu != nullptr) : flat_suits_forward_integ(planes, F, h, w, quad))
         return launch_forward_flat(x, integ, Io<IO>::kKind, bp, fu, out, N, C, F, h, w, normalize, exact, s);
     if (quad) return launch_forward_quad_t<IO>(x, integ, bp, fu, out, N, C, F, h, w, normalize, exact, s);
     // Split the filters of a plane over two CTAs when there are too few planes to balance 148 SMs

@@ -32,8 +32,8 @@ def test_gradients_against_float64(shape, dtype):
     assert max_rel(gp.cpu().numpy(), want_p.cpu().numpy()) < 1e-3 + ROUNDING[dtype]
 
 
-FORWARD = [(1, 2, 3, 72, 133), (3, 2, 4, 96, 132), (2, 75, 1, 130, 50), (40, 4, 6, 280, 26), (1, 2, 4, 1020, 30), (1, 2, 2, 1024, 32), (1, 1, 3, 31, 1020), (2, 3, 2, 93, 157), (150, 1, 2, 110, 117),
-           (1, 3, 4, 126, 252), (1, 16, 2, 192, 136), (5, 2, 1, 40, 300)]
+FORWARD = [(1, 2, 3, 72, 133), (3, 2, 4, 96, 132), (2, 75, 1, 130, 50), (40, 4, 6, 280, 26), (1, 2, 4, 1020, 30), (1, 2, 2, 1024, 32), (1, 1, 3, 31, 1020), (2, 3, 3, 93, 157), (150, 1, 2, 110, 117),
+           (2, 4, 4, 126, 252), (1, 16, 2, 192, 136), (5, 2, 1, 40, 300)]
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
