@@ -221,6 +221,7 @@ __device__ __forceinline__ void flat_scan(FlatBlock &v, float (&carry)[kFlatRows
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < kFlatRows; ++i) carry[i] = lds<0>(half[i >> 2] + (i & 3) * kPitch + lane * 4);
+    if (T > 1) __syncwarp();      // with two tiles a warp flat_publish() stores over these words
 }
 // Second part: the parts of the row in other tiles, and the strip's last row as what it adds to those below.  Followed by a barrier.
 __device__ __forceinline__ void flat_publish(FlatBlock &v, float (&carry)[kFlatRows], const FlatSmem &s, int first, int tile, uint32_t starts, int lane)

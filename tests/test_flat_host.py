@@ -1,10 +1,13 @@
 """The whole-plane kernels that deal out strips (csrc/bc_flat.cuh), compiled for the host: what a launch asks for is what the device and the
 packed fields of a strip hold, every plane that the kernel's predecessor took still fits, rows are where the kernels' clamped sums of offsets say,
-and neighbouring strips fall into neighbouring banks across row groups and planes.  CPU only."""
+neighbouring strips fall into neighbouring banks across row groups and planes, and scans need no order among lanes but that of their own
+barriers.  CPU only."""
 import ctypes
 import os
+import shutil
 import subprocess
 
+import numpy as np
 import pytest
 
 from conftest import PKG_DIR, ROOT
@@ -77,3 +80,34 @@ def test_layout(flat):
                 for j in range(9):
                     row = min(max(group * 8 + a + j, 0), h)
                     assert flat.flat_offset(h, w, group, a, j) == flat.flat_row(h, w, row), (h, w, group, a, j)
+
+
+@pytest.fixture(scope="module")
+def warp(tmp_path_factory):
+    at = tmp_path_factory.mktemp("warp")
+    shutil.copy(os.path.join(PKG_DIR, "csrc", "bc_flat.cuh"), at)
+    for name in ("bc_quad.cuh", "bc_tile_io.cuh", "bc_tmem.cuh"):
+        (at / name).write_text("")
+    out = str(at / "libwarp.so")
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I", str(at), "-o", out,
+                           os.path.join(ROOT, "tests", "host_emulation", "flat_warp.cpp")])
+    return ctypes.CDLL(out)
+
+
+# tiles a warp, rows, columns: strips that divide a tile (no barrier of the CTA between the scan and what follows it) and rows over two tiles
+@pytest.mark.parametrize("T,h,w", [(2, 512, 4), (2, 256, 8), (2, 128, 16), (2, 64, 32), (2, 32, 64), (2, 16, 128), (2, 63, 31), (2, 32, 60), (2, 24, 77), (2, 8, 250),
+                                   (1, 32, 32), (1, 15, 64), (1, 24, 40), (1, 8, 125)])
+@pytest.mark.parametrize("backwards", [0, 1])
+def test_scans_with_lanes_one_after_the_other(warp, T, h, w, backwards):
+    """Between two barriers lanes may run in any order: whole numbers, so that sums are exact."""
+    plane = np.random.RandomState(h + w).randint(-99, 100, (h, w)).astype(np.float32)
+    out, published = np.full((32 * T, 8, 4), np.nan, np.float32), np.full((32 * T, 4), np.nan, np.float32)
+    p = [a.ctypes.data_as(ctypes.c_void_p) for a in (plane, out, published)]
+    warp.flat_warp(T, backwards, h, w, *p)
+    strips, groups = -(-w // 4), -(-h // 8)
+    assert 32 * (T - 1) < strips * groups <= 32 * T
+    padded = np.zeros((groups * 8, strips * 4), np.float32)
+    padded[:h, :w] = plane
+    want = padded.reshape(groups, 8, strips * 4).cumsum(1).cumsum(2).reshape(groups, 8, strips, 4).transpose(0, 2, 1, 3).reshape(-1, 8, 4)
+    assert np.array_equal(out[:len(want)], want)
+    assert np.array_equal(published[:len(want)], want[:, 7])

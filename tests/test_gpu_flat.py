@@ -18,7 +18,7 @@ pytestmark = pytest.mark.gpu
 
 # samples, channels, filters, rows, columns
 SHAPES = [(1, 1, 1, 1, 1), (3, 2, 2, 7, 3), (2, 1, 3, 9, 29), (700, 1, 2, 8, 4), (650, 2, 1, 20, 25), (331, 2, 2, 21, 31), (301, 1, 4, 33, 37), (75, 4, 2, 72, 48), (2, 3, 3, 65, 61),
-          (1, 4, 2, 64, 300), (2, 2, 5, 24, 516), (1, 3, 8, 40, 260), (150, 1, 2, 88, 124), (3, 1, 4, 100, 130), (1, 150, 1, 110, 117), (2, 2, 3, 200, 60), (1, 2, 2, 280, 26), (1, 2, 6, 1020, 30),
+          (1, 4, 2, 64, 300), (2, 2, 5, 24, 516), (1, 3, 8, 40, 260), (150, 1, 2, 88, 124), (3, 1, 4, 100, 130), (1, 150, 1, 110, 117), (2, 2, 3, 200, 60), (1, 2, 2, 280, 26), (1, 2, 6, 1020, 30), (150, 1, 2, 256, 64),
           (1, 2, 3, 31, 1020), (2, 3, 4, 120, 200), (1, 2, 4, 126, 252)]
 
 
