@@ -659,13 +659,17 @@ inline bool plane_prefers_slabs_backward(int64_t planes, int F, int h, int w)
 }
 
 // On which planes the kernel that deals out strips (box_flat.cu) is faster than those with fixed tiles: it has fewer lanes without a
-// pixel, and a fifth more instructions a strip.  `strips`: a 32nd of its tiles.  The rules ask for sides and filters only,
-// so that a part of a batch runs on the kernel of the whole.  Samples, channels, filters, rows, columns:
+// pixel, and a fifth more instructions a strip.  `strips`: a 32nd of its tiles.  Samples, channels, filters, rows, columns:
 // against 8 x 128 tiles (795,2,4,40,150) 201 us -> 130; (2611,1,4,120,72) 438 -> 308; (202,3,4,48,144) 83 -> 64; but (1265,1,2,56,96), 7 tiles
 // for 5.25, 53.6 -> 56.8; (2104,1,4,80,120), 10 for 9.4, 213 -> 260; (111,8,6,86,126) 179 -> 209;
-// against pairs of them (575,1,4,128,72) 88 -> 76; (593,1,4,72,168) 166 -> 103; (653,1,8,80,240), 20 for 18.8, 318 -> 404; with one or two filters a wash;
+// against pairs of them, or few planes of which one tile a warp: (575,1,4,128,72) 88 -> 76; (593,1,4,72,168) 166 -> 103; (653,1,8,80,240), 20 for 18.8, 318 ->
+// 404; 14 and 16 tiles for two thirds of them to nine tenths (1500,1,8,112,92) 391 -> 424, (148,1,6,56,176) 34.8 -> 39.8, (149,1,8,64,200) 80 -> 102, though with
+// few planes, whose filters strips spread over a cluster, (37,1,6,64,200) 35.7 -> 26.0; with one or two filters up to 148 planes
+// (148,1,2,128,76) 16.3 -> 18.6, (37,1,2,64,140) 15.8 -> 15.0, above a wash but for the emptiest (700,1,2,56,136) 58 -> 45;
 // against 32 x 32 tiles, more than eight: always (below); fewer, aligned: (1042,1,8,72,40) 144 -> 83; (64,40), 4 for 2.5, 61 -> 62, with fewer
 // planes 1.1 to 1.4 times as long; unaligned (2857,1,6,47,36) 233 -> 106, (2858,1,4,110,36) in bfloat16 424 -> 149.
+// The rules ask for sides and filters only: kernels of different tiles add up in different orders, and a part of a batch is to
+// get the grad-input of the whole to the last bit.
 inline bool flat_beats_quad(int F, int h, int w)
 {
     const int tiles = quad_row_tiles(h) * quad_col_tiles(w), strips = ((w + 3) / 4) * ((h + 7) / 8);
@@ -677,13 +681,27 @@ inline bool flat_beats_pair(int F, int h, int w)
 {
     const int tiles = quad_row_tiles(h) * quad_col_tiles(w), strips = ((w + 3) / 4) * ((h + 7) / 8);
     if (F <= 2) return false;
-    if (tiles <= kQuadMaxWarps) return tiles * 32 * 20 > strips * 27;
+    if (tiles <= kQuadMaxWarps) return tiles * 32 * 10 > strips * 15;
     return strips <= 24 * 32 && tiles * 32 * 20 > strips * 25;
 }
 inline bool flat_beats_square(int F, int h, int w)
 {
     const int tiles = warp_tiles(h, w), strips = ((w + 3) / 4) * ((h + 7) / 8);
     return F > 1 && tiles > 4 && tiles * 32 * 10 > strips * 17;
+}
+
+// The backward kernel of a plane.  `pair_rows`: the input itself is given and all addresses fit the pair kernel's accesses; `fast`: rows and addresses
+// fit vector accesses.  The number of planes decides between the two kernels of 8 x 128 tiles, which add up alike, and, with one or two filters, between
+// pairs of them and strips for planes of 72 to 96 rows and 132 to 160 columns: only there does a part of a batch get another order of additions.
+enum PlaneBackward { BACKWARD_PAIR, BACKWARD_QUAD, BACKWARD_SQUARE, BACKWARD_STRIPS };
+inline PlaneBackward plane_backward_choice(int64_t planes, int F, int h, int w, bool wide, bool pair_rows, bool fast)
+{
+    const bool pairs = pair_rows && quad_pair_fits_backward(F, h, w, wide);
+    if (!(pairs ? flat_beats_pair(F, h, w) : flat_beats_quad(F, h, w))) {
+        if (pairs && quad_pair_suits_backward(planes, F, h, w, wide)) return BACKWARD_PAIR;
+        if (quad_fits_backward(F, h, w)) return BACKWARD_QUAD;
+    }
+    return !fast || w >= kQuadMinWidth || warp_tiles(h, w) > 8 || flat_beats_square(F, h, w) ? BACKWARD_STRIPS : BACKWARD_SQUARE;
 }
 
 // The same in the forward, by the fixed tiles that it has or else would have (`quad`: of 8 x 128).
@@ -695,6 +713,7 @@ inline bool flat_beats_square(int F, int h, int w)
 // 41 such planes 0.81).
 // Not against 8 x 128 of a few planes so large that these are split by rows ((5,1,4,112,246) fused 10.6 us, 13.5; (3,1,4,214,115) 8.9, 10.4), nor with one or
 // two filters of some ((64,1,1,91,159) 9.0, 10.9; (15,1,1,168,90) 7.6, 8.6; fused ones gain).
+// Unlike the backward's, these rules ask for the number of planes: outputs of a part of a batch that crosses a line agree with the whole's to rounding.
 inline bool flat_suits_forward(int64_t planes, int F, int h, int w, bool quad, bool aligned, bool fused)
 {
     const int tiles = quad ? quad_row_tiles(h) * quad_col_tiles(w) : warp_tiles(h, w), strips = ((w + 3) / 4) * ((h + 7) / 8);
@@ -766,20 +785,19 @@ int launch_backward_plane_t(const IO *x, const float *x_integ, const IO *grad_ou
     const bool need_params = (need_mask & (BC_NEED_ALL & ~BC_NEED_INPUT)) != 0;
     const bool write_gin = (need_mask & BC_NEED_INPUT) != 0;
     const int vec = Io<IO>::kVecBytes;
-    const bool pair = x && quad_pair_suits_backward(planes, F, h, w, IsFloat<IO>::value) && aligned_to(x, vec) && aligned_to(grad_output, 16) &&
-                      (!write_gin || aligned_to(grad_input, vec));
-    if (pair && !flat_beats_pair(F, h, w))
+    const bool fits = aligned_to(x, vec) && (!write_gin || aligned_to(grad_input, vec));
+    const PlaneBackward choice = plane_backward_choice(planes, F, h, w, IsFloat<IO>::value, x && fits && aligned_to(grad_output, 16),
+                                                       h % kR == 0 && w % kStrip == 0 && fits && aligned_to(grad_output, vec));
+    if (choice == BACKWARD_PAIR)
         return launch_backward_quad_pair_t<IO>(x, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input, grad_params,
                                                grad_params_kind, partials, s);
-    if (!pair && quad_fits_backward(F, h, w) && !flat_beats_quad(F, h, w))
+    if (choice == BACKWARD_QUAD)
         return launch_backward_quad_t<IO>(x, x_integ, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
                                           grad_params, grad_params_kind, partials, s);
-    const bool fast = (h % kR == 0) && (w % kStrip == 0) && aligned_to(x, vec) && aligned_to(grad_output, vec) &&
-                      (!write_gin || aligned_to(grad_input, vec));
-    const int tiles = warp_tiles(h, w);
-    if (!fast || w >= kQuadMinWidth || tiles > 8 || flat_beats_square(F, h, w))
+    if (choice == BACKWARD_STRIPS)
         return launch_backward_flat(x, x_integ, Io<IO>::kKind, grad_output, bp, rep_h, rep_w, N, C, F, h, w, normalize, exact, need_mask, grad_input,
                                     grad_params, grad_params_kind, partials, s);
+    const int tiles = warp_tiles(h, w);
     const size_t io = sizeof(IO);
     // bulk copies need 16-byte aligned planes of a multiple of 16 bytes and room for the staging buffer;
     // staging must not cost a resident CTA (two fit below ~112 KB each)

@@ -680,14 +680,20 @@ inline int quad_pair_max_threads(int col_tiles, int warps)
 // 14 and 16 tiles, which as one tile a warp have an SM to themselves: two CTAs of half the warps, if there are planes for two
 // ((16,32,4,128,128): 94, 105; (16,32,4,64,256): 91, 108; (64,32,4,112,96): 258, 329).  Not of 10 and 12 tiles, two CTAs an SM either
 // way ((16,32,4,96,128): 73, 68; (16,32,4,40,248): 71, 65).
-inline bool quad_pair_suits_backward(int64_t planes, int F, int h, int w, bool wide)
+// Two rules: of which sides and filters the kernel holds planes, and for how many planes it is the faster one of those with fixed tiles.
+inline bool quad_pair_fits_backward(int F, int h, int w, bool wide)
 {
     const int col_tiles = quad_col_tiles(w), tiles = quad_row_tiles(h) * col_tiles, square = ((h + 31) / 32) * ((w + 31) / 32);
     if (w < kQuadMinWidth || w > 256 || w % 4 || h % kTileRows || F > kMaxFilters || tiles % 2 || quad_backward_smem(F, h, w) > kQuadMaxSmem) return false;
-    if (tiles <= kQuadMaxWarps) return tiles > 12 && planes > 148;
-    if (col_tiles != 2 || tiles > 2 * kQuadMaxWarps) return false;
-    if (square <= 16 && F < 8 && !(planes <= 148 || (planes > 296 && planes <= 444))) return false;
-    return wide || 2 * tiles <= 3 * square;
+    if (tiles <= kQuadMaxWarps) return tiles > 12;
+    return col_tiles == 2 && tiles <= 2 * kQuadMaxWarps && (wide || 2 * tiles <= 3 * square);
+}
+inline bool quad_pair_suits_backward(int64_t planes, int F, int h, int w, bool wide)
+{
+    const int tiles = quad_row_tiles(h) * quad_col_tiles(w), square = ((h + 31) / 32) * ((w + 31) / 32);
+    if (!quad_pair_fits_backward(F, h, w, wide)) return false;
+    if (tiles <= kQuadMaxWarps) return planes > 148;
+    return square > 16 || F >= 8 || planes <= 148 || (planes > 296 && planes <= 444);
 }
 
 template <typename IO>

@@ -15,6 +15,13 @@ extern "C" int rule_pair_backward(int64_t planes, int F, int h, int w, int wide,
     return warps * 32;
 }
 
+// Which kernel the backward of an aligned plane runs in: 0 pairs of tiles, 1 one tile a warp, 2 square tiles, 3 strips.
+extern "C" int rule_backward(int64_t planes, int F, int h, int w, int wide)
+{
+    const bool fast = h % kTileRows == 0 && w % kStrip == 0;
+    return plane_backward_choice(planes, F, h, w, wide != 0, fast, fast);
+}
+
 // Does the forward through tensor memory serve the plane?  If so, the tiles of a plane, the warps that build it and the
 // tensor-memory columns of a CTA.
 extern "C" int rule_tmem_forward(int64_t planes, int F, int h, int w, int *tiles, int *warps, int *columns)

@@ -19,6 +19,7 @@ def rules(tmp_path_factory):
                            "-I", os.path.join(PKG_DIR, "csrc"), "-o", out, src])
     lib = ctypes.CDLL(out)
     lib.rule_pair_backward.argtypes = [ctypes.c_int64] + [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)] * 2
+    lib.rule_backward.argtypes = [ctypes.c_int64] + [ctypes.c_int] * 4
     lib.rule_tmem_forward.argtypes = [ctypes.c_int64] + [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_int)] * 3
     return lib
 
@@ -75,3 +76,26 @@ def test_sizes_that_other_kernels_are_faster_on_go_there(rules):
     assert all(rules.rule_tmem_forward(*c, *n) for c in FORWARD_HERE)
     assert not [c for c in PAIR_ELSEWHERE if rules.rule_pair_backward(*c, *n[:2])]
     assert all(rules.rule_pair_backward(*c, *n[:2]) for c in PAIR_HERE)
+
+
+# 14 and 16 tiles of 8 x 128: strips where a third of the lanes would idle, with three filters or more, for any number of planes
+STRIPS_HERE = [(575, 4, 128, 72, 1), (593, 4, 56, 140, 1), (37, 3, 64, 164, 1), (148, 8, 112, 84, 0), (1300, 4, 80, 144, 1), (722, 16, 88, 136, 1)]
+STRIPS_ELSEWHERE = [(148, 6, 56, 176, 0), (37, 6, 64, 200, 1), (1500, 8, 112, 92, 1), (149, 8, 64, 200, 1), (148, 2, 128, 76, 0), (300, 2, 128, 72, 1)]
+
+
+def test_backward_tiles_do_not_depend_on_the_number_of_planes(rules):
+    """Tiles of 8 x 128 add up alike one or two a warp, all others differently.  One or two filters on planes of 17 to 32 tiles that 16
+    square ones hold are the exception."""
+    assert all(rules.rule_backward(*c) == 3 for c in STRIPS_HERE)
+    assert not [c for c in STRIPS_ELSEWHERE if rules.rule_backward(*c) not in (0, 1)]
+    seen = set()
+    for h in list(range(8, 289, 8)) + [1, 33, 93]:
+        for w in list(range(4, 289, 4)) + [1, 65, 157]:
+            for F in (1, 2, 3, 4, 6, 8, 32):
+                if F <= 2 and 72 <= h <= 96 and 132 <= w <= 160:
+                    continue
+                for wide in (0, 1):
+                    kinds = [rules.rule_backward(planes, F, h, w, wide) for planes in (1, 37, 74, 148, 149, 296, 297, 444, 445, 5000)]
+                    assert len({max(k, 1) for k in kinds}) == 1, (F, h, w, wide, kinds)
+                    seen |= set(kinds)
+    assert seen == {0, 1, 2, 3}

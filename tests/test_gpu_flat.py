@@ -91,13 +91,18 @@ def test_four_functions_and_subsets(shape):
     assert max_rel(x.grad.cpu().numpy(), gin.cpu().numpy()) < 1e-6
 
 
-@pytest.mark.parametrize("shape", [(40, 8, 6, 50, 40), (300, 1, 5, 90, 60), (160, 1, 3, 152, 96)])
-def test_a_part_of_a_batch_gives_the_bits_of_the_whole(shape):
-    """Few samples have their filters spread over a cluster of CTAs."""
+# (the last one or two: tiles of 8 x 128, one a warp up to 148 planes and two above)
+@pytest.mark.parametrize("shape,kernels", [((40, 8, 6, 50, 40), {"backward_plane_kernel"}), ((300, 1, 5, 90, 60), {"backward_plane_kernel"}), ((160, 1, 3, 152, 96), {"backward_plane_kernel"}),
+                                           ((200, 1, 3, 72, 160), {"backward_plane_kernel"}), ((300, 1, 4, 128, 72), {"backward_plane_kernel"}),
+                                           ((150, 1, 2, 56, 160), {"backward_quad_kernel", "backward_quad_pair_kernel"}), ((300, 1, 2, 128, 72), {"backward_quad_kernel", "backward_quad_pair_kernel"}),
+                                           ((80, 2, 4, 64, 200), {"backward_quad_kernel", "backward_quad_pair_kernel"}), ((75, 2, 6, 112, 92), {"backward_quad_kernel", "backward_quad_pair_kernel"})])
+def test_a_part_of_a_batch_gives_the_bits_of_the_whole(shape, kernels):
+    """Few samples have their filters spread over a cluster of CTAs, or one tile a warp instead of two."""
     m, x, g = _case(shape, True, True)
     whole, _ = _grads(m, x, g)
-    assert "backward_plane_kernel" in kernels_run(lambda: _grads(m, x[:3], g[:3]))
-    for a, b in ((0, 1), (5, 8), (shape[0] - 30, shape[0])):
+    ran = [k for n in (3, shape[0]) for k in kernels_run(lambda: _grads(m, x[:n], g[:n])) if k.startswith("backward")]
+    assert set(ran) == kernels
+    for a, b in ((0, 1), (5, 8), (3, 40), (shape[0] - 30, shape[0])):
         part, _ = _grads(m, x[a:b], g[a:b])
         assert torch.equal(part, whole[a:b])
 
