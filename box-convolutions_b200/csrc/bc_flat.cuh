@@ -9,6 +9,8 @@
 // words (S strips a row), planes such that the next plane's first strip goes on where the last one ended: the 32 lanes of a
 // warp read and write 32 different banks although they work on several rows or planes.
 #pragma once
+#include <climits>
+
 #include "bc_quad.cuh"
 #include "bc_tile_io.cuh"
 #include "bc_tmem.cuh"
@@ -402,6 +404,18 @@ inline int flat_samples(int N, int C, int h, int w)
     return planes > 1 ? (int)planes : 1;
 }
 
+// CTAs of a backward that an SM holds (80 registers a thread, with two tiles a warp 128), and clusters of them that a GPU runs at once: as many as the
+// occupancy calculator has where each CTA needs an SM, because the GPU's parts have 14 to 20 SMs each and a cluster lies in one part.
+constexpr int kFlatMaxCluster = 8, kFlatClusters[kFlatMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+inline int flat_ctas_an_sm(int tiles_a_warp, int warps, int columns, size_t smem)
+{
+    const int most[] = {512 / columns, (tiles_a_warp == 1 ? 25 : 16) / warps, (int)(228 * 1024 / (smem + 1024))};
+    int n = 32;
+    for (int m : most) n = n > m ? m : n;
+    return n > 1 ? n : 1;
+}
+inline int64_t flat_clusters_at_once(int ctas, int an_sm) { return (int64_t)kFlatClusters[ctas] * an_sm; }
+
 struct FlatPlan {
     FlatShape sh;
     int tiles_a_warp, warps;
@@ -411,7 +425,9 @@ struct FlatPlan {
 // One tile a warp where the CTA's registers allow it (80 a thread, 24 warps): with two, half as many warps cover latencies ((134,3,8,128,147),
 // 19 tiles: 313 us against 226; (1335,1,3,232,104), 24 tiles: 429 against 351).  13 to 16 tiles: two, if there are planes for the second
 // CTA that then fits an SM ((217,1,1,192,80): 24.0 us, 24.6; (103,1,4,168,88), fewer planes than SMs: 45 with two, 33 with one).
-// Filters over several CTAs: 12 planes of 120 x 133, F = 8, 119 us -> 25; (5,1,8,280,34) 96 -> 18.
+// Filters over several CTAs: 12 planes of 120 x 133, F = 8, 119 us -> 25; (5,1,8,280,34) 96 -> 18.  Over as many as make rounds of clusters
+// times filters each (and one, for what a CTA does besides) least: 34 clusters of four, of which 33 run at once, took as long as 66 ((36,1,4,96,144) 32.0 us with
+// four CTAs, 24.8 with two; (18,1,8,136,112) 35.8 with eight, 27.6 with four; (48,1,3,48,320) 31.9 with three, 24.3 with two; 24 such launches 0.79 of the time).
 inline FlatPlan flat_backward_plan(int N, int C, int F, int h, int w, bool write_gin)
 {
     const int planes = flat_samples(N, C, h, w);
@@ -426,13 +442,19 @@ inline FlatPlan flat_backward_plan(int N, int C, int F, int h, int w, bool write
     const size_t rows = (size_t)p.sh.tiles * 32 * kFlatRows * 16;
     // A cluster's CTAs have to find room at once, with no more than eight warps on an SM and the tensor memory that their filters take.
     const int64_t room = 148 * (p.warps >= 8 ? 1 : 8 / p.warps);
-    for (int k = 2, best = F; k <= F && k <= 8 && ctas * k <= room; ++k) {
-        const int each = (F + k - 1) / k;
-        if (each < best && ctas * k <= 148 * (512 / pow2_columns(slot * each)) && rows * each <= kFlatMaxSmem) { best = each; p.sh.split = k; }
+    const size_t own = p.smem;
+    p.sh.columns = pow2_columns(slot);
+    for (int k = 1, least = INT_MAX; k <= F && k <= kFlatMaxCluster; ++k) {
+        const int each = (F + k - 1) / k, columns = pow2_columns(k > 1 ? slot * each : slot);
+        const size_t smem = k > 1 && write_gin && own < rows * each ? rows * each : own;
+        if (k > 1 && (ctas * k > room || ctas * k > 148 * (512 / columns) || rows * each > kFlatMaxSmem)) continue;
+        const int cost = (int)((ctas - 1) / flat_clusters_at_once(k, flat_ctas_an_sm(p.tiles_a_warp, p.warps, columns, smem)) + 1) * (each + 1);
+        if (cost >= least) continue;
+        least = cost;
+        p.sh.split = k;
+        p.sh.columns = columns;
+        p.smem = smem;
     }
-    const int each = p.sh.split > 1 ? (F + p.sh.split - 1) / p.sh.split : 1;
-    p.sh.columns = pow2_columns(slot * each);
-    if (p.sh.split > 1 && write_gin && p.smem < rows * each) p.smem = rows * each;
     return p;
 }
 

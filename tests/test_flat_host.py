@@ -57,6 +57,13 @@ def test_launches_fit(flat):
                     assert p["tiles"] * 4096 * each <= p["smem"], at
 
 
+# Planes with an SM to a CTA: (planes, filters, CTAs of a cluster) on both sides of what a GPU runs at once: 74 clusters of two, 45 of three, 33 of four, 15 of eight
+@pytest.mark.parametrize("planes,F,split", [(74, 4, 2), (75, 4, 1), (45, 3, 3), (46, 3, 2), (33, 4, 4), (34, 4, 2), (15, 8, 8), (16, 8, 4), (33, 8, 4)])
+@pytest.mark.parametrize("h,w", [(96, 144), (112, 132)])
+def test_clusters_run_at_once(flat, planes, F, split, h, w):
+    assert plan(flat, planes, 1, F, h, w)["split"] == split
+
+
 def test_forward_launches_fit(flat):
     for h, w in served():
         for N, C, F in ((1, 1, 1), (1, 3, 4), (7, 1, 6), (150, 1, 32), (3000, 2, 4)):
