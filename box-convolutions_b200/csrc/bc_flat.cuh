@@ -9,8 +9,6 @@
 // words (S strips a row), planes such that the next plane's first strip goes on where the last one ended: the 32 lanes of a
 // warp read and write 32 different banks although they work on several rows or planes.
 #pragma once
-#include <climits>
-
 #include "bc_quad.cuh"
 #include "bc_tile_io.cuh"
 #include "bc_tmem.cuh"
@@ -420,6 +418,8 @@ struct FlatPlan {
     FlatShape sh;
     int tiles_a_warp, warps;
     size_t smem;
+    int each, rounds;      // filters of a CTA; how often the GPU fills with CTAs
+    int full;              // percent of the room for CTAs that has filters to work on meanwhile
 };
 // How many samples share a CTA, tiles a warp, and how many CTAs share a plane's filters.
 // One tile a warp where the CTA's registers allow it (80 a thread, 24 warps): with two, half as many warps cover latencies ((134,3,8,128,147),
@@ -443,17 +443,21 @@ inline FlatPlan flat_backward_plan(int N, int C, int F, int h, int w, bool write
     // A cluster's CTAs have to find room at once, with no more than eight warps on an SM and the tensor memory that their filters take.
     const int64_t room = 148 * (p.warps >= 8 ? 1 : 8 / p.warps);
     const size_t own = p.smem;
-    p.sh.columns = pow2_columns(slot);
-    for (int k = 1, least = INT_MAX; k <= F && k <= kFlatMaxCluster; ++k) {
+    int64_t least = 0;
+    for (int k = 1; k <= F && k <= kFlatMaxCluster; ++k) {
         const int each = (F + k - 1) / k, columns = pow2_columns(k > 1 ? slot * each : slot);
         const size_t smem = k > 1 && write_gin && own < rows * each ? rows * each : own;
         if (k > 1 && (ctas * k > room || ctas * k > 148 * (512 / columns) || rows * each > kFlatMaxSmem)) continue;
-        const int cost = (int)((ctas - 1) / flat_clusters_at_once(k, flat_ctas_an_sm(p.tiles_a_warp, p.warps, columns, smem)) + 1) * (each + 1);
-        if (cost >= least) continue;
-        least = cost;
+        const int an_sm = flat_ctas_an_sm(p.tiles_a_warp, p.warps, columns, smem);
+        const int64_t rounds = (ctas - 1) / flat_clusters_at_once(k, an_sm) + 1;
+        if (k > 1 && rounds * (each + 1) >= least) continue;
+        least = rounds * (each + 1);
         p.sh.split = k;
         p.sh.columns = columns;
         p.smem = smem;
+        p.each = each;
+        p.rounds = (int)rounds;
+        p.full = (int)(ctas * F * 100 / (rounds * each * 148 * an_sm));
     }
     return p;
 }

@@ -38,6 +38,7 @@
 #pragma once
 #include "bc_common.cuh"
 #include "bc_finish.cuh"
+#include "bc_flat.cuh"
 #include "bc_smem_walk.cuh"
 #include "bc_tile_io.cuh"
 #include "bc_tmem.cuh"
@@ -646,16 +647,24 @@ inline bool plane_prefers_global_forward_integ(int64_t planes, int F, int h, int
 inline bool plane_fits_backward(int F, int h, int w) { return warp_tiles(h, w) <= kMaxTiles && flat_fits_backward(F, h, w); }
 
 // From the input's integral image, large planes are better off as slabs where they are wide enough or leave half of
-// the SMs idle ((8,1,1,43,326): 13.2 us against 16.8; (43,1,6,176,108), 19 tiles of strips: 38, 62), unless 16 tiles of strips hold them and the
-// filters are worth spreading over CTAs ((4,16,4,96,160): 31.6 as slabs, 27.3; (8,1,8,104,144) 31.0, 21.0; with four filters not of few rows:
-// (48,1,4,40,352) 23.6, 26.6), or 12 do and few samples spread them or many fill the GPU ((573,1,6,29,336): 174, 132; (17,1,6,24,338): 24, 18;
-// but (45,1,8,20,396): 32, 50).
+// the SMs idle ((8,1,1,43,326): 13.2 us against 16.8; (43,1,6,176,108), 19 tiles of strips: 38, 62), unless 12 tiles of strips hold them and few samples
+// spread their filters over CTAs or many fill the GPU ((573,1,6,29,336): 174, 132; (17,1,6,24,338): 24, 18; but (45,1,8,20,396): 32, 50).
+// 13 to 16 tiles of strips with four filters or more (few rows: six) take a CTA an SM, or two of two tiles a warp, and win where the GPU is full of them.
+// Filters over CTAs, all at once: with one each ((1,1,8,40,328) 26.4 us as slabs, 19.7; (2,1,4,86,175) 20.0, 20.8), eight filters or more ((20,1,8,80,188)
+// 34, 29; (10,1,16,203,64) 53, 31; in two rounds (37,1,8,75,194) 40, 59), or half of the SMs at work ((4,16,4,96,160) 31.8, 27.3; (34,1,4,190,78), 46 %,
+// 27, 30).  Not shared: 60 % at work ((8,16,4,96,160) 53, 35; (16,16,4,96,160) 91, 68; (64,16,4,96,160) 309, 220; (16,16,6,104,144) 146, 96;
+// (180,5,6,88,144) 379, 291; but (25,2,32,95,134), 34 %, 163, 246; (37,2,6,72,208), half, 41, 49; (80,2,8,88,144), 54 %, 108, 112), with fewer rows, which
+// slabs cut less, 88 % ((74,2,6,48,340) 71, 51; (45,2,8,25,446), 61 %, 52, 67; (125,2,32,26,395), 84 %, 434, 551).  Of 216 drawn launches: always
+// slabs 1, always strips 0.99 of that time, by this rule 0.90.
 inline bool plane_prefers_slabs_backward(int64_t planes, int F, int h, int w)
 {
     const int strips = ((w + 3) / 4) * ((h + 7) / 8);
-    if (strips <= 12 * 32 && (planes <= 20 || planes > 148)) return false;
-    if (strips > 12 * 32 && strips <= 16 * 32 && (F >= 6 || (F >= 4 && h >= 64))) return false;
-    return (w > 96 || planes <= 74) && warp_tiles(h, w) > 8 && !quad_fits_backward(F, h, w);
+    if ((w <= 96 && planes > 74) || warp_tiles(h, w) <= 8 || quad_fits_backward(F, h, w)) return false;
+    if (strips <= 12 * 32) return planes > 20 && planes <= 148;
+    if (strips > 16 * 32 || F < (h >= 64 ? 4 : 6)) return true;
+    const FlatPlan p = flat_backward_plan((int)(planes < 0x7fffffff ? planes : 0x7fffffff), 1, F, h, w, true);
+    if (p.sh.split > 1) return p.rounds > 1 || (p.each > 1 && F < 8 && p.full < 50);
+    return p.full < (h >= 64 ? 60 : 88);
 }
 
 // On which planes the kernel that deals out strips (box_flat.cu) is faster than those with fixed tiles: it has fewer lanes without a

@@ -22,6 +22,9 @@ extern "C" int rule_backward(int64_t planes, int F, int h, int w, int wide)
     return plane_backward_choice(planes, F, h, w, wide != 0, fast, fast);
 }
 
+// Backward from the input's integral image: by slabs?
+extern "C" int rule_slabs_backward(int64_t planes, int F, int h, int w) { return plane_prefers_slabs_backward(planes, F, h, w); }
+
 // Does the forward through tensor memory serve the plane?  If so, the tiles of a plane, the warps that build it and the
 // tensor-memory columns of a CTA.
 extern "C" int rule_tmem_forward(int64_t planes, int F, int h, int w, int *tiles, int *warps, int *columns)

@@ -20,6 +20,7 @@ def rules(tmp_path_factory):
     lib = ctypes.CDLL(out)
     lib.rule_pair_backward.argtypes = [ctypes.c_int64] + [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)] * 2
     lib.rule_backward.argtypes = [ctypes.c_int64] + [ctypes.c_int] * 4
+    lib.rule_slabs_backward.argtypes = [ctypes.c_int64] + [ctypes.c_int] * 3
     lib.rule_tmem_forward.argtypes = [ctypes.c_int64] + [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_int)] * 3
     return lib
 
@@ -99,3 +100,15 @@ def test_backward_tiles_do_not_depend_on_the_number_of_planes(rules):
                     assert len({max(k, 1) for k in kinds}) == 1, (F, h, w, wide, kinds)
                     seen |= set(kinds)
     assert seen == {0, 1, 2, 3}
+
+
+# Backward from the input's integral image, planes of 13 to 16 tiles of strips: planes, filters, rows, columns.
+SLABS_HERE = [(10, 32, 72, 184), (37, 16, 32, 492), (37, 8, 75, 194), (50, 6, 152, 96), (50, 32, 95, 134), (64, 6, 48, 284), (34, 4, 190, 78), (74, 6, 72, 208), (90, 8, 25, 446), (160, 8, 88, 144),
+              (160, 16, 38, 356), (200, 4, 48, 284), (250, 32, 26, 395), (1 << 40, 4, 48, 284)]
+SLABS_ELSEWHERE = [(1, 8, 40, 328), (8, 8, 104, 144), (10, 16, 203, 64), (20, 8, 80, 188), (50, 4, 120, 132), (64, 4, 96, 160), (128, 4, 96, 160), (256, 4, 96, 160), (1024, 4, 96, 160), (256, 6, 104, 144),
+                   (148, 6, 48, 340), (90, 8, 105, 136), (900, 6, 88, 144)]
+
+
+def test_slabs_where_strips_would_leave_the_gpu_idle(rules):
+    assert all(rules.rule_slabs_backward(*c) for c in SLABS_HERE)
+    assert not [c for c in SLABS_ELSEWHERE if rules.rule_slabs_backward(*c)]
