@@ -64,7 +64,7 @@ enum KernelId {
     KID_INTEGRAL = 1, KID_FORWARD_GLOBAL, KID_BACKWARD_GLOBAL, KID_FINISH_PARAM_GRADS, KID_CLIP,
     KID_FORWARD_PLANE, KID_BACKWARD_PLANE, KID_SUM_CHUNKS, KID_BACKWARD_BAND, KID_INTEGRAL_BANDS, KID_FORWARD_BAND,
     KID_FORWARD_SLAB, KID_BACKWARD_SLAB, KID_FORWARD_QUAD, KID_BACKWARD_QUAD,
-    KID_FORWARD_TMEM, KID_FORWARD_TMEM_STREAM, KID_BACKWARD_QUAD_PAIR, KID_BACKWARD_SQUARE, KID_COUNT
+    KID_FORWARD_TMEM, KID_FORWARD_TMEM_STREAM, KID_BACKWARD_QUAD_PAIR, KID_BACKWARD_SQUARE, KID_FORWARD_FLAT, KID_COUNT
 };
 
 // Put around a kernel launch: counts it and, while profiling is enabled, records a CUDA event on

@@ -424,7 +424,7 @@ int launch_forward_flat_t(const IO *x, const float *integ, const BoxParams &bp, 
     if (st != BC_OK) return st;
     const Fusion none{0, nullptr, nullptr, nullptr, 0};
     {
-        LaunchScope scope(KID_FORWARD_PLANE, s);
+        LaunchScope scope(KID_FORWARD_FLAT, s);
         if (cudaError_t e = launch_overlapped(kern, (unsigned)(ctas * tsplit), plan.warps * 32, plan.smem, s, x, integ, bp, out, N, C, F, h, w, plan.sh, plan.fsplit,
                                               tsplit, plan.tight, normalize, exact, fu ? *fu : none))
             return cuda_failed(e, "forward_flat");

@@ -803,6 +803,7 @@ const char *bc_kernel_name(int kernel_id)
         case KID_FORWARD_TMEM_STREAM: return "forward_tmem_stream_kernel";
         case KID_BACKWARD_QUAD_PAIR: return "backward_quad_pair_kernel";
         case KID_BACKWARD_SQUARE: return "backward_square_kernel";
+        case KID_FORWARD_FLAT: return "forward_flat_kernel";
         default: return "unknown";
     }
 }

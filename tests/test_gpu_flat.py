@@ -19,13 +19,16 @@ pytestmark = pytest.mark.gpu
 # samples, channels, filters, rows, columns
 SHAPES = [(1, 1, 1, 1, 1), (3, 2, 2, 7, 3), (2, 1, 3, 9, 29), (700, 1, 2, 8, 4), (650, 2, 1, 20, 25), (331, 2, 2, 21, 31), (301, 1, 4, 33, 37), (75, 4, 2, 72, 48), (2, 3, 3, 65, 61),
           (1, 4, 2, 64, 300), (2, 2, 5, 24, 516), (1, 3, 8, 40, 260), (150, 1, 2, 88, 124), (3, 1, 4, 100, 130), (1, 150, 1, 110, 117), (2, 2, 3, 200, 60), (1, 2, 2, 280, 26), (1, 2, 6, 1020, 30), (150, 1, 2, 256, 64),
-          (1, 2, 3, 31, 1020), (2, 3, 4, 120, 200), (1, 2, 4, 126, 252)]
+          (1, 2, 3, 31, 1020), (2, 3, 4, 120, 200), (1, 2, 4, 126, 252), (150, 1, 3, 96, 140), (149, 1, 2, 110, 130)]
+# ... of which fixed tiles serve
+FIXED = {(700, 1, 2, 8, 4): "backward_square_kernel", (150, 1, 2, 88, 124): "backward_quad_kernel", (1, 150, 1, 110, 117): "backward_quad_kernel"}
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("shape", SHAPES)
 def test_gradients_against_float64(shape, dtype):
     m, x, g = _case(shape, shape[3] % 3 != 0, True, dtype)
+    assert FIXED.get(shape, "backward_plane_kernel") in kernels_run(lambda: _grads(m, x, g))
     gin, gp = _grads(m, x, g)
     want_in, want_p = _grads(m.double(), x.double(), g.double())
     assert max_rel(gin.double().cpu().numpy(), want_in.cpu().numpy()) < 1e-4 + ROUNDING[dtype]
@@ -42,10 +45,42 @@ def test_outputs_against_float64(shape, dtype):
     m, x, _ = _case(shape, shape[3] % 3 != 0, True, dtype)
     with torch.no_grad():
         m.eval()
-        assert "forward_plane_kernel" in kernels_run(lambda: m(x))
+        assert "forward_flat_kernel" in kernels_run(lambda: m(x))
         out = m(x)
         want = m.double()(x.double())
     assert max_rel(out.double().cpu().numpy(), want.cpu().numpy()) < 1e-4 + ROUNDING[dtype]
+
+
+# (no room for scan corners in the tall ones)
+@pytest.mark.parametrize("shape", [(20, 1, 3, 72, 133), (20, 1, 4, 1020, 30), (20, 1, 3, 1024, 32), (20, 1, 3, 31, 1020), (19, 1, 3, 93, 157), (20, 2, 3, 126, 252)])
+def test_outputs_from_the_integral_image_alone(shape):
+    import box_convolution as bc
+    m, x, _ = _case(shape, True, True)
+    pixels = [p.detach() for p in m.get_actual_parameters()]
+    integ = bc.integral_image(x.double()).float()
+    assert kernels_run(lambda: bc.box_convolution_forward(integ, *pixels, True, True)) == ["forward_flat_kernel"]
+    out = bc.box_convolution_forward(integ, *pixels, True, True)
+    with torch.no_grad():
+        want = m.eval().double()(x.double())
+    assert max_rel(out.cpu().numpy(), want.cpu().numpy()) < 1e-4
+
+
+@pytest.mark.parametrize("shape", [(180, 1, 4, 96, 132), (180, 1, 4, 97, 133), (33, 1, 4, 96, 144), (20, 1, 8, 80, 188)])
+def test_gradients_from_the_integral_image_alone(shape):
+    """13 to 16 tiles: two a warp, and filters over clusters of as many CTAs as run at once."""
+    import box_convolution as bc
+    m, x, g = _case(shape, True, True)
+    pixels = [p.detach() for p in m.get_actual_parameters()]
+    integ = bc.integral_image(x.double()).float()
+
+    def grads():
+        return bc.box_convolution_backward(integ, *pixels, g, g, m.reparametrization_h, m.reparametrization_w, True, True, True, True, True, True, True)
+    assert "backward_plane_kernel" in kernels_run(grads)
+    got = grads()
+    want_in, want_p = _grads(m.double(), x.double(), g.double())
+    rounding = 8 * 2.0 ** -24 * float(integ.abs().max())      # (as below)
+    assert max_rel(got[0].cpu().numpy(), want_in.cpu().numpy()) < 1e-4
+    assert max_rel(torch.stack([t.double() for t in got[1:]]).cpu().numpy(), want_p.cpu().numpy()) < 1e-3 + rounding
 
 
 @pytest.mark.parametrize("shape", FORWARD)
@@ -105,6 +140,21 @@ def test_a_part_of_a_batch_gives_the_bits_of_the_whole(shape, kernels):
     for a, b in ((0, 1), (5, 8), (3, 40), (shape[0] - 30, shape[0])):
         part, _ = _grads(m, x[a:b], g[a:b])
         assert torch.equal(part, whole[a:b])
+
+
+@pytest.mark.parametrize("shape,same", [((64, 2, 3, 93, 157), True), ((16, 16, 4, 160, 64), False)])
+def test_outputs_of_a_part_of_a_batch(shape, same):
+    """Equal within a kernel; where few samples have another, equal to rounding."""
+    m, x, _ = _case(shape, True, True)
+    m.eval()
+    with torch.no_grad():
+        whole, part = m(x), m(x[3:5])
+        kernels = set(kernels_run(lambda: (m(x), m(x[3:5]))))
+    assert kernels == ({"forward_flat_kernel"} if same else {"forward_plane_kernel", "forward_flat_kernel"})
+    if same:
+        assert torch.equal(part, whole[3:5])
+    else:
+        assert max_rel(part.cpu().numpy(), whole[3:5].cpu().numpy()) < 1e-5
 
 
 @pytest.mark.parametrize("shape", [(2, 2, 2, 65, 61), (300, 1, 2, 21, 31), (1, 1, 2, 13, 300)])
