@@ -440,6 +440,7 @@ bool flat_fits_backward(int F, int h, int w)
     return flat_backward_plan(1, 1, F, h, w, true).smem <= kFlatMaxSmem;
 }
 
+// (Samples share a CTA only up to eight tiles of them and 56 KB of images: what holds one plane of more holds those.)
 bool flat_fits_forward(int F, int h, int w)
 {
     if (F > kMaxFilters || (int64_t)flat_strips(w) * flat_groups(h) > 32 * kFlatMaxTiles) return false;

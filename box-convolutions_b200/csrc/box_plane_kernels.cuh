@@ -627,9 +627,10 @@ inline size_t plane_backward_smem_bytes(int h, int w, bool need_params, bool sta
            (staged ? (size_t)h * w * io_bytes : 0);
 }
 
+// (A rule on numbers of planes and alignments chooses between the kernel in 32 x 32 tiles and strips, so the plane has to fit both.)
 inline bool plane_fits_forward(int F, int h, int w)
 {
-    return F <= kMaxFilters && warp_tiles(h, w) <= kMaxTiles && plane_forward_smem_bytes(h, w) <= kMaxSmem;
+    return F <= kMaxFilters && warp_tiles(h, w) <= kMaxTiles && plane_forward_smem_bytes(h, w) <= kMaxSmem && flat_fits_forward(F, h, w);
 }
 
 // Forward from the input's integral image: copying it to shared memory pays where several filters, or several CTAs an

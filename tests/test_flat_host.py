@@ -89,6 +89,21 @@ def test_layout(flat):
                     assert flat.flat_offset(h, w, group, a, j) == flat.flat_row(h, w, row), (h, w, group, a, j)
 
 
+# samples, channels, filters: around one and two CTAs an SM, and around the numbers of clusters that run at once
+@pytest.mark.parametrize("N,C,F", [(1, 1, 1), (1, 1, 32), (1, 3, 4), (7, 1, 8), (15, 1, 8), (16, 1, 8), (33, 1, 4), (9, 4, 6), (37, 2, 2), (148, 1, 32), (149, 1, 32), (33, 4, 2), (297, 1, 3), (3000, 2, 4)])
+def test_every_launch_fits(flat, N, C, F):
+    at, sizes = (ctypes.c_int64 * 2)(), ctypes.c_int64()
+    for gin in (0, 1):
+        assert not flat.flat_walk_backward(N, C, F, gin, at, ctypes.byref(sizes)), list(at)
+    assert not flat.flat_walk_forward(N, C, F, at, ctypes.byref(sizes)), list(at)
+    assert sizes.value > 100000
+
+
+def test_every_layout(flat):
+    at, sizes = (ctypes.c_int64 * 2)(), ctypes.c_int64()
+    assert not flat.flat_walk_layout(at, ctypes.byref(sizes)), list(at)
+
+
 @pytest.fixture(scope="module")
 def warp(tmp_path_factory):
     at = tmp_path_factory.mktemp("warp")
