@@ -440,8 +440,9 @@ inline FlatPlan flat_backward_plan(int N, int C, int F, int h, int w, bool write
     p.smem = flat_smem(p.sh, p.tiles_a_warp, F) + (size_t)F * p.warps * kNumSums * sizeof(float);
     const int slot = flat_slot_columns(p.tiles_a_warp, p.warps);
     const size_t rows = (size_t)p.sh.tiles * 32 * kFlatRows * 16;
-    // A cluster's CTAs have to find room at once, with no more than eight warps on an SM and the tensor memory that their filters take.
-    const int64_t room = 148 * (p.warps >= 8 ? 1 : 8 / p.warps);
+    // A cluster's CTAs have to find room at once, with no more than eight warps and four CTAs on an SM (eight of one warp: (510,1,2,22,20) 27.2 us, 19.7 without
+    // clusters; (141,1,8,39,19) 35.8, 29.7 in clusters of four) and the tensor memory that their filters take.
+    const int64_t room = 148 * (p.warps >= 8 ? 1 : p.warps <= 2 ? 4 : 8 / p.warps);
     const size_t own = p.smem;
     int64_t least = 0;
     for (int k = 1; k <= F && k <= kFlatMaxCluster; ++k) {

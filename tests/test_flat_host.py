@@ -64,6 +64,13 @@ def test_clusters_run_at_once(flat, planes, F, split, h, w):
     assert plan(flat, planes, 1, F, h, w)["split"] == split
 
 
+def test_small_ctas_share_an_sm_by_four(flat):
+    for h, w, warps in ((22, 20, 1), (39, 19, 1), (37, 60, 3), (70, 24, 2)):
+        for planes in (74, 141, 147, 272, 296, 510):
+            p = plan(flat, planes, 1, 8, h, w)
+            assert p["warps"] == warps and (p["split"] == 1 or planes * p["split"] <= 148 * (8 // warps if warps > 2 else 4)), (planes, p)
+
+
 def test_forward_launches_fit(flat):
     for h, w in served():
         for N, C, F in ((1, 1, 1), (1, 3, 4), (7, 1, 6), (150, 1, 32), (3000, 2, 4)):
