@@ -82,7 +82,7 @@ BUFFER_SETS = 4          # rotated between steps so that the footprint exceeds t
 NCU_TRAFFIC = {
     # profiles/plane_kernels_cfg2_ncu_full.md (batch 16: 4 194 304 input elements) and
     # profiles/plane_kernels_cfg5_dram_bytes.md (batch 256: 67 108 864 input elements)
-    "backward_plane_kernel": [(88.25e6, 4194304), (1591.1e6, 67108864)],
+    "backward_square_kernel": [(88.25e6, 4194304), (1591.1e6, 67108864)],
     "forward_plane_kernel": [(29.05e6, 4194304), (1281.5e6, 67108864)],
     # profiles/quad_slab_kernels_ncu.md
     "backward_quad_kernel": [(84.23e6, 4194304), (1589.4e6, 67108864)],
@@ -480,7 +480,9 @@ def kernel_algorithmic_bytes(kernel, N, C, F, h, w):
         "forward_tmem_stream_kernel": 4 * E * (1 + F),
         "backward_quad_pair_kernel": 4 * E * (F + 2),
         "forward_plane_kernel": 4 * E * (1 + F),
+        "forward_flat_kernel": 4 * E * (1 + F),
         "backward_plane_kernel": 4 * E * (F + 2),
+        "backward_square_kernel": 4 * E * (F + 2),
     }.get(kernel)
 
 

@@ -669,14 +669,13 @@ inline int quad_pair_max_threads(int col_tiles, int warps)
 }
 
 // Aligned planes with two tiles a warp, so with an even number of tiles.
-// 18 to 32 tiles in two columns (one column of them has no kernel of more than eight warps: 32 x 32 tiles).  In 16 bits, whose
-// 32 x 32-tile kernel leaves room for a second CTA, where these tiles waste little more than those ((10,16,4,96,160), 24 tiles for
-// 15: 67 us against 58; (10,16,4,80,240), 20 for 24: 68 against 105); float always ((55,16,4,128,156): 274, 351; (30,16,2,88,188):
-// 83, 121; (40,16,4,104,224): 215, 330).  But of at most 16 tiles of 32 x 32 an SM runs two planes, at about half the rate: a
-// round of 148 planes here then has to save half a round there, which it does in the first and the third, and with eight filters or
-// more in any.  Planes, filters, rows, columns: (84,4,96,144) 36 us, 46; (272,4,88,160) 70, 67; (360,8,80,152) 186, 219; (425,6,80,160)
-// 147, 160; (748,2,80,132) 116, 103; (1100,4,96,156) 285, 258; (722,16,88,136) 593, 692; in bfloat16 (564,4,88,140) 136, 128;
-// (1471,1,88,156) 129, 105; (592,16,72,140) 474, 501.
+// 18 to 32 tiles in two columns (one column of them has no kernel of more than eight warps: strips).  In 16 bits not where these tiles waste
+// half as much again as square ones ((10,16,4,96,160), 24 tiles for 15: 67 us against 58 in those; (10,16,4,80,240), 20 for 24: 68 against 105); float
+// always ((55,16,4,128,156): 274, 351; (30,16,2,88,188): 83, 121; (40,16,4,104,224): 215, 330).  Of at most 16 tiles of 32 x 32 (72 to 96 rows, 132 to 160
+// columns) strips take 0.60 to 1.00 of the time for any number of planes ((37,1,4,80,132) 34.0 us, 21.5; (1300,1,4,80,144) 306, 198), and with three filters
+// or more they have them (flat_beats_pair()).  With one or two the line by the number of planes is the one that was measured against 32 x 32 tiles, two
+// planes an SM at about half the rate, where a round of 148 planes here has to save half a round there: the first and the third do.  Strips would gain
+// there too: (148,1,2,72,136) 20.9, 18.2; (370,1,1,72,156) 36.6, 27.4.
 // 14 and 16 tiles, which as one tile a warp have an SM to themselves: two CTAs of half the warps, if there are planes for two
 // ((16,32,4,128,128): 94, 105; (16,32,4,64,256): 91, 108; (64,32,4,112,96): 258, 329).  Not of 10 and 12 tiles, two CTAs an SM either
 // way ((16,32,4,96,128): 73, 68; (16,32,4,40,248): 71, 65).
