@@ -34,6 +34,17 @@ def test_as_the_base_class(cls, args):
             assert p.grad is None or torch.equal(p.grad, q.grad), n
 
 
+@pytest.mark.parametrize("name,value", [("parameters", lambda m: iter([m.x_min])), ("named_parameters", lambda m: iter([("x_min", m.x_min)]))])
+def test_methods_set_on_the_object(name, value):
+    m, want = _module(), _module()
+    for each in (m, want):
+        setattr(each, name, lambda *args, each=each, **kwargs: value(each))
+    m.zero_grad()
+    torch.nn.Module.zero_grad(want)
+    assert want.x_min.grad is None and want.x_max.grad is not None
+    assert m.x_min.grad is None and m.x_max.grad is not None
+
+
 def test_submodules_and_parametrizations():
     m = _module()
     m.inner = torch.nn.Linear(2, 2)
