@@ -414,9 +414,14 @@ int launch_forward_flat_t(const IO *x, const float *integ, const BoxParams &bp, 
     void (*kern)(const IO *, const float *, BoxParams, IO *, int, int, int, int, int, FlatShape, int, int, bool, bool, bool, Fusion);
     auto pick = [&](auto vecs) {
         constexpr bool V = decltype(vecs)::value, FL = IsFloat<IO>::value;
-        // residual rows in flight want registers, unless they cost an SM its second CTA
-        if (fu) kern = plan.warps <= 10 || (plan.warps <= 20 && ctas * tsplit <= 148) ? forward_flat_kernel<IO, V, FL, false, 640> : forward_flat_kernel<IO, V, FL, false, 1024>;
-        else kern = x ? forward_flat_kernel<IO, V, false, false, 1024> : forward_flat_kernel<IO, V, false, FL, 1024>;
+        if constexpr (FL) {      // (the fused steps are float's)
+            // residual rows in flight want registers, unless they cost an SM its second CTA
+            if (fu) {
+                kern = plan.warps <= 10 || (plan.warps <= 20 && ctas * tsplit <= 148) ? forward_flat_kernel<IO, V, true, false, 640> : forward_flat_kernel<IO, V, true, false, 1024>;
+                return;
+            }
+        }
+        kern = x ? forward_flat_kernel<IO, V, false, false, 1024> : forward_flat_kernel<IO, V, false, FL, 1024>;
     };
     if (fast) pick(Flag<true>{});
     else pick(Flag<false>{});
